@@ -486,16 +486,45 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     emit(a, t4);
 }
 
+// ---- renormalisation shift ----------------------------------------------------------------------------
+// After a range update the reference shifts while low and high agree in their top bit, then while low
+// starts 01 and high 10 (enc_new.cu:275-293, dec_new.cu:284-301).  Both kinds double the interval, and
+// together they stop at the largest s for which [low, high] lies inside a window of 2^(32-s) values that
+// starts at a multiple of half its size (the midpoint windows of the second kind included).  With
+// d = high - low and b the position of d's top bit, that is 32-s = b+1 when [low, high] touches only two
+// cells of 2^b values and b+2 when it touches three, and it touches three exactly when the low b bits
+// of low and of d carry into bit b.  So 32-s = b + 1 + carry: one leading-bit search, two shifts that move
+// the b low bits to the top of a word, an add for its carry and an add that takes it.  Only the bits of
+// low below b matter, so low may carry anything in its top bit after the shift.
+CG_HD uint32_t renorm_right_shift(uint32_t low, uint32_t d) {
+#if defined(__CUDA_ARCH__)
+    uint32_t n, b;
+    asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(d));
+    const uint32_t l = __funnelshift_r(0u, low, b), m = __funnelshift_r(0u, d, b);
+    asm("{ .reg .u32 t; add.cc.u32 t, %1, %2; addc.u32 %0, %3, 1; }" : "=r"(n) : "r"(l), "r"(m), "r"(b));
+    return n;
+#else
+    const uint32_t b = 31u - static_cast<uint32_t>(cg_clz(d));
+    const uint32_t l = (b & 31u) ? low << (32u - (b & 31u)) : 0u, m = (b & 31u) ? d << (32u - (b & 31u)) : 0u;
+    return b + 1u + (l + m < l ? 1u : 0u);
+#endif
+}
+
 // ---- MSB-first bit writer into one scratch row (add_bits_to_output, enc_new.cu:21-97) ---------------------
 // Output bits collect in a 64-bit accumulator.  Whole 32-bit words leave it, big-endian, into the
 // stream's scratch row; the common case does that for the whole warp at once (see EncoderState::step)
 // so that the store is not a per-lane branch.
+//
+// The bits are those of the interval's lower end as one long binary fraction, so a later range update can
+// still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above them (a
+// word leaves nothing behind it) and is added to the stored words when the next word goes out; that
+// takes a run of ones from there to the last stored word, which real tables about never give.
 struct BitSink {
     uint32_t *row;    // 4-byte aligned scratch row of this stream
     uint32_t cap_w;   // words that fit in the row
     uint32_t nwords;  // words produced so far (may exceed cap_w: then nothing more is stored)
-    uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo)
-    uint32_t nacc;            // number of bits pending, < 64
+    uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo), and a carry above them
+    uint32_t nacc;            // number of bits pending, < 63
 
     CG_HD void init(uint8_t *p, int64_t stride) {
         row = reinterpret_cast<uint32_t *>(p);
@@ -505,44 +534,34 @@ struct BitSink {
         acc_lo = 0;
         nacc = 0;
     }
-    // appends the low n bits of v (v has no bits above n), n <= 32; needs nacc + n <= 64
-    CG_HD void put(uint32_t v, uint32_t n) {
-        acc_hi = cg_fshl_clamp(acc_lo, acc_hi, n);
-        acc_lo = cg_shl(acc_lo, n) | v;
-        nacc += n;
+    // adds one to the number that the stored words form
+    CG_HD void carry_into_row() {
+        if (nwords > cap_w) return;  // the words before are not in the row: reported as an overflow
+        for (uint32_t i = nwords; i > 0u;) {
+            --i;
+            const uint32_t v = cg_bswap32(row[i]) + 1u;
+            row[i] = cg_bswap32(v);
+            if (v) return;
+        }
     }
-    // the same for n < 32 (what the straight-line encoder step appends): plain funnel shifts
-    CG_HD void put_short(uint32_t v, uint32_t n) {
-        acc_hi = cg_fshl(acc_lo, acc_hi, n);
-        acc_lo = acc_lo * cg_shl(1u, n) + v;  // a multiply-add for shift and or: off the integer pipe, which binds the encoder
-        nacc += n;
-    }
-    // moves the oldest 32 bits out; needs nacc >= 32
+    // moves the oldest 32 bits out; needs 32 <= nacc < 63
     CG_HD void store_word() {
         nacc -= 32u;
-        const uint32_t w = cg_fshr_clamp(acc_lo, acc_hi, nacc);  // nacc < 32: the low word of (hi:lo) >> nacc
+        const uint32_t w = cg_fshr_clamp(acc_lo, acc_hi, nacc);  // the low word of (hi:lo) >> nacc
+        if (cg_fshr_clamp(acc_hi, 0u, nacc)) carry_into_row();
+        acc_hi = 0u;
+        acc_lo &= ~cg_shl(0xFFFFFFFFu, nacc);
         if (nwords < cap_w) row[nwords] = cg_bswap32(w);
         nwords++;
     }
-    CG_HD void drain() {
-        while (nacc >= 32u) store_word();
-    }
-    // `count` copies of `bit`, any count
-    CG_HD void put_run(uint32_t bit, uint32_t count) {
-        const uint32_t ones = 0u - bit;  // 0 or 0xFFFFFFFF
-        while (count) {
-            drain();
-            const uint32_t n = count < 32u ? count : 32u;
-            put(ones >> (32u - n), n);
-            count -= n;
-        }
-    }
     // zero-fills to a byte boundary; returns the stream length in bytes
     CG_HD uint32_t finish() {
-        drain();
+        if (nacc > 62u) nacc = 62u;  // only a table that does not increase gets here
+        if (nacc >= 32u) store_word();
+        if (cg_fshr_clamp(acc_lo, acc_hi, nacc)) carry_into_row();
         const uint32_t bytes = nwords * 4u + ((nacc + 7u) >> 3);
         if (nacc) {
-            const uint32_t w = acc_lo << (32u - nacc);  // after drain: 0 < nacc < 32
+            const uint32_t w = acc_lo << (32u - nacc);
             if (nwords < cap_w) row[nwords] = cg_bswap32(w);
         }
         return bytes;
@@ -550,131 +569,63 @@ struct BitSink {
 };
 
 // ---- encoder state and step -----------------------------------------------------------------------------
-constexpr uint32_t kSinkHighWater = 48;  // a symbol starts with fewer bits than this in the accumulator
-constexpr uint32_t kFastEmitBits = 16;   // ... so up to this many more fit without a store
+// A symbol starts with fewer bits than this in the accumulator; it adds at most 18 (the updated interval of a
+// strictly increasing table spans at least 2^14 values), which leaves room for a carry.
+constexpr uint32_t kSinkHighWater = 44;
 
+// The coder without the reference's count of pending bits.  low is the current 32-bit window of the
+// interval's lower end L, and all bits of L above the window are in the sink: a range update adds to
+// low and carries into the sink, a shift by s moves low's top s bits there.  The reference's underflow
+// shifts (low = 01..., high = 10...: drop the second bit, remember one pending bit) are the same
+// shift: the bits they leave open are 01..1 in L here, with the last 1 as low's top bit, and become
+// 10..0 by the carry exactly when the reference decides for a 1 followed by zeros.
 struct EncoderState {
-    uint32_t low, span32, pending;  // span32 = (high - low + 1) mod 2^32, 0 for the full range
-    // 1 and -1 as values the compiler cannot see through (the kernel reads them from constant memory):
-    // a + b written as a * one + b is a multiply-add, which keeps it off the integer pipe that binds the
-    // encoder's step; a plain a + b would be folded back into an integer add
-    uint32_t one, minus_one;
-    CG_HD void init(uint32_t opaque_one = 1u, uint32_t opaque_minus_one = 0xFFFFFFFFu) {
+    uint32_t low, span32;  // span32 = (high - low + 1) mod 2^32, 0 for the full range
+    CG_HD void init() {
         low = 0u;
         span32 = 0u;
-        pending = 0u;
-        one = opaque_one;
-        minus_one = opaque_minus_one;
     }
-    CG_HD uint32_t add_f(uint32_t a, uint32_t b) const { return a * one + b; }
-    CG_HD uint32_t sub_f(uint32_t a, uint32_t b) const { return b * minus_one + a; }  // a - b
-    // One symbol s in [0, maxsym] (enc_new.cu:257-295), any state, any number of output bits; stores
-    // whole words as needed but leaves up to 63 bits in the accumulator.  The table column must have
-    // a readable row after the last symbol's.
-    CG_HD void step_general(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, BitSink &out) {
-        const uint32_t a = col + s * kTableRowBytes;
-        const uint32_t flo = scale_exact(span32, sm.ld(a));
-        const uint32_t fnext = scale_exact(span32, sm.ld(a + kTableRowBytes));
-        const uint32_t fhi = (s == maxsym) ? span32 : fnext;
-        low += flo;
-        span32 = fhi - flo;
-        const uint32_t high = low + span32 - 1u;
-        // equal-top-bit shifts: their n1 bits are low's top bits; the first is followed by the pending
-        // (inverted) bits of earlier underflow shifts (enc_new.cu:275-287)
-        const uint32_t n1 = static_cast<uint32_t>(equal_shifts(low, high));
-        if (n1) {
-            const uint32_t bits = low >> (32u - n1);
-            const uint32_t first = bits >> (n1 - 1u);
-            const uint32_t rest = bits & ((1u << (n1 - 1u)) - 1u);
-            out.drain();
-            out.put(first, 1u);
-            out.put_run(1u - first, pending);
-            out.drain();
-            out.put(rest, n1 - 1u);
-            pending = 0u;
-        }
-        // underflow shifts (enc_new.cu:288-293) only raise the pending count; both kinds of shift
-        // double the span
-        const uint32_t k = static_cast<uint32_t>(cg_clz(((((~low) | high) << n1) << 1) | 1u));
-        pending += k;
-        const uint32_t sh = (n1 + k) & 31u;
-        low = (low << sh) & 0x7FFFFFFFu;
-        span32 <<= sh;
+    CG_HD void add_to_low(uint32_t v, BitSink &out) {
+#if defined(__CUDA_ARCH__)
+        asm("add.cc.u32 %0, %0, %3; addc.cc.u32 %1, %1, 0; addc.u32 %2, %2, 0;"
+            : "+r"(low), "+r"(out.acc_lo), "+r"(out.acc_hi) : "r"(v));
+#else
+        low += v;
+        if (low < v && ++out.acc_lo == 0u) ++out.acc_hi;
+#endif
     }
-    // The same symbol in straight-line code for the usual case -- the range is not the full 2^32 (it is
-    // only for a stream's first symbol, and after a shift that lands on it exactly) and at most
-    // kFastEmitBits bits come out.  step_try does the step on that assumption and says whether it held
-    // (`before` keeps what is needed to take the step again); step_finish repairs a lane for which
-    // it did not, through step_general, and stores a full word of the accumulator.  Between the two
-    // goes ONE warp vote (see step), so that neither the repair nor the store is a per-lane branch in
-    // the usual case.
-    struct Before {
-        uint32_t low, span32, pending, nacc, acc_hi, acc_lo;
-    };
-    CG_HD bool step_try(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, BitSink &out, Before &before) {
-        before.low = low;
-        before.span32 = span32;
-        before.pending = pending;
-        before.nacc = out.nacc;
-        before.acc_hi = out.acc_hi;
-        before.acc_lo = out.acc_lo;
-        const uint32_t a = col + s * kTableRowBytes;
-        const uint32_t flo = cg_umulhi(span32, sm.ld(a));
-        const uint32_t fnext = cg_umulhi(span32, sm.ld(a + kTableRowBytes));
-        const uint32_t fhi = (s == maxsym) ? span32 : fnext;
-        low = add_f(low, flo);
-        span32 = sub_f(fhi, flo);
-        const uint32_t high = low + span32 - 1u;
-        // low == high (32 here) and k == 32 below only come from a table that is not increasing: the first
-        // sends the lane to the general path (total > kFastEmitBits), the second makes the shifts give 0
-        const uint32_t n1 = static_cast<uint32_t>(cg_clz(low ^ high));
-        const uint32_t y = cg_shl((~low) | high, n1);
-        const uint32_t k = static_cast<uint32_t>(cg_clz(y + y));
-        // Output when n1 != 0: low's top bit, then the pending bits as its inverse, then low's next
-        // n1 - 1 bits.  As a number that is (2^q - 1) * 2^(n1 - 1) + (low's top n1 bits), q the pending
-        // count: the sum carries into the top bit's place exactly when that bit is 1.  With n1 == 0 nothing
-        // goes out: q is taken as 0 then, which makes the value 0 and the bit count 0 without a mask.  A
-        // lane that has to take the step again may append anything: step_finish puts its accumulator back.
-        const uint32_t q = n1 ? pending : 0u;
-        const uint32_t nput = add_f(n1, q);
-        const bool redo = (before.span32 == 0u) | (nput > kFastEmitBits);
-        const uint32_t ones = cg_shl(1u, q) - 1u;
-        out.put_short(cg_shl(ones, n1 - 1u) + cg_fshl(low, 0u, n1), nput);
-        pending = add_f(sub_f(pending, q), k);
-        const uint32_t sh = add_f(n1, k);  // at most 18 with an increasing table
-        const uint32_t p2 = cg_shl(1u, sh);  // one shift and two multiplies for two shifts: see put_short
-        low = (low * p2) & 0x7FFFFFFFu;
-        span32 = span32 * p2;
-        return redo;
-    }
-    CG_HD void step_finish(bool redo, const Before &before, Smem sm, uint32_t col, uint32_t s, uint32_t maxsym,
-                           BitSink &out) {
-        if (redo) {
-            low = before.low;
-            span32 = before.span32;
-            pending = before.pending;
-            out.acc_hi = before.acc_hi;
-            out.acc_lo = before.acc_lo;
-            out.nacc = before.nacc;
-            step_general(sm, col, s, maxsym, out);
-        }
-        if (out.nacc >= 32u) out.store_word();
-    }
-    // One symbol of one stream per lane.  lanes: the warp's lanes that encode together (same token
-    // count).  Every lane with a full word stores it as soon as one lane is near the accumulator's
-    // high-water mark.
+    // One symbol s of one stream per lane (enc_new.cu:257-295), s <= maxsym.  lanes: the warp's lanes that
+    // encode together (same token count).  ONE warp vote a symbol covers what is rare: a full word in the
+    // accumulator (every lane that has one stores it as soon as one lane is near the high-water mark), the
+    // full 2^32 range (a stream's first symbol; later only if a shift lands on it exactly) and the table's last
+    // symbol, whose upper bound is the range's end.
     CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, BitSink &out, uint32_t lanes) {
-        Before before;
-        const bool redo = step_try(sm, col, s, maxsym, out, before);
-        if (cg_any_lane(lanes, redo || out.nacc >= kSinkHighWater)) step_finish(redo, before, sm, col, s, maxsym, out);
+        const uint32_t a = col + s * kTableRowBytes;
+        const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + kTableRowBytes);
+        uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
+        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (s == maxsym))) {
+            if (out.nacc >= 32u) out.store_word();
+            flo = scale_exact(span32, e0);
+            fhi = s == maxsym ? span32 : scale_exact(span32, e1);
+        }
+        add_to_low(flo, out);
+        span32 = fhi - flo;
+        const uint32_t n = renorm_right_shift(low, span32 - 1u);
+        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, n);
+        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, n);
+        low = cg_fshr_clamp(0u, low, n);
+        span32 = cg_fshr_clamp(0u, span32, n);
+        out.nacc += 32u - n;
     }
-    // final flush (enc_new.cu:298-306); returns the stream length in bytes
+    // final flush (enc_new.cu:298-306): two bits that place the stream's value inside the interval, 01 or
+    // 10 above the reference's low with its pending bits, which is L plus a quarter of the window cut
+    // to two bits; returns the stream length in bytes
     CG_HD uint32_t flush(BitSink &out) {
-        pending += 1u;
-        const uint32_t last = (low < 0x40000000u) ? 0u : 1u;
-        out.drain();
-        out.put(last, 1u);
-        out.put_run(1u - last, pending);
+        add_to_low(0x40000000u, out);
+        if (out.nacc >= 32u && out.nacc < 63u) out.store_word();
+        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, 30u);
+        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, 30u);
+        out.nacc += 2u;
         return out.finish();
     }
 };
