@@ -89,9 +89,6 @@ CG_HD uint32_t cg_load_stream_word(const uint32_t *p) {
 #endif
 }
 
-// Count of equal-top-bit shifts for the interval [low, high] (the |1 keeps it below 32 on a
-// degenerate interval, which only a corrupt table can produce).
-CG_HD int equal_shifts(uint32_t low, uint32_t high) { return cg_clz((low ^ high) | 1u); }
 // ---- shared-memory access --------------------------------------------------------------------------------
 // A stream's table is the column tab[m][tid] = cdf[m] << 16 of a [rows][128] uint32 array, addressed
 // by byte address: entry m of the column starting at `col` is at col + m * kTableRowBytes.  On the
@@ -113,6 +110,40 @@ struct Smem {
     void st(uint32_t addr, uint32_t v) const { *reinterpret_cast<uint32_t *>(base + addr) = v; }
 #endif
 };
+
+// ---- renormalisation shift ----------------------------------------------------------------------------
+// After a range update the reference shifts while low and high agree in their top bit, then while low
+// starts 01 and high 10 (enc_new.cu:275-293, dec_new.cu:284-301).  Both kinds double the interval, and
+// together they stop at the largest s for which [low, high] lies inside a window of 2^(32-s) values that
+// starts at a multiple of half its size (the midpoint windows of the second kind included).  With
+// d = high - low and b the position of d's top bit, that is 32-s = b+1 when [low, high] touches only two
+// cells of 2^b values and b+2 when it touches three, and it touches three exactly when the low b bits
+// of low and of d carry into bit b.  So 32-s = b + 1 + carry: one leading-bit search, two shifts that move
+// the b low bits to the top of a word, an add for its carry and an add that takes it.  Only the bits of
+// low below b matter, so low may carry anything in its top bit after the shift.
+//
+// Returns n = 32 - s for the funnel shifts that take other words' bits in, and 2^s for the words that are
+// only shifted left, where a multiply does it off the integer pipe (the pipe that binds the coders: a
+// shift, a compare or a select takes it for two cycles a warp, and so does a multiply-high).
+struct Renorm {
+    uint32_t n, p2;
+};
+CG_HD Renorm renorm_shift(uint32_t low, uint32_t d) {
+    Renorm r;
+#if defined(__CUDA_ARCH__)
+    uint32_t b;
+    asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(d));
+    const uint32_t q = __funnelshift_r(0u, 1u, b);  // 2^(32-b)
+    asm("{ .reg .u32 t; add.cc.u32 t, %1, %2; addc.u32 %0, %3, 1; }" : "=r"(r.n) : "r"(low * q), "r"(d * q), "r"(b));
+    r.p2 = __funnelshift_rc(0u, 1u, r.n);
+#else
+    const uint32_t b = 31u - static_cast<uint32_t>(cg_clz(d));
+    const uint32_t q = (b & 31u) ? 1u << (32u - (b & 31u)) : 0u;
+    r.n = b + 1u + (low * q + d * q < d * q ? 1u : 0u);
+    r.p2 = cg_fshr_clamp(0u, 1u, r.n);
+#endif
+    return r;
+}
 
 // ---- register bit window + warp-synchronous refill -----------------------------------------------------------
 // The next 96 unread bits of the stream live in three registers.  The byte array is read as aligned
@@ -167,12 +198,12 @@ struct BitWindow {
         next = 4;
         return cg_fshl(w1, w0, off);
     }
-    // drops the s (< 32) bits just shifted into the coder's value
-    CG_HD void consume(uint32_t s) {
-        hi = cg_fshl(mid, hi, s);
-        mid = cg_fshl(lo, mid, s);
-        lo <<= s;
-        nbits -= static_cast<int>(s);
+    // drops the bits just shifted into the coder's value
+    CG_HD void consume(Renorm r) {
+        hi = cg_fshr_clamp(mid, hi, r.n);
+        mid = cg_fshr_clamp(lo, mid, r.n);
+        lo *= r.p2;
+        nbits += static_cast<int>(r.n) - 32;
     }
     CG_HD bool low_water() const { return nbits <= 32; }
     // fewer valid bits than one symbol can take: a range update shifts by at most 18 bits when the
@@ -211,36 +242,6 @@ struct BitWindow {
 // exactly when the range is the full 2^32 (then the product is c16 itself).
 CG_HD uint32_t scale_exact(uint32_t span32, uint32_t c16) { return span32 ? cg_umulhi(span32, c16) : c16; }
 
-// Search steps of the fast path (span32 != 0): the candidate entry is IMM bytes above `a`.
-template <int B>
-struct FastSearch {
-    static CG_HD uint32_t run(Smem sm, uint32_t a, uint32_t span32, uint32_t target) {
-        const uint32_t ca = a + (static_cast<uint32_t>(kTableRowBytes) << B);
-        a = cg_umulhi(span32, sm.ld(ca)) <= target ? ca : a;
-        return FastSearch<B - 1>::run(sm, a, span32, target);
-    }
-};
-template <>
-struct FastSearch<-1> {
-    static CG_HD uint32_t run(Smem, uint32_t a, uint32_t, uint32_t) { return a; }
-};
-
-// Exact, clamped search: any table length, any span; candidates above the last symbol are never taken
-// (and never read).
-template <int B>
-struct ExactSearch {
-    static CG_HD uint32_t run(Smem sm, uint32_t a, uint32_t a_max, uint32_t span32, uint32_t target) {
-        const uint32_t ca = a + (static_cast<uint32_t>(kTableRowBytes) << B);
-        const bool ok = ca <= a_max;
-        const bool take = ok && (scale_exact(span32, sm.ld(ok ? ca : a)) <= target);
-        return ExactSearch<B - 1>::run(sm, take ? ca : a, a_max, span32, target);
-    }
-};
-template <>
-struct ExactSearch<-1> {
-    static CG_HD uint32_t run(Smem, uint32_t a, uint32_t, uint32_t, uint32_t) { return a; }
-};
-
 // The decoder's arithmetic state: low, span32 = (high - low + 1) mod 2^32 and offset = value - low.
 // In this form both kinds of renormalisation shift act alike on the pair (offset, span) --
 // offset = 2*offset + next bit, span = 2*span -- so the reference's "value -= 2^30" of the underflow
@@ -250,106 +251,21 @@ struct DecoderState {
     uint32_t low, span32, offset;
 
     // range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation
-    // (dec_new.cu:277-301): equal-top-bit shifts and underflow shifts applied in one go
+    // (dec_new.cu:277-301), both kinds of shift applied in one go.  On a table that is not increasing the
+    // shift count is anything up to 32; every later read stays inside the table column and the stream.
     CG_HD void update(uint32_t flo, uint32_t fhi, BitWindow &bw) {
         offset -= flo;
         low += flo;
         span32 = fhi - flo;
-        const uint32_t high = low + span32 - 1u;
-        const uint32_t n1 = static_cast<uint32_t>(equal_shifts(low, high));
-        const uint32_t k = static_cast<uint32_t>(cg_clz(((((~low) | high) << n1) << 1) | 1u));
-        const uint32_t s = n1 + k;  // at most 18 for any strictly increasing table; shifts below wrap at 32
-        // The reference also clears low's top bit after underflow shifts.  Here low is only ever
-        // compared with high = low + span - 1 bit by bit, offset carries value - low separately, and
-        // a set top bit flips the top bit of low and high alike: it changes neither shift count.
-        low = cg_fshl(0u, low, s);
-        span32 = cg_fshl(0u, span32, s);
-        offset = cg_fshl(bw.hi, offset, s);
-        bw.consume(s);
+        const Renorm r = renorm_shift(low, span32 - 1u);
+        low *= r.p2;
+        span32 *= r.p2;
+        offset = cg_fshr_clamp(bw.hi, offset, r.n);
+        bw.consume(r);
     }
 };
 
-// The same update for the decode_streams loop: no "| 1" guards on the two leading-zero counts.  With a
-// strictly increasing table the updated interval spans at least 2^14 values, so neither operand can be
-// zero; on a corrupt table a count of 32 only makes the shifts below wrap, and every later read stays
-// inside the table column and the stream.
-CG_HD void update_unguarded(DecoderState &st, uint32_t flo, uint32_t fhi, BitWindow &bw) {
-    st.offset -= flo;
-    st.low += flo;
-    st.span32 = fhi - flo;
-    const uint32_t high = st.low + st.span32 - 1u;
-    const uint32_t n1 = static_cast<uint32_t>(cg_clz(st.low ^ high));
-    const uint32_t y = cg_shl((~st.low) | high, n1);  // top bit set: low has 0 and high 1 at the first bit they differ in
-    const uint32_t s = n1 + static_cast<uint32_t>(cg_clz(y + y));
-    st.low = cg_fshl(0u, st.low, s);
-    st.span32 = cg_fshl(0u, st.span32, s);
-    st.offset = cg_fshl(bw.hi, st.offset, s);
-    bw.consume(s);
-}
-
-// One stream.  col: address of the stream's table column, entries cdf << 16, rows kTableRowBytes apart,
-// one readable row past the last symbol's; emit(a) receives, token after token, the address of the
-// decoded symbol's table entry (symbol = (a - col) / kTableRowBytes).  lanes: the warp's lanes that
-// run this loop together (they must all have the same ntok).
-// LEVELS: search depth, 2^LEVELS >= maxsym + 1.  POW2: 2^LEVELS == maxsym + 1 (with LEVELS >= 3): the
-// middle symbols then take the fast path -- entries of the first two search levels in registers,
-// no bound checks, one multiply-high per step -- and leave it only for a symbol that starts from the
-// full 2^32 range (the first one, and about never again), which the exact path decodes.
-template <int LEVELS, bool POW2, class Emit>
-CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *stream, uint32_t len, int ntok,
-                         uint32_t lanes, Emit emit) {
-    BitWindow bw;
-    DecoderState st;
-    st.low = 0u;
-    st.span32 = 0u;
-    st.offset = bw.open(stream, len);
-    const uint32_t a_max = col + static_cast<uint32_t>(maxsym) * kTableRowBytes;
-
-    // exact step; with_update = false for the last symbol (dec_new.cu:273-275)
-    auto exact_step = [&](bool with_update) {
-        const uint32_t a = ExactSearch<LEVELS - 1>::run(sm, col, a_max, st.span32, st.offset);
-        emit(a);
-        if (with_update) {
-            const uint32_t flo = scale_exact(st.span32, sm.ld(a));
-            const uint32_t fhi = (a == a_max) ? st.span32 : scale_exact(st.span32, sm.ld(a + kTableRowBytes));
-            st.update(flo, fhi, bw);
-        }
-    };
-
-    constexpr bool kFast = POW2 && LEVELS >= 3;
-    constexpr uint32_t kTop = static_cast<uint32_t>(kTableRowBytes) << (LEVELS > 0 ? LEVELS - 1 : 0);
-    constexpr uint32_t kHalf = kTop >> 1;
-    uint32_t r_mid = 0u, r_lo = 0u, r_hi = 0u;
-    if (kFast) {
-        r_mid = sm.ld(col + kTop);
-        r_lo = sm.ld(col + kHalf);
-        r_hi = sm.ld(col + kTop + kHalf);
-    }
-    for (int left = ntok - 1; left > 0; --left) {
-        // rare, and taken by the whole warp: a lane is low on bits, or starts this symbol from the full range
-        if (cg_any_lane(lanes, bw.low_water() || (kFast && st.span32 == 0u)) || !kFast) {
-            if (cg_any_lane(lanes, bw.low_water())) bw.refill();
-            if (!kFast || cg_any_lane(lanes, st.span32 == 0u)) {
-                exact_step(true);
-                continue;
-            }
-        }
-        // levels 1 and 2 from registers, the rest from the table column
-        const bool t1 = cg_umulhi(st.span32, r_mid) <= st.offset;
-        uint32_t a = t1 ? col + kTop : col;
-        const bool t2 = cg_umulhi(st.span32, t1 ? r_hi : r_lo) <= st.offset;
-        a = t2 ? a + kHalf : a;
-        a = FastSearch<(kFast ? LEVELS - 3 : -1)>::run(sm, a, st.span32, st.offset);
-        emit(a);
-        const uint32_t flo = cg_umulhi(st.span32, sm.ld(a));
-        const uint32_t fnext = cg_umulhi(st.span32, sm.ld(a + kTableRowBytes));
-        st.update(flo, (a == a_max) ? st.span32 : fnext, bw);
-    }
-    if (cg_any_lane(lanes, bw.low_water())) bw.refill();
-    exact_step(false);
-}
-
-// ---- decode loop, NS streams per lane, search depth chosen by the caller ---------------------------------
+// ---- decode loop: NS streams per lane, search depth chosen by the caller ---------------------------------
 // Exact search with a run-time depth (the rare path of decode_streams).
 CG_HD uint32_t exact_search(Smem sm, uint32_t col, uint32_t a_max, uint32_t span32, uint32_t target, int levels) {
     uint32_t a = col;
@@ -370,31 +286,65 @@ CG_HD int fast_levels_for(int nsym, int full_levels) {
     return fl;
 }
 
+// offset / span as a 32-bit fraction, to about 2^-22 (the low nine bits are zero); anything when the span is the
+// full 2^32 (span32 == 0).
+CG_HD uint32_t ratio_estimate(uint32_t offset, uint32_t span32) {
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_rn(span32)));
+    return __float_as_uint(__fmaf_rn(__uint2float_rn(offset), r, 1.0f)) * 512u;  // the 23 bits after the point, at the top
+#else
+    const float q = span32 ? static_cast<float>(offset) / static_cast<float>(span32) + 1.0f : 1.0f;
+    uint32_t bits;
+    __builtin_memcpy(&bits, &q, 4);
+    return bits * 512u;
+#endif
+}
+
+// Search steps on a ratio estimate: the candidate entry is kTableRowBytes << B bytes above `a`.
+template <int B>
+struct RatioSearch {
+    static CG_HD uint32_t run(Smem sm, uint32_t a, uint32_t ratio) {
+        const uint32_t ca = a + (static_cast<uint32_t>(kTableRowBytes) << B);
+        a = sm.ld(ca) <= ratio ? ca : a;
+        return RatioSearch<B - 1>::run(sm, a, ratio);
+    }
+};
+template <>
+struct RatioSearch<-1> {
+    static CG_HD uint32_t run(Smem, uint32_t a, uint32_t) { return a; }
+};
+
 // NS streams of one lane decoded side by side (same token count, same table length), the fast
 // search limited to the first 2^FL table entries.
 //
-// The caller picks FL from what it knows about the symbols (a row quantised to `bins` bins holds
-// symbols 0 .. bins-2, so 2^FL >= bins is enough); the result never depends on that choice: a fast
-// search that ends on or above entry D = min(2^FL - 1, maxsym) -- the only way a symbol >= D, a
-// symbol that starts from the full 2^32 range (span32 == 0 makes every comparison true) or a probe
-// of a padding entry can show -- is thrown away and the whole warp repeats that symbol with the
-// exact, full-depth search.  Entries above maxsym must be staged as 0xFFFFFFFF (never "<= offset"
-// unless offset is span-1, which then lands above D) and the column needs 2^FL + 1 readable rows.
+// The fast search compares the table entries with an estimate of offset / span, which costs one compare a
+// level where the scaled entry costs a multiply-high as well (four cycles of the multiply pipe and two of the
+// integer pipe a warp, measured).  The symbol is then checked exactly: the offset must lie inside its scaled
+// bounds, which the range update needs anyway.  The caller picks FL from what it knows about the symbols (a
+// row quantised to `bins` bins holds symbols 0 .. bins-2, so 2^FL >= bins is enough).  The result depends
+// on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol
+// >= 2^FL - 1, a symbol that starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away
+// and the whole warp repeats that symbol with the exact, full-depth search.
+//
+// The table's last symbol has no upper entry.  With LAST_REPEATED the rows above its entry hold copies of it,
+// so that its bounds are equal and the check fails; otherwise they hold 0xFFFFFFFF (never "<= ratio") and
+// a symbol at or above the address threshold det is repeated as well.  The column needs 2^FL + 1
+// readable rows either way.
 //   col[i]    table column of stream i (see decode_stream)
-//   det       address threshold of entry D: column-independent because a column's offset inside a
-//             table row is below kTableRowBytes (det = table base + D * kTableRowBytes)
+//   det       address threshold of entry min(2^FL - 1, maxsym): column-independent because a column's offset
+//             inside a table row is below kTableRowBytes (det = table base + entry * kTableRowBytes)
 //   emit(a, t4)  receives the NS table-entry addresses of one token's symbols and four times the
 //             token's index (ntok >= 1)
-template <int FL, int NS, class Emit>
+template <int FL, int NS, bool LAST_REPEATED = false, class Emit>
 CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int maxsym, int full_levels,
                           const uint8_t *const (&stream)[NS], const uint32_t (&len)[NS], int ntok, uint32_t lanes,
                           Emit emit) {
-    static_assert(FL >= 2, "the first two levels are held in registers");
+    static_assert(FL >= 2, "the first level's entry is held in a register");
     BitWindow bw[NS];
     DecoderState st[NS];
-    uint32_t r_mid[NS], r_lo[NS], r_hi[NS], a_max[NS], col_top[NS];
+    uint32_t r_mid[NS], a_max[NS], col_top[NS];
     constexpr uint32_t kTop = static_cast<uint32_t>(kTableRowBytes) << (FL - 1);
-    constexpr uint32_t kHalf = kTop >> 1;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
@@ -405,30 +355,27 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
         a_max[i] = col[i] + static_cast<uint32_t>(maxsym) * kTableRowBytes;
         col_top[i] = col[i] + kTop;
         r_mid[i] = sm.ld(col[i] + kTop);
-        r_lo[i] = sm.ld(col[i] + kHalf);
-        r_hi[i] = sm.ld(col[i] + kTop + kHalf);
     }
     uint32_t a[NS];
     // One back edge and one vote per token: the rare path (a refill of the bit windows, or the exact
-    // search when the fast one cannot be trusted) only tops the windows up or replaces the symbol and
+    // search when the fast one failed) only tops the windows up or replaces the symbol and
     // its scaled bounds; the range update below is shared.
     const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
     uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
     for (; t4 != last4; t4 += 4u) {
-        uint32_t flo[NS], fhi[NS];
-        bool rare = false;  // a lane short of bits, or a search that ended on or above entry D
+        uint32_t flo[NS], fhi[NS], ratio[NS];
+        bool rare = false;  // a lane short of bits, or a symbol that fails the check
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
         for (int i = 0; i < NS; ++i) {
-            const bool t1 = cg_umulhi(st[i].span32, r_mid[i]) <= st[i].offset;
-            uint32_t x = t1 ? col_top[i] : col[i];
-            a[i] = cg_umulhi(st[i].span32, t1 ? r_hi[i] : r_lo[i]) <= st[i].offset ? x + kHalf : x;
+            ratio[i] = ratio_estimate(st[i].offset, st[i].span32);
+            a[i] = r_mid[i] <= ratio[i] ? col_top[i] : col[i];
         }
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-        for (int i = 0; i < NS; ++i) a[i] = FastSearch<FL - 3>::run(sm, a[i], st[i].span32, st[i].offset);
+        for (int i = 0; i < NS; ++i) a[i] = RatioSearch<FL - 2>::run(sm, a[i], ratio[i]);
         uint32_t e0[NS], e1[NS];
 #if defined(__CUDA_ARCH__)
 #pragma unroll
@@ -441,9 +388,10 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 #pragma unroll
 #endif
         for (int i = 0; i < NS; ++i) {
-            rare = rare || a[i] >= det || bw[i].short_of_bits();
             flo[i] = cg_umulhi(st[i].span32, e0[i]);
             fhi[i] = cg_umulhi(st[i].span32, e1[i]);
+            rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]) | bw[i].short_of_bits();
+            if (!LAST_REPEATED) rare = rare | (a[i] >= det);
         }
         if (cg_any_lane(lanes, rare)) {
             bool low = false, odd = false;
@@ -452,7 +400,8 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 #endif
             for (int i = 0; i < NS; ++i) {
                 low = low || bw[i].short_of_bits();
-                odd = odd || a[i] >= det;
+                odd = odd || st[i].offset - flo[i] >= fhi[i] - flo[i];
+                if (!LAST_REPEATED) odd = odd || a[i] >= det;
             }
             if (cg_any_lane(lanes, low)) {
 #if defined(__CUDA_ARCH__)
@@ -476,7 +425,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-        for (int i = 0; i < NS; ++i) update_unguarded(st[i], flo[i], fhi[i], bw[i]);
+        for (int i = 0; i < NS; ++i) st[i].update(flo[i], fhi[i], bw[i]);
     }
     // last symbol: no range update (dec_new.cu:273-275), so no new bits either
 #if defined(__CUDA_ARCH__)
@@ -486,28 +435,20 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     emit(a, t4);
 }
 
-// ---- renormalisation shift ----------------------------------------------------------------------------
-// After a range update the reference shifts while low and high agree in their top bit, then while low
-// starts 01 and high 10 (enc_new.cu:275-293, dec_new.cu:284-301).  Both kinds double the interval, and
-// together they stop at the largest s for which [low, high] lies inside a window of 2^(32-s) values that
-// starts at a multiple of half its size (the midpoint windows of the second kind included).  With
-// d = high - low and b the position of d's top bit, that is 32-s = b+1 when [low, high] touches only two
-// cells of 2^b values and b+2 when it touches three, and it touches three exactly when the low b bits
-// of low and of d carry into bit b.  So 32-s = b + 1 + carry: one leading-bit search, two shifts that move
-// the b low bits to the top of a word, an add for its carry and an add that takes it.  Only the bits of
-// low below b matter, so low may carry anything in its top bit after the shift.
-CG_HD uint32_t renorm_right_shift(uint32_t low, uint32_t d) {
-#if defined(__CUDA_ARCH__)
-    uint32_t n, b;
-    asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(d));
-    const uint32_t l = __funnelshift_r(0u, low, b), m = __funnelshift_r(0u, d, b);
-    asm("{ .reg .u32 t; add.cc.u32 t, %1, %2; addc.u32 %0, %3, 1; }" : "=r"(n) : "r"(l), "r"(m), "r"(b));
-    return n;
-#else
-    const uint32_t b = 31u - static_cast<uint32_t>(cg_clz(d));
-    const uint32_t l = (b & 31u) ? low << (32u - (b & 31u)) : 0u, m = (b & 31u) ? d << (32u - (b & 31u)) : 0u;
-    return b + 1u + (l + m < l ? 1u : 0u);
-#endif
+// One stream.  col: address of the stream's table column, entries cdf << 16, rows kTableRowBytes apart,
+// 2^LEVELS + 1 of them readable, 2^LEVELS >= maxsym + 1; emit(a) receives, token after token, the address of the
+// decoded symbol's table entry (symbol = (a - col) / kTableRowBytes).  lanes: the warp's lanes that
+// run this loop together (they must all have the same ntok).  FULL: the table has exactly 2^LEVELS symbols (the
+// search is the same).
+template <int LEVELS, bool FULL, class Emit>
+CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *stream, uint32_t len, int ntok,
+                         uint32_t lanes, Emit emit) {
+    const uint32_t cols[1] = {col}, lens[1] = {len};
+    const uint8_t *const streams[1] = {stream};
+    const int top = (1 << LEVELS) - 1;
+    const uint32_t det = col + static_cast<uint32_t>(FULL || top < maxsym ? top : maxsym) * kTableRowBytes;
+    decode_streams<LEVELS, 1>(sm, cols, det, maxsym, LEVELS, streams, lens, ntok, lanes,
+                              [&](const uint32_t(&a)[1], uint32_t) { emit(a[0]); });
 }
 
 // ---- MSB-first bit writer into one scratch row (add_bits_to_output, enc_new.cu:21-97) ---------------------
@@ -610,12 +551,12 @@ struct EncoderState {
         }
         add_to_low(flo, out);
         span32 = fhi - flo;
-        const uint32_t n = renorm_right_shift(low, span32 - 1u);
-        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, n);
-        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, n);
-        low = cg_fshr_clamp(0u, low, n);
-        span32 = cg_fshr_clamp(0u, span32, n);
-        out.nacc += 32u - n;
+        const Renorm r = renorm_shift(low, span32 - 1u);
+        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, r.n);
+        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, r.n);
+        low *= r.p2;
+        span32 *= r.p2;
+        out.nacc += 32u - r.n;
     }
     // final flush (enc_new.cu:298-306): two bits that place the stream's value inside the interval, 01 or
     // 10 above the reference's low with its pending bits, which is L plus a quarter of the window cut

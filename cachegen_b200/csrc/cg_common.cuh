@@ -46,20 +46,27 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 // cdf[m] << 16 so that lane i always hits bank i, whatever entry m each lane is at.  Each thread
 // fills (and later reads) only its own column, so no block barrier is needed.  Only the entries of
 // the symbols, 0 .. lp-2, are staged; the rows above them hold kTablePadding, which a search step
-// of the decoder takes for "above the target" (see decode_streams in cg_coder.cuh).
+// of the decoder takes for "above the target", or with REPEAT_LAST copies of the last entry (see
+// decode_streams in cg_coder.cuh).
 constexpr uint32_t kTablePadding = 0xFFFFFFFFu;
+template <bool REPEAT_LAST = false>
 __device__ __forceinline__ void stage_table_column(uint32_t *tab, const int16_t *cdf_row, int lp,
                                                    int rows, int tid) {
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    for (int m = 0; m < n; ++m)
-        tab[m * kGroup + tid] = static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))) << 16;
-    for (int m = n; m < rows; ++m) tab[m * kGroup + tid] = kTablePadding;
+    uint32_t pad = kTablePadding, e = 0u;
+    for (int m = 0; m < n; ++m) {
+        e = static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))) << 16;
+        tab[m * kGroup + tid] = e;
+    }
+    if (REPEAT_LAST) pad = e;
+    for (int m = n; m < rows; ++m) tab[m * kGroup + tid] = pad;
 }
 
 // The same column from the byte counts of the non-centre symbols (CG_TABLES_COUNTS):
 // cdf[i] = (uint16)((0xFFFF - max_bins) * #{sym < i} / ntokens) + i, as calculate_cdf builds it
 // (cal_cdf.cu:11-15,40-49 in the reference).  cnt points at this channel's first count; counts of one
 // symbol are `stride` bytes apart; cq = bins // 2 - 1 is the centre symbol, whose count is implied.
+template <bool REPEAT_LAST = false>
 __device__ __forceinline__ void stage_table_column_from_counts(uint32_t *tab, const uint8_t *cnt, int64_t stride,
                                                                int cq, int ntokens, int lp, int rows, int tid) {
     const int max_bins = lp - 1;
@@ -71,23 +78,26 @@ __device__ __forceinline__ void stage_table_column_from_counts(uint32_t *tab, co
     const bool pow2 = (total & (total - 1u)) == 0u;
     const int sh = 31 - __clz(static_cast<int>(total | 1u));
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    uint32_t cum = 0;
+    uint32_t cum = 0, pad = kTablePadding;
     for (int i = 0; i < n; ++i) {
         const uint32_t prod = scale * (cum & 0xFFFFu);
         const uint32_t nv = total ? (pow2 ? (prod >> sh) : (prod / total)) : 0u;
-        tab[i * kGroup + tid] = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        const uint32_t e = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        tab[i * kGroup + tid] = e;
+        if (REPEAT_LAST) pad = e;
         uint32_t count = 0;
         if (i < cq) count = __ldg(cnt + i * stride);
         else if (i == cq) count = centre;
         else if (i <= 2 * cq) count = __ldg(cnt + (i - 1) * stride);
         cum += count;
     }
-    for (int i = n; i < rows; ++i) tab[i * kGroup + tid] = kTablePadding;
+    for (int i = n; i < rows; ++i) tab[i * kGroup + tid] = pad;
 }
 
 // The same column from the sparse byte counts (CG_TABLES_SPARSE): `mask` has bit j set when stored
 // symbol j (centre skipped) has a non-zero count, and `nz` points at those counts in rising symbol
 // order (nullptr: read them all as zero).
+template <bool REPEAT_LAST = false>
 __device__ __forceinline__ void stage_table_column_from_sparse(uint32_t *tab, uint32_t mask, const uint8_t *nz, int cq,
                                                                int ntokens, int lp, int rows, int tid) {
     const int max_bins = lp - 1;
@@ -101,11 +111,13 @@ __device__ __forceinline__ void stage_table_column_from_sparse(uint32_t *tab, ui
     const bool pow2 = (total & (total - 1u)) == 0u;
     const int sh = 31 - __clz(static_cast<int>(total | 1u));
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    uint32_t cum = 0;
+    uint32_t cum = 0, pad = kTablePadding;
     for (int i = 0; i < n; ++i) {
         const uint32_t prod = scale * (cum & 0xFFFFu);
         const uint32_t nv = total ? (pow2 ? (prod >> sh) : (prod / total)) : 0u;
-        tab[i * kGroup + tid] = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        const uint32_t e = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        tab[i * kGroup + tid] = e;
+        if (REPEAT_LAST) pad = e;
         uint32_t count = 0;
         if (i == cq) {
             count = centre;
@@ -115,7 +127,7 @@ __device__ __forceinline__ void stage_table_column_from_sparse(uint32_t *tab, ui
         }
         cum += count;
     }
-    for (int i = n; i < rows; ++i) tab[i * kGroup + tid] = kTablePadding;
+    for (int i = n; i < rows; ++i) tab[i * kGroup + tid] = pad;
 }
 
 // ---- block-wide exclusive scan over 32 * NWARPS ints --------------------------------------------

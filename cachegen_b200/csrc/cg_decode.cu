@@ -26,7 +26,7 @@ struct SymDecodeParams {
     int32_t *status;
 };
 
-template <int LEVELS, bool POW2, int MODE>
+template <int LEVELS, int MODE>
 __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeParams p) {
     extern __shared__ uint32_t tab[];
     const int tid = threadIdx.x;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
         *o = static_cast<uint8_t>((a - col) / kRowBytes);
         o += o1;
     };
-    decode_stream<LEVELS, POW2>(Smem{}, col, p.lp - 2, p.bytes + start, static_cast<uint32_t>(len), p.ntokens,
+    decode_stream<LEVELS, false>(Smem{}, col, p.lp - 2, p.bytes + start, static_cast<uint32_t>(len), p.ntokens,
                                 lanes, emit);
 }
 
@@ -122,7 +122,7 @@ struct FusedDecodeParams {
     cg_decode_job jobs[CG_MAX_DECODE_JOBS];
 };
 
-template <int LEVELS, bool POW2, int SCALE_DT, int OUT_DT>
+template <int LEVELS, int SCALE_DT, int OUT_DT>
 __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_constant__ FusedDecodeParams p) {
     extern __shared__ uint32_t smem[];
     __shared__ float scale_f[kSubTokens];
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
         o += o_token;
         sc_a += 4u;
     };
-    decode_stream<LEVELS, POW2>(Smem{}, col, p.lp - 2, job.bytes + start, static_cast<uint32_t>(len), ntok_r,
+    decode_stream<LEVELS, false>(Smem{}, col, p.lp - 2, job.bytes + start, static_cast<uint32_t>(len), ntok_r,
                                 lanes, emit);
 }
 
@@ -361,7 +361,7 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
         if (active) {
 #pragma unroll
             for (int i = 0; i < NS; ++i) {
-                stage_table_column_from_sparse(tabs[i], mask[i], fits ? base + at : nullptr, cq, job.scale_stride, p.lp,
+                stage_table_column_from_sparse<true>(tabs[i], mask[i], fits ? base + at : nullptr, cq, job.scale_stride, p.lp,
                                                rows + 1, 0);
                 at += nset[i];
             }
@@ -373,10 +373,10 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
                 const int64_t at = __ldg(job.table_row_off + row) + c0 + i;
                 const bool fits = at >= 0 && at + static_cast<int64_t>(2 * cq - 1) * p.nchannels < job.tables_nbytes;
                 if (!fits && p.status) atomicOr(p.status, CG_S_BAD_TABLE);
-                stage_table_column_from_counts(tabs[i], static_cast<const uint8_t *>(job.tables) + (fits ? at : 0),
+                stage_table_column_from_counts<true>(tabs[i], static_cast<const uint8_t *>(job.tables) + (fits ? at : 0),
                                                p.nchannels, fits ? cq : 0, job.scale_stride, p.lp, rows + 1, 0);
             } else {
-                stage_table_column(tabs[i], static_cast<const int16_t *>(job.tables) + (g + i) * p.lp, p.lp, rows + 1, 0);
+                stage_table_column<true>(tabs[i], static_cast<const int16_t *>(job.tables) + (g + i) * p.lp, p.lp, rows + 1, 0);
             }
         }
     }
@@ -437,11 +437,11 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
         lens[i] = static_cast<uint32_t>(len[i]);
     }
     switch (fl) {
-    case 2: decode_streams<2, NS>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 3: decode_streams<3, NS>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 4: decode_streams<4, NS>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 5: decode_streams<5, NS>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    default: decode_streams<6, NS>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    case 2: decode_streams<2, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    case 3: decode_streams<3, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    case 4: decode_streams<4, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    case 5: decode_streams<5, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    default: decode_streams<6, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
     }
 }
 
@@ -451,28 +451,23 @@ static size_t table_bytes(int lp, int levels) {
     return static_cast<size_t>(table_rows(lp, levels) + 1) * kRowBytes;  // +1: the row read past the last symbol
 }
 
-// Instantiated search depths: exact power-of-two tables for lp = 9, 17, 33 and clamped searches of
-// depth 3..6 for every other lp <= 64.
+// Instantiated search depths: 3..6, whatever the table length.
 template <int MODE>
 static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) {
     const int need = search_levels(p.lp);
-    const bool pow2 = (1 << need) == p.lp - 1;
     const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows), block(kGroup);
-#define CG_LAUNCH_SYM(L, P2)                                                                              \
+#define CG_LAUNCH_SYM(L)                                                                                 \
     do {                                                                                                  \
         const size_t smem = table_bytes(p.lp, L);                                                         \
         if (smem > 48 * 1024)                                                                             \
-            cudaFuncSetAttribute(decode_symbols_kernel<L, P2, MODE>,                                      \
+            cudaFuncSetAttribute(decode_symbols_kernel<L, MODE>,                                      \
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));    \
-        decode_symbols_kernel<L, P2, MODE><<<grid, block, smem, st>>>(p);                                 \
+        decode_symbols_kernel<L, MODE><<<grid, block, smem, st>>>(p);                                 \
     } while (0)
-    if (pow2 && need == 5) CG_LAUNCH_SYM(5, true);
-    else if (pow2 && need == 4) CG_LAUNCH_SYM(4, true);
-    else if (pow2 && need == 3) CG_LAUNCH_SYM(3, true);
-    else if (need <= 3) CG_LAUNCH_SYM(3, false);
-    else if (need == 4) CG_LAUNCH_SYM(4, false);
-    else if (need == 5) CG_LAUNCH_SYM(5, false);
-    else CG_LAUNCH_SYM(6, false);
+    if (need <= 3) CG_LAUNCH_SYM(3);
+    else if (need == 4) CG_LAUNCH_SYM(4);
+    else if (need == 5) CG_LAUNCH_SYM(5);
+    else CG_LAUNCH_SYM(6);
 #undef CG_LAUNCH_SYM
     return check_launch();
 }
@@ -480,23 +475,19 @@ static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) 
 template <int SCALE_DT, int OUT_DT>
 static int launch_fused(const FusedDecodeParams &p, cudaStream_t st) {
     const int need = search_levels(p.lp);
-    const bool pow2 = (1 << need) == p.lp - 1;
     const dim3 grid(p.nslab, 2 * p.nlayers, p.njobs), block(kGroup);
-#define CG_LAUNCH_FUSED(L, P2)                                                                            \
+#define CG_LAUNCH_FUSED(L)                                                                               \
     do {                                                                                                  \
         const size_t smem = table_bytes(p.lp, L);                                                         \
         if (smem > 48 * 1024)                                                                             \
-            cudaFuncSetAttribute(decode_dequant_kernel<L, P2, SCALE_DT, OUT_DT>,                          \
+            cudaFuncSetAttribute(decode_dequant_kernel<L, SCALE_DT, OUT_DT>,                          \
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));    \
-        decode_dequant_kernel<L, P2, SCALE_DT, OUT_DT><<<grid, block, smem, st>>>(p);                     \
+        decode_dequant_kernel<L, SCALE_DT, OUT_DT><<<grid, block, smem, st>>>(p);                     \
     } while (0)
-    if (pow2 && need == 5) CG_LAUNCH_FUSED(5, true);
-    else if (pow2 && need == 4) CG_LAUNCH_FUSED(4, true);
-    else if (pow2 && need == 3) CG_LAUNCH_FUSED(3, true);
-    else if (need <= 3) CG_LAUNCH_FUSED(3, false);
-    else if (need == 4) CG_LAUNCH_FUSED(4, false);
-    else if (need == 5) CG_LAUNCH_FUSED(5, false);
-    else CG_LAUNCH_FUSED(6, false);
+    if (need <= 3) CG_LAUNCH_FUSED(3);
+    else if (need == 4) CG_LAUNCH_FUSED(4);
+    else if (need == 5) CG_LAUNCH_FUSED(5);
+    else CG_LAUNCH_FUSED(6);
 #undef CG_LAUNCH_FUSED
     return check_launch();
 }
