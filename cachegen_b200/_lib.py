@@ -47,7 +47,25 @@ class WorkspaceSizes(ctypes.Structure):
                                               "encode_group_off", "encode_sub_off", "decode_group_off", "symbols")]
 
 
+class EncodeKvJob(ctypes.Structure):
+    """cg_encode_kv_job"""
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("kv", "bins", "res_bins", "scales_k", "scales_v", "cdf", "counts",
+                                                "table_row_off", "workspace", "tail")] +
+                [(n, ctypes.c_int64) for n in ("workspace_bytes", "s_layer", "s_kv", "s_token", "s_head")] +
+                [(n, ctypes.c_int32) for n in ("dtype", "nlayers", "ntokens", "nheads", "head_size", "max_bins",
+                                               "delta_group", "reserved")])
+
+
+class FlatLayout(ctypes.Structure):
+    """cg_flat_layout"""
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("blob", "header_host", "sub_off_host", "mask_row_off")] +
+                [(n, ctypes.c_int64) for n in ("header_bytes", "off_scales", "off_tables", "tables_bytes", "off_lengths",
+                                               "off_payload", "off_masks", "off_counts")] +
+                [(n, ctypes.c_int32) for n in ("table_kind", "reserved")])
+
+
 EXPORTS = [
+    "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_wait", "cg_encode_kv_gather", "cg_encode_kv_flat",
     "cg_version", "cg_status_string", "cg_last_cuda_error", "cg_workspace_bytes",
     "cg_calculate_cdf", "cg_encode_padded", "cg_decode_padded", "cg_decode_prefsum", "cg_decode_prefsum_warp",
     "cg_quantize_cdf", "cg_row_absmax", "cg_quantize_cdf_scaled", "cg_pack_sparse_tables", "cg_encode_chunk", "cg_compact_streams",
@@ -96,10 +114,17 @@ def lib():
     L.cg_decode_dequant_static.argtypes = L.cg_decode_dequant.argtypes
     L.cg_quantize_cdf_delta.argtypes = [p, i, i64, i64, i64, i64, i, i, i, i, p, i, i, p, p, p, p, p, p, p, p]
     L.cg_decode_dequant_delta.argtypes = [ctypes.POINTER(DecodeJob), i, i, i, i, i, p, i, p, i, i, i64, i64, i64, i64, p, p]
+    job = ctypes.POINTER(EncodeKvJob)
+    L.cg_encode_kv_workspace.argtypes = [i, i, i, i]
+    L.cg_encode_kv.argtypes = [job, p]
+    L.cg_encode_kv_wait.argtypes = [job, p]
+    L.cg_encode_kv_gather.argtypes = [job, ctypes.POINTER(p), ctypes.POINTER(p), p]
+    L.cg_encode_kv_flat.argtypes = [job, ctypes.POINTER(FlatLayout), p]
     for name in EXPORTS:
         fn = getattr(L, name)
         if name not in ("cg_version", "cg_status_string", "cg_last_cuda_error"):
             fn.restype = i
+    L.cg_encode_kv_workspace.restype = i64
     _lib = L
     return L
 

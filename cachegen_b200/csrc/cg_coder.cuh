@@ -539,15 +539,16 @@ struct EncoderState {
     // encode together (same token count).  ONE warp vote a symbol covers what is rare: a full word in the
     // accumulator (every lane that has one stores it as soon as one lane is near the high-water mark), the
     // full 2^32 range (a stream's first symbol; later only if a shift lands on it exactly) and the table's last
-    // symbol, whose upper bound is the range's end.
+    // symbol, whose upper bound is the range's end (LAST = false: s < maxsym is known).
+    template <bool LAST = true>
     CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, BitSink &out, uint32_t lanes) {
         const uint32_t a = col + s * kTableRowBytes;
         const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + kTableRowBytes);
         uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
-        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (s == maxsym))) {
+        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (LAST && s == maxsym))) {
             if (out.nacc >= 32u) out.store_word();
             flo = scale_exact(span32, e0);
-            fhi = s == maxsym ? span32 : scale_exact(span32, e1);
+            fhi = LAST && s == maxsym ? span32 : scale_exact(span32, e1);
         }
         add_to_low(flo, out);
         span32 = fhi - flo;

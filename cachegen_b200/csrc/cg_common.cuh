@@ -23,6 +23,13 @@ inline int check_launch() {
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
 
+// cg_tables.cu: group offsets of sparse tables, and the tables in one pass once those are known
+int launch_sparse_write(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
+                        const uint32_t *group_off, void *masks, const int64_t *mask_row_off, uint8_t *out,
+                        cudaStream_t st);
+int launch_sparse_sizes(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
+                        uint32_t *group_off, cudaStream_t st);
+
 // ---- search depth for a table of lp entries ---------------------------------------------------
 // Symbols are 0 .. lp-2.  levels = smallest n with 2^n >= lp-1; pow2 when 2^n == lp-1.
 inline int search_levels(int lp) {

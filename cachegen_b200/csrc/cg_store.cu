@@ -1,0 +1,820 @@
+// The whole encode of one chunk as three launches: quantise (one pass over the KV), histogram + tables +
+// arithmetic coding + offsets, gather.  What the separate calls (cg_quantize_cdf, cg_encode_chunk,
+// cg_compact_streams) do in seven launches and with three more passes over memory; same tables, streams and scales.
+//
+// Between the first two, the symbols of four consecutive tokens of one channel are one 32-bit word,
+// sym4[row][token / 4][channel] (first token in the low byte): the coder, whose thread owns a channel, reads
+// them coalesced, four symbols a load.
+#include <string.h>
+
+#include "cg_common.cuh"
+
+namespace cg {
+
+struct KvView {
+    const uint16_t *kv;
+    int64_t s_layer, s_kv, s_token, s_head;
+    int nlayers, ntokens, nheads, head_size;
+};
+
+// ---- pass 1: max|x| and quantise ---------------------------------------------------------------------------
+// One block per (row, four tokens), one thread per eight channels: the block holds its tokens' channels in
+// registers, so max|x| over the channels (cachegen_encoder.py:55) and the quantisation (:56-57) need one
+// read of the KV where a max pass and a quantise pass read it twice (a 256-token Llama-7B chunk, 134 MB,
+// does not stay in the L2 in between).  Four tokens a block because their symbols share a word; four
+// 128-bit loads a thread in flight.
+constexpr int kTokensPerWord = 4;
+
+template <int DT>
+__global__ void __launch_bounds__(1024) quantize_tokens_kernel(const KvView v, const float *__restrict__ bins, int max_bins,
+                                                               uint16_t *__restrict__ scales_k,
+                                                               uint16_t *__restrict__ scales_v,
+                                                               uint32_t *__restrict__ sym4, uint32_t *zeroed, int nzeroed) {
+    __shared__ uint4 part[32];
+    __shared__ float4 factor_s;
+    __shared__ uint32_t keep_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = blockIdx.y, t0 = blockIdx.x * kTokensPerWord;
+    const int C = v.nheads * v.head_size, c = tid * 8;
+    const int layer = row % v.nlayers, kv = row / v.nlayers;
+    if (row == 0 && blockIdx.x == 0)  // the counters of the launches after this one
+        for (int i = tid; i < nzeroed; i += blockDim.x) zeroed[i] = 0u;
+    uint4 x[kTokensPerWord];
+#pragma unroll
+    for (int j = 0; j < kTokensPerWord; ++j) x[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (c < C) {
+        const int h = c / v.head_size;
+        const uint16_t *p = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token + h * v.s_head + (c - h * v.head_size);
+#pragma unroll
+        for (int j = 0; j < kTokensPerWord; ++j)
+            if (t0 + j < v.ntokens) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+    }
+    // |x| as an ordered integer: 16-bit float magnitudes compare like their bit patterns
+    uint32_t m[kTokensPerWord];
+#pragma unroll
+    for (int j = 0; j < kTokensPerWord; ++j) {
+        const uint32_t a = __vmaxu2(__vmaxu2(x[j].x & 0x7FFF7FFFu, x[j].y & 0x7FFF7FFFu),
+                                    __vmaxu2(x[j].z & 0x7FFF7FFFu, x[j].w & 0x7FFF7FFFu));
+        m[j] = __reduce_max_sync(0xFFFFFFFFu, max(a & 0xFFFFu, a >> 16));
+    }
+    if (lane == 0) part[warp] = make_uint4(m[0], m[1], m[2], m[3]);
+    const float MAX = half_range(__ldg(bins + row));
+    __syncthreads();
+    if (warp == 0) {
+        const uint4 q = lane < (blockDim.x >> 5) ? part[lane] : make_uint4(0u, 0u, 0u, 0u);
+        m[0] = __reduce_max_sync(0xFFFFFFFFu, q.x);
+        m[1] = __reduce_max_sync(0xFFFFFFFFu, q.y);
+        m[2] = __reduce_max_sync(0xFFFFFFFFu, q.z);
+        m[3] = __reduce_max_sync(0xFFFFFFFFu, q.w);
+        if (lane < kTokensPerWord) {
+            const uint32_t mine = lane == 0 ? m[0] : lane == 1 ? m[1] : lane == 2 ? m[2] : m[3];
+            reinterpret_cast<float *>(&factor_s)[lane] = __fdiv_rn(MAX, Half16<DT>::to_float(static_cast<uint16_t>(mine)));
+            // an all-zero token: 0 * inf = NaN, which the reference's cast makes symbol 0
+            reinterpret_cast<uint8_t *>(&keep_s)[lane] = mine ? 0xFFu : 0u;
+            if (t0 + lane < v.ntokens) {
+                uint16_t *s = row < v.nlayers ? scales_k + static_cast<int64_t>(row) * v.ntokens
+                                              : scales_v + static_cast<int64_t>(row - v.nlayers) * v.ntokens;
+                s[t0 + lane] = static_cast<uint16_t>(mine);
+            }
+        }
+    }
+    __syncthreads();
+    if (c >= C) return;
+    const float f[kTokensPerWord] = {factor_s.x, factor_s.y, factor_s.z, factor_s.w};
+    const uint32_t keep = keep_s;
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        uint32_t b[kTokensPerWord];
+#pragma unroll
+        for (int j = 0; j < kTokensPerWord; ++j) {
+            const uint32_t pair = k < 2 ? x[j].x : k < 4 ? x[j].y : k < 6 ? x[j].z : x[j].w;
+            const uint16_t hb = static_cast<uint16_t>(k & 1 ? pair >> 16 : pair);
+            // three separately rounded fp32 operations, then round-half-even (enc.py:56-57)
+            b[j] = __float_as_uint(__fadd_rn(__fadd_rn(__fmul_rn(Half16<DT>::to_float(hb), f[j]), MAX), 8388608.0f));
+        }
+        w[k] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410) & keep;
+    }
+    // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
+    // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
+    if (2.0f * MAX >= static_cast<float>(max_bins - 1)) {
+        const uint32_t limit = static_cast<uint32_t>(max_bins - 1) * 0x01010101u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] |= __vcmpgeu4(w[k], limit);
+    }
+    uint4 *o = reinterpret_cast<uint4 *>(sym4 + (static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * C + c);
+    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// ---- tables ------------------------------------------------------------------------------------------------
+struct TableOut {
+    int16_t *cdf;                 // [nrows, C, lp]
+    uint8_t *counts;              // byte counts of the non-centre symbols (CG_TABLES_COUNTS), or nullptr
+    const int64_t *table_row_off;
+    const float *bins;
+    uint32_t *group_nz;           // non-zero byte counts per (row, group), or nullptr
+};
+
+// The counts of one channel, hist[m * kGroup] for symbols m < lp - 1, become its table in place (entries
+// cdf << 16, one row more than there are symbols) and, as 16-bit entries, in stage[0 .. lp-1]
+// (normalize_cdf_value, cal_cdf.cu:11-15,40-49).  Returns the number of non-zero non-centre counts.
+__device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage, int lp, uint32_t ntokens, int cq,
+                                                uint8_t *counts, int64_t counts_stride, bool *overflow) {
+    const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(lp - 1);
+    const uint32_t total = ntokens & 0xFFFFu;  // the reference accumulates in uint16
+    // scale * cum / total by the rounded-down reciprocal, one below the quotient at most
+    const uint32_t inv = total > 1u ? 0xFFFFFFFFu / total : 0u;
+    uint32_t cum = 0;
+    int nz = 0;
+    for (int m = 0; m < lp; ++m) {
+        const uint32_t n = hist[m * kGroup];
+        const uint32_t prod = scale * (cum & 0xFFFFu);
+        uint32_t q = __umulhi(prod, inv);
+        if (prod - q * total >= total) ++q;
+        if (total <= 1u) q = total ? prod : 0u;
+        const uint32_t e = (q + static_cast<uint32_t>(m)) & 0xFFFFu;
+        hist[m * kGroup] = e << 16;
+        stage[m] = static_cast<uint16_t>(e);
+        cum += n;
+        if (counts && m < lp - 1) {
+            if (m != cq && m <= 2 * cq) {
+                *counts = static_cast<uint8_t>(n);
+                counts += counts_stride;
+                nz += n != 0u;
+                *overflow |= n > 255u;
+            } else if (m > 2 * cq) {
+                *overflow |= n != 0u;
+            }
+        }
+    }
+    return nz;
+}
+
+// One warp's tables, staged as 16-bit entries channel after channel, to their place: one contiguous run.
+__device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst, int n, int lane) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (n & 7) == 0) {
+        const uint4 *s = reinterpret_cast<const uint4 *>(stage);
+        uint4 *d = reinterpret_cast<uint4 *>(dst);
+        for (int i = lane; i < n / 8; i += 32) d[i] = s[i];
+    } else {
+        for (int i = lane; i < n; i += 32) dst[i] = stage[i];
+    }
+}
+
+__device__ __forceinline__ void count_symbol(uint32_t addr) {
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void count_word(uint32_t col, uint32_t w) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+}
+
+// Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
+// block (slab, row), thread (channel, part) counts every kParts-th word of its channel.
+constexpr int kTableThreads = 512, kParts = kTableThreads / kGroup;
+__global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint32_t *__restrict__ sym4, int ntokens,
+                                                                      int nchannels, int lp, const TableOut out,
+                                                                      int32_t *status) {
+    extern __shared__ uint4 smem4[];
+    uint32_t *hist = reinterpret_cast<uint32_t *>(smem4);
+    uint16_t *stage = reinterpret_cast<uint16_t *>(hist + lp * kGroup);
+    __shared__ uint32_t nz_total;
+    const int tid = threadIdx.x, cl = tid % kGroup, part = tid / kGroup;
+    const int row = blockIdx.y, c = blockIdx.x * kGroup + cl;
+    for (int i = tid; i < lp * kGroup; i += kTableThreads) hist[i] = 0u;
+    if (tid == 0) nz_total = 0u;
+    __syncthreads();
+    const int words = (ntokens + 3) / 4, whole = ntokens / 4;
+    if (c < nchannels) {
+        const uint32_t col = smem_addr(hist + cl);
+        const uint32_t *p = sym4 + static_cast<int64_t>(row) * words * nchannels + c;
+        for (int i = part; i < words; i += kParts) {
+            uint32_t w = __ldg(p + static_cast<int64_t>(i) * nchannels);
+            if (w & 0x80808080u) w = 0u;  // reported by the coder
+            if (i < whole) {
+                count_word(col, w);
+            } else {
+                for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+            }
+        }
+    }
+    __syncthreads();
+    bool overflow = false;
+    if (tid < kGroup) {
+        int nz = 0;
+        if (c < nchannels) {
+            const int cq = static_cast<int>(half_range(__ldg(out.bins + row)));
+            nz = counts_to_column(hist + cl, stage + cl * lp, lp, ntokens, cq,
+                                  out.counts ? out.counts + __ldg(out.table_row_off + row) + c : nullptr, nchannels, &overflow);
+        }
+        if (out.group_nz) {
+            nz = __reduce_add_sync(0xFFFFFFFFu, nz);
+            if ((tid & 31) == 0 && nz) atomicAdd(&nz_total, static_cast<uint32_t>(nz));
+        }
+        __syncwarp();
+        const int first = blockIdx.x * kGroup + (tid & ~31);
+        const int nch = min(32, nchannels - first);
+        if (nch > 0)
+            copy_tables(stage + (tid & ~31) * lp,
+                        reinterpret_cast<uint16_t *>(out.cdf) + (static_cast<int64_t>(row) * nchannels + first) * lp,
+                        nch * lp, tid & 31);
+    }
+    if (overflow && status) atomicOr(status, CG_S_COUNT_OVERFLOW);
+    __syncthreads();
+    if (tid == 0 && out.group_nz) out.group_nz[row * gridDim.x + blockIdx.x] = nz_total;
+}
+
+// ---- pass 2: (histogram, tables,) arithmetic coding, offsets -------------------------------------------------
+struct StoreParams {
+    const uint32_t *sym4;
+    TableOut out;
+    int ntokens, nchannels, lp, nrows, nsub;
+    uint8_t *scratch;     // [nsub, nrows * C, stride]
+    int64_t stride;
+    int32_t *lengths;     // [nsub, nrows * C]
+    int64_t *group_off;   // [nsub, nrows * nslab]: byte offset of each 128-channel group inside its sub-chunk
+    int64_t *sub_bytes;   // [nsub]
+    uint32_t *tickets;    // [nsub + 1], zero
+    int32_t *status;      // zero before pass 1
+    int64_t *tail;        // [nsub + 4], see cg_encode_kv_job
+};
+
+// Exclusive scan of n values in place by one block of kGroup threads; returns the sum.
+template <class T>
+__device__ __forceinline__ int64_t block_scan_in_place(T *v, int n, int64_t *warp_sums, int tid) {
+    constexpr int kPer = 8;
+    const int lane = tid & 31, w = tid >> 5;
+    int64_t base = 0;
+    for (int b = 0; b < n; b += kGroup * kPer) {
+        const int at = b + tid * kPer;
+        int64_t x[kPer], s = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            x[k] = at + k < n ? static_cast<int64_t>(__ldcg(v + at + k)) : 0;
+            s += x[k];
+        }
+        int64_t incl = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int64_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += y;
+        }
+        __syncthreads();
+        if (lane == 31) warp_sums[w] = incl;
+        __syncthreads();
+        int64_t run = base + incl - s;
+#pragma unroll
+        for (int k = 0; k < kGroup / 32; ++k) {
+            if (k < w) run += warp_sums[k];
+            base += warp_sums[k];
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (at + k < n) v[at + k] = static_cast<T>(run);
+            run += x[k];
+        }
+    }
+    return base;
+}
+
+constexpr int kWordsAhead = 4;  // words (of four symbols) fetched one group ahead of the coder
+
+// One thread per stream, 128 adjacent channels of one row and sub-chunk per block.  TABLES: the chunk is one
+// sub-chunk, so the block's symbols are all there are for its tables: it counts them (each thread in its
+// own shared-memory column, where its table then stands), writes the tables out and codes; the symbols'
+// second read comes from the L2.  Otherwise the tables come from packed_tables_kernel.
+// The last block of a sub-chunk turns the group sizes into offsets, the last of all writes the tail.
+template <bool TABLES>
+__global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_constant__ StoreParams p) {
+    extern __shared__ uint4 smem4[];
+    uint32_t *tab = reinterpret_cast<uint32_t *>(smem4);
+    __shared__ int64_t warp_sums[kGroup / 32];
+    __shared__ int block_sums[2][kGroup / 32];
+    __shared__ int last_block;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = blockIdx.y, sub = blockIdx.z, nslab = gridDim.x;
+    const int c = blockIdx.x * kGroup + tid;
+    const bool active = c < p.nchannels;
+    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, active);
+    const int t0 = sub * kSubTokens, n = min(kSubTokens, p.ntokens - t0);
+    const int64_t C = p.nchannels;
+    const int64_t g = row * C + c;
+    const uint32_t col = smem_addr(tab + tid);
+    const uint32_t *sp = p.sym4 + (static_cast<int64_t>(row) * ((p.ntokens + 3) / 4) + t0 / 4) * C + c;
+    uint32_t bad = 0;
+    int nbytes = 0, nz = 0;
+
+    if (TABLES) {
+        uint16_t *stage = reinterpret_cast<uint16_t *>(tab + p.lp * kGroup);
+        bool overflow = false;
+        if (active) {
+            for (int m = 0; m < p.lp; ++m) tab[m * kGroup + tid] = 0u;
+            const uint32_t *q = sp;
+            int i = 0;
+            for (; i + 4 * kWordsAhead <= n; i += 4 * kWordsAhead) {
+                uint32_t w[kWordsAhead];
+#pragma unroll
+                for (int k = 0; k < kWordsAhead; ++k) w[k] = __ldg(q + k * C);
+                q += kWordsAhead * C;
+#pragma unroll
+                for (int k = 0; k < kWordsAhead; ++k) {
+                    if (w[k] & 0x80808080u) w[k] = 0u;
+                    count_word(col, w[k]);
+                }
+            }
+            for (; i < n; i += 4) {
+                uint32_t w = __ldg(q);
+                q += C;
+                if (w & 0x80808080u) w = 0u;
+                for (int k = 0; k < min(4, n - i); ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+            }
+            const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
+            nz = counts_to_column(tab + tid, stage + tid * p.lp, p.lp, n, cq,
+                                  p.out.counts ? p.out.counts + __ldg(p.out.table_row_off + row) + c : nullptr, C, &overflow);
+        }
+        if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
+        __syncwarp();
+        const int first = blockIdx.x * kGroup + warp * 32;
+        const int nch = min(32, p.nchannels - first);
+        if (nch > 0)
+            copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp,
+                        nch * p.lp, lane);
+    } else if (active) {
+        stage_table_column(tab, p.out.cdf + g * p.lp, p.lp, p.lp, tid);
+    }
+
+    if (active) {
+        const int64_t slot = static_cast<int64_t>(sub) * p.nrows * C + g;
+        const uint32_t top = static_cast<uint32_t>(p.lp - 2);
+        BitSink out;
+        out.init(p.scratch + slot * p.stride, p.stride);
+        EncoderState enc;
+        enc.init();
+        constexpr int kAhead = 4 * kWordsAhead;
+        uint32_t w[kWordsAhead], next[kWordsAhead];
+#pragma unroll
+        for (int k = 0; k < kWordsAhead; ++k) w[k] = 4 * k < n ? __ldg(sp + k * C) : 0u;
+        int i = 0;
+        for (; i + kAhead <= n; i += kAhead) {
+            sp += kWordsAhead * C;
+#pragma unroll
+            for (int k = 0; k < kWordsAhead; ++k) next[k] = i + kAhead + 4 * k < n ? __ldg(sp + k * C) : 0u;
+            const uint32_t any = w[0] | w[1] | w[2] | w[3];
+            if (any & 0x80808080u) {
+                bad = 1u;
+#pragma unroll
+                for (int k = 0; k < kWordsAhead; ++k) w[k] = 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < kWordsAhead; ++k) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    enc.step<false>(Smem{}, col, (w[k] >> (8 * j)) & 0xFFu, top, out, lanes);
+            }
+#pragma unroll
+            for (int k = 0; k < kWordsAhead; ++k) w[k] = next[k];
+        }
+        for (; i < n; ++i) {  // fewer than kAhead left, all in w
+            uint32_t s = w[0] & 0xFFu;
+            if (s >= top) {
+                bad = 1u;
+                s = 0u;
+            }
+            enc.step<false>(Smem{}, col, s, top, out, lanes);
+            w[0] >>= 8;
+            if ((i & 3) == 3) {
+#pragma unroll
+                for (int k = 0; k + 1 < kWordsAhead; ++k) w[k] = w[k + 1];
+            }
+        }
+        nbytes = static_cast<int>(enc.flush(out));
+        p.lengths[slot] = nbytes;
+        int bits = 0;
+        if (nbytes > p.stride) {
+            bits |= CG_S_STREAM_OVERFLOW;
+            nbytes = static_cast<int>(p.stride);
+        }
+        if (bad) bits |= CG_S_BAD_SYMBOL;
+        if (bits) atomicOr(p.status, bits);
+    }
+
+    // group sizes, and whose turn it is to make offsets of them
+    const int sum = __reduce_add_sync(0xFFFFFFFFu, nbytes);
+    const int nz_sum = TABLES && p.out.group_nz ? __reduce_add_sync(0xFFFFFFFFu, nz) : 0;
+    if (lane == 0) {
+        block_sums[0][warp] = sum;
+        block_sums[1][warp] = nz_sum;
+    }
+    __syncthreads();
+    const int ngroups = p.nrows * nslab;
+    int64_t *goff = p.group_off + static_cast<int64_t>(sub) * ngroups;
+    if (tid == 0) {
+        int s = 0, z = 0;
+        for (int k = 0; k < kGroup / 32; ++k) {
+            s += block_sums[0][k];
+            z += block_sums[1][k];
+        }
+        goff[row * nslab + blockIdx.x] = s;
+        if (TABLES && p.out.group_nz) p.out.group_nz[row * nslab + blockIdx.x] = static_cast<uint32_t>(z);
+        __threadfence();
+        last_block = atomicAdd(p.tickets + sub, 1u) == static_cast<uint32_t>(ngroups - 1);
+    }
+    __syncthreads();
+    if (!last_block) return;
+    __threadfence();
+    const int64_t bytes = block_scan_in_place(goff, ngroups, warp_sums, tid);
+    if (tid == 0) {
+        p.sub_bytes[sub] = bytes;
+        __threadfence();
+        last_block = atomicAdd(p.tickets + p.nsub, 1u) == static_cast<uint32_t>(p.nsub - 1);
+    }
+    __syncthreads();
+    if (!last_block) return;
+    __threadfence();
+    int64_t nz_total = 0;
+    if (p.out.group_nz) {
+        nz_total = block_scan_in_place(p.out.group_nz, ngroups, warp_sums, tid);
+        if (tid == 0) p.out.group_nz[ngroups] = static_cast<uint32_t>(nz_total);
+    }
+    if (tid == 0) {
+        int64_t run = 0;
+        for (int k = 0; k < p.nsub; ++k) {
+            p.tail[k] = run;
+            run += __ldcg(p.sub_bytes + k);
+        }
+        p.tail[p.nsub] = run;
+        p.tail[p.nsub + 1] = atomicOr(p.status, 0);
+        p.tail[p.nsub + 2] = nz_total;
+        __threadfence_system();
+        *reinterpret_cast<volatile int64_t *>(p.tail + p.nsub + 3) = 1;
+    }
+}
+
+// the tail of the separate calls' results (shapes that the fused passes do not take)
+__global__ void publish_tail_kernel(const int64_t *sub_off, const int32_t *status, int nsub, const uint32_t *nz, int64_t *tail) {
+    for (int k = threadIdx.x; k <= nsub; k += blockDim.x) tail[k] = sub_off[k];
+    if (threadIdx.x == 0) {
+        tail[nsub + 1] = *status;
+        tail[nsub + 2] = nz ? *nz : 0;
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile int64_t *>(tail + nsub + 3) = 1;
+}
+
+// ---- pass 3: gather ------------------------------------------------------------------------------------------
+// Destinations of up to kGatherSubs sub-chunks (kernel parameters).
+constexpr int kGatherSubs = 64;
+struct GatherTargets {
+    uint8_t *bytes[kGatherSubs];
+    void *lengths[kGatherSubs];  // int32 or uint16 [nrows, C]
+};
+
+// One block per (group, row, sub-chunk), eight lanes per stream, sixteen streams in flight.  Streams lie back to
+// back, at any byte: the words that are aligned at the destination are put together from two source words, so
+// that a stream of n bytes takes n / 4 word stores and at most six byte stores where copying byte by byte
+// takes n of them (a 256-token Llama-7B chunk, 11.8 MB of streams of 45 bytes: the stores were what bound it).
+template <class Len>
+__global__ void __launch_bounds__(kGroup) gather_kernel(const uint8_t *__restrict__ scratch, int64_t stride,
+                                                        const int32_t *__restrict__ lengths,
+                                                        const int64_t *__restrict__ group_off, int nchannels, int sub0,
+                                                        const __grid_constant__ GatherTargets out) {
+    __shared__ int warp_sums[kGroup / 32];
+    __shared__ int2 place[kGroup];  // offset, length
+    const int tid = threadIdx.x, row = blockIdx.y, sub = sub0 + blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
+    const int c = blockIdx.x * kGroup + tid;
+    const int64_t slot0 = (static_cast<int64_t>(sub) * nrows + row) * nchannels + blockIdx.x * kGroup;
+    const int len = c < nchannels ? __ldg(lengths + slot0 + tid) : 0;
+    const int64_t at = __ldg(group_off + (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x);
+    if (c < nchannels) static_cast<Len *>(out.lengths[blockIdx.z])[static_cast<int64_t>(row) * nchannels + c] = static_cast<Len>(len);
+    const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
+    place[tid] = make_int2(excl, len);
+    __syncthreads();
+    uint8_t *dst0 = out.bytes[blockIdx.z] + at;
+    constexpr int kLanes = 8;
+    const int part = tid % kLanes;
+    for (int s = tid / kLanes; s < kGroup; s += kGroup / kLanes) {
+        const int2 q = place[s];
+        const int n = q.y;
+        const uint8_t *src = scratch + (slot0 + s) * stride;  // 4-byte aligned
+        uint8_t *dst = dst0 + q.x;
+        const int head = min(n, static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 3u));
+        const int words = (n - head) >> 2, tail = (n - head) & 3;
+        const uint32_t *src4 = reinterpret_cast<const uint32_t *>(src);
+        uint32_t *dst4 = reinterpret_cast<uint32_t *>(dst + head);
+        const uint32_t sh = static_cast<uint32_t>(head & 3) * 8u;
+        for (int k = part; k < words; k += kLanes) {
+            const int w = (head + 4 * k) >> 2;
+            const uint32_t lo = __ldg(src4 + w), hi = sh ? __ldg(src4 + w + 1) : 0u;
+            dst4[k] = __funnelshift_r(lo, hi, sh);
+        }
+        // the bytes before the first and after the last whole word
+        const int e = part < 4 ? part : n - tail + part - 4;
+        if (part < 4 ? part < head : part - 4 < tail) dst[e] = __ldg(src + e);
+    }
+}
+
+// Header, scales and the sparse tables' group offsets of a container (flat_format.py) to their places.
+constexpr int kMaxHeader = 128 + 8 * (65536 / kSubTokens + 1);
+struct FlatHeader {
+    uint8_t bytes[kMaxHeader];
+};
+__global__ void __launch_bounds__(256) flat_front_kernel(const __grid_constant__ FlatHeader h, int header_bytes,
+                                                         uint8_t *blob, const uint16_t *scales_k,
+                                                         const uint16_t *scales_v, int64_t n, int64_t off_scales,
+                                                         const uint32_t *group_off, int ngroups, int64_t off_tables) {
+    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = i0; i < header_bytes; i += step) blob[i] = h.bytes[i];
+    uint16_t *s = reinterpret_cast<uint16_t *>(blob + off_scales);
+    for (int64_t i = i0; i < n; i += step) {
+        s[i] = scales_k[i];
+        s[n + i] = scales_v[i];
+    }
+    if (group_off) {
+        uint32_t *t = reinterpret_cast<uint32_t *>(blob + off_tables);
+        for (int64_t i = i0; i <= ngroups; i += step) t[i] = group_off[i];
+    }
+}
+
+}  // namespace cg
+
+using namespace cg;
+
+namespace {
+
+constexpr int64_t kSmemPerSM = 228 * 1024, kSmemPerBlock = 227 * 1024, kSmemReserved = 1024;
+
+int sm_count() {
+    static int count[64];  // per device; a racing first call writes the same number
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!count[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        count[dev] = n;
+    }
+    return count[dev];
+}
+
+// Shared memory to ask for so that the grid's last wave is as full as the others.  The coder's blocks all take
+// the same time, so 2,048 blocks at 8 resident ones per SM are one full wave and one that fills 73 % of the
+// GPU; at 7 they are two that fill 99 %.  Seven blocks (28 warps) still cover the latencies.
+size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes) {
+    const int64_t need = static_cast<int64_t>(dynamic + static_bytes) + kSmemReserved;
+    const int64_t resident = kSmemPerSM / need;
+    if (resident < 1) return dynamic;
+    const int64_t sms = sm_count();
+    const int64_t waves = (blocks + sms * resident - 1) / (sms * resident);
+    const int64_t per = (blocks + sms * waves - 1) / (sms * waves);
+    if (per >= resident || per < 1) return dynamic;
+    int64_t padded = kSmemPerSM / per - kSmemReserved - static_cast<int64_t>(static_bytes) - 256;
+    if (padded > kSmemPerBlock - static_cast<int64_t>(static_bytes)) padded = kSmemPerBlock - static_cast<int64_t>(static_bytes);
+    return padded > static_cast<int64_t>(dynamic) ? static_cast<size_t>(padded) : dynamic;
+}
+
+template <class K>
+void allow_smem(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
+struct Sizes {
+    int nrows, nchannels, nslab, nsub;
+    int64_t words, stride;
+    int64_t sym, scratch, lengths, group_off, sub_bytes, counters, group_nz, sub_off, scales, total;
+};
+
+Sizes sizes_of(int nlayers, int ntokens, int nheads, int head_size) {
+    Sizes z;
+    z.nrows = 2 * nlayers;
+    z.nchannels = nheads * head_size;
+    z.nslab = (z.nchannels + kGroup - 1) / kGroup;
+    z.nsub = (ntokens + kSubTokens - 1) / kSubTokens;
+    z.words = (ntokens + 3) / 4;
+    z.stride = (CG_STREAM_CAPACITY(ntokens < kSubTokens ? ntokens : kSubTokens) + 3) / 4 * 4;
+    const int64_t streams = static_cast<int64_t>(z.nrows) * z.nchannels, groups = static_cast<int64_t>(z.nrows) * z.nslab;
+    int64_t at = 0;
+    const auto take = [&](int64_t bytes) {
+        const int64_t here = at;
+        at += (bytes + 255) / 256 * 256;
+        return here;
+    };
+    z.sym = take(streams * z.words * 4);
+    z.scratch = take(z.nsub * streams * z.stride);
+    z.lengths = take(z.nsub * streams * 4);
+    z.group_off = take(z.nsub * groups * 8);
+    z.sub_bytes = take(z.nsub * 8);
+    z.counters = take((z.nsub + 2) * 4);  // the status word, then the tickets
+    z.group_nz = take((groups + 1) * 4);
+    z.sub_off = take((z.nsub + 1) * 8);
+    z.scales = take(static_cast<int64_t>(z.nrows) * ntokens * 2);
+    z.total = at;
+    return z;
+}
+
+int check_job(const cg_encode_kv_job *job) {
+    if (!job) return CG_E_NULL;
+    const cg_encode_kv_job &b = *job;
+    if (!b.kv || !b.bins || !b.scales_k || !b.scales_v || !b.cdf || !b.workspace || !b.tail) return CG_E_NULL;
+    if (b.counts && !b.table_row_off) return CG_E_NULL;
+    if (b.nlayers <= 0 || b.ntokens <= 0 || b.nheads <= 0 || b.head_size <= 0 || 2 * b.nlayers > 65535) return CG_E_SHAPE;
+    if (static_cast<int64_t>(b.nheads) * b.head_size > 0x7FFFFFFF - kGroup) return CG_E_SHAPE;
+    if (b.ntokens >= 65536) return CG_E_HIST;
+    if (b.dtype != CG_F16 && b.dtype != CG_BF16) return CG_E_DTYPE;
+    if (b.max_bins < 1 || b.max_bins >= CG_MAX_LP) return CG_E_LP;
+    if (b.delta_group && !b.res_bins) return CG_E_NULL;
+    if (reinterpret_cast<uintptr_t>(b.workspace) & 255) return CG_E_ALIGN;
+    if (b.workspace_bytes < sizes_of(b.nlayers, b.ntokens, b.nheads, b.head_size).total) return CG_E_CAPACITY;
+    return CG_OK;
+}
+
+// Shapes of the fused passes: eight-channel runs inside one head at 16-byte boundaries, a token's channels in one
+// block.  The rest, and delta coding, takes the separate calls.
+bool fused_ok(const cg_encode_kv_job &b) {
+    return !b.delta_group && b.head_size % 8 == 0 && b.nheads * b.head_size <= 8192 &&
+           ((reinterpret_cast<uintptr_t>(b.kv) & 15) | (b.s_layer & 7) | (b.s_kv & 7) | (b.s_token & 7) | (b.s_head & 7)) == 0;
+}
+
+}  // namespace
+
+extern "C" int64_t cg_encode_kv_workspace(int nlayers, int ntokens, int nheads, int head_size) {
+    if (nlayers <= 0 || ntokens <= 0 || nheads <= 0 || head_size <= 0) return CG_E_SHAPE;
+    return sizes_of(nlayers, ntokens, nheads, head_size).total;
+}
+
+extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
+    if (int rc = check_job(job)) return rc;
+    const cg_encode_kv_job &b = *job;
+    const Sizes z = sizes_of(b.nlayers, b.ntokens, b.nheads, b.head_size);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    uint8_t *ws = static_cast<uint8_t *>(b.workspace);
+    int32_t *status = reinterpret_cast<int32_t *>(ws + z.counters);
+    uint32_t *group_nz = b.counts ? reinterpret_cast<uint32_t *>(ws + z.group_nz) : nullptr;
+    int32_t *lengths = reinterpret_cast<int32_t *>(ws + z.lengths);
+    int64_t *group_off = reinterpret_cast<int64_t *>(ws + z.group_off);
+    const int lp = b.max_bins + 1;
+    b.tail[z.nsub + 3] = 0;  // host memory: the flag that cg_encode_kv_wait watches
+    if (!fused_ok(b)) {
+        const cudaError_t e = cudaMemsetAsync(status, 0, 4, st);
+        if (e != cudaSuccess) return set_cuda_error(e);
+        uint16_t *scales = reinterpret_cast<uint16_t *>(ws + z.scales);
+        int8_t *sym = reinterpret_cast<int8_t *>(ws + z.sym);
+        if (int rc = cg_quantize_cdf_delta(b.kv, b.dtype, b.s_layer, b.s_kv, b.s_token, b.s_head, b.nlayers, b.ntokens,
+                                           b.nheads, b.head_size, b.bins, b.max_bins, b.delta_group, b.res_bins, sym, scales,
+                                           b.cdf, b.counts, b.table_row_off, status, stream))
+            return rc;
+        const size_t half = static_cast<size_t>(b.nlayers) * b.ntokens;
+        const cudaError_t e1 = cudaMemcpyAsync(b.scales_k, scales, half * 2, cudaMemcpyDeviceToDevice, st);
+        const cudaError_t e2 = cudaMemcpyAsync(b.scales_v, scales + half, half * 2, cudaMemcpyDeviceToDevice, st);
+        if (e1 != cudaSuccess || e2 != cudaSuccess) return set_cuda_error(e1 != cudaSuccess ? e1 : e2);
+        int64_t *sub_off = reinterpret_cast<int64_t *>(ws + z.sub_off);
+        if (int rc = cg_encode_chunk(b.cdf, sym, z.nrows, b.ntokens, z.nchannels, lp, ws + z.scratch, z.stride, lengths,
+                                     group_off, sub_off, status, stream))
+            return rc;
+        if (b.counts)
+            if (int rc = launch_sparse_sizes(b.counts, b.table_row_off, b.bins, z.nrows, z.nchannels, group_nz, st)) return rc;
+        publish_tail_kernel<<<1, 128, 0, st>>>(sub_off, status, z.nsub,
+                                               group_nz ? group_nz + static_cast<int64_t>(z.nrows) * z.nslab : nullptr, b.tail);
+        return check_launch();
+    }
+    const KvView v{static_cast<const uint16_t *>(b.kv), b.s_layer, b.s_kv, b.s_token, b.s_head,
+                   b.nlayers, b.ntokens, b.nheads, b.head_size};
+    uint32_t *sym4 = reinterpret_cast<uint32_t *>(ws + z.sym);
+    const dim3 qgrid(static_cast<unsigned>(z.words), z.nrows);
+    const int qthreads = (z.nchannels / 8 + 31) / 32 * 32;
+    uint32_t *zeroed = reinterpret_cast<uint32_t *>(status);
+    uint16_t *sk = static_cast<uint16_t *>(b.scales_k), *sv = static_cast<uint16_t *>(b.scales_v);
+    if (b.dtype == CG_F16)
+        quantize_tokens_kernel<CG_F16><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, z.nsub + 2);
+    else
+        quantize_tokens_kernel<CG_BF16><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, z.nsub + 2);
+    if (int rc = check_launch()) return rc;
+    StoreParams p;
+    p.sym4 = sym4;
+    p.out = TableOut{b.cdf, b.counts, b.table_row_off, b.bins, group_nz};
+    p.ntokens = b.ntokens;
+    p.nchannels = z.nchannels;
+    p.lp = lp;
+    p.nrows = z.nrows;
+    p.nsub = z.nsub;
+    p.scratch = ws + z.scratch;
+    p.stride = z.stride;
+    p.lengths = lengths;
+    p.group_off = group_off;
+    p.sub_bytes = reinterpret_cast<int64_t *>(ws + z.sub_bytes);
+    p.tickets = zeroed + 1;
+    p.status = status;
+    p.tail = b.tail;
+    const dim3 grid(z.nslab, z.nrows, z.nsub);
+    const int64_t blocks = static_cast<int64_t>(z.nslab) * z.nrows * z.nsub;
+    const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
+    if (z.nsub == 1) {
+        const size_t smem = even_waves_smem(blocks, columns + staged, 128);
+        allow_smem(store_encode_kernel<true>, smem);
+        store_encode_kernel<true><<<grid, kGroup, smem, st>>>(p);
+        return check_launch();
+    }
+    allow_smem(packed_tables_kernel, columns + staged);
+    packed_tables_kernel<<<dim3(z.nslab, z.nrows), kTableThreads, columns + staged, st>>>(sym4, b.ntokens, z.nchannels, lp,
+                                                                                         p.out, status);
+    if (int rc = check_launch()) return rc;
+    const size_t smem = even_waves_smem(blocks, columns, 128);
+    allow_smem(store_encode_kernel<false>, smem);
+    store_encode_kernel<false><<<grid, kGroup, smem, st>>>(p);
+    return check_launch();
+}
+
+extern "C" int cg_encode_kv_wait(const cg_encode_kv_job *job, void *stream) {
+    if (!job || !job->tail) return CG_E_NULL;
+    const int nsub = (job->ntokens + kSubTokens - 1) / kSubTokens;
+    volatile int64_t *flag = job->tail + nsub + 3;
+    for (;;) {
+        for (int spin = 0; spin < 2000; ++spin)
+            if (*flag) {
+                __sync_synchronize();
+                return CG_OK;
+            }
+        const cudaError_t e = cudaStreamQuery(static_cast<cudaStream_t>(stream));
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return set_cuda_error(e);
+        return *flag ? CG_OK : CG_E_SHAPE;  // everything has run and nothing was published: not a started job
+    }
+}
+
+namespace {
+template <class Len>
+int launch_gather(const cg_encode_kv_job &b, const Sizes &z, uint8_t *const *bytes, void *const *lengths, cudaStream_t st) {
+    const uint8_t *ws = static_cast<const uint8_t *>(b.workspace);
+    for (int s0 = 0; s0 < z.nsub; s0 += kGatherSubs) {
+        const int n = z.nsub - s0 < kGatherSubs ? z.nsub - s0 : kGatherSubs;
+        GatherTargets t;
+        for (int k = 0; k < n; ++k) {
+            t.bytes[k] = bytes[s0 + k];
+            t.lengths[k] = lengths[s0 + k];
+        }
+        gather_kernel<Len><<<dim3(z.nslab, z.nrows, n), kGroup, 0, st>>>(
+            ws + z.scratch, z.stride, reinterpret_cast<const int32_t *>(ws + z.lengths),
+            reinterpret_cast<const int64_t *>(ws + z.group_off), z.nchannels, s0, t);
+        if (int rc = check_launch()) return rc;
+    }
+    return CG_OK;
+}
+}  // namespace
+
+extern "C" int cg_encode_kv_gather(const cg_encode_kv_job *job, uint8_t *const *bytes_host, int32_t *const *lengths_host,
+                                   void *stream) {
+    if (int rc = check_job(job)) return rc;
+    if (!bytes_host || !lengths_host) return CG_E_NULL;
+    const Sizes z = sizes_of(job->nlayers, job->ntokens, job->nheads, job->head_size);
+    for (int k = 0; k < z.nsub; ++k)
+        if (!bytes_host[k] || !lengths_host[k]) return CG_E_NULL;
+    return launch_gather<int32_t>(*job, z, bytes_host, reinterpret_cast<void *const *>(lengths_host),
+                                  static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cg_encode_kv_flat(const cg_encode_kv_job *job, const cg_flat_layout *layout, void *stream) {
+    if (int rc = check_job(job)) return rc;
+    if (!layout) return CG_E_NULL;
+    const cg_encode_kv_job &b = *job;
+    const cg_flat_layout &f = *layout;
+    const Sizes z = sizes_of(b.nlayers, b.ntokens, b.nheads, b.head_size);
+    if (!f.blob || !f.header_host || !f.sub_off_host || !f.mask_row_off) return CG_E_NULL;
+    if (f.header_bytes <= 0 || f.header_bytes > kMaxHeader || f.off_scales < f.header_bytes || f.off_tables < f.off_scales ||
+        f.off_lengths < f.off_tables || f.off_payload < f.off_lengths)
+        return CG_E_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(f.blob) | f.off_scales | f.off_tables | f.off_lengths) & 15) return CG_E_ALIGN;
+    if ((f.table_kind != CG_TABLES_CDF && !b.counts) || f.table_kind < CG_TABLES_CDF || f.table_kind > CG_TABLES_SPARSE) return CG_E_SHAPE;
+    if (z.nsub > kMaxHeader / 8) return CG_E_CAPACITY;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool sparse = f.table_kind == CG_TABLES_SPARSE;
+    // the gaps between sections (and inside sparse tables) are zero: the same KV gives the same bytes
+    cudaError_t e = cudaMemsetAsync(f.blob, 0, static_cast<size_t>(sparse ? f.off_payload : f.off_tables), st);
+    if (e == cudaSuccess && !sparse) e = cudaMemsetAsync(f.blob + f.off_tables + f.tables_bytes, 0,
+                                                        static_cast<size_t>(f.off_payload - f.off_tables - f.tables_bytes), st);
+    if (e == cudaSuccess && !sparse)
+        e = cudaMemcpyAsync(f.blob + f.off_tables, f.table_kind == CG_TABLES_CDF ? static_cast<const void *>(b.cdf) : b.counts,
+                            static_cast<size_t>(f.tables_bytes), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    const uint8_t *ws = static_cast<const uint8_t *>(b.workspace);
+    const uint32_t *group_nz = reinterpret_cast<const uint32_t *>(ws + z.group_nz);
+    FlatHeader h;
+    memcpy(h.bytes, f.header_host, static_cast<size_t>(f.header_bytes));
+    flat_front_kernel<<<32, 256, 0, st>>>(h, static_cast<int>(f.header_bytes), f.blob, static_cast<const uint16_t *>(b.scales_k),
+                                          static_cast<const uint16_t *>(b.scales_v),
+                                          static_cast<int64_t>(b.nlayers) * b.ntokens, f.off_scales,
+                                          sparse ? group_nz : nullptr, z.nrows * z.nslab, f.off_tables);
+    if (int rc = check_launch()) return rc;
+    if (sparse)
+        if (int rc = launch_sparse_write(b.counts, b.table_row_off, b.bins, z.nrows, z.nchannels, group_nz,
+                                         f.blob + f.off_tables + f.off_masks, f.mask_row_off,
+                                         f.blob + f.off_tables + f.off_counts, st))
+            return rc;
+    uint8_t *bytes[kMaxHeader / 8];
+    void *lengths[kMaxHeader / 8];
+    const int64_t streams = static_cast<int64_t>(z.nrows) * z.nchannels;
+    for (int k = 0; k < z.nsub; ++k) {
+        bytes[k] = f.blob + f.off_payload + f.sub_off_host[k];
+        lengths[k] = f.blob + f.off_lengths + k * streams * 2;
+    }
+    return launch_gather<uint16_t>(b, z, bytes, lengths, st);
+}

@@ -4,18 +4,22 @@
 byte-identical to what the reference produces from the same input -- with the reference's chain of
 torch ops and per-sub-chunk launches replaced by three C-ABI calls:
 
-    cg_quantize_cdf      split K/V + quantise + histogram + tables      (enc.py:257-267)
-    cg_encode_chunk      every sub-chunk's streams + offsets            (enc.py:269-292, 225-236)
-    cg_compact_streams   gather of the streams                          (enc.py:210-222)
+    cg_encode_kv         split K/V + quantise + tables + every sub-chunk's streams + offsets  (enc.py:257-292, 225-236)
+    cg_encode_kv_wait    waits for the payload sizes, all that the host needs to know
+    cg_encode_kv_gather  gather of the streams                                                (enc.py:210-222)
 
-Beside it: encode_many (a whole cache, up to a batch of chunks in flight and no wait in between), encode_levels
-(one chunk at several bin settings: cg_row_absmax + cg_quantize_cdf_scaled per level) and encode_flat
-(the CGB2 container of flat_format.py, tables packed by cg_pack_sparse_tables).
+Beside it: encode_many (a whole cache, chunks in flight on several streams and no wait in between), encode_levels
+(one chunk at several bin settings) and encode_flat (the CGB2 container of flat_format.py, filled by
+cg_encode_kv_flat).  quantize_and_tables, encode_streams and pack_sparse_tables are the same steps one by one.
 
 (enc.py = cachegen_encoder.py of the reference.)
 """
 import collections
+import contextlib
 import ctypes
+import dataclasses
+import threading
+import weakref
 from typing import Tuple
 
 import torch
@@ -242,79 +246,182 @@ def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = N
     return out, lengths, offs
 
 
-def _table_bins(key_bins: torch.Tensor, value_bins: torch.Tensor, max_bins: int = None) -> int:
-    """max_bins of the chunk's tables.  The reference builds key and value tables with their own
-    maximum and concatenates them, which needs the two to be equal (enc.py:265-267).  `max_bins`
-    overrides that: a layer shard of a model must use the whole model's value so that its tables and
-    streams are the ones an unsharded encode produces."""
-    kmax, vmax = int(key_bins.max()), int(value_bins.max())
-    if max_bins is not None:
-        if max_bins < max(kmax, vmax):
-            raise RuntimeError(f"max_bins {max_bins} is below the largest bin count {max(kmax, vmax)}")
-        return int(max_bins)
-    if kmax != vmax:
-        raise RuntimeError(f"Sizes of tensors must match: key tables have {kmax + 1} entries, value tables {vmax + 1}")
-    return kmax
+class _BinsInfo:
+    """What a pair of bins tensors means to an encode: read back from the GPU once, not on every call."""
+
+    def __init__(self, key_bins, value_bins):
+        self.value_ref = weakref.ref(value_bins)
+        self.versions = (key_bins._version, value_bins._version)
+        self.cpu = torch.cat((key_bins.detach().cpu(), value_bins.detach().cpu())).to(torch.float32)
+        self.nlayers = key_bins.numel()
+        self.kmax, self.vmax = int(key_bins.max()), int(value_bins.max())
+        self.on_device = {}   # device -> float32 [2L]
+        self.row_offsets = {}  # (device, channels) -> (int64 offsets of the byte counts, size, of the masks, size)
+
+    def on(self, dev):
+        t = self.on_device.get(dev)
+        if t is None:
+            t = self.on_device[dev] = self.cpu.to(dev)
+        return t
+
+    def offsets(self, dev, nchannels):
+        o = self.row_offsets.get((dev, nchannels))
+        if o is None:
+            counts = flat_format.table_row_offsets(self.cpu, nchannels)
+            masks = flat_format.mask_row_offsets(self.cpu, nchannels)
+            o = (torch.tensor(counts, dtype=torch.int64, device=dev), counts[-1],
+                 torch.tensor(masks, dtype=torch.int64, device=dev), masks[-1])
+            self.row_offsets[dev, nchannels] = o
+        return o
+
+    def table_bins(self, max_bins=None):
+        """max_bins of the chunk's tables.  The reference builds key and value tables with their own
+        maximum and concatenates them, which needs the two to be equal (enc.py:265-267).  `max_bins`
+        overrides that: a layer shard of a model must use the whole model's value so that its tables and
+        streams are the ones an unsharded encode produces."""
+        if max_bins is not None:
+            if max_bins < max(self.kmax, self.vmax):
+                raise RuntimeError(f"max_bins {max_bins} is below the largest bin count {max(self.kmax, self.vmax)}")
+            return int(max_bins)
+        if self.kmax != self.vmax:
+            raise RuntimeError(f"Sizes of tensors must match: key tables have {self.kmax + 1} entries, value tables {self.vmax + 1}")
+        return self.kmax
+
+
+_BINS_INFOS = {}  # id of a living key tensor -> (weak reference to it, _BinsInfo)
+
+
+def _bins_info(key_bins: torch.Tensor, value_bins: torch.Tensor) -> _BinsInfo:
+    """The pair's _BinsInfo, kept while the key tensor lives and for as long as neither is written to."""
+    key = id(key_bins)
+    ref, info = _BINS_INFOS.get(key, (None, None))
+    if (ref is None or ref() is not key_bins or info.value_ref() is not value_bins or
+            info.versions != (key_bins._version, value_bins._version)):
+        info = _BinsInfo(key_bins, value_bins)
+        _BINS_INFOS[key] = (weakref.ref(key_bins, lambda gone, key=key: _forget_bins(key, gone)), info)
+    return info
+
+
+def _forget_bins(key, gone):
+    if _BINS_INFOS.get(key, (None,))[0] is gone:
+        del _BINS_INFOS[key]
+
+
+_local = threading.local()
+_KEPT_TAILS = 32
+
+
+def _take_tail(n: int) -> torch.Tensor:
+    """Pinned int64 memory for an encode's sizes, from this thread's pool (at most _KEPT_TAILS buffers)."""
+    pool = _local.__dict__.setdefault("tails", [])
+    for i in range(len(pool) - 1, -1, -1):
+        if pool[i].numel() >= n:
+            return pool.pop(i)
+    return torch.empty(max(n, 64), dtype=torch.int64, pin_memory=True)
+
+
+def _give_tail(t: torch.Tensor) -> None:
+    pool = _local.__dict__.setdefault("tails", [])
+    if len(pool) < _KEPT_TAILS:
+        pool.append(t)
+
+
+_NOTHING = contextlib.nullcontext()
+
+
+def _current(dev):
+    """Context in which `dev` is the current device; nothing to do in the usual case."""
+    return _NOTHING if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 class _PendingChunk:
-    """One chunk whose quantise / table / coder kernels are enqueued but whose payload size is not
-    yet known on the host."""
+    """One chunk whose kernels up to the streams and their offsets are enqueued on `stream` (default: the
+    current one), but whose payload size is not yet known on the host.  finish() waits for that and
+    enqueues the gather.  Buffers come from the current stream's pool whatever `stream` is."""
 
-    def __init__(self, kv, key_bins, value_bins, max_bins, scales=None, delta=None):
-        self.L, _, self.T, self.H, self.D = kv.shape
-        self.dtype = kv.dtype
-        self.sym, self.scales, self.cdf = quantize_and_tables(kv, key_bins, value_bins, max_bins, scales=scales,
-                                                              delta=delta)
-        NL, T, C = self.sym.shape
-        dev = self.sym.device
-        self.nsub = (T + CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK - 1) // CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
-        self.stride = (_lib.stream_capacity(min(T, CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK)) + 3) // 4 * 4
-        nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
-        self.scratch = torch.empty((self.nsub, NL * C, self.stride), dtype=torch.uint8, device=dev)
-        self.lengths = torch.empty((self.nsub, NL, C), dtype=torch.int32, device=dev)
-        self.group_off = torch.empty((self.nsub, NL * nslab), dtype=torch.int64, device=dev)
-        # sub_off[0..nsub] then the status word, so that one transfer brings both to the host
-        self.tail = torch.zeros(self.nsub + 2, dtype=torch.int64, device=dev)
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
-        with torch.cuda.device(dev):
-            rc = _lib.lib().cg_encode_chunk(_ptr(self.cdf), _ptr(self.sym), NL, T, C, self.cdf.shape[2],
-                                            _ptr(self.scratch), self.stride, _ptr(self.lengths), _ptr(self.group_off),
-                                            _ptr(self.tail), _ptr(self.status), _stream(dev))
-        _lib.check(rc, "cg_encode_chunk")
-        self.tail[self.nsub + 1:].copy_(self.status)
-        self.sym = None  # symbols are consumed; free them early
-
-    def finish(self, host_tail) -> CacheGenGPUEncoderOutput:
-        bits = int(host_tail[self.nsub + 1])
-        if bits:
-            raise RuntimeError("cachegen encode: " + _lib.status_text(bits))
-        offs = [int(v) for v in host_tail[:self.nsub + 1]]
-        dev = self.cdf.device
-        NL, C = 2 * self.L, self.H * self.D
-        pieces = [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=dev) for j in range(self.nsub)]
-        with torch.cuda.device(dev):
-            if self.nsub == 1:
-                rc = _lib.lib().cg_compact_streams(_ptr(self.scratch), self.stride, _ptr(self.lengths),
-                                                   _ptr(self.group_off), _ptr(self.tail), 1, NL, C, _ptr(pieces[0]),
-                                                   _stream(dev))
-                _lib.check(rc, "cg_compact_streams")
-            else:
-                out = torch.empty(offs[-1], dtype=torch.uint8, device=dev)
-                rc = _lib.lib().cg_compact_streams(_ptr(self.scratch), self.stride, _ptr(self.lengths),
-                                                   _ptr(self.group_off), _ptr(self.tail), self.nsub, NL, C, _ptr(out),
-                                                   _stream(dev))
-                _lib.check(rc, "cg_compact_streams")
-                pieces = [out[offs[j]:offs[j + 1]].clone() for j in range(self.nsub)]
+    def __init__(self, kv, info, max_bins, delta=None, stream=None, workspace=None, with_counts=False):
+        if kv.dim() != 5 or kv.shape[1] != 2:
+            raise RuntimeError(f"expected a KV blob of shape [L, 2, T, H, D], got {tuple(kv.shape)}")
+        if kv.dtype not in _DTYPES:
+            raise TypeError(f"the codec takes float16 or bfloat16 KV, got {kv.dtype}")
+        if not kv.is_cuda:
+            raise RuntimeError("KV must be a CUDA tensor")
+        if kv.stride(4) != 1:
+            kv = kv.contiguous()
+        L, _, T, H, D = kv.shape
+        if info.nlayers != L:
+            raise RuntimeError(f"bins describe {info.nlayers} layers, the KV blob has {L}")
+        dev = kv.device
+        self.kv, self.info, self.dev = kv, info, dev
+        self.L, self.T, self.H, self.D, self.max_bins = L, T, H, D, max_bins
         step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
-        data_chunks = [CacheGenGPUBytestream(pieces[j], self.lengths[j] if self.nsub == 1 else self.lengths[j].clone(),
-                                             min(step, self.T - j * step)) for j in range(self.nsub)]
-        for t in (self.scratch, self.group_off, self.tail):
-            t.record_stream(torch.cuda.current_stream(dev))
-        return CacheGenGPUEncoderOutput(data_chunks, self.cdf,
-                                        max_tensors_key=self.scales[:self.L].clone().unsqueeze(-1),
-                                        max_tensors_value=self.scales[self.L:].clone().unsqueeze(-1),
-                                        num_heads=self.H, head_size=self.D)
+        self.nsub = (T + step - 1) // step
+        self.lib = _lib.lib()
+        self.stream = torch.cuda.current_stream(dev) if stream is None else stream
+        self.stream_ptr = ctypes.c_void_p(self.stream.cuda_stream)
+        self.bins = info.on(dev)
+        self.scales = torch.empty((2, L, T, 1), dtype=kv.dtype, device=dev) if with_counts else None
+        self.scales_k = self.scales[0] if with_counts else torch.empty((L, T, 1), dtype=kv.dtype, device=dev)
+        self.scales_v = self.scales[1] if with_counts else torch.empty((L, T, 1), dtype=kv.dtype, device=dev)
+        self.cdf = torch.empty((2 * L, H * D, max_bins + 1), dtype=torch.int16, device=dev)
+        need = self.lib.cg_encode_kv_workspace(L, T, H, D)
+        if need < 0:
+            _lib.check(need, "cg_encode_kv_workspace")
+        if workspace is None or workspace.numel() < need:
+            workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        self.workspace = workspace
+        self.tail = _take_tail(self.nsub + 4)
+        job = self.job = _lib.EncodeKvJob()
+        job.kv, job.bins, job.cdf = kv.data_ptr(), self.bins.data_ptr(), self.cdf.data_ptr()
+        job.scales_k, job.scales_v = self.scales_k.data_ptr(), self.scales_v.data_ptr()
+        job.workspace, job.workspace_bytes, job.tail = workspace.data_ptr(), workspace.numel(), self.tail.data_ptr()
+        job.s_layer, job.s_kv, job.s_token, job.s_head, _ = kv.stride()
+        job.dtype, job.nlayers, job.ntokens, job.nheads, job.head_size = _DTYPES[kv.dtype], L, T, H, D
+        job.max_bins = max_bins
+        self.counts = self.res_bins = None
+        if with_counts:
+            row_off, size, self.mask_off, self.mask_bytes = info.offsets(dev, H * D)
+            self.counts = torch.empty(size, dtype=torch.uint8, device=dev)
+            job.counts, job.table_row_off = self.counts.data_ptr(), row_off.data_ptr()
+        if delta is not None:
+            self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
+            job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
+        with _current(dev):
+            _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
+
+    def sizes(self):
+        """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
+        with _current(self.dev):
+            _lib.check(self.lib.cg_encode_kv_wait(ctypes.byref(self.job), self.stream_ptr), "cg_encode_kv_wait")
+        host = self.tail[:self.nsub + 3].tolist()
+        _give_tail(self.tail)
+        self.tail = None
+        bits = host[self.nsub + 1]
+        if bits & ~_lib.CG_S_COUNT_OVERFLOW:
+            raise RuntimeError("cachegen encode: " + _lib.status_text(bits & ~_lib.CG_S_COUNT_OVERFLOW))
+        return host[:self.nsub + 1], bits, host[self.nsub + 2]
+
+    def finish(self) -> CacheGenGPUEncoderOutput:
+        offs, _, _ = self.sizes()
+        n, NL, C = self.nsub, 2 * self.L, self.H * self.D
+        # every sub-chunk in tensors of its own: a view would pickle the whole buffer
+        pieces = [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(n)]
+        lengths = [torch.empty((NL, C), dtype=torch.int32, device=self.dev) for _ in range(n)]
+        array = ctypes.c_void_p * n
+        with _current(self.dev):
+            rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), array(*[t.data_ptr() for t in pieces]),
+                                              array(*[t.data_ptr() for t in lengths]), self.stream_ptr)
+        _lib.check(rc, "cg_encode_kv_gather")
+        step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
+        return CacheGenGPUEncoderOutput([CacheGenGPUBytestream(pieces[j], lengths[j], min(step, self.T - j * step))
+                                         for j in range(n)], self.cdf, self.scales_k, self.scales_v, self.H, self.D)
+
+    def abandon(self) -> None:
+        """Gives the buffers up after an error elsewhere: the GPU may still be writing to them."""
+        if self.tail is not None:
+            self.stream.synchronize()
+            _give_tail(self.tail)
+            self.tail = None
 
 
 def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tensor, chunk_tokens: int,
@@ -322,47 +429,46 @@ def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     """Encodes a whole KV cache [L, 2, T, H, D] (GPU, unit innermost stride) chunk by chunk, as
     LMCacheEngine.store does with one to_bytes call per chunk (LMCache/lmcache/cache_engine.py:205-255
     in the reference), but without waiting for a chunk's payload size before the next chunk's kernels
-    are enqueued: up to `batch` chunks are in flight; a chunk's sizes come back by an asynchronous copy
-    into pinned memory, and its streams are gathered once `batch` later chunks have been enqueued, so
-    the host never waits for the GPU except at the end.  Every chunk in flight keeps its own scratch
-    (136 MB for a 7B-shape chunk).  Consecutive chunks run on `streams` side streams in turn (see
-    _side_streams); the caller's stream waits for them before the call returns.
+    are enqueued: up to `batch` chunks, two a stream, are in flight; a chunk's streams are gathered when its
+    turn to be replaced comes, so the host waits for sizes that arrived long ago.  Every chunk in
+    flight keeps its own workspace (200 MB for a 7B-shape chunk).  Consecutive chunks run on `streams` side
+    streams in turn (see _side_streams); the caller's stream waits for them before the call returns.
     Returns the chunks' CacheGenGPUEncoderOutput objects, identical to per-chunk encode_function calls."""
-    kmax = _table_bins(key_bins, value_bins, max_bins)
+    info = _bins_info(key_bins, value_bins)
+    kmax = info.table_bins(max_bins)
     T = kv.shape[2]
+    info.on(kv.device)
     caller = torch.cuda.current_stream(kv.device)
     lanes = _side_streams(kv.device, streams)
     for side in lanes:
         side.wait_stream(caller)  # the cache is ready on the caller's stream
+    spare = [[] for _ in lanes]   # workspaces whose chunk has been gathered on that stream
     result, in_flight = [], collections.deque()
 
     def finish_oldest():
-        p, host, arrived, side = in_flight.popleft()
-        arrived.synchronize()
-        with torch.cuda.stream(side):
-            out = p.finish(host)
-        # made on a side stream, used and freed by the caller on its own
-        for t in _tensors_of(out):
-            t.record_stream(caller)
-        result.append(out)
+        p, lane = in_flight.popleft()
+        try:
+            result.append(p.finish())
+        finally:
+            p.abandon()
+        spare[lane].append(p.workspace)
 
-    for i, s in enumerate(range(0, T, chunk_tokens)):
-        side = lanes[i % len(lanes)]
-        with torch.cuda.stream(side):
-            p = _PendingChunk(kv[:, :, s:s + chunk_tokens], key_bins, value_bins, kmax, delta=delta)
-            host = torch.empty(p.tail.shape, dtype=p.tail.dtype, pin_memory=True)
-            host.copy_(p.tail, non_blocking=True)
-            arrived = torch.cuda.Event()
-            arrived.record(side)
-        in_flight.append((p, host, arrived, side))
-        # the oldest chunk's sizes arrived long ago: its gather queues up behind the kernels of the chunks
-        # after it, and the host work of finishing it runs while the GPU is busy with them
-        if len(in_flight) > batch:
+    try:
+        for i, s in enumerate(range(0, T, chunk_tokens)):
+            lane = i % len(lanes)
+            if len(in_flight) >= max(1, min(batch, 2 * len(lanes))):
+                finish_oldest()
+            ws = spare[lane].pop() if spare[lane] else None
+            # tensors come from the caller's stream's pool, and go back to it after the waits below
+            in_flight.append((_PendingChunk(kv[:, :, s:s + chunk_tokens], info, kmax, delta=delta, stream=lanes[lane],
+                                            workspace=ws), lane))
+        while in_flight:
             finish_oldest()
-    while in_flight:
-        finish_oldest()
-    for side in lanes:
-        caller.wait_stream(side)
+    finally:
+        for p, _ in in_flight:
+            p.abandon()
+        for side in lanes:
+            caller.wait_stream(side)
     return result
 
 
@@ -371,8 +477,8 @@ _SIDE_STREAMS = {}
 
 def _side_streams(device, n):
     """n streams of `device`, made once and kept: consecutive chunks of encode_many go to different
-    streams, so that one chunk's kernels fill the SMs that the last, partly filled wave of the previous
-    chunk's coder kernel leaves idle (2,048 blocks over 1,480 resident ones: 1.4 waves)."""
+    streams, so that one chunk's quantisation, which is bound by memory, runs beside another's coder, which
+    is bound by instruction issue, and fills what its last wave leaves idle."""
     key = (torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device())
     have = _SIDE_STREAMS.setdefault(key, [])
     while len(have) < n:
@@ -380,59 +486,34 @@ def _side_streams(device, n):
     return have[:n]
 
 
-def _tensors_of(out: CacheGenGPUEncoderOutput):
-    yield out.cdf
-    yield out.max_tensors_key
-    yield out.max_tensors_value
-    for piece in out.data_chunks:
-        yield piece.bytestream
-        yield piece.bytestream_lengths
-
-
 def encode_levels(kv: torch.Tensor, levels: list) -> list:
     """One chunk of KV, [L, 2, T, H, D] on the GPU, encoded at several bin settings: `levels` is a list
     of (key_bins, value_bins) pairs, the result one CacheGenGPUEncoderOutput per pair, each identical
     to what encode_function gives with those bins.  This is what the reference's adaptation scripts
     store per chunk (one blob per QUANT_LEVEL, run_adaptation.py:61-72) so that config_selection can
-    pick a level per chunk (src/utils.py:294-314).  The levels share the max|x| pass and one host
-    synchronisation; the coder runs once per level, and it is what an encode spends most time in."""
+    pick a level per chunk (src/utils.py:294-314).  All levels are enqueued before the host waits for the
+    first one's size."""
     if kv.stride(4) != 1:
         kv = kv.contiguous()
-    scales = row_scales(kv)
-    pending = [_PendingChunk(kv, kb, vb, _table_bins(kb, vb), scales=scales) for kb, vb in levels]
-    host = torch.cat([p.tail for p in pending]).cpu()  # the one synchronisation
-    out, pos = [], 0
-    for p in pending:
-        out.append(p.finish(host[pos:pos + p.nsub + 2]))
-        pos += p.nsub + 2
-    return out
+    infos = [_bins_info(kb, vb) for kb, vb in levels]
+    pending = []
+    try:
+        for info in infos:
+            pending.append(_PendingChunk(kv, info, info.table_bins()))
+        return [p.finish() for p in pending]
+    finally:
+        for p in pending:
+            p.abandon()
 
 
 @_lmcache_nvtx_annotate
 def encode_function(kv: torch.Tensor, config: CacheGenConfig, key_bins: torch.Tensor, value_bins: torch.Tensor,
                     chunk_size: int, max_bins: int = None, delta=None) -> CacheGenGPUEncoderOutput:
     """Encodes one chunk of KV, [L, 2, T, H, D] on the GPU, T == chunk_size (enc.py:247-301)."""
-    num_heads, head_size = kv.shape[-2:]
-    L = kv.shape[0]
     if kv.shape[2] != chunk_size:
         raise RuntimeError(f"chunk_size {chunk_size} does not match the {kv.shape[2]} tokens of the blob")
-    kmax = _table_bins(key_bins, value_bins, max_bins)
-    sym, scales, cdf = quantize_and_tables(kv, key_bins, value_bins, kmax, delta=delta)
-    stream_bytes, lengths, offs = encode_streams(cdf, sym)
-    data_chunks = []
-    step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
-    nsub = len(offs) - 1
-    for j in range(nsub):
-        piece = stream_bytes[offs[j]:offs[j + 1]]
-        data_chunks.append(CacheGenGPUBytestream(
-            bytestream=piece if nsub == 1 else piece.clone(),  # a view would pickle the whole buffer
-            bytestream_lengths=lengths[j] if nsub == 1 else lengths[j].clone(),
-            ntokens=min(step, chunk_size - j * step)))
-    return CacheGenGPUEncoderOutput(
-        data_chunks, cdf,
-        max_tensors_key=scales[:L].clone().unsqueeze(-1),
-        max_tensors_value=scales[L:].clone().unsqueeze(-1),
-        num_heads=num_heads, head_size=head_size)
+    info = _bins_info(key_bins, value_bins)
+    return _PendingChunk(kv, info, info.table_bins(max_bins), delta=delta).finish()
 
 
 def pack_sparse_tables(counts: torch.Tensor, bins: torch.Tensor, nchannels: int, bins_cpu: torch.Tensor = None):
@@ -465,41 +546,33 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     the tables in the smallest form that can hold them.  compact_tables: True (sparse byte counts when
     every non-centre histogram count fits a byte and no row has more than 32 of them, else dense byte
     counts when the counts fit, else the int16 tables), "counts" (never sparse) or False (always int16)."""
-    L, _, T, H, D = kv.shape
-    C = H * D
-    kmax = _table_bins(key_bins, value_bins, max_bins)
-    bins = torch.cat((key_bins, value_bins)).to(device=kv.device, dtype=torch.float32).contiguous()
-    bins_cpu = bins.cpu()
-    sym, scales, cdf, counts, qstatus = quantize_and_tables(kv, key_bins, value_bins, kmax, with_counts=True,
-                                                            bins_cpu=bins_cpu, delta=delta)
-    try_sparse = compact_tables is True and flat_format.sparse_representable(bins_cpu)
-    if try_sparse:
-        sparse, written, off_counts = pack_sparse_tables(counts, bins, C, bins_cpu)
-        extra = torch.cat((qstatus.to(torch.int64), written.to(torch.int64)))
-        stream_bytes, lengths, offs, (qbits, nwritten) = encode_streams(cdf, sym, extra_status=extra)
-    else:
-        stream_bytes, lengths, offs, qbits = encode_streams(cdf, sym, extra_status=qstatus)
-    fits = bool(compact_tables) and not (qbits & _lib.CG_S_COUNT_OVERFLOW)
-    if fits and try_sparse:
-        kind, tables = flat_format.TABLES_SPARSE, sparse[:off_counts + nwritten]
+    info = _bins_info(key_bins, value_bins)
+    kmax = info.table_bins(max_bins)
+    p = _PendingChunk(kv, info, kmax, delta=delta, with_counts=True)
+    offs, bits, nonzero = p.sizes()
+    fits = bool(compact_tables) and not (bits & _lib.CG_S_COUNT_OVERFLOW)
+    off_masks, off_counts = flat_format.sparse_parts(2 * p.L, p.H * p.D, p.mask_bytes)
+    if fits and compact_tables is True and flat_format.sparse_representable(info.cpu):
+        kind, size = flat_format.TABLES_SPARSE, off_counts + nonzero
     elif fits:
-        kind, tables = flat_format.TABLES_COUNTS, counts
+        kind, size = flat_format.TABLES_COUNTS, p.counts.numel()
     else:
-        kind, tables = flat_format.TABLES_CDF, cdf.view(torch.uint8).reshape(-1)
-    header = flat_format.layout(L, H, D, T, kmax + 1, kv.dtype, kind, tables.numel(), flat_format.LENGTHS_U16, offs,
-                                bins_checksum=flat_format.bins_checksum(bins_cpu, delta))
-    # zeroed, so that the alignment gaps between the sections are defined: the same KV gives the same bytes
-    blob = torch.zeros(header.total, dtype=torch.uint8, device=kv.device)
+        kind, size = flat_format.TABLES_CDF, 2 * p.cdf.numel()
+    header = flat_format.layout(p.L, p.H, p.D, p.T, kmax + 1, p.kv.dtype, kind, size, flat_format.LENGTHS_U16, offs,
+                                bins_checksum=flat_format.bins_checksum(info.cpu, delta))
     head = header.pack()
-    blob[:len(head)].copy_(torch.frombuffer(bytearray(head), dtype=torch.uint8), non_blocking=True)
-    chunk = flat_format.FlatChunk(blob, header)
-    chunk.scales().copy_(scales)
-    blob[header.off_tables:header.off_tables + tables.numel()].copy_(tables)
-    n = 2 * L * C
-    blob[header.off_lengths:header.off_lengths + len(offs[:-1]) * n * 2].view(torch.int16).copy_(
-        lengths.reshape(-1).to(torch.int16))  # at most 520: fits
-    blob[header.off_payload:header.off_payload + offs[-1]].copy_(stream_bytes)
-    return chunk
+    blob = torch.empty(header.total, dtype=torch.uint8, device=p.dev)
+    f = _lib.FlatLayout()
+    sub_off = (ctypes.c_int64 * p.nsub)(*offs[:p.nsub])
+    f.blob, f.mask_row_off = blob.data_ptr(), p.mask_off.data_ptr()
+    f.header_host, f.header_bytes = ctypes.cast(ctypes.c_char_p(head), ctypes.c_void_p), len(head)
+    f.sub_off_host = ctypes.cast(sub_off, ctypes.c_void_p)
+    f.off_scales, f.off_tables, f.tables_bytes = header.off_scales, header.off_tables, size
+    f.off_lengths, f.off_payload = header.off_lengths, header.off_payload
+    f.off_masks, f.off_counts, f.table_kind = off_masks, off_counts, kind
+    with _current(p.dev):
+        _lib.check(p.lib.cg_encode_kv_flat(ctypes.byref(p.job), ctypes.byref(f), p.stream_ptr), "cg_encode_kv_flat")
+    return flat_format.FlatChunk(blob, header)
 
 
 class CacheGenSerializer(Serializer):
@@ -522,6 +595,7 @@ class CacheGenSerializer(Serializer):
         self.fmt = metadata.fmt
         self.key_bins = self.make_key_bins(self.cachegen_config)
         self.value_bins = self.make_value_bins(self.cachegen_config)
+        self._levels = {}
 
     def make_key_bins(self, config: CacheGenConfig) -> torch.Tensor:
         return CGBasics.make_key_bins(config, "cuda")
@@ -555,8 +629,15 @@ class CacheGenSerializer(Serializer):
         if self.fmt == "huggingface":
             tensor = tensor.permute(0, 1, 3, 2, 4)
         tensor = tensor.cuda()
-        return encode_levels(tensor, [(CGBasics.make_key_bins(c, tensor.device), CGBasics.make_value_bins(c, tensor.device))
-                                      for c in cachegen_configs])
+        return encode_levels(tensor, [self._level_bins(c, tensor.device) for c in cachegen_configs])
+
+    def _level_bins(self, config: CacheGenConfig, device):
+        """The bins of a quality level, made once per setting."""
+        key = (device, dataclasses.astuple(config))
+        bins = self._levels.get(key)
+        if bins is None:
+            bins = self._levels[key] = (CGBasics.make_key_bins(config, device), CGBasics.make_value_bins(config, device))
+        return bins
 
     def encode_flat(self, tensor: torch.Tensor, compact_tables=True) -> flat_format.FlatChunk:
         """The chunk as a CGB2 container on the GPU."""

@@ -276,6 +276,57 @@ int cg_compact_streams(const uint8_t *scratch, int64_t scratch_stride, const int
                        const int64_t *group_off, const int64_t *sub_off, int nsub, int nrows,
                        int nchannels, uint8_t *bytes_out, void *stream);
 
+/*
+ * The whole encode of one chunk (cachegen_encoder.py:247-301) without a host wait inside: cg_encode_kv enqueues
+ * quantisation, tables, arithmetic coding and offsets; the sizes of the sub-chunks' payloads then arrive in
+ * `tail`, which cg_encode_kv_wait waits for; cg_encode_kv_gather (or cg_encode_kv_flat) enqueues the
+ * gather of the streams into buffers of those sizes.  Same tables, scales, streams and lengths as
+ * cg_quantize_cdf + cg_encode_chunk + cg_compact_streams, in fewer launches and passes over memory.
+ * Symbols must lie below max_bins - 1, which holds when bins[row] <= max_bins and the KV is finite;
+ * others raise CG_S_BAD_SYMBOL.
+ */
+typedef struct cg_encode_kv_job {
+    const void *kv;           /* 16-bit KV, element (layer, k/v, token, head, d) at the strides below */
+    const float *bins;        /* [2L] */
+    const float *res_bins;    /* [2L], delta coding only */
+    void *scales_k, *scales_v; /* out: max|x| per (layer, token), [L, ntokens] in the KV's type each */
+    int16_t *cdf;             /* out: [2L, C, max_bins + 1] */
+    uint8_t *counts;          /* out: byte counts (CG_TABLES_COUNTS), or NULL */
+    const int64_t *table_row_off; /* [2L + 1] offsets into counts, with counts only */
+    void *workspace;          /* cg_encode_kv_workspace bytes, 256-byte aligned; in use until the gather has run */
+    int64_t *tail;            /* [nsub + 4], HOST memory the GPU can write (pinned): payload offsets of the sub-chunks
+                                 [0 .. nsub], status bits, number of non-zero byte counts (with counts only),
+                                 then a word that becomes 1 when the others are there */
+    int64_t workspace_bytes;
+    int64_t s_layer, s_kv, s_token, s_head;
+    int32_t dtype, nlayers, ntokens, nheads, head_size, max_bins;
+    int32_t delta_group;      /* 0, or tokens per group (cg_quantize_cdf_delta) */
+    int32_t reserved;
+} cg_encode_kv_job;
+
+/* bytes of cg_encode_kv_job.workspace; CG_E_SHAPE for non-positive extents */
+int64_t cg_encode_kv_workspace(int nlayers, int ntokens, int nheads, int head_size);
+int cg_encode_kv(const cg_encode_kv_job *job_host, void *stream);
+/* returns when job's tail is complete; CG_E_CUDA if the stream failed before */
+int cg_encode_kv_wait(const cg_encode_kv_job *job_host, void *stream);
+/* bytes_host[j], lengths_host[j]: device buffers of sub-chunk j, tail[j+1] - tail[j] bytes and int32 [2L, C] */
+int cg_encode_kv_gather(const cg_encode_kv_job *job_host, uint8_t *const *bytes_host, int32_t *const *lengths_host,
+                        void *stream);
+
+/* A CGB2 container (serde/flat_format.py) filled from an encoded chunk: header, scales, tables of the given kind,
+ * uint16 lengths, payload, zero bytes between them. */
+typedef struct cg_flat_layout {
+    uint8_t *blob;             /* device, 16-byte aligned */
+    const void *header_host;
+    const int64_t *sub_off_host;   /* [nsub]: payload offsets, from tail */
+    const int64_t *mask_row_off;   /* device [2L + 1], sparse tables */
+    int64_t header_bytes, off_scales, off_tables, tables_bytes, off_lengths, off_payload;
+    int64_t off_masks, off_counts; /* inside the tables section, sparse tables */
+    int32_t table_kind;        /* CG_TABLES_*; the byte-count kinds need job->counts */
+    int32_t reserved;
+} cg_flat_layout;
+int cg_encode_kv_flat(const cg_encode_kv_job *job_host, const cg_flat_layout *layout_host, void *stream);
+
 /* ------------------------------------------------------------------------------------------
  * fused decode side
  * ------------------------------------------------------------------------------------------ */
