@@ -460,16 +460,20 @@ CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *strea
 // still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above them (a
 // word leaves nothing behind it) and is added to the stored words when the next word goes out; that
 // takes a run of ones from there to the last stored word, which real tables about never give.
-struct BitSink {
+// STEP: words between consecutive words of the row (32: the rows of a warp's streams interleaved, so that
+// they take no more cache lines than they have data for and are read back coalesced).
+template <int STEP>
+struct BitSinkT {
     uint32_t *row;    // 4-byte aligned scratch row of this stream
     uint32_t cap_w;   // words that fit in the row
     uint32_t nwords;  // words produced so far (may exceed cap_w: then nothing more is stored)
     uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo), and a carry above them
     uint32_t nacc;            // number of bits pending, < 63
 
-    CG_HD void init(uint8_t *p, int64_t stride) {
+    // p: where the stream's first word goes; nbytes: room for the stream
+    CG_HD void init(uint8_t *p, int64_t nbytes) {
         row = reinterpret_cast<uint32_t *>(p);
-        cap_w = static_cast<uint32_t>(stride >> 2);
+        cap_w = static_cast<uint32_t>(nbytes >> 2);
         nwords = 0;
         acc_hi = 0;
         acc_lo = 0;
@@ -480,8 +484,8 @@ struct BitSink {
         if (nwords > cap_w) return;  // the words before are not in the row: reported as an overflow
         for (uint32_t i = nwords; i > 0u;) {
             --i;
-            const uint32_t v = cg_bswap32(row[i]) + 1u;
-            row[i] = cg_bswap32(v);
+            const uint32_t v = cg_bswap32(row[i * STEP]) + 1u;
+            row[i * STEP] = cg_bswap32(v);
             if (v) return;
         }
     }
@@ -492,7 +496,7 @@ struct BitSink {
         if (cg_fshr_clamp(acc_hi, 0u, nacc)) carry_into_row();
         acc_hi = 0u;
         acc_lo &= ~cg_shl(0xFFFFFFFFu, nacc);
-        if (nwords < cap_w) row[nwords] = cg_bswap32(w);
+        if (nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
         nwords++;
     }
     // zero-fills to a byte boundary; returns the stream length in bytes
@@ -503,11 +507,13 @@ struct BitSink {
         const uint32_t bytes = nwords * 4u + ((nacc + 7u) >> 3);
         if (nacc) {
             const uint32_t w = acc_lo << (32u - nacc);
-            if (nwords < cap_w) row[nwords] = cg_bswap32(w);
+            if (nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
         }
         return bytes;
     }
 };
+
+using BitSink = BitSinkT<1>;
 
 // ---- encoder state and step -----------------------------------------------------------------------------
 // A symbol starts with fewer bits than this in the accumulator; it adds at most 18 (the updated interval of a
@@ -526,7 +532,8 @@ struct EncoderState {
         low = 0u;
         span32 = 0u;
     }
-    CG_HD void add_to_low(uint32_t v, BitSink &out) {
+    template <class Sink>
+    CG_HD void add_to_low(uint32_t v, Sink &out) {
 #if defined(__CUDA_ARCH__)
         asm("add.cc.u32 %0, %0, %3; addc.cc.u32 %1, %1, 0; addc.u32 %2, %2, 0;"
             : "+r"(low), "+r"(out.acc_lo), "+r"(out.acc_hi) : "r"(v));
@@ -540,15 +547,18 @@ struct EncoderState {
     // accumulator (every lane that has one stores it as soon as one lane is near the high-water mark), the
     // full 2^32 range (a stream's first symbol; later only if a shift lands on it exactly) and the table's last
     // symbol, whose upper bound is the range's end (LAST = false: s < maxsym is known).
-    template <bool LAST = true>
-    CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, BitSink &out, uint32_t lanes) {
+    template <bool LAST = true, class Sink>
+    CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, Sink &out, uint32_t lanes) {
         const uint32_t a = col + s * kTableRowBytes;
         const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + kTableRowBytes);
         uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
         if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (LAST && s == maxsym))) {
             if (out.nacc >= 32u) out.store_word();
-            flo = scale_exact(span32, e0);
-            fhi = LAST && s == maxsym ? span32 : scale_exact(span32, e1);
+            if (span32 == 0u) {
+                flo = e0;
+                fhi = e1;
+            }
+            if (LAST && s == maxsym) fhi = span32;
         }
         add_to_low(flo, out);
         span32 = fhi - flo;
@@ -562,7 +572,8 @@ struct EncoderState {
     // final flush (enc_new.cu:298-306): two bits that place the stream's value inside the interval, 01 or
     // 10 above the reference's low with its pending bits, which is L plus a quarter of the window cut
     // to two bits; returns the stream length in bytes
-    CG_HD uint32_t flush(BitSink &out) {
+    template <class Sink>
+    CG_HD uint32_t flush(Sink &out) {
         add_to_low(0x40000000u, out);
         if (out.nacc >= 32u && out.nacc < 63u) out.store_word();
         out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, 30u);

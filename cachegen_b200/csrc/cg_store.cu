@@ -15,6 +15,7 @@ struct KvView {
     const uint16_t *kv;
     int64_t s_layer, s_kv, s_token, s_head;
     int nlayers, ntokens, nheads, head_size;
+    uint32_t head_inv;  // ceil(2^32 / head_size): channel / head_size by a multiply-high, exact below 2^16
 };
 
 // ---- pass 1: max|x| and quantise ---------------------------------------------------------------------------
@@ -25,8 +26,24 @@ struct KvView {
 // 128-bit loads a thread in flight.
 constexpr int kTokensPerWord = 4;
 
-template <int DT>
-__global__ void __launch_bounds__(1024) quantize_tokens_kernel(const KvView v, const float *__restrict__ bins, int max_bins,
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// (x * f + m) + 2^23 for two values: three separately rounded fp32 operations each (enc.py:56-57), the last of which
+// rounds half to even and leaves the symbol in the low byte.  The products stay scalar: a packed product in
+// front of a packed sum came out as one fused multiply-add (a symbol in 10^7 differed).
+__device__ __forceinline__ void quantize2(float x0, float x1, float f, uint64_t m, uint32_t *b0, uint32_t *b1) {
+    const uint64_t magic = 0x4B0000004B000000ull;
+    uint64_t v = pack2(__fmul_rn(x0, f), __fmul_rn(x1, f));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(m));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(magic));
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(*b0), "=r"(*b1) : "l"(v));
+}
+
+template <int DT, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const KvView v, const float *__restrict__ bins, int max_bins,
                                                                uint16_t *__restrict__ scales_k,
                                                                uint16_t *__restrict__ scales_v,
                                                                uint32_t *__restrict__ sym4, uint32_t *zeroed, int nzeroed) {
@@ -43,7 +60,7 @@ __global__ void __launch_bounds__(1024) quantize_tokens_kernel(const KvView v, c
 #pragma unroll
     for (int j = 0; j < kTokensPerWord; ++j) x[j] = make_uint4(0u, 0u, 0u, 0u);
     if (c < C) {
-        const int h = c / v.head_size;
+        const int h = static_cast<int>(__umulhi(static_cast<uint32_t>(c), v.head_inv));
         const uint16_t *p = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token + h * v.s_head + (c - h * v.head_size);
 #pragma unroll
         for (int j = 0; j < kTokensPerWord; ++j)
@@ -82,18 +99,19 @@ __global__ void __launch_bounds__(1024) quantize_tokens_kernel(const KvView v, c
     if (c >= C) return;
     const float f[kTokensPerWord] = {factor_s.x, factor_s.y, factor_s.z, factor_s.w};
     const uint32_t keep = keep_s;
+    const uint64_t m2 = pack2(MAX, MAX);
     uint32_t w[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        uint32_t b[kTokensPerWord];
+    for (int k = 0; k < 8; k += 2) {
+        uint32_t b0[kTokensPerWord], b1[kTokensPerWord];
 #pragma unroll
         for (int j = 0; j < kTokensPerWord; ++j) {
-            const uint32_t pair = k < 2 ? x[j].x : k < 4 ? x[j].y : k < 6 ? x[j].z : x[j].w;
-            const uint16_t hb = static_cast<uint16_t>(k & 1 ? pair >> 16 : pair);
-            // three separately rounded fp32 operations, then round-half-even (enc.py:56-57)
-            b[j] = __float_as_uint(__fadd_rn(__fadd_rn(__fmul_rn(Half16<DT>::to_float(hb), f[j]), MAX), 8388608.0f));
+            const uint32_t pair = k == 0 ? x[j].x : k == 2 ? x[j].y : k == 4 ? x[j].z : x[j].w;
+            quantize2(Half16<DT>::to_float(static_cast<uint16_t>(pair)), Half16<DT>::to_float(static_cast<uint16_t>(pair >> 16)),
+                      f[j], m2, &b0[j], &b1[j]);
         }
-        w[k] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410) & keep;
+        w[k] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410) & keep;
+        w[k + 1] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410) & keep;
     }
     // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
     // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
@@ -123,16 +141,23 @@ __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage,
                                                 uint8_t *counts, int64_t counts_stride, bool *overflow) {
     const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(lp - 1);
     const uint32_t total = ntokens & 0xFFFFu;  // the reference accumulates in uint16
-    // scale * cum / total by the rounded-down reciprocal, one below the quotient at most
-    const uint32_t inv = total > 1u ? 0xFFFFFFFFu / total : 0u;
+    // scale * cum / total: a shift, or the rounded-down reciprocal, whose product is at most one below the quotient
+    const bool pow2 = (total & (total - 1u)) == 0u;
+    const int sh = 31 - __clz(static_cast<int>(total | 1u));
+    const uint32_t inv = 0xFFFFFFFFu / (total | (total == 0u));
     uint32_t cum = 0;
-    int nz = 0;
-    for (int m = 0; m < lp; ++m) {
+    int nz = 0, m = 0;
+    for (; m < lp; ++m) {
+        if (cum == ntokens) break;  // every symbol is below m: the entries from here on only count up
         const uint32_t n = hist[m * kGroup];
         const uint32_t prod = scale * (cum & 0xFFFFu);
-        uint32_t q = __umulhi(prod, inv);
-        if (prod - q * total >= total) ++q;
-        if (total <= 1u) q = total ? prod : 0u;
+        uint32_t q;
+        if (pow2) {
+            q = prod >> sh;
+        } else {
+            q = __umulhi(prod, inv);
+            if (prod - q * total >= total) ++q;
+        }
         const uint32_t e = (q + static_cast<uint32_t>(m)) & 0xFFFFu;
         hist[m * kGroup] = e << 16;
         stage[m] = static_cast<uint16_t>(e);
@@ -148,6 +173,17 @@ __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage,
             }
         }
     }
+    if (counts)
+        for (int j = m; j <= 2 * cq && j < lp - 1; ++j)
+            if (j != cq) {
+                *counts = 0u;
+                counts += counts_stride;
+            }
+    for (; m < lp; ++m) {
+        const uint32_t e = (scale + static_cast<uint32_t>(m)) & 0xFFFFu;
+        hist[m * kGroup] = e << 16;
+        stage[m] = static_cast<uint16_t>(e);
+    }
     return nz;
 }
 
@@ -162,12 +198,13 @@ __device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst
     }
 }
 
+__device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return __byte_perm(w, 0u, 0x4440u + k); }
 __device__ __forceinline__ void count_symbol(uint32_t addr) {
     asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
 }
 __device__ __forceinline__ void count_word(uint32_t col, uint32_t w) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+    for (int k = 0; k < 4; ++k) count_symbol(col + byte_of(w, k) * kRowBytes);
 }
 
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
@@ -189,13 +226,23 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint
     if (c < nchannels) {
         const uint32_t col = smem_addr(hist + cl);
         const uint32_t *p = sym4 + static_cast<int64_t>(row) * words * nchannels + c;
-        for (int i = part; i < words; i += kParts) {
-            uint32_t w = __ldg(p + static_cast<int64_t>(i) * nchannels);
-            if (w & 0x80808080u) w = 0u;  // reported by the coder
-            if (i < whole) {
-                count_word(col, w);
-            } else {
-                for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+        constexpr int kAhead = 8;  // loads in flight
+        for (int i0 = part; i0 < words; i0 += kParts * kAhead) {
+            uint32_t w[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const int i = i0 + j * kParts;
+                w[j] = i < words ? __ldg(p + static_cast<int64_t>(i) * nchannels) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const int i = i0 + j * kParts;
+                if (w[j] & 0x80808080u) w[j] = 0u;  // reported by the coder
+                if (i < whole) {
+                    count_word(col, w[j]);
+                } else if (i < words) {
+                    for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w[j] >> (8 * k)) & 0xFFu) * kRowBytes);
+                }
             }
         }
     }
@@ -230,7 +277,7 @@ struct StoreParams {
     const uint32_t *sym4;
     TableOut out;
     int ntokens, nchannels, lp, nrows, nsub;
-    uint8_t *scratch;     // [nsub, nrows * C, stride]
+    uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4, 32 lanes] words
     int64_t stride;
     int32_t *lengths;     // [nsub, nrows * C]
     int64_t *group_off;   // [nsub, nrows * nslab]: byte offset of each 128-channel group inside its sub-chunk
@@ -239,6 +286,14 @@ struct StoreParams {
     int32_t *status;      // zero before pass 1
     int64_t *tail;        // [nsub + 4], see cg_encode_kv_job
 };
+
+// The scratch rows of the 32 streams of a warp lie interleaved: word k of stream `lane` is word 32 k + lane of
+// the warp's 32 * stride bytes.  A stream takes 45 of its 520 bytes on the usual workload: laid out row by
+// row that is a cache line or two for every stream (70 MB of lines a Llama-7B chunk, which the L2 did not
+// keep), interleaved it is as many lines as there is data, and the gather reads them whole.
+__device__ __forceinline__ uint32_t *scratch_word(uint8_t *scratch, int64_t stride, int64_t group, int tid) {
+    return reinterpret_cast<uint32_t *>(scratch + (group * (kGroup / 32) + (tid >> 5)) * 32 * stride) + (tid & 31);
+}
 
 // Exclusive scan of n values in place by one block of kGroup threads; returns the sum.
 template <class T>
@@ -311,23 +366,28 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
         if (active) {
             for (int m = 0; m < p.lp; ++m) tab[m * kGroup + tid] = 0u;
             const uint32_t *q = sp;
+            constexpr int kAhead = 2 * kWordsAhead;
+            uint32_t w[kAhead], next[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) w[k] = 4 * k < n ? __ldg(q + k * C) : 0u;
             int i = 0;
-            for (; i + 4 * kWordsAhead <= n; i += 4 * kWordsAhead) {
-                uint32_t w[kWordsAhead];
+            for (; i + 4 * kAhead <= n; i += 4 * kAhead) {
+                q += kAhead * C;
 #pragma unroll
-                for (int k = 0; k < kWordsAhead; ++k) w[k] = __ldg(q + k * C);
-                q += kWordsAhead * C;
+                for (int k = 0; k < kAhead; ++k) next[k] = i + 4 * (kAhead + k) < n ? __ldg(q + k * C) : 0u;
 #pragma unroll
-                for (int k = 0; k < kWordsAhead; ++k) {
+                for (int k = 0; k < kAhead; ++k) {
                     if (w[k] & 0x80808080u) w[k] = 0u;
                     count_word(col, w[k]);
+                    w[k] = next[k];
                 }
             }
-            for (; i < n; i += 4) {
-                uint32_t w = __ldg(q);
-                q += C;
-                if (w & 0x80808080u) w = 0u;
-                for (int k = 0; k < min(4, n - i); ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kRowBytes);
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                if (w[k] & 0x80808080u) w[k] = 0u;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (i + 4 * k + j < n) count_symbol(col + byte_of(w[k], j) * kRowBytes);
             }
             const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
             nz = counts_to_column(tab + tid, stage + tid * p.lp, p.lp, n, cq,
@@ -347,8 +407,9 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     if (active) {
         const int64_t slot = static_cast<int64_t>(sub) * p.nrows * C + g;
         const uint32_t top = static_cast<uint32_t>(p.lp - 2);
-        BitSink out;
-        out.init(p.scratch + slot * p.stride, p.stride);
+        BitSinkT<32> out;  // see scratch_word
+        out.init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x, tid)),
+                 p.stride);
         EncoderState enc;
         enc.init();
         constexpr int kAhead = 4 * kWordsAhead;
@@ -370,7 +431,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
             for (int k = 0; k < kWordsAhead; ++k) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    enc.step<false>(Smem{}, col, (w[k] >> (8 * j)) & 0xFFu, top, out, lanes);
+                    enc.step<false>(Smem{}, col, byte_of(w[k], j), top, out, lanes);
             }
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) w[k] = next[k];
@@ -471,47 +532,78 @@ struct GatherTargets {
     void *lengths[kGatherSubs];  // int32 or uint16 [nrows, C]
 };
 
-// One block per (group, row, sub-chunk), eight lanes per stream, sixteen streams in flight.  Streams lie back to
-// back, at any byte: the words that are aligned at the destination are put together from two source words, so
-// that a stream of n bytes takes n / 4 word stores and at most six byte stores where copying byte by byte
-// takes n of them (a 256-token Llama-7B chunk, 11.8 MB of streams of 45 bytes: the stores were what bound it).
-template <class Len>
+// One block per (group, row, sub-chunk), one thread per stream.  A warp's streams are one run of the output: each
+// lane shifts its words to the byte they start at and puts them together in shared memory (a word that two
+// streams share by an atomic or), and the warp writes the run with 128-bit stores.  Copying stream after stream
+// to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
+// with words assembled from two source words 24 us: one short dependent copy after the other.
+constexpr int kGatherWords = 1536;  // words of shared memory a warp; longer runs take the lanes' own byte stores
+template <class Len, bool INTERLEAVED>
 __global__ void __launch_bounds__(kGroup) gather_kernel(const uint8_t *__restrict__ scratch, int64_t stride,
                                                         const int32_t *__restrict__ lengths,
                                                         const int64_t *__restrict__ group_off, int nchannels, int sub0,
                                                         const __grid_constant__ GatherTargets out) {
+    __shared__ uint4 stage[kGroup / 32][kGatherWords / 4];
     __shared__ int warp_sums[kGroup / 32];
-    __shared__ int2 place[kGroup];  // offset, length
-    const int tid = threadIdx.x, row = blockIdx.y, sub = sub0 + blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = blockIdx.y, sub = sub0 + blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
     const int c = blockIdx.x * kGroup + tid;
-    const int64_t slot0 = (static_cast<int64_t>(sub) * nrows + row) * nchannels + blockIdx.x * kGroup;
-    const int len = c < nchannels ? __ldg(lengths + slot0 + tid) : 0;
-    const int64_t at = __ldg(group_off + (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x);
+    const int64_t group = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
+    const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
+    int len = c < nchannels ? __ldg(lengths + slot) : 0;
+    const int64_t at = __ldg(group_off + group);
     if (c < nchannels) static_cast<Len *>(out.lengths[blockIdx.z])[static_cast<int64_t>(row) * nchannels + c] = static_cast<Len>(len);
+    len = min(len, static_cast<int>(stride));  // a longer stream was truncated and reported by the encoder
     const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
-    place[tid] = make_int2(excl, len);
-    __syncthreads();
-    uint8_t *dst0 = out.bytes[blockIdx.z] + at;
-    constexpr int kLanes = 8;
-    const int part = tid % kLanes;
-    for (int s = tid / kLanes; s < kGroup; s += kGroup / kLanes) {
-        const int2 q = place[s];
-        const int n = q.y;
-        const uint8_t *src = scratch + (slot0 + s) * stride;  // 4-byte aligned
-        uint8_t *dst = dst0 + q.x;
-        const int head = min(n, static_cast<int>(-reinterpret_cast<uintptr_t>(dst) & 3u));
-        const int words = (n - head) >> 2, tail = (n - head) & 3;
-        const uint32_t *src4 = reinterpret_cast<const uint32_t *>(src);
-        uint32_t *dst4 = reinterpret_cast<uint32_t *>(dst + head);
-        const uint32_t sh = static_cast<uint32_t>(head & 3) * 8u;
-        for (int k = part; k < words; k += kLanes) {
-            const int w = (head + 4 * k) >> 2;
-            const uint32_t lo = __ldg(src4 + w), hi = sh ? __ldg(src4 + w + 1) : 0u;
-            dst4[k] = __funnelshift_r(lo, hi, sh);
+    const int first = __shfl_sync(0xFFFFFFFFu, excl, 0);
+    const int total = __shfl_sync(0xFFFFFFFFu, excl + len, 31) - first;
+    uint8_t *dst = out.bytes[blockIdx.z] + at + first;
+    const uint32_t *src = INTERLEAVED ? scratch_word(const_cast<uint8_t *>(scratch), stride, group, tid)
+                                      : reinterpret_cast<const uint32_t *>(scratch + slot * stride);
+    constexpr int kStep = INTERLEAVED ? 32 : 1;
+    const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 15u);
+    const int nw = (len + 3) >> 2;
+    if (mis + total > kGatherWords * 4) {
+        uint8_t *d = dst + (excl - first);
+        for (int k = 0; k < len; ++k) d[k] = static_cast<uint8_t>(__ldg(src + (k >> 2) * kStep) >> (8 * (k & 3)));
+        return;
+    }
+    uint32_t *st = reinterpret_cast<uint32_t *>(stage[warp]);
+    const int units = (mis + total + 15) >> 4;
+    for (int i = lane; i < units; i += 32) stage[warp][i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    const int o = mis + excl - first, w = o >> 2;
+    const uint32_t sh = static_cast<uint32_t>(o & 3) * 8u;
+    const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
+    constexpr int kAhead = 8;  // loads in flight
+    uint32_t prev = 0u;
+    for (int k0 = 0; k0 < most; k0 += kAhead) {
+        uint32_t x[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) x[j] = k0 + j < nw ? __ldg(src + (k0 + j) * kStep) : 0u;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const int k = k0 + j;
+            if (k < nw) {
+                const uint32_t v = __funnelshift_l(prev, x[j], sh);
+                if (k == 0 || k == nw - 1) atomicOr(st + w + k, v);
+                else st[w + k] = v;
+                prev = x[j];
+            }
         }
-        // the bytes before the first and after the last whole word
-        const int e = part < 4 ? part : n - tail + part - 4;
-        if (part < 4 ? part < head : part - 4 < tail) dst[e] = __ldg(src + e);
+    }
+    // what the shift pushed past the last word; a stream's bytes past its end are zero
+    const uint32_t over = __funnelshift_l(prev, 0u, sh);
+    if (over) atomicOr(st + w + nw, over);
+    __syncwarp();
+    uint4 *d16 = reinterpret_cast<uint4 *>(dst - mis);
+    for (int i = lane; i < units; i += 32) {
+        if (i * 16 >= mis && i * 16 + 16 <= mis + total) {
+            d16[i] = stage[warp][i];
+        } else {
+            const uint8_t *b = reinterpret_cast<const uint8_t *>(stage[warp]);
+            for (int k = max(i * 16, mis); k < min(i * 16 + 16, mis + total); ++k) (dst - mis)[k] = b[k];
+        }
     }
 }
 
@@ -600,7 +692,7 @@ Sizes sizes_of(int nlayers, int ntokens, int nheads, int head_size) {
         return here;
     };
     z.sym = take(streams * z.words * 4);
-    z.scratch = take(z.nsub * streams * z.stride);
+    z.scratch = take(z.nsub * groups * kGroup * z.stride);
     z.lengths = take(z.nsub * streams * 4);
     z.group_off = take(z.nsub * groups * 8);
     z.sub_bytes = take(z.nsub * 8);
@@ -678,16 +770,24 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
         return check_launch();
     }
     const KvView v{static_cast<const uint16_t *>(b.kv), b.s_layer, b.s_kv, b.s_token, b.s_head,
-                   b.nlayers, b.ntokens, b.nheads, b.head_size};
+                   b.nlayers, b.ntokens, b.nheads, b.head_size,
+                   0xFFFFFFFFu / static_cast<uint32_t>(b.head_size) + 1u};
     uint32_t *sym4 = reinterpret_cast<uint32_t *>(ws + z.sym);
     const dim3 qgrid(static_cast<unsigned>(z.words), z.nrows);
     const int qthreads = (z.nchannels / 8 + 31) / 32 * 32;
     uint32_t *zeroed = reinterpret_cast<uint32_t *>(status);
     uint16_t *sk = static_cast<uint16_t *>(b.scales_k), *sv = static_cast<uint16_t *>(b.scales_v);
-    if (b.dtype == CG_F16)
-        quantize_tokens_kernel<CG_F16><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, z.nsub + 2);
-    else
-        quantize_tokens_kernel<CG_BF16><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, z.nsub + 2);
+#define CG_LAUNCH_QT(DT, THREADS, BLOCKS)                                                                    \
+    quantize_tokens_kernel<DT, THREADS, BLOCKS><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, \
+                                                                            z.nsub + 2)
+    if (b.dtype == CG_F16) {
+        if (qthreads <= 512) CG_LAUNCH_QT(CG_F16, 512, 3);
+        else CG_LAUNCH_QT(CG_F16, 1024, 1);
+    } else {
+        if (qthreads <= 512) CG_LAUNCH_QT(CG_BF16, 512, 3);
+        else CG_LAUNCH_QT(CG_BF16, 1024, 1);
+    }
+#undef CG_LAUNCH_QT
     if (int rc = check_launch()) return rc;
     StoreParams p;
     p.sym4 = sym4;
@@ -752,9 +852,13 @@ int launch_gather(const cg_encode_kv_job &b, const Sizes &z, uint8_t *const *byt
             t.bytes[k] = bytes[s0 + k];
             t.lengths[k] = lengths[s0 + k];
         }
-        gather_kernel<Len><<<dim3(z.nslab, z.nrows, n), kGroup, 0, st>>>(
-            ws + z.scratch, z.stride, reinterpret_cast<const int32_t *>(ws + z.lengths),
-            reinterpret_cast<const int64_t *>(ws + z.group_off), z.nchannels, s0, t);
+        const dim3 grid(z.nslab, z.nrows, n);
+        const int32_t *lens = reinterpret_cast<const int32_t *>(ws + z.lengths);
+        const int64_t *goff = reinterpret_cast<const int64_t *>(ws + z.group_off);
+        if (fused_ok(b))  // which of the two encoders wrote the scratch
+            gather_kernel<Len, true><<<grid, kGroup, 0, st>>>(ws + z.scratch, z.stride, lens, goff, z.nchannels, s0, t);
+        else
+            gather_kernel<Len, false><<<grid, kGroup, 0, st>>>(ws + z.scratch, z.stride, lens, goff, z.nchannels, s0, t);
         if (int rc = check_launch()) return rc;
     }
     return CG_OK;
