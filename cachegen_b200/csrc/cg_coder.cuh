@@ -457,16 +457,20 @@ CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *strea
 // so that the store is not a per-lane branch.
 //
 // The bits are those of the interval's lower end as one long binary fraction, so a later range update can
-// still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above them (a
-// word leaves nothing behind it) and is added to the stored words when the next word goes out; that
-// takes a run of ones from there to the last stored word, which real tables about never give.
+// still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above
+// them (a word leaves nothing behind it) and goes on to the word before when the next word leaves.  That word is
+// held back in a register until then: the run of ones that lets a carry through reaches the accumulator's end
+// for one word in seven (symbols of 2.5 bits), but past the held word about never.
 // STEP: words between consecutive words of the row (32: the rows of a warp's streams interleaved, so that
-// they take no more cache lines than they have data for and are read back coalesced).
-template <int STEP>
+// they take no more cache lines than they have data for and are read back coalesced).  BOUNDED: the row may be
+// too short for the stream; otherwise it holds CG_STREAM_CAPACITY bytes, which a strictly increasing table
+// never exceeds, and the word in front of its first may be overwritten.
+template <int STEP, bool BOUNDED = true>
 struct BitSinkT {
     uint32_t *row;    // 4-byte aligned scratch row of this stream
     uint32_t cap_w;   // words that fit in the row
-    uint32_t nwords;  // words produced so far (may exceed cap_w: then nothing more is stored)
+    uint32_t nwords;  // words produced so far, the held one included (may exceed cap_w: then nothing more is stored)
+    uint32_t hold;    // the last of them, not yet in the row
     uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo), and a carry above them
     uint32_t nacc;            // number of bits pending, < 63
 
@@ -475,39 +479,58 @@ struct BitSinkT {
         row = reinterpret_cast<uint32_t *>(p);
         cap_w = static_cast<uint32_t>(nbytes >> 2);
         nwords = 0;
+        hold = 0;
         acc_hi = 0;
         acc_lo = 0;
         nacc = 0;
     }
-    // adds one to the number that the stored words form
+    // adds one to the number that the words in the row form
     CG_HD void carry_into_row() {
-        if (nwords > cap_w) return;  // the words before are not in the row: reported as an overflow
-        for (uint32_t i = nwords; i > 0u;) {
+        if (BOUNDED && nwords > cap_w) return;  // the words before are not in the row: reported as an overflow
+        for (uint32_t i = nwords; i > 1u;) {
             --i;
-            const uint32_t v = cg_bswap32(row[i * STEP]) + 1u;
-            row[i * STEP] = cg_bswap32(v);
+            const uint32_t v = cg_bswap32(row[(i - 1u) * STEP]) + 1u;
+            row[(i - 1u) * STEP] = cg_bswap32(v);
             if (v) return;
         }
     }
-    // moves the oldest 32 bits out; needs 32 <= nacc < 63
-    CG_HD void store_word() {
-        nacc -= 32u;
-        const uint32_t w = cg_fshr_clamp(acc_lo, acc_hi, nacc);  // the low word of (hi:lo) >> nacc
-        if (cg_fshr_clamp(acc_hi, 0u, nacc)) carry_into_row();
-        acc_hi = 0u;
-        acc_lo &= ~cg_shl(0xFFFFFFFFu, nacc);
-        if (nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
-        nwords++;
+    // adds a carry (0 or 1) to the held word and puts it in the row
+    CG_HD void store_held(uint32_t carry) {
+        hold += carry;
+        if (hold < carry) carry_into_row();
+        if (!BOUNDED || nwords - 1u < cap_w) row[static_cast<int>(nwords - 1u) * STEP] = cg_bswap32(hold);
+    }
+    // Moves the oldest 32 bits out where there are 32; needs nacc < 63.  Straight-line code: every lane of the
+    // warp runs it whatever it needs.
+    CG_HD void store_word_if_full() {
+        const bool full = nacc >= 32u;
+        const uint32_t left = full ? nacc - 32u : nacc;
+        const uint32_t w = cg_fshr_clamp(acc_lo, acc_hi, left);  // the low word of (hi:lo) >> left
+        const uint32_t carry = full ? cg_fshr_clamp(acc_hi, 0u, left) : 0u;
+        const uint32_t held = hold + carry;
+        if (held < carry) carry_into_row();
+#if defined(__CUDA_ARCH__)
+        const bool stored = full && (!BOUNDED || nwords - 1u < cap_w);
+        asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.global.u32 [%1], %2; }" ::"r"(static_cast<uint32_t>(stored)),
+                     "l"(row + static_cast<int>(nwords - 1u) * STEP), "r"(cg_bswap32(held)) : "memory");
+#else
+        if (full && nwords && (!BOUNDED || nwords - 1u < cap_w)) row[(nwords - 1u) * STEP] = cg_bswap32(held);
+#endif
+        nwords += full ? 1u : 0u;
+        hold = full ? w : hold;
+        acc_hi = full ? 0u : acc_hi;
+        acc_lo = full ? acc_lo & ~cg_shl(0xFFFFFFFFu, left) : acc_lo;
+        nacc = left;
     }
     // zero-fills to a byte boundary; returns the stream length in bytes
     CG_HD uint32_t finish() {
         if (nacc > 62u) nacc = 62u;  // only a table that does not increase gets here
-        if (nacc >= 32u) store_word();
-        if (cg_fshr_clamp(acc_lo, acc_hi, nacc)) carry_into_row();
+        store_word_if_full();
+        if (nwords) store_held(cg_fshr_clamp(acc_lo, acc_hi, nacc));
         const uint32_t bytes = nwords * 4u + ((nacc + 7u) >> 3);
         if (nacc) {
             const uint32_t w = acc_lo << (32u - nacc);
-            if (nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
+            if (!BOUNDED || nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
         }
         return bytes;
     }
@@ -535,8 +558,12 @@ struct EncoderState {
     template <class Sink>
     CG_HD void add_to_low(uint32_t v, Sink &out) {
 #if defined(__CUDA_ARCH__)
-        asm("add.cc.u32 %0, %0, %3; addc.cc.u32 %1, %1, 0; addc.u32 %2, %2, 0;"
-            : "+r"(low), "+r"(out.acc_lo), "+r"(out.acc_hi) : "r"(v));
+        uint32_t l, a, b;
+        asm("add.cc.u32 %0, %3, %6; addc.cc.u32 %1, %4, 0; addc.u32 %2, %5, 0;"
+            : "=&r"(l), "=&r"(a), "=r"(b) : "r"(low), "r"(out.acc_lo), "r"(out.acc_hi), "r"(v));
+        low = l;
+        out.acc_lo = a;
+        out.acc_hi = b;
 #else
         low += v;
         if (low < v && ++out.acc_lo == 0u) ++out.acc_hi;
@@ -553,11 +580,9 @@ struct EncoderState {
         const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + kTableRowBytes);
         uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
         if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (LAST && s == maxsym))) {
-            if (out.nacc >= 32u) out.store_word();
-            if (span32 == 0u) {
-                flo = e0;
-                fhi = e1;
-            }
+            out.store_word_if_full();
+            flo = span32 ? flo : e0;
+            fhi = span32 ? fhi : e1;
             if (LAST && s == maxsym) fhi = span32;
         }
         add_to_low(flo, out);
@@ -575,7 +600,7 @@ struct EncoderState {
     template <class Sink>
     CG_HD uint32_t flush(Sink &out) {
         add_to_low(0x40000000u, out);
-        if (out.nacc >= 32u && out.nacc < 63u) out.store_word();
+        if (out.nacc < 63u) out.store_word_if_full();
         out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, 30u);
         out.acc_lo = cg_fshr_clamp(low, out.acc_lo, 30u);
         out.nacc += 2u;

@@ -277,7 +277,7 @@ struct StoreParams {
     const uint32_t *sym4;
     TableOut out;
     int ntokens, nchannels, lp, nrows, nsub;
-    uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4, 32 lanes] words
+    uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4 + 1, 32 lanes] words
     int64_t stride;
     int32_t *lengths;     // [nsub, nrows * C]
     int64_t *group_off;   // [nsub, nrows * nslab]: byte offset of each 128-channel group inside its sub-chunk
@@ -287,12 +287,13 @@ struct StoreParams {
     int64_t *tail;        // [nsub + 4], see cg_encode_kv_job
 };
 
-// The scratch rows of the 32 streams of a warp lie interleaved: word k of stream `lane` is word 32 k + lane of
-// the warp's 32 * stride bytes.  A stream takes 45 of its 520 bytes on the usual workload: laid out row by
+// The scratch rows of the 32 streams of a warp lie interleaved: word k of stream `lane` is word 32 (k + 1) + lane
+// of the warp's 32 * (stride + 4) bytes.  A stream takes 45 of its 520 bytes on the usual workload: laid out row by
 // row that is a cache line or two for every stream (70 MB of lines a Llama-7B chunk, which the L2 did not
-// keep), interleaved it is as many lines as there is data, and the gather reads them whole.
+// keep), interleaved it is as many lines as there is data, and the gather reads them whole.  One more row in front
+// of the first word's (see BitSinkT).
 __device__ __forceinline__ uint32_t *scratch_word(uint8_t *scratch, int64_t stride, int64_t group, int tid) {
-    return reinterpret_cast<uint32_t *>(scratch + (group * (kGroup / 32) + (tid >> 5)) * 32 * stride) + (tid & 31);
+    return reinterpret_cast<uint32_t *>(scratch + (group * (kGroup / 32) + (tid >> 5)) * 32 * (stride + 4)) + 32 + (tid & 31);
 }
 
 // Exclusive scan of n values in place by one block of kGroup threads; returns the sum.
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     if (active) {
         const int64_t slot = static_cast<int64_t>(sub) * p.nrows * C + g;
         const uint32_t top = static_cast<uint32_t>(p.lp - 2);
-        BitSinkT<32> out;  // see scratch_word
+        BitSinkT<32, false> out;  // see scratch_word
         out.init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x, tid)),
                  p.stride);
         EncoderState enc;
@@ -692,7 +693,7 @@ Sizes sizes_of(int nlayers, int ntokens, int nheads, int head_size) {
         return here;
     };
     z.sym = take(streams * z.words * 4);
-    z.scratch = take(z.nsub * groups * kGroup * z.stride);
+    z.scratch = take(z.nsub * groups * kGroup * (z.stride + 4));
     z.lengths = take(z.nsub * streams * 4);
     z.group_off = take(z.nsub * groups * 8);
     z.sub_bytes = take(z.nsub * 8);
