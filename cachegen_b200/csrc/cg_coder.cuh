@@ -570,20 +570,24 @@ struct EncoderState {
 #endif
     }
     // One symbol s of one stream per lane (enc_new.cu:257-295), s <= maxsym.  lanes: the warp's lanes that
-    // encode together (same token count).  ONE warp vote a symbol covers what is rare: a full word in the
-    // accumulator (every lane that has one stores it as soon as one lane is near the high-water mark), the
-    // full 2^32 range (a stream's first symbol; later only if a shift lands on it exactly) and the table's last
-    // symbol, whose upper bound is the range's end (LAST = false: s < maxsym is known).
-    template <bool LAST = true, class Sink>
+    // encode together (same token count).
+    template <class Sink>
     CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, Sink &out, uint32_t lanes) {
-        const uint32_t a = col + s * kTableRowBytes;
-        const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + kTableRowBytes);
+        step_at<kTableRowBytes>(sm, col + s * kTableRowBytes, s == maxsym, out, lanes);
+    }
+    // The same by the address a of the symbol's table entry, the next one ROW bytes further.  ONE warp vote a
+    // symbol covers what is rare: a full word in the accumulator (every lane that has one stores it as soon as
+    // one lane is near the high-water mark), the full 2^32 range (a stream's first symbol; later only if a shift
+    // lands on it exactly) and the table's last symbol, whose upper bound is the range's end.
+    template <int ROW, class Sink>
+    CG_HD void step_at(Smem sm, uint32_t a, bool last, Sink &out, uint32_t lanes) {
+        const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + ROW);
         uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
-        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | (LAST && s == maxsym))) {
+        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | last)) {
             out.store_word_if_full();
             flo = span32 ? flo : e0;
             fhi = span32 ? fhi : e1;
-            if (LAST && s == maxsym) fhi = span32;
+            if (last) fhi = span32;
         }
         add_to_low(flo, out);
         span32 = fhi - flo;

@@ -56,17 +56,17 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 // of the decoder takes for "above the target", or with REPEAT_LAST copies of the last entry (see
 // decode_streams in cg_coder.cuh).
 constexpr uint32_t kTablePadding = 0xFFFFFFFFu;
-template <bool REPEAT_LAST = false>
+template <bool REPEAT_LAST = false, int STRIDE = kGroup>
 __device__ __forceinline__ void stage_table_column(uint32_t *tab, const int16_t *cdf_row, int lp,
                                                    int rows, int tid) {
     const int n = lp - 1 < rows ? lp - 1 : rows;
     uint32_t pad = kTablePadding, e = 0u;
     for (int m = 0; m < n; ++m) {
         e = static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))) << 16;
-        tab[m * kGroup + tid] = e;
+        tab[m * STRIDE + tid] = e;
     }
     if (REPEAT_LAST) pad = e;
-    for (int m = n; m < rows; ++m) tab[m * kGroup + tid] = pad;
+    for (int m = n; m < rows; ++m) tab[m * STRIDE + tid] = pad;
 }
 
 // The same column from the byte counts of the non-centre symbols (CG_TABLES_COUNTS):

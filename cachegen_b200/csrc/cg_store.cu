@@ -134,9 +134,10 @@ struct TableOut {
     uint32_t *group_nz;           // non-zero byte counts per (row, group), or nullptr
 };
 
-// The counts of one channel, hist[m * kGroup] for symbols m < lp - 1, become its table in place (entries
+// The counts of one channel, hist[m * STRIDE] for symbols m < lp - 1, become its table in place (entries
 // cdf << 16, one row more than there are symbols) and, as 16-bit entries, in stage[0 .. lp-1]
 // (normalize_cdf_value, cal_cdf.cu:11-15,40-49).  Returns the number of non-zero non-centre counts.
+template <int STRIDE>
 __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage, int lp, uint32_t ntokens, int cq,
                                                 uint8_t *counts, int64_t counts_stride, bool *overflow) {
     const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(lp - 1);
@@ -149,7 +150,7 @@ __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage,
     int nz = 0, m = 0;
     for (; m < lp; ++m) {
         if (cum == ntokens) break;  // every symbol is below m: the entries from here on only count up
-        const uint32_t n = hist[m * kGroup];
+        const uint32_t n = hist[m * STRIDE];
         const uint32_t prod = scale * (cum & 0xFFFFu);
         uint32_t q;
         if (pow2) {
@@ -159,7 +160,7 @@ __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage,
             if (prod - q * total >= total) ++q;
         }
         const uint32_t e = (q + static_cast<uint32_t>(m)) & 0xFFFFu;
-        hist[m * kGroup] = e << 16;
+        hist[m * STRIDE] = e << 16;
         stage[m] = static_cast<uint16_t>(e);
         cum += n;
         if (counts && m < lp - 1) {
@@ -181,7 +182,7 @@ __device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage,
             }
     for (; m < lp; ++m) {
         const uint32_t e = (scale + static_cast<uint32_t>(m)) & 0xFFFFu;
-        hist[m * kGroup] = e << 16;
+        hist[m * STRIDE] = e << 16;
         stage[m] = static_cast<uint16_t>(e);
     }
     return nz;
@@ -198,13 +199,15 @@ __device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst
     }
 }
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return __byte_perm(w, 0u, 0x4440u + k); }
+// Shared-memory columns of a warp's 32 channels: entry m of lane l at word 32 m + l.  With rows of 128 bytes the
+// address of the entry that byte k of a word of symbols names is one dot product: the byte times 128, plus
+// the column.
+constexpr int kWarpRow = 128;
+__device__ __forceinline__ uint32_t entry_of(uint32_t col, uint32_t w, int k) {
+    return __dp4a(w, static_cast<uint32_t>(kWarpRow) << (8 * k), col);
+}
 __device__ __forceinline__ void count_symbol(uint32_t addr) {
     asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
-}
-__device__ __forceinline__ void count_word(uint32_t col, uint32_t w) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) count_symbol(col + byte_of(w, k) * kRowBytes);
 }
 
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint
     __syncthreads();
     const int words = (ntokens + 3) / 4, whole = ntokens / 4;
     if (c < nchannels) {
-        const uint32_t col = smem_addr(hist + cl);
+        const uint32_t col = smem_addr(hist + (cl >> 5) * 32 * lp + (cl & 31));
         const uint32_t *p = sym4 + static_cast<int64_t>(row) * words * nchannels + c;
         constexpr int kAhead = 8;  // loads in flight
         for (int i0 = part; i0 < words; i0 += kParts * kAhead) {
@@ -239,9 +242,10 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint
                 const int i = i0 + j * kParts;
                 if (w[j] & 0x80808080u) w[j] = 0u;  // reported by the coder
                 if (i < whole) {
-                    count_word(col, w[j]);
+                    #pragma unroll
+                    for (int k = 0; k < 4; ++k) count_symbol(entry_of(col, w[j], k));
                 } else if (i < words) {
-                    for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w[j] >> (8 * k)) & 0xFFu) * kRowBytes);
+                    for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w[j] >> (8 * k)) & 0xFFu) * kWarpRow);
                 }
             }
         }
@@ -252,7 +256,7 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint
         int nz = 0;
         if (c < nchannels) {
             const int cq = static_cast<int>(half_range(__ldg(out.bins + row)));
-            nz = counts_to_column(hist + cl, stage + cl * lp, lp, ntokens, cq,
+            nz = counts_to_column<32>(hist + (cl >> 5) * 32 * lp + (cl & 31), stage + cl * lp, lp, ntokens, cq,
                                   out.counts ? out.counts + __ldg(out.table_row_off + row) + c : nullptr, nchannels, &overflow);
         }
         if (out.group_nz) {
@@ -356,7 +360,8 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     const int t0 = sub * kSubTokens, n = min(kSubTokens, p.ntokens - t0);
     const int64_t C = p.nchannels;
     const int64_t g = row * C + c;
-    const uint32_t col = smem_addr(tab + tid);
+    uint32_t *column = tab + warp * 32 * p.lp + lane;
+    const uint32_t col = smem_addr(column);
     const uint32_t *sp = p.sym4 + (static_cast<int64_t>(row) * ((p.ntokens + 3) / 4) + t0 / 4) * C + c;
     uint32_t bad = 0;
     int nbytes = 0, nz = 0;
@@ -365,7 +370,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
         uint16_t *stage = reinterpret_cast<uint16_t *>(tab + p.lp * kGroup);
         bool overflow = false;
         if (active) {
-            for (int m = 0; m < p.lp; ++m) tab[m * kGroup + tid] = 0u;
+            for (int m = 0; m < p.lp; ++m) column[m * 32] = 0u;
             const uint32_t *q = sp;
             constexpr int kAhead = 2 * kWordsAhead;
             uint32_t w[kAhead], next[kAhead];
@@ -379,7 +384,8 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
 #pragma unroll
                 for (int k = 0; k < kAhead; ++k) {
                     if (w[k] & 0x80808080u) w[k] = 0u;
-                    count_word(col, w[k]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) count_symbol(entry_of(col, w[k], j));
                     w[k] = next[k];
                 }
             }
@@ -388,10 +394,10 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
                 if (w[k] & 0x80808080u) w[k] = 0u;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (i + 4 * k + j < n) count_symbol(col + byte_of(w[k], j) * kRowBytes);
+                    if (i + 4 * k + j < n) count_symbol(entry_of(col, w[k], j));
             }
             const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
-            nz = counts_to_column(tab + tid, stage + tid * p.lp, p.lp, n, cq,
+            nz = counts_to_column<32>(column, stage + tid * p.lp, p.lp, n, cq,
                                   p.out.counts ? p.out.counts + __ldg(p.out.table_row_off + row) + c : nullptr, C, &overflow);
         }
         if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
@@ -402,7 +408,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
             copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp,
                         nch * p.lp, lane);
     } else if (active) {
-        stage_table_column(tab, p.out.cdf + g * p.lp, p.lp, p.lp, tid);
+        stage_table_column<false, 32>(column, p.out.cdf + g * p.lp, p.lp, p.lp, 0);
     }
 
     if (active) {
@@ -432,7 +438,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
             for (int k = 0; k < kWordsAhead; ++k) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    enc.step<false>(Smem{}, col, byte_of(w[k], j), top, out, lanes);
+                    enc.step_at<kWarpRow>(Smem{}, entry_of(col, w[k], j), false, out, lanes);
             }
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) w[k] = next[k];
@@ -443,7 +449,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
                 bad = 1u;
                 s = 0u;
             }
-            enc.step<false>(Smem{}, col, s, top, out, lanes);
+            enc.step_at<kWarpRow>(Smem{}, col + s * kWarpRow, false, out, lanes);
             w[0] >>= 8;
             if ((i & 3) == 3) {
 #pragma unroll
