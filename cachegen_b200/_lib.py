@@ -64,7 +64,13 @@ class FlatLayout(ctypes.Structure):
                 [(n, ctypes.c_int32) for n in ("table_kind", "reserved")])
 
 
+class HostSegment(ctypes.Structure):
+    """cg_host_segment"""
+    _fields_ = [("host", ctypes.c_void_p), ("device", ctypes.c_void_p), ("bytes", ctypes.c_int64)]
+
+
 EXPORTS = [
+    "cg_host_upload", "cg_host_download", "cg_decode_kv",
     "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_wait", "cg_encode_kv_gather", "cg_encode_kv_flat",
     "cg_version", "cg_status_string", "cg_last_cuda_error", "cg_workspace_bytes",
     "cg_calculate_cdf", "cg_encode_padded", "cg_decode_padded", "cg_decode_prefsum", "cg_decode_prefsum_warp",
@@ -120,6 +126,9 @@ def lib():
     L.cg_encode_kv_wait.argtypes = [job, p]
     L.cg_encode_kv_gather.argtypes = [job, ctypes.POINTER(p), ctypes.POINTER(p), p]
     L.cg_encode_kv_flat.argtypes = [job, ctypes.POINTER(FlatLayout), p]
+    L.cg_decode_kv.argtypes = [ctypes.POINTER(DecodeJob), i, i, i, i, i, p, i, p, i, i, i64, i64, i64, i64, p, p]
+    L.cg_host_upload.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, p]
+    L.cg_host_download.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, i, p]
     for name in EXPORTS:
         fn = getattr(L, name)
         if name not in ("cg_version", "cg_status_string", "cg_last_cuda_error"):

@@ -119,8 +119,61 @@ struct FusedDecodeParams {
     const float *bins;
     int64_t o_layer, o_kv, o_token, o_head;
     int32_t *status;
+    int after;  // see DecodeAfter
     cg_decode_job jobs[CG_MAX_DECODE_JOBS];
 };
+
+// What a decode launch follows, when it is launched so that its blocks may start before the launch in front of it
+// has ended (programmatic dependent launch).  kAfterOffsets: the group offsets it needs; everything up to
+// reading them runs beside that launch.  kAfterBatch: another batch of the same call, on which it does not depend,
+// so that its blocks fill what that one's last wave leaves idle; it only must not end first.
+enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---- table staging by the block --------------------------------------------------------------------------
+// The int16 tables of a block's 128 channels are one contiguous run.  Read channel by channel they are 2-byte
+// loads 66 bytes apart, 66 of them one after the other in a thread; here the run is copied to the upper part
+// of the table area with 16-byte asynchronous copies and spread into columns from there: the rows below it at
+// once, the rest from registers once every thread has read its part.
+__device__ __forceinline__ void copy_run_async(void *smem, const void *global, int bytes, int tid, int nthreads) {
+    const uint32_t d = smem_addr(smem);
+    for (int i = tid * 16; i < bytes; i += nthreads * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + i), "l"(static_cast<const char *>(global) + i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+constexpr int kMaxStagedLp = 33;  // longer tables would need more registers than the decode loop has
+__device__ __forceinline__ int staged_run_offset(int lp, int rows) { return rows * kRowBytes - lp * kGroup * 2; }
+// Thread t's channels are 2t and 2t + 1, in columns t and t + 64.  rows: the columns' rows, filled up with the last
+// entry.  Called by all threads.
+__device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int tid) {
+    constexpr int kHold = (kMaxStagedLp + 1) / 2;
+    const int off = staged_run_offset(lp, rows), below = off / kRowBytes, n = lp - 1;
+    const uint16_t *run = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(tab) + off) + 2 * tid * lp;
+    uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
+    const int direct = min(n, below);
+    for (int m = 0; m < direct; ++m) {
+        c0[m * kGroup] = static_cast<uint32_t>(run[m]) << 16;
+        c1[m * kGroup] = static_cast<uint32_t>(run[lp + m]) << 16;
+    }
+    uint32_t hold[kHold];
+#pragma unroll
+    for (int k = 0; k < kHold; ++k)
+        hold[k] = direct + k < n ? static_cast<uint32_t>(run[direct + k]) | static_cast<uint32_t>(run[lp + direct + k]) << 16 : 0u;
+    const uint32_t last0 = static_cast<uint32_t>(run[n - 1]) << 16, last1 = static_cast<uint32_t>(run[lp + n - 1]) << 16;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kHold; ++k)
+        if (direct + k < n) {
+            c0[(direct + k) * kGroup] = hold[k] << 16;
+            c1[(direct + k) * kGroup] = hold[k] & 0xFFFF0000u;
+        }
+    for (int m = n; m < rows; ++m) {
+        c0[m * kGroup] = last0;
+        c1[m * kGroup] = last1;
+    }
+}
 
 template <int LEVELS, int SCALE_DT, int OUT_DT>
 __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_constant__ FusedDecodeParams p) {
@@ -148,6 +201,8 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
     if (len < 0) { len = 0; bad = true; }
     if (len > (1 << 20)) { len = 1 << 20; bad = true; }
     const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
+    wait_for_launch_before();
+    let_next_launch_start();
     int64_t start = __ldg(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
     if (start < 0) { start = 0; len = 0; bad = true; }
     if (start > job.nbytes) { start = job.nbytes; bad = true; }
@@ -274,7 +329,16 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     const int layer = row % p.nlayers, kv = row / p.nlayers;
     const int64_t g = static_cast<int64_t>(row) * p.nchannels + c0;
 
-    // stream offsets: group base + exclusive scan of this block's lengths (cachegen_decoder.py:70)
+    const int rows = table_rows(p.lp, full_levels < 2 ? 2 : full_levels);  // the register level reads entries 1..3
+    // whole groups of 16-byte aligned tables are staged by the block
+    const bool run_staged = NS == 2 && job.table_kind == CG_TABLES_CDF && p.lp <= kMaxStagedLp && (p.nchannels & 7) == 0 &&
+                            (reinterpret_cast<uintptr_t>(job.tables) & 15) == 0 && static_cast<int>((blockIdx.x + 1) * kGroup) <= p.nchannels;
+    if (run_staged)
+        copy_run_async(reinterpret_cast<char *>(smem) + staged_run_offset(p.lp, rows + 1),
+                       static_cast<const int16_t *>(job.tables) + (static_cast<int64_t>(row) * p.nchannels + blockIdx.x * kGroup) * p.lp,
+                       p.lp * kGroup * 2, tid, kThreads);
+
+    // stream lengths
     int len[NS];
     bool bad = false;
     int len_sum = 0;
@@ -289,18 +353,6 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
         if (len[i] > (1 << 20)) { len[i] = 1 << 20; bad = true; }
         len_sum += len[i];
     }
-    const int excl = block_exclusive_scan<kWarps>(len_sum, warp_sums, tid, nullptr);
-    int64_t start[NS];
-    start[0] = __ldg(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
-#pragma unroll
-    for (int i = 1; i < NS; ++i) start[i] = start[i - 1] + len[i - 1];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {
-        if (start[i] < 0) { start[i] = 0; len[i] = 0; bad = true; }
-        if (start[i] > job.nbytes) { start[i] = job.nbytes; bad = true; }
-        if (start[i] + len[i] > job.nbytes) { len[i] = static_cast<int>(job.nbytes - start[i]); bad = true; }
-    }
-    if (bad && active && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
 
     // per-token scales of this row and the row's (s - Cq) / Cq table (cachegen_decoder.py:30-32)
     const uint16_t *sc = static_cast<const uint16_t *>(kv ? job.scales_v : job.scales_k) +
@@ -326,11 +378,14 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
         }
     }
     const int cq = cqf >= 0.0f && cqf < 64.0f ? static_cast<int>(cqf) : 64;
-    const int rows = table_rows(p.lp, full_levels < 2 ? 2 : full_levels);  // the register levels read entries 1..3
     uint32_t *tabs[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i) tabs[i] = smem + tid + i * kThreads;
-    if (job.table_kind == CG_TABLES_SPARSE) {  // the whole block: the counts are found by a scan of the masks
+    if (run_staged) {
+        wait_copies();
+        __syncthreads();
+        spread_run(smem, p.lp, rows + 1, tid);
+    } else if (job.table_kind == CG_TABLES_SPARSE) {  // the whole block: the counts are found by a scan of the masks
         const int nrows = 2 * p.nlayers;
         const uint8_t *base = static_cast<const uint8_t *>(job.tables);
         const int64_t off_masks = (static_cast<int64_t>(nrows) * p.nslab + 1) * 4 + 15 & ~int64_t{15};
@@ -351,7 +406,6 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
             nset[i] = __popc(mask[i]);
             nset_sum += nset[i];
         }
-        __syncthreads();  // warp_sums is free again
         const int before = block_exclusive_scan<kWarps>(nset_sum, warp_sums, tid, nullptr);
         int64_t at = off_counts +
                      __ldg(reinterpret_cast<const uint32_t *>(base) + static_cast<int64_t>(row) * p.nslab + blockIdx.x) +
@@ -380,8 +434,27 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
             }
         }
     }
+    __syncthreads();  // warp_sums is free again
+    // stream offsets: group base + exclusive scan of this block's lengths (cachegen_decoder.py:70)
+    const int excl = block_exclusive_scan<kWarps>(len_sum, warp_sums, tid, nullptr);
+    if (p.after == kAfterOffsets) wait_for_launch_before();
+    let_next_launch_start();
+    int64_t start[NS];
+    start[0] = __ldg(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
+#pragma unroll
+    for (int i = 1; i < NS; ++i) start[i] = start[i - 1] + len[i - 1];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        if (start[i] < 0) { start[i] = 0; len[i] = 0; bad = true; }
+        if (start[i] > job.nbytes) { start[i] = job.nbytes; bad = true; }
+        if (start[i] + len[i] > job.nbytes) { len[i] = static_cast<int>(job.nbytes - start[i]); bad = true; }
+    }
+    if (bad && active && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
     __syncthreads();
-    if (!active) return;
+    if (!active) {
+        if (p.after == kAfterBatch) wait_for_launch_before();
+        return;
+    }
 
     const int h = c0 / p.head_size, d = c0 - h * p.head_size;
     uint16_t *o = static_cast<uint16_t *>(job.out) + layer * p.o_layer + kv * p.o_kv + h * p.o_head + d;
@@ -443,6 +516,7 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     case 5: decode_streams<5, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
     default: decode_streams<6, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
     }
+    if (p.after == kAfterBatch) wait_for_launch_before();
 }
 
 // ---- launch helpers -------------------------------------------------------------------------------------
@@ -472,24 +546,36 @@ static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) 
     return check_launch();
 }
 
+// early: the blocks may start before the launch in front has ended (see DecodeAfter)
+template <class... Args>
+static int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t st, Args... args) {
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    return e == cudaSuccess ? CG_OK : set_cuda_error(e);
+}
+
 template <int SCALE_DT, int OUT_DT>
-static int launch_fused(const FusedDecodeParams &p, cudaStream_t st) {
+static int launch_fused(const FusedDecodeParams &p, bool early, cudaStream_t st) {
     const int need = search_levels(p.lp);
-    const dim3 grid(p.nslab, 2 * p.nlayers, p.njobs), block(kGroup);
-#define CG_LAUNCH_FUSED(L)                                                                               \
-    do {                                                                                                  \
-        const size_t smem = table_bytes(p.lp, L);                                                         \
-        if (smem > 48 * 1024)                                                                             \
-            cudaFuncSetAttribute(decode_dequant_kernel<L, SCALE_DT, OUT_DT>,                          \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));    \
-        decode_dequant_kernel<L, SCALE_DT, OUT_DT><<<grid, block, smem, st>>>(p);                     \
-    } while (0)
+    const dim3 grid(p.nslab, 2 * p.nlayers, p.njobs);
+#define CG_LAUNCH_FUSED(L) \
+    return launch(decode_dequant_kernel<L, SCALE_DT, OUT_DT>, grid, kGroup, table_bytes(p.lp, L), early, st, p)
     if (need <= 3) CG_LAUNCH_FUSED(3);
-    else if (need == 4) CG_LAUNCH_FUSED(4);
-    else if (need == 5) CG_LAUNCH_FUSED(5);
-    else CG_LAUNCH_FUSED(6);
+    if (need == 4) CG_LAUNCH_FUSED(4);
+    if (need == 5) CG_LAUNCH_FUSED(5);
+    CG_LAUNCH_FUSED(6);
 #undef CG_LAUNCH_FUSED
-    return check_launch();
 }
 
 // The NS-channels-per-thread kernel needs the NS channels of a thread in one head and aligned packed stores.
@@ -501,14 +587,118 @@ static bool multi_layout_ok(const FusedDecodeParams &p, int ns) {
 }
 
 template <int NS, int OUT_DT, bool DELTA>
-static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, cudaStream_t st) {
+static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool early, cudaStream_t st) {
     const int full = search_levels(p.lp);
-    const size_t smem = table_bytes(p.lp, full < 2 ? 2 : full);
-    const dim3 grid(p.nslab, 2 * p.nlayers, p.njobs), block(kGroup / NS);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(decode_dequant_multi_kernel<NS, OUT_DT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-    decode_dequant_multi_kernel<NS, OUT_DT, DELTA><<<grid, block, smem, st>>>(p, scale_dt, full);
+    return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA>, dim3(p.nslab, 2 * p.nlayers, p.njobs), kGroup / NS,
+                  table_bytes(p.lp, full < 2 ? 2 : full), early, st, p, scale_dt, full);
+}
+
+// ---- group offsets ------------------------------------------------------------------------------------------
+// One cluster of eight blocks per job: every block sums the lengths of an eighth of the 128-channel groups and
+// scans its sums, then adds the totals of the blocks before it, which it reads in their shared memory.  One
+// launch where a sum kernel and a scan kernel were two (5 us of 23 for a 37-token chunk), and nothing to zero.
+struct OffsetJobs {
+    const void *lengths[CG_MAX_DECODE_JOBS];
+    int64_t *group_off[CG_MAX_DECODE_JOBS];
+    int64_t expect[CG_MAX_DECODE_JOBS];
+    int32_t kind[CG_MAX_DECODE_JOBS];
+};
+constexpr int kOffsetBlocks = 8, kOffsetThreads = 512, kMaxOffsetGroups = 8 * 8192;
+
+__device__ __forceinline__ int clamped_length(int v, bool *bad) {
+    if (v < 0) { v = 0; *bad = true; }
+    if (v > (1 << 20)) { v = 1 << 20; *bad = true; }
+    return v;
+}
+
+__global__ void __cluster_dims__(kOffsetBlocks, 1, 1) __launch_bounds__(kOffsetThreads)
+group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nchannels, int nslab, int32_t *status) {
+    extern __shared__ int sums[];  // the groups of this block
+    __shared__ int64_t warp_sums[kOffsetThreads / 32];
+    __shared__ int64_t block_total;
+    let_next_launch_start();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int j = blockIdx.x / kOffsetBlocks, rank = blockIdx.x % kOffsetBlocks;
+    const int ngroups = nrows * nslab, per = (ngroups + kOffsetBlocks - 1) / kOffsetBlocks;
+    const int first = min(ngroups, rank * per), count = min(ngroups, first + per) - first;
+    const bool u16 = jobs.kind[j] == CG_LENGTHS_U16;
+    const void *lengths = jobs.lengths[j];
+    // four lengths a load where the rows allow it
+    const bool vec = nchannels % kGroup == 0 && (reinterpret_cast<uintptr_t>(lengths) & (u16 ? 7 : 15)) == 0;
+    bool bad = false;
+    for (int k = warp; k < count; k += kOffsetThreads / 32) {
+        const int gid = first + k;
+        int s = 0;
+        if (vec) {
+            if (u16) {
+                const ushort4 q = __ldg(static_cast<const ushort4 *>(lengths) + static_cast<int64_t>(gid) * 32 + lane);
+                s = q.x + q.y + q.z + q.w;
+            } else {
+                const int4 q = __ldg(static_cast<const int4 *>(lengths) + static_cast<int64_t>(gid) * 32 + lane);
+                s = clamped_length(q.x, &bad) + clamped_length(q.y, &bad) + clamped_length(q.z, &bad) + clamped_length(q.w, &bad);
+            }
+        } else {
+            const int row = gid / nslab, slab = gid % nslab;
+            for (int c = slab * kGroup + lane; c < min(nchannels, (slab + 1) * kGroup); c += 32) {
+                const int64_t at = static_cast<int64_t>(row) * nchannels + c;
+                s += clamped_length(u16 ? static_cast<int>(__ldg(static_cast<const uint16_t *>(lengths) + at))
+                                        : __ldg(static_cast<const int32_t *>(lengths) + at), &bad);
+            }
+        }
+        s = __reduce_add_sync(0xFFFFFFFFu, s);
+        if (lane == 0) sums[k] = s;
+    }
+    __syncthreads();
+    // exclusive scan: a run of groups per thread
+    const int run = (count + kOffsetThreads - 1) / kOffsetThreads, b = min(count, tid * run), e = min(count, b + run);
+    int64_t local = 0;
+    for (int k = b; k < e; ++k) local += sums[k];
+    int64_t incl = local;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int64_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    int64_t at = incl - local, total = 0;
+#pragma unroll
+    for (int k = 0; k < kOffsetThreads / 32; ++k) {
+        if (k < warp) at += warp_sums[k];
+        total += warp_sums[k];
+    }
+    if (tid == 0) block_total = total;
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    int64_t all = 0;
+#pragma unroll
+    for (int r = 0; r < kOffsetBlocks; ++r) {
+        uint32_t remote;
+        int64_t v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&block_total)), "r"(r));
+        asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(remote));
+        if (r < rank) at += v;
+        all += v;
+    }
+    int64_t *out = jobs.group_off[j] + first;
+    for (int k = b; k < e; ++k) {
+        out[k] = at;
+        at += sums[k];
+    }
+    if (status && (bad || (rank == 0 && tid == 0 && all != jobs.expect[j]))) atomicOr(status, CG_S_BAD_LENGTHS);
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");  // the totals have been read
+}
+
+static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int nchannels, int32_t *status, cudaStream_t st) {
+    OffsetJobs o;
+    for (int j = 0; j < njobs; ++j) {
+        o.lengths[j] = jobs[j].lengths;
+        o.group_off[j] = const_cast<int64_t *>(jobs[j].group_off);
+        o.expect[j] = jobs[j].nbytes;
+        o.kind[j] = jobs[j].length_kind;
+    }
+    const int nslab = (nchannels + kGroup - 1) / kGroup;
+    const size_t smem = static_cast<size_t>((static_cast<int64_t>(nrows) * nslab + kOffsetBlocks - 1) / kOffsetBlocks) * sizeof(int);
+    group_offsets_kernel<<<njobs * kOffsetBlocks, kOffsetThreads, smem, st>>>(o, nrows, nchannels, nslab, status);
     return check_launch();
 }
 
@@ -593,6 +783,7 @@ static int fused_params(const cg_decode_job *jobs_host, int njobs, int nlayers, 
     p.o_token = o_token;
     p.o_head = o_head;
     p.status = status;
+    p.after = kAfterOffsets;
     for (int j = 0; j < njobs; ++j) {
         const cg_decode_job &jb = jobs_host[j];
         if (!jb.tables || !jb.lengths || !jb.group_off || !jb.scales_k || !jb.scales_v || !jb.out ||
@@ -613,19 +804,19 @@ static int fused_params(const cg_decode_job *jobs_host, int njobs, int nlayers, 
     return CG_OK;
 }
 
-static int launch_fused_any(const FusedDecodeParams &p, int scale_dtype, int out_dtype, cudaStream_t st) {
+static int launch_fused_any(const FusedDecodeParams &p, int scale_dtype, int out_dtype, cudaStream_t st, bool early = false) {
     if (p.delta_group > 0) {  // only the two-channels-per-thread kernel knows about anchors
         if (!multi_layout_ok(p, 2)) return CG_E_ALIGN;
-        return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, true>(p, scale_dtype, st)
-                                   : launch_fused_multi<2, CG_BF16, true>(p, scale_dtype, st);
+        return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, true>(p, scale_dtype, early, st)
+                                   : launch_fused_multi<2, CG_BF16, true>(p, scale_dtype, early, st);
     }
     if (multi_layout_ok(p, 2))
-        return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, false>(p, scale_dtype, st)
-                                   : launch_fused_multi<2, CG_BF16, false>(p, scale_dtype, st);
-    if (scale_dtype == CG_F16 && out_dtype == CG_F16) return launch_fused<CG_F16, CG_F16>(p, st);
-    if (scale_dtype == CG_F16 && out_dtype == CG_BF16) return launch_fused<CG_F16, CG_BF16>(p, st);
-    if (scale_dtype == CG_BF16 && out_dtype == CG_F16) return launch_fused<CG_BF16, CG_F16>(p, st);
-    return launch_fused<CG_BF16, CG_BF16>(p, st);
+        return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, false>(p, scale_dtype, early, st)
+                                   : launch_fused_multi<2, CG_BF16, false>(p, scale_dtype, early, st);
+    if (scale_dtype == CG_F16 && out_dtype == CG_F16) return launch_fused<CG_F16, CG_F16>(p, early, st);
+    if (scale_dtype == CG_F16 && out_dtype == CG_BF16) return launch_fused<CG_F16, CG_BF16>(p, early, st);
+    if (scale_dtype == CG_BF16 && out_dtype == CG_F16) return launch_fused<CG_BF16, CG_F16>(p, early, st);
+    return launch_fused<CG_BF16, CG_BF16>(p, early, st);
 }
 
 extern "C" int cg_decode_dequant(const cg_decode_job *jobs_host, int njobs, int nlayers, int nheads,
@@ -655,6 +846,55 @@ extern "C" int cg_decode_dequant_delta(const cg_decode_job *jobs_host, int njobs
         p.res_bins = res_bins;
     }
     return launch_fused_any(p, scale_dtype, out_dtype, static_cast<cudaStream_t>(stream));
+}
+
+// ---- offsets and decode of any number of sub-chunks -----------------------------------------------------------
+extern "C" int cg_decode_kv(const cg_decode_job *jobs_host, int njobs, int nlayers, int nheads, int head_size, int lp,
+                            const float *bins, int delta_group, const float *res_bins, int scale_dtype, int out_dtype,
+                            int64_t o_layer, int64_t o_kv, int64_t o_token, int64_t o_head, int32_t *status,
+                            void *stream) {
+    if (!jobs_host || !bins) return CG_E_NULL;
+    if (njobs <= 0) return CG_E_SHAPE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // all arguments are checked before anything is launched
+    FusedDecodeParams p;
+    const auto fill = [&](int b) {
+        const int n = njobs - b < CG_MAX_DECODE_JOBS ? njobs - b : CG_MAX_DECODE_JOBS;
+        if (int rc = fused_params(jobs_host + b, n, nlayers, nheads, head_size, lp, bins, scale_dtype, out_dtype, o_layer, o_kv,
+                                  o_token, o_head, status, p))
+            return rc;
+        if (delta_group) {
+            if (!res_bins) return CG_E_NULL;
+            if (delta_group < 2 || delta_group > CG_MAX_TOKENS_PER_STREAM || CG_MAX_TOKENS_PER_STREAM % delta_group) return CG_E_SHAPE;
+            if (!multi_layout_ok(p, 2)) return CG_E_ALIGN;
+            p.delta_group = delta_group;
+            p.res_bins = res_bins;
+        }
+        return CG_OK;
+    };
+    for (int b = 0; b < njobs; b += CG_MAX_DECODE_JOBS)
+        if (int rc = fill(b)) return rc;
+    const int nrows = 2 * nlayers, nchannels = nheads * head_size, nslab = (nchannels + kGroup - 1) / kGroup;
+    const bool fused_offsets = static_cast<int64_t>(nrows) * nslab <= kMaxOffsetGroups;
+    for (int b = 0; b < njobs; b += CG_MAX_DECODE_JOBS) {
+        const int n = njobs - b < CG_MAX_DECODE_JOBS ? njobs - b : CG_MAX_DECODE_JOBS;
+        int rc;
+        if (fused_offsets) {
+            rc = launch_offsets(jobs_host + b, n, nrows, nchannels, status, st);
+        } else {
+            rc = CG_OK;
+            for (int j = b; j < b + n && rc == CG_OK; ++j)
+                rc = cg_decode_offsets(jobs_host + j, 1, nrows, nchannels, const_cast<int64_t *>(jobs_host[j].group_off), status, stream);
+        }
+        if (rc) return rc;
+    }
+    for (int b = 0; b < njobs; b += CG_MAX_DECODE_JOBS) {
+        if (int rc = fill(b)) return rc;
+        // the one-channel kernel waits for the launch in front either way
+        p.after = b ? kAfterBatch : kAfterOffsets;
+        if (int rc = launch_fused_any(p, scale_dtype, out_dtype, st, true)) return rc;
+    }
+    return CG_OK;
 }
 
 // ---- decode without a caller-provided workspace --------------------------------------------------------------

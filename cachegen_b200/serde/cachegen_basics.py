@@ -7,14 +7,20 @@ classes pickle under the reference's module path `lmcache.storage_backend.serde.
 when no `lmcache` package is importable, alias modules of that name are registered at import time
 (see cachegen_b200.compat).
 """
+import ctypes
+import functools
 import io
 import os
 import pickle
+import sys
 import threading
+from collections import OrderedDict
 from dataclasses import dataclass, replace
 from typing import List
 
 import torch
+
+from .. import _lib
 
 CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK = 256
 
@@ -187,7 +193,9 @@ class CacheGenGPUEncoderOutput:
 # its storage to pageable host memory, writing a legacy `torch.save` stream of it into one buffer,
 # copying that into the pickle and the pickle into the result: 34 ms for a 30 MB chunk.  dump_blob
 # writes the same bytes -- the same outer pickle, and for each storage the same legacy stream, built
-# by _legacy_stream_head -- from one asynchronous copy of all tensors into pinned memory.
+# by _legacy_stream_head.  The outer pickle is made with placeholders of the storages' sizes while the tensors
+# are on their way into pinned memory, and every tensor's bytes are copied once, from there to their place in
+# the result, by several threads as they arrive (cg_host_download).
 
 class _PersistentId:
     def __init__(self, pid):
@@ -199,23 +207,52 @@ class _LegacyPickler(pickle.Pickler):
         return obj.pid if isinstance(obj, _PersistentId) else None
 
 
-def _legacy_stream_head(dtype: torch.dtype, key: str, location: str, numel: int) -> bytes:
-    """What torch.save(storage, f, _use_new_zipfile_serialization=False) writes before the storage's
-    raw data (torch/serialization.py, _legacy_save): magic number, protocol version and system info
-    as three pickles, the storage as a persistent id, the list of storage keys, the element count."""
-    import sys
+def _legacy_preamble() -> bytes:
+    """Magic number, protocol version and system info of a legacy stream, as three pickles."""
     ser = torch.serialization
-    f = io.BytesIO()
     info = {"protocol_version": ser.PROTOCOL_VERSION, "little_endian": sys.byteorder == "little",
             "type_sizes": {"short": ser.SHORT_SIZE, "int": ser.INT_SIZE, "long": ser.LONG_SIZE}}
-    for part in (ser.MAGIC_NUMBER, ser.PROTOCOL_VERSION, info):
-        pickle.dump(part, f, protocol=ser.DEFAULT_PROTOCOL)
+    return b"".join(pickle.dumps(part, protocol=ser.DEFAULT_PROTOCOL)
+                    for part in (ser.MAGIC_NUMBER, ser.PROTOCOL_VERSION, info))
+
+
+def _pickle_stream_head(dtype: torch.dtype, key: str, location: str, numel: int) -> bytes:
+    """What torch.save(storage, f, _use_new_zipfile_serialization=False) writes before the storage's
+    raw data (torch/serialization.py, _legacy_save): the preamble, the storage as a persistent id, the list
+    of storage keys, the element count."""
+    f = io.BytesIO()
+    f.write(_legacy_preamble())
     storage_type = getattr(torch, torch.storage._dtype_to_storage_type_map()[dtype])
-    _LegacyPickler(f, protocol=ser.DEFAULT_PROTOCOL).dump(
+    _LegacyPickler(f, protocol=torch.serialization.DEFAULT_PROTOCOL).dump(
         _PersistentId(("storage", storage_type, key, location, numel, None)))
-    pickle.dump([key], f, protocol=ser.DEFAULT_PROTOCOL)
+    pickle.dump([key], f, protocol=torch.serialization.DEFAULT_PROTOCOL)
     f.write(int(numel).to_bytes(8, sys.byteorder))
     return f.getvalue()
+
+
+_HEAD_PARTS = {}  # (dtype, location) -> the constant pieces of a head around its key, element count and key
+_KEY, _COUNT = "<a storage's key>", 0x01234567
+
+
+def _pickled_str(v: str) -> bytes:
+    raw = v.encode("utf-8", "surrogatepass")
+    return b"X" + len(raw).to_bytes(4, "little") + raw
+
+
+def _pickled_int(v: int) -> bytes:
+    return pickle.dumps(v, protocol=torch.serialization.DEFAULT_PROTOCOL)[2:-1]
+
+
+def _legacy_stream_head(dtype: torch.dtype, key: str, location: str, numel: int) -> bytes:
+    """_pickle_stream_head's bytes, put together from the pieces of one made before."""
+    parts = _HEAD_PARTS.get((dtype, location))
+    if parts is None:
+        sample = _pickle_stream_head(dtype, _KEY, location, _COUNT)[:-8]
+        before, between, after = sample.split(_pickled_str(_KEY))
+        first, second = between.split(_pickled_int(_COUNT))
+        parts = _HEAD_PARTS[dtype, location] = (before, first, second, after)
+    k = _pickled_str(key)
+    return b"".join((parts[0], k, parts[1], _pickled_int(numel), parts[2], k, parts[3], int(numel).to_bytes(8, sys.byteorder)))
 
 
 class _StreamedStorage:
@@ -239,40 +276,38 @@ _PLACEHOLDER_LEN = 1 << 16  # pickle writes byte strings of at least this size o
 
 
 class _BlobPickler(pickle.Pickler):
-    """Pickles the tensors whose bytes are in `raw_of` (by id) from those bytes; everything else as
-    pickle.dump does.  A large storage stream is not built here: a placeholder byte string of
-    _PLACEHOLDER_LEN bytes stands in for it (pickle frames it the same way: outside the frames) and
-    `deferred` remembers, by the placeholder's id, the stream's head and raw bytes; _assemble puts
-    them in place, so the tensor's bytes are copied once, into the final blob."""
+    """Pickles the tensors in `sizes` (id -> bytes of raw data) with a placeholder for their storage stream;
+    everything else as pickle.dump does.  A placeholder of _PLACEHOLDER_LEN bytes stands for a stream of at
+    least that size (pickle frames both the same way: outside the frames) and reaches the file as the object
+    it is; a smaller one is as long as its stream and is found again by the marker it starts with.
+    `streams` lists (placeholder, head, tensor, stream length) in the order written."""
 
-    def __init__(self, file, raw_of: dict):
+    def __init__(self, file, sizes: dict):
         super().__init__(file)
-        self.raw_of = raw_of
-        self.deferred = {}
-        self.keep = []
+        self.sizes = sizes
+        self.streams = []
 
     def reducer_override(self, obj):
-        if isinstance(obj, torch.Tensor) and id(obj) in self.raw_of:
-            from collections import OrderedDict
+        if isinstance(obj, torch.Tensor) and id(obj) in self.sizes:
             head = _legacy_stream_head(obj.dtype, str(obj.untyped_storage()._cdata),
                                        torch.serialization.location_tag(obj.untyped_storage()), obj.numel())
-            raw = self.raw_of[id(obj)]
-            n = len(head) + len(raw)
-            if _PLACEHOLDER_LEN <= n < (1 << 32):
-                stream = bytes(_PLACEHOLDER_LEN)
-                self.deferred[id(stream)] = (head, raw, n)
-                self.keep.append(stream)  # ids must stay unique until the blob is assembled
-            else:
-                stream = b"".join((head, raw))
-            storage = _StreamedStorage(stream)
+            n = len(head) + self.sizes[id(obj)]
+            if n >= 1 << 32:
+                return NotImplemented  # another opcode: left to torch
+            marker = _MARKER + len(self.streams).to_bytes(4, "little")
+            stream = bytes(_PLACEHOLDER_LEN) if n >= _PLACEHOLDER_LEN else marker + bytes(n - len(marker))
+            self.streams.append((stream, head, obj, n))
             return (torch._utils._rebuild_tensor_v2,
-                    (storage, 0, tuple(obj.size()), obj.stride(), False, OrderedDict()))
+                    (_StreamedStorage(stream), 0, tuple(obj.size()), obj.stride(), False, OrderedDict()))
         return NotImplemented
+
+
+_MARKER = bytes.fromhex("e1f7c36a905d4b2887d21e5cb0394fa6")
 
 
 class _PartsWriter:
     """File object that keeps what is written as a list of byte strings: the pickler hands a large
-    byte string over as the object it was given, so nothing is copied until the final join."""
+    byte string over as the object it was given, so nothing is copied until the blob is put together."""
 
     def __init__(self):
         self.parts = []
@@ -282,84 +317,82 @@ class _PartsWriter:
         return len(b)
 
 
-def _assemble(parts: list, deferred: dict) -> bytes:
-    """The blob from the pickler's writes, every placeholder replaced by its stream: the 4-byte length
-    before it is corrected, then everything is copied once into a new bytes object -- the large pieces
-    by torch's multi-threaded copy, which also spreads the page faults of the fresh allocation."""
-    import ctypes
-    import struct
-    pieces = []  # (bytes-like, length)
-    for i, part in enumerate(parts):
-        d = deferred.get(id(part))
-        if d is None:
-            pieces.append(part)
+def _place_streams(parts: list, streams: list):
+    """Where everything goes: ([(offset, bytes)] of the pickle itself and the streams' heads, [(offset, tensor)]
+    of the streams' raw data, total size), every placeholder replaced by its stream and the 4-byte
+    length before a large one corrected."""
+    large = {id(s[0]): s for s in streams if len(s[0]) == _PLACEHOLDER_LEN}
+    small = [(i, s) for i, s in enumerate(streams) if len(s[0]) < _PLACEHOLDER_LEN]
+    fixed, raw, pos, last = [], [], 0, -1  # last: the pickle's own piece before
+    for part in parts:
+        d = large.get(id(part))
+        if d is not None:
+            _, head, t, n = d
+            at, before = fixed[last] if last >= 0 else (0, b"")
+            # BINBYTES + length, the last thing written before the payload
+            if at + len(before) != pos or not before.endswith(b"B" + _PLACEHOLDER_LEN.to_bytes(4, "little")):
+                raise RuntimeError("unexpected pickle layout around a storage stream")
+            fixed[last] = (at, before[:-4] + n.to_bytes(4, "little"))
+            fixed.append((pos, head))
+            raw.append((pos + len(head), t))
+            pos += n
             continue
-        head, raw, n = d
-        prev = pieces[-1]
-        marker = b"B" + struct.pack("<I", _PLACEHOLDER_LEN)  # BINBYTES + length, the last thing written before the payload
-        if not prev.endswith(marker):
-            raise RuntimeError("unexpected pickle layout around a storage stream")
-        pieces[-1] = prev[:-4] + struct.pack("<I", n)
-        pieces.append(head)
-        pieces.append(raw)
-    total = sum(len(x) for x in pieces)
-    api = ctypes.pythonapi
-    api.PyBytes_FromStringAndSize.restype = ctypes.py_object
-    api.PyBytes_FromStringAndSize.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
-    api.PyBytes_AsString.restype = ctypes.c_void_p
-    api.PyBytes_AsString.argtypes = [ctypes.py_object]
-    blob = api.PyBytes_FromStringAndSize(None, total)  # uninitialised, ours alone until it is returned
-    base = api.PyBytes_AsString(blob)
-    import warnings
-    with warnings.catch_warnings():
-        warnings.simplefilter("ignore")
-        dst = torch.frombuffer((ctypes.c_ubyte * total).from_address(base), dtype=torch.uint8) if total else None
-    pos = 0
-    for x in pieces:
-        n = len(x)
-        if n >= (1 << 20):
-            with warnings.catch_warnings():
-                warnings.simplefilter("ignore")  # a read-only source buffer, and it is only read
-                dst[pos:pos + n].copy_(torch.frombuffer(x, dtype=torch.uint8))
-        elif n:
-            ctypes.memmove(base + pos, bytes(x) if not isinstance(x, bytes) else x, n)
-        pos += n
-    return blob
+        last = len(fixed)
+        fixed.append((pos, part))
+        k = 0
+        while small:
+            i, (stream, head, t, n) = small[0]
+            k = part.find(_MARKER + i.to_bytes(4, "little"), k)
+            if k < 0:
+                break
+            fixed.append((pos + k, head))
+            raw.append((pos + k + len(head), t))
+            small.pop(0)
+            k += n
+        pos += len(part)
+    if small or len(raw) != len(streams):
+        raise RuntimeError("a storage stream's placeholder is missing from the pickle")
+    return fixed, raw, pos
+
+
+_bytes_new = ctypes.pythonapi.PyBytes_FromStringAndSize
+_bytes_new.restype, _bytes_new.argtypes = ctypes.py_object, [ctypes.c_char_p, ctypes.c_ssize_t]
+_bytes_at = ctypes.pythonapi.PyBytes_AsString
+_bytes_at.restype, _bytes_at.argtypes = ctypes.c_void_p, [ctypes.py_object]
 
 
 def dump_blob(eo: "CacheGenGPUEncoderOutput") -> bytes:
     """The pickle of an encoded chunk, byte for byte what pickle.dump writes (cachegen_basics.py:146-151).
-    Tensors that own their storage are read through pinned memory (one asynchronous copy each, one
-    synchronisation) and their legacy streams built here; the others are left to torch."""
+    Tensors that own their storage have their legacy streams built here; the others are left to torch."""
     tensors = [eo.cdf, eo.max_tensors_key, eo.max_tensors_value]
     for dc in eo.data_chunks:
         tensors += [dc.bytestream, dc.bytestream_lengths]
-    fast = [t for t in tensors if isinstance(t, torch.Tensor) and _owns_its_storage(t)]
-    raw_of = {}
-    on_gpu = [t for t in fast if t.is_cuda and t.numel()]
+    sizes = {id(t): t.numel() * t.element_size() for t in tensors if isinstance(t, torch.Tensor) and _owns_its_storage(t)}
+    devices = {t.device for t in tensors if id(t) in sizes and t.is_cuda}
+    if len(devices) > 1:  # one stream carries the transfers: the tensors of another GPU are left to torch
+        sizes = {id(t): sizes[id(t)] for t in tensors if id(t) in sizes and (not t.is_cuda or t.device == tensors[0].device)}
+    on_gpu = [t for t in tensors if id(t) in sizes and t.is_cuda and t.numel()]
+    st = staging()
     if on_gpu:
-        st = staging()
-        sizes = [t.numel() * t.element_size() for t in on_gpu]
-        st.begin(sum((n + 255) // 256 * 256 for n in sizes))
-        pos, slices = 0, []
-        for t, n in zip(on_gpu, sizes):
-            piece = st.buf[pos:pos + n]
-            piece.copy_(t.reshape(-1).view(torch.uint8), non_blocking=True)
-            slices.append(piece)
-            pos += (n + 255) // 256 * 256
-        for dev in {t.device for t in on_gpu}:
-            torch.cuda.current_stream(dev).synchronize()
-        for t, piece in zip(on_gpu, slices):
-            raw_of[id(t)] = memoryview(piece.numpy())
-    for t in fast:
-        if id(t) not in raw_of:
-            raw_of[id(t)] = memoryview(t.reshape(-1).view(torch.uint8).numpy()) if t.numel() else b""
-    out = _PartsWriter()
-    pickler = _BlobPickler(out, raw_of)
-    pickler.dump(eo)
-    blob = _assemble(out.parts, pickler.deferred)
-    if on_gpu:
+        st.fetch(on_gpu)
+    try:
+        out = _PartsWriter()
+        pickler = _BlobPickler(out, sizes)
+        pickler.dump(eo)
+        fixed, raw, total = _place_streams(out.parts, pickler.streams)
+        blob = _bytes_new(None, total)  # uninitialised, ours alone until it is returned
+        base = _bytes_at(blob)
+        for at, piece in fixed:
+            ctypes.memmove(base + at, piece, len(piece))
+        where = {id(t): base + at for at, t in raw}
+        for at, t in raw:
+            if not t.is_cuda and t.numel():
+                ctypes.memmove(base + at, t.data_ptr(), sizes[id(t)])
+    except BaseException:
         st.end()
+        raise
+    if on_gpu:
+        st.collect([where[id(t)] for t in on_gpu])
     return blob
 
 
@@ -398,7 +431,39 @@ def _load_storage_from_bytes(b: bytes):
         return torch.storage._load_from_bytes(bytes(b))
 
 
-def _load_storage_fast(b):
+_HEAD_START = _legacy_preamble() + b"\x80\x02(X\x07\x00\x00\x00storageq\x00ctorch\n"
+_INT_SIZES = {75: 1, 77: 2, 74: 4}  # BININT1, BININT2, BININT
+
+
+def _read_stream_head(b):
+    """(storage class name, location, element count, offset of the raw data) of a legacy stream as
+    _pickle_stream_head writes it, or None."""
+    head = bytes(b[:1024])
+    at = len(_HEAD_START)
+    end = head.find(b"\n", at)
+    if head[:at] != _HEAD_START or end < 0 or head[end + 1:end + 4] != b"q\x01X":
+        return None
+    name = head[at:end]
+    at = end + 8 + int.from_bytes(head[end + 4:end + 8], "little")
+    key = head[end + 3:at]
+    n = int.from_bytes(head[at + 3:at + 7], "little")
+    location = head[at + 7:at + 7 + n]
+    if head[at:at + 3] != b"q\x02X" or head[at + 7 + n:at + 9 + n] != b"q\x03":
+        return None
+    at += 9 + n
+    size = _INT_SIZES.get(head[at]) if at < len(head) else None
+    if size is None:
+        return None
+    numel = int.from_bytes(head[at + 1:at + 1 + size], "little")
+    tail = b"Ntq\x04Q.\x80\x02]q\x00" + key + b"q\x01a." + numel.to_bytes(8, "little")
+    at += 1 + size
+    if head[at:at + len(tail)] != tail:
+        return None
+    return name.decode(), location.decode(), numel, at + len(tail)
+
+
+def _parse_stream_head(b):
+    """The same from any legacy stream, by unpickling its parts; raises what it cannot read."""
     f = io.BytesIO(bytes(b[:1 << 16]))  # the stream's head: small pickles, then the raw data (b may be a view)
     if pickle.load(f) != torch.serialization.MAGIC_NUMBER or pickle.load(f) != torch.serialization.PROTOCOL_VERSION:
         raise ValueError("not a legacy stream")
@@ -413,14 +478,20 @@ def _load_storage_fast(b):
     typename, storage_type, key, location, numel, view = rec.seen[0]
     if typename != "storage" or view is not None or keys[0] != key:
         raise ValueError("storage view")
-    dtype = torch.uint8 if storage_type is torch.UntypedStorage else storage_type.dtype
-    esz = torch._utils._element_size(dtype)
     off = f.tell()
     if off + 8 > min(len(b), 1 << 16):
         raise ValueError("header too long")
-    count = int.from_bytes(b[off:off + 8], "little")
-    nbytes = count * esz
-    if count != numel or off + 8 + nbytes != len(b):
+    if int.from_bytes(b[off:off + 8], "little") != numel:
+        raise ValueError("size mismatch")
+    return storage_type.__name__, location, numel, off + 8
+
+
+def _load_storage_fast(b):
+    name, location, numel, off = _read_stream_head(b) or _parse_stream_head(b)
+    storage_type = getattr(torch, name)
+    dtype = torch.uint8 if storage_type is torch.UntypedStorage else storage_type.dtype
+    nbytes = numel * torch._utils._element_size(dtype)
+    if off + nbytes != len(b):
         raise ValueError("size mismatch")
     device = torch.device(location)
     if device.type == "cuda" and not (torch.cuda.is_available() and (device.index or 0) < torch.cuda.device_count()):
@@ -428,7 +499,7 @@ def _load_storage_fast(b):
     if nbytes == 0:
         raw = torch.empty(0, dtype=torch.uint8, device=device)
     else:
-        view_cpu = torch.frombuffer(b, dtype=torch.uint8, count=nbytes, offset=off + 8)  # read-only, only read
+        view_cpu = torch.frombuffer(b, dtype=torch.uint8, count=nbytes, offset=off)  # read-only, only read
         if device.type == "cpu":
             raw = view_cpu.clone()
         else:
@@ -438,17 +509,17 @@ def _load_storage_fast(b):
 
 class _Staging:
     """Pinned host memory that a thread's blob loads and dumps pass through: bytes are copied into it
-    by torch's multi-threaded CPU copy and leave it by an asynchronous copy on the current stream
-    (or arrive in it from the GPU), several times faster than a copy to or from pageable memory.
-    Two buffers per thread, used in turn and grown on demand, so that filling one overlaps the
-    copies still leaving the other; `begin` waits until the chosen buffer's last copies are done."""
+    by several threads and leave it by asynchronous copies on the current stream (or arrive in it from
+    the GPU), several times faster than a copy to or from pageable memory (cg_host_upload,
+    cg_host_download).  Two buffers per thread, used in turn and grown on demand, so that filling one overlaps
+    the copies still leaving the other; `begin` waits until the chosen buffer's last copies are done."""
 
     def __init__(self):
         self.bufs = [None, None]
         self.events = [None, None]
         self.turn = 0
         self.buf = None
-        self.pos = 0
+        self.waiting = None  # (host view, device tensor) pairs of the load in progress
 
     def begin(self, nbytes: int) -> None:
         self.turn ^= 1
@@ -462,46 +533,86 @@ class _Staging:
             if torch.cuda.is_available():
                 self.bufs[i] = self.bufs[i].pin_memory()
         self.buf = self.bufs[i]
-        self.pos = 0
 
     def end(self) -> None:
-        """Storages loaded outside a blob load do not pass through the staging memory."""
         self.buf = None
 
+    # -- to the GPU: a load collects the tensors it makes, and sends them together
+    def open(self) -> None:
+        self.waiting = []
+
     def to_device(self, view_cpu: torch.Tensor, device) -> torch.Tensor:
-        n = view_cpu.numel()
-        if self.buf is None or self.pos + n > self.buf.numel():
-            return view_cpu.to(device)  # no load in progress, or more data than the blob announced
-        stage = self.buf[self.pos:self.pos + n]
-        self.pos += (n + 255) // 256 * 256
-        stage.copy_(view_cpu)
-        out = torch.empty(n, dtype=torch.uint8, device=device)
-        out.copy_(stage, non_blocking=True)
-        self.events[self.turn] = torch.cuda.Event()
-        self.events[self.turn].record(torch.cuda.current_stream(device))
+        if self.waiting is None:
+            return view_cpu.to(device)  # no load in progress
+        out = torch.empty(view_cpu.numel(), dtype=torch.uint8, device=device)
+        self.waiting.append((view_cpu.data_ptr(), view_cpu.numel(), out, view_cpu))
         return out
 
+    def send(self, pairs: list = None, stream=None) -> None:
+        """The collected tensors' bytes (or another load's) on their way, in the order they were made; on `stream`,
+        or each device's current one."""
+        if pairs is None:
+            pairs, self.waiting = self.waiting, None
+        while pairs:
+            device = pairs[0][2].device
+            mine = [p for p in pairs if p[2].device == device]
+            pairs = [p for p in pairs if p[2].device != device]
+            segs = (_lib.HostSegment * len(mine))(*[(at, o.data_ptr(), n) for at, n, o, _ in mine])
+            self.begin(sum((n + 255) // 256 * 256 for _, n, _, _ in mine))
+            try:
+                with torch.cuda.device(device):
+                    on = torch.cuda.current_stream(device) if stream is None else stream
+                    rc = _lib.lib().cg_host_upload(segs, len(mine), self.buf.data_ptr(), self.buf.numel(), on.cuda_stream)
+                    self.events[self.turn] = torch.cuda.Event()
+                    self.events[self.turn].record(on)
+            finally:
+                self.end()
+            _lib.check(rc, "cg_host_upload")
+
+    def drop(self) -> None:
+        """Forgets a load that failed."""
+        self.waiting = None
 
     def whole_to_device(self, view_cpu: torch.Tensor, device) -> torch.Tensor:
         """One host buffer (any memory) to the GPU through the staging memory."""
-        self.begin(view_cpu.numel())
+        self.open()
+        out = self.to_device(view_cpu, device)
+        self.send()
+        return out
+
+    # -- from the GPU
+    def fetch(self, tensors: list) -> None:
+        """Enqueues the transfers of contiguous tensors of one GPU; `collect` does the rest."""
+        sizes = [t.numel() * t.element_size() for t in tensors]
+        self.segs = (_lib.HostSegment * len(tensors))(*[(None, t.data_ptr(), n) for t, n in zip(tensors, sizes)])
+        self.begin(sum((n + 255) // 256 * 256 for n in sizes))
+        self.fetched = tensors
+        self._download(1)
+
+    def collect(self, pointers: list) -> None:
+        """The bytes of the fetched tensors to these addresses."""
+        for seg, at in zip(self.segs, pointers):
+            seg.host = at
         try:
-            return self.to_device(view_cpu, device)
+            self._download(2)
         finally:
+            self.fetched = None
             self.end()
 
+    def _download(self, phase: int) -> None:
+        device = self.fetched[0].device
+        with torch.cuda.device(device):
+            rc = _lib.lib().cg_host_download(self.segs, len(self.segs), self.buf.data_ptr(), self.buf.numel(), phase,
+                                             torch.cuda.current_stream(device).cuda_stream)
+        _lib.check(rc, "cg_host_download")
+
     def whole_from_device(self, t: torch.Tensor) -> bytes:
-        """The bytes of a contiguous GPU tensor: one asynchronous copy into the staging memory, one
-        synchronisation, one copy into the result."""
-        flat = t.reshape(-1).view(torch.uint8)
-        self.begin(flat.numel())
-        try:
-            stage = self.buf[:flat.numel()]
-            stage.copy_(flat, non_blocking=True)
-            torch.cuda.current_stream(t.device).synchronize()
-            return bytes(memoryview(stage.numpy()))
-        finally:
-            self.end()
+        """The bytes of a contiguous GPU tensor."""
+        n = t.numel() * t.element_size()
+        self.fetch([t])
+        out = _bytes_new(None, n)
+        self.collect([_bytes_at(out)])
+        return out
 
 
 _staging_local = threading.local()
@@ -568,20 +679,139 @@ class _ViewUnpickler(pickle._Unpickler):
         return _find_wire_class(module, name) or super().find_class(module, name)
 
 
-def load_blob(bs):
-    """Unpickles a CacheGenGPUEncoderOutput written by this package or by the reference."""
-    staged = False
+_MAGIC_PICKLE = pickle.dumps(torch.serialization.MAGIC_NUMBER, protocol=torch.serialization.DEFAULT_PROTOCOL)
+_TOKEN = b"cachegen storage"
+
+
+def _cut_streams(bs: bytes):
+    """The pickle with its large storage streams cut out, and those streams: ([bytes of the pickle, a token in
+    place of each stream], {token: (offset, view) of the stream}).  A legacy stream starts with torch's magic number, and
+    the four bytes before it, behind the BINBYTES opcode, are its length; the search goes on behind it, so
+    that the tensors' own bytes are never looked at."""
+    view, pieces, streams, start, at = memoryview(bs), [], {}, 0, 0
+    while True:
+        p = bs.find(_MAGIC_PICKLE, at)
+        if p < 0:
+            break
+        at = p + 1
+        if p < 5 or bs[p - 5] != 66:  # BINBYTES; another opcode stays as it is
+            continue
+        n = int.from_bytes(bs[p - 4:p], "little")
+        if p + n > len(bs):
+            raise ValueError("truncated storage stream")
+        at = p + n
+        if n < _PLACEHOLDER_LEN:
+            continue  # inside a frame of the pickle, whose length counts it
+        token = _TOKEN + len(streams).to_bytes(4, "little")
+        streams[token] = (p, view[p:p + n])
+        pieces += [bs[start:p - 4], len(token).to_bytes(4, "little"), token]
+        start = p + n
+    pieces.append(bs[start:])
+    return b"".join(pieces), streams
+
+
+_STORAGE_DTYPES = {name: dtype for dtype, name in torch.storage._dtype_to_storage_type_map().items()}
+_dtype_of = _STORAGE_DTYPES.get
+
+
+class _CudaStream:
+    """A storage on a GPU whose bytes are still in the blob."""
+
+    def __init__(self, at, dtype, numel, device, view):
+        self.at, self.dtype, self.numel, self.device, self.view = at, dtype, numel, device, view
+
+
+def _stream_storage(streams, base, b):
+    """What a pickled storage is: its bytes b, or a token in place of a stream that was cut out."""
+    at, stream = streams.get(b, (0, b))
+    head = _read_stream_head(stream) if at and torch.cuda.is_available() else None
+    if head is not None and head[1].startswith("cuda"):
+        name, location, numel, off = head
+        dtype = _dtype_of(name)
+        device = torch.device(location)
+        if (dtype is not None and off + numel * dtype.itemsize == len(stream) and numel and
+                (device.index or 0) < torch.cuda.device_count()):
+            return _CudaStream(base + at + off, dtype, numel, device, stream)
+    return _load_storage_from_bytes(stream)
+
+
+def _stream_tensor(storage, offset, size, stride, requires_grad, hooks, metadata=None):
+    """torch._utils._rebuild_tensor_v2 on what _stream_storage gives."""
+    if isinstance(storage, _CudaStream):
+        if offset == 0 and not requires_grad and metadata is None:
+            t = torch.empty(size, dtype=storage.dtype, device=storage.device)
+            if t.numel() == storage.numel and t.stride() == stride:
+                staging().waiting.append((storage.at, storage.numel * t.element_size(), t, storage.view))
+                return t
+        storage = _load_storage_from_bytes(storage.view)
+    return torch._utils._rebuild_tensor_v2(storage, offset, size, stride, requires_grad, hooks, metadata)
+
+
+class _CutUnpickler(pickle.Unpickler):
+    """The loader for a pickle whose large streams were cut out: on the C unpickler, which would copy them.
+    What it puts in its memo must not refer back to it: the cycle would keep the blob until a collection."""
+
+    def __init__(self, bs: bytes):
+        skeleton, streams = _cut_streams(bs)
+        self.storage = functools.partial(_stream_storage, streams, _bytes_at(bs))
+        super().__init__(io.BytesIO(skeleton))
+
+    def find_class(self, module, name):
+        if module == "torch.storage" and name == "_load_from_bytes":
+            return self.storage
+        if module == "torch._utils" and name == "_rebuild_tensor_v2":
+            return _stream_tensor
+        return _find_wire_class(module, name) or super().find_class(module, name)
+
+
+def _unpickle(bs):
+    """The object in a blob, its tensors collected in the open staging load."""
+    if isinstance(bs, bytes):
+        try:
+            return _CutUnpickler(bs).load()
+        except Exception:
+            staging().open()
     try:
-        if torch.cuda.is_available():
-            staging().begin(len(bs))
-            staged = True
         return _ViewUnpickler(bs).load()
     except Exception:
-        with io.BytesIO(bs) as f:
-            return _Unpickler(f).load()
+        staging().open()
+    with io.BytesIO(bs) as f:
+        return _Unpickler(f).load()
+
+
+class BlobLoad:
+    """One blob parsed, its tensors made, but their bytes not yet sent: parsing and sending may be done by two
+    threads.  unpickle / flat inside the `with`, send after it."""
+
+    def __enter__(self):
+        staging().open()
+        return self
+
+    def __exit__(self, *exc):
+        self.pairs = staging().waiting
+        staging().drop()
+
+    def unpickle(self, bs):
+        return _unpickle(bs)
+
+    def flat(self, buf, device):
+        from . import flat_format
+        return flat_format.wrap(buf, lambda view: staging().to_device(view, device))
+
+    def send(self, stream) -> None:
+        staging().send(self.pairs, stream)
+
+
+def load_blob(bs):
+    """Unpickles a CacheGenGPUEncoderOutput written by this package or by the reference."""
+    st = staging()
+    st.open()
+    try:
+        eo = _unpickle(bs)
+        st.send()
     finally:
-        if staged:
-            staging().end()
+        st.drop()
+    return eo
 
 
 def _adopt_reference_module_path():

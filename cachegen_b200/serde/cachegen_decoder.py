@@ -6,7 +6,11 @@ per-sub-chunk launches and the fp32 dequantise / stack / permute / cast chain re
 calls: cg_decode_offsets (the cumsum of dec.py:70) and cg_decode_dequant (everything else).
 (dec.py = cachegen_decoder.py of the reference.)
 """
+import contextlib
 import ctypes
+import functools
+import queue
+import threading
 from typing import List
 
 import torch
@@ -21,6 +25,14 @@ from .cachegen_basics import CacheGenConfig, CacheGenGPUBytestream, CacheGenGPUE
 from .serde import Deserializer
 
 _DTYPES = {torch.float16: _lib.CG_F16, torch.bfloat16: _lib.CG_BF16}
+
+
+_NOTHING = contextlib.nullcontext()
+
+
+def _current(dev):
+    """Context in which `dev` is the current device; nothing to do in the usual case."""
+    return _NOTHING if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def _stream(device):
@@ -107,11 +119,11 @@ def _check_chunk(eo: CacheGenGPUEncoderOutput):
     return L, C, lp, T
 
 
-def _to_device(t: torch.Tensor, dev) -> torch.Tensor:
-    """Encoded chunks may arrive with their tensors in (pinned) host memory: stage them on `dev`."""
-    if t.device == dev:
-        return t
-    return t.to(dev, non_blocking=True)
+def _staged(t: torch.Tensor, dev) -> torch.Tensor:
+    """Encoded chunks may arrive with their tensors in (pinned) host memory: stage them on `dev`, contiguous."""
+    if t.device != dev:
+        t = t.to(dev, non_blocking=True)
+    return t if t.is_contiguous() else t.contiguous()
 
 
 class _ChunkView:
@@ -156,22 +168,24 @@ class _ChunkView:
             self.L, self.C, self.lp, self.T = L, C, lp, T
             self.H, self.D = eo.num_heads, eo.head_size
             self.scale_dtype = eo.max_tensors_key.dtype
-            self.mk = _to_device(eo.max_tensors_key, dev).reshape(L, T).contiguous()
-            self.mv = _to_device(eo.max_tensors_value, dev).reshape(L, T).contiguous()
-            self.tables = _to_device(eo.cdf, dev).contiguous()
+            self.mk = _staged(eo.max_tensors_key, dev)
+            self.mv = _staged(eo.max_tensors_value, dev)
+            self.tables = _staged(eo.cdf, dev)
             self.table_kind = _lib.CG_TABLES_CDF
             self.length_kind = _lib.CG_LENGTHS_I32
             self.subs = []
             for dc in eo.data_chunks:
-                if dc.bytestream.dtype != torch.uint8 or dc.bytestream.dim() != 1:
+                bs, ln = dc.bytestream, dc.bytestream_lengths
+                if bs.dtype != torch.uint8 or bs.dim() != 1:
                     raise RuntimeError("bytestream must be a 1-D uint8 tensor")
-                if dc.bytestream_lengths.dtype != torch.int32 or dc.bytestream_lengths.numel() != 2 * L * C:
+                if ln.dtype != torch.int32 or ln.numel() != 2 * L * C:
                     raise RuntimeError("bytestream_lengths must be int32 [2L, C]")
-                self.subs.append((_to_device(dc.bytestream, dev).contiguous(),
-                                  _to_device(dc.bytestream_lengths, dev).contiguous(), dc.ntokens))
+                self.subs.append((_staged(bs, dev), _staged(ln, dev), dc.ntokens))
             self.table_bytes = self.tables.numel() * 2
             self.length_bytes = len(self.subs) * 2 * L * C * 4
-            self.keep += [self.mk, self.mv, self.tables] + [t for s in self.subs for t in s[:2]]
+            self.keep += (self.mk, self.mv, self.tables)
+            for sub in self.subs:
+                self.keep += sub[:2]
         if sum(s[2] for s in self.subs) != self.T:
             raise RuntimeError("sub-chunk token counts do not add up to the chunk's tokens")
         for _, _, ntok in self.subs:
@@ -208,7 +222,7 @@ class DecodePlan:
         if bins_cpu is None or bins_cpu.numel() != bins.numel():
             bins_cpu = bins.cpu()
             ws["bins_cpu"] = bins_cpu
-        with torch.cuda.device(dev):
+        with _current(dev):
             views = [_ChunkView(eo, dev, bins_cpu, delta) for eo in encoder_outputs]
         v0 = views[0]
         L, C, lp, H, D, scale_dtype = v0.L, v0.C, v0.lp, v0.H, v0.D, v0.scale_dtype
@@ -256,39 +270,30 @@ class DecodePlan:
 
         esz = out.element_size()
         self.keep = list(row_offs.values())  # tensors that must outlive the launches
-        jobs_all = []
+        jobs = self.jobs = (_lib.DecodeJob * njobs_total)()
         self.payload_bytes = self.table_bytes = self.length_bytes = 0
-        t0 = 0
+        at_out, at_off = out.data_ptr(), goff.data_ptr()
+        k = 0
         for v in views:
             self.keep += v.keep
             self.table_bytes += v.table_bytes
             self.length_bytes += v.length_bytes
-            tc = 0
+            tables, mk, mv = v.tables.data_ptr(), v.mk.data_ptr(), v.mv.data_ptr()
+            row_off = row_offs[v.table_kind].data_ptr() if v.table_kind in row_offs else None
             for bs, ln, ntok in v.subs:
-                self.payload_bytes += bs.numel()
-                job = _lib.DecodeJob()
-                job.tables = v.tables.data_ptr()
-                job.bytes = bs.data_ptr()
-                job.lengths = ln.data_ptr()
-                job.group_off = goff.data_ptr() + 8 * len(jobs_all) * ngroups
-                job.scales_k = v.mk.data_ptr() + v.mk.element_size() * tc
-                job.scales_v = v.mv.data_ptr() + v.mv.element_size() * tc
-                job.out = out.data_ptr() + esz * (t0 + tc) * o_token
-                job.table_row_off = row_offs[v.table_kind].data_ptr() if v.table_kind in row_offs else None
-                job.nbytes = bs.numel()
-                job.tables_nbytes = v.table_bytes
-                job.ntokens = ntok
-                job.scale_stride = v.T
-                job.table_kind = v.table_kind
-                job.length_kind = v.length_kind
-                jobs_all.append(job)
-                tc += ntok
-            t0 += v.T
-        self.batches = []
-        for b in range(0, njobs_total, _lib.CG_MAX_DECODE_JOBS):
-            batch = jobs_all[b:b + _lib.CG_MAX_DECODE_JOBS]
-            self.batches.append(((_lib.DecodeJob * len(batch))(*batch), len(batch),
-                                 ctypes.c_void_p(goff.data_ptr() + 8 * b * ngroups)))
+                nbytes = bs.numel()
+                self.payload_bytes += nbytes
+                job = jobs[k]
+                job.tables, job.bytes, job.lengths, job.group_off = tables, bs.data_ptr(), ln.data_ptr(), at_off
+                job.scales_k, job.scales_v, job.out, job.table_row_off = mk, mv, at_out, row_off
+                job.nbytes, job.tables_nbytes, job.ntokens, job.scale_stride = nbytes, v.table_bytes, ntok, v.T
+                job.table_kind, job.length_kind = v.table_kind, v.length_kind
+                mk += 2 * ntok
+                mv += 2 * ntok
+                at_out += esz * o_token * ntok
+                at_off += 8 * ngroups
+                k += 1
+        self.njobs = njobs_total
         self.delta_group, self.res_bins = 0, None
         if delta is not None:
             self.delta_group = delta.group
@@ -298,51 +303,60 @@ class DecodePlan:
         self.dims = (L, H, D, C, lp, NL, total_T)
         self.strides = (o_layer, o_kv, o_token, o_head)
         self.dtypes = (_DTYPES[scale_dtype], _DTYPES[out_dtype])
-        self.njobs = njobs_total
         # bytes one decode pass must move: 16-bit KV out, payload, tables, lengths, scales in
         self.scale_bytes = NL * total_T * 2
         self.output_bytes = NL * total_T * C * esz
 
+    @functools.cached_property
+    def batches(self):
+        """(jobs, how many, their group offsets) of every cg_decode_offsets / cg_decode_dequant call."""
+        ngroups = self.dims[5] * ((self.dims[3] + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS)
+        most, size = _lib.CG_MAX_DECODE_JOBS, ctypes.sizeof(_lib.DecodeJob)
+        return [((_lib.DecodeJob * min(most, self.njobs - b)).from_buffer(self.jobs, b * size), min(most, self.njobs - b),
+                 ctypes.c_void_p(self.goff.data_ptr() + 8 * b * ngroups)) for b in range(0, self.njobs, most)]
+
     # launches per call: 2 per batch
     def run_offsets(self) -> None:
         lib = _lib.lib()
-        L, H, D, C, lp, NL, _ = self.dims
-        with torch.cuda.device(self.dev):
+        NL, C = self.dims[5], self.dims[3]
+        with _current(self.dev):
             st = _stream(self.dev)
             for arr, n, goff in self.batches:
-                rc = lib.cg_decode_offsets(arr, n, NL, C, goff, ctypes.c_void_p(self.status.data_ptr()), st)
+                rc = lib.cg_decode_offsets(arr, n, NL, C, goff, self.status.data_ptr(), st)
                 _lib.check(rc, "cg_decode_offsets")
 
     # launches per call: 1 per batch
     def run_decode(self) -> None:
         lib = _lib.lib()
         L, H, D, C, lp, NL, _ = self.dims
-        o_layer, o_kv, o_token, o_head = self.strides
-        with torch.cuda.device(self.dev):
+        with _current(self.dev):
             st = _stream(self.dev)
             for arr, n, _ in self.batches:
                 if self.delta_group:
-                    rc = lib.cg_decode_dequant_delta(arr, n, L, H, D, lp, ctypes.c_void_p(self.bins.data_ptr()),
-                                                     self.delta_group, ctypes.c_void_p(self.res_bins.data_ptr()),
-                                                     self.dtypes[0], self.dtypes[1], o_layer, o_kv, o_token, o_head,
-                                                     ctypes.c_void_p(self.status.data_ptr()), st)
+                    rc = lib.cg_decode_dequant_delta(arr, n, L, H, D, lp, self.bins.data_ptr(), self.delta_group,
+                                                     self.res_bins.data_ptr(), *self.dtypes, *self.strides,
+                                                     self.status.data_ptr(), st)
                 else:
-                    rc = lib.cg_decode_dequant(arr, n, L, H, D, lp, ctypes.c_void_p(self.bins.data_ptr()),
-                                               self.dtypes[0], self.dtypes[1], o_layer, o_kv, o_token, o_head,
-                                               ctypes.c_void_p(self.status.data_ptr()), st)
+                    rc = lib.cg_decode_dequant(arr, n, L, H, D, lp, self.bins.data_ptr(), *self.dtypes, *self.strides,
+                                               self.status.data_ptr(), st)
                 _lib.check(rc, "cg_decode_dequant")
 
+    # launches per call: 2 per batch
     def run(self) -> torch.Tensor:
-        self.run_offsets()
-        self.run_decode()
+        L, H, D, _, lp, _, _ = self.dims
         cur = torch.cuda.current_stream(self.dev)
+        with _current(self.dev):
+            rc = _lib.lib().cg_decode_kv(self.jobs, self.njobs, L, H, D, lp, self.bins.data_ptr(), self.delta_group,
+                                         self.res_bins.data_ptr() if self.delta_group else None, *self.dtypes, *self.strides,
+                                         self.status.data_ptr(), cur.cuda_stream)
+        _lib.check(rc, "cg_decode_kv")
         for t in self.keep:
             t.record_stream(cur)
         return self.out
 
     @property
     def launches(self) -> int:
-        return 3 * len(self.batches)
+        return 2 * ((self.njobs + _lib.CG_MAX_DECODE_JOBS - 1) // _lib.CG_MAX_DECODE_JOBS)
 
 
 def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Tensor, fmt: str,
@@ -364,6 +378,13 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
 
 
 _copy_streams = {}
+
+
+def _copy_stream(dev) -> torch.cuda.Stream:
+    stream = _copy_streams.get(dev)
+    if stream is None:
+        stream = _copy_streams[dev] = torch.cuda.Stream(device=dev)
+    return stream
 
 
 def _chunk_tokens(eo) -> int:
@@ -390,10 +411,7 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
         out = torch.empty(shape, dtype=out_dtype, device=dev)
     elif tuple(out.shape) != shape:
         raise RuntimeError("output tensor has the wrong shape")
-    copy_stream = _copy_streams.get(dev)
-    if copy_stream is None:
-        copy_stream = torch.cuda.Stream(device=dev)
-        _copy_streams[dev] = copy_stream
+    copy_stream = _copy_stream(dev)
     cur = torch.cuda.current_stream(dev)
     copy_stream.wait_stream(cur)
     if workspaces is None:
@@ -533,12 +551,78 @@ class CacheGenDeserializer(Deserializer):
 
     def from_bytes_many(self, blobs: List[bytes], out: torch.Tensor = None) -> torch.Tensor:
         """from_bytes for the blobs of consecutive chunks of one KV cache: one result tensor, as
-        decode_many builds it; each blob is loaded while the copies of the one before are still on
-        their way to the GPU."""
+        decode_many builds it.  Three things run side by side: the blobs' bytes on their way to the GPU (on a
+        copy stream), the parsing of the blobs after the first (on a thread; the copies leave the interpreter to
+        it), and the decode of each chunk that has arrived."""
+        if not blobs:
+            raise RuntimeError("nothing to decode")
         dev = torch.device("cuda", torch.cuda.current_device())
-        chunks = [flat_format.from_bytes(b, device=dev) if flat_format.is_flat(b) else CacheGenGPUEncoderOutput.from_bytes(b)
-                  for b in blobs]
-        return self.decode_many(chunks, out=out)
+        cur, copies = torch.cuda.current_stream(dev), _copy_stream(dev)
+        copies.wait_stream(cur)  # the tensors come from the current stream's pool
+        total = len(blobs)
+        parsed = queue.SimpleQueue()
+
+        def parse(blob):
+            load = CGBasics.BlobLoad()
+            with load:
+                chunk = (load.flat(blob, dev) if flat_format.is_flat(blob) else load.unpickle(blob))
+            ntokens = _chunk_tokens(chunk)
+            if ntokens > self.chunk_size:
+                raise RuntimeError(f"a blob holds more tokens than chunk_size = {self.chunk_size}")
+            return load, chunk, ntokens
+
+        def parse_rest():
+            try:
+                with torch.cuda.device(dev), torch.cuda.stream(cur):
+                    for blob in blobs[1:]:
+                        parsed.put(parse(blob))
+            except BaseException as e:  # handed to the caller's thread
+                parsed.put(e)
+
+        first = parse(blobs[0])
+        if total > 1:
+            threading.Thread(target=parse_rest, daemon=True).start()
+        chunks, tokens, done, at = [], 0, 0, 0
+        waiting = []
+        try:
+            while done < total:
+                item = first if done == 0 else (waiting.pop(0) if waiting else parsed.get())
+                if isinstance(item, BaseException):
+                    raise item
+                load, chunk, ntokens = item
+                load.send(copies)
+                arrived = torch.cuda.Event()
+                arrived.record(copies)
+                chunks.append((chunk, ntokens, arrived))
+                tokens += ntokens
+                done += 1
+                while not parsed.empty():
+                    waiting.append(parsed.get())
+                if done + len(waiting) < total or any(isinstance(w, BaseException) for w in waiting):
+                    continue  # the result's size is not known yet
+                if at == 0:
+                    out = self._blob_for(chunks[0][0], tokens + sum(w[2] for w in waiting), dev, out)
+                    start = 0
+                for chunk, n, arrived in chunks[at:]:
+                    cur.wait_event(arrived)
+                    part = out[:, :, start:start + n] if self.fmt == "vllm" else out[:, :, :, start:start + n]
+                    decode_many([chunk], self._bins_on(dev), self.fmt, self.out_dtype, out=part,
+                                workspace=self._workspace, delta=self.delta)
+                    start += n
+                at = len(chunks)
+        finally:
+            cur.wait_stream(copies)
+        return out
+
+    def _blob_for(self, chunk, ntokens, dev, out):
+        """The result of a decode of ntokens tokens: `out`, checked, or a new tensor."""
+        L, H, D = self._bins.numel() // 2, chunk.num_heads, chunk.head_size
+        shape = (L, 2, ntokens, H, D) if self.fmt == "vllm" else (L, 2, H, ntokens, D)
+        if out is None:
+            return torch.empty(shape, dtype=self.out_dtype, device=dev)
+        if tuple(out.shape) != shape:
+            raise RuntimeError("output tensor has the wrong shape, dtype, device or innermost stride")
+        return out
 
     @_lmcache_nvtx_annotate
     def from_bytes(self, bs: bytes) -> torch.Tensor:

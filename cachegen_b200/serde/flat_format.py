@@ -27,6 +27,7 @@ Sections start on 256-byte boundaries.  Like the reference's blob, the container
 the bin settings: encoder and decoder must be configured alike.
 """
 import struct
+import warnings
 import zlib
 from dataclasses import dataclass
 from typing import List
@@ -264,18 +265,23 @@ class FlatChunk:
         return self.header.sub_off[-1]
 
 
+def wrap(buf, to_device) -> FlatChunk:
+    """A bytes-like CGB2 container on a GPU: to_device makes the GPU tensor of a view of its bytes."""
+    header = FlatHeader.parse(buf)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")  # a read-only buffer, and it is only read
+        view = torch.frombuffer(buf, dtype=torch.uint8)
+    return FlatChunk(to_device(view), header)
+
+
 def from_bytes(buf, device=None) -> FlatChunk:
     """Wraps a bytes-like CGB2 container; with `device` the bytes are copied there (to a GPU through
     pinned staging memory, straight from `buf`)."""
-    header = FlatHeader.parse(buf)
     device = torch.device(device) if device is not None else None
     if device is not None and device.type == "cuda":
-        import warnings
         from .cachegen_basics import staging
-        with warnings.catch_warnings():
-            warnings.simplefilter("ignore")  # a read-only buffer, and it is only read
-            view = torch.frombuffer(buf, dtype=torch.uint8)
-        return FlatChunk(staging().whole_to_device(view, device), header)
+        return wrap(buf, lambda view: staging().whole_to_device(view, device))
+    header = FlatHeader.parse(buf)
     t = torch.frombuffer(bytearray(buf) if isinstance(buf, bytes) else buf, dtype=torch.uint8)
     chunk = FlatChunk(t, header)
     return chunk.to(device) if device is not None else chunk

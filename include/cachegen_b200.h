@@ -421,6 +421,37 @@ int cg_decode_dequant_static(const cg_decode_job *jobs_host, int njobs, int nlay
                              int64_t o_layer, int64_t o_kv, int64_t o_token, int64_t o_head,
                              int32_t *status, void *stream);
 
+/*
+ * cg_decode_offsets and cg_decode_dequant (with delta_group, cg_decode_dequant_delta) for any number of sub-chunks:
+ * jobs_host[j].group_off is the job's own room for nrows * ceil(nchannels/128) int64 offsets, written and then
+ * read.  Batches of CG_MAX_DECODE_JOBS overlap each other's ends.
+ */
+int cg_decode_kv(const cg_decode_job *jobs_host, int njobs, int nlayers, int nheads, int head_size, int lp,
+                 const float *bins, int delta_group, const float *res_bins, int scale_dtype, int out_dtype,
+                 int64_t o_layer, int64_t o_kv, int64_t o_token, int64_t o_head, int32_t *status, void *stream);
+
+/* ------------------------------------------------------------------------------------------
+ * byte strings in host memory
+ * ------------------------------------------------------------------------------------------ */
+
+/*
+ * Host memory that is not pinned to the GPU (upload) and back (download), through `staging`, pinned memory of
+ * at least the sum of the segments' sizes, each rounded up to 256.  The copies between host memories are
+ * spread over the calling thread and up to eight helper threads (started on demand, ended after five idle
+ * seconds) and overlap the transfers.  cg_host_upload returns when the segments' host memory has been read and
+ * every transfer is enqueued: `staging` is in use until the stream has passed them.  cg_host_download returns
+ * when the segments' host memory has been written.  phase 0: all of it; 1: enqueues the transfers only (the segments'
+ * `host` is not looked at); 2: the rest, by the same thread with the same segments and no other download between.
+ */
+typedef struct cg_host_segment {
+    void *host;
+    void *device;
+    int64_t bytes;
+} cg_host_segment;
+int cg_host_upload(const cg_host_segment *segments_host, int nsegments, void *staging, int64_t staging_bytes, void *stream);
+int cg_host_download(const cg_host_segment *segments_host, int nsegments, void *staging, int64_t staging_bytes, int phase,
+                     void *stream);
+
 #ifdef __cplusplus
 }
 #endif
