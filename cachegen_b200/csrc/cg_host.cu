@@ -78,7 +78,7 @@ struct Job {
         } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
         Piece &p = pieces[i];
         if (p.src) copy_piece(p.dst, p.src, p.bytes);
-        else for (int64_t k = 0; k < p.bytes; k += 4096) reinterpret_cast<volatile uint8_t *>(p.dst)[k] = 0;
+        else for (int64_t k = 0; k < p.bytes; k += 4096) asm volatile("lock; orb $0, %0" : "+m"(p.dst[k]));  // may already hold data
         p.done.store(true, std::memory_order_release);
         return true;
     }
