@@ -11,6 +11,7 @@ CG_MAX_TOKENS_PER_STREAM = 256
 CG_MAX_LP = 64
 CG_GROUP_CHANNELS = 128
 CG_MAX_DECODE_JOBS = 40
+CG_MAX_OFFSET_GROUPS = 96000
 CG_S_STREAM_OVERFLOW, CG_S_BAD_LENGTHS, CG_S_BAD_SYMBOL, CG_S_COUNT_OVERFLOW, CG_S_BAD_TABLE = 1, 2, 4, 8, 16
 CG_TABLES_CDF, CG_TABLES_COUNTS, CG_TABLES_SPARSE = 0, 1, 2
 CG_LENGTHS_I32, CG_LENGTHS_U16 = 0, 1
@@ -71,6 +72,7 @@ class HostSegment(ctypes.Structure):
 
 EXPORTS = [
     "cg_host_upload", "cg_host_download", "cg_decode_kv",
+    "cg_stream_sizes", "cg_decode_packed", "cg_wait_word",
     "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_wait", "cg_encode_kv_gather", "cg_encode_kv_flat",
     "cg_version", "cg_status_string", "cg_last_cuda_error", "cg_workspace_bytes",
     "cg_calculate_cdf", "cg_encode_padded", "cg_decode_padded", "cg_decode_prefsum", "cg_decode_prefsum_warp",
@@ -126,6 +128,9 @@ def lib():
     L.cg_encode_kv_wait.argtypes = [job, p]
     L.cg_encode_kv_gather.argtypes = [job, ctypes.POINTER(p), ctypes.POINTER(p), p]
     L.cg_encode_kv_flat.argtypes = [job, ctypes.POINTER(FlatLayout), p]
+    L.cg_stream_sizes.argtypes = [p, i, i, i, p, p, p, p]
+    L.cg_decode_packed.argtypes = [p, p, i64, p, p, p, S3, i, i, i, i, p, p]
+    L.cg_wait_word.argtypes = [p, p]
     L.cg_decode_kv.argtypes = [ctypes.POINTER(DecodeJob), i, i, i, i, i, p, i, p, i, i, i64, i64, i64, i64, p, p]
     L.cg_host_upload.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, p]
     L.cg_host_download.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, i, p]

@@ -12,13 +12,22 @@ __host__ __device__ inline int table_rows(int lp, int levels) {
     return (1 << levels) > lp - 1 ? (1 << levels) : lp - 1;
 }
 
+// What a decode launch follows, when it is launched so that its blocks may start before the launch in front of it
+// has ended (programmatic dependent launch).  kAfterOffsets: the group offsets it needs; everything up to
+// reading them runs beside that launch.  kAfterBatch: another batch of the same call, on which it does not depend,
+// so that its blocks fill what that one's last wave leaves idle; it only must not end first.
+enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- symbol-output kernels (decode_fast_prefsum / decode_fast_new) -----------------------------------
 struct SymDecodeParams {
     const int16_t *cdf;
     const uint8_t *bytes;
     int64_t nbytes;          // total bytes addressable from `bytes`
     const int64_t *prefsum;  // mode 0
-    const int32_t *lengths;  // mode 1
+    const int32_t *lengths;  // modes 1 and 2
+    const int64_t *group_off;  // mode 2: offset of each 128-channel group
     int64_t stream_stride;   // mode 1
     uint8_t *out;
     int64_t o0, o1, o2;
@@ -26,6 +35,8 @@ struct SymDecodeParams {
     int32_t *status;
 };
 
+// MODE 0: streams back to back, placed by an inclusive prefix sum of their lengths; 1: one per padded row; 2: back to
+// back, placed by group offsets and a scan of the block's lengths.
 template <int LEVELS, int MODE>
 __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeParams p) {
     extern __shared__ uint32_t tab[];
@@ -34,13 +45,21 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
     const int c = blockIdx.x * kGroup + tid;
     // the lanes that decode together, taken while the warp is still converged
     const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, c < p.nchannels);
-    if (c >= p.nchannels) return;  // no block barrier in this kernel
     const int64_t g = static_cast<int64_t>(row) * p.nchannels + c;
     int64_t start, len;
+    if (MODE == 2) {
+        __shared__ int warp_sums[kGroup / 32];
+        const int n = c < p.nchannels ? max(0, min(__ldg(p.lengths + g), 1 << 20)) : 0;
+        const int excl = block_exclusive_scan_128(n, warp_sums, tid, nullptr);
+        wait_for_launch_before();
+        start = __ldg(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
+        len = n;
+    }
+    if (c >= p.nchannels) return;  // no block barrier from here on
     if (MODE == 0) {
         start = g ? p.prefsum[g - 1] : 0;
         len = p.prefsum[g] - start;
-    } else {
+    } else if (MODE == 1) {
         start = g * p.stream_stride;
         len = p.lengths[g];
         if (len > p.stream_stride) len = p.stream_stride;
@@ -122,14 +141,6 @@ struct FusedDecodeParams {
     int after;  // see DecodeAfter
     cg_decode_job jobs[CG_MAX_DECODE_JOBS];
 };
-
-// What a decode launch follows, when it is launched so that its blocks may start before the launch in front of it
-// has ended (programmatic dependent launch).  kAfterOffsets: the group offsets it needs; everything up to
-// reading them runs beside that launch.  kAfterBatch: another batch of the same call, on which it does not depend,
-// so that its blocks fill what that one's last wave leaves idle; it only must not end first.
-enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
-__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- table staging by the block --------------------------------------------------------------------------
 // The int16 tables of a block's 128 channels are one contiguous run.  Read channel by channel they are 2-byte
@@ -525,27 +536,6 @@ static size_t table_bytes(int lp, int levels) {
     return static_cast<size_t>(table_rows(lp, levels) + 1) * kRowBytes;  // +1: the row read past the last symbol
 }
 
-// Instantiated search depths: 3..6, whatever the table length.
-template <int MODE>
-static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) {
-    const int need = search_levels(p.lp);
-    const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows), block(kGroup);
-#define CG_LAUNCH_SYM(L)                                                                                 \
-    do {                                                                                                  \
-        const size_t smem = table_bytes(p.lp, L);                                                         \
-        if (smem > 48 * 1024)                                                                             \
-            cudaFuncSetAttribute(decode_symbols_kernel<L, MODE>,                                      \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));    \
-        decode_symbols_kernel<L, MODE><<<grid, block, smem, st>>>(p);                                 \
-    } while (0)
-    if (need <= 3) CG_LAUNCH_SYM(3);
-    else if (need == 4) CG_LAUNCH_SYM(4);
-    else if (need == 5) CG_LAUNCH_SYM(5);
-    else CG_LAUNCH_SYM(6);
-#undef CG_LAUNCH_SYM
-    return check_launch();
-}
-
 // early: the blocks may start before the launch in front has ended (see DecodeAfter)
 template <class... Args>
 static int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t st, Args... args) {
@@ -563,6 +553,19 @@ static int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, 
     cfg.numAttrs = early ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
+}
+
+// Instantiated search depths: 3..6, whatever the table length.
+template <int MODE>
+static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) {
+    const int need = search_levels(p.lp);
+    const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows);
+#define CG_LAUNCH_SYM(L) return launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
+    if (need <= 3) CG_LAUNCH_SYM(3);
+    if (need == 4) CG_LAUNCH_SYM(4);
+    if (need == 5) CG_LAUNCH_SYM(5);
+    CG_LAUNCH_SYM(6);
+#undef CG_LAUNCH_SYM
 }
 
 template <int SCALE_DT, int OUT_DT>
@@ -603,21 +606,32 @@ struct OffsetJobs {
     int64_t expect[CG_MAX_DECODE_JOBS];
     int32_t kind[CG_MAX_DECODE_JOBS];
 };
-constexpr int kOffsetBlocks = 8, kOffsetThreads = 512, kMaxOffsetGroups = 8 * 8192;
+constexpr int kOffsetBlocks = 8, kOffsetThreads = 512, kMaxOffsetGroups = CG_MAX_OFFSET_GROUPS;
 
-__device__ __forceinline__ int clamped_length(int v, bool *bad) {
+// For callers that wait for the sum of one job's lengths (tail: host memory that the GPU can write): [0] the sum,
+// [1] 1 if a length is negative or above `longest`, [2] the word at `extra`, then [3] becomes 1.
+struct StreamSizes {
+    int64_t *tail;
+    const int32_t *extra;
+    int longest;
+};
+
+__device__ __forceinline__ int clamped_length(int v, int longest, bool *bad) {
     if (v < 0) { v = 0; *bad = true; }
-    if (v > (1 << 20)) { v = 1 << 20; *bad = true; }
+    if (v > longest) { v = longest; *bad = true; }
     return v;
 }
 
 __global__ void __cluster_dims__(kOffsetBlocks, 1, 1) __launch_bounds__(kOffsetThreads)
-group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nchannels, int nslab, int32_t *status) {
+group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nchannels, int nslab, int32_t *status,
+                     const StreamSizes sizes) {
     extern __shared__ int sums[];  // the groups of this block
     __shared__ int64_t warp_sums[kOffsetThreads / 32];
     __shared__ int64_t block_total;
+    __shared__ uint32_t block_bad;
     let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) block_bad = 0u;
     const int j = blockIdx.x / kOffsetBlocks, rank = blockIdx.x % kOffsetBlocks;
     const int ngroups = nrows * nslab, per = (ngroups + kOffsetBlocks - 1) / kOffsetBlocks;
     const int first = min(ngroups, rank * per), count = min(ngroups, first + per) - first;
@@ -635,20 +649,21 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
                 s = q.x + q.y + q.z + q.w;
             } else {
                 const int4 q = __ldg(static_cast<const int4 *>(lengths) + static_cast<int64_t>(gid) * 32 + lane);
-                s = clamped_length(q.x, &bad) + clamped_length(q.y, &bad) + clamped_length(q.z, &bad) + clamped_length(q.w, &bad);
+                s = clamped_length(q.x, sizes.longest, &bad) + clamped_length(q.y, sizes.longest, &bad) + clamped_length(q.z, sizes.longest, &bad) + clamped_length(q.w, sizes.longest, &bad);
             }
         } else {
             const int row = gid / nslab, slab = gid % nslab;
             for (int c = slab * kGroup + lane; c < min(nchannels, (slab + 1) * kGroup); c += 32) {
                 const int64_t at = static_cast<int64_t>(row) * nchannels + c;
                 s += clamped_length(u16 ? static_cast<int>(__ldg(static_cast<const uint16_t *>(lengths) + at))
-                                        : __ldg(static_cast<const int32_t *>(lengths) + at), &bad);
+                                        : __ldg(static_cast<const int32_t *>(lengths) + at), sizes.longest, &bad);
             }
         }
         s = __reduce_add_sync(0xFFFFFFFFu, s);
         if (lane == 0) sums[k] = s;
     }
     __syncthreads();
+    if (bad) block_bad = 1u;
     // exclusive scan: a run of groups per thread
     const int run = (count + kOffsetThreads - 1) / kOffsetThreads, b = min(count, tid * run), e = min(count, b + run);
     int64_t local = 0;
@@ -685,10 +700,25 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
         at += sums[k];
     }
     if (status && (bad || (rank == 0 && tid == 0 && all != jobs.expect[j]))) atomicOr(status, CG_S_BAD_LENGTHS);
+    if (sizes.tail && rank == 0 && tid == 0) {
+        uint32_t any = 0;
+        for (int r = 0; r < kOffsetBlocks; ++r) {
+            uint32_t remote, v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&block_bad)), "r"(r));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote));
+            any |= v;
+        }
+        sizes.tail[0] = all;
+        sizes.tail[1] = any;
+        sizes.tail[2] = sizes.extra ? *sizes.extra : 0;
+        __threadfence_system();
+        *reinterpret_cast<volatile int64_t *>(sizes.tail + 3) = 1;
+    }
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");  // the totals have been read
 }
 
-static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int nchannels, int32_t *status, cudaStream_t st) {
+static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int nchannels, int32_t *status, cudaStream_t st,
+                          const StreamSizes &sizes = StreamSizes{nullptr, nullptr, 1 << 20}) {
     OffsetJobs o;
     for (int j = 0; j < njobs; ++j) {
         o.lengths[j] = jobs[j].lengths;
@@ -698,7 +728,7 @@ static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int n
     }
     const int nslab = (nchannels + kGroup - 1) / kGroup;
     const size_t smem = static_cast<size_t>((static_cast<int64_t>(nrows) * nslab + kOffsetBlocks - 1) / kOffsetBlocks) * sizeof(int);
-    group_offsets_kernel<<<njobs * kOffsetBlocks, kOffsetThreads, smem, st>>>(o, nrows, nchannels, nslab, status);
+    group_offsets_kernel<<<njobs * kOffsetBlocks, kOffsetThreads, smem, st>>>(o, nrows, nchannels, nslab, status, sizes);
     return check_launch();
 }
 
@@ -721,7 +751,7 @@ extern "C" int cg_decode_prefsum(const int16_t *cdf, const uint8_t *bytes, int64
     if (!cdf || !prefsum || !out || !out_strides || (!bytes && nbytes > 0)) return CG_E_NULL;
     if (nbytes < 0) return CG_E_SHAPE;
     if (int rc = check_coder_shape(nrows, ntokens, nchannels, lp)) return rc;
-    SymDecodeParams p{cdf, bytes, nbytes, prefsum, nullptr, 0, out, out_strides[0], out_strides[1],
+    SymDecodeParams p{cdf, bytes, nbytes, prefsum, nullptr, nullptr, 0, out, out_strides[0], out_strides[1],
                       out_strides[2], ntokens, nchannels, lp, status};
     return launch_symbols<0>(p, nrows, static_cast<cudaStream_t>(stream));
 }
@@ -734,7 +764,7 @@ extern "C" int cg_decode_prefsum_warp(const int16_t *cdf, const uint8_t *bytes, 
     if (nbytes < 0) return CG_E_SHAPE;
     if (int rc = check_coder_shape(nrows, ntokens, nchannels, lp)) return rc;
     if (lp > 33) return CG_E_LP;
-    SymDecodeParams p{cdf, bytes, nbytes, prefsum, nullptr, 0, out, out_strides[0], out_strides[1],
+    SymDecodeParams p{cdf, bytes, nbytes, prefsum, nullptr, nullptr, 0, out, out_strides[0], out_strides[1],
                       out_strides[2], ntokens, nchannels, lp, status};
     const int64_t nstreams = static_cast<int64_t>(nrows) * nchannels;
     const int64_t blocks = (nstreams * 32 + kGroup - 1) / kGroup;
@@ -751,7 +781,7 @@ extern "C" int cg_decode_padded(const int16_t *cdf, const uint8_t *streams, int6
     if (stream_stride <= 0) return CG_E_SHAPE;
     if (int rc = check_coder_shape(nrows, ntokens, nchannels, lp)) return rc;
     SymDecodeParams p{cdf, streams, static_cast<int64_t>(nrows) * nchannels * stream_stride, nullptr,
-                      lengths, stream_stride, out, out_strides[0], out_strides[1], out_strides[2],
+                      lengths, nullptr, stream_stride, out, out_strides[0], out_strides[1], out_strides[2],
                       ntokens, nchannels, lp, status};
     return launch_symbols<1>(p, nrows, static_cast<cudaStream_t>(stream));
 }
@@ -846,6 +876,42 @@ extern "C" int cg_decode_dequant_delta(const cg_decode_job *jobs_host, int njobs
         p.res_bins = res_bins;
     }
     return launch_fused_any(p, scale_dtype, out_dtype, static_cast<cudaStream_t>(stream));
+}
+
+// ---- streams located by their lengths -------------------------------------------------------------------------
+static int one_offsets(const int32_t *lengths, int64_t nbytes, int nrows, int nchannels, int64_t *group_off, int32_t *status,
+                       cudaStream_t st, const StreamSizes &sizes) {
+    if (nrows <= 0 || nchannels <= 0 || nrows > 65535) return CG_E_SHAPE;
+    if (static_cast<int64_t>(nrows) * ((nchannels + kGroup - 1) / kGroup) > kMaxOffsetGroups) return CG_E_CAPACITY;
+    cg_decode_job job{};
+    job.lengths = lengths;
+    job.group_off = group_off;
+    job.nbytes = nbytes;
+    job.length_kind = CG_LENGTHS_I32;
+    return launch_offsets(&job, 1, nrows, nchannels, status, st, sizes);
+}
+
+extern "C" int cg_stream_sizes(const int32_t *lengths, int nrows, int nchannels, int longest, const int32_t *extra,
+                               int64_t *group_off_out, int64_t *tail, void *stream) {
+    if (!lengths || !group_off_out || !tail) return CG_E_NULL;
+    if (longest < 0) return CG_E_SHAPE;
+    tail[3] = 0;
+    return one_offsets(lengths, 0, nrows, nchannels, group_off_out, nullptr, static_cast<cudaStream_t>(stream),
+                       StreamSizes{tail, extra, longest});
+}
+
+extern "C" int cg_decode_packed(const int16_t *cdf, const uint8_t *bytes, int64_t nbytes, const int32_t *lengths,
+                                int64_t *group_off, uint8_t *out, const int64_t out_strides[3], int nrows, int ntokens,
+                                int nchannels, int lp, int32_t *status, void *stream) {
+    if (!cdf || !lengths || !group_off || !out || !out_strides || (!bytes && nbytes > 0)) return CG_E_NULL;
+    if (nbytes < 0) return CG_E_SHAPE;
+    if (int rc = check_coder_shape(nrows, ntokens, nchannels, lp)) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (int rc = one_offsets(lengths, nbytes, nrows, nchannels, group_off, status, st, StreamSizes{nullptr, nullptr, 1 << 20}))
+        return rc;
+    SymDecodeParams p{cdf, bytes, nbytes, nullptr, lengths, group_off, 0, out, out_strides[0], out_strides[1],
+                      out_strides[2], ntokens, nchannels, lp, status};
+    return launch_symbols<2>(p, nrows, st);
 }
 
 // ---- offsets and decode of any number of sub-chunks -----------------------------------------------------------

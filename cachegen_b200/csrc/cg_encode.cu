@@ -2,6 +2,8 @@
 // every sub-chunk of a chunk in one launch; then offsets by a two-level scan and a gather.
 //
 // The per-symbol step lives in cg_coder.cuh.
+#include <type_traits>
+
 #include "cg_common.cuh"
 
 namespace cg {
@@ -19,7 +21,9 @@ struct EncodeParams {
 
 constexpr int kPrefetch = 8;  // symbols fetched ahead of the coder
 
-__global__ void __launch_bounds__(kGroup) encode_kernel(const EncodeParams p) {
+// NARROW: the symbols of a row lie within 4 GB of its first, so that a symbol's address is a 32-bit offset
+template <bool NARROW>
+__global__ void __launch_bounds__(kGroup, 10) encode_kernel(const EncodeParams p) {
     extern __shared__ uint32_t tab[];
     const int tid = threadIdx.x;
     const int row = blockIdx.y, sub = blockIdx.z;
@@ -39,31 +43,34 @@ __global__ void __launch_bounds__(kGroup) encode_kernel(const EncodeParams p) {
     BitSink out;
     out.init(p.scratch + slot * p.stride, p.stride);
 
-    const int8_t *sp = p.sym + row * p.s0 + static_cast<int64_t>(t0) * p.s1 + c * p.s2;
+    using Offset = typename std::conditional<NARROW, uint32_t, int64_t>::type;
+    const uint8_t *base = reinterpret_cast<const uint8_t *>(p.sym) + row * p.s0 + static_cast<int64_t>(t0) * p.s1;
+    const Offset s1 = static_cast<Offset>(p.s1);
+    Offset at = static_cast<Offset>(c * p.s2);
     EncoderState enc;
     enc.init();
     uint32_t largest = 0;  // the largest symbol met: one above maxsym is reported and coded as maxsym
 
     // whole groups of kPrefetch symbols: their loads are issued together, ahead of the coder, with no
     // bound checks; the last, shorter group goes symbol by symbol
-    const int64_t s1 = p.s1;
-    const uint8_t *sp8 = reinterpret_cast<const uint8_t *>(sp);
     const uint32_t top = static_cast<uint32_t>(maxsym);
-    int base = 0;
-    for (; base + kPrefetch <= n; base += kPrefetch) {
+    int i = 0;
+    for (; i + kPrefetch <= n; i += kPrefetch) {
         uint32_t buf[kPrefetch];
 #pragma unroll
-        for (int j = 0; j < kPrefetch; ++j) buf[j] = __ldg(sp8 + j * s1);
-        sp8 += kPrefetch * s1;
+        for (int j = 0; j < kPrefetch; ++j) {
+            buf[j] = __ldg(base + at);
+            at += s1;
+        }
 #pragma unroll
         for (int j = 0; j < kPrefetch; ++j) {
             largest = max(largest, buf[j]);
             enc.step(Smem{}, col, min(buf[j], top), top, out, lanes);
         }
     }
-    for (; base < n; ++base) {
-        const uint32_t s = __ldg(sp8);
-        sp8 += s1;
+    for (; i < n; ++i) {
+        const uint32_t s = __ldg(base + at);
+        at += s1;
         largest = max(largest, s);
         enc.step(Smem{}, col, min(s, top), top, out, lanes);
     }
@@ -170,42 +177,17 @@ __global__ void segment_offsets_kernel(const int64_t *totals, int nsub, int64_t 
 }
 
 // ---- gather (second half of collect_bytes, cachegen_encoder.py:210-222) ------------------------------------
-// One block per (group, row, sub-chunk).  Eight lanes copy one stream: its scratch row is read as
-// aligned 32-bit words (one per lane and step) and written byte by byte to where the stream goes
-// (streams lie back to back, so the destination has no alignment); a warp has four streams in flight
-// and a block sixteen, which is what hides the latency of these short dependent copies.
+// One block per (group, row, sub-chunk).  A stream longer than its row was truncated and reported by the encoder.
 __global__ void __launch_bounds__(kGroup) compact_kernel(const uint8_t *scratch, int64_t stride,
                                                          const int32_t *lengths, const int64_t *group_off,
                                                          const int64_t *sub_off, int nchannels,
                                                          uint8_t *bytes_out) {
-    __shared__ int warp_sums[kGroup / 32];
-    __shared__ int offs[kGroup];
-    __shared__ int lens[kGroup];
-    const int tid = threadIdx.x;
     const int row = blockIdx.y, sub = blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
-    const int c = blockIdx.x * kGroup + tid;
-    const int64_t slot0 = (static_cast<int64_t>(sub) * nrows + row) * nchannels + blockIdx.x * kGroup;
-    const int len = (c < nchannels) ? lengths[slot0 + tid] : 0;
-    const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
-    offs[tid] = excl;
-    lens[tid] = len;
-    __syncthreads();
+    const int c = blockIdx.x * kGroup + threadIdx.x;
+    const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
+    const int len = c < nchannels ? max(0, min(__ldg(lengths + slot), static_cast<int>(stride))) : 0;
     const int64_t gid = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
-    uint8_t *dst0 = bytes_out + sub_off[sub] + group_off[gid];
-    constexpr int kLanesPerStream = 8;
-    const int part = tid % kLanesPerStream;
-    for (int s = tid / kLanesPerStream; s < kGroup; s += kGroup / kLanesPerStream) {
-        const int n = min(lens[s], static_cast<int>(stride));  // a longer stream was truncated and reported by the encoder
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(scratch + (slot0 + s) * stride);
-        uint8_t *dst = dst0 + offs[s];
-        for (int j = part * 4; j < n; j += kLanesPerStream * 4) {
-            const uint32_t w = __ldg(src + (j >> 2));
-            dst[j] = static_cast<uint8_t>(w);
-            if (j + 1 < n) dst[j + 1] = static_cast<uint8_t>(w >> 8);
-            if (j + 2 < n) dst[j + 2] = static_cast<uint8_t>(w >> 16);
-            if (j + 3 < n) dst[j + 3] = static_cast<uint8_t>(w >> 24);
-        }
-    }
+    gather_run<1>(reinterpret_cast<const uint32_t *>(scratch + slot * stride), len, bytes_out + sub_off[sub] + group_off[gid]);
 }
 
 }  // namespace cg
@@ -214,8 +196,14 @@ using namespace cg;
 
 static int launch_encode(const EncodeParams &p, int nrows, int nsub, cudaStream_t st) {
     const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows, nsub);
-    const size_t smem = static_cast<size_t>(p.lp) * kRowBytes;
-    encode_kernel<<<grid, kGroup, smem, st>>>(p);
+    const size_t smem = even_waves_smem(static_cast<int64_t>(grid.x) * grid.y * grid.z, static_cast<size_t>(p.lp) * kRowBytes, 0);
+    const bool narrow = p.s1 >= 0 && p.s2 >= 0 && p.s1 <= 0xFFFFFFFF / (kSubTokens + 1) &&
+                        p.s1 * kSubTokens + p.s2 * p.nchannels <= 0xFFFFFFFF;
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(narrow ? encode_kernel<true> : encode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem));
+    if (narrow) encode_kernel<true><<<grid, kGroup, smem, st>>>(p);
+    else encode_kernel<false><<<grid, kGroup, smem, st>>>(p);
     return check_launch();
 }
 

@@ -148,10 +148,12 @@ __device__ __forceinline__ void counts_to_table(const uint32_t *hist, int max_bi
     for (int i = 0; i < max_bins; ++i) total += hist[i * kGroup + cl];
     total &= 0xFFFFu;  // the reference accumulates in uint16
     const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(max_bins);
+    const bool pow2 = (total & (total - 1u)) == 0u;
+    const int sh = 31 - __clz(static_cast<int>(total | 1u));
     uint32_t cum = 0;
     for (int i = 0; i <= max_bins; ++i) {
         if (i) cum = (cum + hist[(i - 1) * kGroup + cl]) & 0xFFFFu;
-        const uint32_t nv = total ? (scale * cum / total) : 0u;
+        const uint32_t nv = total ? (pow2 ? scale * cum >> sh : scale * cum / total) : 0u;
         out16[cl * lp + i] = static_cast<uint16_t>(nv + i);
     }
 }
@@ -326,8 +328,11 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_cdf_kernel(
     store_tables(out16, cdf_out, row, c0, C, lp, tid, kQuantThreads);
 }
 
-// calculate_cdf on int8 symbols with arbitrary strides: grid (nslab, nrows), 256 threads, thread
-// (channel = tid % 128, token parity = tid / 128).
+// calculate_cdf on int8 symbols: grid (nslab, nrows).  VEC: adjacent channels are adjacent bytes at 4-byte
+// boundaries, and a thread counts four channels of every eighth token, with one load for four symbols and
+// four tokens in flight; the lanes of a warp start their counts at different ones of their four channels so that they
+// hit 32 banks.  Otherwise (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
+template <bool VEC>
 __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t *__restrict__ sym, int64_t s0,
                                                                    int64_t s1, int64_t s2, int ntokens,
                                                                    int nchannels, int max_bins,
@@ -335,19 +340,49 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
     extern __shared__ uint32_t hist[];
     const int lp = max_bins + 1;
     uint16_t *out16 = reinterpret_cast<uint16_t *>(hist + lp * kGroup);
-    const int tid = threadIdx.x, cl = tid % kGroup, tsub = tid / kGroup;
-    const int row = blockIdx.y, c0 = blockIdx.x * kGroup, c = c0 + cl;
+    const int tid = threadIdx.x;
+    const int row = blockIdx.y, c0 = blockIdx.x * kGroup;
     for (int i = tid; i < lp * kGroup; i += kQuantThreads) hist[i] = 0u;
     __syncthreads();
-    if (c < nchannels) {
-        const int8_t *p = sym + row * s0 + c * s2;
-        for (int t = tsub; t < ntokens; t += kQuantThreads / kGroup) {
-            const uint32_t s = static_cast<uint8_t>(__ldg(p + t * s1));
-            atomicAdd(&hist[min(s, static_cast<uint32_t>(max_bins)) * kGroup + cl], 1u);
+    const uint32_t top = static_cast<uint32_t>(max_bins);
+    if (VEC) {
+        constexpr int kStep = kQuantThreads / 32, kAhead = 4;
+        const int q = tid & 31, c = c0 + 4 * q;
+        uint32_t place[4], pick[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t e = static_cast<uint32_t>(k + (q >> 3)) & 3u;
+            place[k] = smem_addr(hist + 4 * q + e);
+            pick[k] = 0x4440u + e;
+        }
+        if (c < nchannels) {
+            const int8_t *p = sym + row * s0 + c;
+            for (int t0 = tid >> 5; t0 < ntokens; t0 += kStep * kAhead) {
+                uint32_t w[kAhead];
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j)
+                    w[j] = t0 + j * kStep < ntokens ? __ldg(reinterpret_cast<const uint32_t *>(p + (t0 + j * kStep) * s1)) : 0u;
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j)
+                    if (t0 + j * kStep < ntokens) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(min(__byte_perm(w[j], 0u, pick[k]), top) * kRowBytes + place[k]) : "memory");
+                    }
+            }
+        }
+    } else {
+        const int cl = tid % kGroup, c = c0 + cl;
+        if (c < nchannels) {
+            const int8_t *p = sym + row * s0 + c * s2;
+            for (int t = tid / kGroup; t < ntokens; t += kQuantThreads / kGroup) {
+                const uint32_t s = static_cast<uint8_t>(__ldg(p + t * s1));
+                atomicAdd(&hist[min(s, top) * kGroup + cl], 1u);
+            }
         }
     }
     __syncthreads();
-    if (tid < kGroup && c < nchannels) counts_to_table(hist, max_bins, tid, out16);
+    if (tid < kGroup && c0 + tid < nchannels) counts_to_table(hist, max_bins, tid, out16);
     __syncthreads();
     store_tables(out16, cdf_out, row, c0, nchannels, lp, tid, kQuantThreads);
 }
@@ -368,7 +403,10 @@ extern "C" int cg_calculate_cdf(const int8_t *sym, const int64_t sym_strides[3],
     if (max_bins < 1 || max_bins >= CG_MAX_LP) return CG_E_LP;
     if (ntokens >= 65536) return CG_E_HIST;
     const dim3 grid((nchannels + kGroup - 1) / kGroup, nrows);
-    symbol_cdf_kernel<<<grid, kQuantThreads, hist_smem_bytes(max_bins), static_cast<cudaStream_t>(stream)>>>(
+    const bool vec = sym_strides[2] == 1 && nchannels % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(sym) | static_cast<uintptr_t>(sym_strides[0]) | static_cast<uintptr_t>(sym_strides[1])) & 3) == 0;
+    const auto kernel = vec ? symbol_cdf_kernel<true> : symbol_cdf_kernel<false>;
+    kernel<<<grid, kQuantThreads, hist_smem_bytes(max_bins), static_cast<cudaStream_t>(stream)>>>(
         sym, sym_strides[0], sym_strides[1], sym_strides[2], ntokens, nchannels, max_bins, cdf_out);
     return check_launch();
 }

@@ -539,79 +539,22 @@ struct GatherTargets {
     void *lengths[kGatherSubs];  // int32 or uint16 [nrows, C]
 };
 
-// One block per (group, row, sub-chunk), one thread per stream.  A warp's streams are one run of the output: each
-// lane shifts its words to the byte they start at and puts them together in shared memory (a word that two
-// streams share by an atomic or), and the warp writes the run with 128-bit stores.  Copying stream after stream
-// to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
-// with words assembled from two source words 24 us: one short dependent copy after the other.
-constexpr int kGatherWords = 1536;  // words of shared memory a warp; longer runs take the lanes' own byte stores
+// The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.
 template <class Len, bool INTERLEAVED>
 __global__ void __launch_bounds__(kGroup) gather_kernel(const uint8_t *__restrict__ scratch, int64_t stride,
                                                         const int32_t *__restrict__ lengths,
                                                         const int64_t *__restrict__ group_off, int nchannels, int sub0,
                                                         const __grid_constant__ GatherTargets out) {
-    __shared__ uint4 stage[kGroup / 32][kGatherWords / 4];
-    __shared__ int warp_sums[kGroup / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int row = blockIdx.y, sub = sub0 + blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
     const int c = blockIdx.x * kGroup + tid;
     const int64_t group = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
     const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
-    int len = c < nchannels ? __ldg(lengths + slot) : 0;
-    const int64_t at = __ldg(group_off + group);
+    const int len = c < nchannels ? __ldg(lengths + slot) : 0;
     if (c < nchannels) static_cast<Len *>(out.lengths[blockIdx.z])[static_cast<int64_t>(row) * nchannels + c] = static_cast<Len>(len);
-    len = min(len, static_cast<int>(stride));  // a longer stream was truncated and reported by the encoder
-    const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
-    const int first = __shfl_sync(0xFFFFFFFFu, excl, 0);
-    const int total = __shfl_sync(0xFFFFFFFFu, excl + len, 31) - first;
-    uint8_t *dst = out.bytes[blockIdx.z] + at + first;
     const uint32_t *src = INTERLEAVED ? scratch_word(const_cast<uint8_t *>(scratch), stride, group, tid)
                                       : reinterpret_cast<const uint32_t *>(scratch + slot * stride);
-    constexpr int kStep = INTERLEAVED ? 32 : 1;
-    const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 15u);
-    const int nw = (len + 3) >> 2;
-    if (mis + total > kGatherWords * 4) {
-        uint8_t *d = dst + (excl - first);
-        for (int k = 0; k < len; ++k) d[k] = static_cast<uint8_t>(__ldg(src + (k >> 2) * kStep) >> (8 * (k & 3)));
-        return;
-    }
-    uint32_t *st = reinterpret_cast<uint32_t *>(stage[warp]);
-    const int units = (mis + total + 15) >> 4;
-    for (int i = lane; i < units; i += 32) stage[warp][i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncwarp();
-    const int o = mis + excl - first, w = o >> 2;
-    const uint32_t sh = static_cast<uint32_t>(o & 3) * 8u;
-    const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
-    constexpr int kAhead = 8;  // loads in flight
-    uint32_t prev = 0u;
-    for (int k0 = 0; k0 < most; k0 += kAhead) {
-        uint32_t x[kAhead];
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) x[j] = k0 + j < nw ? __ldg(src + (k0 + j) * kStep) : 0u;
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) {
-            const int k = k0 + j;
-            if (k < nw) {
-                const uint32_t v = __funnelshift_l(prev, x[j], sh);
-                if (k == 0 || k == nw - 1) atomicOr(st + w + k, v);
-                else st[w + k] = v;
-                prev = x[j];
-            }
-        }
-    }
-    // what the shift pushed past the last word; a stream's bytes past its end are zero
-    const uint32_t over = __funnelshift_l(prev, 0u, sh);
-    if (over) atomicOr(st + w + nw, over);
-    __syncwarp();
-    uint4 *d16 = reinterpret_cast<uint4 *>(dst - mis);
-    for (int i = lane; i < units; i += 32) {
-        if (i * 16 >= mis && i * 16 + 16 <= mis + total) {
-            d16[i] = stage[warp][i];
-        } else {
-            const uint8_t *b = reinterpret_cast<const uint8_t *>(stage[warp]);
-            for (int k = max(i * 16, mis); k < min(i * 16 + 16, mis + total); ++k) (dst - mis)[k] = b[k];
-        }
-    }
+    gather_run<INTERLEAVED ? 32 : 1>(src, min(len, static_cast<int>(stride)), out.bytes[blockIdx.z] + __ldg(group_off + group));
 }
 
 // Header, scales and the sparse tables' group offsets of a container (flat_format.py) to their places.
@@ -636,15 +579,9 @@ __global__ void __launch_bounds__(256) flat_front_kernel(const __grid_constant__
     }
 }
 
-}  // namespace cg
-
-using namespace cg;
-
-namespace {
-
 constexpr int64_t kSmemPerSM = 228 * 1024, kSmemPerBlock = 227 * 1024, kSmemReserved = 1024;
 
-int sm_count() {
+static int sm_count() {
     static int count[64];  // per device; a racing first call writes the same number
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
@@ -671,6 +608,13 @@ size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes) {
     if (padded > kSmemPerBlock - static_cast<int64_t>(static_bytes)) padded = kSmemPerBlock - static_cast<int64_t>(static_bytes);
     return padded > static_cast<int64_t>(dynamic) ? static_cast<size_t>(padded) : dynamic;
 }
+
+}  // namespace cg
+
+using namespace cg;
+
+namespace {
+
 
 template <class K>
 void allow_smem(K kernel, size_t bytes) {
@@ -833,8 +777,12 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
 
 extern "C" int cg_encode_kv_wait(const cg_encode_kv_job *job, void *stream) {
     if (!job || !job->tail) return CG_E_NULL;
-    const int nsub = (job->ntokens + kSubTokens - 1) / kSubTokens;
-    volatile int64_t *flag = job->tail + nsub + 3;
+    return cg_wait_word(job->tail + (job->ntokens + kSubTokens - 1) / kSubTokens + 3, stream);
+}
+
+extern "C" int cg_wait_word(const int64_t *word, void *stream) {
+    if (!word) return CG_E_NULL;
+    const volatile int64_t *flag = word;
     for (;;) {
         for (int spin = 0; spin < 2000; ++spin)
             if (*flag) {

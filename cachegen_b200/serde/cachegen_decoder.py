@@ -79,9 +79,7 @@ def recombine_bytes(bytes_tensor: torch.Tensor, output_lengths: torch.Tensor) ->
 @_lmcache_nvtx_annotate
 def decode_chunk(cdf: torch.Tensor, data_chunk: CacheGenGPUBytestream, target_buffer: torch.Tensor) -> None:
     """Symbols of one sub-chunk into target_buffer [2L, ntokens, C] uint8, strided ok (dec.py:53-75)."""
-    lengths = data_chunk.bytestream_lengths
-    length_prefsum = lengths.flatten().cumsum(0).reshape(lengths.shape)
-    torchac_cuda.decode_fast_prefsum(cdf, data_chunk.bytestream, length_prefsum, target_buffer)
+    torchac_cuda.decode_by_lengths(cdf, data_chunk.bytestream, data_chunk.bytestream_lengths, target_buffer)
 
 
 @_lmcache_nvtx_annotate

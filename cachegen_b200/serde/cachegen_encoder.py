@@ -18,6 +18,7 @@ import collections
 import contextlib
 import ctypes
 import dataclasses
+import functools
 import threading
 import weakref
 from typing import Tuple
@@ -89,6 +90,11 @@ def concat_max(max1) -> torch.Tensor:
 def collect_bytes(output_buffer: torch.Tensor, output_lengths: torch.Tensor) -> torch.Tensor:
     """The first output_lengths[r, c] bytes of every row output_buffer[r, c, :], back to back in
     (r, c) order, as one uint8 tensor (enc.py:210-222), on the offset and compaction kernels."""
+    return _collect(output_buffer, output_lengths)[0]
+
+
+def _collect(output_buffer: torch.Tensor, output_lengths: torch.Tensor, status: torch.Tensor = None):
+    """collect_bytes with one wait, for the total size; also returns the status word as it then is."""
     if output_buffer.dim() != 3 or output_buffer.dtype != torch.uint8 or not output_buffer.is_cuda:
         raise TypeError("expected a CUDA uint8 buffer [nlayers, nchannels, row]")
     buf, lengths = output_buffer.contiguous(), output_lengths.to(torch.int32).contiguous()
@@ -96,26 +102,38 @@ def collect_bytes(output_buffer: torch.Tensor, output_lengths: torch.Tensor) -> 
     if tuple(lengths.shape) != (NL, C):
         raise RuntimeError("output_lengths must have shape [nlayers, nchannels]")
     dev = buf.device
-    total, outside = torch.stack((lengths.sum(dtype=torch.int64),
-                                  ((lengths < 0) | (lengths > stride)).sum(dtype=torch.int64))).tolist()
-    if outside:
-        raise RuntimeError("collect_bytes: a length is negative or exceeds the buffer's row size")
     nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
-    group_off = torch.empty(NL * nslab, dtype=torch.int64, device=dev)
-    sub_off = torch.tensor([0, total], dtype=torch.int64, device=dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    out = torch.empty(total, dtype=torch.uint8, device=dev)
-    job = _lib.DecodeJob()
-    job.lengths, job.nbytes, job.length_kind = lengths.data_ptr(), total, _lib.CG_LENGTHS_I32
-    with torch.cuda.device(dev):
-        rc = _lib.lib().cg_decode_offsets((_lib.DecodeJob * 1)(job), 1, NL, C, _ptr(group_off), _ptr(status), _stream(dev))
-        _lib.check(rc, "cg_decode_offsets")
-        rc = _lib.lib().cg_compact_streams(_ptr(buf), stride, _ptr(lengths), _ptr(group_off), _ptr(sub_off), 1, NL, C,
-                                           _ptr(out), _stream(dev))
-        _lib.check(rc, "cg_compact_streams")
-    if int(status.item()):
-        raise RuntimeError("collect_bytes: " + _lib.status_text(int(status.item())))
-    return out
+    offsets = torch.empty(NL * nslab, dtype=torch.int64, device=dev)
+    lib, stream = _lib.lib(), _stream(dev)
+    with _current(dev):
+        if NL * nslab <= _lib.CG_MAX_OFFSET_GROUPS:
+            tail = _take_tail(4)
+            rc = lib.cg_stream_sizes(_ptr(lengths), NL, C, min(stride, 1 << 20),
+                                     None if status is None else status.data_ptr(), offsets.data_ptr(), tail.data_ptr(), stream)
+            if rc == 0:
+                rc = lib.cg_wait_word(tail.data_ptr() + 24, stream)
+            total, outside, bits, _ = tail[:4].tolist()
+            _give_tail(tail)
+        else:
+            total, outside, bits = torch.stack((lengths.sum(dtype=torch.int64),
+                                                ((lengths < 0) | (lengths > stride)).sum(dtype=torch.int64),
+                                                lengths.new_zeros((), dtype=torch.int64) if status is None else status[0].to(torch.int64))).tolist()
+            job = _lib.DecodeJob()
+            job.lengths, job.nbytes, job.length_kind = lengths.data_ptr(), total, _lib.CG_LENGTHS_I32
+            rc = lib.cg_decode_offsets((_lib.DecodeJob * 1)(job), 1, NL, C, _ptr(offsets), None, stream)
+        _lib.check(rc, "cg_stream_sizes")
+        if outside:
+            raise RuntimeError("collect_bytes: a length is negative or exceeds the buffer's row size")
+        out = torch.empty(total, dtype=torch.uint8, device=dev)
+        rc = lib.cg_compact_streams(_ptr(buf), stride, _ptr(lengths), _ptr(offsets), _ptr(_zero(dev)), 1, NL, C, _ptr(out), stream)
+    _lib.check(rc, "cg_compact_streams")
+    return out, bits
+
+
+@functools.lru_cache(maxsize=64)
+def _zero(dev) -> torch.Tensor:
+    """The offset of an only sub-chunk."""
+    return torch.zeros(1, dtype=torch.int64, device=dev)
 
 
 @_lmcache_nvtx_annotate
@@ -124,8 +142,16 @@ def encode_ntokens(cdf_int: torch.Tensor, encode_input: torch.Tensor, output_buf
     """encode_fast_new into the caller's buffers, then collect_bytes (enc.py:225-242)."""
     from .. import torchac_cuda
     torchac_cuda.encode_fast_new(cdf_int, encode_input, output_buffer, output_lengths)
-    torchac_cuda.check_status(cdf_int.device)
-    return collect_bytes(output_buffer, output_lengths)
+    status = torchac_cuda._status_word(cdf_int.device)
+    # a stream that outgrew its row has a length that collect_bytes would refuse: the status comes first
+    try:
+        out, bits = _collect(output_buffer, output_lengths, status)
+    except RuntimeError:
+        torchac_cuda.check_status(cdf_int.device)
+        raise
+    if bits:
+        torchac_cuda.check_status(cdf_int.device)
+    return out
 
 
 def row_scales(kv: torch.Tensor) -> torch.Tensor:

@@ -144,7 +144,8 @@ def decode_fast_new(cdf: torch.Tensor, bytestreams: torch.Tensor, lengths: torch
     _lib.check(rc, "decode_fast_new")
 
 
-def _decode_prefsum(entry: str, cdf, bytestreams, lengths_prefsum, output) -> None:
+def _check_packed(cdf, bytestreams, lengths_prefsum, output):
+    """The checks of the calls on back-to-back streams; returns (ntokens, lp)."""
     _check(cdf.is_cuda, "CDF should be on GPU")
     _check(bytestreams.is_cuda, "Bytestreams should be on GPU")
     _check(lengths_prefsum.is_cuda, "Lengths should be on GPU")
@@ -163,8 +164,14 @@ def _decode_prefsum(entry: str, cdf, bytestreams, lengths_prefsum, output) -> No
     _check(lp <= MAX_LP_DECODE, f"CDF should have at most{MAX_LP_DECODE}Lps")
     _check(cdf.is_contiguous() and bytestreams.is_contiguous() and lengths_prefsum.is_contiguous(),
            "cdf, bytestreams and lengths must be contiguous")
-    _check(lengths_prefsum.dtype == torch.int64 and cdf.dtype == torch.int16 and bytestreams.dim() == 1,
-           "expected int16 cdf, 1-D bytestreams and int64 prefix sums")
+    _check(cdf.dtype == torch.int16 and bytestreams.dim() == 1, "expected int16 cdf, 1-D bytestreams and int64 prefix sums")
+    return ntokens, lp
+
+
+def _decode_prefsum(entry: str, cdf, bytestreams, lengths_prefsum, output) -> None:
+    ntokens, lp = _check_packed(cdf, bytestreams, lengths_prefsum, output)
+    nlayers, nchannels = cdf.shape[0], cdf.shape[1]
+    _check(lengths_prefsum.dtype == torch.int64, "expected int16 cdf, 1-D bytestreams and int64 prefix sums")
     status = _status_word(cdf.device)
     with torch.cuda.device(cdf.device):
         rc = getattr(_lib.lib(), entry)(_ptr(cdf), _ptr(bytestreams), bytestreams.numel(), _ptr(lengths_prefsum),
@@ -179,6 +186,24 @@ def decode_fast_prefsum(cdf: torch.Tensor, bytestreams: torch.Tensor, lengths_pr
     uint8 symbols [nlayers, ntokens, nchannels], strided output allowed
     (torchac_kernel_dec_new.cu:403-479)."""
     _decode_prefsum("cg_decode_prefsum", cdf, bytestreams, lengths_prefsum, output)
+
+
+def decode_by_lengths(cdf: torch.Tensor, bytestreams: torch.Tensor, lengths: torch.Tensor,
+                      output: torch.Tensor) -> None:
+    """decode_fast_prefsum with the lengths themselves (any integer type, [nlayers, nchannels]) in place of their
+    prefix sum, which the kernels make (no counterpart in the reference's module)."""
+    nlayers, nchannels = cdf.shape[0], cdf.shape[1]
+    groups = nlayers * ((nchannels + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS)
+    if lengths.dtype != torch.int32 or not lengths.is_contiguous() or not lengths.is_cuda or groups > _lib.CG_MAX_OFFSET_GROUPS:
+        decode_fast_prefsum(cdf, bytestreams, lengths.flatten().cumsum(0).reshape(lengths.shape), output)
+        return
+    ntokens, lp = _check_packed(cdf, bytestreams, lengths, output)
+    group_off = torch.empty(groups, dtype=torch.int64, device=cdf.device)
+    with torch.cuda.device(cdf.device):
+        rc = _lib.lib().cg_decode_packed(_ptr(cdf), _ptr(bytestreams), bytestreams.numel(), _ptr(lengths), _ptr(group_off),
+                                         _ptr(output), _lib.strides3(output), nlayers, ntokens, nchannels, lp,
+                                         _ptr(_status_word(cdf.device)), _stream(cdf))
+    _lib.check(rc, "decode_by_lengths")
 
 
 def decode_fast_prefsum_warp(cdf: torch.Tensor, bytestreams: torch.Tensor, lengths_prefsum: torch.Tensor,

@@ -45,6 +45,8 @@ extern "C" {
 #define CG_STREAM_CAPACITY(ntokens) (2 * (ntokens) + 8)
 /* channels of one row handled by one thread block (one thread per stream) */
 #define CG_GROUP_CHANNELS 128
+/* 128-channel groups (all rows) whose offsets one cluster of blocks can hold */
+#define CG_MAX_OFFSET_GROUPS 96000
 /* sub-chunks one fused decode launch can take */
 #define CG_MAX_DECODE_JOBS 40
 
@@ -429,6 +431,21 @@ int cg_decode_dequant_static(const cg_decode_job *jobs_host, int njobs, int nlay
 int cg_decode_kv(const cg_decode_job *jobs_host, int njobs, int nlayers, int nheads, int head_size, int lp,
                  const float *bins, int delta_group, const float *res_bins, int scale_dtype, int out_dtype,
                  int64_t o_layer, int64_t o_kv, int64_t o_token, int64_t o_head, int32_t *status, void *stream);
+
+/*
+ * Streams back to back, located by their int32 lengths [nrows, nchannels] alone (no prefix sum; at most
+ * CG_MAX_OFFSET_GROUPS groups).  cg_stream_sizes: offsets of the groups, and for the host (tail: int64 [4], host memory
+ * the GPU can write) [0] the sum of the lengths, [1] 1 if one is negative or above `longest` (<= 2^20), [2] the word at
+ * `extra` (may be NULL), then [3] becomes 1 (cg_wait_word).  cg_decode_packed: cg_decode_prefsum's symbols;
+ * group_off: room for nrows * ceil(nchannels/128) int64.
+ */
+int cg_stream_sizes(const int32_t *lengths, int nrows, int nchannels, int longest, const int32_t *extra,
+                    int64_t *group_off_out, int64_t *tail, void *stream);
+int cg_decode_packed(const int16_t *cdf, const uint8_t *bytes, int64_t nbytes, const int32_t *lengths,
+                     int64_t *group_off, uint8_t *out, const int64_t out_strides[3], int nrows, int ntokens,
+                     int nchannels, int lp, int32_t *status, void *stream);
+/* returns when the word, host memory that a kernel on `stream` writes, is not 0; CG_E_CUDA if the stream failed before */
+int cg_wait_word(const int64_t *word_host, void *stream);
 
 /* ------------------------------------------------------------------------------------------
  * byte strings in host memory
