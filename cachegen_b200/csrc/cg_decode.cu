@@ -20,6 +20,50 @@ enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
 __device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---- table staging by the block --------------------------------------------------------------------------
+// The int16 tables of a block's 128 channels are one contiguous run.  Read channel by channel they are 2-byte
+// loads 66 bytes apart, 66 of them one after the other in a thread; here the run is copied to the upper part
+// of the table area with 16-byte asynchronous copies and spread into columns from there: the rows below it at
+// once, the rest from registers once every thread has read its part.
+__device__ __forceinline__ void copy_run_async(void *smem, const void *global, int bytes, int tid, int nthreads) {
+    const uint32_t d = smem_addr(smem);
+    for (int i = tid * 16; i < bytes; i += nthreads * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + i), "l"(static_cast<const char *>(global) + i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+constexpr int kMaxStagedLp = 33;  // longer tables would need more registers than the decode loop has
+__device__ __forceinline__ int staged_run_offset(int lp, int rows) { return rows * kRowBytes - lp * kGroup * 2; }
+// Thread t's channels are 2t and 2t + 1, in columns t and t + 64.  rows: the columns' rows, filled up with the last
+// entry.  Called by all threads.
+__device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int tid) {
+    constexpr int kHold = (kMaxStagedLp + 1) / 2;
+    const int off = staged_run_offset(lp, rows), below = off / kRowBytes, n = lp - 1;
+    const uint16_t *run = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(tab) + off) + 2 * tid * lp;
+    uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
+    const int direct = min(n, below);
+    for (int m = 0; m < direct; ++m) {
+        c0[m * kGroup] = static_cast<uint32_t>(run[m]) << 16;
+        c1[m * kGroup] = static_cast<uint32_t>(run[lp + m]) << 16;
+    }
+    uint32_t hold[kHold];
+#pragma unroll
+    for (int k = 0; k < kHold; ++k)
+        hold[k] = direct + k < n ? static_cast<uint32_t>(run[direct + k]) | static_cast<uint32_t>(run[lp + direct + k]) << 16 : 0u;
+    const uint32_t last0 = static_cast<uint32_t>(run[n - 1]) << 16, last1 = static_cast<uint32_t>(run[lp + n - 1]) << 16;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kHold; ++k)
+        if (direct + k < n) {
+            c0[(direct + k) * kGroup] = hold[k] << 16;
+            c1[(direct + k) * kGroup] = hold[k] & 0xFFFF0000u;
+        }
+    for (int m = n; m < rows; ++m) {
+        c0[m * kGroup] = last0;
+        c1[m * kGroup] = last1;
+    }
+}
+
 // ---- symbol-output kernels (decode_fast_prefsum / decode_fast_new) -----------------------------------
 struct SymDecodeParams {
     const int16_t *cdf;
@@ -85,6 +129,86 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
                                 lanes, emit);
 }
 
+// The same with two adjacent channels per thread, whose symbols are adjacent bytes (see decode_dequant_multi_kernel):
+// 64 threads a block, one 16-bit store a token.
+// Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
+// more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
+constexpr int kMultiBlocksPerSM = 12;
+template <int LEVELS, int MODE>
+__global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_pair_kernel(const SymDecodeParams p) {
+    extern __shared__ uint32_t tab[];
+    __shared__ int warp_sums[kGroup / 64];
+    constexpr int kThreads = kGroup / 2;
+    const int tid = threadIdx.x;
+    const int row = blockIdx.y, c0 = blockIdx.x * kGroup + 2 * tid;
+    const bool active = c0 < p.nchannels;  // nchannels is even
+    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, active);
+    const int64_t g = static_cast<int64_t>(row) * p.nchannels + c0;
+    const int rows = table_rows(p.lp, LEVELS) + 1;
+    const bool run_staged = p.lp <= kMaxStagedLp && (p.nchannels & 7) == 0 && (reinterpret_cast<uintptr_t>(p.cdf) & 15) == 0 &&
+                            static_cast<int>((blockIdx.x + 1) * kGroup) <= p.nchannels;
+    if (run_staged)
+        copy_run_async(reinterpret_cast<char *>(tab) + staged_run_offset(p.lp, rows),
+                       p.cdf + (static_cast<int64_t>(row) * p.nchannels + blockIdx.x * kGroup) * p.lp, p.lp * kGroup * 2, tid, kThreads);
+    int64_t start[2] = {0, 0}, len[2] = {0, 0};
+    if (MODE == 0) {
+        if (active) {
+            const int64_t a = g ? p.prefsum[g - 1] : 0, b = p.prefsum[g], e = p.prefsum[g + 1];
+            start[0] = a;
+            len[0] = b - a;
+            start[1] = b;
+            len[1] = e - b;
+        }
+    } else if (MODE == 1) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            start[i] = (g + i) * p.stream_stride;
+            len[i] = active ? min(static_cast<int64_t>(p.lengths[g + i]), p.stream_stride) : 0;
+        }
+    } else {
+        if (active) {
+            len[0] = max(0, min(__ldg(p.lengths + g), 1 << 20));
+            len[1] = max(0, min(__ldg(p.lengths + g + 1), 1 << 20));
+        }
+        const int excl = block_exclusive_scan<kGroup / 64>(static_cast<int>(len[0] + len[1]), warp_sums, tid, nullptr);
+        wait_for_launch_before();
+        start[0] = __ldg(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
+        start[1] = start[0] + len[0];
+    }
+    if (run_staged) {
+        wait_copies();
+        __syncthreads();
+        spread_run(tab, p.lp, rows, tid);
+    } else if (active) {
+        stage_table_column<true>(tab, p.cdf + g * p.lp, p.lp, rows, tid);
+        stage_table_column<true>(tab, p.cdf + (g + 1) * p.lp, p.lp, rows, tid + kThreads);
+    }
+    if (!active) return;  // a thread reads its own columns only
+    bool bad = false;
+    const uint8_t *streams[2];
+    uint32_t lens[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        if (len[i] < 0) { len[i] = 0; bad = true; }
+        if (start[i] < 0) { start[i] = 0; len[i] = 0; bad = true; }
+        if (start[i] > p.nbytes) { start[i] = p.nbytes; bad = true; }
+        if (start[i] + len[i] > p.nbytes) { len[i] = p.nbytes - start[i]; bad = true; }
+        if (len[i] > (1 << 20)) len[i] = 1 << 20;
+        streams[i] = p.bytes + start[i];
+        lens[i] = static_cast<uint32_t>(len[i]);
+    }
+    if (bad && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
+    uint8_t *o = p.out + row * p.o0 + c0;
+    int64_t o1 = p.o1;
+    asm volatile("" : "+l"(o1));
+    const uint32_t col[2] = {smem_addr(tab + tid), smem_addr(tab + tid + kThreads)};
+    auto emit = [&](const uint32_t (&a)[2], uint32_t) {
+        *reinterpret_cast<uint16_t *>(o) = static_cast<uint16_t>((a[0] - col[0]) / kRowBytes | (a[1] - col[1]) / kRowBytes << 8);
+        o += o1;
+    };
+    decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
+}
+
 // ---- one warp per stream (kept for comparison) -------------------------------------------------------------
 // The layout usually drawn for a GPU arithmetic decoder: a warp owns one stream, lane m holds table
 // entry m in a register, a ballot over "(span * cdf[m]) >> 16 <= value - low" finds the symbol and two
@@ -141,50 +265,6 @@ struct FusedDecodeParams {
     int after;  // see DecodeAfter
     cg_decode_job jobs[CG_MAX_DECODE_JOBS];
 };
-
-// ---- table staging by the block --------------------------------------------------------------------------
-// The int16 tables of a block's 128 channels are one contiguous run.  Read channel by channel they are 2-byte
-// loads 66 bytes apart, 66 of them one after the other in a thread; here the run is copied to the upper part
-// of the table area with 16-byte asynchronous copies and spread into columns from there: the rows below it at
-// once, the rest from registers once every thread has read its part.
-__device__ __forceinline__ void copy_run_async(void *smem, const void *global, int bytes, int tid, int nthreads) {
-    const uint32_t d = smem_addr(smem);
-    for (int i = tid * 16; i < bytes; i += nthreads * 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + i), "l"(static_cast<const char *>(global) + i) : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-constexpr int kMaxStagedLp = 33;  // longer tables would need more registers than the decode loop has
-__device__ __forceinline__ int staged_run_offset(int lp, int rows) { return rows * kRowBytes - lp * kGroup * 2; }
-// Thread t's channels are 2t and 2t + 1, in columns t and t + 64.  rows: the columns' rows, filled up with the last
-// entry.  Called by all threads.
-__device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int tid) {
-    constexpr int kHold = (kMaxStagedLp + 1) / 2;
-    const int off = staged_run_offset(lp, rows), below = off / kRowBytes, n = lp - 1;
-    const uint16_t *run = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(tab) + off) + 2 * tid * lp;
-    uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
-    const int direct = min(n, below);
-    for (int m = 0; m < direct; ++m) {
-        c0[m * kGroup] = static_cast<uint32_t>(run[m]) << 16;
-        c1[m * kGroup] = static_cast<uint32_t>(run[lp + m]) << 16;
-    }
-    uint32_t hold[kHold];
-#pragma unroll
-    for (int k = 0; k < kHold; ++k)
-        hold[k] = direct + k < n ? static_cast<uint32_t>(run[direct + k]) | static_cast<uint32_t>(run[lp + direct + k]) << 16 : 0u;
-    const uint32_t last0 = static_cast<uint32_t>(run[n - 1]) << 16, last1 = static_cast<uint32_t>(run[lp + n - 1]) << 16;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kHold; ++k)
-        if (direct + k < n) {
-            c0[(direct + k) * kGroup] = hold[k] << 16;
-            c1[(direct + k) * kGroup] = hold[k] & 0xFFFF0000u;
-        }
-    for (int m = n; m < rows; ++m) {
-        c0[m * kGroup] = last0;
-        c1[m * kGroup] = last1;
-    }
-}
 
 template <int LEVELS, int SCALE_DT, int OUT_DT>
 __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_constant__ FusedDecodeParams p) {
@@ -312,10 +392,6 @@ __device__ __forceinline__ uint32_t pack_pair<CG_BF16>(float v0, float v1) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
-
-// Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
-// more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
-constexpr int kMultiBlocksPerSM = 12;
 
 // DELTA (anchor-token delta, see cg_decode_dequant_delta): in rows with residual bins every token that is
 // not the first of its group of delta_group adds its value, ((sym - Cq_a) / Cq_r) * max, to its
@@ -560,7 +636,10 @@ template <int MODE>
 static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) {
     const int need = search_levels(p.lp);
     const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows);
-#define CG_LAUNCH_SYM(L) return launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
+    const bool pairs = p.o2 == 1 && ((p.o0 | p.o1 | p.nchannels) & 1) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 1) == 0;
+#define CG_LAUNCH_SYM(L)                                                                                      \
+    return pairs ? launch(decode_symbols_pair_kernel<L, MODE>, grid, kGroup / 2, table_bytes(p.lp, L), MODE == 2, st, p) \
+                 : launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
     if (need <= 3) CG_LAUNCH_SYM(3);
     if (need == 4) CG_LAUNCH_SYM(4);
     if (need == 5) CG_LAUNCH_SYM(5);
@@ -640,27 +719,44 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
     // four lengths a load where the rows allow it
     const bool vec = nchannels % kGroup == 0 && (reinterpret_cast<uintptr_t>(lengths) & (u16 ? 7 : 15)) == 0;
     bool bad = false;
-    for (int k = warp; k < count; k += kOffsetThreads / 32) {
-        const int gid = first + k;
-        int s = 0;
-        if (vec) {
-            if (u16) {
-                const ushort4 q = __ldg(static_cast<const ushort4 *>(lengths) + static_cast<int64_t>(gid) * 32 + lane);
-                s = q.x + q.y + q.z + q.w;
-            } else {
-                const int4 q = __ldg(static_cast<const int4 *>(lengths) + static_cast<int64_t>(gid) * 32 + lane);
-                s = clamped_length(q.x, sizes.longest, &bad) + clamped_length(q.y, sizes.longest, &bad) + clamped_length(q.z, sizes.longest, &bad) + clamped_length(q.w, sizes.longest, &bad);
+    constexpr int kWarps = kOffsetThreads / 32, kAhead = 4;  // groups a warp has in flight
+    if (vec) {
+        for (int k0 = warp; k0 < count; k0 += kWarps * kAhead) {
+            int s[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const int k = k0 + i * kWarps;
+                const int64_t at = static_cast<int64_t>(first + k) * 32 + lane;
+                int4 q = make_int4(0, 0, 0, 0);
+                if (k < count) {
+                    if (u16) {
+                        const ushort4 h = __ldg(static_cast<const ushort4 *>(lengths) + at);
+                        q = make_int4(h.x, h.y, h.z, h.w);
+                    } else {
+                        q = __ldg(static_cast<const int4 *>(lengths) + at);
+                    }
+                }
+                s[i] = clamped_length(q.x, sizes.longest, &bad) + clamped_length(q.y, sizes.longest, &bad) +
+                       clamped_length(q.z, sizes.longest, &bad) + clamped_length(q.w, sizes.longest, &bad);
             }
-        } else {
-            const int row = gid / nslab, slab = gid % nslab;
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                s[i] = __reduce_add_sync(0xFFFFFFFFu, s[i]);
+                if (lane == 0 && k0 + i * kWarps < count) sums[k0 + i * kWarps] = s[i];
+            }
+        }
+    } else {
+        for (int k = warp; k < count; k += kWarps) {
+            const int row = (first + k) / nslab, slab = (first + k) % nslab;
+            int s = 0;
             for (int c = slab * kGroup + lane; c < min(nchannels, (slab + 1) * kGroup); c += 32) {
                 const int64_t at = static_cast<int64_t>(row) * nchannels + c;
                 s += clamped_length(u16 ? static_cast<int>(__ldg(static_cast<const uint16_t *>(lengths) + at))
                                         : __ldg(static_cast<const int32_t *>(lengths) + at), sizes.longest, &bad);
             }
+            s = __reduce_add_sync(0xFFFFFFFFu, s);
+            if (lane == 0) sums[k] = s;
         }
-        s = __reduce_add_sync(0xFFFFFFFFu, s);
-        if (lane == 0) sums[k] = s;
     }
     __syncthreads();
     if (bad) block_bad = 1u;

@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(kGroup) compact_kernel(const uint8_t *scratch,
     const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
     const int len = c < nchannels ? max(0, min(__ldg(lengths + slot), static_cast<int>(stride))) : 0;
     const int64_t gid = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
-    gather_run<1>(reinterpret_cast<const uint32_t *>(scratch + slot * stride), len, bytes_out + sub_off[sub] + group_off[gid]);
+    gather_run<1>(reinterpret_cast<const uint32_t *>(scratch + slot * stride), len, bytes_out + sub_off[sub] + group_off[gid],
+                  ((reinterpret_cast<uintptr_t>(scratch) | static_cast<uintptr_t>(stride)) & 7) == 0);
 }
 
 }  // namespace cg
