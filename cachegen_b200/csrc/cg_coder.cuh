@@ -208,7 +208,8 @@ struct BitWindow {
     CG_HD bool low_water() const { return nbits <= 32; }
     // fewer valid bits than one symbol can take: a range update shifts by at most 18 bits when the
     // table is strictly increasing (the updated interval spans at least 2^14 values)
-    CG_HD bool short_of_bits() const { return nbits < 18; }
+    static constexpr int kShort = 18;
+    CG_HD bool short_of_bits() const { return nbits < kShort; }
     // Tops the window up with the whole words that fit (none above 64 valid bits, one above 32, two
     // otherwise), straight-line: every lane of the warp runs the same instructions whatever it needs.
     CG_HD void refill() {
@@ -362,9 +363,13 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     // its scaled bounds; the range update below is shared.
     const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
     uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
+#if defined(__CUDA_ARCH__)
+#pragma unroll 2
+#endif
     for (; t4 != last4; t4 += 4u) {
         uint32_t flo[NS], fhi[NS], ratio[NS];
-        bool rare = false;  // a lane short of bits, or a symbol that fails the check
+        bool rare = false;  // a symbol that fails the check
+        int fewest = bw[0].nbits;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
@@ -390,10 +395,11 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
         for (int i = 0; i < NS; ++i) {
             flo[i] = cg_umulhi(st[i].span32, e0[i]);
             fhi[i] = cg_umulhi(st[i].span32, e1[i]);
-            rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]) | bw[i].short_of_bits();
+            rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]);
+            fewest = fewest < bw[i].nbits ? fewest : bw[i].nbits;
             if (!LAST_REPEATED) rare = rare | (a[i] >= det);
         }
-        if (cg_any_lane(lanes, rare)) {
+        if (cg_any_lane(lanes, rare | (fewest < BitWindow::kShort))) {
             bool low = false, odd = false;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
