@@ -136,54 +136,67 @@ struct TableOut {
 
 // The counts of one channel, hist[m * STRIDE] for symbols m < lp - 1, become its table in place (entries
 // cdf << 16, one row more than there are symbols) and, as 16-bit entries, in stage[0 .. lp-1]
-// (normalize_cdf_value, cal_cdf.cu:11-15,40-49).  Returns the number of non-zero non-centre counts.
+// (normalize_cdf_value, cal_cdf.cu:11-15,40-49): entry m is m + scale * #{sym < m} / ntokens.
 template <int STRIDE>
-__device__ __forceinline__ int counts_to_column(uint32_t *hist, uint16_t *stage, int lp, uint32_t ntokens, int cq,
-                                                uint8_t *counts, int64_t counts_stride, bool *overflow) {
+__device__ __forceinline__ void counts_to_column(uint32_t *hist, uint16_t *stage, int lp, uint32_t ntokens, int cq) {
     const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(lp - 1);
     const uint32_t total = ntokens & 0xFFFFu;  // the reference accumulates in uint16
-    // scale * cum / total: a shift, or the rounded-down reciprocal, whose product is at most one below the quotient
+    // the division: a shift, or the rounded-down reciprocal, whose product is at most one below the quotient
     const bool pow2 = (total & (total - 1u)) == 0u;
     const int sh = 31 - __clz(static_cast<int>(total | 1u));
     const uint32_t inv = 0xFFFFFFFFu / (total | (total == 0u));
     uint32_t cum = 0;
-    int nz = 0, m = 0;
-    for (; m < lp; ++m) {
-        if (cum == ntokens) break;  // every symbol is below m: the entries from here on only count up
-        const uint32_t n = hist[m * STRIDE];
-        const uint32_t prod = scale * (cum & 0xFFFFu);
-        uint32_t q;
-        if (pow2) {
-            q = prod >> sh;
-        } else {
-            q = __umulhi(prod, inv);
-            if (prod - q * total >= total) ++q;
-        }
-        const uint32_t e = (q + static_cast<uint32_t>(m)) & 0xFFFFu;
+    const auto entry = [&](int m, uint32_t q) {
+        const uint32_t e = q + static_cast<uint32_t>(m);
         hist[m * STRIDE] = e << 16;
         stage[m] = static_cast<uint16_t>(e);
-        cum += n;
-        if (counts && m < lp - 1) {
-            if (m != cq && m <= 2 * cq) {
-                *counts = static_cast<uint8_t>(n);
-                counts += counts_stride;
-                nz += n != 0u;
-                *overflow |= n > 255u;
-            } else if (m > 2 * cq) {
-                *overflow |= n != 0u;
-            }
+    };
+    const auto divided = [&](uint32_t prod) {
+        uint32_t q = __umulhi(prod, inv);
+        if (prod - q * total >= total) ++q;
+        return q;
+    };
+    const int used = min(2 * cq + 1, lp - 1);  // the row's symbols, all that a quantiser of its bins makes
+    int m = 0;
+    if (pow2) {
+#pragma unroll 4
+        for (; m < used; ++m) {
+            const uint32_t n = hist[m * STRIDE];
+            entry(m, scale * (cum & 0xFFFFu) >> sh);
+            cum += n;
+        }
+    } else {
+#pragma unroll 4
+        for (; m < used; ++m) {
+            const uint32_t n = hist[m * STRIDE];
+            entry(m, divided(scale * (cum & 0xFFFFu)));
+            cum += n;
         }
     }
-    if (counts)
-        for (int j = m; j <= 2 * cq && j < lp - 1; ++j)
-            if (j != cq) {
-                *counts = 0u;
-                counts += counts_stride;
-            }
-    for (; m < lp; ++m) {
-        const uint32_t e = (scale + static_cast<uint32_t>(m)) & 0xFFFFu;
-        hist[m * STRIDE] = e << 16;
-        stage[m] = static_cast<uint16_t>(e);
+    for (; cum != ntokens && m < lp; ++m) {  // symbols above those (never with matching bins)
+        const uint32_t n = hist[m * STRIDE];
+        const uint32_t prod = scale * (cum & 0xFFFFu);
+        entry(m, pow2 ? prod >> sh : divided(prod));
+        cum += n;
+    }
+#pragma unroll 4
+    for (; m < lp; ++m) entry(m, scale);  // every symbol is below m
+}
+
+// The byte counts of one channel (CG_TABLES_COUNTS), before counts_to_column; returns how many are not zero.
+template <int STRIDE>
+__device__ __forceinline__ int store_counts(const uint32_t *hist, int lp, int cq, uint8_t *counts, int64_t stride, bool *overflow) {
+    int nz = 0;
+    for (int m = 0; m < lp - 1; ++m) {
+        const uint32_t n = hist[m * STRIDE];
+        if (m > 2 * cq) {
+            *overflow |= n != 0u;
+        } else if (m != cq) {
+            *counts = static_cast<uint8_t>(n);
+            counts += stride;
+            nz += n != 0u;
+            *overflow |= n > 255u;
+        }
     }
     return nz;
 }
@@ -256,8 +269,9 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint
         int nz = 0;
         if (c < nchannels) {
             const int cq = static_cast<int>(half_range(__ldg(out.bins + row)));
-            nz = counts_to_column<32>(hist + (cl >> 5) * 32 * lp + (cl & 31), stage + cl * lp, lp, ntokens, cq,
-                                  out.counts ? out.counts + __ldg(out.table_row_off + row) + c : nullptr, nchannels, &overflow);
+            uint32_t *column = hist + (cl >> 5) * 32 * lp + (cl & 31);
+            if (out.counts) nz = store_counts<32>(column, lp, cq, out.counts + __ldg(out.table_row_off + row) + c, nchannels, &overflow);
+            counts_to_column<32>(column, stage + cl * lp, lp, ntokens, cq);
         }
         if (out.group_nz) {
             nz = __reduce_add_sync(0xFFFFFFFFu, nz);
@@ -372,33 +386,39 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
         if (active) {
             for (int m = 0; m < p.lp; ++m) column[m * 32] = 0u;
             const uint32_t *q = sp;
-            constexpr int kAhead = 2 * kWordsAhead;
-            uint32_t w[kAhead], next[kAhead];
-#pragma unroll
-            for (int k = 0; k < kAhead; ++k) w[k] = 4 * k < n ? __ldg(q + k * C) : 0u;
+            constexpr int kAhead = 16;  // words in flight: the counts of one group cover the loads of the next warp's
             int i = 0;
             for (; i + 4 * kAhead <= n; i += 4 * kAhead) {
-                q += kAhead * C;
-#pragma unroll
-                for (int k = 0; k < kAhead; ++k) next[k] = i + 4 * (kAhead + k) < n ? __ldg(q + k * C) : 0u;
+                uint32_t w[kAhead], any = 0u;
 #pragma unroll
                 for (int k = 0; k < kAhead; ++k) {
-                    if (w[k] & 0x80808080u) w[k] = 0u;
+                    w[k] = __ldg(q);
+                    q += C;
+                }
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) any |= w[k];
+                if (any & 0x80808080u) {  // reported below
+#pragma unroll
+                    for (int k = 0; k < kAhead; ++k) w[k] = 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) count_symbol(entry_of(col, w[k], j));
-                    w[k] = next[k];
                 }
             }
-#pragma unroll
-            for (int k = 0; k < kAhead; ++k) {
-                if (w[k] & 0x80808080u) w[k] = 0u;
+            for (; i < n; i += 4) {
+                uint32_t w = __ldg(q);
+                q += C;
+                if (w & 0x80808080u) w = 0u;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (i + 4 * k + j < n) count_symbol(entry_of(col, w[k], j));
+                    if (i + j < n) count_symbol(entry_of(col, w, j));
             }
             const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
-            nz = counts_to_column<32>(column, stage + tid * p.lp, p.lp, n, cq,
-                                  p.out.counts ? p.out.counts + __ldg(p.out.table_row_off + row) + c : nullptr, C, &overflow);
+            if (p.out.counts)
+                nz = store_counts<32>(column, p.lp, cq, p.out.counts + __ldg(p.out.table_row_off + row) + c, C, &overflow);
+            counts_to_column<32>(column, stage + tid * p.lp, p.lp, n, cq);
         }
         if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
         __syncwarp();
