@@ -7,6 +7,7 @@ classes pickle under the reference's module path `lmcache.storage_backend.serde.
 when no `lmcache` package is importable, alias modules of that name are registered at import time
 (see cachegen_b200.compat).
 """
+import contextlib
 import ctypes
 import functools
 import io
@@ -507,6 +508,14 @@ def _load_storage_fast(b):
     return torch.storage.TypedStorage(wrap_storage=raw.untyped_storage(), dtype=dtype, _internal=True)
 
 
+_NOTHING = contextlib.nullcontext()
+
+
+def on_device(dev):
+    """Context in which `dev` is the current device; nothing to do in the usual case."""
+    return _NOTHING if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
+
+
 class _Staging:
     """Pinned host memory that a thread's blob loads and dumps pass through: bytes are copied into it
     by several threads and leave it by asynchronous copies on the current stream (or arrive in it from
@@ -516,7 +525,8 @@ class _Staging:
 
     def __init__(self):
         self.bufs = [None, None]
-        self.events = [None, None]
+        self.events = [None, None]     # (device, event) of each buffer's last copies, recorded again and again
+        self.leaving = [False, False]  # whether that event may still be outstanding
         self.turn = 0
         self.buf = None
         self.waiting = None  # (host view, device tensor) pairs of the load in progress
@@ -524,9 +534,9 @@ class _Staging:
     def begin(self, nbytes: int) -> None:
         self.turn ^= 1
         i = self.turn
-        if self.events[i] is not None:
-            self.events[i].synchronize()
-            self.events[i] = None
+        if self.leaving[i]:
+            self.events[i][1].synchronize()
+            self.leaving[i] = False
         if self.bufs[i] is None or self.bufs[i].numel() < nbytes:
             self.bufs[i] = None
             self.bufs[i] = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8)
@@ -560,11 +570,13 @@ class _Staging:
             segs = (_lib.HostSegment * len(mine))(*[(at, o.data_ptr(), n) for at, n, o, _ in mine])
             self.begin(sum((n + 255) // 256 * 256 for _, n, _, _ in mine))
             try:
-                with torch.cuda.device(device):
+                with on_device(device):
                     on = torch.cuda.current_stream(device) if stream is None else stream
+                    if self.events[self.turn] is None or self.events[self.turn][0] != device:
+                        self.events[self.turn] = (device, torch.cuda.Event())
                     rc = _lib.lib().cg_host_upload(segs, len(mine), self.buf.data_ptr(), self.buf.numel(), on.cuda_stream)
-                    self.events[self.turn] = torch.cuda.Event()
-                    self.events[self.turn].record(on)
+                    self.events[self.turn][1].record(on)
+                    self.leaving[self.turn] = True
             finally:
                 self.end()
             _lib.check(rc, "cg_host_upload")
@@ -601,7 +613,7 @@ class _Staging:
 
     def _download(self, phase: int) -> None:
         device = self.fetched[0].device
-        with torch.cuda.device(device):
+        with on_device(device):
             rc = _lib.lib().cg_host_download(self.segs, len(self.segs), self.buf.data_ptr(), self.buf.numel(), phase,
                                              torch.cuda.current_stream(device).cuda_stream)
         _lib.check(rc, "cg_host_download")

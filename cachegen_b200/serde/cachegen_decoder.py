@@ -6,7 +6,6 @@ per-sub-chunk launches and the fp32 dequantise / stack / permute / cast chain re
 calls: cg_decode_offsets (the cumsum of dec.py:70) and cg_decode_dequant (everything else).
 (dec.py = cachegen_decoder.py of the reference.)
 """
-import contextlib
 import ctypes
 import functools
 import queue
@@ -21,18 +20,10 @@ from ..config import LMCacheEngineConfig, LMCacheEngineMetadata
 from ..utils import _lmcache_nvtx_annotate
 from . import cachegen_basics as CGBasics
 from . import flat_format
-from .cachegen_basics import CacheGenConfig, CacheGenGPUBytestream, CacheGenGPUEncoderOutput
+from .cachegen_basics import CacheGenConfig, CacheGenGPUBytestream, CacheGenGPUEncoderOutput, on_device
 from .serde import Deserializer
 
 _DTYPES = {torch.float16: _lib.CG_F16, torch.bfloat16: _lib.CG_BF16}
-
-
-_NOTHING = contextlib.nullcontext()
-
-
-def _current(dev):
-    """Context in which `dev` is the current device; nothing to do in the usual case."""
-    return _NOTHING if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def _stream(device):
@@ -124,10 +115,38 @@ def _staged(t: torch.Tensor, dev) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+class _HostBins:
+    """What the bins a decoder was set up with say about the containers it reads; kept in its workspace."""
+
+    def __init__(self, bins: torch.Tensor):
+        self.cpu = bins.cpu()
+        self.sparse = flat_format.sparse_representable(self.cpu)
+        self._checksums, self._counts, self._sparse = {}, {}, {}
+
+    def checksum(self, delta) -> int:
+        key = None if delta is None else (delta.group, delta.divisor, delta.rows)
+        if key not in self._checksums:
+            self._checksums[key] = flat_format.bins_checksum(self.cpu, delta)
+        return self._checksums[key]
+
+    def counts_bytes(self, nchannels: int) -> int:
+        if nchannels not in self._counts:
+            self._counts[nchannels] = flat_format.table_row_offsets(self.cpu, nchannels)[-1]
+        return self._counts[nchannels]
+
+    def sparse_bytes(self, nchannels: int) -> int:
+        """Of the masks and what stands in front of them."""
+        if nchannels not in self._sparse:
+            masks = flat_format.mask_row_offsets(self.cpu, nchannels)[-1]
+            self._sparse[nchannels] = flat_format.sparse_parts(self.cpu.numel(), nchannels, masks)[1]
+        return self._sparse[nchannels]
+
+
 class _ChunkView:
     """What a decode needs from one encoded chunk, whichever container it came in, on the GPU."""
 
-    def __init__(self, eo, dev, bins_cpu, delta=None):
+    def __init__(self, eo, dev, bins, delta=None):
+        """`bins`: a _HostBins.  tables, mk, mv and the first and third part of each of `subs` are addresses."""
         self.keep = []
         if isinstance(eo, flat_format.FlatChunk):
             fc = eo if eo.blob.device == dev else eo.to(dev, non_blocking=True)
@@ -135,29 +154,31 @@ class _ChunkView:
             self.L, self.H, self.D, self.T, self.lp = h.L, h.H, h.D, h.T, h.lp
             self.C = h.H * h.D
             self.scale_dtype = fc.scale_dtype
-            sc = fc.scales()
-            self.mk, self.mv = sc[:h.L], sc[h.L:]
-            self.tables = fc.tables()
-            self.table_kind = h.table_kind
-            if ((h.table_kind != flat_format.TABLES_CDF or delta is not None) and h.bins_checksum and
-                    h.bins_checksum != flat_format.bins_checksum(bins_cpu, delta)):
-                raise RuntimeError("the container was written with other bin or delta settings")
-            if (delta is None and h.table_kind == flat_format.TABLES_CDF and h.bins_checksum and
-                    h.bins_checksum != flat_format.bins_checksum(bins_cpu)):
-                # int16 tables decode with any bins, but a chunk written with delta coding does not
+            self.table_kind, self.length_kind = h.table_kind, h.length_kind
+            # int16 tables decode with any bins, but a chunk written with delta coding does not
+            if h.bins_checksum and h.bins_checksum != bins.checksum(delta):
                 raise RuntimeError("the container was written with other bin or delta settings")
             if h.table_kind == flat_format.TABLES_COUNTS:
-                need = flat_format.table_row_offsets(bins_cpu, self.C)[-1]
-                if h.off_lengths - h.off_tables < need:
+                if h.off_lengths - h.off_tables < bins.counts_bytes(self.C):
                     raise RuntimeError("the container's byte-count tables are smaller than the configured bins need")
             elif h.table_kind == flat_format.TABLES_SPARSE:
-                if not flat_format.sparse_representable(bins_cpu):
+                if not bins.sparse:
                     raise RuntimeError("sparse tables cannot describe the configured bins")
-                need = flat_format.sparse_parts(2 * h.L, self.C, flat_format.mask_row_offsets(bins_cpu, self.C)[-1])[1]
-                if h.off_lengths - h.off_tables < need:
+                if h.off_lengths - h.off_tables < bins.sparse_bytes(self.C):
                     raise RuntimeError("the container's sparse tables are smaller than the configured bins need")
-            self.length_kind = h.length_kind
-            self.subs = [(fc.payload(j), fc.lengths(j), fc.sub_tokens(j)) for j in range(h.nsub)]
+            # addresses inside the container: a view for each takes longer to make than a short chunk to decode
+            at, size, wide = fc.blob.data_ptr(), fc.blob.numel(), 2 if h.length_kind == flat_format.LENGTHS_U16 else 4
+            row = 2 * h.L * self.C * wide
+            if size < h.off_lengths + h.nsub * row or (at + h.off_scales) % 2 or (at + h.off_lengths) % wide or (
+                    h.table_kind == flat_format.TABLES_CDF and (at + h.off_tables) % 2):
+                raise RuntimeError("the container's sections are cut short or misaligned")
+            self.mk = at + h.off_scales
+            self.mv = self.mk + 2 * h.L * h.T
+            self.tables = at + h.off_tables
+            self.subs = []
+            for j in range(h.nsub):
+                start, end = (min(h.off_payload + o, size) for o in h.sub_off[j:j + 2])
+                self.subs.append((at + start, end - start, at + h.off_lengths + j * row, fc.sub_tokens(j)))
             self.table_bytes = h.off_lengths - h.off_tables
             self.length_bytes = h.off_payload - h.off_lengths
             self.keep.append(fc.blob)
@@ -166,9 +187,9 @@ class _ChunkView:
             self.L, self.C, self.lp, self.T = L, C, lp, T
             self.H, self.D = eo.num_heads, eo.head_size
             self.scale_dtype = eo.max_tensors_key.dtype
-            self.mk = _staged(eo.max_tensors_key, dev)
-            self.mv = _staged(eo.max_tensors_value, dev)
-            self.tables = _staged(eo.cdf, dev)
+            mk, mv, tables = (_staged(t, dev) for t in (eo.max_tensors_key, eo.max_tensors_value, eo.cdf))
+            self.mk, self.mv, self.tables = mk.data_ptr(), mv.data_ptr(), tables.data_ptr()
+            self.keep += (mk, mv, tables)
             self.table_kind = _lib.CG_TABLES_CDF
             self.length_kind = _lib.CG_LENGTHS_I32
             self.subs = []
@@ -178,16 +199,15 @@ class _ChunkView:
                     raise RuntimeError("bytestream must be a 1-D uint8 tensor")
                 if ln.dtype != torch.int32 or ln.numel() != 2 * L * C:
                     raise RuntimeError("bytestream_lengths must be int32 [2L, C]")
-                self.subs.append((_staged(bs, dev), _staged(ln, dev), dc.ntokens))
-            self.table_bytes = self.tables.numel() * 2
+                bs, ln = _staged(bs, dev), _staged(ln, dev)
+                self.subs.append((bs.data_ptr(), bs.numel(), ln.data_ptr(), dc.ntokens))
+                self.keep += (bs, ln)
+            self.table_bytes = tables.numel() * 2
             self.length_bytes = len(self.subs) * 2 * L * C * 4
-            self.keep += (self.mk, self.mv, self.tables)
-            for sub in self.subs:
-                self.keep += sub[:2]
-        if sum(s[2] for s in self.subs) != self.T:
+        if sum(s[3] for s in self.subs) != self.T:
             raise RuntimeError("sub-chunk token counts do not add up to the chunk's tokens")
-        for _, _, ntok in self.subs:
-            if not 0 < ntok <= CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK:
+        for s in self.subs:
+            if not 0 < s[3] <= CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK:
                 raise RuntimeError("a sub-chunk holds 1..256 tokens")
 
 
@@ -216,12 +236,11 @@ class DecodePlan:
         dev = torch.device(device) if device is not None else (
             _device_of(first) if _on_gpu(first) else torch.device("cuda", torch.cuda.current_device()))
         ws = workspace if workspace is not None else {}
-        bins_cpu = ws.get("bins_cpu")
-        if bins_cpu is None or bins_cpu.numel() != bins.numel():
-            bins_cpu = bins.cpu()
-            ws["bins_cpu"] = bins_cpu
-        with _current(dev):
-            views = [_ChunkView(eo, dev, bins_cpu, delta) for eo in encoder_outputs]
+        host_bins = ws.get("host_bins")
+        if host_bins is None or host_bins.cpu.numel() != bins.numel():
+            host_bins = ws["host_bins"] = _HostBins(bins)
+        with on_device(dev):
+            views = [_ChunkView(eo, dev, host_bins, delta) for eo in encoder_outputs]
         v0 = views[0]
         L, C, lp, H, D, scale_dtype = v0.L, v0.C, v0.lp, v0.H, v0.D, v0.scale_dtype
         NL = 2 * L
@@ -262,7 +281,7 @@ class DecodePlan:
             if any(v.table_kind == kind for v in views):
                 t = ws.get(name)
                 if t is None or t.device != dev or ws.get(name + "_c") != C:
-                    t = torch.tensor(fn(bins_cpu, C), dtype=torch.int64, device=dev)
+                    t = torch.tensor(fn(host_bins.cpu, C), dtype=torch.int64, device=dev)
                     ws[name], ws[name + "_c"] = t, C
                 row_offs[kind] = t
 
@@ -276,13 +295,12 @@ class DecodePlan:
             self.keep += v.keep
             self.table_bytes += v.table_bytes
             self.length_bytes += v.length_bytes
-            tables, mk, mv = v.tables.data_ptr(), v.mk.data_ptr(), v.mv.data_ptr()
+            mk, mv = v.mk, v.mv
             row_off = row_offs[v.table_kind].data_ptr() if v.table_kind in row_offs else None
-            for bs, ln, ntok in v.subs:
-                nbytes = bs.numel()
+            for at_bytes, nbytes, at_lengths, ntok in v.subs:
                 self.payload_bytes += nbytes
                 job = jobs[k]
-                job.tables, job.bytes, job.lengths, job.group_off = tables, bs.data_ptr(), ln.data_ptr(), at_off
+                job.tables, job.bytes, job.lengths, job.group_off = v.tables, at_bytes, at_lengths, at_off
                 job.scales_k, job.scales_v, job.out, job.table_row_off = mk, mv, at_out, row_off
                 job.nbytes, job.tables_nbytes, job.ntokens, job.scale_stride = nbytes, v.table_bytes, ntok, v.T
                 job.table_kind, job.length_kind = v.table_kind, v.length_kind
@@ -317,7 +335,7 @@ class DecodePlan:
     def run_offsets(self) -> None:
         lib = _lib.lib()
         NL, C = self.dims[5], self.dims[3]
-        with _current(self.dev):
+        with on_device(self.dev):
             st = _stream(self.dev)
             for arr, n, goff in self.batches:
                 rc = lib.cg_decode_offsets(arr, n, NL, C, goff, self.status.data_ptr(), st)
@@ -327,7 +345,7 @@ class DecodePlan:
     def run_decode(self) -> None:
         lib = _lib.lib()
         L, H, D, C, lp, NL, _ = self.dims
-        with _current(self.dev):
+        with on_device(self.dev):
             st = _stream(self.dev)
             for arr, n, _ in self.batches:
                 if self.delta_group:
@@ -343,7 +361,7 @@ class DecodePlan:
     def run(self) -> torch.Tensor:
         L, H, D, _, lp, _, _ = self.dims
         cur = torch.cuda.current_stream(self.dev)
-        with _current(self.dev):
+        with on_device(self.dev):
             rc = _lib.lib().cg_decode_kv(self.jobs, self.njobs, L, H, D, lp, self.bins.data_ptr(), self.delta_group,
                                          self.res_bins.data_ptr() if self.delta_group else None, *self.dtypes, *self.strides,
                                          self.status.data_ptr(), cur.cuda_stream)

@@ -15,7 +15,6 @@ cg_encode_kv_flat).  quantize_and_tables, encode_streams and pack_sparse_tables 
 (enc.py = cachegen_encoder.py of the reference.)
 """
 import collections
-import contextlib
 import ctypes
 import dataclasses
 import functools
@@ -30,7 +29,7 @@ from ..config import LMCacheEngineConfig, LMCacheEngineMetadata
 from ..utils import _lmcache_nvtx_annotate
 from . import cachegen_basics as CGBasics
 from . import flat_format
-from .cachegen_basics import CacheGenConfig, CacheGenGPUBytestream, CacheGenGPUEncoderOutput
+from .cachegen_basics import CacheGenConfig, CacheGenGPUBytestream, CacheGenGPUEncoderOutput, on_device
 from .serde import Serializer
 
 _DTYPES = {torch.float16: _lib.CG_F16, torch.bfloat16: _lib.CG_BF16}
@@ -105,7 +104,7 @@ def _collect(output_buffer: torch.Tensor, output_lengths: torch.Tensor, status: 
     nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
     offsets = torch.empty(NL * nslab, dtype=torch.int64, device=dev)
     lib, stream = _lib.lib(), _stream(dev)
-    with _current(dev):
+    with on_device(dev):
         if NL * nslab <= _lib.CG_MAX_OFFSET_GROUPS:
             tail = _take_tail(4)
             rc = lib.cg_stream_sizes(_ptr(lengths), NL, C, min(stride, 1 << 20),
@@ -282,6 +281,8 @@ class _BinsInfo:
         self.nlayers = key_bins.numel()
         self.kmax, self.vmax = int(key_bins.max()), int(value_bins.max())
         self.on_device = {}   # device -> float32 [2L]
+        self.sparse = flat_format.sparse_representable(self.cpu)
+        self.checksums = {}   # delta settings -> bins_checksum
         self.row_offsets = {}  # (device, channels) -> (int64 offsets of the byte counts, size, of the masks, size)
 
     def on(self, dev):
@@ -289,6 +290,12 @@ class _BinsInfo:
         if t is None:
             t = self.on_device[dev] = self.cpu.to(dev)
         return t
+
+    def checksum(self, delta):
+        key = None if delta is None else (delta.group, delta.divisor, delta.rows)
+        if key not in self.checksums:
+            self.checksums[key] = flat_format.bins_checksum(self.cpu, delta)
+        return self.checksums[key]
 
     def offsets(self, dev, nchannels):
         o = self.row_offsets.get((dev, nchannels))
@@ -352,14 +359,6 @@ def _give_tail(t: torch.Tensor) -> None:
         pool.append(t)
 
 
-_NOTHING = contextlib.nullcontext()
-
-
-def _current(dev):
-    """Context in which `dev` is the current device; nothing to do in the usual case."""
-    return _NOTHING if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
-
-
 class _PendingChunk:
     """One chunk whose kernels up to the streams and their offsets are enqueued on `stream` (default: the
     current one), but whose payload size is not yet known on the host.  finish() waits for that and
@@ -412,12 +411,12 @@ class _PendingChunk:
         if delta is not None:
             self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
             job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
-        with _current(dev):
+        with on_device(dev):
             _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
 
     def sizes(self):
         """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
-        with _current(self.dev):
+        with on_device(self.dev):
             _lib.check(self.lib.cg_encode_kv_wait(ctypes.byref(self.job), self.stream_ptr), "cg_encode_kv_wait")
         host = self.tail[:self.nsub + 3].tolist()
         _give_tail(self.tail)
@@ -434,7 +433,7 @@ class _PendingChunk:
         pieces = [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(n)]
         lengths = [torch.empty((NL, C), dtype=torch.int32, device=self.dev) for _ in range(n)]
         array = ctypes.c_void_p * n
-        with _current(self.dev):
+        with on_device(self.dev):
             rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), array(*[t.data_ptr() for t in pieces]),
                                               array(*[t.data_ptr() for t in lengths]), self.stream_ptr)
         _lib.check(rc, "cg_encode_kv_gather")
@@ -578,14 +577,14 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     offs, bits, nonzero = p.sizes()
     fits = bool(compact_tables) and not (bits & _lib.CG_S_COUNT_OVERFLOW)
     off_masks, off_counts = flat_format.sparse_parts(2 * p.L, p.H * p.D, p.mask_bytes)
-    if fits and compact_tables is True and flat_format.sparse_representable(info.cpu):
+    if fits and compact_tables is True and info.sparse:
         kind, size = flat_format.TABLES_SPARSE, off_counts + nonzero
     elif fits:
         kind, size = flat_format.TABLES_COUNTS, p.counts.numel()
     else:
         kind, size = flat_format.TABLES_CDF, 2 * p.cdf.numel()
     header = flat_format.layout(p.L, p.H, p.D, p.T, kmax + 1, p.kv.dtype, kind, size, flat_format.LENGTHS_U16, offs,
-                                bins_checksum=flat_format.bins_checksum(info.cpu, delta))
+                                bins_checksum=info.checksum(delta))
     head = header.pack()
     blob = torch.empty(header.total, dtype=torch.uint8, device=p.dev)
     f = _lib.FlatLayout()
@@ -596,7 +595,7 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     f.off_scales, f.off_tables, f.tables_bytes = header.off_scales, header.off_tables, size
     f.off_lengths, f.off_payload = header.off_lengths, header.off_payload
     f.off_masks, f.off_counts, f.table_kind = off_masks, off_counts, kind
-    with _current(p.dev):
+    with on_device(p.dev):
         _lib.check(p.lib.cg_encode_kv_flat(ctypes.byref(p.job), ctypes.byref(f), p.stream_ptr), "cg_encode_kv_flat")
     return flat_format.FlatChunk(blob, header)
 
