@@ -69,7 +69,7 @@ def test_kv_that_is_not_finite_is_reported(value):
     E.encode_function(make_kv(2, 40, 2, 64, torch.float16, 9), None, kb, vb, 40)  # and nothing is left behind
 
 
-@pytest.mark.parametrize("nbytes", [1, 255, 256, 4097, (512 << 10) + 1, (9 << 20) + 13])
+@pytest.mark.parametrize("nbytes", [1, 255, 256, 4097, 128 << 10, (512 << 10) + 1, (9 << 20) + 13])
 def test_byte_strings_to_the_gpu_and_back(nbytes):
     from cachegen_b200.serde.cachegen_basics import staging
     g = torch.Generator().manual_seed(nbytes)
