@@ -17,6 +17,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -207,34 +208,24 @@ int check_segments(const cg_host_segment *segs, int n, const void *staging, int6
 
 using namespace cg;
 
-extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *staging, int64_t staging_bytes, void *stream) {
-    int64_t count;
-    if (int rc = check_segments(segs, nsegs, staging, staging_bytes, &count)) return rc;
-    if (!count) return CG_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint8_t *stage = static_cast<uint8_t *>(staging);
-    Job job(static_cast<int>(count));
-    std::vector<uint8_t *> to(static_cast<size_t>(count));  // where each piece goes on the GPU
-    int k = 0;
-    for (int i = 0; i < nsegs; ++i) {
-        const uint8_t *src = static_cast<const uint8_t *>(segs[i].host);
-        for (int64_t a = 0; a < segs[i].bytes; a += kPiece, ++k) {
-            job.pieces[k].dst = stage + a;
-            job.pieces[k].src = src + a;
-            job.pieces[k].bytes = segs[i].bytes - a < kPiece ? segs[i].bytes - a : kPiece;
-            to[k] = static_cast<uint8_t *>(segs[i].device) + a;
-        }
-        stage += round_up(segs[i].bytes);
-    }
-    const int n = static_cast<int>(count);
-    job.ready.store(n, std::memory_order_release);
-    if (n > 1) helpers().add(&job);
-    cudaError_t err = cudaSuccess;
-    int sent = 0, end = 0;
+namespace {
+// A part of a transfer to the GPU: it can go once the job's first `upto` pieces have been copied.
+struct Part {
+    uint8_t *to;
+    const uint8_t *from;
+    int64_t bytes;
+    int upto;
+};
+
+// Sends the parts, in order, as the job's pieces are copied; the caller copies with the helpers.
+cudaError_t send_parts(Job &job, const std::vector<Part> &parts, cudaStream_t st) {
+    const int n = static_cast<int>(parts.size());
+    int sent = 0, end = 0, copied_pieces = 0;
     int64_t left = 0, copied = 0, most = kFirstSend;  // bytes not sent yet; of those, the ones up to `end`
-    for (const Piece &p : job.pieces) left += p.bytes;
+    for (const Part &p : parts) left += p.bytes;
     while (sent < n) {
-        for (; end < n && job.pieces[end].done.load(std::memory_order_acquire); ++end) copied += job.pieces[end].bytes;
+        while (copied_pieces < static_cast<int>(job.pieces.size()) && job.pieces[copied_pieces].done.load(std::memory_order_acquire)) ++copied_pieces;
+        for (; end < n && parts[end].upto <= copied_pieces; ++end) copied += parts[end].bytes;
         // all that has been copied in a row of the same tensor goes as one transfer
         const bool enough = end == n || copied >= part_of(left, kFirstSend, most);
         if (enough) {
@@ -242,19 +233,102 @@ extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *stag
             left -= copied;
             copied = 0;
         }
-        while (enough && sent < end && err == cudaSuccess) {
-            int64_t bytes = job.pieces[sent].bytes;
+        while (enough && sent < end) {
+            int64_t bytes = parts[sent].bytes;
             int e = sent + 1;
-            while (e < end && to[e] == to[sent] + bytes && job.pieces[e].dst == job.pieces[sent].dst + bytes) bytes += job.pieces[e++].bytes;
-            err = cudaMemcpyAsync(to[sent], job.pieces[sent].dst, static_cast<size_t>(bytes), cudaMemcpyHostToDevice, st);
+            while (e < end && parts[e].to == parts[sent].to + bytes && parts[e].from == parts[sent].from + bytes) bytes += parts[e++].bytes;
+            const cudaError_t err = cudaMemcpyAsync(parts[sent].to, parts[sent].from, static_cast<size_t>(bytes), cudaMemcpyHostToDevice, st);
+            if (err != cudaSuccess) return err;
             sent = e;
         }
-        if (err != cudaSuccess) break;
         if (sent < n && !job.work()) _mm_pause();
     }
+    return cudaSuccess;
+}
+
+// A byte string on its way into staging memory (cg_host_stage).
+struct Stage {
+    Stage(const void *h, int64_t n, void *s)
+        : host(static_cast<const uint8_t *>(h)), staging(static_cast<uint8_t *>(s)), bytes(n), job(static_cast<int>((n + kPiece - 1) / kPiece)) {
+        for (size_t k = 0; k < job.pieces.size(); ++k) {
+            const int64_t a = static_cast<int64_t>(k) * kPiece;
+            job.pieces[k].dst = staging + a;
+            job.pieces[k].src = host + a;
+            job.pieces[k].bytes = n - a < kPiece ? n - a : kPiece;
+        }
+        job.ready.store(static_cast<int>(job.pieces.size()), std::memory_order_release);
+    }
+    const uint8_t *host;
+    uint8_t *staging;
+    int64_t bytes;
+    Job job;
+};
+}  // namespace
+
+extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *staging, int64_t staging_bytes, void *stream) {
+    int64_t count;
+    if (int rc = check_segments(segs, nsegs, staging, staging_bytes, &count)) return rc;
+    if (!count) return CG_OK;
+    uint8_t *stage = static_cast<uint8_t *>(staging);
+    Job job(static_cast<int>(count));
+    std::vector<Part> parts(static_cast<size_t>(count));
+    int k = 0;
+    for (int i = 0; i < nsegs; ++i) {
+        const uint8_t *src = static_cast<const uint8_t *>(segs[i].host);
+        for (int64_t a = 0; a < segs[i].bytes; a += kPiece, ++k) {
+            job.pieces[k].dst = stage + a;
+            job.pieces[k].src = src + a;
+            job.pieces[k].bytes = segs[i].bytes - a < kPiece ? segs[i].bytes - a : kPiece;
+            parts[k] = Part{static_cast<uint8_t *>(segs[i].device) + a, stage + a, job.pieces[k].bytes, k + 1};
+        }
+        stage += round_up(segs[i].bytes);
+    }
+    job.ready.store(k, std::memory_order_release);
+    if (k > 1) helpers().add(&job);
+    const cudaError_t err = send_parts(job, parts, static_cast<cudaStream_t>(stream));
     while (!job.taken()) job.work();  // only after an error: nobody may touch the job once it is gone
-    if (n > 1) helpers().remove(&job);
+    if (k > 1) helpers().remove(&job);
     return err == cudaSuccess ? CG_OK : set_cuda_error(err);
+}
+
+extern "C" int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle) {
+    if (!host || !staging || !handle) return CG_E_NULL;
+    if (bytes <= 0 || (bytes + kPiece - 1) / kPiece > 0x7FFFFFFF) return CG_E_SHAPE;
+    if (bytes > staging_bytes) return CG_E_CAPACITY;
+    Stage *s = new (std::nothrow) Stage(host, bytes, staging);
+    if (!s) return CG_E_CAPACITY;
+    helpers().add(&s->job);
+    *handle = s;
+    return CG_OK;
+}
+
+extern "C" int cg_host_stage_send(void *handle, const cg_host_segment *segs, int nsegs, void *stream) {
+    if (!handle || !segs) return CG_E_NULL;
+    Stage &s = *static_cast<Stage *>(handle);
+    std::vector<Part> parts;
+    for (int i = 0; i < nsegs; ++i) {
+        const uint8_t *host = static_cast<const uint8_t *>(segs[i].host);
+        if (segs[i].bytes < 0 || host < s.host || segs[i].bytes > s.bytes - (host - s.host)) return CG_E_SHAPE;
+        if (segs[i].bytes && !segs[i].device) return CG_E_NULL;
+        const int64_t at = host - s.host;
+        for (int64_t a = 0; a < segs[i].bytes;) {  // up to the end of the piece
+            const int64_t k = (at + a) / kPiece, room = (k + 1) * kPiece - (at + a);
+            const int64_t n = room < segs[i].bytes - a ? room : segs[i].bytes - a;
+            parts.push_back(Part{static_cast<uint8_t *>(segs[i].device) + a, s.staging + at + a, n, static_cast<int>(k) + 1});
+            a += n;
+        }
+    }
+    const cudaError_t err = send_parts(s.job, parts, static_cast<cudaStream_t>(stream));
+    return err == cudaSuccess ? CG_OK : set_cuda_error(err);
+}
+
+extern "C" int cg_host_stage_end(void *handle) {
+    if (!handle) return CG_E_NULL;
+    Stage *s = static_cast<Stage *>(handle);
+    s->job.next.store(static_cast<int>(s->job.pieces.size()), std::memory_order_relaxed);  // what has not been sent is not wanted
+    helpers().remove(&s->job);
+    delete s;
+    return CG_OK;
 }
 
 namespace {

@@ -578,9 +578,11 @@ class CacheGenDeserializer(Deserializer):
         total = len(blobs)
         parsed = queue.SimpleQueue()
 
-        def parse(blob):
+        def parse(blob, ahead=False):
             load = CGBasics.BlobLoad()
             with load:
+                if ahead and isinstance(blob, bytes) and not flat_format.is_flat(blob):
+                    CGBasics.staging().start(blob)
                 chunk = (load.flat(blob, dev) if flat_format.is_flat(blob) else load.unpickle(blob))
             ntokens = _chunk_tokens(chunk)
             if ntokens > self.chunk_size:
@@ -595,12 +597,12 @@ class CacheGenDeserializer(Deserializer):
             except BaseException as e:  # handed to the caller's thread
                 parsed.put(e)
 
-        first = parse(blobs[0])
-        if total > 1:
-            threading.Thread(target=parse_rest, daemon=True).start()
         chunks, tokens, done, at = [], 0, 0, 0
         waiting = []
         try:
+            first = parse(blobs[0], ahead=True)  # the others are parsed while their predecessors travel
+            if total > 1:
+                threading.Thread(target=parse_rest, daemon=True).start()
             while done < total:
                 item = first if done == 0 else (waiting.pop(0) if waiting else parsed.get())
                 if isinstance(item, BaseException):
@@ -627,6 +629,7 @@ class CacheGenDeserializer(Deserializer):
                     start += n
                 at = len(chunks)
         finally:
+            CGBasics.staging().finish()
             cur.wait_stream(copies)
         return out
 

@@ -469,6 +469,16 @@ int cg_host_upload(const cg_host_segment *segments_host, int nsegments, void *st
 int cg_host_download(const cg_host_segment *segments_host, int nsegments, void *staging, int64_t staging_bytes, int phase,
                      void *stream);
 
+/*
+ * cg_host_upload in steps, for a byte string whose tensors are found while it is being copied.  cg_host_stage starts the
+ * helper threads on copying all of it to `staging`, which holds it at the same offsets; cg_host_stage_send takes
+ * segments inside it; cg_host_stage_end, called once whatever happened before, waits for the threads.  `host`
+ * must stay until then, `staging` until the stream has passed the segments' transfers.
+ */
+int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle_host);
+int cg_host_stage_send(void *handle_host, const cg_host_segment *segments_host, int nsegments, void *stream);
+int cg_host_stage_end(void *handle_host);
+
 #ifdef __cplusplus
 }
 #endif
