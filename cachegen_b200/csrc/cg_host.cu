@@ -248,8 +248,8 @@ cudaError_t send_parts(Job &job, const std::vector<Part> &parts, cudaStream_t st
 
 // A byte string on its way into staging memory (cg_host_stage).
 struct Stage {
-    Stage(const void *h, int64_t n, void *s)
-        : host(static_cast<const uint8_t *>(h)), staging(static_cast<uint8_t *>(s)), bytes(n), job(static_cast<int>((n + kPiece - 1) / kPiece)) {
+    Stage(const void *h, int64_t n, void *s, int64_t size)
+        : host(static_cast<const uint8_t *>(h)), staging(static_cast<uint8_t *>(s)), bytes(n), spare(round_up(n)), room(size), job(static_cast<int>((n + kPiece - 1) / kPiece)) {
         for (size_t k = 0; k < job.pieces.size(); ++k) {
             const int64_t a = static_cast<int64_t>(k) * kPiece;
             job.pieces[k].dst = staging + a;
@@ -260,7 +260,7 @@ struct Stage {
     }
     const uint8_t *host;
     uint8_t *staging;
-    int64_t bytes;
+    int64_t bytes, spare, room;  // of the byte string; where the staging memory is free; its size
     Job job;
 };
 }  // namespace
@@ -295,7 +295,7 @@ extern "C" int cg_host_stage(const void *host, int64_t bytes, void *staging, int
     if (!host || !staging || !handle) return CG_E_NULL;
     if (bytes <= 0 || (bytes + kPiece - 1) / kPiece > 0x7FFFFFFF) return CG_E_SHAPE;
     if (bytes > staging_bytes) return CG_E_CAPACITY;
-    Stage *s = new (std::nothrow) Stage(host, bytes, staging);
+    Stage *s = new (std::nothrow) Stage(host, bytes, staging, staging_bytes);
     if (!s) return CG_E_CAPACITY;
     helpers().add(&s->job);
     *handle = s;
@@ -307,10 +307,19 @@ extern "C" int cg_host_stage_send(void *handle, const cg_host_segment *segs, int
     Stage &s = *static_cast<Stage *>(handle);
     std::vector<Part> parts;
     for (int i = 0; i < nsegs; ++i) {
+        if (segs[i].bytes < 0) return CG_E_SHAPE;
+        if (segs[i].bytes && (!segs[i].device || !segs[i].host)) return CG_E_NULL;
         const uint8_t *host = static_cast<const uint8_t *>(segs[i].host);
-        if (segs[i].bytes < 0 || host < s.host || segs[i].bytes > s.bytes - (host - s.host)) return CG_E_SHAPE;
-        if (segs[i].bytes && !segs[i].device) return CG_E_NULL;
-        const int64_t at = host - s.host;
+        const uintptr_t in = reinterpret_cast<uintptr_t>(host) - reinterpret_cast<uintptr_t>(s.host);
+        if (in >= static_cast<uintptr_t>(s.bytes)) {  // outside the byte string: to the free part, by the caller
+            if (segs[i].bytes > s.room - s.spare) return CG_E_CAPACITY;
+            memcpy(s.staging + s.spare, host, static_cast<size_t>(segs[i].bytes));
+            parts.push_back(Part{static_cast<uint8_t *>(segs[i].device), s.staging + s.spare, segs[i].bytes, 0});
+            s.spare += round_up(segs[i].bytes);
+            continue;
+        }
+        if (segs[i].bytes > s.bytes - static_cast<int64_t>(in)) return CG_E_SHAPE;
+        const int64_t at = static_cast<int64_t>(in);
         for (int64_t a = 0; a < segs[i].bytes;) {  // up to the end of the piece
             const int64_t k = (at + a) / kPiece, room = (k + 1) * kPiece - (at + a);
             const int64_t n = room < segs[i].bytes - a ? room : segs[i].bytes - a;

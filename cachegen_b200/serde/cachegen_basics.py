@@ -509,6 +509,7 @@ def _load_storage_fast(b):
 
 
 _NOTHING = contextlib.nullcontext()
+_EARLY_SPARE = 256 << 10  # room behind the byte string for tensors that are not part of it
 _EARLY_FROM = 2 << 20  # below, parsing and copying take less time than the threads take to wake
 
 
@@ -565,7 +566,7 @@ class _Staging:
         blob takes 130 us, as long as a quarter of its 30 MB take over the bus, and waking the threads 50."""
         if len(bs) < _EARLY_FROM or not torch.cuda.is_available():
             return
-        self.begin(len(bs))
+        self.begin(len(bs) + _EARLY_SPARE)
         handle = ctypes.c_void_p()
         at = _bytes_at(bs)
         rc = _lib.lib().cg_host_stage(at, len(bs), self.buf.data_ptr(), self.buf.numel(), ctypes.byref(handle))
@@ -573,16 +574,22 @@ class _Staging:
         self.early = (handle, at, len(bs))
 
     def _send_early(self, pairs: list, stream) -> list:
-        """Sends the tensors that lie in the byte string of `start`, if they are on one GPU; returns the others."""
+        """Sends the tensors that lie in the byte string of `start`, and small ones beside it (a blob's scales: the
+        unpickler copies short streams), if they are on one GPU; returns the others."""
         handle, at, size = self.early
-        inside, others = [], []
+        mine, others, spare = [], [], _EARLY_SPARE - 256
         for p in pairs:
-            (inside if at <= p[0] and p[0] + p[1] <= at + size else others).append(p)
+            if not at <= p[0] < at + size:
+                spare -= (p[1] + 255) // 256 * 256
+                if spare < 0:
+                    others.append(p)
+                    continue
+            mine.append(p)
         try:
-            if not inside or any(p[2].device != inside[0][2].device for p in inside):
+            if not mine or any(p[2].device != mine[0][2].device for p in mine):
                 return pairs
-            segs = (_lib.HostSegment * len(inside))(*[(a, o.data_ptr(), n) for a, n, o, _ in inside])
-            self._send(lambda on: _lib.lib().cg_host_stage_send(handle, segs, len(inside), on), inside[0][2].device, stream)
+            segs = (_lib.HostSegment * len(mine))(*[(a, o.data_ptr(), n) for a, n, o, _ in mine])
+            self._send(lambda on: _lib.lib().cg_host_stage_send(handle, segs, len(mine), on), mine[0][2].device, stream)
         finally:
             self.finish()
         return others

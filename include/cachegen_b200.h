@@ -472,7 +472,7 @@ int cg_host_download(const cg_host_segment *segments_host, int nsegments, void *
 /*
  * cg_host_upload in steps, for a byte string whose tensors are found while it is being copied.  cg_host_stage starts the
  * helper threads on copying all of it to `staging`, which holds it at the same offsets; cg_host_stage_send takes
- * segments inside it; cg_host_stage_end, called once whatever happened before, waits for the threads.  `host`
+ * segments inside it, or small ones elsewhere for which `staging` has room behind it (each rounded up to 256); cg_host_stage_end, called once whatever happened before, waits for the threads.  `host`
  * must stay until then, `staging` until the stream has passed the segments' transfers.
  */
 int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle_host);
