@@ -413,6 +413,11 @@ class _PendingChunk:
             job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
         with on_device(dev):
             _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
+        # made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do
+        self.lengths = [] if with_counts else [torch.empty((2 * L, H * D), dtype=torch.int32, device=dev)
+                                               for _ in range(self.nsub)]
+        self.pointers = ctypes.c_void_p * self.nsub
+        self.length_pointers = self.pointers(*[t.data_ptr() for t in self.lengths])
 
     def sizes(self):
         """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
@@ -428,14 +433,12 @@ class _PendingChunk:
 
     def finish(self) -> CacheGenGPUEncoderOutput:
         offs, _, _ = self.sizes()
-        n, NL, C = self.nsub, 2 * self.L, self.H * self.D
+        n, lengths = self.nsub, self.lengths
         # every sub-chunk in tensors of its own: a view would pickle the whole buffer
         pieces = [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(n)]
-        lengths = [torch.empty((NL, C), dtype=torch.int32, device=self.dev) for _ in range(n)]
-        array = ctypes.c_void_p * n
         with on_device(self.dev):
-            rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), array(*[t.data_ptr() for t in pieces]),
-                                              array(*[t.data_ptr() for t in lengths]), self.stream_ptr)
+            rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), self.pointers(*[t.data_ptr() for t in pieces]),
+                                              self.length_pointers, self.stream_ptr)
         _lib.check(rc, "cg_encode_kv_gather")
         step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
         return CacheGenGPUEncoderOutput([CacheGenGPUBytestream(pieces[j], lengths[j], min(step, self.T - j * step))
