@@ -599,6 +599,11 @@ struct EncoderState {
             fhi = span32 ? fhi : e1;
             if (last) fhi = span32;
         }
+        take(flo, fhi, out);
+    }
+    // range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation
+    template <class Sink>
+    CG_HD void take(uint32_t flo, uint32_t fhi, Sink &out) {
         add_to_low(flo, out);
         span32 = fhi - flo;
         const Renorm r = renorm_shift(low, span32 - 1u);
@@ -607,6 +612,31 @@ struct EncoderState {
         low *= r.p2;
         span32 *= r.p2;
         out.nacc += 32u - r.n;
+    }
+    // step_at for NS streams a lane, none of whose symbols is the table's last: their chains are independent, and
+    // the vote is paid once.
+    template <int ROW, int NS, class Sink>
+    static CG_HD void steps_at(Smem sm, const uint32_t (&a)[NS], EncoderState (&enc)[NS], Sink (&out)[NS], uint32_t lanes) {
+        uint32_t e0[NS], e1[NS], flo[NS], fhi[NS];
+        bool rare = false;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            e0[i] = sm.ld(a[i]);
+            e1[i] = sm.ld(a[i] + ROW);
+            flo[i] = cg_umulhi(enc[i].span32, e0[i]);
+            fhi[i] = cg_umulhi(enc[i].span32, e1[i]);
+            rare |= (out[i].nacc >= kSinkHighWater) | (enc[i].span32 == 0u);
+        }
+        if (cg_any_lane(lanes, rare)) {
+#pragma unroll
+            for (int i = 0; i < NS; ++i) {
+                out[i].store_word_if_full();
+                flo[i] = enc[i].span32 ? flo[i] : e0[i];
+                fhi[i] = enc[i].span32 ? fhi[i] : e1[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NS; ++i) enc[i].take(flo[i], fhi[i], out[i]);
     }
     // final flush (enc_new.cu:298-306): two bits that place the stream's value inside the interval, 01 or
     // 10 above the reference's low with its pending bits, which is L plus a quarter of the window cut

@@ -323,13 +323,13 @@ __device__ __forceinline__ uint32_t *scratch_word(uint8_t *scratch, int64_t stri
     return reinterpret_cast<uint32_t *>(scratch + (group * (kGroup / 32) + (tid >> 5)) * 32 * (stride + 4)) + 32 + (tid & 31);
 }
 
-// Exclusive scan of n values in place by one block of kGroup threads; returns the sum.
-template <class T>
+// Exclusive scan of n values in place by one block of THREADS threads; returns the sum.
+template <int THREADS, class T>
 __device__ __forceinline__ int64_t block_scan_in_place(T *v, int n, int64_t *warp_sums, int tid) {
     constexpr int kPer = 8;
     const int lane = tid & 31, w = tid >> 5;
     int64_t base = 0;
-    for (int b = 0; b < n; b += kGroup * kPer) {
+    for (int b = 0; b < n; b += THREADS * kPer) {
         const int at = b + tid * kPer;
         int64_t x[kPer], s = 0;
 #pragma unroll
@@ -348,7 +348,7 @@ __device__ __forceinline__ int64_t block_scan_in_place(T *v, int n, int64_t *war
         __syncthreads();
         int64_t run = base + incl - s;
 #pragma unroll
-        for (int k = 0; k < kGroup / 32; ++k) {
+        for (int k = 0; k < THREADS / 32; ++k) {
             if (k < w) run += warp_sums[k];
             base += warp_sums[k];
         }
@@ -361,142 +361,196 @@ __device__ __forceinline__ int64_t block_scan_in_place(T *v, int n, int64_t *war
     return base;
 }
 
-constexpr int kWordsAhead = 4;  // words (of four symbols) fetched one group ahead of the coder
-
-// One thread per stream, 128 adjacent channels of one row and sub-chunk per block.  TABLES: the chunk is one
+// NS streams per thread, 128 adjacent channels of one row and sub-chunk per block.  TABLES: the chunk is one
 // sub-chunk, so the block's symbols are all there are for its tables: it counts them (each thread in its
-// own shared-memory column, where its table then stands), writes the tables out and codes; the symbols'
+// own shared-memory columns, where its tables then stand), writes the tables out and codes; the symbols'
 // second read comes from the L2.  Otherwise the tables come from packed_tables_kernel.
 // The last block of a sub-chunk turns the group sizes into offsets, the last of all writes the tail.
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
-// chunk takes 122 us with its tables, 0.55 T symbols/s, where the coder alone took 160 us at first and 129 without
+// chunk takes 118 us with its tables, 0.57 T symbols/s, where the coder alone took 160 us at first and 129 without
 // the pending-bit count, the tables being a part of the quantise pass.  Eight blocks an SM leave the compiler 64
 // registers; the shared memory asked for on top evens the last wave out (even_waves_smem).
-template <bool TABLES>
-__global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_constant__ StoreParams p) {
+// Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
+// channels in 165 us, 180 with one.  The tables' part wants the warps more than the chains (a 256-token chunk
+// 129 us with two), so it keeps one; and so does a last group of channels that would leave the second without work.
+template <bool TABLES, int NS>
+__global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_kernel(const __grid_constant__ StoreParams p) {
+    constexpr int kThreads = kGroup / NS, kWarps = kThreads / 32;
+    constexpr int kWordsAhead = NS == 1 ? 4 : 2;  // words (of four symbols) fetched one group ahead of the coder
     extern __shared__ uint4 smem4[];
     uint32_t *tab = reinterpret_cast<uint32_t *>(smem4);
-    __shared__ int64_t warp_sums[kGroup / 32];
-    __shared__ int block_sums[2][kGroup / 32];
+    __shared__ int64_t warp_sums[kWarps];
+    __shared__ int block_sums[2][kWarps];
     __shared__ int last_block;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.y, sub = blockIdx.z, nslab = gridDim.x;
-    const int c = blockIdx.x * kGroup + tid;
-    const bool active = c < p.nchannels;
-    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, active);
     const int t0 = sub * kSubTokens, n = min(kSubTokens, p.ntokens - t0);
     const int64_t C = p.nchannels;
-    const int64_t g = row * C + c;
-    uint32_t *column = tab + warp * 32 * p.lp + lane;
-    const uint32_t col = smem_addr(column);
-    const uint32_t *sp = p.sym4 + (static_cast<int64_t>(row) * ((p.ntokens + 3) / 4) + t0 / 4) * C + c;
+    // channel s of this thread is number tid + kThreads * s of the group; one past the last channel repeats the last
+    // and is written nowhere but to its own scratch row
+    bool active[NS];
+    int64_t g[NS];
+    uint32_t *column[NS];
+    uint32_t col[NS];
+    const uint32_t *sp[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const int slot = s * kThreads + tid, c = min(blockIdx.x * kGroup + slot, p.nchannels - 1);
+        active[s] = blockIdx.x * kGroup + slot < p.nchannels;
+        g[s] = row * C + c;
+        column[s] = tab + (slot >> 5) * 32 * p.lp + lane;
+        col[s] = smem_addr(column[s]);
+        sp[s] = p.sym4 + (static_cast<int64_t>(row) * ((p.ntokens + 3) / 4) + t0 / 4) * C + c;
+    }
+    // the same for a warp; with two streams every warp has channels
+    const bool any_active = NS > 1 || blockIdx.x * kGroup + warp * 32 < p.nchannels;
     uint32_t bad = 0;
     int nbytes = 0, nz = 0;
 
-    if (TABLES) {
+    if (TABLES && any_active) {
         uint16_t *stage = reinterpret_cast<uint16_t *>(tab + p.lp * kGroup);
         bool overflow = false;
-        if (active) {
-            for (int m = 0; m < p.lp; ++m) column[m * 32] = 0u;
-            const uint32_t *q = sp;
-            constexpr int kAhead = 16;  // words in flight: the counts of one group cover the loads of the next warp's
-            int i = 0;
-            for (; i + 4 * kAhead <= n; i += 4 * kAhead) {
-                uint32_t w[kAhead], any = 0u;
+        for (int m = 0; m < p.lp; ++m) {
 #pragma unroll
-                for (int k = 0; k < kAhead; ++k) {
-                    w[k] = __ldg(q);
-                    q += C;
-                }
+            for (int s = 0; s < NS; ++s) column[s][m * 32] = 0u;
+        }
+        constexpr int kAhead = 16 / NS;  // words of a channel in flight
+        const uint32_t *q[NS];
 #pragma unroll
-                for (int k = 0; k < kAhead; ++k) any |= w[k];
-                if (any & 0x80808080u) {  // reported below
+        for (int s = 0; s < NS; ++s) q[s] = sp[s];
+        int i = 0;
+        for (; i + 4 * kAhead <= n; i += 4 * kAhead) {
+            uint32_t w[NS][kAhead], any = 0u;
 #pragma unroll
-                    for (int k = 0; k < kAhead; ++k) w[k] = 0u;
-                }
+            for (int k = 0; k < kAhead; ++k) {
 #pragma unroll
-                for (int k = 0; k < kAhead; ++k) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) count_symbol(entry_of(col, w[k], j));
+                for (int s = 0; s < NS; ++s) {
+                    w[s][k] = __ldg(q[s]);
+                    q[s] += C;
                 }
             }
-            for (; i < n; i += 4) {
-                uint32_t w = __ldg(q);
-                q += C;
+#pragma unroll
+            for (int k = 0; k < kAhead * NS; ++k) any |= w[k / kAhead][k % kAhead];
+            if (any & 0x80808080u) {  // reported below
+#pragma unroll
+                for (int k = 0; k < kAhead * NS; ++k) w[k / kAhead][k % kAhead] = 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) count_symbol(entry_of(col[s], w[s][k], j));
+                }
+            }
+        }
+        for (; i < n; i += 4) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                uint32_t w = __ldg(q[s]);
+                q[s] += C;
                 if (w & 0x80808080u) w = 0u;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (i + j < n) count_symbol(entry_of(col, w, j));
+                    if (i + j < n) count_symbol(entry_of(col[s], w, j));
             }
-            const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
-            if (p.out.counts)
-                nz = store_counts<32>(column, p.lp, cq, p.out.counts + __ldg(p.out.table_row_off + row) + c, C, &overflow);
-            counts_to_column<32>(column, stage + tid * p.lp, p.lp, n, cq);
+        }
+        const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
+        const int64_t at = p.out.counts ? __ldg(p.out.table_row_off + row) - row * C : 0;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            if (p.out.counts && active[s]) nz += store_counts<32>(column[s], p.lp, cq, p.out.counts + at + g[s], C, &overflow);
+            counts_to_column<32>(column[s], stage + (s * kThreads + tid) * p.lp, p.lp, n, cq);
         }
         if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
         __syncwarp();
-        const int first = blockIdx.x * kGroup + warp * 32;
-        const int nch = min(32, p.nchannels - first);
-        if (nch > 0)
-            copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp,
-                        nch * p.lp, lane);
-    } else if (active) {
-        stage_table_column<false, 32>(column, p.out.cdf + g * p.lp, p.lp, p.lp, 0);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int slot = s * kThreads + warp * 32, first = blockIdx.x * kGroup + slot;
+            const int nch = min(32, p.nchannels - first);
+            if (nch > 0)
+                copy_tables(stage + slot * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp,
+                            nch * p.lp, lane);
+        }
+    } else if (any_active) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) stage_table_column<false, 32>(column[s], p.out.cdf + g[s] * p.lp, p.lp, p.lp, 0);
     }
 
-    if (active) {
-        const int64_t slot = static_cast<int64_t>(sub) * p.nrows * C + g;
+    if (any_active) {
         const uint32_t top = static_cast<uint32_t>(p.lp - 2);
-        BitSinkT<32, false> out;  // see scratch_word
-        out.init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x, tid)),
-                 p.stride);
-        EncoderState enc;
-        enc.init();
-        constexpr int kAhead = 4 * kWordsAhead;
-        uint32_t w[kWordsAhead], next[kWordsAhead];
+        BitSinkT<32, false> out[NS];  // see scratch_word
+        EncoderState enc[NS];
+        uint32_t w[NS][kWordsAhead], next[NS][kWordsAhead];
 #pragma unroll
-        for (int k = 0; k < kWordsAhead; ++k) w[k] = 4 * k < n ? __ldg(sp + k * C) : 0u;
+        for (int s = 0; s < NS; ++s) {
+            out[s].init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x, s * kThreads + tid)),
+                        p.stride);
+            enc[s].init();
+#pragma unroll
+            for (int k = 0; k < kWordsAhead; ++k) w[s][k] = 4 * k < n ? __ldg(sp[s] + k * C) : 0u;
+        }
+        constexpr int kAhead = 4 * kWordsAhead;
         int i = 0;
         for (; i + kAhead <= n; i += kAhead) {
-            sp += kWordsAhead * C;
+            uint32_t any = 0u;
 #pragma unroll
-            for (int k = 0; k < kWordsAhead; ++k) next[k] = i + kAhead + 4 * k < n ? __ldg(sp + k * C) : 0u;
-            const uint32_t any = w[0] | w[1] | w[2] | w[3];
+            for (int s = 0; s < NS; ++s) {
+                sp[s] += kWordsAhead * C;
+#pragma unroll
+                for (int k = 0; k < kWordsAhead; ++k) {
+                    next[s][k] = i + kAhead + 4 * k < n ? __ldg(sp[s] + k * C) : 0u;
+                    any |= w[s][k];
+                }
+            }
             if (any & 0x80808080u) {
                 bad = 1u;
 #pragma unroll
-                for (int k = 0; k < kWordsAhead; ++k) w[k] = 0u;
+                for (int k = 0; k < kWordsAhead * NS; ++k) w[k / kWordsAhead][k % kWordsAhead] = 0u;
             }
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    enc.step_at<kWarpRow>(Smem{}, entry_of(col, w[k], j), false, out, lanes);
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t a[NS];
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) a[s] = entry_of(col[s], w[s][k], j);
+                    EncoderState::steps_at<kWarpRow>(Smem{}, a, enc, out, 0xFFFFFFFFu);
+                }
             }
 #pragma unroll
-            for (int k = 0; k < kWordsAhead; ++k) w[k] = next[k];
+            for (int k = 0; k < kWordsAhead * NS; ++k) w[k / kWordsAhead][k % kWordsAhead] = next[k / kWordsAhead][k % kWordsAhead];
         }
         for (; i < n; ++i) {  // fewer than kAhead left, all in w
-            uint32_t s = w[0] & 0xFFu;
-            if (s >= top) {
-                bad = 1u;
-                s = 0u;
-            }
-            enc.step_at<kWarpRow>(Smem{}, col + s * kWarpRow, false, out, lanes);
-            w[0] >>= 8;
-            if ((i & 3) == 3) {
+            uint32_t a[NS];
 #pragma unroll
-                for (int k = 0; k + 1 < kWordsAhead; ++k) w[k] = w[k + 1];
+            for (int s = 0; s < NS; ++s) {
+                uint32_t m = w[s][0] & 0xFFu;
+                if (m >= top) {
+                    bad = 1u;
+                    m = 0u;
+                }
+                a[s] = col[s] + m * kWarpRow;
+                w[s][0] >>= 8;
+                if ((i & 3) == 3) {
+#pragma unroll
+                    for (int k = 0; k + 1 < kWordsAhead; ++k) w[s][k] = w[s][k + 1];
+                }
             }
+            EncoderState::steps_at<kWarpRow>(Smem{}, a, enc, out, 0xFFFFFFFFu);
         }
-        nbytes = static_cast<int>(enc.flush(out));
-        p.lengths[slot] = nbytes;
-        int bits = 0;
-        if (nbytes > p.stride) {
-            bits |= CG_S_STREAM_OVERFLOW;
-            nbytes = static_cast<int>(p.stride);
+        int bits = bad ? CG_S_BAD_SYMBOL : 0;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            int len = static_cast<int>(enc[s].flush(out[s]));
+            if (!active[s]) continue;
+            p.lengths[static_cast<int64_t>(sub) * p.nrows * C + g[s]] = len;
+            if (len > p.stride) {
+                bits |= CG_S_STREAM_OVERFLOW;
+                len = static_cast<int>(p.stride);
+            }
+            nbytes += len;
         }
-        if (bad) bits |= CG_S_BAD_SYMBOL;
         if (bits) atomicOr(p.status, bits);
     }
 
@@ -512,7 +566,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     int64_t *goff = p.group_off + static_cast<int64_t>(sub) * ngroups;
     if (tid == 0) {
         int s = 0, z = 0;
-        for (int k = 0; k < kGroup / 32; ++k) {
+        for (int k = 0; k < kWarps; ++k) {
             s += block_sums[0][k];
             z += block_sums[1][k];
         }
@@ -524,7 +578,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     __syncthreads();
     if (!last_block) return;
     __threadfence();
-    const int64_t bytes = block_scan_in_place(goff, ngroups, warp_sums, tid);
+    const int64_t bytes = block_scan_in_place<kThreads>(goff, ngroups, warp_sums, tid);
     if (tid == 0) {
         p.sub_bytes[sub] = bytes;
         __threadfence();
@@ -535,7 +589,7 @@ __global__ void __launch_bounds__(kGroup, 8) store_encode_kernel(const __grid_co
     __threadfence();
     int64_t nz_total = 0;
     if (p.out.group_nz) {
-        nz_total = block_scan_in_place(p.out.group_nz, ngroups, warp_sums, tid);
+        nz_total = block_scan_in_place<kThreads>(p.out.group_nz, ngroups, warp_sums, tid);
         if (tid == 0) p.out.group_nz[ngroups] = static_cast<uint32_t>(nz_total);
     }
     if (tid == 0) {
@@ -795,8 +849,8 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
     if (z.nsub == 1) {
         const size_t smem = even_waves_smem(blocks, columns + staged, 128);
-        allow_smem(store_encode_kernel<true>, smem);
-        store_encode_kernel<true><<<grid, kGroup, smem, st>>>(p);
+        allow_smem(store_encode_kernel<true, 1>, smem);
+        store_encode_kernel<true, 1><<<grid, kGroup, smem, st>>>(p);
         return check_launch();
     }
     allow_smem(packed_tables_kernel, columns + staged);
@@ -804,8 +858,15 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
                                                                                          p.out, status);
     if (int rc = check_launch()) return rc;
     const size_t smem = even_waves_smem(blocks, columns, 128);
-    allow_smem(store_encode_kernel<false>, smem);
-    store_encode_kernel<false><<<grid, kGroup, smem, st>>>(p);
+    // two streams a thread unless the last group has channels for the first alone
+    const int last = z.nchannels % kGroup;
+    if (last == 0 || last > kGroup / 2) {
+        allow_smem(store_encode_kernel<false, 2>, smem);
+        store_encode_kernel<false, 2><<<grid, kGroup / 2, smem, st>>>(p);
+    } else {
+        allow_smem(store_encode_kernel<false, 1>, smem);
+        store_encode_kernel<false, 1><<<grid, kGroup, smem, st>>>(p);
+    }
     return check_launch();
 }
 
