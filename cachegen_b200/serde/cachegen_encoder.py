@@ -19,7 +19,6 @@ import ctypes
 import dataclasses
 import functools
 import threading
-import weakref
 from typing import Tuple
 
 import torch
@@ -272,14 +271,15 @@ def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = N
 
 
 class _BinsInfo:
-    """What a pair of bins tensors means to an encode: read back from the GPU once, not on every call."""
+    """What the values of a pair of bins tensors mean to an encode.  Tensors on a GPU are read back here, which waits
+    for it, and what is kept belongs to these values: whoever keeps an info must know that the tensors it came from
+    have not been written to since (see CacheGenSerializer._bins)."""
 
     def __init__(self, key_bins, value_bins):
-        self.value_ref = weakref.ref(value_bins)
-        self.versions = (key_bins._version, value_bins._version)
-        self.cpu = torch.cat((key_bins.detach().cpu(), value_bins.detach().cpu())).to(torch.float32)
-        self.nlayers = key_bins.numel()
-        self.kmax, self.vmax = int(key_bins.max()), int(value_bins.max())
+        keys, values = (t.detach().cpu().to(torch.float32) for t in (key_bins, value_bins))
+        self.cpu = torch.cat((keys, values))
+        self.nlayers = keys.numel()
+        self.kmax, self.vmax = int(keys.max()), int(values.max())
         self.on_device = {}   # device -> float32 [2L]
         self.sparse = flat_format.sparse_representable(self.cpu)
         self.checksums = {}   # delta settings -> bins_checksum
@@ -319,25 +319,6 @@ class _BinsInfo:
         if self.kmax != self.vmax:
             raise RuntimeError(f"Sizes of tensors must match: key tables have {self.kmax + 1} entries, value tables {self.vmax + 1}")
         return self.kmax
-
-
-_BINS_INFOS = {}  # id of a living key tensor -> (weak reference to it, _BinsInfo)
-
-
-def _bins_info(key_bins: torch.Tensor, value_bins: torch.Tensor) -> _BinsInfo:
-    """The pair's _BinsInfo, kept while the key tensor lives and for as long as neither is written to."""
-    key = id(key_bins)
-    ref, info = _BINS_INFOS.get(key, (None, None))
-    if (ref is None or ref() is not key_bins or info.value_ref() is not value_bins or
-            info.versions != (key_bins._version, value_bins._version)):
-        info = _BinsInfo(key_bins, value_bins)
-        _BINS_INFOS[key] = (weakref.ref(key_bins, lambda gone, key=key: _forget_bins(key, gone)), info)
-    return info
-
-
-def _forget_bins(key, gone):
-    if _BINS_INFOS.get(key, (None,))[0] is gone:
-        del _BINS_INFOS[key]
 
 
 _local = threading.local()
@@ -453,7 +434,7 @@ class _PendingChunk:
 
 
 def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tensor, chunk_tokens: int,
-                batch: int = 16, max_bins: int = None, delta=None, streams: int = 3) -> list:
+                batch: int = 16, max_bins: int = None, delta=None, streams: int = 3, info: _BinsInfo = None) -> list:
     """Encodes a whole KV cache [L, 2, T, H, D] (GPU, unit innermost stride) chunk by chunk, as
     LMCacheEngine.store does with one to_bytes call per chunk (LMCache/lmcache/cache_engine.py:205-255
     in the reference), but without waiting for a chunk's payload size before the next chunk's kernels
@@ -461,8 +442,9 @@ def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     turn to be replaced comes, so the host waits for sizes that arrived long ago.  Every chunk in
     flight keeps its own workspace (200 MB for a 7B-shape chunk).  Consecutive chunks run on `streams` side
     streams in turn (see _side_streams); the caller's stream waits for them before the call returns.
-    Returns the chunks' CacheGenGPUEncoderOutput objects, identical to per-chunk encode_function calls."""
-    info = _bins_info(key_bins, value_bins)
+    Returns the chunks' CacheGenGPUEncoderOutput objects, identical to per-chunk encode_function calls.
+    `info`: what the bins are, when the caller knows (see CacheGenSerializer._bins); read from the tensors otherwise."""
+    info = info or _BinsInfo(key_bins, value_bins)
     kmax = info.table_bins(max_bins)
     T = kv.shape[2]
     info.on(kv.device)
@@ -521,9 +503,12 @@ def encode_levels(kv: torch.Tensor, levels: list) -> list:
     store per chunk (one blob per QUANT_LEVEL, run_adaptation.py:61-72) so that config_selection can
     pick a level per chunk (src/utils.py:294-314).  All levels are enqueued before the host waits for the
     first one's size."""
+    return _encode_infos(kv, [_BinsInfo(kb, vb) for kb, vb in levels])
+
+
+def _encode_infos(kv, infos) -> list:
     if kv.stride(4) != 1:
         kv = kv.contiguous()
-    infos = [_bins_info(kb, vb) for kb, vb in levels]
     pending = []
     try:
         for info in infos:
@@ -536,11 +521,11 @@ def encode_levels(kv: torch.Tensor, levels: list) -> list:
 
 @_lmcache_nvtx_annotate
 def encode_function(kv: torch.Tensor, config: CacheGenConfig, key_bins: torch.Tensor, value_bins: torch.Tensor,
-                    chunk_size: int, max_bins: int = None, delta=None) -> CacheGenGPUEncoderOutput:
-    """Encodes one chunk of KV, [L, 2, T, H, D] on the GPU, T == chunk_size (enc.py:247-301)."""
+                    chunk_size: int, max_bins: int = None, delta=None, info: _BinsInfo = None) -> CacheGenGPUEncoderOutput:
+    """Encodes one chunk of KV, [L, 2, T, H, D] on the GPU, T == chunk_size (enc.py:247-301).  `info`: as for encode_many."""
     if kv.shape[2] != chunk_size:
         raise RuntimeError(f"chunk_size {chunk_size} does not match the {kv.shape[2]} tokens of the blob")
-    info = _bins_info(key_bins, value_bins)
+    info = info or _BinsInfo(key_bins, value_bins)
     return _PendingChunk(kv, info, info.table_bins(max_bins), delta=delta).finish()
 
 
@@ -568,13 +553,13 @@ def pack_sparse_tables(counts: torch.Tensor, bins: torch.Tensor, nchannels: int,
 
 
 def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tensor,
-                compact_tables=True, max_bins: int = None, delta=None) -> flat_format.FlatChunk:
+                compact_tables=True, max_bins: int = None, delta=None, info: _BinsInfo = None) -> flat_format.FlatChunk:
     """Encodes one chunk of KV, [L, 2, T, H, D] on the GPU, into a CGB2 container on the GPU
     (flat_format.py): the same tables, lengths and streams as encode_function, with uint16 lengths and
     the tables in the smallest form that can hold them.  compact_tables: True (sparse byte counts when
     every non-centre histogram count fits a byte and no row has more than 32 of them, else dense byte
     counts when the counts fit, else the int16 tables), "counts" (never sparse) or False (always int16)."""
-    info = _bins_info(key_bins, value_bins)
+    info = info or _BinsInfo(key_bins, value_bins)
     kmax = info.table_bins(max_bins)
     p = _PendingChunk(kv, info, kmax, delta=delta, with_counts=True)
     offs, bits, nonzero = p.sizes()
@@ -621,9 +606,47 @@ class CacheGenSerializer(Serializer):
         self.cachegen_config = cachegen_config or CacheGenConfig.from_model_name(metadata.model_name)
         self.chunk_size = config.chunk_size
         self.fmt = metadata.fmt
-        self.key_bins = self.make_key_bins(self.cachegen_config)
-        self.value_bins = self.make_value_bins(self.cachegen_config)
-        self._levels = {}
+        self._key_bins = self.make_key_bins(self.cachegen_config)
+        self._value_bins = self.make_value_bins(self.cachegen_config)
+        # the values are known from the configuration, unless a subclass makes the tensors its own way
+        cls, own = type(self), CacheGenSerializer
+        self._bins_shared = cls.make_key_bins is not own.make_key_bins or cls.make_value_bins is not own.make_value_bins
+        self._info = (_BinsInfo(self._key_bins, self._value_bins) if self._bins_shared else
+                      self._config_info(self.cachegen_config))
+        self._levels = {}  # settings -> _BinsInfo
+
+    # The bins tensors are the caller's to read, write and replace.  Once one has been handed out, or was handed in, nothing
+    # says whether it has been written to (a tensor made in inference mode has no version counter, and writes
+    # through .data do not count in one): from then on every call reads them back.
+    @property
+    def key_bins(self) -> torch.Tensor:
+        self._bins_shared = True
+        return self._key_bins
+
+    @key_bins.setter
+    def key_bins(self, bins: torch.Tensor) -> None:
+        self._key_bins, self._bins_shared = bins, True
+
+    @property
+    def value_bins(self) -> torch.Tensor:
+        self._bins_shared = True
+        return self._value_bins
+
+    @value_bins.setter
+    def value_bins(self, bins: torch.Tensor) -> None:
+        self._value_bins, self._bins_shared = bins, True
+
+    def _bins(self) -> _BinsInfo:
+        info = self._info
+        if self._bins_shared:
+            now = _BinsInfo(self._key_bins, self._value_bins)
+            if now.nlayers != info.nlayers or not torch.equal(now.cpu, info.cpu):
+                info = self._info = now
+        return info
+
+    @staticmethod
+    def _config_info(config: CacheGenConfig) -> _BinsInfo:
+        return _BinsInfo(CGBasics.make_key_bins(config, "cpu"), CGBasics.make_value_bins(config, "cpu"))
 
     def make_key_bins(self, config: CacheGenConfig) -> torch.Tensor:
         return CGBasics.make_key_bins(config, "cuda")
@@ -636,8 +659,8 @@ class CacheGenSerializer(Serializer):
         if self.fmt == "huggingface":
             tensor = tensor.permute(0, 1, 3, 2, 4)  # a view; the kernels read it through its strides
         ntokens = tensor.shape[2]
-        return encode_function(tensor.cuda(), self.cachegen_config, self.key_bins, self.value_bins, ntokens,
-                               max_bins=self.table_max_bins, delta=self.delta)
+        return encode_function(tensor.cuda(), self.cachegen_config, self._key_bins, self._value_bins, ntokens,
+                               max_bins=self.table_max_bins, delta=self.delta, info=self._bins())
 
     def encode_many(self, tensor: torch.Tensor, chunk_tokens: int = None, batch: int = 16, streams: int = 3) -> list:
         """A whole KV cache, one encoded chunk per `chunk_tokens` (default: the configured chunk size)
@@ -647,8 +670,8 @@ class CacheGenSerializer(Serializer):
         tensor = tensor.cuda()
         if tensor.stride(4) != 1:
             tensor = tensor.contiguous()
-        return encode_many(tensor, self.key_bins, self.value_bins, chunk_tokens or self.chunk_size, batch,
-                           max_bins=self.table_max_bins, delta=self.delta, streams=streams)
+        return encode_many(tensor, self._key_bins, self._value_bins, chunk_tokens or self.chunk_size, batch,
+                           max_bins=self.table_max_bins, delta=self.delta, streams=streams, info=self._bins())
 
     def encode_levels(self, tensor: torch.Tensor, cachegen_configs: list) -> list:
         """The chunk encoded with each of `cachegen_configs` (CacheGenConfig objects, e.g. the three
@@ -656,16 +679,15 @@ class CacheGenSerializer(Serializer):
         a serializer built with that configuration returns from `encode`."""
         if self.fmt == "huggingface":
             tensor = tensor.permute(0, 1, 3, 2, 4)
-        tensor = tensor.cuda()
-        return encode_levels(tensor, [self._level_bins(c, tensor.device) for c in cachegen_configs])
+        return _encode_infos(tensor.cuda(), [self._level_info(c) for c in cachegen_configs])
 
-    def _level_bins(self, config: CacheGenConfig, device):
+    def _level_info(self, config: CacheGenConfig) -> _BinsInfo:
         """The bins of a quality level, made once per setting."""
-        key = (device, dataclasses.astuple(config))
-        bins = self._levels.get(key)
-        if bins is None:
-            bins = self._levels[key] = (CGBasics.make_key_bins(config, device), CGBasics.make_value_bins(config, device))
-        return bins
+        key = dataclasses.astuple(config)
+        info = self._levels.get(key)
+        if info is None:
+            info = self._levels[key] = self._config_info(config)
+        return info
 
     def encode_flat(self, tensor: torch.Tensor, compact_tables=True) -> flat_format.FlatChunk:
         """The chunk as a CGB2 container on the GPU."""
@@ -674,8 +696,8 @@ class CacheGenSerializer(Serializer):
         tensor = tensor.cuda()
         if tensor.stride(4) != 1:
             tensor = tensor.contiguous()
-        return encode_flat(tensor, self.key_bins, self.value_bins, compact_tables, max_bins=self.table_max_bins,
-                           delta=self.delta)
+        return encode_flat(tensor, self._key_bins, self._value_bins, compact_tables, max_bins=self.table_max_bins,
+                           delta=self.delta, info=self._bins())
 
     @_lmcache_nvtx_annotate
     def to_bytes(self, tensor: torch.Tensor) -> bytes:

@@ -1,0 +1,95 @@
+"""The bins an encode runs with are those that the tensors hold at the call, however they were made or written to."""
+import pytest
+import torch
+
+
+def configs():
+    from cachegen_b200.serde.cachegen_basics import CacheGenConfig
+    base = CacheGenConfig(1, 2, 4, 32, 16, 16, 2, 32, 16)
+    return base, base.with_bins_divided(2)
+
+
+def serializer(config):
+    from cachegen_b200.config import LMCacheEngineConfig, LMCacheEngineMetadata
+    from cachegen_b200.serde import CacheGenSerializer
+    return CacheGenSerializer(LMCacheEngineConfig.from_defaults(chunk_size=256),
+                              LMCacheEngineMetadata("bins", 1, 0, "vllm"), config)
+
+
+def make_kv():
+    return torch.randn((4, 2, 70, 2, 64), generator=torch.Generator().manual_seed(4)).half().cuda()
+
+
+def parts(eo):
+    return [eo.cdf, eo.max_tensors_key.view(torch.int16), eo.max_tensors_value.view(torch.int16),
+            eo.data_chunks[0].bytestream, eo.data_chunks[0].bytestream_lengths]
+
+
+def same(a, b):
+    return all(torch.equal(x, y) for x, y in zip(parts(a), parts(b)))
+
+
+def test_bins_made_in_inference_mode():
+    from cachegen_b200.serde import cachegen_basics as B, cachegen_encoder as E
+    base, _ = configs()
+    with torch.inference_mode():
+        info = E._BinsInfo(B.make_key_bins(base, "cpu"), B.make_value_bins(base, "cpu"))
+    assert info.cpu.tolist() == [32, 16, 16, 16, 32, 32, 16, 16] and info.table_bins() == 32
+
+
+@pytest.mark.gpu
+def test_a_serializer_made_in_inference_mode_encodes():
+    base, half = configs()
+    kv = make_kv()
+    want, want_half = serializer(base).encode(kv), serializer(half).encode(kv)
+    flat, many = serializer(base).encode_flat(kv), serializer(base).encode_many(kv, 30)
+    with torch.inference_mode():
+        ser = serializer(base)
+        assert same(ser.encode(kv), want)
+        assert all(same(a, b) for a, b in zip(ser.encode_levels(kv, [base, half]), (want, want_half)))
+        assert all(same(a, b) for a, b in zip(ser.encode_many(kv, 30), many))
+        assert torch.equal(ser.encode_flat(kv).blob, flat.blob)
+        assert len(ser.key_bins) == 4 and same(ser.encode(kv), want)
+    assert same(ser.encode(kv), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("inference", [False, True])
+def test_bins_that_were_written_to(inference):
+    from cachegen_b200.serde import cachegen_basics as B, cachegen_encoder as E
+    base, half = configs()
+    kv = make_kv()
+    want, want_half = serializer(base).encode(kv), serializer(half).encode(kv)
+    with torch.inference_mode(inference):
+        kb, vb = B.make_key_bins(base), B.make_value_bins(base)
+        assert same(E.encode_function(kv, None, kb, vb, 70), want)
+        kb.data.copy_(B.make_key_bins(half))  # no version counter sees this
+        vb.data.copy_(B.make_value_bins(half))
+        assert same(E.encode_function(kv, None, kb, vb, 70), want_half)
+
+        ser = serializer(base)
+        assert same(ser.encode(kv), want)
+        ser.key_bins.data.copy_(kb)
+        ser.value_bins.copy_(vb)
+        assert same(ser.encode(kv), want_half)
+        ser.key_bins, ser.value_bins = B.make_key_bins(base), B.make_value_bins(base)
+        assert same(ser.encode(kv), want)
+        assert torch.equal(ser.encode_flat(kv).blob, serializer(base).encode_flat(kv).blob)
+
+
+@pytest.mark.gpu
+def test_bins_of_a_subclass():
+    from cachegen_b200.serde import CacheGenSerializer
+    base, half = configs()
+
+    class Halved(CacheGenSerializer):
+        def make_key_bins(self, config):
+            return super().make_key_bins(half)
+
+        def make_value_bins(self, config):
+            return super().make_value_bins(half)
+
+    plain = serializer(half)
+    ser = Halved(type("C", (), {"chunk_size": 256}), type("M", (), {"fmt": "vllm"}), base)
+    kv = make_kv()
+    assert same(ser.encode(kv), plain.encode(kv))
