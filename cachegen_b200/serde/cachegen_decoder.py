@@ -116,12 +116,24 @@ def _staged(t: torch.Tensor, dev) -> torch.Tensor:
 
 
 class _HostBins:
-    """What the bins a decoder was set up with say about the containers it reads; kept in its workspace."""
+    """What the bins of a decode say about the containers it reads and about delta coding.  The values of a tensor
+    on a GPU are read back when they are first asked for, which plain pickled chunks never do."""
 
     def __init__(self, bins: torch.Tensor):
-        self.cpu = bins.cpu()
-        self.sparse = flat_format.sparse_representable(self.cpu)
+        self._bins = bins
         self._checksums, self._counts, self._sparse = {}, {}, {}
+
+    @functools.cached_property
+    def cpu(self) -> torch.Tensor:
+        return self._bins.cpu()
+
+    @functools.cached_property
+    def values(self) -> tuple:
+        return tuple(self.cpu.tolist())
+
+    @functools.cached_property
+    def sparse(self) -> bool:
+        return flat_format.sparse_representable(self.cpu)
 
     def checksum(self, delta) -> int:
         key = None if delta is None else (delta.group, delta.divisor, delta.rows)
@@ -227,7 +239,7 @@ class DecodePlan:
 
     def __init__(self, encoder_outputs: list, bins: torch.Tensor, fmt: str,
                  out_dtype: torch.dtype, out: torch.Tensor = None, workspace: dict = None, device=None,
-                 peer_out: bool = False, delta=None):
+                 peer_out: bool = False, delta=None, host_bins: _HostBins = None):
         if not encoder_outputs:
             raise RuntimeError("nothing to decode")
         if fmt not in ("vllm", "huggingface"):
@@ -236,9 +248,8 @@ class DecodePlan:
         dev = torch.device(device) if device is not None else (
             _device_of(first) if _on_gpu(first) else torch.device("cuda", torch.cuda.current_device()))
         ws = workspace if workspace is not None else {}
-        host_bins = ws.get("host_bins")
-        if host_bins is None or host_bins.cpu.numel() != bins.numel():
-            host_bins = ws["host_bins"] = _HostBins(bins)
+        if host_bins is None:  # a workspace may serve calls with other bins
+            host_bins = _HostBins(bins)
         with on_device(dev):
             views = [_ChunkView(eo, dev, host_bins, delta) for eo in encoder_outputs]
         v0 = views[0]
@@ -279,10 +290,10 @@ class DecodePlan:
         for kind, name, fn in ((_lib.CG_TABLES_COUNTS, "table_row_off", flat_format.table_row_offsets),
                                (_lib.CG_TABLES_SPARSE, "mask_row_off", flat_format.mask_row_offsets)):
             if any(v.table_kind == kind for v in views):
-                t = ws.get(name)
-                if t is None or t.device != dev or ws.get(name + "_c") != C:
+                t, key = ws.get(name), (C, host_bins.values)
+                if t is None or t.device != dev or ws.get(name + "_of") != key:
                     t = torch.tensor(fn(host_bins.cpu, C), dtype=torch.int64, device=dev)
-                    ws[name], ws[name + "_c"] = t, C
+                    ws[name], ws[name + "_of"] = t, key
                 row_offs[kind] = t
 
         esz = out.element_size()
@@ -376,7 +387,8 @@ class DecodePlan:
 
 
 def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Tensor, fmt: str,
-                out_dtype: torch.dtype, out: torch.Tensor = None, workspace: dict = None, delta=None) -> torch.Tensor:
+                out_dtype: torch.dtype, out: torch.Tensor = None, workspace: dict = None, delta=None,
+                host_bins: _HostBins = None) -> torch.Tensor:
     """Fused decode of consecutive encoded chunks of one KV cache into one blob.
 
     The chunks' tokens are laid one after the other along the token axis of the result, which has
@@ -388,9 +400,11 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
     The chunks' tensors may live on the GPU or in (pinned) host memory; host tensors are copied to the
     GPU on the current stream first.  bins: float32 [2L] on the GPU (key bins then value bins).
     `out`, when given, must have the result's shape and dtype with a unit innermost stride (any other
-    strides).  `workspace` caches the small offset / status buffers between calls.
+    strides).  `workspace` caches the small offset / status buffers between calls.  `host_bins`: the values of `bins`,
+    when the caller knows them; read from the tensor otherwise, if the chunks ask for them.
     """
-    return DecodePlan(encoder_outputs, bins, fmt, out_dtype, out=out, workspace=workspace, delta=delta).run()
+    return DecodePlan(encoder_outputs, bins, fmt, out_dtype, out=out, workspace=workspace, delta=delta,
+                      host_bins=host_bins).run()
 
 
 _copy_streams = {}
@@ -409,17 +423,19 @@ def _chunk_tokens(eo) -> int:
 
 def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Tensor, fmt: str,
                           out_dtype: torch.dtype, out: torch.Tensor = None, groups: int = 4,
-                          workspaces: list = None, delta=None) -> torch.Tensor:
+                          workspaces: list = None, delta=None, host_bins: _HostBins = None) -> torch.Tensor:
     """decode_many for encoded chunks held in pinned host memory, with the host-to-device copies of
     one group of chunks overlapped with the decode of the previous group (a copy stream per device;
-    the decode launches stay on the caller's current stream).  `workspaces`: one dict per group."""
+    the decode launches stay on the caller's current stream).  `workspaces`: one dict per group; `host_bins`: as for
+    decode_many."""
+    host_bins = host_bins or _HostBins(bins)
     n = len(encoder_outputs)
     groups = max(1, min(groups, n))
     first = encoder_outputs[0]
     dev = _device_of(first) if _on_gpu(first) else torch.device("cuda", torch.cuda.current_device())
     if groups == 1 or _on_gpu(first):
         return decode_many(encoder_outputs, bins, fmt, out_dtype, out=out,
-                           workspace=workspaces[0] if workspaces else None)
+                           workspace=workspaces[0] if workspaces else None, host_bins=host_bins)
     L, H, D = bins.numel() // 2, first.num_heads, first.head_size
     total_T = sum(_chunk_tokens(eo) for eo in encoder_outputs)
     shape = (L, 2, total_T, H, D) if fmt == "vllm" else (L, 2, H, total_T, D)
@@ -442,7 +458,8 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
         view = out[:, :, t0:t0 + tg] if fmt == "vllm" else out[:, :, :, t0:t0 + tg]
         with torch.cuda.stream(copy_stream):
             part = _stage_flat(part, workspaces[g], dev)
-            plan = DecodePlan(part, bins, fmt, out_dtype, out=view, workspace=workspaces[g], device=dev, delta=delta)
+            plan = DecodePlan(part, bins, fmt, out_dtype, out=view, workspace=workspaces[g], device=dev, delta=delta,
+                              host_bins=host_bins)
             ready = torch.cuda.Event()
             ready.record(copy_stream)
         cur.wait_event(ready)
@@ -474,9 +491,9 @@ def _stage_flat(part: list, ws: dict, dev) -> list:
 
 
 def decode_to_kv(encoder_output: CacheGenGPUEncoderOutput, bins: torch.Tensor, fmt: str, out_dtype: torch.dtype,
-                 out: torch.Tensor = None, workspace: dict = None, delta=None) -> torch.Tensor:
+                 out: torch.Tensor = None, workspace: dict = None, delta=None, host_bins: _HostBins = None) -> torch.Tensor:
     """Fused decode of one encoded chunk into its KV blob (see decode_many)."""
-    return decode_many([encoder_output], bins, fmt, out_dtype, out=out, workspace=workspace, delta=delta)
+    return decode_many([encoder_output], bins, fmt, out_dtype, out=out, workspace=workspace, delta=delta, host_bins=host_bins)
 
 
 class CacheGenDeserializer(Deserializer):
@@ -497,6 +514,13 @@ class CacheGenDeserializer(Deserializer):
         self.key_bins = self.make_key_bins(self.cachegen_config)
         self.value_bins = self.make_value_bins(self.cachegen_config)
         self._bins = torch.cat((self.key_bins, self.value_bins)).contiguous()
+        # their values: from the configuration, unless a subclass makes the tensors its own way
+        cls, own = type(self), CacheGenDeserializer
+        if cls.make_key_bins is own.make_key_bins and cls.make_value_bins is own.make_value_bins:
+            self._host_bins = _HostBins(torch.cat((CGBasics.make_key_bins(self.cachegen_config, "cpu"),
+                                                   CGBasics.make_value_bins(self.cachegen_config, "cpu"))))
+        else:
+            self._host_bins = _HostBins(self._bins)
         self._workspace = {}
 
     def make_key_bins(self, config: CacheGenConfig) -> torch.Tensor:
@@ -512,7 +536,7 @@ class CacheGenDeserializer(Deserializer):
             # the reference slices a chunk_size-row buffer and fails in its reshape (dec.py:138-141,101)
             raise RuntimeError(f"blob holds {ntokens} tokens, more than chunk_size = {self.chunk_size}")
         return decode_to_kv(encoder_output, self._bins_on(_device_of(encoder_output)), self.fmt, self.out_dtype,
-                            out=out, workspace=self._workspace, delta=self.delta)
+                            out=out, workspace=self._workspace, delta=self.delta, host_bins=self._host_bins)
 
     def decode_many(self, encoder_outputs: List[CacheGenGPUEncoderOutput], out: torch.Tensor = None) -> torch.Tensor:
         """Consecutive chunks of one KV cache into one blob, in as few launches as possible."""
@@ -520,7 +544,7 @@ class CacheGenDeserializer(Deserializer):
             if _chunk_tokens(eo) > self.chunk_size:
                 raise RuntimeError(f"a blob holds more tokens than chunk_size = {self.chunk_size}")
         return decode_many(encoder_outputs, self._bins_on(_device_of(encoder_outputs[0])), self.fmt, self.out_dtype,
-                           out=out, workspace=self._workspace, delta=self.delta)
+                           out=out, workspace=self._workspace, delta=self.delta, host_bins=self._host_bins)
 
     def decode_many_host(self, encoder_outputs: List[CacheGenGPUEncoderOutput], out: torch.Tensor = None,
                          groups: int = None) -> torch.Tensor:
@@ -533,7 +557,8 @@ class CacheGenDeserializer(Deserializer):
         if len(ws) < groups:
             ws += [dict() for _ in range(groups - len(ws))]
         return decode_many_pipelined(encoder_outputs, self._bins_on(_device_of(encoder_outputs[0])), self.fmt,
-                                     self.out_dtype, out=out, groups=groups, workspaces=ws, delta=self.delta)
+                                     self.out_dtype, out=out, groups=groups, workspaces=ws, delta=self.delta,
+                                     host_bins=self._host_bins)
 
     def group_status_words(self):
         """Status words of the pipelined path's per-group workspaces."""
@@ -547,7 +572,7 @@ class CacheGenDeserializer(Deserializer):
         `run_decode` alone is only valid while no other plan of the workspace has run in between."""
         return DecodePlan(encoder_outputs, self._bins_on(_device_of(encoder_outputs[0])), self.fmt, self.out_dtype,
                           out=out, workspace=self._workspace if workspace is None else workspace, peer_out=peer_out,
-                          delta=self.delta)
+                          delta=self.delta, host_bins=self._host_bins)
 
     def _bins_on(self, dev) -> torch.Tensor:
         if not dev.type == "cuda":
@@ -626,7 +651,7 @@ class CacheGenDeserializer(Deserializer):
                     cur.wait_event(arrived)
                     part = out[:, :, start:start + n] if self.fmt == "vllm" else out[:, :, :, start:start + n]
                     decode_many([chunk], self._bins_on(dev), self.fmt, self.out_dtype, out=part,
-                                workspace=self._workspace, delta=self.delta)
+                                workspace=self._workspace, delta=self.delta, host_bins=self._host_bins)
                     start += n
                 at = len(chunks)
         finally:

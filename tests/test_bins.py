@@ -93,3 +93,16 @@ def test_bins_of_a_subclass():
     ser = Halved(type("C", (), {"chunk_size": 256}), type("M", (), {"fmt": "vllm"}), base)
     kv = make_kv()
     assert same(ser.encode(kv), plain.encode(kv))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("compact", [True, "counts", False])
+def test_one_workspace_for_decodes_with_different_bins(compact):
+    from cachegen_b200.serde import cachegen_basics as B, cachegen_decoder as D, cachegen_encoder as E
+    kv, ws = make_kv(), {}
+    for config in (*configs(), configs()[0]):
+        kb, vb = B.make_key_bins(config), B.make_value_bins(config)
+        chunk, bins = E.encode_flat(kv, kb, vb, compact_tables=compact), torch.cat((kb, vb))
+        got = D.decode_to_kv(chunk, bins, "vllm", torch.float16, workspace=ws)
+        assert torch.equal(got, D.decode_to_kv(E.encode_function(kv, None, kb, vb, 70), bins, "vllm", torch.float16))
+        assert int(ws["status"].item()) == 0
