@@ -115,11 +115,12 @@ class DeltaCoding:
         self._res_bins = {}
 
     def residual_bins(self, key_bins: torch.Tensor, value_bins: torch.Tensor, device) -> torch.Tensor:
-        """float32 [2L] on `device`: residual bin counts of the key rows then the value rows, 0 = no delta."""
-        key = (str(device), key_bins.numel(), value_bins.numel())
+        """float32 [2L] on `device`: residual bin counts of the key rows then the value rows, 0 = no delta.  The
+        result is kept by the bins' values, so tensors on a GPU are read back on every call."""
+        kb, vb = key_bins.detach().cpu().float(), value_bins.detach().cpu().float()
+        key = (str(device), tuple(kb.tolist()), tuple(vb.tolist()))
         t = self._res_bins.get(key)
         if t is None:
-            kb, vb = key_bins.detach().cpu().float(), value_bins.detach().cpu().float()
             res_k = torch.clamp(torch.div(kb, self.divisor, rounding_mode="floor"), min=4.0)
             res_v = torch.clamp(torch.div(vb, self.divisor, rounding_mode="floor"), min=4.0)
             if self.rows == "keys":

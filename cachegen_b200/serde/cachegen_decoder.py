@@ -324,7 +324,7 @@ class DecodePlan:
         self.delta_group, self.res_bins = 0, None
         if delta is not None:
             self.delta_group = delta.group
-            self.res_bins = delta.residual_bins(bins[:L], bins[L:], dev)
+            self.res_bins = delta.residual_bins(host_bins.cpu[:L], host_bins.cpu[L:], dev)
             self.keep.append(self.res_bins)
         self.out, self.dev, self.bins, self.status, self.goff = out, dev, bins, status, goff
         self.dims = (L, H, D, C, lp, NL, total_T)

@@ -37,6 +37,16 @@ def test_bins_made_in_inference_mode():
     assert info.cpu.tolist() == [32, 16, 16, 16, 32, 32, 16, 16] and info.table_bins() == 32
 
 
+def test_residual_bins_are_those_of_the_values():
+    from cachegen_b200.serde.cachegen_basics import DeltaCoding
+    delta = DeltaCoding(4, 2, "all")
+    kb, vb = torch.tensor([32.0, 16.0]), torch.tensor([16.0, 16.0])
+    assert delta.residual_bins(kb, vb, "cpu").tolist() == [16, 8, 8, 8]
+    assert delta.residual_bins(vb, kb, "cpu").tolist() == [8, 8, 16, 8]
+    kb.data[0] = 12
+    assert delta.residual_bins(kb, vb, "cpu").tolist() == [6, 8, 8, 8]
+
+
 @pytest.mark.gpu
 def test_a_serializer_made_in_inference_mode_encodes():
     base, half = configs()
