@@ -278,7 +278,6 @@ class _BinsInfo:
     def __init__(self, key_bins, value_bins):
         keys, values = (t.detach().cpu().to(torch.float32) for t in (key_bins, value_bins))
         self.cpu = torch.cat((keys, values))
-        self.nlayers = keys.numel()
         self.kmax, self.vmax = int(keys.max()), int(values.max())
         self.on_device = {}   # device -> float32 [2L]
         self.sparse = flat_format.sparse_representable(self.cpu)
@@ -355,8 +354,8 @@ class _PendingChunk:
         if kv.stride(4) != 1:
             kv = kv.contiguous()
         L, _, T, H, D = kv.shape
-        if info.nlayers != L:
-            raise RuntimeError(f"bins describe {info.nlayers} layers, the KV blob has {L}")
+        if info.cpu.numel() != 2 * L:  # the kernels read 2L of them
+            raise RuntimeError(f"bins describe {info.cpu.numel() // 2} layers, the KV blob has {L}")
         dev = kv.device
         self.kv, self.info, self.dev = kv, info, dev
         self.L, self.T, self.H, self.D, self.max_bins = L, T, H, D, max_bins
@@ -640,7 +639,7 @@ class CacheGenSerializer(Serializer):
         info = self._info
         if self._bins_shared:
             now = _BinsInfo(self._key_bins, self._value_bins)
-            if now.nlayers != info.nlayers or not torch.equal(now.cpu, info.cpu):
+            if (now.kmax, now.vmax) != (info.kmax, info.vmax) or not torch.equal(now.cpu, info.cpu):
                 info = self._info = now
         return info
 

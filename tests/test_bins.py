@@ -37,6 +37,27 @@ def test_bins_made_in_inference_mode():
     assert info.cpu.tolist() == [32, 16, 16, 16, 32, 32, 16, 16] and info.table_bins() == 32
 
 
+class _Blob:
+    """Looks like a KV blob on a GPU up to the checks."""
+    dtype, is_cuda, shape, device = torch.float16, True, (4, 2, 70, 2, 64), "no device"
+
+    def dim(self):
+        return 5
+
+    def stride(self, *at):
+        return (2 * 70 * 128, 70 * 128, 128, 64, 1)[at[0]] if at else (2 * 70 * 128, 70 * 128, 128, 64, 1)
+
+
+@pytest.mark.parametrize("keys,values", [(4, 3), (4, 5), (3, 4), (5, 4), (2, 2)])
+def test_bins_of_other_counts_than_the_blob_has_rows_are_refused(keys, values):
+    from cachegen_b200.serde import cachegen_encoder as E
+    pair = torch.full((keys,), 16.0), torch.full((values,), 16.0)
+    for encode in (lambda: E.encode_function(_Blob(), None, *pair, 70, max_bins=16), lambda: E.encode_levels(_Blob(), [pair]),
+                   lambda: E.encode_flat(_Blob(), *pair, max_bins=16)):
+        with pytest.raises(RuntimeError, match="bins describe"):
+            encode()
+
+
 def test_residual_bins_are_those_of_the_values():
     from cachegen_b200.serde.cachegen_basics import DeltaCoding
     delta = DeltaCoding(4, 2, "all")
