@@ -173,7 +173,9 @@ __device__ __forceinline__ int block_exclusive_scan_128(int v, int *warp_sums, i
 // to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
 // with words assembled from two source words 24 us: one short dependent copy after the other.
 // src: the stream's first word, its words STEP words apart, read-only for the launch; dst0: where the group's
-// streams go; pairs: (STEP 1) the words can be read in pairs, to the end of the last one.
+// streams go; pairs: (STEP 1) the words can be read in pairs, to the end of the last one.  Whatever the row holds behind
+// its stream: the last word is cut to the stream's bytes, since what it shares a word with there is the next stream (and
+// behind the run's last stream the next warp's stage).
 constexpr int kGatherWords = 1536;  // words of shared memory a warp; longer runs take the lanes' own byte stores
 template <int STEP>
 __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t *dst0, bool pairs = false) {
@@ -197,6 +199,7 @@ __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t
     __syncwarp();
     const int o = mis + excl - first, w = o >> 2;
     const uint32_t sh = static_cast<uint32_t>(o & 3) * 8u;
+    const uint32_t last_bytes = 0xFFFFFFFFu >> ((-len & 3) * 8);  // of the last word
     const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
     constexpr int kAhead = 8;  // loads in flight
     uint32_t prev = 0u;
@@ -217,6 +220,7 @@ __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t
         for (int j = 0; j < kAhead; ++j) {
             const int k = k0 + j;
             if (k < nw) {
+                if (k == nw - 1) x[j] &= last_bytes;
                 const uint32_t v = __funnelshift_l(prev, x[j], sh);
                 if (k == 0 || k == nw - 1) atomicOr(st + w + k, v);
                 else st[w + k] = v;
@@ -224,7 +228,7 @@ __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t
             }
         }
     }
-    // what the shift pushed past the last word; a stream's bytes past its end are zero
+    // what the shift pushed past the last word: not 0 only if the stream's bytes reach into the word there
     const uint32_t over = __funnelshift_l(prev, 0u, sh);
     if (over) atomicOr(st + w + nw, over);
     __syncwarp();

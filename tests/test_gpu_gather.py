@@ -1,0 +1,66 @@
+"""The gather of streams takes `length` bytes of every row and none of what lies behind them."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rows_of(rng, NL, C, stride, most):
+    buf = rng.integers(0, 256, (NL, C, stride), dtype=np.uint8)  # no row is zero behind its stream
+    lens = rng.integers(0, most + 1, (NL, C)).astype(np.int32)
+    lens[0, C - 1], lens[0, 0] = 0, most
+    return buf, lens
+
+
+def gathered(buf, lens):
+    b, n = buf.reshape(-1, buf.shape[-1]), lens.reshape(-1)
+    return np.concatenate([b[i, :n[i]] for i in range(len(n))])
+
+
+@pytest.mark.parametrize("C", [1, 31, 32, 33, 127, 128, 129, 300])
+# the shared memory of a warp holds 6,144 bytes: runs below it, around it (32 rows of 188 to 196) and above
+@pytest.mark.parametrize("stride,most", [(4, 1), (4, 4), (8, 7), (12, 9), (64, 61), (188, 188), (192, 192), (196, 195), (520, 519)])
+def test_collect_bytes_of_rows_with_data_behind_the_streams(C, stride, most):
+    from cachegen_b200.serde import cachegen_encoder as E
+    buf, lens = rows_of(np.random.default_rng(C * 1000 + stride), 3, C, stride, most)
+    got = E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda())
+    assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
+
+
+@pytest.mark.parametrize("short", [0, 1, 2, 3, 5, 16])
+def test_runs_that_fill_a_warps_shared_memory(short):
+    from cachegen_b200.serde import cachegen_encoder as E
+    # 32 streams of 192 bytes are a whole run; the first one starts its warp's run at every offset from 16 bytes
+    buf, lens = rows_of(np.random.default_rng(short), 2, 128, 196, 192)
+    lens[:] = 192
+    lens[:, 32] -= short
+    lens[0, 5] = 192 - short
+    got = E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda())
+    assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
+
+
+def test_several_sub_chunks_through_the_c_abi():
+    from cachegen_b200 import _lib
+    NL, C, stride, nsub = 2, 200, 100, 3
+    rng = np.random.default_rng(8)
+    parts = [rows_of(rng, NL, C, stride, 99) for _ in range(nsub)]
+    sizes = np.array([[p[1][r, c:c + 128].sum() for r in range(NL) for c in range(0, C, 128)] for p in parts], dtype=np.int64)
+    group_off = np.cumsum(sizes, axis=1) - sizes
+    sub_off = np.concatenate(([0], np.cumsum(sizes.sum(axis=1))))
+    dev = [torch.from_numpy(a).cuda() for a in (np.stack([p[0] for p in parts]), np.stack([p[1] for p in parts]), group_off, sub_off)]
+    out = torch.empty(int(sub_off[-1]), dtype=torch.uint8, device="cuda")
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (*dev, out)]
+    rc = _lib.lib().cg_compact_streams(p[0], stride, p[1], p[2], p[3], nsub, NL, C, p[4],
+                                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0 and out.cpu().numpy().tobytes() == np.concatenate([gathered(*q) for q in parts]).tobytes()
+
+
+def test_recombined_rows_are_collected_again():
+    from cachegen_b200.serde import cachegen_decoder as D, cachegen_encoder as E
+    buf, lens = rows_of(np.random.default_rng(3), 4, 130, 256, 90)
+    lens_t = torch.from_numpy(lens).cuda()
+    b = torch.from_numpy(gathered(buf, lens)).cuda()
+    assert torch.equal(E.collect_bytes(D.recombine_bytes(b, lens_t), lens_t), b)
