@@ -603,9 +603,9 @@ class _Staging:
             self.end()
 
     def _send(self, upload, device, stream) -> None:
-        """Runs an upload from the chosen buffer on `stream`, or the device's current one."""
+        """Runs an upload from the chosen buffer on `stream`, if it is one of the device's, or its current one."""
         with on_device(device):
-            on = torch.cuda.current_stream(device) if stream is None else stream
+            on = torch.cuda.current_stream(device) if stream is None or stream.device != device else stream
             if self.events[self.turn] is None or self.events[self.turn][0] != device:
                 self.events[self.turn] = (device, torch.cuda.Event())
             rc = upload(on.cuda_stream)

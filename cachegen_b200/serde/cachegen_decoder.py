@@ -594,16 +594,15 @@ class CacheGenDeserializer(Deserializer):
         """from_bytes for the blobs of consecutive chunks of one KV cache: one result tensor, as
         decode_many builds it.  Three things run side by side: the blobs' bytes on their way to the GPU (on a
         copy stream), the parsing of the blobs after the first (on a thread; the copies leave the interpreter to
-        it), and the decode of each chunk that has arrived."""
+        it), and the decode of each chunk that has arrived.  A pickled chunk's tensors come back on the GPU they were
+        saved from; all are decoded on the first chunk's."""
         if not blobs:
             raise RuntimeError("nothing to decode")
-        dev = torch.device("cuda", torch.cuda.current_device())
-        cur, copies = torch.cuda.current_stream(dev), _copy_stream(dev)
-        copies.wait_stream(cur)  # the tensors come from the current stream's pool
         total = len(blobs)
         parsed = queue.SimpleQueue()
+        cur = copies = None
 
-        def parse(blob, ahead=False):
+        def parse(blob, dev, ahead=False):
             load = CGBasics.BlobLoad()
             with load:
                 if ahead and isinstance(blob, bytes) and not flat_format.is_flat(blob):
@@ -618,14 +617,18 @@ class CacheGenDeserializer(Deserializer):
             try:
                 with torch.cuda.device(dev), torch.cuda.stream(cur):
                     for blob in blobs[1:]:
-                        parsed.put(parse(blob))
+                        parsed.put(parse(blob, dev))
             except BaseException as e:  # handed to the caller's thread
                 parsed.put(e)
 
         chunks, tokens, done, at = [], 0, 0, 0
         waiting = []
         try:
-            first = parse(blobs[0], ahead=True)  # the others are parsed while their predecessors travel
+            here = torch.device("cuda", torch.cuda.current_device())
+            first = parse(blobs[0], here, ahead=True)  # the others are parsed while their predecessors travel
+            dev = _device_of(first[1]) if _on_gpu(first[1]) else here
+            cur, copies = torch.cuda.current_stream(dev), _copy_stream(dev)
+            copies.wait_stream(cur)  # the tensors come from the current stream's pool
             if total > 1:
                 # (a threading.Thread's start waits until the thread runs: 140 us before the first bytes left)
                 _thread.start_new_thread(parse_rest, ())
@@ -634,7 +637,13 @@ class CacheGenDeserializer(Deserializer):
                 if isinstance(item, BaseException):
                     raise item
                 load, chunk, ntokens = item
+                # tensors of another GPU, made on a stream there that is not known here
+                others = {p[2].device for p in load.pairs if p[2].device != dev}
+                for d in others:
+                    torch.cuda.synchronize(d)
                 load.send(copies)
+                for d in others:
+                    torch.cuda.synchronize(d)
                 arrived = torch.cuda.Event()
                 arrived.record(copies)
                 chunks.append((chunk, ntokens, arrived))
@@ -650,13 +659,14 @@ class CacheGenDeserializer(Deserializer):
                 for chunk, n, arrived in chunks[at:]:
                     cur.wait_event(arrived)
                     part = out[:, :, start:start + n] if self.fmt == "vllm" else out[:, :, :, start:start + n]
-                    decode_many([chunk], self._bins_on(dev), self.fmt, self.out_dtype, out=part,
-                                workspace=self._workspace, delta=self.delta, host_bins=self._host_bins)
+                    DecodePlan([chunk], self._bins_on(dev), self.fmt, self.out_dtype, out=part, workspace=self._workspace,
+                               device=dev, delta=self.delta, host_bins=self._host_bins).run()
                     start += n
                 at = len(chunks)
         finally:
             CGBasics.staging().finish()
-            cur.wait_stream(copies)
+            if copies is not None:
+                cur.wait_stream(copies)
         return out
 
     def _blob_for(self, chunk, ntokens, dev, out):
