@@ -7,7 +7,6 @@
 // 2 MB 632, of 8 MB 589, in one 577.  So the bytes are copied in small pieces but travel in transfers that grow from
 // the first pieces on (to the GPU, where the copies come first) or shrink towards the last ones (from it): 30 MB
 // to the GPU in 660 us, against 703 when every piece was sent as soon as it was copied.
-#include <immintrin.h>
 #include <string.h>
 #include <sys/mman.h>
 #include <time.h>
@@ -22,6 +21,7 @@
 #include <vector>
 
 #include "cg_common.cuh"
+#include "cg_hostcopy.h"
 
 namespace {
 
@@ -32,35 +32,6 @@ constexpr int64_t kHugeFrom = 8 << 20;  // results from this size on ask for 2 M
 constexpr int kMaxThreads = 8;          // helpers at most: half the cores, up to this
 constexpr int kSpinMicros = 60;         // a helper that has run out of work looks for more for this long
 constexpr int kIdleSeconds = 5;         // ... sleeps for this long, and then ends
-
-__attribute__((target("avx2"))) void copy_streaming(uint8_t *d, const uint8_t *s, int64_t n) {
-    const int64_t head = (32 - (reinterpret_cast<uintptr_t>(d) & 31)) & 31;
-    if (n < 4096) {
-        memcpy(d, s, static_cast<size_t>(n));
-        return;
-    }
-    memcpy(d, s, static_cast<size_t>(head));
-    d += head;
-    s += head;
-    n -= head;
-    for (; n >= 128; n -= 128, d += 128, s += 128) {
-        const __m256i a = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(s));
-        const __m256i b = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(s + 32));
-        const __m256i c = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(s + 64));
-        const __m256i e = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(s + 96));
-        _mm256_stream_si256(reinterpret_cast<__m256i *>(d), a);
-        _mm256_stream_si256(reinterpret_cast<__m256i *>(d + 32), b);
-        _mm256_stream_si256(reinterpret_cast<__m256i *>(d + 64), c);
-        _mm256_stream_si256(reinterpret_cast<__m256i *>(d + 96), e);
-    }
-    memcpy(d, s, static_cast<size_t>(n));
-    _mm_sfence();
-}
-void copy_piece(uint8_t *d, const uint8_t *s, int64_t n) {
-    static const bool avx2 = __builtin_cpu_supports("avx2");
-    if (avx2) copy_streaming(d, s, n);
-    else memcpy(d, s, static_cast<size_t>(n));
-}
 
 struct Piece {
     uint8_t *dst;
@@ -81,8 +52,8 @@ struct Job {
             if (i >= ready.load(std::memory_order_acquire)) return false;
         } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
         Piece &p = pieces[i];
-        if (p.src) copy_piece(p.dst, p.src, p.bytes);
-        else for (int64_t k = 0; k < p.bytes; k += 4096) asm volatile("lock; orb $0, %0" : "+m"(p.dst[k]));  // may already hold data
+        if (p.src) cg::copy_piece(p.dst, p.src, p.bytes);
+        else for (int64_t k = 0; k < p.bytes; k += 4096) cg::touch_page(p.dst + k);  // may already hold data
         p.done.store(true, std::memory_order_release);
         return true;
     }
@@ -138,7 +109,7 @@ class Helpers {
             }
             if (j) {
                 while (!j->taken())
-                    if (!j->work()) _mm_pause();
+                    if (!j->work()) cg::spin_pause();
                 j->helpers.fetch_sub(1, std::memory_order_release);
                 idle_since = clock::now();
                 continue;
@@ -146,7 +117,7 @@ class Helpers {
             if (clock::now() - idle_since < std::chrono::microseconds(kSpinMicros)) {
                 while (generation_.load(std::memory_order_acquire) == seen &&
                        clock::now() - idle_since < std::chrono::microseconds(kSpinMicros))
-                    _mm_pause();
+                    cg::spin_pause();
                 continue;
             }
             std::unique_lock<std::mutex> lock(mu_);
@@ -241,7 +212,7 @@ cudaError_t send_parts(Job &job, const std::vector<Part> &parts, cudaStream_t st
             if (err != cudaSuccess) return err;
             sent = e;
         }
-        if (sent < n && !job.work()) _mm_pause();
+        if (sent < n && !job.work()) cg::spin_pause();
     }
     return cudaSuccess;
 }
@@ -467,7 +438,7 @@ extern "C" int cg_host_download(const cg_host_segment *segs, int nsegs, void *st
                 break;
             }
         }
-        if (!job.work()) _mm_pause();
+        if (!job.work()) cg::spin_pause();
     }
     if (err != cudaSuccess) job.next.store(lead + n, std::memory_order_relaxed);  // nothing more to take
     if (n > 1) helpers().remove(&job);
