@@ -23,6 +23,18 @@ inline int check_launch() {
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
 
+// Dynamic shared memory beyond the 48 KB that a launch gets by itself.  Every launch raises its kernel's limit to the same
+// value, the most that any of them asks for: a limit that followed the launch could be lowered by another thread between
+// this thread's setting it and its launch.
+constexpr int64_t kSmemByItself = 48 * 1024, kSmemPerBlock = 227 * 1024;
+constexpr int64_t kMostStaticSmem = 256;  // of the kernels that ask
+constexpr int64_t kMostDynamicSmem = kSmemPerBlock - kMostStaticSmem;
+template <class K>
+int allow_smem(K kernel, size_t bytes) {
+    if (bytes <= kSmemByItself) return CG_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMostDynamicSmem));
+    return e == cudaSuccess ? CG_OK : set_cuda_error(e);
+}
 // cg_store.cu: dynamic shared memory that makes the last wave of `blocks` equal blocks as full as the others
 size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes);
 // cg_tables.cu: group offsets of sparse tables, and the tables in one pass once those are known

@@ -609,16 +609,15 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
 }
 
 // ---- launch helpers -------------------------------------------------------------------------------------
-// dynamic shared memory of a decoder block: the streams' table columns
+// dynamic shared memory of a decoder block: the streams' table columns, at most 33 KB
 static size_t table_bytes(int lp, int levels) {
     return static_cast<size_t>(table_rows(lp, levels) + 1) * kRowBytes;  // +1: the row read past the last symbol
 }
+static_assert((CG_MAX_LP + 1) * kRowBytes + 4 * (kSubTokens + 2 * CG_MAX_LP) + 64 <= kSmemByItself, "a decoder block's shared memory");
 
 // early: the blocks may start before the launch in front has ended (see DecodeAfter)
 template <class... Args>
 static int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t st, Args... args) {
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(static_cast<unsigned>(threads));

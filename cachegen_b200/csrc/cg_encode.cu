@@ -201,11 +201,9 @@ static int launch_encode(const EncodeParams &p, int nrows, int nsub, cudaStream_
     const size_t smem = even_waves_smem(static_cast<int64_t>(grid.x) * grid.y * grid.z, static_cast<size_t>(p.lp) * kRowBytes, 0);
     const bool narrow = p.s1 >= 0 && p.s2 >= 0 && p.s1 <= 0xFFFFFFFF / (kSubTokens + 1) &&
                         p.s1 * kSubTokens + p.s2 * p.nchannels <= 0xFFFFFFFF;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(narrow ? encode_kernel<true> : encode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-    if (narrow) encode_kernel<true><<<grid, kGroup, smem, st>>>(p);
-    else encode_kernel<false><<<grid, kGroup, smem, st>>>(p);
+    const auto kernel = narrow ? encode_kernel<true> : encode_kernel<false>;
+    if (int rc = allow_smem(kernel, smem)) return rc;
+    kernel<<<grid, kGroup, smem, st>>>(p);
     return check_launch();
 }
 

@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(256) flat_front_kernel(const __grid_constant__
     }
 }
 
-constexpr int64_t kSmemPerSM = 228 * 1024, kSmemPerBlock = 227 * 1024, kSmemReserved = 1024;
+constexpr int64_t kSmemPerSM = 228 * 1024, kSmemReserved = 1024;
 
 static int sm_count() {
     static int count[64];  // per device; a racing first call writes the same number
@@ -693,7 +693,7 @@ size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes) {
     const int64_t per = (blocks + sms * waves - 1) / (sms * waves);
     if (per >= resident || per < 1) return dynamic;
     int64_t padded = kSmemPerSM / per - kSmemReserved - static_cast<int64_t>(static_bytes) - 256;
-    if (padded > kSmemPerBlock - static_cast<int64_t>(static_bytes)) padded = kSmemPerBlock - static_cast<int64_t>(static_bytes);
+    if (padded > kMostDynamicSmem) padded = kMostDynamicSmem;
     return padded > static_cast<int64_t>(dynamic) ? static_cast<size_t>(padded) : dynamic;
 }
 
@@ -702,12 +702,6 @@ size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes) {
 using namespace cg;
 
 namespace {
-
-
-template <class K>
-void allow_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-}
 
 struct Sizes {
     int nrows, nchannels, nslab, nsub;
@@ -849,11 +843,11 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
     if (z.nsub == 1) {
         const size_t smem = even_waves_smem(blocks, columns + staged, 128);
-        allow_smem(store_encode_kernel<true, 1>, smem);
+        if (int rc = allow_smem(store_encode_kernel<true, 1>, smem)) return rc;
         store_encode_kernel<true, 1><<<grid, kGroup, smem, st>>>(p);
         return check_launch();
     }
-    allow_smem(packed_tables_kernel, columns + staged);
+    if (int rc = allow_smem(packed_tables_kernel, columns + staged)) return rc;
     packed_tables_kernel<<<dim3(z.nslab, z.nrows), kTableThreads, columns + staged, st>>>(sym4, b.ntokens, z.nchannels, lp,
                                                                                          p.out, status);
     if (int rc = check_launch()) return rc;
@@ -861,10 +855,10 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     // two streams a thread unless the last group has channels for the first alone
     const int last = z.nchannels % kGroup;
     if (last == 0 || last > kGroup / 2) {
-        allow_smem(store_encode_kernel<false, 2>, smem);
+        if (int rc = allow_smem(store_encode_kernel<false, 2>, smem)) return rc;
         store_encode_kernel<false, 2><<<grid, kGroup / 2, smem, st>>>(p);
     } else {
-        allow_smem(store_encode_kernel<false, 1>, smem);
+        if (int rc = allow_smem(store_encode_kernel<false, 1>, smem)) return rc;
         store_encode_kernel<false, 1><<<grid, kGroup, smem, st>>>(p);
     }
     return check_launch();
