@@ -23,7 +23,8 @@ inline int check_launch() {
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
 
-// Dynamic shared memory beyond the 48 KB that a launch gets by itself.  Every launch raises its kernel's limit to the same
+// Dynamic shared memory beyond what a launch gets by itself, 48 KB with the kernel's own arrays: the columns of 64-entry
+// tables and their 16-bit copies are 48 KB alone.  Every launch raises its kernel's limit to the same
 // value, the most that any of them asks for: a limit that followed the launch could be lowered by another thread between
 // this thread's setting it and its launch.
 constexpr int64_t kSmemByItself = 48 * 1024, kSmemPerBlock = 227 * 1024;
@@ -31,7 +32,7 @@ constexpr int64_t kMostStaticSmem = 256;  // of the kernels that ask
 constexpr int64_t kMostDynamicSmem = kSmemPerBlock - kMostStaticSmem;
 template <class K>
 int allow_smem(K kernel, size_t bytes) {
-    if (bytes <= kSmemByItself) return CG_OK;
+    if (static_cast<int64_t>(bytes) <= kSmemByItself - kMostStaticSmem) return CG_OK;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMostDynamicSmem));
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }

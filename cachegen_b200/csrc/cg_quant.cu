@@ -456,18 +456,18 @@ int launch_quantize(const uint16_t *x, int dtype, const QuantShape &q, const flo
     const int C = q.L.nheads * q.L.head_size;
     const dim3 grid((C + kGroup - 1) / kGroup, nrows);
     const size_t smem = hist_smem_bytes(max_bins);
-#define CG_LAUNCH_Q(DT, V, D) \
-    quantize_cdf_kernel<DT, V, D><<<grid, kQuantThreads, smem, st>>>(x, q.L, bins, sc, max_bins, sym_out, cdf_out, \
-                                                                     counts_out, table_row_off, status, res_bins, group, row0)
+    const auto launch = [&](auto kernel) {
+        if (int rc = allow_smem(kernel, smem)) return rc;
+        kernel<<<grid, kQuantThreads, smem, st>>>(x, q.L, bins, sc, max_bins, sym_out, cdf_out, counts_out, table_row_off, status,
+                                                  res_bins, group, row0);
+        return check_launch();
+    };
     if (group > 0) {
-        if (dtype == CG_F16) { if (q.vec) CG_LAUNCH_Q(CG_F16, 8, true); else CG_LAUNCH_Q(CG_F16, 1, true); }
-        else { if (q.vec) CG_LAUNCH_Q(CG_BF16, 8, true); else CG_LAUNCH_Q(CG_BF16, 1, true); }
-    } else {
-        if (dtype == CG_F16) { if (q.vec) CG_LAUNCH_Q(CG_F16, 8, false); else CG_LAUNCH_Q(CG_F16, 1, false); }
-        else { if (q.vec) CG_LAUNCH_Q(CG_BF16, 8, false); else CG_LAUNCH_Q(CG_BF16, 1, false); }
+        if (dtype == CG_F16) return q.vec ? launch(quantize_cdf_kernel<CG_F16, 8, true>) : launch(quantize_cdf_kernel<CG_F16, 1, true>);
+        return q.vec ? launch(quantize_cdf_kernel<CG_BF16, 8, true>) : launch(quantize_cdf_kernel<CG_BF16, 1, true>);
     }
-#undef CG_LAUNCH_Q
-    return check_launch();
+    if (dtype == CG_F16) return q.vec ? launch(quantize_cdf_kernel<CG_F16, 8, false>) : launch(quantize_cdf_kernel<CG_F16, 1, false>);
+    return q.vec ? launch(quantize_cdf_kernel<CG_BF16, 8, false>) : launch(quantize_cdf_kernel<CG_BF16, 1, false>);
 }
 
 int launch_residual_absmax(const uint16_t *x, int dtype, const QuantShape &q, const float *bins,
