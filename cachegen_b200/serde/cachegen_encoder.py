@@ -106,12 +106,17 @@ def _collect(output_buffer: torch.Tensor, output_lengths: torch.Tensor, status: 
     with on_device(dev):
         if NL * nslab <= _lib.CG_MAX_OFFSET_GROUPS:
             tail = _take_tail(4)
-            rc = lib.cg_stream_sizes(_ptr(lengths), NL, C, min(stride, 1 << 20),
-                                     None if status is None else status.data_ptr(), offsets.data_ptr(), tail.data_ptr(), stream)
-            if rc == 0:
-                rc = lib.cg_wait_word(tail.data_ptr() + 24, stream)
-            total, outside, bits, _ = tail[:4].tolist()
-            _give_tail(tail)
+            try:
+                rc = lib.cg_stream_sizes(_ptr(lengths), NL, C, min(stride, 1 << 20),
+                                         None if status is None else status.data_ptr(), offsets.data_ptr(), tail.data_ptr(), stream)
+                if rc == 0:
+                    rc = lib.cg_wait_word(tail.data_ptr() + 24, stream)
+                total, outside, bits, _ = tail[:4].tolist()
+            except BaseException:
+                torch.cuda.current_stream(dev).synchronize()  # the GPU may still be about to write to it
+                raise
+            finally:
+                _give_tail(tail)
         else:
             total, outside, bits = torch.stack((lengths.sum(dtype=torch.int64),
                                                 ((lengths < 0) | (lengths > stride)).sum(dtype=torch.int64),
@@ -391,13 +396,17 @@ class _PendingChunk:
         if delta is not None:
             self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
             job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
-        with on_device(dev):
-            _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
-        # made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do
-        self.lengths = [] if with_counts else [torch.empty((2 * L, H * D), dtype=torch.int32, device=dev)
-                                               for _ in range(self.nsub)]
-        self.pointers = ctypes.c_void_p * self.nsub
-        self.length_pointers = self.pointers(*[t.data_ptr() for t in self.lengths])
+        try:
+            with on_device(dev):
+                _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
+            # made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do
+            self.lengths = [] if with_counts else [torch.empty((2 * L, H * D), dtype=torch.int32, device=dev)
+                                                   for _ in range(self.nsub)]
+            self.pointers = ctypes.c_void_p * self.nsub
+            self.length_pointers = self.pointers(*[t.data_ptr() for t in self.lengths])
+        except BaseException:
+            self.abandon()
+            raise
 
     def sizes(self):
         """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
@@ -425,7 +434,8 @@ class _PendingChunk:
                                          for j in range(n)], self.cdf, self.scales_k, self.scales_v, self.H, self.D)
 
     def abandon(self) -> None:
-        """Gives the buffers up after an error elsewhere: the GPU may still be writing to them."""
+        """Gives the buffers up after an error: the GPU may still be writing to them, the pinned one among them, which
+        would go to whoever asks torch for pinned memory next.  Nothing to do once the sizes have been read."""
         if self.tail is not None:
             self.stream.synchronize()
             _give_tail(self.tail)
@@ -525,7 +535,11 @@ def encode_function(kv: torch.Tensor, config: CacheGenConfig, key_bins: torch.Te
     if kv.shape[2] != chunk_size:
         raise RuntimeError(f"chunk_size {chunk_size} does not match the {kv.shape[2]} tokens of the blob")
     info = info or _BinsInfo(key_bins, value_bins)
-    return _PendingChunk(kv, info, info.table_bins(max_bins), delta=delta).finish()
+    p = _PendingChunk(kv, info, info.table_bins(max_bins), delta=delta)
+    try:
+        return p.finish()
+    finally:
+        p.abandon()
 
 
 def pack_sparse_tables(counts: torch.Tensor, bins: torch.Tensor, nchannels: int, bins_cpu: torch.Tensor = None):
@@ -561,7 +575,10 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     info = info or _BinsInfo(key_bins, value_bins)
     kmax = info.table_bins(max_bins)
     p = _PendingChunk(kv, info, kmax, delta=delta, with_counts=True)
-    offs, bits, nonzero = p.sizes()
+    try:
+        offs, bits, nonzero = p.sizes()
+    finally:
+        p.abandon()
     fits = bool(compact_tables) and not (bits & _lib.CG_S_COUNT_OVERFLOW)
     off_masks, off_counts = flat_format.sparse_parts(2 * p.L, p.H * p.D, p.mask_bytes)
     if fits and compact_tables is True and info.sparse:

@@ -1,0 +1,41 @@
+"""Pinned memory that the GPU still writes to, or reads from, stays what it is until the GPU is done: after errors, and when
+the thread that it belongs to has ended."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BUSY = 100_000_000  # cycles, some 50 ms: what is enqueued behind them has not run when the call returns
+
+
+class Stop(Exception):
+    pass
+
+
+def written_after(buffer):
+    """Whether the GPU writes to the buffer from here on."""
+    buffer.zero_()
+    torch.cuda.synchronize()
+    return bool(buffer.any())
+
+
+@pytest.mark.parametrize("call", ["encode_function", "encode_levels", "encode_many"])
+def test_sizes_of_an_encode_that_fails_after_its_launch(monkeypatch, call):
+    from cachegen_b200.serde import cachegen_encoder as E
+    kv = torch.randn((2, 2, 40, 2, 64), generator=torch.Generator().manual_seed(1)).half().cuda()
+    b = torch.full((2,), 16.0).cuda()
+    run = {"encode_function": lambda: E.encode_function(kv, None, b, b, 40), "encode_levels": lambda: E.encode_levels(kv, [(b, b)]),
+           "encode_many": lambda: E.encode_many(kv, b, b, 40)}[call]
+    run()
+    tail, empty = torch.zeros(64, dtype=torch.int64, pin_memory=True), torch.empty
+
+    def no_memory(*size, **kw):
+        if kw.get("dtype") == torch.int32:  # the lengths' tensors, made when the kernels have been launched
+            raise Stop
+        return empty(*size, **kw)
+    monkeypatch.setattr(E, "_take_tail", lambda n: tail)
+    monkeypatch.setattr(torch, "empty", no_memory)
+    torch.cuda._sleep(BUSY)
+    with pytest.raises(Stop):
+        run()
+    assert not written_after(tail)
