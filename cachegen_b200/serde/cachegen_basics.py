@@ -375,9 +375,9 @@ def dump_blob(eo: "CacheGenGPUEncoderOutput") -> bytes:
         sizes = {id(t): sizes[id(t)] for t in tensors if id(t) in sizes and (not t.is_cuda or t.device == tensors[0].device)}
     on_gpu = [t for t in tensors if id(t) in sizes and t.is_cuda and t.numel()]
     st = staging()
-    if on_gpu:
-        st.fetch(on_gpu)
     try:
+        if on_gpu:
+            st.fetch(on_gpu)
         out = _PartsWriter()
         pickler = _BlobPickler(out, sizes)
         pickler.dump(eo)
@@ -391,7 +391,7 @@ def dump_blob(eo: "CacheGenGPUEncoderOutput") -> bytes:
             if not t.is_cuda and t.numel():
                 ctypes.memmove(base + at, t.data_ptr(), sizes[id(t)])
     except BaseException:
-        st.end()
+        st.cancel()
         raise
     if on_gpu:
         st.collect([where[id(t)] for t in on_gpu])
@@ -534,6 +534,8 @@ class _Staging:
         self.buf = None
         self.waiting = None  # (host view, device tensor) pairs of the load in progress
         self.early = None    # (handle, address, size) of a byte string whose copy runs ahead of its parsing
+        self.fetched = None  # the tensors whose transfers into the chosen buffer are on their way, and their stream
+        self.fetching = None
 
     def begin(self, nbytes: int) -> None:
         self.turn ^= 1
@@ -608,9 +610,11 @@ class _Staging:
             on = torch.cuda.current_stream(device) if stream is None or stream.device != device else stream
             if self.events[self.turn] is None or self.events[self.turn][0] != device:
                 self.events[self.turn] = (device, torch.cuda.Event())
-            rc = upload(on.cuda_stream)
-            self.events[self.turn][1].record(on)
-            self.leaving[self.turn] = True
+            try:
+                rc = upload(on.cuda_stream)
+            finally:
+                self.events[self.turn][1].record(on)
+                self.leaving[self.turn] = True
         _lib.check(rc, "cg_host_upload")
 
     def send(self, pairs: list = None, stream=None) -> None:
@@ -649,31 +653,43 @@ class _Staging:
         sizes = [t.numel() * t.element_size() for t in tensors]
         self.segs = (_lib.HostSegment * len(tensors))(*[(None, t.data_ptr(), n) for t, n in zip(tensors, sizes)])
         self.begin(sum((n + 255) // 256 * 256 for n in sizes))
-        self.fetched = tensors
-        self._download(1)
+        self.fetched, self.fetching = tensors, torch.cuda.current_stream(tensors[0].device)
+        try:
+            self._download(1)
+        except BaseException:
+            self.cancel()
+            raise
 
     def collect(self, pointers: list) -> None:
         """The bytes of the fetched tensors to these addresses."""
-        for seg, at in zip(self.segs, pointers):
-            seg.host = at
         try:
+            for seg, at in zip(self.segs, pointers):
+                seg.host = at
             self._download(2)
-        finally:
-            self.fetched = None
-            self.end()
+        except BaseException:
+            self.cancel()
+            raise
+        self.fetched = self.fetching = None
+        self.end()
+
+    def cancel(self) -> None:
+        """Ends a fetch whose bytes are not wanted (any more): waits for the transfers that still write to the buffer."""
+        if self.fetched is not None:
+            self.fetching.synchronize()
+            self.fetched = self.fetching = None
+        self.end()
 
     def _download(self, phase: int) -> None:
-        device = self.fetched[0].device
-        with on_device(device):
+        with on_device(self.fetched[0].device):
             rc = _lib.lib().cg_host_download(self.segs, len(self.segs), self.buf.data_ptr(), self.buf.numel(), phase,
-                                             torch.cuda.current_stream(device).cuda_stream)
+                                             self.fetching.cuda_stream)
         _lib.check(rc, "cg_host_download")
 
     def whole_from_device(self, t: torch.Tensor) -> bytes:
         """The bytes of a contiguous GPU tensor."""
         n = t.numel() * t.element_size()
-        self.fetch([t])
         out = _bytes_new(None, n)
+        self.fetch([t])
         self.collect([_bytes_at(out)])
         return out
 

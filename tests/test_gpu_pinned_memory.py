@@ -39,3 +39,31 @@ def test_sizes_of_an_encode_that_fails_after_its_launch(monkeypatch, call):
     with pytest.raises(Stop):
         run()
     assert not written_after(tail)
+
+
+@pytest.mark.parametrize("step", ["pickling", "collecting"])
+def test_transfers_of_a_dump_that_fails(monkeypatch, step):
+    from cachegen_b200.serde import cachegen_basics as B
+    one = torch.arange(1 << 20, dtype=torch.int32).cuda()
+    eo = B.CacheGenGPUEncoderOutput([B.CacheGenGPUBytestream(one.to(torch.uint8), one, 1)], one.short(), one.half(), one.half(), 1, 1)
+    for _ in range(2):
+        B.dump_blob(eo)  # both buffers are large enough from here on
+    st, download = B.staging(), B._Staging._download
+
+    def fail(*a):
+        raise Stop
+
+    def fail_second(self, phase):
+        if phase == 2:
+            raise Stop
+        download(self, phase)
+    if step == "pickling":
+        monkeypatch.setattr(B._BlobPickler, "dump", fail)
+    else:
+        monkeypatch.setattr(B._Staging, "_download", fail_second)
+    torch.cuda._sleep(BUSY)
+    with pytest.raises(Stop):
+        B.dump_blob(eo)
+    assert not written_after(st.bufs[st.turn])
+    monkeypatch.undo()
+    assert B.load_blob(B.dump_blob(eo)).cdf.equal(eo.cdf)
