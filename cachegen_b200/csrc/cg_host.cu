@@ -316,6 +316,9 @@ namespace {
 struct Events {
     int device = -1;
     std::vector<cudaEvent_t> list;
+    ~Events() {
+        for (cudaEvent_t v : list) cudaEventDestroy(v);
+    }
     cudaError_t want(size_t n) {
         int dev;
         cudaError_t e = cudaGetDevice(&dev);

@@ -553,6 +553,15 @@ class _Staging:
     def end(self) -> None:
         self.buf = None
 
+    def __del__(self):
+        # the thread has ended: torch would give its buffers to others while copies may still leave them
+        for i in range(2):
+            if self.leaving[i]:
+                try:
+                    self.events[i][1].synchronize()
+                except Exception:
+                    pass  # the process is ending, or the GPU has failed: nobody gets the memory
+
     # -- to the GPU: a load collects the tensors it makes, and sends them together
     def open(self) -> None:
         self.waiting = []

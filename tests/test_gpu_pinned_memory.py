@@ -67,3 +67,36 @@ def test_transfers_of_a_dump_that_fails(monkeypatch, step):
     assert not written_after(st.bufs[st.turn])
     monkeypatch.undo()
     assert B.load_blob(B.dump_blob(eo)).cdf.equal(eo.cdf)
+
+
+def test_uploads_of_a_thread_that_has_ended():
+    import threading
+    from cachegen_b200.serde import cachegen_basics as B
+    host = torch.arange(3 << 20, dtype=torch.int32).to(torch.uint8)
+    device, got = torch.device("cuda", torch.cuda.current_device()), []
+
+    def upload():
+        B.staging().begin(host.numel())  # pins the memory; the copies below take the other buffer
+        B.staging().end()
+        torch.cuda._sleep(BUSY)
+        got.append((B.staging().whole_to_device(host, device), B.staging().bufs[B.staging().turn].numel()))
+    t = threading.Thread(target=upload)
+    t.start()
+    t.join()
+    del t
+    others = [torch.empty(got[0][1], dtype=torch.uint8, pin_memory=True).fill_(255) for _ in range(4)]
+    assert torch.equal(got[0][0].cpu(), host) and len(others) == 4
+
+
+def test_threads_that_come_and_go():
+    import threading
+    from cachegen_b200.serde import cachegen_basics as B
+    data, same = torch.arange(1 << 18, dtype=torch.int32).cuda(), []
+
+    def there_and_back():
+        same.append(B.staging().whole_from_device(data) == data.cpu().numpy().tobytes())
+    for _ in range(20):
+        t = threading.Thread(target=there_and_back)
+        t.start()
+        t.join()
+    assert same == [True] * 20
