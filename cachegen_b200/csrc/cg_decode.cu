@@ -19,6 +19,10 @@ __host__ __device__ inline int table_rows(int lp, int levels) {
 enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
 __device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A group offset that the launch in front wrote, behind the wait for it (in a later batch: that launch had ended when the
+// first batch's blocks let this one start).  From the L2: __ldg is for data that nothing writes while the kernel runs, and
+// these blocks may start while that launch still does.
+__device__ __forceinline__ int64_t written_offset(const int64_t *p) { return __ldcg(reinterpret_cast<const long long *>(p)); }
 
 // ---- table staging by the block --------------------------------------------------------------------------
 // The int16 tables of a block's 128 channels are one contiguous run.  Read channel by channel they are 2-byte
@@ -96,7 +100,7 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
         const int n = c < p.nchannels ? max(0, min(__ldg(p.lengths + g), 1 << 20)) : 0;
         const int excl = block_exclusive_scan_128(n, warp_sums, tid, nullptr);
         wait_for_launch_before();
-        start = __ldg(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
+        start = written_offset(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
         len = n;
     }
     if (c >= p.nchannels) return;  // no block barrier from here on
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         }
         const int excl = block_exclusive_scan<kGroup / 64>(static_cast<int>(len[0] + len[1]), warp_sums, tid, nullptr);
         wait_for_launch_before();
-        start[0] = __ldg(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
+        start[0] = written_offset(p.group_off + static_cast<int64_t>(row) * gridDim.x + blockIdx.x) + excl;
         start[1] = start[0] + len[0];
     }
     if (run_staged) {
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
     const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
     wait_for_launch_before();
     let_next_launch_start();
-    int64_t start = __ldg(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
+    int64_t start = written_offset(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
     if (start < 0) { start = 0; len = 0; bad = true; }
     if (start > job.nbytes) { start = job.nbytes; bad = true; }
     if (start + len > job.nbytes) { len = static_cast<int>(job.nbytes - start); bad = true; }
@@ -529,7 +533,7 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     if (p.after == kAfterOffsets) wait_for_launch_before();
     let_next_launch_start();
     int64_t start[NS];
-    start[0] = __ldg(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
+    start[0] = written_offset(job.group_off + static_cast<int64_t>(row) * p.nslab + blockIdx.x) + excl;
 #pragma unroll
     for (int i = 1; i < NS; ++i) start[i] = start[i - 1] + len[i - 1];
 #pragma unroll
