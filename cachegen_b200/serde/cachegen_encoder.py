@@ -17,7 +17,6 @@ cg_encode_kv_flat).  quantize_and_tables, encode_streams and pack_sparse_tables 
 import collections
 import ctypes
 import dataclasses
-import functools
 import threading
 from typing import Tuple
 
@@ -128,15 +127,10 @@ def _collect(output_buffer: torch.Tensor, output_lengths: torch.Tensor, status: 
         if outside:
             raise RuntimeError("collect_bytes: a length is negative or exceeds the buffer's row size")
         out = torch.empty(total, dtype=torch.uint8, device=dev)
-        rc = lib.cg_compact_streams(_ptr(buf), stride, _ptr(lengths), _ptr(offsets), _ptr(_zero(dev)), 1, NL, C, _ptr(out), stream)
+        # the only sub-chunk starts where its first group does, at 0
+        rc = lib.cg_compact_streams(_ptr(buf), stride, _ptr(lengths), _ptr(offsets), _ptr(offsets), 1, NL, C, _ptr(out), stream)
     _lib.check(rc, "cg_compact_streams")
     return out, bits
-
-
-@functools.lru_cache(maxsize=64)
-def _zero(dev) -> torch.Tensor:
-    """The offset of an only sub-chunk."""
-    return torch.zeros(1, dtype=torch.int64, device=dev)
 
 
 @_lmcache_nvtx_annotate

@@ -64,3 +64,23 @@ def test_recombined_rows_are_collected_again():
     lens_t = torch.from_numpy(lens).cuda()
     b = torch.from_numpy(gathered(buf, lens)).cuda()
     assert torch.equal(E.collect_bytes(D.recombine_bytes(b, lens_t), lens_t), b)
+
+
+def test_collect_bytes_keeps_no_tensor_filled_on_one_callers_stream(monkeypatch):
+    """A tensor that is filled on the first caller's stream and kept would be read on another stream before it is."""
+    from cachegen_b200.serde import cachegen_encoder as E
+    buf, lens = rows_of(np.random.default_rng(4), 2, 60, 64, 50)
+    buf_t, lens_t = torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda()
+
+    def refuse(*a, **kw):
+        raise AssertionError("a filled tensor")
+    for name in ("zeros", "full", "tensor", "zeros_like"):
+        monkeypatch.setattr(torch, name, refuse)
+    for value in vars(E).values():
+        if hasattr(value, "cache_clear"):
+            value.cache_clear()
+    for _ in range(2):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+            got = E.collect_bytes(buf_t, lens_t).cpu()
+        assert got.numpy().tobytes() == gathered(buf, lens).tobytes()
