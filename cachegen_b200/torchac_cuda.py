@@ -47,7 +47,9 @@ def _status_word(device):
     w = _status.get(key)
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=device)
-        _status[key] = w
+        if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(w.device).synchronize()  # zero on every stream that uses it from here on
+        w = _status.setdefault(key, w)
     return w
 
 
