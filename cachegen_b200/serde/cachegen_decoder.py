@@ -435,7 +435,7 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
     dev = _device_of(first) if _on_gpu(first) else torch.device("cuda", torch.cuda.current_device())
     if groups == 1 or _on_gpu(first):
         return decode_many(encoder_outputs, bins, fmt, out_dtype, out=out,
-                           workspace=workspaces[0] if workspaces else None, host_bins=host_bins)
+                           workspace=workspaces[0] if workspaces else None, delta=delta, host_bins=host_bins)
     L, H, D = bins.numel() // 2, first.num_heads, first.head_size
     total_T = sum(_chunk_tokens(eo) for eo in encoder_outputs)
     shape = (L, 2, total_T, H, D) if fmt == "vllm" else (L, 2, H, total_T, D)

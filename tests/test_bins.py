@@ -16,6 +16,13 @@ def serializer(config):
                               LMCacheEngineMetadata("bins", 1, 0, "vllm"), config)
 
 
+def deserializer(config, delta=None):
+    from cachegen_b200.config import LMCacheEngineConfig, LMCacheEngineMetadata
+    from cachegen_b200.serde import CacheGenDeserializer
+    return CacheGenDeserializer(LMCacheEngineConfig.from_defaults(chunk_size=256),
+                                LMCacheEngineMetadata("bins", 1, 0, "vllm"), config, torch.float16, delta)
+
+
 def make_kv():
     return torch.randn((4, 2, 70, 2, 64), generator=torch.Generator().manual_seed(4)).half().cuda()
 
@@ -137,3 +144,33 @@ def test_one_workspace_for_decodes_with_different_bins(compact):
         got = D.decode_to_kv(chunk, bins, "vllm", torch.float16, workspace=ws)
         assert torch.equal(got, D.decode_to_kv(E.encode_function(kv, None, kb, vb, 70), bins, "vllm", torch.float16))
         assert int(ws["status"].item()) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wire", ["pickle", "flat"])
+@pytest.mark.parametrize("host,groups", [(False, 1), (False, 2), (True, 1), (True, 2), (True, None)])
+def test_delta_coded_chunks_through_the_pipelined_decode(wire, host, groups):
+    import dataclasses
+    from cachegen_b200.serde import cachegen_basics as B, cachegen_decoder as D
+    base, _ = configs()
+    delta = B.DeltaCoding(4)
+    ser, de = serializer(base), deserializer(base, delta)
+    ser.delta = delta
+    kvs = [make_kv(), make_kv().flip(2), make_kv().flip(0)]
+    chunks = [ser.encode_flat(kv) if wire == "flat" else ser.encode(kv) for kv in kvs]
+    want = torch.cat([de.decode(c) for c in chunks], dim=2)
+
+    def pinned(c):
+        if wire == "flat":
+            return c.pin_memory()
+        pin = lambda t: t.cpu().pin_memory()
+        data = [dataclasses.replace(d, bytestream=pin(d.bytestream), bytestream_lengths=pin(d.bytestream_lengths)) for d in c.data_chunks]
+        return dataclasses.replace(c, data_chunks=data, cdf=pin(c.cdf), max_tensors_key=pin(c.max_tensors_key),
+                                   max_tensors_value=pin(c.max_tensors_value))
+    given = [pinned(c) for c in chunks] if host else chunks
+    for some in (given, given[:1]):
+        got = de.decode_many_host(some, groups=groups)
+        assert torch.equal(got, want[:, :, :70 * len(some)])
+    bins = torch.cat((B.make_key_bins(base), B.make_value_bins(base)))
+    got = D.decode_many_pipelined(given, bins, "vllm", torch.float16, groups=groups or 4, delta=delta)
+    assert torch.equal(got, want)
