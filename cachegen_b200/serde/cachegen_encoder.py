@@ -449,6 +449,8 @@ def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     `info`: what the bins are, when the caller knows (see CacheGenSerializer._bins); read from the tensors otherwise."""
     info = info or _BinsInfo(key_bins, value_bins)
     kmax = info.table_bins(max_bins)
+    if kv.stride(4) != 1:
+        kv = kv.contiguous()  # on the caller's stream, before the others wait for it
     T = kv.shape[2]
     info.on(kv.device)
     caller = torch.cuda.current_stream(kv.device)

@@ -91,3 +91,23 @@ def test_more_sub_chunks_than_one_launch_takes():
     got = D.decode_many(chunks, bins, "vllm", torch.float16, workspace=ws)
     want = torch.cat([D.decode_to_kv(c, bins, "vllm", torch.float16) for c in chunks], dim=2)
     assert int(ws["status"].item()) == 0 and torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+def test_encode_many_of_a_cache_with_another_innermost_stride(monkeypatch):
+    """What has to be copied first is copied before the side streams start, not beside them."""
+    from cachegen_b200.serde import cachegen_encoder as E
+    kb, vb = bins_of(2, 16)
+    kv = make_kv(2, 90, 2, 64, torch.float16, 6)
+    want = E.encode_many(kv, kb, vb, 30)
+    strided, contiguous = kv.transpose(3, 4).contiguous().transpose(3, 4), torch.Tensor.contiguous
+
+    def late(t, *a, **kw):  # copies of the cache, or of a part of it, run some 20 ms after they were asked for
+        if t.dim() == 5:
+            torch.cuda._sleep(40_000_000)
+        return contiguous(t, *a, **kw)
+    monkeypatch.setattr(torch.Tensor, "contiguous", late)
+    torch.cuda.synchronize()
+    got = E.encode_many(strided, kb, vb, 30)
+    assert strided.stride(4) != 1 and len(got) == 3
+    for a, b in zip(got, want):
+        assert torch.equal(a.cdf, b.cdf) and torch.equal(a.data_chunks[0].bytestream, b.data_chunks[0].bytestream)
