@@ -99,7 +99,8 @@ def _check_chunk(eo: CacheGenGPUEncoderOutput):
     L = NL // 2
     mk, mv = eo.max_tensors_key, eo.max_tensors_value
     T = mk.shape[1]
-    if eo.num_heads * eo.head_size != C or mk.shape[0] != L or mv.shape[0] != L or mv.shape[1] != T:
+    if eo.num_heads * eo.head_size != C or mk.shape[0] != L or mv.shape[0] != L or mv.shape[1] != T or not (
+            mk.numel() == mv.numel() == L * T):  # one scale per (layer, token): they are read by address
         raise RuntimeError("inconsistent shapes in the encoded chunk")
     if mk.dtype not in _DTYPES or mk.dtype != mv.dtype:
         raise TypeError(f"scales must be float16 or bfloat16, got {mk.dtype} / {mv.dtype}")
