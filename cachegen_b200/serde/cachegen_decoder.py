@@ -465,6 +465,9 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
             ready.record(copy_stream)
         cur.wait_event(ready)
         plan.run()
+        # the workspace's tensors come from the copy stream's pool; run sees to the plan's other inputs
+        for t in (plan.goff, plan.status):
+            t.record_stream(cur)
         t0 += tg
     return out
 
