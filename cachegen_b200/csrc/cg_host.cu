@@ -15,8 +15,9 @@
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
+#include <exception>
+#include <memory>
 #include <mutex>
-#include <new>
 #include <thread>
 #include <vector>
 
@@ -236,7 +237,9 @@ struct Stage {
 };
 }  // namespace
 
-extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *staging, int64_t staging_bytes, void *stream) {
+// No C++ exception may leave an entry: the callers are C.  What can throw is host memory that is not there, before the helpers know
+// of a job, so nothing is in use when a job goes away.
+extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *staging, int64_t staging_bytes, void *stream) try {
     int64_t count;
     if (int rc = check_segments(segs, nsegs, staging, staging_bytes, &count)) return rc;
     if (!count) return CG_OK;
@@ -260,20 +263,23 @@ extern "C" int cg_host_upload(const cg_host_segment *segs, int nsegs, void *stag
     while (!job.taken()) job.work();  // only after an error: nobody may touch the job once it is gone
     if (k > 1) helpers().remove(&job);
     return err == cudaSuccess ? CG_OK : set_cuda_error(err);
+} catch (const std::exception &) {
+    return CG_E_CAPACITY;
 }
 
-extern "C" int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle) {
+extern "C" int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle) try {
     if (!host || !staging || !handle) return CG_E_NULL;
     if (bytes <= 0 || (bytes + kPiece - 1) / kPiece > 0x7FFFFFFF) return CG_E_SHAPE;
     if (bytes > staging_bytes) return CG_E_CAPACITY;
-    Stage *s = new (std::nothrow) Stage(host, bytes, staging, staging_bytes);
-    if (!s) return CG_E_CAPACITY;
+    std::unique_ptr<Stage> s(new Stage(host, bytes, staging, staging_bytes));
     helpers().add(&s->job);
-    *handle = s;
+    *handle = s.release();
     return CG_OK;
+} catch (const std::exception &) {
+    return CG_E_CAPACITY;
 }
 
-extern "C" int cg_host_stage_send(void *handle, const cg_host_segment *segs, int nsegs, void *stream) {
+extern "C" int cg_host_stage_send(void *handle, const cg_host_segment *segs, int nsegs, void *stream) try {
     if (!handle || !segs) return CG_E_NULL;
     Stage &s = *static_cast<Stage *>(handle);
     std::vector<Part> parts;
@@ -300,6 +306,8 @@ extern "C" int cg_host_stage_send(void *handle, const cg_host_segment *segs, int
     }
     const cudaError_t err = send_parts(s.job, parts, static_cast<cudaStream_t>(stream));
     return err == cudaSuccess ? CG_OK : set_cuda_error(err);
+} catch (const std::exception &) {
+    return CG_E_CAPACITY;
 }
 
 extern "C" int cg_host_stage_end(void *handle) {
@@ -341,7 +349,7 @@ constexpr int64_t kMaxUnits = 64;
 }  // namespace
 
 extern "C" int cg_host_download(const cg_host_segment *segs, int nsegs, void *staging, int64_t staging_bytes, int phase,
-                                void *stream) {
+                                void *stream) try {
     int64_t count;
     if (phase < 0 || phase > 2) return CG_E_SHAPE;
     if (!segs || !staging) return CG_E_NULL;
@@ -446,4 +454,7 @@ extern "C" int cg_host_download(const cg_host_segment *segs, int nsegs, void *st
     if (err != cudaSuccess) job.next.store(lead + n, std::memory_order_relaxed);  // nothing more to take
     if (n > 1) helpers().remove(&job);
     return err == cudaSuccess ? CG_OK : set_cuda_error(err);
+} catch (const std::exception &) {
+    cudaStreamSynchronize(static_cast<cudaStream_t>(stream));  // transfers may be on their way to the staging memory
+    return CG_E_CAPACITY;
 }

@@ -43,3 +43,24 @@ def test_processor_instructions_stand_behind_the_guard():
         if name.endswith((".cu", ".cuh", ".h")) and name != "cg_hostcopy.h":
             text = open(os.path.join(csrc, name)).read()
             assert not re.search(r"immintrin|_mm\d*_|__m(128|256|512)|target\(\"|\"lock|__builtin_cpu", text), name
+
+
+OUT_OF_MEMORY = """
+import ctypes, resource, sys
+sys.path.insert(0, {root!r})
+from cachegen_b200 import _lib
+lib, here = _lib.lib(), ctypes.create_string_buffer(4096)
+at, n = ctypes.addressof(here), 1 << 40  # 2^40 bytes are 2^23 pieces, whose list takes more than is left
+used = 4096 * int(open("/proc/self/statm").read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (used + (64 << 20), used + (64 << 20)))
+handle = ctypes.c_void_p()
+seg = (_lib.HostSegment * 1)((at, at, n))
+print(lib.cg_host_stage(at, n, at, n, ctypes.byref(handle)), lib.cg_host_upload(seg, 1, at, n, None), handle.value)
+"""
+
+
+def test_no_exception_leaves_an_entry():
+    """Host memory that is not there is an error code, not the end of the process."""
+    import sys
+    run = subprocess.run([sys.executable, "-c", OUT_OF_MEMORY.format(root=ROOT)], capture_output=True, text=True)
+    assert run.returncode == 0 and run.stdout.split() == ["-6", "-6", "None"], run.stdout + run.stderr
