@@ -439,8 +439,7 @@ int quant_shape(const void *kv, int dtype, int64_t s_layer, int64_t s_kv, int64_
 // 0.60 ms against 0.54 ms for the whole encode.  So one window: all rows.
 int window_rows(const QuantShape &q) { return 2 * q.L.nlayers; }
 
-int launch_absmax(const uint16_t *x, const QuantShape &q, uint16_t *sc, cudaStream_t st, int row0 = 0, int nrows = -1) {
-    if (nrows < 0) nrows = 2 * q.L.nlayers;
+int launch_absmax(const uint16_t *x, const QuantShape &q, uint16_t *sc, cudaStream_t st, int row0, int nrows) {
     const int64_t nwarps = static_cast<int64_t>(nrows) * q.L.ntokens;
     const unsigned ablocks = static_cast<unsigned>((nwarps * 32 + 255) / 256);
     if (q.vec) row_absmax_kernel<8><<<ablocks, 256, 0, st>>>(x, q.L, sc, row0, nrows);
@@ -450,9 +449,8 @@ int launch_absmax(const uint16_t *x, const QuantShape &q, uint16_t *sc, cudaStre
 
 int launch_quantize(const uint16_t *x, int dtype, const QuantShape &q, const float *bins, const uint16_t *sc,
                     int max_bins, int8_t *sym_out, int16_t *cdf_out, uint8_t *counts_out,
-                    const int64_t *table_row_off, int32_t *status, cudaStream_t st, const float *res_bins = nullptr,
-                    int group = 0, int row0 = 0, int nrows = -1) {
-    if (nrows < 0) nrows = 2 * q.L.nlayers;
+                    const int64_t *table_row_off, int32_t *status, cudaStream_t st, const float *res_bins, int group, int row0,
+                    int nrows) {
     const int C = q.L.nheads * q.L.head_size;
     const dim3 grid((C + kGroup - 1) / kGroup, nrows);
     const size_t smem = hist_smem_bytes(max_bins);
@@ -485,34 +483,6 @@ int launch_residual_absmax(const uint16_t *x, int dtype, const QuantShape &q, co
 }
 
 }  // namespace
-
-extern "C" int cg_row_absmax(const void *kv, int dtype, int64_t s_layer, int64_t s_kv, int64_t s_token,
-                             int64_t s_head, int nlayers, int ntokens, int nheads, int head_size,
-                             void *scales_out, void *stream) {
-    if (!kv || !scales_out) return CG_E_NULL;
-    QuantShape q;
-    // the symbol pointer only matters for the quantise pass: any 8-byte aligned value keeps the choice of load width
-    if (int rc = quant_shape(kv, dtype, s_layer, s_kv, s_token, s_head, nlayers, ntokens, nheads, head_size, nullptr, &q))
-        return rc;
-    return launch_absmax(static_cast<const uint16_t *>(kv), q, static_cast<uint16_t *>(scales_out),
-                         static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int cg_quantize_cdf_scaled(const void *kv, int dtype, int64_t s_layer, int64_t s_kv, int64_t s_token,
-                                      int64_t s_head, int nlayers, int ntokens, int nheads, int head_size,
-                                      const float *bins, int max_bins, const void *scales, int8_t *sym_out,
-                                      int16_t *cdf_out, uint8_t *counts_out, const int64_t *table_row_off,
-                                      int32_t *status, void *stream) {
-    if (!kv || !bins || !sym_out || !scales || !cdf_out) return CG_E_NULL;
-    if (counts_out && !table_row_off) return CG_E_NULL;
-    if (max_bins < 1 || max_bins >= CG_MAX_LP) return CG_E_LP;
-    QuantShape q;
-    if (int rc = quant_shape(kv, dtype, s_layer, s_kv, s_token, s_head, nlayers, ntokens, nheads, head_size, sym_out, &q))
-        return rc;
-    return launch_quantize(static_cast<const uint16_t *>(kv), dtype, q, bins, static_cast<const uint16_t *>(scales),
-                           max_bins, sym_out, cdf_out, counts_out, table_row_off, status,
-                           static_cast<cudaStream_t>(stream));
-}
 
 extern "C" int cg_quantize_cdf(const void *kv, int dtype, int64_t s_layer, int64_t s_kv, int64_t s_token,
                                int64_t s_head, int nlayers, int ntokens, int nheads, int head_size,

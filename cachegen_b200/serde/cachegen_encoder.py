@@ -10,7 +10,7 @@ torch ops and per-sub-chunk launches replaced by three C-ABI calls:
 
 Beside it: encode_many (a whole cache, chunks in flight on several streams and no wait in between), encode_levels
 (one chunk at several bin settings) and encode_flat (the CGB2 container of flat_format.py, filled by
-cg_encode_kv_flat).  quantize_and_tables, encode_streams and pack_sparse_tables are the same steps one by one.
+cg_encode_kv_flat).  quantize_and_tables and encode_streams are the same steps one by one.
 
 (enc.py = cachegen_encoder.py of the reference.)
 """
@@ -151,23 +151,8 @@ def encode_ntokens(cdf_int: torch.Tensor, encode_input: torch.Tensor, output_buf
     return out
 
 
-def row_scales(kv: torch.Tensor) -> torch.Tensor:
-    """max|x| over the channels of every (row, token): [2L, T] in kv.dtype, key rows then value rows
-    (the max1 of torch_quant_vectorized, enc.py:55).  It does not depend on the bin settings."""
-    if kv.dim() != 5 or kv.shape[1] != 2 or kv.dtype not in _DTYPES or not kv.is_cuda or kv.stride(4) != 1:
-        raise RuntimeError("expected a CUDA float16/bfloat16 KV blob [L, 2, T, H, D] with a unit innermost stride")
-    L, _, T, H, D = kv.shape
-    scales = torch.empty((2 * L, T), dtype=kv.dtype, device=kv.device)
-    with torch.cuda.device(kv.device):
-        rc = _lib.lib().cg_row_absmax(_ptr(kv), _DTYPES[kv.dtype], kv.stride(0), kv.stride(1), kv.stride(2),
-                                      kv.stride(3), L, T, H, D, _ptr(scales), _stream(kv.device))
-    _lib.check(rc, "cg_row_absmax")
-    return scales
-
-
 def quantize_and_tables(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tensor, max_bins: int,
-                        with_counts: bool = False, scales: torch.Tensor = None, bins_cpu: torch.Tensor = None,
-                        delta: "CGBasics.DeltaCoding" = None):
+                        with_counts: bool = False, delta: "CGBasics.DeltaCoding" = None):
     """Fused torch_quant_vectorized (K and V) + calculate_cdf (K and V) + the two torch.cat of
     encode_function (enc.py:42-59, 257-267).
 
@@ -175,9 +160,7 @@ def quantize_and_tables(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: to
         the permuted view of a "huggingface" blob is read in place).
     Returns (symbols int8 [2L, T, C], scales [2L, T] in kv.dtype, tables int16 [2L, C, max_bins + 1]);
     with_counts adds (byte counts uint8 of the compact table form, int32 status word whose
-    CG_S_COUNT_OVERFLOW bit says they are unusable for this chunk).  `scales`: the result of row_scales
-    for this blob, when it is already known (encoding one chunk at several bin settings).  `bins_cpu`:
-    a host copy of the concatenated bins, to save the transfer.
+    CG_S_COUNT_OVERFLOW bit says they are unusable for this chunk).
     """
     if kv.dim() != 5 or kv.shape[1] != 2:
         raise RuntimeError(f"expected a KV blob of shape [L, 2, T, H, D], got {tuple(kv.shape)}")
@@ -194,16 +177,11 @@ def quantize_and_tables(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: to
     if bins.numel() != 2 * L:
         raise RuntimeError(f"bins describe {bins.numel() // 2} layers, the KV blob has {L}")
     sym = torch.empty((2 * L, T, C), dtype=torch.int8, device=dev)
-    given = scales is not None
-    if given and (tuple(scales.shape) != (2 * L, T) or scales.dtype != kv.dtype or scales.device != dev or
-                  not scales.is_contiguous()):
-        raise RuntimeError("scales must be a contiguous [2L, T] tensor of the blob's dtype on its device")
-    if not given:
-        scales = torch.empty((2 * L, T), dtype=kv.dtype, device=dev)
+    scales = torch.empty((2 * L, T), dtype=kv.dtype, device=dev)
     cdf = torch.empty((2 * L, C, max_bins + 1), dtype=torch.int16, device=dev)
     counts = row_off = status = None
     if with_counts:
-        offs = flat_format.table_row_offsets(bins.cpu() if bins_cpu is None else bins_cpu, C)
+        offs = flat_format.table_row_offsets(bins.cpu(), C)
         row_off = torch.tensor(offs, dtype=torch.int64, device=dev)
         counts = torch.empty(offs[-1], dtype=torch.uint8, device=dev)
         status = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -214,12 +192,8 @@ def quantize_and_tables(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: to
             _ptr(bins), int(max_bins))
     with torch.cuda.device(dev):
         if delta is not None:
-            if given:
-                raise RuntimeError("precomputed scales cannot be combined with delta coding")
             res_bins = delta.residual_bins(key_bins, value_bins, dev)
             rc = _lib.lib().cg_quantize_cdf_delta(*head, delta.group, _ptr(res_bins), _ptr(sym), _ptr(scales), *tail)
-        elif given:
-            rc = _lib.lib().cg_quantize_cdf_scaled(*head, _ptr(scales), _ptr(sym), *tail)
         else:
             rc = _lib.lib().cg_quantize_cdf(*head, _ptr(sym), _ptr(scales), *tail)
     _lib.check(rc, "cg_quantize_cdf")
@@ -228,13 +202,12 @@ def quantize_and_tables(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: to
     return sym, scales, cdf
 
 
-def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = None, extra_status: torch.Tensor = None):
+def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = None):
     """The sub-chunk loop of encode_function in one pass (enc.py:269-292).
 
     cdf int16 [2L, C, Lp], sym int8 [2L, T, C] contiguous.  Returns (bytes uint8 [total], lengths int32
     [nsub, 2L, C], sub_off: python list of nsub+1 byte offsets of the sub-chunks inside `bytes`).
-    Synchronises once, to size the output; `extra_status` (one or more integer words on the GPU) is read
-    in the same transfer and appended to the result (an int, or a list of ints for several words).
+    Synchronises once, to size the output.
     """
     NL, T, C = sym.shape
     lp = cdf.shape[2]
@@ -253,8 +226,7 @@ def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = N
         rc = L.cg_encode_chunk(_ptr(cdf), _ptr(sym), NL, T, C, lp, _ptr(scratch), stride, _ptr(lengths),
                                _ptr(group_off), _ptr(sub_off), _ptr(status), _stream(dev))
         _lib.check(rc, "cg_encode_chunk")
-        words = [sub_off, status.to(torch.int64)] + ([extra_status.to(torch.int64)] if extra_status is not None else [])
-        host = torch.cat(words).cpu()  # the one synchronisation
+        host = torch.cat((sub_off, status.to(torch.int64))).cpu()  # the one synchronisation
         bits = int(host[nsub + 1])
         if bits:
             raise RuntimeError("cachegen encode: " + _lib.status_text(bits))
@@ -263,9 +235,6 @@ def encode_streams(cdf: torch.Tensor, sym: torch.Tensor, scratch_stride: int = N
         rc = L.cg_compact_streams(_ptr(scratch), stride, _ptr(lengths), _ptr(group_off), _ptr(sub_off), nsub, NL,
                                   C, _ptr(out), _stream(dev))
         _lib.check(rc, "cg_compact_streams")
-    if extra_status is not None:
-        extra = [int(v) for v in host[nsub + 2:]]
-        return out, lengths, offs, (extra[0] if len(extra) == 1 else extra)
     return out, lengths, offs
 
 
@@ -536,29 +505,6 @@ def encode_function(kv: torch.Tensor, config: CacheGenConfig, key_bins: torch.Te
         return p.finish()
     finally:
         p.abandon()
-
-
-def pack_sparse_tables(counts: torch.Tensor, bins: torch.Tensor, nchannels: int, bins_cpu: torch.Tensor = None):
-    """Byte counts of quantize_and_tables -> the parts of the sparse table form (cg_pack_sparse_tables).
-    Returns (tables uint8 with room for every count, int32 word holding the number of counts written,
-    offset of the counts inside `tables`); the used size is that offset plus that number."""
-    dev = counts.device
-    bins_cpu = bins.cpu() if bins_cpu is None else bins_cpu
-    nrows = bins_cpu.numel()
-    count_off = torch.tensor(flat_format.table_row_offsets(bins_cpu, nchannels), dtype=torch.int64, device=dev)
-    moffs = flat_format.mask_row_offsets(bins_cpu, nchannels)
-    mask_off = torch.tensor(moffs, dtype=torch.int64, device=dev)
-    off_masks, off_counts = flat_format.sparse_parts(nrows, nchannels, moffs[-1])
-    tables = torch.zeros(off_counts + counts.numel(), dtype=torch.uint8, device=dev)
-    ngroups = nrows * ((nchannels + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().cg_pack_sparse_tables(_ptr(counts), _ptr(count_off), _ptr(bins), nrows, nchannels,
-                                              _ptr(tables), ctypes.c_void_p(tables.data_ptr() + off_masks),
-                                              _ptr(mask_off), ctypes.c_void_p(tables.data_ptr() + off_counts),
-                                              _stream(dev))
-    _lib.check(rc, "cg_pack_sparse_tables")
-    written = tables[4 * ngroups:4 * ngroups + 4].view(torch.int32)
-    return tables, written, off_counts
 
 
 def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tensor,
