@@ -408,70 +408,49 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     int nbytes = 0, nz = 0;
 
     if (TABLES && any_active) {
+        static_assert(!TABLES || NS == 1, "the tables' part has one stream a thread");
+        uint32_t *const mine = column[0];
         uint16_t *stage = reinterpret_cast<uint16_t *>(tab + p.lp * kGroup);
         bool overflow = false;
-        for (int m = 0; m < p.lp; ++m) {
-#pragma unroll
-            for (int s = 0; s < NS; ++s) column[s][m * 32] = 0u;
-        }
-        constexpr int kAhead = 16 / NS;  // words of a channel in flight
-        const uint32_t *q[NS];
-#pragma unroll
-        for (int s = 0; s < NS; ++s) q[s] = sp[s];
+        for (int m = 0; m < p.lp; ++m) mine[m * 32] = 0u;
+        constexpr int kAhead = 16;  // words in flight
+        const uint32_t *q = sp[0];
         int i = 0;
         for (; i + 4 * kAhead <= n; i += 4 * kAhead) {
-            uint32_t w[NS][kAhead], any = 0u;
+            uint32_t w[kAhead], any = 0u;
 #pragma unroll
             for (int k = 0; k < kAhead; ++k) {
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    w[s][k] = __ldg(q[s]);
-                    q[s] += C;
-                }
+                w[k] = __ldg(q);
+                q += C;
             }
 #pragma unroll
-            for (int k = 0; k < kAhead * NS; ++k) any |= w[k / kAhead][k % kAhead];
+            for (int k = 0; k < kAhead; ++k) any |= w[k];
             if (any & 0x80808080u) {  // reported below
 #pragma unroll
-                for (int k = 0; k < kAhead * NS; ++k) w[k / kAhead][k % kAhead] = 0u;
+                for (int k = 0; k < kAhead; ++k) w[k] = 0u;
             }
 #pragma unroll
             for (int k = 0; k < kAhead; ++k) {
 #pragma unroll
-                for (int s = 0; s < NS; ++s) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) count_symbol(entry_of(col[s], w[s][k], j));
-                }
+                for (int j = 0; j < 4; ++j) count_symbol(entry_of(col[0], w[k], j));
             }
         }
         for (; i < n; i += 4) {
+            uint32_t w = __ldg(q);
+            q += C;
+            if (w & 0x80808080u) w = 0u;
 #pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                uint32_t w = __ldg(q[s]);
-                q[s] += C;
-                if (w & 0x80808080u) w = 0u;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (i + j < n) count_symbol(entry_of(col[s], w, j));
-            }
+            for (int j = 0; j < 4; ++j)
+                if (i + j < n) count_symbol(entry_of(col[0], w, j));
         }
         const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
-        const int64_t at = p.out.counts ? __ldg(p.out.table_row_off + row) - row * C : 0;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            if (p.out.counts && active[s]) nz += store_counts<32>(column[s], p.lp, cq, p.out.counts + at + g[s], C, &overflow);
-            counts_to_column<32>(column[s], stage + (s * kThreads + tid) * p.lp, p.lp, n, cq);
-        }
+        if (p.out.counts && active[0])
+            nz = store_counts<32>(mine, p.lp, cq, p.out.counts + __ldg(p.out.table_row_off + row) - row * C + g[0], C, &overflow);
+        counts_to_column<32>(mine, stage + tid * p.lp, p.lp, n, cq);
         if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
         __syncwarp();
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            const int slot = s * kThreads + warp * 32, first = blockIdx.x * kGroup + slot;
-            const int nch = min(32, p.nchannels - first);
-            if (nch > 0)
-                copy_tables(stage + slot * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp,
-                            nch * p.lp, lane);
-        }
+        const int first = blockIdx.x * kGroup + warp * 32, nch = min(32, p.nchannels - first);
+        copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp, nch * p.lp, lane);
     } else if (any_active) {
 #pragma unroll
         for (int s = 0; s < NS; ++s) stage_table_column<false, 32>(column[s], p.out.cdf + g[s] * p.lp, p.lp, p.lp, 0);
