@@ -285,7 +285,8 @@ class DecodePlan:
             ws["group_off"] = goff
         status = ws.get("status")
         if status is None or status.device != dev:
-            status = torch.zeros(1, dtype=torch.int32, device=dev)
+            with torch.inference_mode(False):  # kept, and written to by later calls in whatever mode those run
+                status = torch.zeros(1, dtype=torch.int32, device=dev)
             ws["status"] = status
         row_offs = {}
         for kind, name, fn in ((_lib.CG_TABLES_COUNTS, "table_row_off", flat_format.table_row_offsets),
@@ -484,7 +485,8 @@ def _stage_flat(part: list, ws: dict, dev) -> list:
         need += (eo.blob.numel() + flat_format.ALIGN - 1) // flat_format.ALIGN * flat_format.ALIGN
     arena = ws.get("arena")
     if arena is None or arena.device != dev or arena.numel() < need:
-        arena = torch.empty(need, dtype=torch.uint8, device=dev)
+        with torch.inference_mode(False):
+            arena = torch.empty(need, dtype=torch.uint8, device=dev)
         ws["arena"] = arena
     staged = []
     for eo, a in zip(part, starts):

@@ -46,7 +46,8 @@ def _status_word(device):
     key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
     w = _status.get(key)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=device)
+        with torch.inference_mode(False):  # kept, and set back in whatever mode the check runs
+            w = torch.zeros(1, dtype=torch.int32, device=device)
         if not torch.cuda.is_current_stream_capturing():
             torch.cuda.current_stream(w.device).synchronize()  # zero on every stream that uses it from here on
         w = _status.setdefault(key, w)

@@ -174,3 +174,21 @@ def test_delta_coded_chunks_through_the_pipelined_decode(wire, host, groups):
     bins = torch.cat((B.make_key_bins(base), B.make_value_bins(base)))
     got = D.decode_many_pipelined(given, bins, "vllm", torch.float16, groups=groups or 4, delta=delta)
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+def test_what_is_kept_from_a_call_in_inference_mode_serves_calls_outside_it(monkeypatch):
+    import cachegen_b200.torchac_cuda as tc
+    base, _ = configs()
+    de, kv = deserializer(base), make_kv()
+    chunks = [serializer(base).encode_flat(kv).pin_memory() for _ in range(2)]
+    monkeypatch.setattr(tc, "_status", {})
+    with torch.inference_mode():
+        want = de.decode_many_host(chunks, groups=2)
+        tc.check_status()
+    assert torch.equal(de.decode_many_host(chunks, groups=2), want)
+    for word, check in ((de.group_status_words()[0], de.check_status), (tc._status_word(kv.device), tc.check_status)):
+        word.fill_(2)
+        with pytest.raises(RuntimeError, match="stream lengths"):
+            check()
+        check()  # set back
