@@ -96,9 +96,9 @@ def _collect(output_buffer: torch.Tensor, output_lengths: torch.Tensor, status: 
         raise TypeError("expected a CUDA uint8 buffer [nlayers, nchannels, row]")
     buf, lengths = output_buffer.contiguous(), output_lengths.to(torch.int32).contiguous()
     NL, C, stride = buf.shape
-    if tuple(lengths.shape) != (NL, C):
-        raise RuntimeError("output_lengths must have shape [nlayers, nchannels]")
     dev = buf.device
+    if tuple(lengths.shape) != (NL, C) or lengths.device != dev:
+        raise RuntimeError("output_lengths must have shape [nlayers, nchannels], on the buffer's GPU")
     nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
     offsets = torch.empty(NL * nslab, dtype=torch.int64, device=dev)
     lib, stream = _lib.lib(), _stream(dev)

@@ -84,3 +84,10 @@ def test_collect_bytes_keeps_no_tensor_filled_on_one_callers_stream(monkeypatch)
             torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
             got = E.collect_bytes(buf_t, lens_t).cpu()
         assert got.numpy().tobytes() == gathered(buf, lens).tobytes()
+
+
+def test_collect_bytes_refuses_lengths_in_host_memory():
+    from cachegen_b200.serde import cachegen_encoder as E
+    buf, lens = rows_of(np.random.default_rng(5), 2, 60, 64, 50)
+    with pytest.raises(RuntimeError, match="on the buffer's GPU"):
+        E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens))
