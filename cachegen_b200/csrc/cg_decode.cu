@@ -383,8 +383,9 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
 // values with one 2*NS-byte store.  Channel NS*t + i keeps its table in column t + i * (128 / NS), so a
 // warp still reads 32 different banks whatever entries its lanes are at.  The search depth is chosen
 // per block from the row's bin count (see decode_streams); the result does not depend on it.
-// Bound by instruction issue (70 % of the slots, the integer and multiply pipes in turn): 8,192 Llama-7B tokens
-// in 4.18 ms, 1,261 GB/s of algorithmic bytes; 4.50 ms before the search on an estimate and the one-shift renormalisation.
+// Bound by instruction issue (58.7 instructions for 32 symbols: 80 % of the slots at 2,048 tokens, 81 % at 8,192, where the
+// last wave weighs less; the integer pipe 63 %): 8,192 Llama-7B tokens in 4.18 ms, 1,261 GB/s of algorithmic bytes; 4.50 ms
+// before the search on an estimate and the one-shift renormalisation.
 // Needs a head size and output strides that are multiples of NS and output pointers aligned to 2*NS bytes.
 template <int OUT_DT>
 __device__ __forceinline__ uint32_t pack_pair(float v0, float v1);

@@ -32,8 +32,8 @@ __device__ __forceinline__ uint64_t pack2(float a, float b) {
     return r;
 }
 // (x * f + m) + 2^23 for two values: three separately rounded fp32 operations each (enc.py:56-57), the last of which
-// rounds half to even and leaves the symbol in the low byte.  The products stay scalar: a packed product in
-// front of a packed sum came out as one fused multiply-add (a symbol in 10^7 differed).
+// rounds half to even and leaves the symbol in the low byte.  The products stay scalar: with packed products in front of
+// the packed sums a symbol in 10^7 differed, as if product and sum had been rounded once.
 __device__ __forceinline__ void quantize2(float x0, float x1, float f, uint64_t m, uint32_t *b0, uint32_t *b1) {
     const uint64_t magic = 0x4B0000004B000000ull;
     uint64_t v = pack2(__fmul_rn(x0, f), __fmul_rn(x1, f));
@@ -231,9 +231,11 @@ __device__ __forceinline__ void count_symbol(uint32_t addr) {
 }
 
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
-// block (slab, row), thread (channel, part) counts every kParts-th word of its channel.  Bound by the shared-memory
-// updates, one a symbol (1.7 cycles a warp and SM): 1,999 tokens of 32 layers x 1,024 channels in 55 us; with 256
-// or 1,024 threads a block 55 and 67.
+// block (slab, row), thread (channel, part) counts every kParts-th word of its channel.  Bound by instruction issue
+// (75 % of the slots, 9.5 instructions for 32 symbols with the tables): 1,999 tokens of 32 layers x 1,024 channels in 55 us;
+// with 256 or 1,024 threads a block 55 and 67.  The updates alone, one a symbol at 1.7 cycles a warp and SM, would
+// take 24, and the shared memory is busy for a third of the time; 512 blocks are 3.5 an SM, and while a block's 128
+// columns become tables its other 384 threads wait.
 constexpr int kTableThreads = 512, kParts = kTableThreads / kGroup;
 __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint32_t *__restrict__ sym4, int ntokens,
                                                                       int nchannels, int lp, const TableOut out,

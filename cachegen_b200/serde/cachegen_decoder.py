@@ -1,10 +1,14 @@
 """CacheGenDeserializer (reference: LMCache/lmcache/storage_backend/serde/cachegen_decoder.py:114-173).
 
 `from_bytes` keeps the reference's contract -- pickled CacheGenGPUEncoderOutput in, KV blob tensor on
-the GPU out, bf16 [L,2,T,H,D] for "vllm" and fp16 [L,2,H,T,D] for "huggingface" -- with the
-per-sub-chunk launches and the fp32 dequantise / stack / permute / cast chain replaced by two C-ABI
-calls: cg_decode_offsets (the cumsum of dec.py:70) and cg_decode_dequant (everything else).
+the GPU out, bf16 [L,2,T,H,D] for "vllm" and fp16 [L,2,H,T,D] for "huggingface" -- with the cumsum of
+dec.py:70, the per-sub-chunk launches and the fp32 dequantise / stack / permute / cast chain replaced by one
+C-ABI call, cg_decode_kv (two launches per 40 sub-chunks).  Its two halves, cg_decode_offsets and
+cg_decode_dequant, are what a plan's run_offsets and run_decode call.
 (dec.py = cachegen_decoder.py of the reference.)
+
+One deserializer's calls share its offset buffer and status word: they belong on one stream, from one thread at a
+time.  Serializers share nothing between calls.
 """
 import _thread
 import ctypes
@@ -233,7 +237,7 @@ def _device_of(eo):
 
 
 class DecodePlan:
-    """Everything cg_decode_offsets / cg_decode_dequant need for a list of encoded chunks, built once:
+    """Everything cg_decode_kv needs for a list of encoded chunks, built once:
     device-resident inputs, the job descriptors, the output blob and the launch arguments.  Chunks are
     CacheGenGPUEncoderOutput objects (the reference's blob, unpickled) or flat_format.FlatChunk
     containers, on the GPU or in (pinned) host memory."""
@@ -397,7 +401,7 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
     shape [L,2,T,H,D] ("vllm") or [L,2,H,T,D] ("huggingface"), T the total token count -- what
     LMCacheEngine.retrive builds with torch.cat from per-chunk from_bytes calls
     (LMCache/lmcache/cache_engine.py:282-320 in the reference).  All sub-chunks of all chunks go
-    through cg_decode_offsets + cg_decode_dequant in batches of up to 40 per launch.
+    through one cg_decode_kv, in batches of up to 40 per launch.
 
     The chunks' tensors may live on the GPU or in (pinned) host memory; host tensors are copied to the
     GPU on the current stream first.  bins: float32 [2L] on the GPU (key bins then value bins).

@@ -410,8 +410,8 @@ def encode_many(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     """Encodes a whole KV cache [L, 2, T, H, D] (GPU, unit innermost stride) chunk by chunk, as
     LMCacheEngine.store does with one to_bytes call per chunk (LMCache/lmcache/cache_engine.py:205-255
     in the reference), but without waiting for a chunk's payload size before the next chunk's kernels
-    are enqueued: up to `batch` chunks, two a stream, are in flight; a chunk's streams are gathered when its
-    turn to be replaced comes, so the host waits for sizes that arrived long ago.  Every chunk in
+    are enqueued: up to `batch` chunks, but no more than two a stream (six by default), are in flight; a chunk's
+    streams are gathered when its turn to be replaced comes, so the host waits for sizes that arrived long ago.  Every chunk in
     flight keeps its own workspace (200 MB for a 7B-shape chunk).  Consecutive chunks run on `streams` side
     streams in turn (see _side_streams); the caller's stream waits for them before the call returns.
     Returns the chunks' CacheGenGPUEncoderOutput objects, identical to per-chunk encode_function calls.
@@ -622,7 +622,8 @@ class CacheGenSerializer(Serializer):
 
     def encode_many(self, tensor: torch.Tensor, chunk_tokens: int = None, batch: int = 16, streams: int = 3) -> list:
         """A whole KV cache, one encoded chunk per `chunk_tokens` (default: the configured chunk size)
-        tokens, with up to `batch` chunks in flight on the GPU, on `streams` streams in turn."""
+        tokens, with up to `batch` chunks, but no more than two a stream, in flight on the GPU, on `streams` streams
+        in turn."""
         if self.fmt == "huggingface":
             tensor = tensor.permute(0, 1, 3, 2, 4)
         tensor = tensor.cuda()

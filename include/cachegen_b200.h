@@ -83,7 +83,7 @@ extern "C" {
 #define CG_E_TOKENS (-3)      /* more than CG_MAX_TOKENS_PER_STREAM tokens in a coder call */
 #define CG_E_LP (-4)          /* CDF length outside [2, CG_MAX_LP] / max_bins outside [1, 63] */
 #define CG_E_ALIGN (-5)       /* pointer or stride breaks an alignment rule of the call */
-#define CG_E_CAPACITY (-6)    /* scratch / workspace too small, or too many jobs */
+#define CG_E_CAPACITY (-6)    /* scratch / workspace too small, too many jobs, or no host memory for a call's lists */
 #define CG_E_DTYPE (-7)       /* unknown 16-bit float code */
 #define CG_E_CUDA (-8)        /* the CUDA runtime refused the launch; see cg_last_cuda_error */
 #define CG_E_HIST (-9)        /* ntokens >= 65536: the reference's uint16 histogram would wrap */
@@ -257,7 +257,7 @@ int cg_encode_chunk(const int16_t *cdf, const int8_t *sym, int nrows, int ntoken
  * Second half of collect_bytes (cachegen_encoder.py:210-222): gathers the first `length` bytes of
  * every scratch row into bytes_out (uint8, sub_off[nsub] bytes, as sized by the caller after
  * reading sub_off_out of cg_encode_chunk), streams back to back in (sub-chunk, row, channel) order.
- * lengths, group_off and sub_off are the arrays cg_encode_chunk wrote.
+ * lengths, group_off and sub_off are the arrays cg_encode_chunk wrote.  Rows may hold anything behind their streams.
  */
 int cg_compact_streams(const uint8_t *scratch, int64_t scratch_stride, const int32_t *lengths,
                        const int64_t *group_off, const int64_t *sub_off, int nsub, int nrows,
