@@ -448,7 +448,7 @@ def leg_reference_cuda_ext(h, ser, de, kv_chunk, eo):
 
 
 def leg_config3(h, args):
-    """the Mistral-7B GQA shape (32 layers x 8 KV heads x 128), 32,768 tokens, key
+    """The Mistral-7B GQA shape (32 layers x 8 KV heads x 128), 32,768 tokens, key
     rho 0.95, decode only from pre-encoded streams on this GPU."""
     torch = h.torch
     from cachegen_b200.synth import WORKLOADS, generate_kv
@@ -503,7 +503,7 @@ def leg_whole_context(h, spec, args):
 
 
 def leg_config5(h, args):
-    """BASELINE config 5, shortened: requests of the Llama-7B shape, 4,096 tokens each (seeds 100..), split
+    """Requests of the Llama-7B shape, 4,096 tokens each (seeds 100..), split
     evenly over three quality levels (default bins, half, quarter with a minimum of 4); every request is
     encoded and decoded on this GPU.  Six requests instead of 64: the per-request work is identical."""
     torch = h.torch
@@ -591,7 +591,7 @@ def leg_anchor_delta(h, spec, kv_part):
 
 
 def leg_delivered_kv(h, args):
-    """BASELINE config 4 in the process group of the --gpus N run: the Llama-70B-shape cache (80 layers x 8
+    """In the process group of the --gpus N run, the Llama-70B-shape cache (80 layers x 8
     KV heads x 128, 16,384 tokens) sharded by layers, every rank decodes its layers and the decoded KV is
     delivered into one blob on GPU 0 -- by pipelined peer copies while the decode runs, and by NCCL
     send/recv after it.  Plain peer copies and NCCL only."""
@@ -645,7 +645,7 @@ def leg_delivered_kv(h, args):
 
 
 def leg_token_sharded(h, args):
-    """BASELINE config 3 on the GPUs of the --gpus N run: ONE request of the Mistral-7B GQA shape (32 layers
+    """On the GPUs of the --gpus N run, ONE request of the Mistral-7B GQA shape (32 layers
     x 8 KV heads x 128, 32,768 tokens = 128 chunks) sharded by token chunks -- every rank decodes a
     contiguous run of the chunks -- with the decoded KV delivered into that token range of one blob on GPU 0
     by pipelined peer copies.  Rank 0 also decodes the whole request alone and compares the delivered blob

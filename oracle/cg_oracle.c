@@ -1,7 +1,7 @@
 /*
  * CPU restatement of the CacheGen KV-cache codec hot path.
  *
- * TEST INFRASTRUCTURE ONLY: this file is the checker the CUDA product is
+ * TEST INFRASTRUCTURE ONLY: this file is the oracle the CUDA product is
  * compared against (and the host-CPU baseline that is timed beside it).  No
  * product code path may call into it.
  *
