@@ -524,9 +524,8 @@ class CacheGenDeserializer(Deserializer):
         self.key_bins = self.make_key_bins(self.cachegen_config)
         self.value_bins = self.make_value_bins(self.cachegen_config)
         self._bins = torch.cat((self.key_bins, self.value_bins)).contiguous()
-        # their values: from the configuration, unless a subclass makes the tensors its own way
-        cls, own = type(self), CacheGenDeserializer
-        if cls.make_key_bins is own.make_key_bins and cls.make_value_bins is own.make_value_bins:
+        # their values: from the configuration, unless somebody else's methods made the tensors
+        if (type(self).make_key_bins, type(self).make_value_bins) == _BINS_MAKERS:
             self._host_bins = _HostBins(torch.cat((CGBasics.make_key_bins(self.cachegen_config, "cpu"),
                                                    CGBasics.make_value_bins(self.cachegen_config, "cpu"))))
         else:
@@ -696,3 +695,6 @@ class CacheGenDeserializer(Deserializer):
             return self.decode(flat_format.from_bytes(bs, device=torch.device("cuda", torch.cuda.current_device())))
         # tensors pickled on a GPU come back on that GPU; anything else is staged by the decode plan
         return self.decode(CacheGenGPUEncoderOutput.from_bytes(bs))
+
+
+_BINS_MAKERS = (CacheGenDeserializer.make_key_bins, CacheGenDeserializer.make_value_bins)

@@ -566,9 +566,8 @@ class CacheGenSerializer(Serializer):
         self.fmt = metadata.fmt
         self._key_bins = self.make_key_bins(self.cachegen_config)
         self._value_bins = self.make_value_bins(self.cachegen_config)
-        # the values are known from the configuration, unless a subclass makes the tensors its own way
-        cls, own = type(self), CacheGenSerializer
-        self._bins_shared = cls.make_key_bins is not own.make_key_bins or cls.make_value_bins is not own.make_value_bins
+        # the values are known from the configuration, unless somebody else's methods made the tensors
+        self._bins_shared = (type(self).make_key_bins, type(self).make_value_bins) != _BINS_MAKERS
         self._info = (_BinsInfo(self._key_bins, self._value_bins) if self._bins_shared else
                       self._config_info(self.cachegen_config))
         self._levels = {}  # settings -> _BinsInfo
@@ -665,3 +664,6 @@ class CacheGenSerializer(Serializer):
         if self.wire_format == "flat":
             return self.encode_flat(tensor).tobytes()
         return self.encode(tensor).to_bytes()
+
+
+_BINS_MAKERS = (CacheGenSerializer.make_key_bins, CacheGenSerializer.make_value_bins)

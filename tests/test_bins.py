@@ -134,6 +134,20 @@ def test_bins_of_a_subclass():
 
 
 @pytest.mark.gpu
+def test_bins_of_replaced_methods(monkeypatch):
+    from cachegen_b200.serde import CacheGenDeserializer, CacheGenSerializer, cachegen_basics as B
+    base, half = configs()
+    kv = make_kv()
+    flat = serializer(half).encode_flat(kv)
+    want = deserializer(half).decode(flat)
+    for cls in (CacheGenSerializer, CacheGenDeserializer):
+        monkeypatch.setattr(cls, "make_key_bins", lambda self, config: B.make_key_bins(half))
+        monkeypatch.setattr(cls, "make_value_bins", lambda self, config: B.make_value_bins(half))
+    assert torch.equal(serializer(base).encode_flat(kv).blob, flat.blob)
+    assert torch.equal(deserializer(base).decode(flat), want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("compact", [True, "counts", False])
 def test_one_workspace_for_decodes_with_different_bins(compact):
     from cachegen_b200.serde import cachegen_basics as B, cachegen_decoder as D, cachegen_encoder as E
