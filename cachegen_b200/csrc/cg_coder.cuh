@@ -89,6 +89,16 @@ CG_HD uint32_t cg_load_stream_word(const uint32_t *p) {
 #endif
 }
 
+// x += N if v <= w, as a compare and a predicated add (see renorm_shift)
+template <uint32_t N>
+CG_HD void add_if_le(uint32_t &x, uint32_t v, uint32_t w) {
+#if defined(__CUDA_ARCH__)
+    asm("{ .reg .pred p; setp.le.u32 p, %1, %2; @p add.u32 %0, %0, %3; }" : "+r"(x) : "r"(v), "r"(w), "n"(N));
+#else
+    if (v <= w) x += N;
+#endif
+}
+
 // ---- shared-memory access --------------------------------------------------------------------------------
 // A stream's table is the column tab[m][tid] = cdf[m] << 16 of a [rows][128] uint32 array, addressed
 // by byte address: entry m of the column starting at `col` is at col + m * kTableRowBytes.  On the
@@ -118,32 +128,42 @@ struct Smem {
 // starts at a multiple of half its size (the midpoint windows of the second kind included).  With
 // d = high - low and b the position of d's top bit, that is 32-s = b+1 when [low, high] touches only two
 // cells of 2^b values and b+2 when it touches three, and it touches three exactly when the low b bits
-// of low and of d carry into bit b.  So 32-s = b + 1 + carry: one leading-bit search, two shifts that move
-// the b low bits to the top of a word, an add for its carry and an add that takes it.  Only the bits of
-// low below b matter, so low may carry anything in its top bit after the shift.
+// of low and of d carry into bit b: when bit b, which d has set, is the same in low and in low + d.  So
+// s is the number of leading zeros of d, less one when that bit of low ^ high is clear: one leading-bit
+// search, one shift for the bit's mask and one three-input test.  Only the bits of low up to b matter, so low
+// may carry anything in its top bit after the shift.  (The carry found by adding the low b bits of both at
+// the top of a word instead, two multiplies and two adds with carry: one instruction more and four more
+// cycles of the multiply pipe a symbol.)
 //
-// Against a search and a shift for each kind this took the fused decode of 8,192 Llama-7B tokens from 4.51 to
-// 4.41 ms, and the encoder, whose pending-bit count went with it, from 160 to 129 us a 256-token chunk.
+// By the size u = d + 1 instead of d (the encoder's loop): the top bit is another one only where u is a power of two, and
+// s one or two less than it could be where low is a multiple of u or of u / 2 as well.  Nothing is lost by that: the next
+// symbol's bounds are exact at any scale of such a range, and its shift makes up for it; and the full range of 2^32, which
+// no word holds, does not come about.  (Only u = 2^31 at a multiple of 2^31 gives -1: see EncoderState::steps_at.)
 //
-// Returns n = 32 - s for the funnel shifts that take other words' bits in, and 2^s for the words that are
-// only shifted left, where a multiply does it off the integer pipe (the pipe that binds the coders: a
-// shift, a compare or a select takes it for two cycles a warp, and so does a multiply-high).
+// Returns s and 2^s: for the words that are only shifted left a multiply does it off the integer pipe (a
+// shift, a compare or a select takes that pipe for two cycles a warp, and a multiply-high the multiply pipe for four).
+//
+// The conditional decrement is written as a predicated add: from `if (...) --s` the compiler makes a
+// decrement, a move and a select (two instructions a symbol more, measured as executed instructions).
 struct Renorm {
-    uint32_t n, p2;
+    uint32_t s, p2;
 };
-CG_HD Renorm renorm_shift(uint32_t low, uint32_t d) {
+// low, high = low + d, d (or u)
+CG_HD Renorm renorm_shift(uint32_t low, uint32_t high, uint32_t d) {
     Renorm r;
 #if defined(__CUDA_ARCH__)
-    uint32_t b;
-    asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(d));
-    const uint32_t q = __funnelshift_r(0u, 1u, b);  // 2^(32-b)
-    asm("{ .reg .u32 t; add.cc.u32 t, %1, %2; addc.u32 %0, %3, 1; }" : "=r"(r.n) : "r"(low * q), "r"(d * q), "r"(b));
-    r.p2 = __funnelshift_rc(0u, 1u, r.n);
+    asm("{ .reg .u32 t, b; .reg .pred p;\n"
+        "bfind.shiftamt.u32 %0, %4;\n"
+        "shf.r.wrap.b32 b, 0x80000000, 0, %0;\n"
+        "lop3.b32 t, %2, %3, b, 0x28;\n"  // (low ^ high) & b
+        "setp.eq.u32 p, t, 0;\n"
+        "@p add.u32 %0, %0, -1;\n"
+        "shf.l.wrap.b32 %1, 0, 1, %0; }"
+        : "=&r"(r.s), "=r"(r.p2) : "r"(low), "r"(high), "r"(d));
 #else
-    const uint32_t b = 31u - static_cast<uint32_t>(cg_clz(d));
-    const uint32_t q = (b & 31u) ? 1u << (32u - (b & 31u)) : 0u;
-    r.n = b + 1u + (low * q + d * q < d * q ? 1u : 0u);
-    r.p2 = cg_fshr_clamp(0u, 1u, r.n);
+    r.s = d ? static_cast<uint32_t>(cg_clz(d)) : 0xFFFFFFFFu;
+    if (((low ^ high) & (0x80000000u >> (r.s & 31u))) == 0u) --r.s;
+    r.p2 = 1u << (r.s & 31u);
 #endif
     return r;
 }
@@ -153,8 +173,8 @@ CG_HD Renorm renorm_shift(uint32_t low, uint32_t d) {
 // 32-bit words; bits before the stream's first byte are shifted out at start-up and words (or word
 // tails) past its last byte read as zero, which is what the reference sees in its zero-padded staging
 // row (dec_new.cu:229-232).  A refill is taken by the whole warp as soon as any of its lanes has fewer
-// bits than a symbol can take and tops every lane up past 64 bits, so the refill code runs once per warp every few
-// symbols instead of once per lane.
+// bits than a symbol can take and gives a word to every lane with room for one, so the refill code runs once per warp every
+// few symbols instead of once per lane.
 CG_HD bool cg_any_lane(uint32_t lanes, bool pred) {
 #if defined(__CUDA_ARCH__)
     return __any_sync(lanes, pred) != 0;
@@ -169,6 +189,27 @@ CG_HD uint32_t cg_umulhi(uint32_t a, uint32_t b) {
     return __umulhi(a, b);
 #else
     return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
+#endif
+}
+// The same as the upper half of a wide product.  A sum with a multiply-high becomes one instruction whose addend has to be
+// moved into a register pair first; the encoder's step takes two instructions fewer with this.
+CG_HD uint32_t cg_umulhi_wide(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    uint64_t p;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(p) : "r"(a), "r"(b));
+    return static_cast<uint32_t>(p >> 32);
+#else
+    return cg_umulhi(a, b);
+#endif
+}
+// a + b - 1 as one instruction
+CG_HD uint32_t cg_add_less_one(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    uint32_t d;
+    asm("{ .reg .u32 t; add.u32 t, %1, %2; add.u32 %0, t, -1; }" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+#else
+    return a + b - 1u;
 #endif
 }
 
@@ -203,41 +244,54 @@ struct BitWindow {
     }
     // drops the bits just shifted into the coder's value
     CG_HD void consume(Renorm r) {
-        hi = cg_fshr_clamp(mid, hi, r.n);
-        mid = cg_fshr_clamp(lo, mid, r.n);
+        hi = cg_fshl(mid, hi, r.s);
+        mid = cg_fshl(lo, mid, r.s);
         lo *= r.p2;
-        nbits += static_cast<int>(r.n) - 32;
+        nbits -= static_cast<int>(r.s);
     }
     CG_HD bool low_water() const { return nbits <= 32; }
     // fewer valid bits than one symbol can take: a range update shifts by at most 18 bits when the
     // table is strictly increasing (the updated interval spans at least 2^14 values)
     static constexpr int kShort = 18;
     CG_HD bool short_of_bits() const { return nbits < kShort; }
-    // Tops the window up with the whole words that fit (none above 64 valid bits, one above 32, two
-    // otherwise), straight-line: every lane of the warp runs the same instructions whatever it needs.
+    // Takes the next word where one fits above 32 bits of room (a stream short of bits has 32 or more afterwards),
+    // straight-line: every lane of the warp runs the same instructions whatever it needs.
+    // Written in predicated instructions (see renorm_shift): filling up to two words a pass with selects took
+    // 4.7 instructions a symbol of the fused decode at 0.055 passes a token; one word, 0.09 passes, takes 1.6.
     CG_HD void refill() {
-        const uint32_t p = static_cast<uint32_t>(nbits < 0 ? 0 : nbits);  // nothing valid below position p
-        const uint32_t k = p <= 32u ? 2u : (p <= 64u ? 1u : 0u);
-        uint32_t wa = fetch(next), wb = fetch(next + 1u);
-        if (k < 2u) wb = 0u;
-        if (k < 1u) wa = 0u;
-        // (wa:wb) goes to bit position p of hi:mid:lo, whose bits from p on are zero
-        const uint32_t q = p & 31u;
-        const uint32_t t0 = cg_fshr_clamp(wa, 0u, q);        // wa >> q
-        const uint32_t t1 = cg_fshr_clamp(wb, wa, q);        // low word of (wa:wb) >> q
-        const uint32_t t2 = cg_fshl_clamp(0u, wb, 32u - q);  // wb << (32 - q), 0 for q == 0
-        if (p < 32u) {
-            hi |= t0;
-            mid |= t1;
-            lo |= t2;
-        } else if (p < 64u) {  // one word fits past position 32, or two exactly at it (q == 0: t1 == wb)
-            mid |= t0;
-            lo |= t1;
-        } else {  // a word fits only at position 64 exactly (wa is 0 beyond it)
-            lo |= t0;
+#if defined(__CUDA_ARCH__)
+        asm("{ .reg .u32 w, rem, t, b; .reg .s32 r; .reg .u64 at; .reg .pred p, q, a;\n"
+            "setp.lt.s32 p, %3, 64;\n"
+            "mad.lo.u32 rem, %4, -32, %6;\n"     // bits of the stream from this word on, negative past its end
+            "mad.wide.u32 at, %4, 4, %5;\n"
+            "mov.u32 w, 0;\n"
+            "setp.gt.and.s32 q, rem, 0, p;\n"
+            "@q ld.global.nc.u32 w, [at];\n"
+            "prmt.b32 w, w, 0, 0x0123;\n"
+            "shr.u32 t, 0xFFFFFFFF, rem;\n"      // (a shift by more than 31 gives 0)
+            "lop3.b32 w, w, t, 0, 0x30;\n"       // w & ~t
+            "shf.r.wrap.b32 t, w, 0, %3;\n"      // the word's upper part, behind the valid bits of their last word
+            "shf.r.wrap.b32 b, 0, w, %3;\n"      // and what goes into the word after that
+            "setp.lt.s32 a, %3, 32;\n"
+            "@a or.b32 %0, %0, t;\n"
+            "@a or.b32 %1, %1, b;\n"
+            "@!a or.b32 %1, %1, t;\n"
+            "@!a or.b32 %2, %2, b;\n"
+            "@p add.s32 %3, %3, 32;\n"
+            "@p add.u32 %4, %4, 1; }"
+            : "+r"(hi), "+r"(mid), "+r"(lo), "+r"(nbits), "+r"(next) : "l"(wp), "r"(end_bit));
+#else
+        if (nbits >= 64) return;
+        const uint32_t w = fetch(next++), p = static_cast<uint32_t>(nbits) & 31u, t = w >> p, b = p ? w << (32u - p) : 0u;
+        if (nbits < 32) {
+            hi |= t;
+            mid |= b;
+        } else {
+            mid |= t;
+            lo |= b;
         }
-        nbits = static_cast<int>(p + 32u * k);
-        next += k;
+        nbits += 32;
+#endif
     }
 };
 
@@ -256,15 +310,16 @@ struct DecoderState {
 
     // range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation
     // (dec_new.cu:277-301), both kinds of shift applied in one go.  On a table that is not increasing the
-    // shift count is anything up to 32; every later read stays inside the table column and the stream.
+    // shift count is anything up to 31; every later read stays inside the table column and the stream.
     CG_HD void update(uint32_t flo, uint32_t fhi, BitWindow &bw) {
         offset -= flo;
         low += flo;
         span32 = fhi - flo;
-        const Renorm r = renorm_shift(low, span32 - 1u);
+        const uint32_t d = span32 - 1u;
+        const Renorm r = renorm_shift(low, low + d, d);
         low *= r.p2;
         span32 *= r.p2;
-        offset = cg_fshr_clamp(bw.hi, offset, r.n);
+        offset = cg_fshl(bw.hi, offset, r.s);
         bw.consume(r);
     }
 };
@@ -309,8 +364,8 @@ CG_HD uint32_t ratio_estimate(uint32_t offset, uint32_t span32) {
 template <int B>
 struct RatioSearch {
     static CG_HD uint32_t run(Smem sm, uint32_t a, uint32_t ratio) {
-        const uint32_t ca = a + (static_cast<uint32_t>(kTableRowBytes) << B);
-        a = sm.ld(ca) <= ratio ? ca : a;
+        const uint32_t v = sm.ld(a + (static_cast<uint32_t>(kTableRowBytes) << B));
+        add_if_le<(static_cast<uint32_t>(kTableRowBytes) << B)>(a, v, ratio);
         return RatioSearch<B - 1>::run(sm, a, ratio);
     }
 };
@@ -367,7 +422,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
     uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
 #if defined(__CUDA_ARCH__)
-#pragma unroll 2
+#pragma unroll 1
 #endif
     for (; t4 != last4; t4 += 4u) {
         uint32_t flo[NS], fhi[NS], ratio[NS];
@@ -462,15 +517,16 @@ CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *strea
 
 // ---- MSB-first bit writer into one scratch row (add_bits_to_output, enc_new.cu:21-97) ---------------------
 // Output bits collect in a 64-bit accumulator.  Whole 32-bit words leave it, big-endian, into the
-// stream's scratch row; the common case does that for the whole warp at once (see EncoderState::step)
+// stream's scratch row; the common case does that for the whole warp at once (see EncoderState::steps_at)
 // so that the store is not a per-lane branch.
 //
 // The bits are those of the interval's lower end as one long binary fraction, so a later range update can
-// still carry into bits that are already here.  A carry out of the accumulator's valid bits stays in the bit above
-// them (a word leaves nothing behind it) and goes on to the word before when the next word leaves.  That word is
-// held back in a register until then: the run of ones that lets a carry through reaches the accumulator's end
+// still carry into bits that are already here, and out of them into the word before.  That word is held back in a
+// register until the next one leaves: the run of ones that lets a carry through reaches the accumulator's end
 // for one word in seven (symbols of 2.5 bits), but past the held word about never.  (With carries added to words
-// already stored the per-lane read-modify-write ran on 15 % of the word stores.)
+// already stored the per-lane read-modify-write ran on 15 % of the word stores.)  Bits that have left as a word
+// stay in the accumulator above the pending ones until they are shifted out, and a carry goes on into
+// them; the last bit of the held word is one of them, so it has changed exactly if the word is to be one more.
 // STEP: words between consecutive words of the row (32: the rows of a warp's streams interleaved, so that
 // they take no more cache lines than they have data for and are read back coalesced).  BOUNDED: the row may be
 // too short for the stream; otherwise it holds CG_STREAM_CAPACITY bytes, which a strictly increasing table
@@ -481,8 +537,8 @@ struct BitSinkT {
     uint32_t cap_w;   // words that fit in the row
     uint32_t nwords;  // words produced so far, the held one included (may exceed cap_w: then nothing more is stored)
     uint32_t hold;    // the last of them, not yet in the row
-    uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo), and a carry above them
-    uint32_t nacc;            // number of bits pending, < 63
+    uint32_t acc_hi, acc_lo;  // pending output bits, right-aligned in (acc_hi:acc_lo), older bits above them
+    int nacc;                 // number of bits pending, < 64; -1: see EncoderState::half_scale
 
     // p: where the stream's first word goes; nbytes: room for the stream
     CG_HD void init(uint8_t *p, int64_t nbytes) {
@@ -494,52 +550,70 @@ struct BitSinkT {
         acc_lo = 0;
         nacc = 0;
     }
-    // adds one to the number that the words in the row form
-    CG_HD void carry_into_row() {
-        if (BOUNDED && nwords > cap_w) return;  // the words before are not in the row: reported as an overflow
-        for (uint32_t i = nwords; i > 1u;) {
-            --i;
-            const uint32_t v = cg_bswap32(row[(i - 1u) * STEP]) + 1u;
-            row[(i - 1u) * STEP] = cg_bswap32(v);
+    // adds one to the number that the first n words in the row form
+    CG_HD void carry_into_row(uint32_t n) {
+        if (BOUNDED && n > cap_w) return;  // they are not in the row: reported as an overflow
+        for (; n > 0u; --n) {
+            const uint32_t v = cg_bswap32(row[(n - 1u) * STEP]) + 1u;
+            row[(n - 1u) * STEP] = cg_bswap32(v);
             if (v) return;
         }
     }
-    // adds a carry (0 or 1) to the held word and puts it in the row
-    CG_HD void store_held(uint32_t carry) {
-        hold += carry;
-        if (hold < carry) carry_into_row();
-        if (!BOUNDED || nwords - 1u < cap_w) row[static_cast<int>(nwords - 1u) * STEP] = cg_bswap32(hold);
-    }
-    // Moves the oldest 32 bits out where there are 32; needs nacc < 63.  Straight-line code: every lane of the
-    // warp runs it whatever it needs.
-    CG_HD void store_word_if_full() {
-        const bool full = nacc >= 32u;
-        const uint32_t left = full ? nacc - 32u : nacc;
-        const uint32_t w = cg_fshr_clamp(acc_lo, acc_hi, left);  // the low word of (hi:lo) >> left
-        const uint32_t carry = full ? cg_fshr_clamp(acc_hi, 0u, left) : 0u;
-        const uint32_t held = hold + carry;
-        if (held < carry) carry_into_row();
+    // Moves the oldest 32 pending bits out where there are 32; needs nacc < 64.  Straight-line code: every lane of the
+    // warp runs it whatever it needs.  Returns whether the held word, which went to the row (as number nwords - 2 now), has
+    // carried into those in front of it, which is left to the caller.
+    CG_HD bool store_word_if_full() {
 #if defined(__CUDA_ARCH__)
-        const bool stored = full && (!BOUNDED || nwords - 1u < cap_w);
-        asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.global.u32 [%1], %2; }" ::"r"(static_cast<uint32_t>(stored)),
-                     "l"(row + static_cast<int>(nwords - 1u) * STEP), "r"(cg_bswap32(held)) : "memory");
+        uint32_t w, held, carry, left;
+        asm("{ .reg .pred p;\n"
+            "add.u32 %3, %6, -32;\n"
+            "setp.ge.s32 p, %6, 32;\n"
+            "shf.r.clamp.b32 %0, %4, %5, %3;\n"  // the low word of (hi:lo) >> left
+            "shf.r.clamp.b32 %2, %5, 0, %3;\n"
+            "lop3.b32 %2, %2, %7, 1, 0x28;\n"    // (acc_hi >> left ^ hold) & 1
+            "@!p mov.u32 %2, 0;\n"
+            "add.u32 %1, %7, %2; }"
+            : "=&r"(w), "=r"(held), "=&r"(carry), "=&r"(left) : "r"(acc_lo), "r"(acc_hi), "r"(nacc), "r"(hold));
+        const bool room = !BOUNDED || nwords - 1u < cap_w;
+        asm volatile("{ .reg .pred p, q;\n"
+            "setp.ge.s32 p, %2, 32;\n"
+            "setp.ne.and.u32 q, %7, 0, p;\n"
+            "@q st.global.u32 [%3], %4;\n"
+            "@p add.u32 %0, %0, 1;\n"
+            "@p mov.u32 %1, %5;\n"
+            "@p mov.u32 %2, %6; }"
+            : "+r"(nwords), "+r"(hold), "+r"(nacc)
+            : "l"(row + static_cast<int>(nwords - 1u) * STEP), "r"(cg_bswap32(held)), "r"(w), "r"(left), "r"(static_cast<uint32_t>(room)) : "memory");
+        return held < carry;
 #else
-        if (full && nwords && (!BOUNDED || nwords - 1u < cap_w)) row[(nwords - 1u) * STEP] = cg_bswap32(held);
+        if (nacc < 32) return false;
+        nacc -= 32;
+        const uint32_t carry = ((acc_hi >> nacc) ^ hold) & 1u;
+        hold += carry;
+        const bool over = hold < carry;
+        if (nwords && (!BOUNDED || nwords - 1u < cap_w)) row[(nwords - 1u) * STEP] = cg_bswap32(hold);
+        ++nwords;
+        hold = cg_fshr_clamp(acc_lo, acc_hi, static_cast<uint32_t>(nacc));
+        return over;
 #endif
-        nwords += full ? 1u : 0u;
-        hold = full ? w : hold;
-        acc_hi = full ? 0u : acc_hi;
-        acc_lo = full ? acc_lo & ~cg_shl(0xFFFFFFFFu, left) : acc_lo;
-        nacc = left;
+    }
+    CG_HD void store_and_carry() {
+        if (store_word_if_full()) carry_into_row(nwords - 2u);
     }
     // zero-fills to a byte boundary; returns the stream length in bytes
     CG_HD uint32_t finish() {
-        if (nacc > 62u) nacc = 62u;  // only a table that does not increase gets here
-        store_word_if_full();
-        if (nwords) store_held(cg_fshr_clamp(acc_lo, acc_hi, nacc));
-        const uint32_t bytes = nwords * 4u + ((nacc + 7u) >> 3);
+        if (nacc > 62) nacc = 62;  // only a table that does not increase gets here, or below
+        if (nacc < 0) nacc = 0;
+        store_and_carry();
+        if (nwords) {
+            const uint32_t carry = ((acc_lo >> nacc) ^ hold) & 1u;
+            hold += carry;
+            if (hold < carry) carry_into_row(nwords - 1u);
+            if (!BOUNDED || nwords - 1u < cap_w) row[static_cast<int>(nwords - 1u) * STEP] = cg_bswap32(hold);
+        }
+        const uint32_t bytes = nwords * 4u + ((static_cast<uint32_t>(nacc) + 7u) >> 3);
         if (nacc) {
-            const uint32_t w = acc_lo << (32u - nacc);
+            const uint32_t w = acc_lo << (32 - nacc);
             if (!BOUNDED || nwords < cap_w) row[nwords * STEP] = cg_bswap32(w);
         }
         return bytes;
@@ -549,9 +623,19 @@ struct BitSinkT {
 using BitSink = BitSinkT<1>;
 
 // ---- encoder state and step -----------------------------------------------------------------------------
-// A symbol starts with fewer bits than this in the accumulator; it adds at most 18 (the updated interval of a
-// strictly increasing table spans at least 2^14 values), which leaves room for a carry.
-constexpr uint32_t kSinkHighWater = 44;
+// Pending bits from which on a lane makes its warp store a word.  Whatever stays below it, or below 32 after the store, has
+// to take `symbols` more symbols' bits below bit 63.  A symbol adds at most 18 (the updated interval of a
+// strictly increasing table spans at least 2^14 values).
+constexpr int kSinkHighWater = 44;
+// The same where the table was counted from the `ntokens` symbols that are coded with it: a symbol that occurs has at
+// least w = floor((0xFFFF - 63) / ntokens) + 1 of the 2^16 shares (normalize_cdf_value), hence an interval of
+// w * 2^14 - 1 values or more, and adds at most 18 - floor(log2 w) bits.  0: two symbols may not fit.
+CG_HD int pair_high_water(int ntokens) {
+    const uint32_t w = (0xFFFFu - 63u) / static_cast<uint32_t>(ntokens) + 1u;
+    const int most = 18 - (31 - cg_clz(w));
+    if (31 + 2 * most > 63) return 0;
+    return 64 - 2 * most < kSinkHighWater ? 64 - 2 * most : kSinkHighWater;
+}
 
 // The coder without the reference's count of pending bits.  low is the current 32-bit window of the
 // interval's lower end L, and all bits of L above the window are in the sink: a range update adds to
@@ -564,6 +648,17 @@ struct EncoderState {
     CG_HD void init() {
         low = 0u;
         span32 = 0u;
+    }
+    // The full range of 2^32 does not fit span32.  It is taken at half scale: a window that takes one bit back from the
+    // sink (at a stream's start the integer bit of L, which stays 0).  Bounds are exact there, and the next
+    // renormalisation shifts by one more.  What uses steps_at starts so.
+    template <class Sink>
+    CG_HD void half_scale(Sink &out) {
+        low = cg_fshl(low, out.acc_lo, 31u);
+        out.acc_lo = cg_fshl(out.acc_lo, out.acc_hi, 31u);
+        out.acc_hi >>= 1;
+        span32 = 0x80000000u;
+        --out.nacc;
     }
     template <class Sink>
     CG_HD void add_to_low(uint32_t v, Sink &out) {
@@ -579,75 +674,83 @@ struct EncoderState {
         if (low < v && ++out.acc_lo == 0u) ++out.acc_hi;
 #endif
     }
-    // One symbol s of one stream per lane (enc_new.cu:257-295), s <= maxsym.  lanes: the warp's lanes that
-    // encode together (same token count).
-    template <class Sink>
-    CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, Sink &out, uint32_t lanes) {
-        step_at<kTableRowBytes>(sm, col + s * kTableRowBytes, s == maxsym, out, lanes);
-    }
-    // The same by the address a of the symbol's table entry, the next one ROW bytes further.  ONE warp vote a
-    // symbol covers what is rare: a full word in the accumulator (every lane that has one stores it as soon as
-    // one lane is near the high-water mark), the full 2^32 range (a stream's first symbol; later only if a shift
-    // lands on it exactly) and the table's last symbol, whose upper bound is the range's end.
-    template <int ROW, class Sink>
-    CG_HD void step_at(Smem sm, uint32_t a, bool last, Sink &out, uint32_t lanes) {
-        const uint32_t e0 = sm.ld(a), e1 = sm.ld(a + ROW);
-        uint32_t flo = cg_umulhi(span32, e0), fhi = cg_umulhi(span32, e1);
-        if (cg_any_lane(lanes, (out.nacc >= kSinkHighWater) | (span32 == 0u) | last)) {
-            out.store_word_if_full();
-            flo = span32 ? flo : e0;
-            fhi = span32 ? fhi : e1;
-            if (last) fhi = span32;
-        }
-        take(flo, fhi, out);
-    }
-    // range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation
-    template <class Sink>
+    // Range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation, by the interval's size (see
+    // renorm_shift) or, EXACT, by its size less one.
+    template <bool EXACT, class Sink>
     CG_HD void take(uint32_t flo, uint32_t fhi, Sink &out) {
+        const uint32_t u = fhi - flo;
         add_to_low(flo, out);
-        span32 = fhi - flo;
-        const Renorm r = renorm_shift(low, span32 - 1u);
-        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, r.n);
-        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, r.n);
-        low *= r.p2;
-        span32 *= r.p2;
-        out.nacc += 32u - r.n;
+        shift(renorm_shift(low, cg_add_less_one(low, u), EXACT ? u - 1u : u), u, out);
     }
-    // step_at for NS streams a lane, none of whose symbols is the table's last: their chains are independent, and
-    // the vote is paid once.
-    template <int ROW, int NS, class Sink>
-    static CG_HD void steps_at(Smem sm, const uint32_t (&a)[NS], EncoderState (&enc)[NS], Sink (&out)[NS], uint32_t lanes) {
-        uint32_t e0[NS], e1[NS], flo[NS], fhi[NS];
-        bool rare = false;
+    template <class Sink>
+    CG_HD void shift(Renorm r, uint32_t u, Sink &out) {
+        out.acc_hi = cg_fshl(out.acc_lo, out.acc_hi, r.s);
+        out.acc_lo = cg_fshl(low, out.acc_lo, r.s);
+        low *= r.p2;
+        span32 = u * r.p2;
+        out.nacc += static_cast<int>(r.s);
+    }
+    // One symbol by the address a of its table entry, the next one ROW bytes further (enc_new.cu:257-295): whatever the
+    // state, by one lane alone.
+    template <int ROW, class Sink>
+    CG_HD void step_alone(Smem sm, uint32_t a, bool last, Sink &out) {
+        out.store_and_carry();
+        if (span32 == 0u) half_scale(out);
+        const uint32_t flo = cg_umulhi_wide(span32, sm.ld(a));
+        take<true>(flo, last ? span32 : cg_umulhi_wide(span32, sm.ld(a + ROW)), out);
+    }
+    // symbol s <= maxsym of one stream
+    template <class Sink>
+    CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, Sink &out, uint32_t) {
+        step_alone<kTableRowBytes>(sm, col + s * kTableRowBytes, s == maxsym, out);
+    }
+    // G symbols (1 or 2) of NS streams a lane, by the addresses of their table entries.  The streams' chains are independent,
+    // and ONE warp vote after them covers a full word in an accumulator: every lane that has one stores it as soon as one
+    // lane is at the high-water mark (kSinkHighWater for one symbol, pair_high_water for two).
+    // LAST: a symbol may be its table's last, whose upper bound is the range's end (told by `last`; G is 1 then).
+    // What hardly ever happens is not mended here but left to encode_again: a carry through a whole word of ones
+    // (`carried`), and a range of 2^31 at a multiple of it, which leaves a span of 0, from where on no symbol has a size, so
+    // that the span is still 0 at the stream's end.  Code for the like inside the loop cost five instructions a symbol in
+    // moves between registers without ever being run.
+    template <int ROW, int G, int NS, bool LAST = false, class Sink>
+    static CG_HD void steps_at(Smem sm, const uint32_t (&a)[G][NS], EncoderState (&enc)[NS], Sink (&out)[NS], int high_water,
+                               uint32_t lanes, bool (&carried)[NS], bool last = false) {
+        uint32_t e0[G][NS], e1[G][NS];
 #pragma unroll
-        for (int i = 0; i < NS; ++i) {
-            e0[i] = sm.ld(a[i]);
-            e1[i] = sm.ld(a[i] + ROW);
-            flo[i] = cg_umulhi(enc[i].span32, e0[i]);
-            fhi[i] = cg_umulhi(enc[i].span32, e1[i]);
-            rare |= (out[i].nacc >= kSinkHighWater) | (enc[i].span32 == 0u);
-        }
-        if (cg_any_lane(lanes, rare)) {
+        for (int g = 0; g < G; ++g)
 #pragma unroll
             for (int i = 0; i < NS; ++i) {
-                out[i].store_word_if_full();
-                flo[i] = enc[i].span32 ? flo[i] : e0[i];
-                fhi[i] = enc[i].span32 ? fhi[i] : e1[i];
+                e0[g][i] = sm.ld(a[g][i]);
+                e1[g][i] = sm.ld(a[g][i] + ROW);
             }
-        }
 #pragma unroll
-        for (int i = 0; i < NS; ++i) enc[i].take(flo[i], fhi[i], out[i]);
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int i = 0; i < NS; ++i) {
+                const uint32_t fhi = cg_umulhi_wide(enc[i].span32, e1[g][i]);
+                enc[i].template take<false>(cg_umulhi_wide(enc[i].span32, e0[g][i]), LAST && last ? enc[i].span32 : fhi, out[i]);
+            }
+        bool full = false;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) full |= out[i].nacc >= high_water;
+        if (cg_any_lane(lanes, full)) {
+#pragma unroll
+            for (int i = 0; i < NS; ++i) carried[i] |= out[i].store_word_if_full();
+        }
     }
+    // whether a stream has met what steps_at leaves
+    CG_HD bool unsettled(bool carried) const { return carried | (span32 == 0u); }
     // final flush (enc_new.cu:298-306): two bits that place the stream's value inside the interval, 01 or
     // 10 above the reference's low with its pending bits, which is L plus a quarter of the window cut
     // to two bits; returns the stream length in bytes
     template <class Sink>
     CG_HD uint32_t flush(Sink &out) {
+        if (span32) shift(renorm_shift(low, cg_add_less_one(low, span32), span32 - 1u), span32, out);  // see take
+        if (out.nacc < 64) out.store_and_carry();
         add_to_low(0x40000000u, out);
-        if (out.nacc < 63u) out.store_word_if_full();
-        out.acc_hi = cg_fshr_clamp(out.acc_lo, out.acc_hi, 30u);
-        out.acc_lo = cg_fshr_clamp(low, out.acc_lo, 30u);
-        out.nacc += 2u;
+        out.acc_hi = cg_fshl(out.acc_lo, out.acc_hi, 2u);
+        out.acc_lo = cg_fshl(low, out.acc_lo, 2u);
+        out.nacc += 2;
         return out.finish();
     }
 };

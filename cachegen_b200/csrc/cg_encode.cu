@@ -21,10 +21,26 @@ struct EncodeParams {
 
 constexpr int kPrefetch = 8;  // symbols fetched ahead of the coder
 
-// Bound by instruction issue: one 256-token Llama-7B chunk in 118 us, 160 before the step without pending bits.
+// See store_encode_kernel's encode_again.
+template <class Offset>
+static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint8_t *base, Offset at, Offset s1, int n, uint32_t top, uint8_t *to, int64_t stride) {
+    BitSink out;
+    EncoderState enc;
+    out.init(to, stride);
+    enc.init();
+    for (int i = 0; i < n; ++i) {
+        const uint32_t s = min(static_cast<uint32_t>(__ldg(base + at)), top);
+        at += s1;
+        enc.step_alone<kRowBytes>(Smem{}, col + s * kRowBytes, s == top, out);
+    }
+    return enc.flush(out);
+}
+
+// Bound by instruction issue: one 256-token Llama-7B chunk in 116 us under counters, 125 before the loop without rare cases and
+// with symbols fetched a group ahead of the coder (three of eight stall cycles were loads).
 // NARROW: the symbols of a row lie within 4 GB of its first, so that a symbol's address is a 32-bit offset
 template <bool NARROW>
-__global__ void __launch_bounds__(kGroup, 10) encode_kernel(const EncodeParams p) {
+__global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p) {
     extern __shared__ uint32_t tab[];
     const int tid = threadIdx.x;
     const int row = blockIdx.y, sub = blockIdx.z;
@@ -41,41 +57,53 @@ __global__ void __launch_bounds__(kGroup, 10) encode_kernel(const EncodeParams p
     stage_table_column(tab, p.cdf + g * p.lp, p.lp, p.lp, tid);
     const uint32_t col = smem_addr(tab + tid);
     const int64_t slot = static_cast<int64_t>(sub) * nrows * p.nchannels + g;
-    BitSink out;
-    out.init(p.scratch + slot * p.stride, p.stride);
+    BitSink out[1];
+    out[0].init(p.scratch + slot * p.stride, p.stride);
 
     using Offset = typename std::conditional<NARROW, uint32_t, int64_t>::type;
     const uint8_t *base = reinterpret_cast<const uint8_t *>(p.sym) + row * p.s0 + static_cast<int64_t>(t0) * p.s1;
     const Offset s1 = static_cast<Offset>(p.s1);
     Offset at = static_cast<Offset>(c * p.s2);
-    EncoderState enc;
-    enc.init();
+    EncoderState enc[1];
+    bool carried[1] = {};
+    enc[0].init();
+    enc[0].half_scale(out[0]);
     uint32_t largest = 0;  // the largest symbol met: one above maxsym is reported and coded as maxsym
 
-    // whole groups of kPrefetch symbols: their loads are issued together, ahead of the coder, with no
-    // bound checks; the last, shorter group goes symbol by symbol
+    // whole groups of kPrefetch symbols: their loads are issued together, one group ahead of the coder; the last, shorter
+    // group goes symbol by symbol
     const uint32_t top = static_cast<uint32_t>(maxsym);
+    const auto code = [&](uint32_t sym) {
+        largest = max(largest, sym);
+        const uint32_t s = min(sym, top), a[1][1] = {{col + s * kRowBytes}};
+        EncoderState::steps_at<kRowBytes, 1, 1, true>(Smem{}, a, enc, out, kSinkHighWater, lanes, carried, s == top);
+    };
+    const Offset first = at;
+    uint32_t buf[kPrefetch], next[kPrefetch];
     int i = 0;
+#pragma unroll
+    for (int j = 0; j < kPrefetch; ++j) {
+        buf[j] = j < n ? __ldg(base + at) : 0u;
+        at += s1;
+    }
     for (; i + kPrefetch <= n; i += kPrefetch) {
-        uint32_t buf[kPrefetch];
 #pragma unroll
         for (int j = 0; j < kPrefetch; ++j) {
-            buf[j] = __ldg(base + at);
+            next[j] = i + kPrefetch + j < n ? __ldg(base + at) : 0u;
             at += s1;
         }
 #pragma unroll
-        for (int j = 0; j < kPrefetch; ++j) {
-            largest = max(largest, buf[j]);
-            enc.step(Smem{}, col, min(buf[j], top), top, out, lanes);
-        }
+        for (int j = 0; j < kPrefetch; ++j) code(buf[j]);
+#pragma unroll
+        for (int j = 0; j < kPrefetch; ++j) buf[j] = next[j];
     }
     for (; i < n; ++i) {
-        const uint32_t s = __ldg(base + at);
-        at += s1;
-        largest = max(largest, s);
-        enc.step(Smem{}, col, min(s, top), top, out, lanes);
+        code(buf[0]);
+#pragma unroll
+        for (int j = 0; j + 1 < kPrefetch; ++j) buf[j] = buf[j + 1];
     }
-    const uint32_t nbytes = enc.flush(out);
+    const uint32_t nbytes = enc[0].unsettled(carried[0]) ? encode_again<Offset>(col, base, first, s1, n, top, p.scratch + slot * p.stride, p.stride)
+                                                         : enc[0].flush(out[0]);
     p.lengths[slot] = static_cast<int32_t>(nbytes);
     if (p.status) {
         int bits = 0;

@@ -306,6 +306,7 @@ struct StoreParams {
     const uint32_t *sym4;
     TableOut out;
     int ntokens, nchannels, lp, nrows, nsub;
+    int high_water;       // see pair_high_water
     uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4 + 1, 32 lanes] words
     int64_t stride;
     int32_t *lengths;     // [nsub, nrows * C]
@@ -363,19 +364,41 @@ __device__ __forceinline__ int64_t block_scan_in_place(T *v, int n, int64_t *war
     return base;
 }
 
+// A stream that has met what the coder's loop leaves (see EncoderState::steps_at) from its start again, by one lane:
+// the stream's words of symbols at sp, C words apart.  Returns its length in bytes.  About never run.
+template <class Sink>
+static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint32_t *sp, int64_t C, int n, uint8_t *to, int64_t stride) {
+    Sink out;
+    EncoderState enc;
+    out.init(to, stride);
+    enc.init();
+    uint32_t w = 0u;
+    for (int i = 0; i < n; ++i) {
+        if ((i & 3) == 0) {
+            w = __ldg(sp + (i >> 2) * C);
+            if (w & 0x80808080u) w = 0u;
+        }
+        enc.step_alone<kWarpRow>(Smem{}, entry_of(col, w, 0), false, out);
+        w >>= 8;
+    }
+    return enc.flush(out);
+}
+
 // NS streams per thread, 128 adjacent channels of one row and sub-chunk per block.  TABLES: the chunk is one
 // sub-chunk, so the block's symbols are all there are for its tables: it counts them (each thread in its
 // own shared-memory columns, where its tables then stand), writes the tables out and codes; the symbols'
 // second read comes from the L2.  Otherwise the tables come from packed_tables_kernel.
 // The last block of a sub-chunk turns the group sizes into offsets, the last of all writes the tail.
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
-// chunk takes 118 us with its tables, 0.57 T symbols/s, where the coder alone took 160 us at first and 129 without
-// the pending-bit count, the tables being a part of the quantise pass.  Eight blocks an SM leave the compiler 64
+// chunk takes 112 us with its tables under counters, 0.60 T symbols/s, 37.2 instructions for 32 symbols; 122 us and 40.4 with
+// the code for rare cases inside the loop and a vote a symbol.  Eight blocks an SM leave the compiler 64
 // registers; the shared memory asked for on top evens the last wave out (even_waves_smem).
 // Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
-// channels in 165 us, 180 with one.  The tables' part wants the warps more than the chains (a 256-token chunk
+// channels in 166 us under counters (29.9 instructions for 32 symbols), 172 before the same change; 180 with one stream.
+// G symbols a vote: two, unless the table may give a symbol more bits than the accumulator has room for twice (pair_high_water:
+// more than 21,824 tokens in one call).  The tables' part wants the warps more than the chains (a 256-token chunk
 // 129 us with two), so it keeps one; and so does a last group of channels that would leave the second without work.
-template <bool TABLES, int NS>
+template <bool TABLES, int NS, int G>
 __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_kernel(const __grid_constant__ StoreParams p) {
     constexpr int kThreads = kGroup / NS, kWarps = kThreads / 32;
     constexpr int kWordsAhead = NS == 1 ? 4 : 2;  // words (of four symbols) fetched one group ahead of the coder
@@ -429,7 +452,8 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
             for (int k = 0; k < kAhead; ++k) any |= w[k];
             if (any & 0x80808080u) {  // reported below
 #pragma unroll
-                for (int k = 0; k < kAhead; ++k) w[k] = 0u;
+                for (int k = 0; k < kAhead; ++k)
+                    if (w[k] & 0x80808080u) w[k] = 0u;
             }
 #pragma unroll
             for (int k = 0; k < kAhead; ++k) {
@@ -459,21 +483,24 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     }
 
     if (any_active) {
-        const uint32_t top = static_cast<uint32_t>(p.lp - 2);
-        BitSinkT<32, false> out[NS];  // see scratch_word
+        using Sink = BitSinkT<32, false>;  // see scratch_word
+        Sink out[NS];
         EncoderState enc[NS];
+        bool carried[NS] = {};
+        const int64_t group = (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x;
         uint32_t w[NS][kWordsAhead], next[NS][kWordsAhead];
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            out[s].init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, (static_cast<int64_t>(sub) * p.nrows + row) * nslab + blockIdx.x, s * kThreads + tid)),
-                        p.stride);
+            out[s].init(reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, group, s * kThreads + tid)), p.stride);
             enc[s].init();
+            enc[s].half_scale(out[s]);
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) w[s][k] = 4 * k < n ? __ldg(sp[s] + k * C) : 0u;
         }
+        const int high_water = G == 1 ? kSinkHighWater : p.high_water;
         constexpr int kAhead = 4 * kWordsAhead;
         int i = 0;
-        for (; i + kAhead <= n; i += kAhead) {
+        for (;; i += kAhead) {
             uint32_t any = 0u;
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
@@ -487,43 +514,50 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
             if (any & 0x80808080u) {
                 bad = 1u;
 #pragma unroll
-                for (int k = 0; k < kWordsAhead * NS; ++k) w[k / kWordsAhead][k % kWordsAhead] = 0u;
+                for (int k = 0; k < kWordsAhead * NS; ++k) {
+                    uint32_t &v = w[k / kWordsAhead][k % kWordsAhead];
+                    if (v & 0x80808080u) v = 0u;  // as the tables count it
+                }
             }
+            if (i + kAhead > n) break;
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t a[NS];
+                for (int j = 0; j < 4; j += G) {
+                    uint32_t a[G][NS];
 #pragma unroll
-                    for (int s = 0; s < NS; ++s) a[s] = entry_of(col[s], w[s][k], j);
-                    EncoderState::steps_at<kWarpRow>(Smem{}, a, enc, out, 0xFFFFFFFFu);
+                    for (int g = 0; g < G; ++g)
+#pragma unroll
+                        for (int s = 0; s < NS; ++s) a[g][s] = entry_of(col[s], w[s][k], j + g);
+                    EncoderState::steps_at<kWarpRow, G>(Smem{}, a, enc, out, high_water, 0xFFFFFFFFu, carried);
                 }
             }
 #pragma unroll
             for (int k = 0; k < kWordsAhead * NS; ++k) w[k / kWordsAhead][k % kWordsAhead] = next[k / kWordsAhead][k % kWordsAhead];
         }
         for (; i < n; ++i) {  // fewer than kAhead left, all in w
-            uint32_t a[NS];
+            uint32_t a[1][NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                uint32_t m = w[s][0] & 0xFFu;
-                if (m >= top) {
-                    bad = 1u;
-                    m = 0u;
-                }
-                a[s] = col[s] + m * kWarpRow;
+                a[0][s] = entry_of(col[s], w[s][0], 0);
                 w[s][0] >>= 8;
                 if ((i & 3) == 3) {
 #pragma unroll
                     for (int k = 0; k + 1 < kWordsAhead; ++k) w[s][k] = w[s][k + 1];
                 }
             }
-            EncoderState::steps_at<kWarpRow>(Smem{}, a, enc, out, 0xFFFFFFFFu);
+            EncoderState::steps_at<kWarpRow, 1>(Smem{}, a, enc, out, kSinkHighWater, 0xFFFFFFFFu, carried);
         }
         int bits = bad ? CG_S_BAD_SYMBOL : 0;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            int len = static_cast<int>(enc[s].flush(out[s]));
+            int len;
+            if (enc[s].unsettled(carried[s]))
+                len = static_cast<int>(encode_again<Sink>(col[s], p.sym4 + (static_cast<int64_t>(row) * ((p.ntokens + 3) / 4) + t0 / 4) * C +
+                                                                      min(blockIdx.x * kGroup + s * kThreads + tid, p.nchannels - 1),
+                                                          C, n, reinterpret_cast<uint8_t *>(scratch_word(p.scratch, p.stride, group, s * kThreads + tid)), p.stride));
+            else
+                len = static_cast<int>(enc[s].flush(out[s]));
             if (!active[s]) continue;
             p.lengths[static_cast<int64_t>(sub) * p.nrows * C + g[s]] = len;
             if (len > p.stride) {
@@ -811,6 +845,7 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     p.lp = lp;
     p.nrows = z.nrows;
     p.nsub = z.nsub;
+    p.high_water = pair_high_water(b.ntokens);
     p.scratch = ws + z.scratch;
     p.stride = z.stride;
     p.lengths = lengths;
@@ -822,27 +857,22 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     const dim3 grid(z.nslab, z.nrows, z.nsub);
     const int64_t blocks = static_cast<int64_t>(z.nslab) * z.nrows * z.nsub;
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
-    if (z.nsub == 1) {
-        const size_t smem = even_waves_smem(blocks, columns + staged, 128);
-        if (int rc = allow_smem(store_encode_kernel<true, 1>, smem)) return rc;
-        store_encode_kernel<true, 1><<<grid, kGroup, smem, st>>>(p);
+    const auto store = [&](auto kernel, int threads, size_t dynamic) {
+        const size_t smem = even_waves_smem(blocks, dynamic, 128);
+        if (int rc = allow_smem(kernel, smem)) return rc;
+        kernel<<<grid, threads, smem, st>>>(p);
         return check_launch();
-    }
+    };
+    if (z.nsub == 1) return store(store_encode_kernel<true, 1, 2>, kGroup, columns + staged);
     if (int rc = allow_smem(packed_tables_kernel, columns + staged)) return rc;
     packed_tables_kernel<<<dim3(z.nslab, z.nrows), kTableThreads, columns + staged, st>>>(sym4, b.ntokens, z.nchannels, lp,
                                                                                          p.out, status);
     if (int rc = check_launch()) return rc;
-    const size_t smem = even_waves_smem(blocks, columns, 128);
+    if (!p.high_water) return store(store_encode_kernel<false, 1, 1>, kGroup, columns);
     // two streams a thread unless the last group has channels for the first alone
     const int last = z.nchannels % kGroup;
-    if (last == 0 || last > kGroup / 2) {
-        if (int rc = allow_smem(store_encode_kernel<false, 2>, smem)) return rc;
-        store_encode_kernel<false, 2><<<grid, kGroup / 2, smem, st>>>(p);
-    } else {
-        if (int rc = allow_smem(store_encode_kernel<false, 1>, smem)) return rc;
-        store_encode_kernel<false, 1><<<grid, kGroup, smem, st>>>(p);
-    }
-    return check_launch();
+    if (last == 0 || last > kGroup / 2) return store(store_encode_kernel<false, 2, 2>, kGroup / 2, columns);
+    return store(store_encode_kernel<false, 1, 2>, kGroup, columns);
 }
 
 extern "C" int cg_encode_kv_wait(const cg_encode_kv_job *job, void *stream) {
