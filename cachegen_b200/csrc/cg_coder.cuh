@@ -89,18 +89,9 @@ CG_HD uint32_t cg_load_stream_word(const uint32_t *p) {
 #endif
 }
 
-// x += N if v <= w, as a compare and a predicated add (see renorm_shift)
-template <uint32_t N>
-CG_HD void add_if_le(uint32_t &x, uint32_t v, uint32_t w) {
-#if defined(__CUDA_ARCH__)
-    asm("{ .reg .pred p; setp.le.u32 p, %1, %2; @p add.u32 %0, %0, %3; }" : "+r"(x) : "r"(v), "r"(w), "n"(N));
-#else
-    if (v <= w) x += N;
-#endif
-}
-
 // ---- shared-memory access --------------------------------------------------------------------------------
-// A stream's table is the column tab[m][tid] = cdf[m] << 16 of a [rows][128] uint32 array, addressed
+// A stream's table is a column tab[m][tid] of a [rows][128] uint32 array (cdf[m] << 16 for the encoder, search_entry(cdf[m])
+// for the decoder), addressed
 // by byte address: entry m of the column starting at `col` is at col + m * kTableRowBytes.  On the
 // device the addresses are shared-memory addresses (bank = lane for every row); on the host they are
 // offsets into a plain array.
@@ -317,21 +308,39 @@ struct DecoderState {
         span32 = fhi - flo;
         const uint32_t d = span32 - 1u;
         const Renorm r = renorm_shift(low, low + d, d);
-        low *= r.p2;
-        span32 *= r.p2;
+        low = cg_fshl(0u, low, r.s);
+        span32 = cg_fshl(0u, span32, r.s);
         offset = cg_fshl(bw.hi, offset, r.s);
         bw.consume(r);
     }
 };
 
 // ---- decode loop: NS streams per lane, search depth chosen by the caller ---------------------------------
+// Table entries as the search takes them: 2^23 (1 + cdf / 2^16) as a float.  Its bits shifted by nine are cdf << 16, and
+// a comparison with an estimate of 2^23 (1 + offset / span) + 1, which is as whole a number, is the difference cut to
+// [0, 1], which is 0 or 1.  A search step is then a subtraction with saturation and a multiply-add on the entry's address
+// (taken as a denormal float, which adds like an integer): both on the two floating-point pipes, where a compare and a
+// predicated add go to the integer pipes, which have half the rate and bind the loop.  8,192 Llama-7B tokens: 4.18 ms with
+// integer entries.
+CG_HD uint32_t search_entry(uint32_t cdf) { return 0x4B000000u | cdf << 7; }
+constexpr uint32_t kSearchPadding = 0x7F800000u;  // +inf: above every estimate
+CG_HD uint32_t ld_entry(Smem sm, uint32_t addr) {
+#if defined(__CUDA_ARCH__)
+    return sm.ld(addr);
+#else
+    const uint32_t v = sm.ld(addr);  // the host's columns hold cdf << 16, padded with 0xFFFFFFFF
+    return v == 0xFFFFFFFFu ? kSearchPadding : search_entry(v >> 16);
+#endif
+}
+CG_HD uint32_t entry_c16(uint32_t entry) { return cg_fshl(0u, entry, 9u); }  // cdf << 16
+
 // Exact search with a run-time depth (the rare path of decode_streams).
 CG_HD uint32_t exact_search(Smem sm, uint32_t col, uint32_t a_max, uint32_t span32, uint32_t target, int levels) {
     uint32_t a = col;
     for (int b = levels - 1; b >= 0; --b) {
         const uint32_t ca = a + (static_cast<uint32_t>(kTableRowBytes) << b);
         const bool ok = ca <= a_max;
-        const bool take = ok && (scale_exact(span32, sm.ld(ok ? ca : a)) <= target);
+        const bool take = ok && (scale_exact(span32, entry_c16(ld_entry(sm, ok ? ca : a))) <= target);
         a = take ? ca : a;
     }
     return a;
@@ -345,33 +354,40 @@ CG_HD int fast_levels_for(int nsym, int full_levels) {
     return fl;
 }
 
-// offset / span as a 32-bit fraction, to about 2^-22 (the low nine bits are zero); anything when the span is the
-// full 2^32 (span32 == 0).
-CG_HD uint32_t ratio_estimate(uint32_t offset, uint32_t span32) {
+// 2^23 (1 + offset / span) + 1, to about 2 (see search_entry); anything when the span is the full 2^32 (span32 == 0).
+CG_HD float ratio_estimate(uint32_t offset, uint32_t span32) {
 #if defined(__CUDA_ARCH__)
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_rn(span32)));
-    return __float_as_uint(__fmaf_rn(__uint2float_rn(offset), r, 1.0f)) * 512u;  // the 23 bits after the point, at the top
+    return __fmaf_rn(__uint2float_rn(offset), r * 8388608.0f, 8388609.0f);
 #else
-    const float q = span32 ? static_cast<float>(offset) / static_cast<float>(span32) + 1.0f : 1.0f;
-    uint32_t bits;
-    __builtin_memcpy(&bits, &q, 4);
-    return bits * 512u;
+    return span32 ? static_cast<float>(offset) * (8388608.0f / static_cast<float>(span32)) + 8388609.0f : 8388609.0f;
 #endif
 }
-
-// Search steps on a ratio estimate: the candidate entry is kTableRowBytes << B bytes above `a`.
+// address a, or a + STEP if the entry is not above the ratio
+template <uint32_t STEP>
+CG_HD uint32_t search_step(uint32_t a, uint32_t entry, float ratio) {
+#if defined(__CUDA_ARCH__)
+    float take;
+    asm("sub.rn.sat.f32 %0, %1, %2;" : "=f"(take) : "f"(ratio), "f"(__uint_as_float(entry)));
+    return __float_as_uint(__fmaf_rn(take, __uint_as_float(STEP), __uint_as_float(a)));
+#else
+    float e;
+    __builtin_memcpy(&e, &entry, 4);
+    return ratio - e >= 1.0f ? a + STEP : a;
+#endif
+}
+// Search steps: the candidate entry is kTableRowBytes << B bytes above `a`.
 template <int B>
 struct RatioSearch {
-    static CG_HD uint32_t run(Smem sm, uint32_t a, uint32_t ratio) {
-        const uint32_t v = sm.ld(a + (static_cast<uint32_t>(kTableRowBytes) << B));
-        add_if_le<(static_cast<uint32_t>(kTableRowBytes) << B)>(a, v, ratio);
-        return RatioSearch<B - 1>::run(sm, a, ratio);
+    static CG_HD uint32_t run(Smem sm, uint32_t a, float ratio) {
+        constexpr uint32_t kStep = static_cast<uint32_t>(kTableRowBytes) << B;
+        return RatioSearch<B - 1>::run(sm, search_step<kStep>(a, ld_entry(sm, a + kStep), ratio), ratio);
     }
 };
 template <>
 struct RatioSearch<-1> {
-    static CG_HD uint32_t run(Smem, uint32_t a, uint32_t) { return a; }
+    static CG_HD uint32_t run(Smem, uint32_t a, float) { return a; }
 };
 
 // NS streams of one lane decoded side by side (same token count, same table length), the fast
@@ -382,12 +398,11 @@ struct RatioSearch<-1> {
 // integer pipe a warp, measured).  The symbol is then checked exactly: the offset must lie inside its scaled
 // bounds, which the range update needs anyway.  The caller picks FL from what it knows about the symbols (a
 // row quantised to `bins` bins holds symbols 0 .. bins-2, so 2^FL >= bins is enough).  The result depends
-// on neither (4.41 -> 4.20 ms for 8,192 Llama-7B tokens): a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol
-// >= 2^FL - 1, a symbol that starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away
+// on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol >= 2^FL - 1, a symbol that starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away
 // and the whole warp repeats that symbol with the exact, full-depth search.
 //
 // The table's last symbol has no upper entry.  With LAST_REPEATED the rows above its entry hold copies of it,
-// so that its bounds are equal and the check fails; otherwise they hold 0xFFFFFFFF (never "<= ratio") and
+// so that its bounds are equal and the check fails; otherwise they hold kSearchPadding and
 // a symbol at or above the address threshold det is repeated as well.  The column needs 2^FL + 1
 // readable rows either way.
 //   col[i]    table column of stream i (see decode_stream)
@@ -402,7 +417,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     static_assert(FL >= 2, "the first level's entry is held in a register");
     BitWindow bw[NS];
     DecoderState st[NS];
-    uint32_t r_mid[NS], a_max[NS], col_top[NS];
+    uint32_t mid[NS], a_max[NS];
     constexpr uint32_t kTop = static_cast<uint32_t>(kTableRowBytes) << (FL - 1);
 #if defined(__CUDA_ARCH__)
 #pragma unroll
@@ -412,77 +427,84 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
         st[i].span32 = 0u;
         st[i].offset = bw[i].open(stream[i], len[i]);
         a_max[i] = col[i] + static_cast<uint32_t>(maxsym) * kTableRowBytes;
-        col_top[i] = col[i] + kTop;
-        r_mid[i] = sm.ld(col[i] + kTop);
+        mid[i] = ld_entry(sm, col[i] + kTop);
     }
-    uint32_t a[NS];
-    // One back edge and one vote per token: the rare path (a refill of the bit windows, or the exact
-    // search when the fast one failed) only tops the windows up or replaces the symbol and
-    // its scaled bounds; the range update below is shared.
+    uint32_t a[NS], flo[NS], fhi[NS];
     const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
     uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
+    // The inner loop is the common case and nothing else, left by one vote for a refill of the bit windows, for a
+    // symbol whose fast search failed and at the last token; with that code inside it, the state of both streams moved
+    // between registers at every pass.
+    for (;;) {
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
-    for (; t4 != last4; t4 += 4u) {
-        uint32_t flo[NS], fhi[NS], ratio[NS];
-        bool rare = false;  // a symbol that fails the check
-        int fewest = bw[0].nbits;
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-        for (int i = 0; i < NS; ++i) {
-            ratio[i] = ratio_estimate(st[i].offset, st[i].span32);
-            a[i] = r_mid[i] <= ratio[i] ? col_top[i] : col[i];
-        }
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-        for (int i = 0; i < NS; ++i) a[i] = RatioSearch<FL - 2>::run(sm, a[i], ratio[i]);
-        uint32_t e0[NS], e1[NS];
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-        for (int i = 0; i < NS; ++i) {
-            e0[i] = sm.ld(a[i]);
-            e1[i] = sm.ld(a[i] + kTableRowBytes);
-        }
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-        for (int i = 0; i < NS; ++i) {
-            flo[i] = cg_umulhi(st[i].span32, e0[i]);
-            fhi[i] = cg_umulhi(st[i].span32, e1[i]);
-            rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]);
-            fewest = fewest < bw[i].nbits ? fewest : bw[i].nbits;
-            if (!LAST_REPEATED) rare = rare | (a[i] >= det);
-        }
-        if (cg_any_lane(lanes, rare | (fewest < BitWindow::kShort))) {
-            bool low = false, odd = false;
+        for (;;) {
+            float ratio[NS];
+            bool rare = false;  // a symbol that fails the check
+            int fewest = bw[0].nbits;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
             for (int i = 0; i < NS; ++i) {
-                low = low || bw[i].short_of_bits();
-                odd = odd || st[i].offset - flo[i] >= fhi[i] - flo[i];
-                if (!LAST_REPEATED) odd = odd || a[i] >= det;
+                ratio[i] = ratio_estimate(st[i].offset, st[i].span32);
+                a[i] = search_step<kTop>(col[i], mid[i], ratio[i]);
             }
-            if (cg_any_lane(lanes, low)) {
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-                for (int i = 0; i < NS; ++i) bw[i].refill();
-            }
-            if (cg_any_lane(lanes, odd)) {
+            for (int i = 0; i < NS; ++i) a[i] = RatioSearch<FL - 2>::run(sm, a[i], ratio[i]);
+            uint32_t e0[NS], e1[NS];
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-                for (int i = 0; i < NS; ++i) {
-                    a[i] = exact_search(sm, col[i], a_max[i], st[i].span32, st[i].offset, full_levels);
-                    flo[i] = scale_exact(st[i].span32, sm.ld(a[i]));
-                    fhi[i] = (a[i] == a_max[i]) ? st[i].span32
-                                                : scale_exact(st[i].span32, sm.ld(a[i] + kTableRowBytes));
-                }
+            for (int i = 0; i < NS; ++i) {
+                e0[i] = entry_c16(ld_entry(sm, a[i]));
+                e1[i] = entry_c16(ld_entry(sm, a[i] + kTableRowBytes));
+            }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) {
+                flo[i] = cg_umulhi(st[i].span32, e0[i]);
+                fhi[i] = cg_umulhi(st[i].span32, e1[i]);
+                rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]);
+                fewest = fewest < bw[i].nbits ? fewest : bw[i].nbits;
+                if (!LAST_REPEATED) rare = rare | (a[i] >= det);
+            }
+            if (cg_any_lane(lanes, rare | (fewest < BitWindow::kShort) | (t4 == last4))) break;
+            emit(a, t4);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) st[i].update(flo[i], fhi[i], bw[i]);
+            t4 += 4u;
+        }
+        if (t4 == last4) break;
+        bool low = false, odd = false;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int i = 0; i < NS; ++i) {
+            low = low || bw[i].short_of_bits();
+            odd = odd || st[i].offset - flo[i] >= fhi[i] - flo[i];
+            if (!LAST_REPEATED) odd = odd || a[i] >= det;
+        }
+        if (cg_any_lane(lanes, low)) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) bw[i].refill();
+        }
+        if (cg_any_lane(lanes, odd)) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) {
+                a[i] = exact_search(sm, col[i], a_max[i], st[i].span32, st[i].offset, full_levels);
+                flo[i] = scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i])));
+                fhi[i] = (a[i] == a_max[i]) ? st[i].span32
+                                            : scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i] + kTableRowBytes)));
             }
         }
         emit(a, t4);
@@ -490,6 +512,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 #pragma unroll
 #endif
         for (int i = 0; i < NS; ++i) st[i].update(flo[i], fhi[i], bw[i]);
+        t4 += 4u;
     }
     // last symbol: no range update (dec_new.cu:273-275), so no new bits either
 #if defined(__CUDA_ARCH__)
@@ -499,7 +522,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     emit(a, t4);
 }
 
-// One stream.  col: address of the stream's table column, entries cdf << 16, rows kTableRowBytes apart,
+// One stream.  col: address of the stream's table column (see search_entry), rows kTableRowBytes apart,
 // 2^LEVELS + 1 of them readable, 2^LEVELS >= maxsym + 1; emit(a) receives, token after token, the address of the
 // decoded symbol's table entry (symbol = (a - col) / kTableRowBytes).  lanes: the warp's lanes that
 // run this loop together (they must all have the same ntok).  FULL: the table has exactly 2^LEVELS symbols (the

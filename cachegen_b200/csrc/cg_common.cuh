@@ -64,24 +64,26 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 }
 
 // ---- table staging ----------------------------------------------------------------------------
-// Every thread owns one (row, channel) table.  It is kept in shared memory as tab[m][tid] =
-// cdf[m] << 16 so that lane i always hits bank i, whatever entry m each lane is at.  Each thread
-// fills (and later reads) only its own column, so no block barrier is needed.  Only the entries of
-// the symbols, 0 .. lp-2, are staged; the rows above them hold kTablePadding, which a search step
-// of the decoder takes for "above the target", or with REPEAT_LAST copies of the last entry (see
-// decode_streams in cg_coder.cuh).
-constexpr uint32_t kTablePadding = 0xFFFFFFFFu;
-template <bool REPEAT_LAST = false, int STRIDE = kGroup>
-__device__ __forceinline__ void stage_table_column(uint32_t *tab, const int16_t *cdf_row, int lp,
-                                                   int rows, int tid) {
+// Every thread owns one (row, channel) table.  It is kept in shared memory as a column tab[m][tid] so that
+// lane i always hits bank i, whatever entry m each lane is at: of cdf[m] << 16 for the encoder, of search_entry(cdf[m])
+// for the decoder.  Each thread fills (and later reads) only its own column, so no block barrier is needed.  Only the
+// entries of the symbols, 0 .. lp-2, are staged; the decoder's rows above them hold kSearchPadding, which a search step
+// takes for "above the target", or with REPEAT_LAST copies of the last entry (see decode_streams in cg_coder.cuh).
+template <int STRIDE>
+__device__ __forceinline__ void stage_encode_column(uint32_t *tab, const int16_t *cdf_row, int lp, int tid) {
+    for (int m = 0; m < lp - 1; ++m) tab[m * STRIDE + tid] = static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))) << 16;
+    tab[(lp - 1) * STRIDE + tid] = 0xFFFFFFFFu;
+}
+template <bool REPEAT_LAST = false>
+__device__ __forceinline__ void stage_table_column(uint32_t *tab, const int16_t *cdf_row, int lp, int rows, int tid) {
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    uint32_t pad = kTablePadding, e = 0u;
+    uint32_t pad = kSearchPadding, e = 0u;
     for (int m = 0; m < n; ++m) {
-        e = static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))) << 16;
-        tab[m * STRIDE + tid] = e;
+        e = search_entry(static_cast<uint32_t>(static_cast<uint16_t>(__ldg(cdf_row + m))));
+        tab[m * kGroup + tid] = e;
     }
     if (REPEAT_LAST) pad = e;
-    for (int m = n; m < rows; ++m) tab[m * STRIDE + tid] = pad;
+    for (int m = n; m < rows; ++m) tab[m * kGroup + tid] = pad;
 }
 
 // The same column from the byte counts of the non-centre symbols (CG_TABLES_COUNTS):
@@ -100,11 +102,11 @@ __device__ __forceinline__ void stage_table_column_from_counts(uint32_t *tab, co
     const bool pow2 = (total & (total - 1u)) == 0u;
     const int sh = 31 - __clz(static_cast<int>(total | 1u));
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    uint32_t cum = 0, pad = kTablePadding;
+    uint32_t cum = 0, pad = kSearchPadding;
     for (int i = 0; i < n; ++i) {
         const uint32_t prod = scale * (cum & 0xFFFFu);
         const uint32_t nv = total ? (pow2 ? (prod >> sh) : (prod / total)) : 0u;
-        const uint32_t e = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        const uint32_t e = search_entry((nv + static_cast<uint32_t>(i)) & 0xFFFFu);
         tab[i * kGroup + tid] = e;
         if (REPEAT_LAST) pad = e;
         uint32_t count = 0;
@@ -133,11 +135,11 @@ __device__ __forceinline__ void stage_table_column_from_sparse(uint32_t *tab, ui
     const bool pow2 = (total & (total - 1u)) == 0u;
     const int sh = 31 - __clz(static_cast<int>(total | 1u));
     const int n = lp - 1 < rows ? lp - 1 : rows;
-    uint32_t cum = 0, pad = kTablePadding;
+    uint32_t cum = 0, pad = kSearchPadding;
     for (int i = 0; i < n; ++i) {
         const uint32_t prod = scale * (cum & 0xFFFFu);
         const uint32_t nv = total ? (pow2 ? (prod >> sh) : (prod / total)) : 0u;
-        const uint32_t e = ((nv + static_cast<uint32_t>(i)) & 0xFFFFu) << 16;
+        const uint32_t e = search_entry((nv + static_cast<uint32_t>(i)) & 0xFFFFu);
         tab[i * kGroup + tid] = e;
         if (REPEAT_LAST) pad = e;
         uint32_t count = 0;

@@ -47,20 +47,20 @@ __device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int 
     uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
     const int direct = min(n, below);
     for (int m = 0; m < direct; ++m) {
-        c0[m * kGroup] = static_cast<uint32_t>(run[m]) << 16;
-        c1[m * kGroup] = static_cast<uint32_t>(run[lp + m]) << 16;
+        c0[m * kGroup] = search_entry(run[m]);
+        c1[m * kGroup] = search_entry(run[lp + m]);
     }
     uint32_t hold[kHold];
 #pragma unroll
     for (int k = 0; k < kHold; ++k)
         hold[k] = direct + k < n ? static_cast<uint32_t>(run[direct + k]) | static_cast<uint32_t>(run[lp + direct + k]) << 16 : 0u;
-    const uint32_t last0 = static_cast<uint32_t>(run[n - 1]) << 16, last1 = static_cast<uint32_t>(run[lp + n - 1]) << 16;
+    const uint32_t last0 = search_entry(run[n - 1]), last1 = search_entry(run[lp + n - 1]);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kHold; ++k)
         if (direct + k < n) {
-            c0[(direct + k) * kGroup] = hold[k] << 16;
-            c1[(direct + k) * kGroup] = hold[k] & 0xFFFF0000u;
+            c0[(direct + k) * kGroup] = search_entry(hold[k] & 0xFFFFu);
+            c1[(direct + k) * kGroup] = search_entry(hold[k] >> 16);
         }
     for (int m = n; m < rows; ++m) {
         c0[m * kGroup] = last0;
@@ -383,9 +383,9 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
 // values with one 2*NS-byte store.  Channel NS*t + i keeps its table in column t + i * (128 / NS), so a
 // warp still reads 32 different banks whatever entries its lanes are at.  The search depth is chosen
 // per block from the row's bin count (see decode_streams); the result does not depend on it.
-// Bound by instruction issue (58.7 instructions for 32 symbols: 80 % of the slots at 2,048 tokens, 81 % at 8,192, where the
-// last wave weighs less; the integer pipe 63 %): 8,192 Llama-7B tokens in 4.18 ms, 1,261 GB/s of algorithmic bytes; 4.50 ms
-// before the search on an estimate and the one-shift renormalisation.
+// Bound by instruction issue and by the two half-rate integer pipes (58.9 instructions for 32 symbols, four issue slots of
+// five): 8,192 Llama-7B tokens in 4.00 ms, 1,317 GB/s of algorithmic bytes; 4.18 ms with the search and the renormalisation on
+// the integer pipes and the rare cases inside the loop, 4.50 before the search on an estimate.
 // Needs a head size and output strides that are multiples of NS and output pointers aligned to 2*NS bytes.
 template <int OUT_DT>
 __device__ __forceinline__ uint32_t pack_pair(float v0, float v1);

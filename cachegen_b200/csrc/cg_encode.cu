@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     const int n = min(kSubTokens, p.ntokens - t0);
     const int maxsym = p.lp - 2;
 
-    stage_table_column(tab, p.cdf + g * p.lp, p.lp, p.lp, tid);
+    stage_encode_column<kGroup>(tab, p.cdf + g * p.lp, p.lp, tid);
     const uint32_t col = smem_addr(tab + tid);
     const int64_t slot = static_cast<int64_t>(sub) * nrows * p.nchannels + g;
     BitSink out[1];

@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
         copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp, nch * p.lp, lane);
     } else if (any_active) {
 #pragma unroll
-        for (int s = 0; s < NS; ++s) stage_table_column<false, 32>(column[s], p.out.cdf + g[s] * p.lp, p.lp, p.lp, 0);
+        for (int s = 0; s < NS; ++s) stage_encode_column<32>(column[s], p.out.cdf + g[s] * p.lp, p.lp, 0);
     }
 
     if (any_active) {
