@@ -11,6 +11,7 @@ CG_MAX_TOKENS_PER_STREAM = 256
 CG_MAX_LP = 64
 CG_GROUP_CHANNELS = 128
 CG_MAX_DECODE_JOBS = 40
+CG_MAX_ENCODE_LEVELS = 4
 CG_MAX_OFFSET_GROUPS = 96000
 CG_S_STREAM_OVERFLOW, CG_S_BAD_LENGTHS, CG_S_BAD_SYMBOL, CG_S_COUNT_OVERFLOW, CG_S_BAD_TABLE = 1, 2, 4, 8, 16
 CG_TABLES_CDF, CG_TABLES_COUNTS, CG_TABLES_SPARSE = 0, 1, 2
@@ -73,7 +74,8 @@ class HostSegment(ctypes.Structure):
 EXPORTS = [
     "cg_host_upload", "cg_host_stage", "cg_host_stage_send", "cg_host_stage_end", "cg_host_download", "cg_decode_kv",
     "cg_stream_sizes", "cg_decode_packed", "cg_wait_word",
-    "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_wait", "cg_encode_kv_gather", "cg_encode_kv_flat",
+    "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_levels", "cg_encode_kv_wait", "cg_encode_kv_gather",
+    "cg_encode_kv_levels_gather", "cg_encode_kv_flat",
     "cg_version", "cg_status_string", "cg_last_cuda_error", "cg_workspace_bytes",
     "cg_calculate_cdf", "cg_encode_padded", "cg_decode_padded", "cg_decode_prefsum", "cg_decode_prefsum_warp",
     "cg_quantize_cdf", "cg_pack_sparse_tables", "cg_encode_chunk", "cg_compact_streams",
@@ -123,8 +125,10 @@ def lib():
     job = ctypes.POINTER(EncodeKvJob)
     L.cg_encode_kv_workspace.argtypes = [i, i, i, i]
     L.cg_encode_kv.argtypes = [job, p]
+    L.cg_encode_kv_levels.argtypes = [job, i, p]
     L.cg_encode_kv_wait.argtypes = [job, p]
     L.cg_encode_kv_gather.argtypes = [job, ctypes.POINTER(p), ctypes.POINTER(p), p]
+    L.cg_encode_kv_levels_gather.argtypes = [job, i, ctypes.POINTER(p), ctypes.POINTER(p), p]
     L.cg_encode_kv_flat.argtypes = [job, ctypes.POINTER(FlatLayout), p]
     L.cg_stream_sizes.argtypes = [p, i, i, i, p, p, p, p]
     L.cg_decode_packed.argtypes = [p, p, i64, p, p, p, S3, i, i, i, i, p, p]

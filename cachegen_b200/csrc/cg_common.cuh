@@ -36,8 +36,6 @@ int allow_smem(K kernel, size_t bytes) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMostDynamicSmem));
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
-// cg_store.cu: dynamic shared memory that makes the last wave of `blocks` equal blocks as full as the others
-size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes);
 // cg_tables.cu: group offsets of sparse tables, and the tables in one pass once those are known
 int launch_sparse_write(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
                         const uint32_t *group_off, void *masks, const int64_t *mask_row_off, uint8_t *out,

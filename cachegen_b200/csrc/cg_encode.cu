@@ -226,7 +226,7 @@ using namespace cg;
 
 static int launch_encode(const EncodeParams &p, int nrows, int nsub, cudaStream_t st) {
     const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows, nsub);
-    const size_t smem = even_waves_smem(static_cast<int64_t>(grid.x) * grid.y * grid.z, static_cast<size_t>(p.lp) * kRowBytes, 0);
+    const size_t smem = static_cast<size_t>(p.lp) * kRowBytes;
     const bool narrow = p.s1 >= 0 && p.s2 >= 0 && p.s1 <= 0xFFFFFFFF / (kSubTokens + 1) &&
                         p.s1 * kSubTokens + p.s2 * p.nchannels <= 0xFFFFFFFF;
     const auto kernel = narrow ? encode_kernel<true> : encode_kernel<false>;

@@ -49,20 +49,30 @@ __device__ __forceinline__ void quantize2(float x0, float x1, float f, uint64_t 
 // 5.0 TB/s, where the two passes took 31 + 61 us (the second with the histogram, which the coder does now).
 // Three blocks of 512 threads an SM (42 registers a thread) keep enough loads in flight; more than 4,096
 // channels need one block of up to 1,024 threads.
-template <int DT, int THREADS, int BLOCKS>
-__global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const KvView v, const float *__restrict__ bins, int max_bins,
-                                                               uint16_t *__restrict__ scales_k,
-                                                               uint16_t *__restrict__ scales_v,
-                                                               uint32_t *__restrict__ sym4, uint32_t *zeroed, int nzeroed) {
+// The same KV at several bin settings takes one read and one reduction: only the quantisation is done for each.
+struct QuantizeOut {
+    const float *bins;
+    uint16_t *scales_k, *scales_v;
+    uint32_t *sym4, *zeroed;
+    int max_bins;
+};
+struct QuantizeLevels {
+    QuantizeOut level[CG_MAX_ENCODE_LEVELS];
+    int n, nzeroed;
+};
+template <int DT, int THREADS, int BLOCKS, bool ONE>
+__global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const KvView v, const __grid_constant__ QuantizeLevels q) {
     __shared__ uint4 part[32];
-    __shared__ float4 factor_s;
+    __shared__ float4 factor_s[ONE ? 1 : CG_MAX_ENCODE_LEVELS];
     __shared__ uint32_t keep_s;
+    const int nlevels = ONE ? 1 : q.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.y, t0 = blockIdx.x * kTokensPerWord;
     const int C = v.nheads * v.head_size, c = tid * 8;
     const int layer = row % v.nlayers, kv = row / v.nlayers;
     if (row == 0 && blockIdx.x == 0)  // the counters of the launches after this one
-        for (int i = tid; i < nzeroed; i += blockDim.x) zeroed[i] = 0u;
+        for (int l = 0; l < nlevels; ++l)
+            for (int i = tid; i < q.nzeroed; i += blockDim.x) q.level[l].zeroed[i] = 0u;
     uint4 x[kTokensPerWord];
 #pragma unroll
     for (int j = 0; j < kTokensPerWord; ++j) x[j] = make_uint4(0u, 0u, 0u, 0u);
@@ -82,54 +92,62 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const 
         m[j] = __reduce_max_sync(0xFFFFFFFFu, max(a & 0xFFFFu, a >> 16));
     }
     if (lane == 0) part[warp] = make_uint4(m[0], m[1], m[2], m[3]);
-    const float MAX = half_range(__ldg(bins + row));
+    const float max_of_first = half_range(__ldg(q.level[0].bins + row));
     __syncthreads();
     if (warp == 0) {
-        const uint4 q = lane < (blockDim.x >> 5) ? part[lane] : make_uint4(0u, 0u, 0u, 0u);
-        m[0] = __reduce_max_sync(0xFFFFFFFFu, q.x);
-        m[1] = __reduce_max_sync(0xFFFFFFFFu, q.y);
-        m[2] = __reduce_max_sync(0xFFFFFFFFu, q.z);
-        m[3] = __reduce_max_sync(0xFFFFFFFFu, q.w);
+        const uint4 r = lane < (blockDim.x >> 5) ? part[lane] : make_uint4(0u, 0u, 0u, 0u);
+        m[0] = __reduce_max_sync(0xFFFFFFFFu, r.x);
+        m[1] = __reduce_max_sync(0xFFFFFFFFu, r.y);
+        m[2] = __reduce_max_sync(0xFFFFFFFFu, r.z);
+        m[3] = __reduce_max_sync(0xFFFFFFFFu, r.w);
         if (lane < kTokensPerWord) {
             const uint32_t mine = lane == 0 ? m[0] : lane == 1 ? m[1] : lane == 2 ? m[2] : m[3];
-            reinterpret_cast<float *>(&factor_s)[lane] = __fdiv_rn(MAX, Half16<DT>::to_float(static_cast<uint16_t>(mine)));
+            for (int l = 0; l < nlevels; ++l) {
+                const float MAX = l ? half_range(__ldg(q.level[l].bins + row)) : max_of_first;
+                reinterpret_cast<float *>(factor_s + l)[lane] = __fdiv_rn(MAX, Half16<DT>::to_float(static_cast<uint16_t>(mine)));
+                if (t0 + lane < v.ntokens) {
+                    uint16_t *s = row < v.nlayers ? q.level[l].scales_k + static_cast<int64_t>(row) * v.ntokens
+                                                  : q.level[l].scales_v + static_cast<int64_t>(row - v.nlayers) * v.ntokens;
+                    s[t0 + lane] = static_cast<uint16_t>(mine);
+                }
+            }
             // an all-zero token: 0 * inf = NaN, which the reference's cast makes symbol 0
             reinterpret_cast<uint8_t *>(&keep_s)[lane] = mine ? 0xFFu : 0u;
-            if (t0 + lane < v.ntokens) {
-                uint16_t *s = row < v.nlayers ? scales_k + static_cast<int64_t>(row) * v.ntokens
-                                              : scales_v + static_cast<int64_t>(row - v.nlayers) * v.ntokens;
-                s[t0 + lane] = static_cast<uint16_t>(mine);
-            }
         }
     }
     __syncthreads();
     if (c >= C) return;
-    const float f[kTokensPerWord] = {factor_s.x, factor_s.y, factor_s.z, factor_s.w};
     const uint32_t keep = keep_s;
-    const uint64_t m2 = pack2(MAX, MAX);
-    uint32_t w[8];
+#pragma unroll 1
+    for (int l = 0; l < nlevels; ++l) {
+        const float f[kTokensPerWord] = {factor_s[l].x, factor_s[l].y, factor_s[l].z, factor_s[l].w};
+        const float MAX = l ? half_range(__ldg(q.level[l].bins + row)) : max_of_first;
+        const uint64_t m2 = pack2(MAX, MAX);
+        uint32_t w[8];
 #pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-        uint32_t b0[kTokensPerWord], b1[kTokensPerWord];
+        for (int k = 0; k < 8; k += 2) {
+            uint32_t b0[kTokensPerWord], b1[kTokensPerWord];
 #pragma unroll
-        for (int j = 0; j < kTokensPerWord; ++j) {
-            const uint32_t pair = k == 0 ? x[j].x : k == 2 ? x[j].y : k == 4 ? x[j].z : x[j].w;
-            quantize2(Half16<DT>::to_float(static_cast<uint16_t>(pair)), Half16<DT>::to_float(static_cast<uint16_t>(pair >> 16)),
-                      f[j], m2, &b0[j], &b1[j]);
+            for (int j = 0; j < kTokensPerWord; ++j) {
+                const uint32_t pair = k == 0 ? x[j].x : k == 2 ? x[j].y : k == 4 ? x[j].z : x[j].w;
+                quantize2(Half16<DT>::to_float(static_cast<uint16_t>(pair)), Half16<DT>::to_float(static_cast<uint16_t>(pair >> 16)),
+                          f[j], m2, &b0[j], &b1[j]);
+            }
+            w[k] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410) & keep;
+            w[k + 1] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410) & keep;
         }
-        w[k] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410) & keep;
-        w[k + 1] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410) & keep;
-    }
-    // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
-    // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
-    if (2.0f * MAX >= static_cast<float>(max_bins - 1)) {
-        const uint32_t limit = static_cast<uint32_t>(max_bins - 1) * 0x01010101u;
+        // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
+        // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
+        const int max_bins = q.level[l].max_bins;
+        if (2.0f * MAX >= static_cast<float>(max_bins - 1)) {
+            const uint32_t limit = static_cast<uint32_t>(max_bins - 1) * 0x01010101u;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] |= __vcmpgeu4(w[k], limit);
+            for (int k = 0; k < 8; ++k) w[k] |= __vcmpgeu4(w[k], limit);
+        }
+        uint4 *o = reinterpret_cast<uint4 *>(q.level[l].sym4 + (static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * C + c);
+        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
-    uint4 *o = reinterpret_cast<uint4 *>(sym4 + (static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * C + c);
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 // ---- tables ------------------------------------------------------------------------------------------------
@@ -237,9 +255,17 @@ __device__ __forceinline__ void count_symbol(uint32_t addr) {
 // take 24, and the shared memory is busy for a third of the time; 512 blocks are 3.5 an SM, and while a block's 128
 // columns become tables its other 384 threads wait.
 constexpr int kTableThreads = 512, kParts = kTableThreads / kGroup;
-__global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const uint32_t *__restrict__ sym4, int ntokens,
-                                                                      int nchannels, int lp, const TableOut out,
-                                                                      int32_t *status) {
+struct TableJobs {
+    TableOut out[CG_MAX_ENCODE_LEVELS];
+    const uint32_t *sym4[CG_MAX_ENCODE_LEVELS];
+    int32_t *status[CG_MAX_ENCODE_LEVELS];
+    int lp[CG_MAX_ENCODE_LEVELS];
+};
+__global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const __grid_constant__ TableJobs jobs, int ntokens, int nchannels) {
+    const TableOut &out = jobs.out[blockIdx.z];
+    const uint32_t *const sym4 = jobs.sym4[blockIdx.z];
+    int32_t *const status = jobs.status[blockIdx.z];
+    const int lp = jobs.lp[blockIdx.z];
     extern __shared__ uint4 smem4[];
     uint32_t *hist = reinterpret_cast<uint32_t *>(smem4);
     uint16_t *stage = reinterpret_cast<uint16_t *>(hist + lp * kGroup);
@@ -317,6 +343,12 @@ struct StoreParams {
     int64_t *tail;        // [nsub + 4], see cg_encode_kv_job
 };
 
+// Several bin settings of one chunk in one launch: their blocks fill the GPU together where those of one chunk of few channels
+// leave most of it idle (a 256-token chunk of 32 layers x 8 heads is 512 blocks, 3.5 an SM).
+struct StoreJobs {
+    StoreParams job[CG_MAX_ENCODE_LEVELS];
+};
+
 // The scratch rows of the 32 streams of a warp lie interleaved: word k of stream `lane` is word 32 (k + 1) + lane
 // of the warp's 32 * (stride + 4) bytes.  A stream takes 45 of its 520 bytes on the usual workload: laid out row by
 // row that is a cache line or two for every stream (70 MB of lines a Llama-7B chunk, which the L2 did not
@@ -392,14 +424,17 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint32_
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
 // chunk takes 112 us with its tables under counters, 0.60 T symbols/s, 37.2 instructions for 32 symbols; 122 us and 40.4 with
 // the code for rare cases inside the loop and a vote a symbol.  Eight blocks an SM leave the compiler 64
-// registers; the shared memory asked for on top evens the last wave out (even_waves_smem).
+// registers.  (Seven, for two even waves of a chunk's 2,048 blocks, were better while a block took longer: 207 against 205 us a
+// whole encode now.)
 // Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
 // channels in 166 us under counters (29.9 instructions for 32 symbols), 172 before the same change; 180 with one stream.
 // G symbols a vote: two, unless the table may give a symbol more bits than the accumulator has room for twice (pair_high_water:
 // more than 21,824 tokens in one call).  The tables' part wants the warps more than the chains (a 256-token chunk
 // 129 us with two), so it keeps one; and so does a last group of channels that would leave the second without work.
 template <bool TABLES, int NS, int G>
-__global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_kernel(const __grid_constant__ StoreParams p) {
+__global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_kernel(const __grid_constant__ StoreJobs jobs) {
+    const int nsub = jobs.job[0].nsub;
+    const StoreParams &p = jobs.job[blockIdx.z / nsub];
     constexpr int kThreads = kGroup / NS, kWarps = kThreads / 32;
     constexpr int kWordsAhead = NS == 1 ? 4 : 2;  // words (of four symbols) fetched one group ahead of the coder
     extern __shared__ uint4 smem4[];
@@ -408,7 +443,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     __shared__ int block_sums[2][kWarps];
     __shared__ int last_block;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row = blockIdx.y, sub = blockIdx.z, nslab = gridDim.x;
+    const int row = blockIdx.y, sub = blockIdx.z % nsub, nslab = gridDim.x;
     const int t0 = sub * kSubTokens, n = min(kSubTokens, p.ntokens - t0);
     const int64_t C = p.nchannels;
     // channel s of this thread is number tid + kThreads * s of the group; one past the last channel repeats the last
@@ -431,6 +466,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     const bool any_active = NS > 1 || blockIdx.x * kGroup + warp * 32 < p.nchannels;
     uint32_t bad = 0;
     int nbytes = 0, nz = 0;
+    const float bins = TABLES ? __ldg(p.out.bins + row) : 0.0f;
 
     if (TABLES && any_active) {
         static_assert(!TABLES || NS == 1, "the tables' part has one stream a thread");
@@ -469,7 +505,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
             for (int j = 0; j < 4; ++j)
                 if (i + j < n) count_symbol(entry_of(col[0], w, j));
         }
-        const int cq = static_cast<int>(half_range(__ldg(p.out.bins + row)));
+        const int cq = static_cast<int>(half_range(bins));
         if (p.out.counts && active[0])
             nz = store_counts<32>(mine, p.lp, cq, p.out.counts + __ldg(p.out.table_row_off + row) - row * C + g[0], C, &overflow);
         counts_to_column<32>(mine, stage + tid * p.lp, p.lp, n, cq);
@@ -593,15 +629,19 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     __syncthreads();
     if (!last_block) return;
     __threadfence();
+    // every stream's status bits are there with its block's ticket
+    const int status = tid == 0 ? __ldcg(p.status) : 0;
     const int64_t bytes = block_scan_in_place<kThreads>(goff, ngroups, warp_sums, tid);
-    if (tid == 0) {
-        p.sub_bytes[sub] = bytes;
+    if (nsub > 1) {
+        if (tid == 0) {
+            p.sub_bytes[sub] = bytes;
+            __threadfence();
+            last_block = atomicAdd(p.tickets + nsub, 1u) == static_cast<uint32_t>(nsub - 1);
+        }
+        __syncthreads();
+        if (!last_block) return;
         __threadfence();
-        last_block = atomicAdd(p.tickets + p.nsub, 1u) == static_cast<uint32_t>(p.nsub - 1);
     }
-    __syncthreads();
-    if (!last_block) return;
-    __threadfence();
     int64_t nz_total = 0;
     if (p.out.group_nz) {
         nz_total = block_scan_in_place<kThreads>(p.out.group_nz, ngroups, warp_sums, tid);
@@ -609,15 +649,15 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
     }
     if (tid == 0) {
         int64_t run = 0;
-        for (int k = 0; k < p.nsub; ++k) {
+        for (int k = 0; k < nsub; ++k) {
             p.tail[k] = run;
-            run += __ldcg(p.sub_bytes + k);
+            run += nsub > 1 ? __ldcg(p.sub_bytes + k) : bytes;
         }
-        p.tail[p.nsub] = run;
-        p.tail[p.nsub + 1] = atomicOr(p.status, 0);
-        p.tail[p.nsub + 2] = nz_total;
+        p.tail[nsub] = run;
+        p.tail[nsub + 1] = nsub > 1 ? __ldcg(p.status) : status;
+        p.tail[nsub + 2] = nz_total;
         __threadfence_system();
-        *reinterpret_cast<volatile int64_t *>(p.tail + p.nsub + 3) = 1;
+        *reinterpret_cast<volatile int64_t *>(p.tail + nsub + 3) = 1;
     }
 }
 
@@ -640,16 +680,24 @@ struct GatherTargets {
     uint8_t *bytes[kGatherSubs];
     void *lengths[kGatherSubs];  // int32 or uint16 [nrows, C]
 };
+struct GatherJobs {
+    const uint8_t *scratch[CG_MAX_ENCODE_LEVELS];
+    const int32_t *lengths[CG_MAX_ENCODE_LEVELS];
+    const int64_t *group_off[CG_MAX_ENCODE_LEVELS];
+    int nsub;
+};
 
 // The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  14.5 us a 256-token
 // Llama-7B chunk (11.8 MB out of scratch that is read in full lines), 20 before.
 template <class Len, bool INTERLEAVED>
-__global__ void __launch_bounds__(kGroup) gather_kernel(const uint8_t *__restrict__ scratch, int64_t stride,
-                                                        const int32_t *__restrict__ lengths,
-                                                        const int64_t *__restrict__ group_off, int nchannels, int sub0,
+__global__ void __launch_bounds__(kGroup) gather_kernel(const __grid_constant__ GatherJobs jobs, int64_t stride, int nchannels, int first,
                                                         const __grid_constant__ GatherTargets out) {
+    const int job = (first + blockIdx.z) / jobs.nsub;  // sub-chunk after sub-chunk, job after job
+    const uint8_t *scratch = jobs.scratch[job];
+    const int32_t *lengths = jobs.lengths[job];
+    const int64_t *group_off = jobs.group_off[job];
     const int tid = threadIdx.x;
-    const int row = blockIdx.y, sub = sub0 + blockIdx.z, nrows = gridDim.y, nslab = gridDim.x;
+    const int row = blockIdx.y, sub = (first + blockIdx.z) % jobs.nsub, nrows = gridDim.y, nslab = gridDim.x;
     const int c = blockIdx.x * kGroup + tid;
     const int64_t group = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
     const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
@@ -680,36 +728,6 @@ __global__ void __launch_bounds__(256) flat_front_kernel(const __grid_constant__
         uint32_t *t = reinterpret_cast<uint32_t *>(blob + off_tables);
         for (int64_t i = i0; i <= ngroups; i += step) t[i] = group_off[i];
     }
-}
-
-constexpr int64_t kSmemPerSM = 228 * 1024, kSmemReserved = 1024;
-
-static int sm_count() {
-    static int count[64];  // per device; a racing first call writes the same number
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (!count[dev]) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        count[dev] = n;
-    }
-    return count[dev];
-}
-
-// Shared memory to ask for so that the grid's last wave is as full as the others.  The coder's blocks all take
-// the same time, so 2,048 blocks at 8 resident ones per SM are one full wave and one that fills 73 % of the
-// GPU; at 7 they are two that fill 99 %.  Seven blocks (28 warps) still cover the latencies.
-size_t even_waves_smem(int64_t blocks, size_t dynamic, size_t static_bytes) {
-    const int64_t need = static_cast<int64_t>(dynamic + static_bytes) + kSmemReserved;
-    const int64_t resident = kSmemPerSM / need;
-    if (resident < 1) return dynamic;
-    const int64_t sms = sm_count();
-    const int64_t waves = (blocks + sms * resident - 1) / (sms * resident);
-    const int64_t per = (blocks + sms * waves - 1) / (sms * waves);
-    if (per >= resident || per < 1) return dynamic;
-    int64_t padded = kSmemPerSM / per - kSmemReserved - static_cast<int64_t>(static_bytes) - 256;
-    if (padded > kMostDynamicSmem) padded = kMostDynamicSmem;
-    return padded > static_cast<int64_t>(dynamic) ? static_cast<size_t>(padded) : dynamic;
 }
 
 }  // namespace cg
@@ -775,6 +793,13 @@ bool fused_ok(const cg_encode_kv_job &b) {
            ((reinterpret_cast<uintptr_t>(b.kv) & 15) | (b.s_layer & 7) | (b.s_kv & 7) | (b.s_token & 7) | (b.s_head & 7)) == 0;
 }
 
+// Jobs of one call: the same KV, read in the same way, at different bin settings.
+bool same_chunk(const cg_encode_kv_job &a, const cg_encode_kv_job &b) {
+    return a.kv == b.kv && a.dtype == b.dtype && a.nlayers == b.nlayers && a.ntokens == b.ntokens && a.nheads == b.nheads &&
+           a.head_size == b.head_size && a.s_layer == b.s_layer && a.s_kv == b.s_kv && a.s_token == b.s_token && a.s_head == b.s_head &&
+           a.delta_group == b.delta_group;
+}
+
 }  // namespace
 
 extern "C" int64_t cg_encode_kv_workspace(int nlayers, int ntokens, int nheads, int head_size) {
@@ -782,52 +807,103 @@ extern "C" int64_t cg_encode_kv_workspace(int nlayers, int ntokens, int nheads, 
     return sizes_of(nlayers, ntokens, nheads, head_size).total;
 }
 
-extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
-    if (int rc = check_job(job)) return rc;
-    const cg_encode_kv_job &b = *job;
+// the separate calls, for what the fused passes do not take
+static int encode_separately(const cg_encode_kv_job &b, cudaStream_t st) {
     const Sizes z = sizes_of(b.nlayers, b.ntokens, b.nheads, b.head_size);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t *ws = static_cast<uint8_t *>(b.workspace);
     int32_t *status = reinterpret_cast<int32_t *>(ws + z.counters);
     uint32_t *group_nz = b.counts ? reinterpret_cast<uint32_t *>(ws + z.group_nz) : nullptr;
     int32_t *lengths = reinterpret_cast<int32_t *>(ws + z.lengths);
     int64_t *group_off = reinterpret_cast<int64_t *>(ws + z.group_off);
     const int lp = b.max_bins + 1;
-    b.tail[z.nsub + 3] = 0;  // host memory: the flag that cg_encode_kv_wait watches
-    if (!fused_ok(b)) {
-        const cudaError_t e = cudaMemsetAsync(status, 0, 4, st);
-        if (e != cudaSuccess) return set_cuda_error(e);
-        uint16_t *scales = reinterpret_cast<uint16_t *>(ws + z.scales);
-        int8_t *sym = reinterpret_cast<int8_t *>(ws + z.sym);
-        if (int rc = cg_quantize_cdf_delta(b.kv, b.dtype, b.s_layer, b.s_kv, b.s_token, b.s_head, b.nlayers, b.ntokens,
-                                           b.nheads, b.head_size, b.bins, b.max_bins, b.delta_group, b.res_bins, sym, scales,
-                                           b.cdf, b.counts, b.table_row_off, status, stream))
-            return rc;
-        const size_t half = static_cast<size_t>(b.nlayers) * b.ntokens;
-        const cudaError_t e1 = cudaMemcpyAsync(b.scales_k, scales, half * 2, cudaMemcpyDeviceToDevice, st);
-        const cudaError_t e2 = cudaMemcpyAsync(b.scales_v, scales + half, half * 2, cudaMemcpyDeviceToDevice, st);
-        if (e1 != cudaSuccess || e2 != cudaSuccess) return set_cuda_error(e1 != cudaSuccess ? e1 : e2);
-        int64_t *sub_off = reinterpret_cast<int64_t *>(ws + z.sub_off);
-        if (int rc = cg_encode_chunk(b.cdf, sym, z.nrows, b.ntokens, z.nchannels, lp, ws + z.scratch, z.stride, lengths,
-                                     group_off, sub_off, status, stream))
-            return rc;
-        if (b.counts)
-            if (int rc = launch_sparse_sizes(b.counts, b.table_row_off, b.bins, z.nrows, z.nchannels, group_nz, st)) return rc;
-        publish_tail_kernel<<<1, 128, 0, st>>>(sub_off, status, z.nsub,
-                                               group_nz ? group_nz + static_cast<int64_t>(z.nrows) * z.nslab : nullptr, b.tail);
-        return check_launch();
+    void *stream = st;
+    const cudaError_t e = cudaMemsetAsync(status, 0, 4, st);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    uint16_t *scales = reinterpret_cast<uint16_t *>(ws + z.scales);
+    int8_t *sym = reinterpret_cast<int8_t *>(ws + z.sym);
+    if (int rc = cg_quantize_cdf_delta(b.kv, b.dtype, b.s_layer, b.s_kv, b.s_token, b.s_head, b.nlayers, b.ntokens,
+                                       b.nheads, b.head_size, b.bins, b.max_bins, b.delta_group, b.res_bins, sym, scales,
+                                       b.cdf, b.counts, b.table_row_off, status, stream))
+        return rc;
+    const size_t half = static_cast<size_t>(b.nlayers) * b.ntokens;
+    const cudaError_t e1 = cudaMemcpyAsync(b.scales_k, scales, half * 2, cudaMemcpyDeviceToDevice, st);
+    const cudaError_t e2 = cudaMemcpyAsync(b.scales_v, scales + half, half * 2, cudaMemcpyDeviceToDevice, st);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return set_cuda_error(e1 != cudaSuccess ? e1 : e2);
+    int64_t *sub_off = reinterpret_cast<int64_t *>(ws + z.sub_off);
+    if (int rc = cg_encode_chunk(b.cdf, sym, z.nrows, b.ntokens, z.nchannels, lp, ws + z.scratch, z.stride, lengths,
+                                 group_off, sub_off, status, stream))
+        return rc;
+    if (b.counts)
+        if (int rc = launch_sparse_sizes(b.counts, b.table_row_off, b.bins, z.nrows, z.nchannels, group_nz, st)) return rc;
+    publish_tail_kernel<<<1, 128, 0, st>>>(sub_off, status, z.nsub,
+                                           group_nz ? group_nz + static_cast<int64_t>(z.nrows) * z.nslab : nullptr, b.tail);
+    return check_launch();
+}
+
+extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) { return cg_encode_kv_levels(job, 1, stream); }
+
+extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void *stream) {
+    if (njobs < 1) return CG_E_SHAPE;
+    if (njobs > CG_MAX_ENCODE_LEVELS) return CG_E_CAPACITY;
+    if (!jobs) return CG_E_NULL;
+    for (int j = 0; j < njobs; ++j) {
+        if (int rc = check_job(jobs + j)) return rc;
+        if (!same_chunk(jobs[0], jobs[j])) return CG_E_SHAPE;
+    }
+    const cg_encode_kv_job &b = jobs[0];
+    const Sizes z = sizes_of(b.nlayers, b.ntokens, b.nheads, b.head_size);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    for (int j = 0; j < njobs; ++j) jobs[j].tail[z.nsub + 3] = 0;  // host memory: the flag that cg_encode_kv_wait watches
+    bool fused = true;
+    for (int j = 0; j < njobs; ++j) fused = fused && fused_ok(jobs[j]);
+    if (!fused) {
+        for (int j = 0; j < njobs; ++j)
+            if (int rc = encode_separately(jobs[j], st)) return rc;
+        return CG_OK;
     }
     const KvView v{static_cast<const uint16_t *>(b.kv), b.s_layer, b.s_kv, b.s_token, b.s_head,
                    b.nlayers, b.ntokens, b.nheads, b.head_size,
                    0xFFFFFFFFu / static_cast<uint32_t>(b.head_size) + 1u};
-    uint32_t *sym4 = reinterpret_cast<uint32_t *>(ws + z.sym);
+    QuantizeLevels q;
+    StoreJobs store_jobs;
+    TableJobs table_jobs;
+    q.n = njobs;
+    q.nzeroed = z.nsub + 2;
+    int lp = 0;
+    for (int j = 0; j < njobs; ++j) {
+        const cg_encode_kv_job &k = jobs[j];
+        uint8_t *ws = static_cast<uint8_t *>(k.workspace);
+        uint32_t *zeroed = reinterpret_cast<uint32_t *>(ws + z.counters);
+        q.level[j] = QuantizeOut{k.bins, static_cast<uint16_t *>(k.scales_k), static_cast<uint16_t *>(k.scales_v),
+                                 reinterpret_cast<uint32_t *>(ws + z.sym), zeroed, k.max_bins};
+        StoreParams &p = store_jobs.job[j];
+        p.sym4 = q.level[j].sym4;
+        p.out = TableOut{k.cdf, k.counts, k.table_row_off, k.bins, k.counts ? reinterpret_cast<uint32_t *>(ws + z.group_nz) : nullptr};
+        p.ntokens = k.ntokens;
+        p.nchannels = z.nchannels;
+        p.lp = k.max_bins + 1;
+        p.nrows = z.nrows;
+        p.nsub = z.nsub;
+        p.high_water = pair_high_water(k.ntokens);
+        p.scratch = ws + z.scratch;
+        p.stride = z.stride;
+        p.lengths = reinterpret_cast<int32_t *>(ws + z.lengths);
+        p.group_off = reinterpret_cast<int64_t *>(ws + z.group_off);
+        p.sub_bytes = reinterpret_cast<int64_t *>(ws + z.sub_bytes);
+        p.tickets = zeroed + 1;
+        p.status = reinterpret_cast<int32_t *>(zeroed);
+        p.tail = k.tail;
+        table_jobs.out[j] = p.out;
+        table_jobs.sym4[j] = p.sym4;
+        table_jobs.status[j] = p.status;
+        table_jobs.lp[j] = p.lp;
+        lp = p.lp > lp ? p.lp : lp;
+    }
     const dim3 qgrid(static_cast<unsigned>(z.words), z.nrows);
     const int qthreads = (z.nchannels / 8 + 31) / 32 * 32;
-    uint32_t *zeroed = reinterpret_cast<uint32_t *>(status);
-    uint16_t *sk = static_cast<uint16_t *>(b.scales_k), *sv = static_cast<uint16_t *>(b.scales_v);
 #define CG_LAUNCH_QT(DT, THREADS, BLOCKS)                                                                    \
-    quantize_tokens_kernel<DT, THREADS, BLOCKS><<<qgrid, qthreads, 0, st>>>(v, b.bins, b.max_bins, sk, sv, sym4, zeroed, \
-                                                                            z.nsub + 2)
+    njobs == 1 ? quantize_tokens_kernel<DT, THREADS, BLOCKS, true><<<qgrid, qthreads, 0, st>>>(v, q)          \
+               : quantize_tokens_kernel<DT, THREADS, BLOCKS, false><<<qgrid, qthreads, 0, st>>>(v, q)
     if (b.dtype == CG_F16) {
         if (qthreads <= 512) CG_LAUNCH_QT(CG_F16, 512, 3);
         else CG_LAUNCH_QT(CG_F16, 1024, 1);
@@ -837,38 +913,18 @@ extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) {
     }
 #undef CG_LAUNCH_QT
     if (int rc = check_launch()) return rc;
-    StoreParams p;
-    p.sym4 = sym4;
-    p.out = TableOut{b.cdf, b.counts, b.table_row_off, b.bins, group_nz};
-    p.ntokens = b.ntokens;
-    p.nchannels = z.nchannels;
-    p.lp = lp;
-    p.nrows = z.nrows;
-    p.nsub = z.nsub;
-    p.high_water = pair_high_water(b.ntokens);
-    p.scratch = ws + z.scratch;
-    p.stride = z.stride;
-    p.lengths = lengths;
-    p.group_off = group_off;
-    p.sub_bytes = reinterpret_cast<int64_t *>(ws + z.sub_bytes);
-    p.tickets = zeroed + 1;
-    p.status = status;
-    p.tail = b.tail;
-    const dim3 grid(z.nslab, z.nrows, z.nsub);
-    const int64_t blocks = static_cast<int64_t>(z.nslab) * z.nrows * z.nsub;
+    const dim3 grid(z.nslab, z.nrows, z.nsub * njobs);
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
-    const auto store = [&](auto kernel, int threads, size_t dynamic) {
-        const size_t smem = even_waves_smem(blocks, dynamic, 128);
+    const auto store = [&](auto kernel, int threads, size_t smem) {
         if (int rc = allow_smem(kernel, smem)) return rc;
-        kernel<<<grid, threads, smem, st>>>(p);
+        kernel<<<grid, threads, smem, st>>>(store_jobs);
         return check_launch();
     };
     if (z.nsub == 1) return store(store_encode_kernel<true, 1, 2>, kGroup, columns + staged);
     if (int rc = allow_smem(packed_tables_kernel, columns + staged)) return rc;
-    packed_tables_kernel<<<dim3(z.nslab, z.nrows), kTableThreads, columns + staged, st>>>(sym4, b.ntokens, z.nchannels, lp,
-                                                                                         p.out, status);
+    packed_tables_kernel<<<dim3(z.nslab, z.nrows, njobs), kTableThreads, columns + staged, st>>>(table_jobs, b.ntokens, z.nchannels);
     if (int rc = check_launch()) return rc;
-    if (!p.high_water) return store(store_encode_kernel<false, 1, 1>, kGroup, columns);
+    if (!store_jobs.job[0].high_water) return store(store_encode_kernel<false, 1, 1>, kGroup, columns);
     // two streams a thread unless the last group has channels for the first alone
     const int last = z.nchannels % kGroup;
     if (last == 0 || last > kGroup / 2) return store(store_encode_kernel<false, 2, 2>, kGroup / 2, columns);
@@ -898,22 +954,27 @@ extern "C" int cg_wait_word(const int64_t *word, void *stream) {
 
 namespace {
 template <class Len>
-int launch_gather(const cg_encode_kv_job &b, const Sizes &z, uint8_t *const *bytes, void *const *lengths, cudaStream_t st) {
-    const uint8_t *ws = static_cast<const uint8_t *>(b.workspace);
-    for (int s0 = 0; s0 < z.nsub; s0 += kGatherSubs) {
-        const int n = z.nsub - s0 < kGatherSubs ? z.nsub - s0 : kGatherSubs;
+int launch_gather(const cg_encode_kv_job *jobs, int njobs, const Sizes &z, uint8_t *const *bytes, void *const *lengths, cudaStream_t st) {
+    GatherJobs g;
+    g.nsub = z.nsub;
+    for (int j = 0; j < njobs; ++j) {
+        const uint8_t *ws = static_cast<const uint8_t *>(jobs[j].workspace);
+        g.scratch[j] = ws + z.scratch;
+        g.lengths[j] = reinterpret_cast<const int32_t *>(ws + z.lengths);
+        g.group_off[j] = reinterpret_cast<const int64_t *>(ws + z.group_off);
+    }
+    for (int s0 = 0; s0 < z.nsub * njobs; s0 += kGatherSubs) {
+        const int n = z.nsub * njobs - s0 < kGatherSubs ? z.nsub * njobs - s0 : kGatherSubs;
         GatherTargets t;
         for (int k = 0; k < n; ++k) {
             t.bytes[k] = bytes[s0 + k];
             t.lengths[k] = lengths[s0 + k];
         }
         const dim3 grid(z.nslab, z.nrows, n);
-        const int32_t *lens = reinterpret_cast<const int32_t *>(ws + z.lengths);
-        const int64_t *goff = reinterpret_cast<const int64_t *>(ws + z.group_off);
-        if (fused_ok(b))  // which of the two encoders wrote the scratch
-            gather_kernel<Len, true><<<grid, kGroup, 0, st>>>(ws + z.scratch, z.stride, lens, goff, z.nchannels, s0, t);
+        if (fused_ok(jobs[0]))  // which of the two encoders wrote the scratch
+            gather_kernel<Len, true><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
         else
-            gather_kernel<Len, false><<<grid, kGroup, 0, st>>>(ws + z.scratch, z.stride, lens, goff, z.nchannels, s0, t);
+            gather_kernel<Len, false><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
         if (int rc = check_launch()) return rc;
     }
     return CG_OK;
@@ -922,12 +983,23 @@ int launch_gather(const cg_encode_kv_job &b, const Sizes &z, uint8_t *const *byt
 
 extern "C" int cg_encode_kv_gather(const cg_encode_kv_job *job, uint8_t *const *bytes_host, int32_t *const *lengths_host,
                                    void *stream) {
-    if (int rc = check_job(job)) return rc;
+    return cg_encode_kv_levels_gather(job, 1, bytes_host, lengths_host, stream);
+}
+
+extern "C" int cg_encode_kv_levels_gather(const cg_encode_kv_job *jobs, int njobs, uint8_t *const *bytes_host,
+                                          int32_t *const *lengths_host, void *stream) {
+    if (njobs < 1) return CG_E_SHAPE;
+    if (njobs > CG_MAX_ENCODE_LEVELS) return CG_E_CAPACITY;
+    if (!jobs) return CG_E_NULL;
+    for (int j = 0; j < njobs; ++j) {
+        if (int rc = check_job(jobs + j)) return rc;
+        if (!same_chunk(jobs[0], jobs[j])) return CG_E_SHAPE;
+    }
     if (!bytes_host || !lengths_host) return CG_E_NULL;
-    const Sizes z = sizes_of(job->nlayers, job->ntokens, job->nheads, job->head_size);
-    for (int k = 0; k < z.nsub; ++k)
+    const Sizes z = sizes_of(jobs->nlayers, jobs->ntokens, jobs->nheads, jobs->head_size);
+    for (int k = 0; k < z.nsub * njobs; ++k)
         if (!bytes_host[k] || !lengths_host[k]) return CG_E_NULL;
-    return launch_gather<int32_t>(*job, z, bytes_host, reinterpret_cast<void *const *>(lengths_host),
+    return launch_gather<int32_t>(jobs, njobs, z, bytes_host, reinterpret_cast<void *const *>(lengths_host),
                                   static_cast<cudaStream_t>(stream));
 }
 
@@ -975,5 +1047,5 @@ extern "C" int cg_encode_kv_flat(const cg_encode_kv_job *job, const cg_flat_layo
         bytes[k] = f.blob + f.off_payload + f.sub_off_host[k];
         lengths[k] = f.blob + f.off_lengths + k * streams * 2;
     }
-    return launch_gather<uint16_t>(b, z, bytes, lengths, st);
+    return launch_gather<uint16_t>(job, 1, z, bytes, lengths, st);
 }

@@ -310,9 +310,10 @@ def _give_tail(t: torch.Tensor) -> None:
 class _PendingChunk:
     """One chunk whose kernels up to the streams and their offsets are enqueued on `stream` (default: the
     current one), but whose payload size is not yet known on the host.  finish() waits for that and
-    enqueues the gather.  Buffers come from the current stream's pool whatever `stream` is."""
+    enqueues the gather.  Buffers come from the current stream's pool whatever `stream` is.  enqueue=False leaves the
+    launches to _enqueue_levels."""
 
-    def __init__(self, kv, info, max_bins, delta=None, stream=None, workspace=None, with_counts=False):
+    def __init__(self, kv, info, max_bins, delta=None, stream=None, workspace=None, with_counts=False, enqueue=True):
         if kv.dim() != 5 or kv.shape[1] != 2:
             raise RuntimeError(f"expected a KV blob of shape [L, 2, T, H, D], got {tuple(kv.shape)}")
         if kv.dtype not in _DTYPES:
@@ -360,8 +361,9 @@ class _PendingChunk:
             self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
             job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
         try:
-            with on_device(dev):
-                _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
+            if enqueue:
+                with on_device(dev):
+                    _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
             # made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do
             self.lengths = [] if with_counts else [torch.empty((2 * L, H * D), dtype=torch.int32, device=dev)
                                                    for _ in range(self.nsub)]
@@ -370,6 +372,25 @@ class _PendingChunk:
         except BaseException:
             self.abandon()
             raise
+
+    def another(self, info, max_bins):
+        """The same KV at other bins, prepared like this chunk (one without delta coding or counts) and not enqueued."""
+        if info.cpu.numel() != 2 * self.L:
+            raise RuntimeError(f"bins describe {info.cpu.numel() // 2} layers, the KV blob has {self.L}")
+        p = object.__new__(_PendingChunk)
+        p.__dict__.update(self.__dict__)
+        p.tail, dev, dtype, shape = None, self.dev, self.kv.dtype, (self.L, self.T, 1)
+        p.info, p.max_bins, p.bins = info, max_bins, info.on(dev)
+        p.scales_k, p.scales_v = torch.empty(shape, dtype=dtype, device=dev), torch.empty(shape, dtype=dtype, device=dev)
+        p.cdf = torch.empty((2 * self.L, self.H * self.D, max_bins + 1), dtype=torch.int16, device=dev)
+        p.workspace = torch.empty(self.workspace.numel(), dtype=torch.uint8, device=dev)
+        p.lengths = [torch.empty((2 * self.L, self.H * self.D), dtype=torch.int32, device=dev) for _ in range(self.nsub)]
+        p.tail = _take_tail(self.nsub + 4)
+        job = p.job = _lib.EncodeKvJob.from_buffer_copy(self.job)
+        job.bins, job.cdf, job.max_bins = p.bins.data_ptr(), p.cdf.data_ptr(), max_bins
+        job.scales_k, job.scales_v = p.scales_k.data_ptr(), p.scales_v.data_ptr()
+        job.workspace, job.tail = p.workspace.data_ptr(), p.tail.data_ptr()
+        return p
 
     def sizes(self):
         """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
@@ -383,18 +404,24 @@ class _PendingChunk:
             raise RuntimeError("cachegen encode: " + _lib.status_text(bits & ~_lib.CG_S_COUNT_OVERFLOW))
         return host[:self.nsub + 1], bits, host[self.nsub + 2]
 
-    def finish(self) -> CacheGenGPUEncoderOutput:
+    def pieces(self):
+        """Waits for the sizes; a tensor for every sub-chunk's streams (a view would pickle the whole buffer)."""
         offs, _, _ = self.sizes()
-        n, lengths = self.nsub, self.lengths
-        # every sub-chunk in tensors of its own: a view would pickle the whole buffer
-        pieces = [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(n)]
+        return [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(self.nsub)]
+
+    def finish(self) -> CacheGenGPUEncoderOutput:
+        pieces = self.pieces()
         with on_device(self.dev):
             rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), self.pointers(*[t.data_ptr() for t in pieces]),
                                               self.length_pointers, self.stream_ptr)
         _lib.check(rc, "cg_encode_kv_gather")
+        return self.output(pieces)
+
+    def output(self, pieces) -> CacheGenGPUEncoderOutput:
         step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
-        return CacheGenGPUEncoderOutput([CacheGenGPUBytestream(pieces[j], lengths[j], min(step, self.T - j * step))
-                                         for j in range(n)], self.cdf, self.scales_k, self.scales_v, self.H, self.D)
+        return CacheGenGPUEncoderOutput([CacheGenGPUBytestream(piece, lengths, min(step, self.T - j * step))
+                                         for j, (piece, lengths) in enumerate(zip(pieces, self.lengths))],
+                                        self.cdf, self.scales_k, self.scales_v, self.H, self.D)
 
     def abandon(self) -> None:
         """Gives the buffers up after an error: the GPU may still be writing to them, the pinned one among them, which
@@ -475,22 +502,46 @@ def encode_levels(kv: torch.Tensor, levels: list) -> list:
     of (key_bins, value_bins) pairs, the result one CacheGenGPUEncoderOutput per pair, each identical
     to what encode_function gives with those bins.  This is what the reference's adaptation scripts
     store per chunk (one blob per QUANT_LEVEL, run_adaptation.py:61-72) so that config_selection can
-    pick a level per chunk (src/utils.py:294-314).  All levels are enqueued before the host waits for the
-    first one's size."""
+    pick a level per chunk (src/utils.py:294-314).  After the first, up to four
+    levels share one read of the KV and one launch for each step."""
     return _encode_infos(kv, [_BinsInfo(kb, vb) for kb, vb in levels])
 
 
 def _encode_infos(kv, infos) -> list:
     if kv.stride(4) != 1:
         kv = kv.contiguous()
-    pending = []
+    groups, step = [], _lib.CG_MAX_ENCODE_LEVELS
+    # The first setting alone: the GPU works on it while the host prepares the others, about 20 us each (three settings of a
+    # 256-token chunk of 32 layers x 8 heads: 231 us, 247 with all three together, 251 one after the other).
+    slices = [infos[s:e] for s, e in [(0, 1)] + [(s, s + step) for s in range(1, len(infos), step)] if infos[s:e]]
     try:
-        for info in infos:
-            pending.append(_PendingChunk(kv, info, info.table_bins()))
-        return [p.finish() for p in pending]
+        first = None
+        for part in slices:
+            groups.append([])
+            for info in part:
+                groups[-1].append(first.another(info, info.table_bins()) if first else
+                                  _PendingChunk(kv, info, info.table_bins(), enqueue=False))
+                first = first or groups[-1][0]
+            jobs = (_lib.EncodeKvJob * len(groups[-1]))(*[p.job for p in groups[-1]])
+            with on_device(first.dev):
+                _lib.check(first.lib.cg_encode_kv_levels(jobs, len(jobs), first.stream_ptr), "cg_encode_kv_levels")
+        result = []
+        for group in groups:
+            first = group[0]
+            jobs = (_lib.EncodeKvJob * len(group))(*[p.job for p in group])
+            pieces = [p.pieces() for p in group]
+            pointers = ctypes.c_void_p * (len(group) * first.nsub)
+            with on_device(first.dev):
+                rc = first.lib.cg_encode_kv_levels_gather(jobs, len(group), pointers(*[t.data_ptr() for one in pieces for t in one]),
+                                                          pointers(*[t.data_ptr() for p in group for t in p.lengths]),
+                                                          first.stream_ptr)
+            _lib.check(rc, "cg_encode_kv_levels_gather")
+            result += [p.output(one) for p, one in zip(group, pieces)]
+        return result
     finally:
-        for p in pending:
-            p.abandon()
+        for group in groups:
+            for p in group:
+                p.abandon()
 
 
 @_lmcache_nvtx_annotate

@@ -48,6 +48,7 @@ extern "C" {
 /* 128-channel groups (all rows) whose offsets one cluster of blocks can hold */
 #define CG_MAX_OFFSET_GROUPS 96000
 /* sub-chunks one fused decode launch can take */
+#define CG_MAX_ENCODE_LEVELS 4 /* jobs of one cg_encode_kv_levels call */
 #define CG_MAX_DECODE_JOBS 40
 
 /* Table kinds of cg_decode_job.tables.
@@ -294,11 +295,18 @@ typedef struct cg_encode_kv_job {
 /* bytes of cg_encode_kv_job.workspace; CG_E_SHAPE for non-positive extents */
 int64_t cg_encode_kv_workspace(int nlayers, int ntokens, int nheads, int head_size);
 int cg_encode_kv(const cg_encode_kv_job *job_host, void *stream);
+/* The same for one chunk at njobs bin settings (1 .. CG_MAX_ENCODE_LEVELS jobs with the same kv, strides, extents, dtype
+ * and delta_group; everything else their own): the KV is read once and each step is one launch for all of them.
+ * cg_encode_kv_wait job by job. */
+int cg_encode_kv_levels(const cg_encode_kv_job *jobs_host, int njobs, void *stream);
 /* returns when job's tail is complete; CG_E_CUDA if the stream failed before */
 int cg_encode_kv_wait(const cg_encode_kv_job *job_host, void *stream);
 /* bytes_host[j], lengths_host[j]: device buffers of sub-chunk j, tail[j+1] - tail[j] bytes and int32 [2L, C] */
 int cg_encode_kv_gather(const cg_encode_kv_job *job_host, uint8_t *const *bytes_host, int32_t *const *lengths_host,
                         void *stream);
+/* the same for the jobs of a cg_encode_kv_levels call: sub-chunk j of job i at index i * nsub + j */
+int cg_encode_kv_levels_gather(const cg_encode_kv_job *jobs_host, int njobs, uint8_t *const *bytes_host,
+                               int32_t *const *lengths_host, void *stream);
 
 /* A CGB2 container (serde/flat_format.py) filled from an encoded chunk: header, scales, tables of the given kind,
  * uint16 lengths, payload, zero bytes between them. */
