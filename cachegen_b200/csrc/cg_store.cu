@@ -249,12 +249,12 @@ __device__ __forceinline__ void count_symbol(uint32_t addr) {
 }
 
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
-// block (slab, row), thread (channel, part) counts every kParts-th word of its channel.  Bound by instruction issue
-// (75 % of the slots, 9.5 instructions for 32 symbols with the tables): 1,999 tokens of 32 layers x 1,024 channels in 55 us;
-// with 256 or 1,024 threads a block 55 and 67.  The updates alone, one a symbol at 1.7 cycles a warp and SM, would
-// take 24, and the shared memory is busy for a third of the time; 512 blocks are 3.5 an SM, and while a block's 128
-// columns become tables its other 384 threads wait.
-constexpr int kTableThreads = 512, kParts = kTableThreads / kGroup;
+// block (slab, row), thread (channel, part) counts every kParts-th word of its channel, eight words a batch without a
+// condition inside.  1,999 tokens of 32 layers x 1,024 channels take 38 us under counters (3.9 instructions for 32 symbols); 57
+// and 9.4 with a test for the last word at each, and 512 threads a block, of which 384 wait while the 128 columns become
+// tables.  128, 512 and 1,024 threads: 56, 44 and 63 us; 12 and 16 words in flight: 40 and 39.  The updates alone, one a
+// symbol at 1.1 cycles a warp and SM, would take 16.
+constexpr int kTableThreads = 256, kParts = kTableThreads / kGroup;
 struct TableJobs {
     TableOut out[CG_MAX_ENCODE_LEVELS];
     const uint32_t *sym4[CG_MAX_ENCODE_LEVELS];
@@ -280,24 +280,35 @@ __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const __gr
         const uint32_t col = smem_addr(hist + (cl >> 5) * 32 * lp + (cl & 31));
         const uint32_t *p = sym4 + static_cast<int64_t>(row) * words * nchannels + c;
         constexpr int kAhead = 8;  // loads in flight
-        for (int i0 = part; i0 < words; i0 += kParts * kAhead) {
-            uint32_t w[kAhead];
+        const int64_t step = static_cast<int64_t>(kParts) * nchannels;
+        int i = part;
+        p += static_cast<int64_t>(part) * nchannels;
+        for (; i + kParts * (kAhead - 1) < whole; i += kParts * kAhead) {
+            uint32_t w[kAhead], any = 0u;
 #pragma unroll
             for (int j = 0; j < kAhead; ++j) {
-                const int i = i0 + j * kParts;
-                w[j] = i < words ? __ldg(p + static_cast<int64_t>(i) * nchannels) : 0u;
+                w[j] = __ldg(p);
+                p += step;
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) any |= w[j];
+            if (any & 0x80808080u) {  // reported by the coder
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j)
+                    if (w[j] & 0x80808080u) w[j] = 0u;
             }
 #pragma unroll
             for (int j = 0; j < kAhead; ++j) {
-                const int i = i0 + j * kParts;
-                if (w[j] & 0x80808080u) w[j] = 0u;  // reported by the coder
-                if (i < whole) {
-                    #pragma unroll
-                    for (int k = 0; k < 4; ++k) count_symbol(entry_of(col, w[j], k));
-                } else if (i < words) {
-                    for (int k = 0; k < (ntokens & 3); ++k) count_symbol(col + ((w[j] >> (8 * k)) & 0xFFu) * kWarpRow);
-                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) count_symbol(entry_of(col, w[j], k));
             }
+        }
+        for (; i < words; i += kParts) {
+            uint32_t w = __ldg(p);
+            p += step;
+            if (w & 0x80808080u) w = 0u;
+            const int n = i < whole ? 4 : ntokens & 3;
+            for (int k = 0; k < n; ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kWarpRow);
         }
     }
     __syncthreads();
