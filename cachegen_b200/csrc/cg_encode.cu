@@ -19,7 +19,7 @@ struct EncodeParams {
     int32_t *status;
 };
 
-constexpr int kPrefetch = 8;  // symbols fetched ahead of the coder
+constexpr int kPrefetch = 16;  // symbols fetched ahead of the coder
 
 // See store_encode_kernel's encode_again.
 template <class Offset>
@@ -80,27 +80,25 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     };
     const Offset first = at;
     uint32_t buf[kPrefetch], next[kPrefetch];
-    int i = 0;
-#pragma unroll
-    for (int j = 0; j < kPrefetch; ++j) {
-        buf[j] = j < n ? __ldg(base + at) : 0u;
-        at += s1;
-    }
-    for (; i + kPrefetch <= n; i += kPrefetch) {
+    const auto fetch = [&](uint32_t (&to)[kPrefetch]) {
 #pragma unroll
         for (int j = 0; j < kPrefetch; ++j) {
-            next[j] = i + kPrefetch + j < n ? __ldg(base + at) : 0u;
+            to[j] = __ldg(base + at);
             at += s1;
         }
+    };
+    int i = 0;
+    if (kPrefetch <= n) fetch(buf);
+    for (; i + kPrefetch <= n; i += kPrefetch) {
+        if (i + 2 * kPrefetch <= n) fetch(next);
 #pragma unroll
         for (int j = 0; j < kPrefetch; ++j) code(buf[j]);
 #pragma unroll
         for (int j = 0; j < kPrefetch; ++j) buf[j] = next[j];
     }
     for (; i < n; ++i) {
-        code(buf[0]);
-#pragma unroll
-        for (int j = 0; j + 1 < kPrefetch; ++j) buf[j] = buf[j + 1];
+        code(__ldg(base + at));
+        at += s1;
     }
     const uint32_t nbytes = enc[0].unsettled(carried[0]) ? encode_again<Offset>(col, base, first, s1, n, top, p.scratch + slot * p.stride, p.stride)
                                                          : enc[0].flush(out[0]);

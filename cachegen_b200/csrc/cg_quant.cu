@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
     __syncthreads();
     const uint32_t top = static_cast<uint32_t>(max_bins);
     if (VEC) {
-        constexpr int kStep = kQuantThreads / 32, kAhead = 4;
+        constexpr int kStep = kQuantThreads / 32, kAhead = 8;
         const int q = tid & 31, c = c0 + 4 * q;
         uint32_t place[4], pick[4];
 #pragma unroll
@@ -357,20 +357,38 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
             place[k] = smem_addr(hist + 4 * q + e);
             pick[k] = 0x4440u + e;
         }
+        const auto count = [&](uint32_t w, int k) {
+            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(__byte_perm(w, 0u, pick[k]) * kRowBytes + place[k]) : "memory");
+        };
         if (c < nchannels) {
-            const int8_t *p = sym + row * s0 + c;
-            for (int t0 = tid >> 5; t0 < ntokens; t0 += kStep * kAhead) {
-                uint32_t w[kAhead];
+            const int8_t *p = sym + row * s0 + c + (tid >> 5) * s1;
+            const int64_t step = kStep * s1;
+            // a byte is above top if its top bit is set, or becomes set with 127 - top added
+            const uint32_t most = top * 0x01010101u, spare = 0x7F7F7F7Fu - most;
+            int t0 = tid >> 5;
+            for (; t0 + (kAhead - 1) * kStep < ntokens; t0 += kStep * kAhead) {
+                uint32_t w[kAhead], any = 0u;
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) {
+                    w[j] = __ldg(reinterpret_cast<const uint32_t *>(p));
+                    p += step;
+                }
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) any |= w[j] | (w[j] + spare);
+                if (any & 0x80808080u) {
+#pragma unroll
+                    for (int j = 0; j < kAhead; ++j) w[j] = __vminu4(w[j], most);
+                }
 #pragma unroll
                 for (int j = 0; j < kAhead; ++j)
-                    w[j] = t0 + j * kStep < ntokens ? __ldg(reinterpret_cast<const uint32_t *>(p + (t0 + j * kStep) * s1)) : 0u;
 #pragma unroll
-                for (int j = 0; j < kAhead; ++j)
-                    if (t0 + j * kStep < ntokens) {
+                    for (int k = 0; k < 4; ++k) count(w[j], k);
+            }
+            for (; t0 < ntokens; t0 += kStep) {
+                const uint32_t w = __vminu4(__ldg(reinterpret_cast<const uint32_t *>(p)), most);
+                p += step;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(min(__byte_perm(w[j], 0u, pick[k]), top) * kRowBytes + place[k]) : "memory");
-                    }
+                for (int k = 0; k < 4; ++k) count(w, k);
             }
         }
     } else {
