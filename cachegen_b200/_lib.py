@@ -72,7 +72,7 @@ class HostSegment(ctypes.Structure):
 
 
 EXPORTS = [
-    "cg_host_upload", "cg_host_stage", "cg_host_stage_send", "cg_host_stage_end", "cg_host_download", "cg_decode_kv",
+    "cg_host_upload", "cg_host_stage", "cg_host_stage_ahead", "cg_host_stage_send", "cg_host_stage_end", "cg_host_download", "cg_decode_kv",
     "cg_stream_sizes", "cg_decode_packed", "cg_wait_word",
     "cg_encode_kv_workspace", "cg_encode_kv", "cg_encode_kv_levels", "cg_encode_kv_wait", "cg_encode_kv_gather",
     "cg_encode_kv_levels_gather", "cg_encode_kv_flat",
@@ -136,6 +136,7 @@ def lib():
     L.cg_decode_kv.argtypes = [ctypes.POINTER(DecodeJob), i, i, i, i, i, p, i, p, i, i, i64, i64, i64, i64, p, p]
     L.cg_host_upload.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, p]
     L.cg_host_stage.argtypes = [p, i64, p, i64, ctypes.POINTER(p)]
+    L.cg_host_stage_ahead.argtypes = [p, i64, p, i64, p, p, ctypes.POINTER(p)]
     L.cg_host_stage_send.argtypes = [p, ctypes.POINTER(HostSegment), i, p]
     L.cg_host_stage_end.argtypes = [p]
     L.cg_host_download.argtypes = [ctypes.POINTER(HostSegment), i, p, i64, i, p]

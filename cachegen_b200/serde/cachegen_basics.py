@@ -511,6 +511,7 @@ def _load_storage_fast(b):
 
 _NOTHING = contextlib.nullcontext()
 _EARLY_SPARE = 256 << 10  # room behind the byte string for tensors that are not part of it
+_AHEAD_SPARE = 64  # room behind a byte string that is sent as it is
 _EARLY_FROM = 2 << 20  # below, parsing and copying take less time than the threads take to wake
 
 
@@ -533,7 +534,7 @@ class _Staging:
         self.turn = 0
         self.buf = None
         self.waiting = None  # (host view, device tensor) pairs of the load in progress
-        self.early = None    # (handle, address, size) of a byte string whose copy runs ahead of its parsing
+        self.early = None    # (handle, address, size, _Ahead or None) of a byte string whose copy runs ahead of its parsing
         self.fetched = None  # the tensors whose transfers into the chosen buffer are on their way, and their stream
         self.fetching = None
 
@@ -573,22 +574,34 @@ class _Staging:
         self.waiting.append((view_cpu.data_ptr(), view_cpu.numel(), out, view_cpu))
         return out
 
-    def start(self, bs: bytes) -> None:
+    def start(self, bs: bytes, ahead: bool = False) -> None:
         """Has the helper threads copy a byte string that is about to be parsed, from _EARLY_FROM bytes on: parsing a
-        blob takes 130 us, as long as a quarter of its 30 MB take over the bus, and waking the threads 50."""
+        blob takes 130 to 200 us, as long as a third of its 30 MB take over the bus, and waking the threads 50.
+        ahead: one of them sends it to the current GPU as well, on the current stream, and the tensors are cut out of it
+        there (a 256-token chunk to pickled bytes and back 2,070 -> 1,940 us; several blobs after each other keep the bus
+        busy as it is)."""
         if len(bs) < _EARLY_FROM or not torch.cuda.is_available():
             return
+        device = torch.device("cuda", torch.cuda.current_device())
+        on, raw = torch.cuda.current_stream(device), None
+        if ahead and not torch.cuda.is_current_stream_capturing():
+            try:
+                raw = torch.empty(len(bs) + _AHEAD_SPARE, dtype=torch.uint8, device=device)
+            except torch.cuda.OutOfMemoryError:
+                pass  # the tensors alone may fit
         self.begin(len(bs) + _EARLY_SPARE)
-        handle = ctypes.c_void_p()
-        at = _bytes_at(bs)
-        rc = _lib.lib().cg_host_stage(at, len(bs), self.buf.data_ptr(), self.buf.numel(), ctypes.byref(handle))
-        _lib.check(rc, "cg_host_stage")
-        self.early = (handle, at, len(bs))
+        handle, at = ctypes.c_void_p(), _bytes_at(bs)
+        lib, args = _lib.lib(), (at, len(bs), self.buf.data_ptr(), self.buf.numel())
+        if raw is None:
+            _lib.check(lib.cg_host_stage(*args, ctypes.byref(handle)), "cg_host_stage")
+        else:
+            _lib.check(lib.cg_host_stage_ahead(*args, raw.data_ptr(), on.cuda_stream, ctypes.byref(handle)), "cg_host_stage_ahead")
+        self.early = (handle, at, len(bs), None if raw is None else (raw, device, on))
 
     def _send_early(self, pairs: list, stream) -> list:
         """Sends the tensors that lie in the byte string of `start`, and small ones beside it (a blob's scales: the
         unpickler copies short streams), if they are on one GPU; returns the others."""
-        handle, at, size = self.early
+        handle, at, size, ahead = self.early
         mine, others, spare = [], [], _EARLY_SPARE - 256
         for p in pairs:
             if not at <= p[0] < at + size:
@@ -600,6 +613,8 @@ class _Staging:
         try:
             if not mine or any(p[2].device != mine[0][2].device for p in mine):
                 return pairs
+            if ahead is not None and (mine[0][2].device != ahead[1] or self._stream_for(ahead[1], stream) != ahead[2]):
+                return pairs  # it went elsewhere
             segs = (_lib.HostSegment * len(mine))(*[(a, o.data_ptr(), n) for a, n, o, _ in mine])
             self._send(lambda on: _lib.lib().cg_host_stage_send(handle, segs, len(mine), on), mine[0][2].device, stream)
         finally:
@@ -609,21 +624,32 @@ class _Staging:
     def finish(self) -> None:
         """Ends a `start` whose bytes are not wanted (any more)."""
         if self.early is not None:
-            handle, self.early = self.early[0], None
+            (handle, _, _, ahead), self.early = self.early, None
             _lib.lib().cg_host_stage_end(handle)
+            if ahead is not None:  # transfers that were begun still read the buffer, wanted or not
+                self._mark(ahead[1], ahead[2])
             self.end()
+
+    @staticmethod
+    def _stream_for(device, stream):
+        return torch.cuda.current_stream(device) if stream is None or stream.device != device else stream
+
+    def _mark(self, device, on) -> None:
+        """Notes that copies from the chosen buffer may be on this stream."""
+        if self.events[self.turn] is None or self.events[self.turn][0] != device:
+            self.events[self.turn] = (device, torch.cuda.Event())
+        with on_device(device):
+            self.events[self.turn][1].record(on)
+        self.leaving[self.turn] = True
 
     def _send(self, upload, device, stream) -> None:
         """Runs an upload from the chosen buffer on `stream`, if it is one of the device's, or its current one."""
         with on_device(device):
-            on = torch.cuda.current_stream(device) if stream is None or stream.device != device else stream
-            if self.events[self.turn] is None or self.events[self.turn][0] != device:
-                self.events[self.turn] = (device, torch.cuda.Event())
+            on = self._stream_for(device, stream)
             try:
                 rc = upload(on.cuda_stream)
             finally:
-                self.events[self.turn][1].record(on)
-                self.leaving[self.turn] = True
+                self._mark(device, on)
         _lib.check(rc, "cg_host_upload")
 
     def send(self, pairs: list = None, stream=None) -> None:
@@ -896,7 +922,7 @@ def load_blob(bs):
     st.open()
     try:
         if isinstance(bs, bytes):
-            st.start(bs)
+            st.start(bs, ahead=True)
         eo = _unpickle(bs)
         st.send()
     finally:

@@ -469,6 +469,11 @@ int cg_host_download(const cg_host_segment *segments_host, int nsegments, void *
  * must stay until then, `staging` until the stream has passed the segments' transfers.
  */
 int cg_host_stage(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void **handle_host);
+/* The same, and one of the threads sends the whole string to `device_copy`, memory of the current device with 16 bytes
+ * to spare behind the string, on `stream`, as it is copied.  cg_host_stage_send, on the same stream, then takes the segments
+ * from there.  When cg_host_stage_end has returned, transfers that were begun may still be on the stream. */
+int cg_host_stage_ahead(const void *host, int64_t bytes, void *staging, int64_t staging_bytes, void *device_copy, void *stream,
+                        void **handle_host);
 int cg_host_stage_send(void *handle_host, const cg_host_segment *segments_host, int nsegments, void *stream);
 int cg_host_stage_end(void *handle_host);
 
