@@ -36,6 +36,27 @@ int allow_smem(K kernel, size_t bytes) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMostDynamicSmem));
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
+// ---- launches that overlap the one in front (programmatic dependent launch) ----------------------------------
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// early: the blocks may start before the launch in front has ended; they call wait_for_launch_before before they touch what
+// it reads or writes
+template <class... Args>
+int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    return e == cudaSuccess ? CG_OK : set_cuda_error(e);
+}
+
 // cg_tables.cu: group offsets of sparse tables, and the tables in one pass once those are known
 int launch_sparse_write(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
                         const uint32_t *group_off, void *masks, const int64_t *mask_row_off, uint8_t *out,
@@ -184,12 +205,13 @@ __device__ __forceinline__ int block_exclusive_scan_128(int v, int *warp_sums, i
 // lane shifts its words to the byte they start at and puts them together in shared memory (a word that two
 // streams share by an atomic or), and the warp writes the run with 128-bit stores.  Copying stream after stream
 // to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
-// with words assembled from two source words 24 us: one short dependent copy after the other.
+// with words assembled from two source words 24 us: one short dependent copy after the other.  Twelve loads in flight and
+// 5 KB of shared memory a warp 15.6 us under counters, eight and 6 KB 17.2.
 // src: the stream's first word, its words STEP words apart, read-only for the launch; dst0: where the group's
 // streams go; pairs: (STEP 1) the words can be read in pairs, to the end of the last one.  Whatever the row holds behind
 // its stream: the last word is cut to the stream's bytes, since what it shares a word with there is the next stream (and
 // behind the run's last stream the next warp's stage).
-constexpr int kGatherWords = 1536;  // words of shared memory a warp; longer runs take the lanes' own byte stores
+constexpr int kGatherWords = 1280;  // words of shared memory a warp; longer runs take the lanes' own byte stores
 template <int STEP>
 __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t *dst0, bool pairs = false) {
     __shared__ uint4 stage[kGroup / 32][kGatherWords / 4];
@@ -214,7 +236,7 @@ __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t
     const uint32_t sh = static_cast<uint32_t>(o & 3) * 8u;
     const uint32_t last_bytes = 0xFFFFFFFFu >> ((-len & 3) * 8);  // of the last word
     const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
-    constexpr int kAhead = 8;  // loads in flight
+    constexpr int kAhead = 12;  // loads in flight
     uint32_t prev = 0u;
     for (int k0 = 0; k0 < most; k0 += kAhead) {
         uint32_t x[kAhead];

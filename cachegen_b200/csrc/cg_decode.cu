@@ -17,8 +17,6 @@ __host__ __device__ inline int table_rows(int lp, int levels) {
 // reading them runs beside that launch.  kAfterBatch: another batch of the same call, on which it does not depend,
 // so that its blocks fill what that one's last wave leaves idle; it only must not end first.
 enum DecodeAfter { kAfterOffsets = 0, kAfterBatch = 1 };
-__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A group offset that the launch in front wrote, behind the wait for it (in a later batch: that launch had ended when the
 // first batch's blocks let this one start).  From the L2: __ldg is for data that nothing writes while the kernel runs, and
 // these blocks may start while that launch still does.
@@ -619,23 +617,6 @@ static size_t table_bytes(int lp, int levels) {
     return static_cast<size_t>(table_rows(lp, levels) + 1) * kRowBytes;  // +1: the row read past the last symbol
 }
 static_assert((CG_MAX_LP + 1) * kRowBytes + 4 * (kSubTokens + 2 * CG_MAX_LP) + 64 <= kSmemByItself, "a decoder block's shared memory");
-
-// early: the blocks may start before the launch in front has ended (see DecodeAfter)
-template <class... Args>
-static int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = early ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-    return e == cudaSuccess ? CG_OK : set_cuda_error(e);
-}
 
 // Instantiated search depths: 3..6, whatever the table length.
 template <int MODE>

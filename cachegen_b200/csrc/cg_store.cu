@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const 
     __shared__ float4 factor_s[ONE ? 1 : CG_MAX_ENCODE_LEVELS];
     __shared__ uint32_t keep_s;
     const int nlevels = ONE ? 1 : q.n;
+    let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.y, t0 = blockIdx.x * kTokensPerWord;
     const int C = v.nheads * v.head_size, c = tid * 8;
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
         uint16_t *stage = reinterpret_cast<uint16_t *>(tab + p.lp * kGroup);
         bool overflow = false;
         for (int m = 0; m < p.lp; ++m) mine[m * 32] = 0u;
+        wait_for_launch_before();
         constexpr int kAhead = 16;  // words in flight
         const uint32_t *q = sp[0];
         int i = 0;
@@ -525,6 +527,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
         const int first = blockIdx.x * kGroup + warp * 32, nch = min(32, p.nchannels - first);
         copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp, nch * p.lp, lane);
     } else if (any_active) {
+        wait_for_launch_before();
 #pragma unroll
         for (int s = 0; s < NS; ++s) stage_encode_column<32>(column[s], p.out.cdf + g[s] * p.lp, p.lp, 0);
     }
@@ -616,6 +619,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
         if (bits) atomicOr(p.status, bits);
     }
 
+    wait_for_launch_before();  // warps without channels
     // group sizes, and whose turn it is to make offsets of them
     const int sum = __reduce_add_sync(0xFFFFFFFFu, nbytes);
     const int nz_sum = TABLES && p.out.group_nz ? __reduce_add_sync(0xFFFFFFFFu, nz) : 0;
@@ -698,8 +702,8 @@ struct GatherJobs {
     int nsub;
 };
 
-// The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  14.5 us a 256-token
-// Llama-7B chunk (11.8 MB out of scratch that is read in full lines), 20 before.
+// The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  15.6 us under
+// counters a 256-token Llama-7B chunk (11.8 MB out of scratch that is read in full lines).
 template <class Len, bool INTERLEAVED>
 __global__ void __launch_bounds__(kGroup) gather_kernel(const __grid_constant__ GatherJobs jobs, int64_t stride, int nchannels, int first,
                                                         const __grid_constant__ GatherTargets out) {
@@ -851,9 +855,14 @@ static int encode_separately(const cg_encode_kv_job &b, cudaStream_t st) {
     return check_launch();
 }
 
-extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) { return cg_encode_kv_levels(job, 1, stream); }
+static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void *stream);
 
-extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void *stream) {
+extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) { return encode_jobs(job, 1, true, stream); }
+
+extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void *stream) { return encode_jobs(jobs, njobs, false, stream); }
+
+// alone: no other encode follows at once on the stream
+static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void *stream) {
     if (njobs < 1) return CG_E_SHAPE;
     if (njobs > CG_MAX_ENCODE_LEVELS) return CG_E_CAPACITY;
     if (!jobs) return CG_E_NULL;
@@ -926,15 +935,19 @@ extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void
     if (int rc = check_launch()) return rc;
     const dim3 grid(z.nslab, z.nrows, z.nsub * njobs);
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
+    // The coder of one sub-chunk starts under the quantiser's last blocks: 206 -> 203 us for a 256-token Llama-7B chunk.  Not
+    // where another quantiser follows at once, which then starts late (three quality levels 262 -> 285 us), and not behind or in
+    // front of the tables' kernel (1,999 tokens in one call 415 -> 420).
+    const bool early = alone && z.nsub == 1;
     const auto store = [&](auto kernel, int threads, size_t smem) {
         if (int rc = allow_smem(kernel, smem)) return rc;
-        kernel<<<grid, threads, smem, st>>>(store_jobs);
-        return check_launch();
+        return launch(kernel, grid, threads, smem, early, st, store_jobs);
     };
     if (z.nsub == 1) return store(store_encode_kernel<true, 1, 2>, kGroup, columns + staged);
     if (int rc = allow_smem(packed_tables_kernel, columns + staged)) return rc;
-    packed_tables_kernel<<<dim3(z.nslab, z.nrows, njobs), kTableThreads, columns + staged, st>>>(table_jobs, b.ntokens, z.nchannels);
-    if (int rc = check_launch()) return rc;
+    if (int rc = launch(packed_tables_kernel, dim3(z.nslab, z.nrows, njobs), kTableThreads, columns + staged, false, st, table_jobs,
+                        static_cast<int>(b.ntokens), static_cast<int>(z.nchannels)))
+        return rc;
     if (!store_jobs.job[0].high_water) return store(store_encode_kernel<false, 1, 1>, kGroup, columns);
     // two streams a thread unless the last group has channels for the first alone
     const int last = z.nchannels % kGroup;
