@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
 }
 
 // The same with two adjacent channels per thread, whose symbols are adjacent bytes (see decode_dequant_multi_kernel):
-// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk: 164 us, 182 with a thread per channel.
+// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk: 168 us under counters, of which the last 272 of
+// 2,048 blocks, which find no room beside the first, take a third.
 // Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
 // more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
 constexpr int kMultiBlocksPerSM = 12;
@@ -185,6 +186,16 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         stage_table_column<true>(tab, p.cdf + g * p.lp, p.lp, rows, tid);
         stage_table_column<true>(tab, p.cdf + (g + 1) * p.lp, p.lp, rows, tid + kThreads);
     }
+    // One search step less where the upper half of the table holds next to nothing, in every channel of the block: the rows of
+    // half the bins in a table made for all rows (52 of 64 of a Llama-7B chunk), whose symbols there have one share of 2^16
+    // each.  Such a symbol takes the exact search.  175 -> 168 us under counters.
+    constexpr uint32_t kHalf = 1u << (LEVELS - 1);
+    bool upper = false;
+    if (LEVELS > 3 && active && p.lp - 1 > static_cast<int>(kHalf)) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) upper |= entry_c16(tab[kHalf * kGroup + tid + i * kThreads]) < (0x10000u - 2u * kHalf) << 16;
+    }
+    const bool shallow = LEVELS > 3 && !__syncthreads_or(upper);
     if (!active) return;  // a thread reads its own columns only
     bool bad = false;
     const uint8_t *streams[2];
@@ -208,7 +219,8 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         *reinterpret_cast<uint16_t *>(o) = static_cast<uint16_t>((a[0] - col[0]) / kRowBytes | (a[1] - col[1]) / kRowBytes << 8);
         o += o1;
     };
-    decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
+    if (shallow) decode_streams<(LEVELS > 3 ? LEVELS - 1 : LEVELS), 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
+    else decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
 }
 
 // ---- one warp per stream (kept for comparison) -------------------------------------------------------------
