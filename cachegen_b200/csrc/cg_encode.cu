@@ -36,7 +36,7 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint8_t
     return enc.flush(out);
 }
 
-// Bound by instruction issue: one 256-token Llama-7B chunk in 116 us under counters, 125 before the loop without rare cases and
+// Bound by instruction issue: one 256-token Llama-7B chunk in 109 us under counters, 125 before the loop without rare cases and
 // with symbols fetched a group ahead of the coder (three of eight stall cycles were loads).
 // NARROW: the symbols of a row lie within 4 GB of its first, so that a symbol's address is a 32-bit offset
 template <bool NARROW>

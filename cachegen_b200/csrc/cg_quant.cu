@@ -330,9 +330,10 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_cdf_kernel(
 
 // calculate_cdf on int8 symbols: grid (nslab, nrows).  VEC: adjacent channels are adjacent bytes at 4-byte
 // boundaries, and a thread counts four channels of every eighth token, with one load for four symbols and
-// four tokens in flight; the lanes of a warp start their counts at different ones of their four channels so that they
-// hit 32 banks.  Bound by issue and the latencies of its loads and barriers (67 % of the issue slots, integer pipe 55 %;
-// the updates alone would take 12 us): one 256-token Llama-7B chunk in 37 us, 62 with a load per symbol.  Otherwise
+// eight tokens in flight; the lanes of a warp start their counts at different ones of their four channels so that they
+// hit 32 banks.  Bound by issue and the latencies of its loads and barriers (70 % of the issue slots, integer pipe 50 %;
+// the updates alone would take 12 us): one 256-token Llama-7B chunk in 28 us, 36 with a condition at every load, 62 with a load
+// per symbol.  Otherwise
 // (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
 template <bool VEC>
 __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t *__restrict__ sym, int64_t s0,

@@ -434,12 +434,12 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint32_
 // second read comes from the L2.  Otherwise the tables come from packed_tables_kernel.
 // The last block of a sub-chunk turns the group sizes into offsets, the last of all writes the tail.
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
-// chunk takes 112 us with its tables under counters, 0.60 T symbols/s, 37.2 instructions for 32 symbols; 122 us and 40.4 with
-// the code for rare cases inside the loop and a vote a symbol.  Eight blocks an SM leave the compiler 64
+// chunk takes 107 us with its tables under counters, 0.63 T symbols/s, 34.6 instructions for 32 symbols; 122 us and 40.4 with
+// the code for rare cases inside the loop, a mask kept as the interval's size and a vote a symbol.  Eight blocks an SM leave the compiler 64
 // registers.  (Seven, for two even waves of a chunk's 2,048 blocks, were better while a block took longer: 207 against 205 us a
 // whole encode now.)
 // Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
-// channels in 166 us under counters (29.9 instructions for 32 symbols), 172 before the same change; 180 with one stream.
+// channels in 164 us under counters (28.5 instructions for 32 symbols), 172 before the same change; 180 with one stream.
 // G symbols a vote: two, unless the table may give a symbol more bits than the accumulator has room for twice (pair_high_water:
 // more than 21,824 tokens in one call).  The tables' part wants the warps more than the chains (a 256-token chunk
 // 129 us with two), so it keeps one; and so does a last group of channels that would leave the second without work.
@@ -935,7 +935,7 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
     if (int rc = check_launch()) return rc;
     const dim3 grid(z.nslab, z.nrows, z.nsub * njobs);
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
-    // The coder of one sub-chunk starts under the quantiser's last blocks: 206 -> 203 us for a 256-token Llama-7B chunk.  Not
+    // The coder of one sub-chunk starts under the quantiser's last blocks: 206 -> 202 us for a 256-token Llama-7B chunk.  Not
     // where another quantiser follows at once, which then starts late (three quality levels 262 -> 285 us), and not behind or in
     // front of the tables' kernel (1,999 tokens in one call 415 -> 420).
     const bool early = alone && z.nsub == 1;
