@@ -293,6 +293,6 @@ __device__ __forceinline__ float half_bits_to_float(uint16_t b, int dtype) {
 }
 
 // Cq of do_dequantize / MAX of torch_quant_vectorized: bins // 2 - 1 on a float tensor.
-__device__ __forceinline__ float half_range(float bins) { return __fsub_rn(floorf(__fdiv_rn(bins, 2.0f)), 1.0f); }
+__device__ __forceinline__ float half_range(float bins) { return __fsub_rn(floorf(__fmul_rn(bins, 0.5f)), 1.0f); }
 
 }  // namespace cg

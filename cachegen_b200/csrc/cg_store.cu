@@ -45,8 +45,10 @@ __device__ __forceinline__ void quantize2(float x0, float x1, float f, uint64_t 
 // Pass 1.  A block takes four tokens of one row, all channels, eight adjacent ones a thread: the 16-bit values stay in
 // registers between the scales (a reduction over the block) and the symbols, so the KV is read once where an
 // absmax pass and a quantise pass read it twice, and four tokens' symbols of a channel leave as one word.  Bound
-// by memory and by about as much issue: a 256-token Llama-7B chunk (134 MB in, 67 MB of symbols out) takes 40 us,
-// 5.0 TB/s, where the two passes took 31 + 61 us (the second with the histogram, which the coder does now).
+// by memory and by about as much issue: a 256-token Llama-7B chunk (134 MB in, 67 MB of symbols out) takes 38 us,
+// 5.3 TB/s, where the two passes took 31 + 61 us (the second with the histogram, which the coder does now).  9.3 instructions
+// for 32 symbols; with the layer and the half of the pair divided out of one grid dimension, the bins halved by a division and
+// every word zeroed before it is loaded 11.6, 40 us, and 63 where 1,999 tokens of 32 layers x 1,024 channels take 58.
 // Three blocks of 512 threads an SM (42 registers a thread) keep enough loads in flight; more than 4,096
 // channels need one block of up to 1,024 threads.
 // The same KV at several bin settings takes one read and one reduction: only the quantisation is done for each.
@@ -68,21 +70,23 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const 
     const int nlevels = ONE ? 1 : q.n;
     let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row = blockIdx.y, t0 = blockIdx.x * kTokensPerWord;
+    const int layer = blockIdx.y, kv = blockIdx.z, row = kv * v.nlayers + layer, t0 = blockIdx.x * kTokensPerWord;
     const int C = v.nheads * v.head_size, c = tid * 8;
-    const int layer = row % v.nlayers, kv = row / v.nlayers;
     if (row == 0 && blockIdx.x == 0)  // the counters of the launches after this one
         for (int l = 0; l < nlevels; ++l)
             for (int i = tid; i < q.nzeroed; i += blockDim.x) q.level[l].zeroed[i] = 0u;
     uint4 x[kTokensPerWord];
+    const int h = static_cast<int>(__umulhi(static_cast<uint32_t>(c), v.head_inv));
+    const uint16_t *p = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token + h * v.s_head + (c - h * v.head_size);
+    if (c < C && t0 + kTokensPerWord <= v.ntokens) {
 #pragma unroll
-    for (int j = 0; j < kTokensPerWord; ++j) x[j] = make_uint4(0u, 0u, 0u, 0u);
-    if (c < C) {
-        const int h = static_cast<int>(__umulhi(static_cast<uint32_t>(c), v.head_inv));
-        const uint16_t *p = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token + h * v.s_head + (c - h * v.head_size);
+        for (int j = 0; j < kTokensPerWord; ++j) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+    } else {
 #pragma unroll
-        for (int j = 0; j < kTokensPerWord; ++j)
-            if (t0 + j < v.ntokens) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+        for (int j = 0; j < kTokensPerWord; ++j) {
+            x[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (c < C && t0 + j < v.ntokens) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+        }
     }
     // |x| as an ordered integer: 16-bit float magnitudes compare like their bit patterns
     uint32_t m[kTokensPerWord];
@@ -919,7 +923,7 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
         table_jobs.lp[j] = p.lp;
         lp = p.lp > lp ? p.lp : lp;
     }
-    const dim3 qgrid(static_cast<unsigned>(z.words), z.nrows);
+    const dim3 qgrid(static_cast<unsigned>(z.words), static_cast<unsigned>(jobs->nlayers), 2);
     const int qthreads = (z.nchannels / 8 + 31) / 32 * 32;
 #define CG_LAUNCH_QT(DT, THREADS, BLOCKS)                                                                    \
     njobs == 1 ? quantize_tokens_kernel<DT, THREADS, BLOCKS, true><<<qgrid, qthreads, 0, st>>>(v, q)          \
