@@ -869,6 +869,28 @@ static int encode_separately(const cg_encode_kv_job &b, cudaStream_t st) {
     return check_launch();
 }
 
+// Shared memory to ask for so that a grid of less than one wave is spread over all SMs.  Blocks that start under the launch in
+// front go where that launch's blocks end, up to the eight that fit on an SM, and leave the SMs that end later without any; with
+// room for no more than their share of the grid on each, they cannot.  The quantiser and the coder of 256-token chunks, us a
+// chunk, with eight blocks an SM and so:
+//     10 layers x 8 heads (160 blocks) 66 -> 32    16 x 8 (256) 69 -> 33    32 x 8 (512) 72 -> 47    40 x 8 (640) 74 -> 56
+//     32 x 12 (768) 77 -> 66                       32 x 16 (1,024) 84 -> 78
+// (one after the other 34, 36, 49, 56, 67 and 79).  Beside chunks on other streams, whose blocks find less room then, it gives
+// and takes: twelve chunks by encode_many, 40 x 8 648 -> 610, 32 x 12 694 -> 702, 32 x 16 883 -> 886.  From one wave on there is nothing to spread, and evening the waves out does
+// not pay: 80 x 8 (1,280 blocks) takes 96 us as it is, 95 at five and at six an SM; 40 x 32 (2,560) 174, and 180 and 176.
+static size_t spread_smem(int64_t blocks, size_t dynamic) {
+    constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024, kMostResident = 8;  // bytes of an SM, of each block; launch bounds
+    const int64_t fit = kSmemPerSM / (static_cast<int64_t>(dynamic) + kMostStaticSmem + kReserved);
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return dynamic;
+    const int64_t share = (blocks + sms - 1) / sms;
+    if (share >= (fit < kMostResident ? fit : kMostResident)) return dynamic;
+    // the least that keeps one more out, so that the first of them find room beside the launch in front
+    const size_t least = static_cast<size_t>(kSmemPerSM / (share + 1) - kReserved + 256);
+    return least > dynamic ? least : dynamic;
+}
+
 static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void *stream);
 
 extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) { return encode_jobs(job, 1, true, stream); }
@@ -954,6 +976,7 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
     // front of the tables' kernel (1,999 tokens in one call 415 -> 420).
     const bool early = alone && z.nsub == 1;
     const auto store = [&](auto kernel, int threads, size_t smem) {
+        if (early) smem = spread_smem(static_cast<int64_t>(grid.x) * grid.y * grid.z, smem);
         if (int rc = allow_smem(kernel, smem)) return rc;
         return launch(kernel, grid, threads, smem, early, st, store_jobs);
     };
