@@ -206,33 +206,24 @@ __device__ __forceinline__ int block_exclusive_scan_128(int v, int *warp_sums, i
 // streams share by an atomic or), and the warp writes the run with 128-bit stores.  Copying stream after stream
 // to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
 // with words assembled from two source words 24 us: one short dependent copy after the other.  Twelve loads in flight and
-// 5 KB of shared memory a warp 15.6 us under counters, eight and 6 KB 17.2.
+// 5 KB of shared memory a warp 15 us under counters, eight and 6 KB 17.
 // src: the stream's first word, its words STEP words apart, read-only for the launch; dst0: where the group's
 // streams go; pairs: (STEP 1) the words can be read in pairs, to the end of the last one.  Whatever the row holds behind
 // its stream: the last word is cut to the stream's bytes, since what it shares a word with there is the next stream (and
 // behind the run's last stream the next warp's stage).
-constexpr int kGatherWords = 1280;  // words of shared memory a warp; longer runs take the lanes' own byte stores
+constexpr int kGatherWords = 1280;  // words of shared memory a warp
+
+// The streams of some lanes, `total` bytes that go to dst on, through the warp's shared memory.  at: where the lane's own
+// stream starts among them, 0 with a len of 0 for the lanes that have no part in it.
 template <int STEP>
-__device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t *dst0, bool pairs = false) {
-    __shared__ uint4 stage[kGroup / 32][kGatherWords / 4];
-    __shared__ int warp_sums[kGroup / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
-    const int first = __shfl_sync(0xFFFFFFFFu, excl, 0);
-    const int total = __shfl_sync(0xFFFFFFFFu, excl + len, 31) - first;
-    uint8_t *dst = dst0 + first;
+__device__ __forceinline__ void gather_lanes(uint4 *stage, const uint32_t *src, int len, int at, uint8_t *dst, int total, int lane, bool pairs) {
     const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 15u);
     const int nw = (len + 3) >> 2;
-    if (mis + total > kGatherWords * 4) {
-        uint8_t *d = dst + (excl - first);
-        for (int k = 0; k < len; ++k) d[k] = static_cast<uint8_t>(__ldg(src + (k >> 2) * STEP) >> (8 * (k & 3)));
-        return;
-    }
-    uint32_t *st = reinterpret_cast<uint32_t *>(stage[warp]);
+    uint32_t *st = reinterpret_cast<uint32_t *>(stage);
     const int units = (mis + total + 15) >> 4;
-    for (int i = lane; i < units; i += 32) stage[warp][i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = lane; i < units; i += 32) stage[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
-    const int o = mis + excl - first, w = o >> 2;
+    const int o = mis + at, w = o >> 2;
     const uint32_t sh = static_cast<uint32_t>(o & 3) * 8u;
     const uint32_t last_bytes = 0xFFFFFFFFu >> ((-len & 3) * 8);  // of the last word
     const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
@@ -270,10 +261,41 @@ __device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t
     uint4 *d16 = reinterpret_cast<uint4 *>(dst - mis);
     for (int i = lane; i < units; i += 32) {
         if (i * 16 >= mis && i * 16 + 16 <= mis + total) {
-            d16[i] = stage[warp][i];
+            d16[i] = stage[i];
         } else {
-            const uint8_t *b = reinterpret_cast<const uint8_t *>(stage[warp]);
+            const uint8_t *b = reinterpret_cast<const uint8_t *>(stage);
             for (int k = max(i * 16, mis); k < min(i * 16 + 16, mis + total); ++k) (dst - mis)[k] = b[k];
+        }
+    }
+}
+
+// A run that does not fit goes in parts of sixteen or of eight streams (of 319 and of 638 bytes on average), and what does not fit
+// then byte by byte.  Uniform values at 36 bins, 161 bytes a stream, 32 layers x 32 heads x 256 tokens: 30 us (19 at 159 bytes, in
+// one part), 375 byte by byte; row after row 46 and 406.  6 KB a warp take runs of 192 bytes a stream in one part, 20 us, but leave
+// room for nine blocks an SM instead of ten: 2,000 tokens of 80 layers x 8 heads, 57 bytes a stream, take 59.9 us instead of 57.6
+// (and so they do at the 56 registers a thread that the compiler takes by itself).
+template <int STEP>
+__device__ __forceinline__ void gather_run(const uint32_t *src, int len, uint8_t *dst0, bool pairs = false) {
+    __shared__ uint4 stage[kGroup / 32][kGatherWords / 4];
+    __shared__ int warp_sums[kGroup / 32];
+    constexpr int kFits = kGatherWords * 4 - 15;  // whatever byte they start at
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int excl = block_exclusive_scan_128(len, warp_sums, tid, nullptr);
+    const int first = __shfl_sync(0xFFFFFFFFu, excl, 0), end = __shfl_sync(0xFFFFFFFFu, excl + len, 31);
+    if (end - first <= kFits) {
+        gather_lanes<STEP>(stage[warp], src, len, excl - first, dst0 + first, end - first, lane, pairs);
+        return;
+    }
+    const int middle = __shfl_sync(0xFFFFFFFFu, excl, 16), part = middle - first <= kFits && end - middle <= kFits ? 16 : 8;
+#pragma unroll 1
+    for (int l = 0; l < 32; l += part) {
+        const int from = __shfl_sync(0xFFFFFFFFu, excl, l), to = __shfl_sync(0xFFFFFFFFu, excl + len, l + part - 1);
+        const bool mine = lane >= l && lane < l + part;
+        if (to - from <= kFits) {
+            __syncwarp();  // the part before has been read
+            gather_lanes<STEP>(stage[warp], src, mine ? len : 0, mine ? excl - from : 0, dst0 + from, to - from, lane, pairs);
+        } else if (mine) {
+            for (int k = 0; k < len; ++k) dst0[excl + k] = static_cast<uint8_t>(__ldg(src + (k >> 2) * STEP) >> (8 * (k & 3)));
         }
     }
 }

@@ -716,10 +716,11 @@ struct GatherJobs {
     int nsub;
 };
 
-// The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  15.6 us under
-// counters a 256-token Llama-7B chunk (11.8 MB out of scratch that is read in full lines).
+// The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  15 us under
+// counters a 256-token Llama-7B chunk (11.8 MB out of scratch that is read in full lines).  Ten blocks an SM are what the
+// shared memory allows (see gather_run).
 template <class Len, bool INTERLEAVED>
-__global__ void __launch_bounds__(kGroup) gather_kernel(const __grid_constant__ GatherJobs jobs, int64_t stride, int nchannels, int first,
+__global__ void __launch_bounds__(kGroup, 10) gather_kernel(const __grid_constant__ GatherJobs jobs, int64_t stride, int nchannels, int first,
                                                         const __grid_constant__ GatherTargets out) {
     const int job = (first + blockIdx.z) / jobs.nsub;  // sub-chunk after sub-chunk, job after job
     const uint8_t *scratch = jobs.scratch[job];
@@ -876,8 +877,9 @@ static int encode_separately(const cg_encode_kv_job &b, cudaStream_t st) {
 //     10 layers x 8 heads (160 blocks) 66 -> 32    16 x 8 (256) 69 -> 33    32 x 8 (512) 72 -> 47    40 x 8 (640) 74 -> 56
 //     32 x 12 (768) 77 -> 66                       32 x 16 (1,024) 84 -> 78
 // (one after the other 34, 36, 49, 56, 67 and 79).  Beside chunks on other streams, whose blocks find less room then, it gives
-// and takes: twelve chunks by encode_many, 40 x 8 648 -> 610, 32 x 12 694 -> 702, 32 x 16 883 -> 886.  From one wave on there is nothing to spread, and evening the waves out does
-// not pay: 80 x 8 (1,280 blocks) takes 96 us as it is, 95 at five and at six an SM; 40 x 32 (2,560) 174, and 180 and 176.
+// and takes: twelve chunks by encode_many, 40 x 8 648 -> 610, 32 x 12 694 -> 702, 32 x 16 883 -> 886.  From one wave on there
+// is nothing to spread, and evening the waves out does not pay: 80 x 8 (1,280 blocks) takes 96 us as it is, 95 at five and at six an SM;
+// 40 x 32 (2,560) 174, and 180 and 176.
 static size_t spread_smem(int64_t blocks, size_t dynamic) {
     constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024, kMostResident = 8;  // bytes of an SM, of each block; launch bounds
     const int64_t fit = kSmemPerSM / (static_cast<int64_t>(dynamic) + kMostStaticSmem + kReserved);

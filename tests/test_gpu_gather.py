@@ -42,6 +42,24 @@ def test_runs_that_fill_a_warps_shared_memory(short):
     assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
 
 
+@pytest.mark.parametrize("C", [1, 31, 128, 161])
+# what a warp's shared memory takes whatever byte its run starts at: 5,105 bytes, as one run, in halves and in quarters of the
+# warp; what does not fit then goes byte by byte
+@pytest.mark.parametrize("parts", [1, 2, 4])
+@pytest.mark.parametrize("above", [-1, 0, 1, 40])
+def test_runs_on_both_sides_of_what_fits(C, parts, above):
+    from cachegen_b200.serde import cachegen_encoder as E
+    n = 32 // parts
+    each, rest = divmod(5105 + above, n)
+    stride = (each + rest + 7) // 4 * 4
+    buf, lens = rows_of(np.random.default_rng(C + 100 * parts + above), 3, C, stride, each)
+    lens[:] = each
+    lens[:, ::n] += rest
+    lens[2] = np.random.default_rng(parts).integers(0, stride + 1, C)  # parts of every kind in a warp
+    got = E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda())
+    assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
+
+
 def test_several_sub_chunks_through_the_c_abi():
     from cachegen_b200 import _lib
     NL, C, stride, nsub = 2, 200, 100, 3
@@ -91,3 +109,32 @@ def test_collect_bytes_refuses_lengths_in_host_memory():
     buf, lens = rows_of(np.random.default_rng(5), 2, 60, 64, 50)
     with pytest.raises(RuntimeError, match="on the buffer's GPU"):
         E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens))
+
+
+def test_the_finest_bins_are_gathered_like_others():
+    """Uniform values at the most bins an encode accepts give streams of 184 bytes: their runs pass through shared memory too
+    (copied byte by byte they take 20 times as long as others)."""
+    from cachegen_b200 import _lib
+    from cachegen_b200.serde import cachegen_encoder as E
+    kv = (torch.rand((8, 2, 256, 32, 128), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda") * 2 - 1).half()
+    times = {}
+    for bins in (24, 63):
+        b = torch.full((8,), float(bins))
+        p = E._PendingChunk(kv, E._BinsInfo(b, b), bins)
+        try:
+            size = p.sizes()[0][1]
+            out = torch.empty(size, dtype=torch.uint8, device="cuda")
+            pointer = p.pointers(out.data_ptr())
+            best = float("inf")
+            for _ in range(12):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                for _ in range(20):
+                    _lib.check(p.lib.cg_encode_kv_gather(ctypes.byref(p.job), pointer, p.length_pointers, p.stream_ptr), "gather")
+                b.record()
+                b.synchronize()
+                best = min(best, a.elapsed_time(b))
+            times[bins] = best / (size / (16 * 4096))
+        finally:
+            p.abandon()
+    assert times[63] < 4 * times[24], times  # a byte
