@@ -579,12 +579,16 @@ class _Staging:
         blob takes 130 to 200 us, as long as a third of its 30 MB take over the bus, and waking the threads 50.
         ahead: one of them sends it to the current GPU as well, on the current stream, and the tensors are cut out of it
         there (a 256-token chunk to pickled bytes and back 2,070 -> 1,940 us; several blobs after each other keep the bus
-        busy as it is)."""
+        busy as it is).  Until they are, the GPU holds the blob's size (30 MB) beside them.  Only for a blob whose first
+        tensor belongs there: what is to stay on the host, or goes to another GPU, would be sent for nothing."""
         if len(bs) < _EARLY_FROM or not torch.cuda.is_available():
+            return
+        where = _blob_location(bs)
+        if where == "cpu":
             return
         device = torch.device("cuda", torch.cuda.current_device())
         on, raw = torch.cuda.current_stream(device), None
-        if ahead and not torch.cuda.is_current_stream_capturing():
+        if ahead and where == str(device) and not torch.cuda.is_current_stream_capturing():
             try:
                 raw = torch.empty(len(bs) + _AHEAD_SPARE, dtype=torch.uint8, device=device)
             except torch.cuda.OutOfMemoryError:
@@ -826,6 +830,16 @@ def _cut_streams(bs: bytes):
 
 _STORAGE_DTYPES = {name: dtype for dtype, name in torch.storage._dtype_to_storage_type_map().items()}
 _dtype_of = _STORAGE_DTYPES.get
+
+
+def _blob_location(bs: bytes):
+    """The device that a blob's first storage names ("cpu", "cuda:0"); None if the blob does not start as one does."""
+    at = bs.find(_MAGIC_PICKLE, 0, _FIRST_STREAM_WITHIN)
+    head = _read_stream_head(memoryview(bs)[at:at + 1024]) if at >= 0 else None
+    return head[1] if head else None
+
+
+_FIRST_STREAM_WITHIN = 4096  # the names of a blob's classes and fields come first, a few hundred bytes
 
 
 class _CudaStream:
