@@ -56,15 +56,6 @@ CG_HD uint32_t cg_fshl(uint32_t lo, uint32_t hi, uint32_t s) {
     return s ? ((hi << s) | (lo >> (32u - s))) : hi;
 #endif
 }
-// upper 32 bits of (hi:lo) << min(s, 32)
-CG_HD uint32_t cg_fshl_clamp(uint32_t lo, uint32_t hi, uint32_t s) {
-#if defined(__CUDA_ARCH__)
-    return __funnelshift_lc(lo, hi, s);
-#else
-    if (s >= 32u) return lo;
-    return s ? ((hi << s) | (lo >> (32u - s))) : hi;
-#endif
-}
 // lower 32 bits of (hi:lo) >> min(s, 32)
 CG_HD uint32_t cg_fshr_clamp(uint32_t lo, uint32_t hi, uint32_t s) {
 #if defined(__CUDA_ARCH__)
@@ -251,7 +242,7 @@ struct BitWindow {
     // 4.7 instructions a symbol of the fused decode at 0.055 passes a token; one word, 0.09 passes, takes 1.6.
     CG_HD void refill() {
 #if defined(__CUDA_ARCH__)
-        asm("{ .reg .u32 w, rem, t, b; .reg .s32 r; .reg .u64 at; .reg .pred p, q, a;\n"
+        asm("{ .reg .u32 w, rem, t, b; .reg .u64 at; .reg .pred p, q, a;\n"
             "setp.lt.s32 p, %3, 64;\n"
             "mad.lo.u32 rem, %4, -32, %6;\n"     // bits of the stream from this word on, negative past its end
             "mad.wide.u32 at, %4, 4, %5;\n"
@@ -525,15 +516,14 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 // One stream.  col: address of the stream's table column (see search_entry), rows kTableRowBytes apart,
 // 2^LEVELS + 1 of them readable, 2^LEVELS >= maxsym + 1; emit(a) receives, token after token, the address of the
 // decoded symbol's table entry (symbol = (a - col) / kTableRowBytes).  lanes: the warp's lanes that
-// run this loop together (they must all have the same ntok).  FULL: the table has exactly 2^LEVELS symbols (the
-// search is the same).
-template <int LEVELS, bool FULL, class Emit>
+// run this loop together (they must all have the same ntok).
+template <int LEVELS, class Emit>
 CG_HD void decode_stream(Smem sm, uint32_t col, int maxsym, const uint8_t *stream, uint32_t len, int ntok,
                          uint32_t lanes, Emit emit) {
     const uint32_t cols[1] = {col}, lens[1] = {len};
     const uint8_t *const streams[1] = {stream};
     const int top = (1 << LEVELS) - 1;
-    const uint32_t det = col + static_cast<uint32_t>(FULL || top < maxsym ? top : maxsym) * kTableRowBytes;
+    const uint32_t det = col + static_cast<uint32_t>(top < maxsym ? top : maxsym) * kTableRowBytes;
     decode_streams<LEVELS, 1>(sm, cols, det, maxsym, LEVELS, streams, lens, ntok, lanes,
                               [&](const uint32_t(&a)[1], uint32_t) { emit(a[0]); });
 }
@@ -721,11 +711,6 @@ struct EncoderState {
         if (span32 == 0u) half_scale(out);
         const uint32_t flo = cg_umulhi_wide(span32, sm.ld(a));
         take<true>(flo, last ? span32 : cg_umulhi_wide(span32, sm.ld(a + ROW)), out);
-    }
-    // symbol s <= maxsym of one stream
-    template <class Sink>
-    CG_HD void step(Smem sm, uint32_t col, uint32_t s, uint32_t maxsym, Sink &out, uint32_t) {
-        step_alone<kTableRowBytes>(sm, col + s * kTableRowBytes, s == maxsym, out);
     }
     // G symbols (1 or 2) of NS streams a lane, by the addresses of their table entries.  The streams' chains are independent,
     // and ONE warp vote after them covers a full word in an accumulator: every lane that has one stores it as soon as one

@@ -127,8 +127,7 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
         *o = static_cast<uint8_t>((a - col) / kRowBytes);
         o += o1;
     };
-    decode_stream<LEVELS, false>(Smem{}, col, p.lp - 2, p.bytes + start, static_cast<uint32_t>(len), p.ntokens,
-                                lanes, emit);
+    decode_stream<LEVELS>(Smem{}, col, p.lp - 2, p.bytes + start, static_cast<uint32_t>(len), p.ntokens, lanes, emit);
 }
 
 // The same with two adjacent channels per thread, whose symbols are adjacent bytes (see decode_dequant_multi_kernel):
@@ -382,8 +381,7 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
         o += o_token;
         sc_a += 4u;
     };
-    decode_stream<LEVELS, false>(Smem{}, col, p.lp - 2, job.bytes + start, static_cast<uint32_t>(len), ntok_r,
-                                lanes, emit);
+    decode_stream<LEVELS>(Smem{}, col, p.lp - 2, job.bytes + start, static_cast<uint32_t>(len), ntok_r, lanes, emit);
 }
 
 // ---- the same with NS adjacent channels per thread ----------------------------------------------------------

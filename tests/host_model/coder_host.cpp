@@ -31,34 +31,32 @@ extern "C" int64_t hm_encode_stream(const uint16_t *cdf, int lp, const int8_t *s
     sink.init(out, cap);
     EncoderState enc;
     enc.init();
-    for (int i = 0; i < n; ++i) enc.step(rd, col, static_cast<uint8_t>(sym[i]), static_cast<uint32_t>(lp - 2), sink, 0xFFFFFFFFu);
+    for (int i = 0; i < n; ++i) {
+        const uint32_t s = static_cast<uint8_t>(sym[i]);
+        enc.step_alone<kTableRowBytes>(rd, col + s * kTableRowBytes, s == static_cast<uint32_t>(lp - 2), sink);
+    }
     return enc.flush(sink);
 }
 
-template <int LEVELS, bool POW2>
+template <int LEVELS>
 static void run_decode(const uint16_t *cdf, int lp, const uint8_t *bytes, int64_t len, int n, uint8_t *out,
                               int tid) {
     const int rows = (1 << LEVELS) > lp - 1 ? (1 << LEVELS) : lp - 1;
     std::vector<uint32_t> tab = make_table(cdf, lp - 1 < rows ? lp - 1 : rows, rows + 1, tid);
     Smem rd{reinterpret_cast<uint8_t *>(tab.data())};
-    decode_stream<LEVELS, POW2>(rd, static_cast<uint32_t>(tid) * 4u, lp - 2, bytes, static_cast<uint32_t>(len),
-                                       n, 0xFFFFFFFFu, [&](uint32_t a) {
-                                           *out++ = static_cast<uint8_t>((a - static_cast<uint32_t>(tid) * 4u) /
-                                                                         kTableRowBytes);
-                                       });
+    decode_stream<LEVELS>(rd, static_cast<uint32_t>(tid) * 4u, lp - 2, bytes, static_cast<uint32_t>(len), n, 0xFFFFFFFFu,
+                          [&](uint32_t a) {
+                              *out++ = static_cast<uint8_t>((a - static_cast<uint32_t>(tid) * 4u) / kTableRowBytes);
+                          });
 }
 
 extern "C" void hm_decode_stream(const uint16_t *cdf, int lp, const uint8_t *bytes, int64_t len, int n,
                                         uint8_t *out, int tid) {
     const int need = search_levels(lp);
-    const bool pow2 = (1 << need) == lp - 1;
-    if (pow2 && need == 5) run_decode<5, true>(cdf, lp, bytes, len, n, out, tid);
-    else if (pow2 && need == 4) run_decode<4, true>(cdf, lp, bytes, len, n, out, tid);
-    else if (pow2 && need == 3) run_decode<3, true>(cdf, lp, bytes, len, n, out, tid);
-    else if (need <= 3) run_decode<3, false>(cdf, lp, bytes, len, n, out, tid);
-    else if (need == 4) run_decode<4, false>(cdf, lp, bytes, len, n, out, tid);
-    else if (need == 5) run_decode<5, false>(cdf, lp, bytes, len, n, out, tid);
-    else run_decode<6, false>(cdf, lp, bytes, len, n, out, tid);
+    if (need <= 3) run_decode<3>(cdf, lp, bytes, len, n, out, tid);
+    else if (need == 4) run_decode<4>(cdf, lp, bytes, len, n, out, tid);
+    else if (need == 5) run_decode<5>(cdf, lp, bytes, len, n, out, tid);
+    else run_decode<6>(cdf, lp, bytes, len, n, out, tid);
 }
 
 
