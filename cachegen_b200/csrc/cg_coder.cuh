@@ -38,8 +38,7 @@ CG_HD int cg_clz(uint32_t x) {
     return x ? __builtin_clz(x) : 32;
 #endif
 }
-// x << n, 0 for n >= 32.  On the device a clamping funnel shift: a plain `<<` by 32 or more is undefined
-// to the compiler, which may then emit the wrapping form.
+// x << n, 0 for n >= 32.  On the device a clamping funnel shift: a plain `<<` by 32 or more is undefined.
 CG_HD uint32_t cg_shl(uint32_t x, uint32_t n) {
 #if defined(__CUDA_ARCH__)
     return __funnelshift_lc(0u, x, n);
@@ -125,8 +124,8 @@ struct Smem {
 // Returns s and 2^s: for the words that are only shifted left a multiply does it off the integer pipe (a
 // shift, a compare or a select takes that pipe for two cycles a warp, and a multiply-high the multiply pipe for four).
 //
-// The conditional decrement is written as a predicated add: from `if (...) --s` the compiler makes a
-// decrement, a move and a select (two instructions a symbol more, measured as executed instructions).
+// The conditional decrement is written as a predicated add: with `if (...) --s` the counters show two executed
+// instructions a symbol more.
 struct Renorm {
     uint32_t s, p2;
 };
@@ -173,8 +172,7 @@ CG_HD uint32_t cg_umulhi(uint32_t a, uint32_t b) {
     return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
 #endif
 }
-// The same as the upper half of a wide product.  A sum with a multiply-high becomes one instruction whose addend has to be
-// moved into a register pair first; the encoder's step takes two instructions fewer with this.
+// The same as the upper half of a wide product: the encoder's step, which adds to it, executes two instructions fewer so.
 CG_HD uint32_t cg_umulhi_wide(uint32_t a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
     uint64_t p;
@@ -184,7 +182,7 @@ CG_HD uint32_t cg_umulhi_wide(uint32_t a, uint32_t b) {
     return cg_umulhi(a, b);
 #endif
 }
-// a + b - 1 as one instruction
+// a + b - 1: one executed instruction fewer than from the C++ form
 CG_HD uint32_t cg_add_less_one(uint32_t a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
     uint32_t d;
@@ -424,8 +422,8 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
     const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
     uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
     // The inner loop is the common case and nothing else, left by one vote for a refill of the bit windows, for a
-    // symbol whose fast search failed and at the last token; with that code inside it, the state of both streams moved
-    // between registers at every pass.
+    // symbol whose fast search failed and at the last token; with that code inside it, every pass executed more
+    // instructions, whether it took that code or not.
     for (;;) {
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
@@ -718,8 +716,8 @@ struct EncoderState {
     // LAST: a symbol may be its table's last, whose upper bound is the range's end (told by `last`; G is 1 then).
     // What hardly ever happens is not mended here but left to encode_again: a carry through a whole word of ones
     // (`carried`), and a range of 2^31 at a multiple of it, which leaves a span of 0, from where on no symbol has a size, so
-    // that the span is still 0 at the stream's end.  Code for the like inside the loop cost five instructions a symbol in
-    // moves between registers without ever being run.
+    // that the span is still 0 at the stream's end.  Code for the like inside the loop cost five executed instructions a
+    // symbol without ever being run.
     template <int ROW, int G, int NS, bool LAST = false, class Sink>
     static CG_HD void steps_at(Smem sm, const uint32_t (&a)[G][NS], EncoderState (&enc)[NS], Sink (&out)[NS], int high_water,
                                uint32_t lanes, bool (&carried)[NS], bool last = false) {

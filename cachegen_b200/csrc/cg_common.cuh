@@ -206,7 +206,7 @@ __device__ __forceinline__ int block_exclusive_scan_128(int v, int *warp_sums, i
 // streams share by an atomic or), and the warp writes the run with 128-bit stores.  Copying stream after stream
 // to its place byte by byte took 20 us a 256-token Llama-7B chunk (11.8 MB in 262,144 streams of 45 bytes),
 // with words assembled from two source words 24 us: one short dependent copy after the other.  Twelve loads in flight and
-// 5 KB of shared memory a warp 15 us under counters, eight and 6 KB 17.
+// 5 KB of shared memory a warp 15 us under counters, eight and 6 KB 17; eight and 5 KB the same as twelve.
 // src: the stream's first word, its words STEP words apart, read-only for the launch; dst0: where the group's
 // streams go; pairs: (STEP 1) the words can be read in pairs, to the end of the last one.  Whatever the row holds behind
 // its stream: the last word is cut to the stream's bytes, since what it shares a word with there is the next stream (and

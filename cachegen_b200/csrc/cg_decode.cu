@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
 // entry m in a register, a ballot over "(span * cdf[m]) >> 16 <= value - low" finds the symbol and two
 // shuffles fetch its scaled bounds.  It needs no shared memory and no search loop, but all 32 lanes
 // repeat the stream's serial range update, so it spends about 30 warp instructions per symbol where
-// the thread-per-stream kernels spend about 70 per 32 symbols.  Same results; tables of at most 33
+// the thread-per-stream kernels spend 58 for 32 symbols.  Same results; tables of at most 33
 // entries; prefix-sum stream layout only.
 __global__ void __launch_bounds__(kGroup) decode_symbols_warp_kernel(const SymDecodeParams p, int nrows) {
     const int lane = threadIdx.x & 31;

@@ -450,8 +450,7 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint32_
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
 // chunk takes 107 us with its tables under counters, 0.63 T symbols/s, 34.6 instructions for 32 symbols; 122 us and 40.4 with
 // the code for rare cases inside the loop, a mask kept as the interval's size and a vote a symbol.  Eight blocks an SM leave the compiler 64
-// registers.  (Seven, for two even waves of a chunk's 2,048 blocks, were better while a block took longer: 207 against 205 us a
-// whole encode now.)
+// registers.  (Seven, for two even waves of a chunk's 2,048 blocks, take the same.)
 // Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
 // channels in 164 us under counters (28.5 instructions for 32 symbols), 172 before the same change; 180 with one stream.
 // G symbols a vote: two, unless the table may give a symbol more bits than the accumulator has room for twice (pair_high_water:

@@ -311,7 +311,7 @@ class _PendingChunk:
     """One chunk whose kernels up to the streams and their offsets are enqueued on `stream` (default: the
     current one), but whose payload size is not yet known on the host.  finish() waits for that and
     enqueues the gather.  Buffers come from the current stream's pool whatever `stream` is.  enqueue=False leaves the
-    launches to _enqueue_levels."""
+    launches to _encode_infos."""
 
     def __init__(self, kv, info, max_bins, delta=None, stream=None, workspace=None, with_counts=False, enqueue=True):
         if kv.dim() != 5 or kv.shape[1] != 2:

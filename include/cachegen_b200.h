@@ -48,8 +48,9 @@ extern "C" {
 /* 128-channel groups (all rows) whose offsets one cluster of blocks can hold */
 #define CG_MAX_OFFSET_GROUPS 96000
 /* sub-chunks one fused decode launch can take */
-#define CG_MAX_ENCODE_LEVELS 4 /* jobs of one cg_encode_kv_levels call */
 #define CG_MAX_DECODE_JOBS 40
+/* jobs of one cg_encode_kv_levels call */
+#define CG_MAX_ENCODE_LEVELS 4
 
 /* Table kinds of cg_decode_job.tables.
  * CG_TABLES_CDF:    int16 [nrows, nchannels, lp], the reference's tables (calculate_cdf).
