@@ -21,7 +21,7 @@ def gathered(buf, lens):
 
 
 @pytest.mark.parametrize("C", [1, 31, 32, 33, 127, 128, 129, 300])
-# the shared memory of a warp holds 6,144 bytes: runs below it, around it (32 rows of 188 to 196) and above
+# runs that a warp's shared memory takes at once (up to 5,105 bytes), in halves (from 32 rows of 160 on) and in quarters
 @pytest.mark.parametrize("stride,most", [(4, 1), (4, 4), (8, 7), (12, 9), (64, 61), (188, 188), (192, 192), (196, 195), (520, 519)])
 def test_collect_bytes_of_rows_with_data_behind_the_streams(C, stride, most):
     from cachegen_b200.serde import cachegen_encoder as E
@@ -33,7 +33,7 @@ def test_collect_bytes_of_rows_with_data_behind_the_streams(C, stride, most):
 @pytest.mark.parametrize("short", [0, 1, 2, 3, 5, 16])
 def test_runs_that_fill_a_warps_shared_memory(short):
     from cachegen_b200.serde import cachegen_encoder as E
-    # 32 streams of 192 bytes are a whole run; the first one starts its warp's run at every offset from 16 bytes
+    # 32 streams of 192 bytes go in halves; the first one starts its warp's run at every offset from 16 bytes
     buf, lens = rows_of(np.random.default_rng(short), 2, 128, 196, 192)
     lens[:] = 192
     lens[:, 32] -= short
@@ -56,6 +56,21 @@ def test_runs_on_both_sides_of_what_fits(C, parts, above):
     lens[:] = each
     lens[:, ::n] += rest
     lens[2] = np.random.default_rng(parts).integers(0, stride + 1, C)  # parts of every kind in a warp
+    got = E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda())
+    assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
+
+
+@pytest.mark.parametrize("offset", range(16))
+def test_the_longest_run_at_once_from_every_byte(offset):
+    from cachegen_b200.serde import cachegen_encoder as E
+    buf, lens = rows_of(np.random.default_rng(offset), 2, 64, 176, 160)
+    lens[:] = 0
+    lens[0, 3] = offset  # the first warp's run; the second one's starts there, 32 streams of 5,105 and then of 5,106 bytes
+    lens[0, 32:] = 159
+    lens[0, 40] += 17
+    lens[1, 32:] = 159
+    lens[1, 32] += 1  # (and starts where the first row's ends)
+    lens[1, 40] += 17
     got = E.collect_bytes(torch.from_numpy(buf).cuda(), torch.from_numpy(lens).cuda())
     assert got.cpu().numpy().tobytes() == gathered(buf, lens).tobytes()
 
