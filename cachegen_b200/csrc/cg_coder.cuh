@@ -13,7 +13,7 @@
 //     value - low directly;
 //   * within one symbol the renormalisation loop does a run of "equal top bit" shifts followed
 //     by a run of "underflow" shifts, never the other way round; their sum comes from one
-//     leading-bit search (renorm_shift), the decoder takes all its new bits in one funnel shift and the
+//     leading-bit search (renorm_shift), by which the decoder moves its position in the stream and the
 //     encoder appends the shifted-out top bits of `low` at once, carries included.
 #pragma once
 
@@ -116,10 +116,11 @@ struct Smem {
 // the top of a word instead, two multiplies and two adds with carry: one instruction more and four more
 // cycles of the multiply pipe a symbol.)
 //
-// By the size u = d + 1 instead of d (the encoder's loop): the top bit is another one only where u is a power of two, and
+// By the size u = d + 1 instead of d (the coders' loops): the top bit is another one only where u is a power of two, and
 // s one or two less than it could be where low is a multiple of u or of u / 2 as well.  Nothing is lost by that: the next
 // symbol's bounds are exact at any scale of such a range, and its shift makes up for it; and the full range of 2^32, which
-// no word holds, does not come about.  (Only u = 2^31 at a multiple of 2^31 gives -1: see EncoderState::steps_at.)
+// no word holds, does not come about.  (Only u = 2^31 at a multiple of 2^31 gives -1: see EncoderState::steps_at and
+// DecoderState.)
 //
 // Returns s and 2^s: for the words that are only shifted left a multiply does it off the integer pipe (a
 // shift, a compare or a select takes that pipe for two cycles a warp, and a multiply-high the multiply pipe for four).
@@ -148,14 +149,26 @@ CG_HD Renorm renorm_shift(uint32_t low, uint32_t high, uint32_t d) {
 #endif
     return r;
 }
+// By the size u alone: two adds fewer where only the shift is wanted.
+CG_HD uint32_t renorm_shift_by_size(uint32_t low, uint32_t u) {
+#if defined(__CUDA_ARCH__)
+    uint32_t s;
+    asm("{ .reg .u32 t, b, h; .reg .pred p;\n"
+        "add.u32 h, %1, %2;\n"
+        "add.u32 h, h, -1;\n"
+        "bfind.shiftamt.u32 %0, %2;\n"
+        "shf.r.wrap.b32 b, 0x80000000, 0, %0;\n"
+        "lop3.b32 t, %1, h, b, 0x28;\n"  // (low ^ high) & b
+        "setp.eq.u32 p, t, 0;\n"
+        "@p add.u32 %0, %0, -1; }"
+        : "=&r"(s) : "r"(low), "r"(u));
+    return s;
+#else
+    return renorm_shift(low, low + u - 1u, u).s;
+#endif
+}
 
-// ---- register bit window + warp-synchronous refill -----------------------------------------------------------
-// The next 96 unread bits of the stream live in three registers.  The byte array is read as aligned
-// 32-bit words; bits before the stream's first byte are shifted out at start-up and words (or word
-// tails) past its last byte read as zero, which is what the reference sees in its zero-padded staging
-// row (dec_new.cu:229-232).  A refill is taken by the whole warp as soon as any of its lanes has fewer
-// bits than a symbol can take and gives a word to every lane with room for one, so the refill code runs once per warp every
-// few symbols instead of once per lane.
+// ---- warp votes and products -------------------------------------------------------------------------------------
 CG_HD bool cg_any_lane(uint32_t lanes, bool pred) {
 #if defined(__CUDA_ARCH__)
     return __any_sync(lanes, pred) != 0;
@@ -172,7 +185,7 @@ CG_HD uint32_t cg_umulhi(uint32_t a, uint32_t b) {
     return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
 #endif
 }
-// The same as the upper half of a wide product: the encoder's step, which adds to it, executes two instructions fewer so.
+// The same as the upper half of a wide product: the coders' steps, which add to it, execute one or two instructions fewer so.
 CG_HD uint32_t cg_umulhi_wide(uint32_t a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
     uint64_t p;
@@ -193,84 +206,84 @@ CG_HD uint32_t cg_add_less_one(uint32_t a, uint32_t b) {
 #endif
 }
 
+// ---- bit window ------------------------------------------------------------------------------------------------------
+// The 64 bits of a stream from bit `at` on, in two registers, which a decoder reads at a position of its own and does not
+// shift: its 32-bit value at position p is one funnel shift, whatever was taken before.  The byte array is read as aligned
+// 32-bit words; bits past the stream's last byte are zero, which is what the reference sees in its zero-padded staging
+// row (dec_new.cu:229-232).
 struct BitWindow {
-    const uint32_t *wp;    // word holding the stream's first byte
-    uint32_t end_bit;      // bit index, counted from wp, one past the stream's last bit
-    uint32_t next;         // next word to fetch
-    uint32_t hi, mid, lo;  // unread bits, hi's top bit first
-    int nbits;             // valid bits in hi:mid:lo
+    const uint32_t *wp;   // the word that holds the window's first bit
+    uint32_t off;         // that bit's place in it
+    int32_t rem;          // bits of the stream from two words further on, negative past its end
+    uint32_t w0, w1, w2;  // the words from wp on, big-endian, bits past the stream's end cleared
+    uint32_t hi, lo;      // the window
 
-    // word j of the stream, big-endian, bits past the stream's end cleared; no branches
-    CG_HD uint32_t fetch(uint32_t j) const {
-        const uint32_t b0 = j * 32u;
+    // word j from wp on; r: bits of the stream from there on
+    CG_HD uint32_t word(int j, int32_t r) const {
         uint32_t w = 0u;
-        if (b0 < end_bit) w = cg_bswap32(cg_load_stream_word(wp + j));
-        const uint32_t rem = end_bit - b0;  // >= 2^31 (clamped to 32 below) when the word lies past the end
-        return w & ~cg_fshr_clamp(0xFFFFFFFFu, 0u, rem);
+        if (r > 0) w = cg_bswap32(cg_load_stream_word(wp + j));
+        return w & ~cg_fshr_clamp(0xFFFFFFFFu, 0u, static_cast<uint32_t>(r));  // (a negative one counts as more than 32)
     }
-    // returns the stream's first 32 bits (the coder's initial `value`, dec_new.cu:257)
-    CG_HD uint32_t open(const uint8_t *p, uint32_t len) {
+    CG_HD void cut() {
+        hi = cg_fshl(w1, w0, off);
+        lo = cg_fshl(w2, w1, off);
+    }
+    CG_HD void open(const uint8_t *p, uint32_t len) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(p);
         wp = reinterpret_cast<const uint32_t *>(a & ~static_cast<uintptr_t>(3));
-        const uint32_t off = static_cast<uint32_t>(a & 3u) * 8u;
-        end_bit = off + len * 8u;
-        const uint32_t w0 = fetch(0), w1 = fetch(1), w2 = fetch(2), w3 = fetch(3);
-        hi = cg_fshl(w2, w1, off);
-        mid = cg_fshl(w3, w2, off);
-        lo = w3 << off;
-        nbits = 96 - static_cast<int>(off);
-        next = 4;
-        return cg_fshl(w1, w0, off);
+        off = static_cast<uint32_t>(a & 3u) * 8u;
+        rem = static_cast<int32_t>(off + len * 8u) - 64;
+        w0 = word(0, rem + 64);
+        w1 = word(1, rem + 32);
+        w2 = word(2, rem);
+        cut();
     }
-    // drops the bits just shifted into the coder's value
-    CG_HD void consume(Renorm r) {
-        hi = cg_fshl(mid, hi, r.s);
-        mid = cg_fshl(lo, mid, r.s);
-        lo *= r.p2;
-        nbits -= static_cast<int>(r.s);
-    }
-    CG_HD bool low_water() const { return nbits <= 32; }
-    // fewer valid bits than one symbol can take: a range update shifts by at most 18 bits when the
-    // table is strictly increasing (the updated interval spans at least 2^14 values)
-    static constexpr int kShort = 18;
-    CG_HD bool short_of_bits() const { return nbits < kShort; }
-    // Takes the next word where one fits above 32 bits of room (a stream short of bits has 32 or more afterwards),
-    // straight-line: every lane of the warp runs the same instructions whatever it needs.
-    // Written in predicated instructions (see renorm_shift): filling up to two words a pass with selects took
-    // 4.7 instructions a symbol of the fused decode at 0.055 passes a token; one word, 0.09 passes, takes 1.6.
-    CG_HD void refill() {
+    // Moves the window on to position p < 64, which becomes 0 (a negative one stays: see DecoderState).  Straight-line: every
+    // lane of the warp runs the same instructions whatever it needs, but only words that a lane has not got are
+    // read: with three words read for every lane each time the loads' wavefronts, not the instructions, bound the decode
+    // (69 % of their rate where this takes 50; 2,048 Llama-7B tokens 986 us, this way 972).
+    CG_HD void advance(int32_t &p) {
+        const uint32_t to = off + static_cast<uint32_t>(p > 0 ? p : 0), k = to >> 5;  // words to move on by: 0, 1 or 2
+        p = p < 0 ? p : 0;
+        off = to & 31u;
+        wp += k;
+        rem -= static_cast<int32_t>(k * 32u);
 #if defined(__CUDA_ARCH__)
-        asm("{ .reg .u32 w, rem, t, b; .reg .u64 at; .reg .pred p, q, a;\n"
-            "setp.lt.s32 p, %3, 64;\n"
-            "mad.lo.u32 rem, %4, -32, %6;\n"     // bits of the stream from this word on, negative past its end
-            "mad.wide.u32 at, %4, 4, %5;\n"
-            "mov.u32 w, 0;\n"
-            "setp.gt.and.s32 q, rem, 0, p;\n"
-            "@q ld.global.nc.u32 w, [at];\n"
-            "prmt.b32 w, w, 0, 0x0123;\n"
-            "shr.u32 t, 0xFFFFFFFF, rem;\n"      // (a shift by more than 31 gives 0)
-            "lop3.b32 w, w, t, 0, 0x30;\n"       // w & ~t
-            "shf.r.wrap.b32 t, w, 0, %3;\n"      // the word's upper part, behind the valid bits of their last word
-            "shf.r.wrap.b32 b, 0, w, %3;\n"      // and what goes into the word after that
-            "setp.lt.s32 a, %3, 32;\n"
-            "@a or.b32 %0, %0, t;\n"
-            "@a or.b32 %1, %1, b;\n"
-            "@!a or.b32 %1, %1, t;\n"
-            "@!a or.b32 %2, %2, b;\n"
-            "@p add.s32 %3, %3, 32;\n"
-            "@p add.u32 %4, %4, 1; }"
-            : "+r"(hi), "+r"(mid), "+r"(lo), "+r"(nbits), "+r"(next) : "l"(wp), "r"(end_bit));
+        asm("{ .reg .u32 t, m; .reg .s32 r; .reg .pred p1, p2, q;\n"
+            "setp.gt.u32 p1, %5, 0;\n"
+            "setp.gt.u32 p2, %5, 1;\n"
+            "@p1 mov.u32 %0, %1;\n"
+            "@p1 mov.u32 %1, %2;\n"
+            "@p2 mov.u32 %0, %1;\n"
+            "setp.gt.and.s32 q, %4, 0, p1;\n"
+            "mov.u32 t, 0;\n"
+            "@q ld.global.nc.u32 t, [%3+8];\n"
+            "prmt.b32 t, t, 0, 0x0123;\n"
+            "shr.u32 m, 0xFFFFFFFF, %4;\n"       // (a shift by more than 31 gives 0)
+            "@p1 lop3.b32 %2, t, m, 0, 0x30;\n"  // t & ~m
+            "add.s32 r, %4, 32;\n"
+            "setp.gt.and.s32 q, r, 0, p2;\n"
+            "mov.u32 t, 0;\n"
+            "@q ld.global.nc.u32 t, [%3+4];\n"
+            "prmt.b32 t, t, 0, 0x0123;\n"
+            "shr.u32 m, 0xFFFFFFFF, r;\n"
+            "@p2 lop3.b32 %1, t, m, 0, 0x30; }"
+            : "+r"(w0), "+r"(w1), "+r"(w2) : "l"(wp), "r"(rem), "r"(k));
 #else
-        if (nbits >= 64) return;
-        const uint32_t w = fetch(next++), p = static_cast<uint32_t>(nbits) & 31u, t = w >> p, b = p ? w << (32u - p) : 0u;
-        if (nbits < 32) {
-            hi |= t;
-            mid |= b;
-        } else {
-            mid |= t;
-            lo |= b;
+        if (k) {
+            w0 = word(0, rem + 64);
+            w1 = word(1, rem + 32);
+            w2 = word(2, rem);
         }
-        nbits += 32;
+#endif
+        cut();
+    }
+    // 32 bits from position p on, 0 <= p <= 32
+    CG_HD uint32_t bits(int32_t p) const {
+#if defined(__CUDA_ARCH__)
+        return __funnelshift_lc(lo, hi, static_cast<uint32_t>(p));
+#else
+        return p >= 32 || p < 0 ? lo : cg_fshl(lo, hi, static_cast<uint32_t>(p));
 #endif
     }
 };
@@ -280,38 +293,51 @@ struct BitWindow {
 // exactly when the range is the full 2^32 (then the product is c16 itself).
 CG_HD uint32_t scale_exact(uint32_t span32, uint32_t c16) { return span32 ? cg_umulhi(span32, c16) : c16; }
 
-// The decoder's arithmetic state: low, span32 = (high - low + 1) mod 2^32 and offset = value - low.
-// In this form both kinds of renormalisation shift act alike on the pair (offset, span) --
-// offset = 2*offset + next bit, span = 2*span -- so the reference's "value -= 2^30" of the underflow
-// case needs no separate step; low is still tracked because the shift counts depend on the bit
-// patterns of low and high.
+// The decoder's arithmetic state: low, span32 = (high - low + 1) mod 2^32 and the position p of the current 32 bits of the
+// stream in its window; value - low of the reference is the difference of those bits and low.  Both kinds of renormalisation
+// shift act alike on it: low is shifted left, and what the underflow shifts drop from it ("value -= 2^30") is dropped from
+// the stream's bits by the same subtraction modulo 2^32.  low is tracked because the shift counts depend on it.
+//
+// The fast step takes the shift by the interval's size (see renorm_shift); where that gives -1 (a size of 2^31 at a multiple of
+// 2^31) what is left is a span of 0, a low of 0 and p one less than it was, and one shift would have been right, which leaves the
+// same span and low and p two more.  So a span of 0 stands for the full range of 2^32 with p two less than the position
+// of its bits: at the stream's start, too.  Its scaled bounds are all 0, which no symbol passes.
 struct DecoderState {
-    uint32_t low, span32, offset;
-
+    static constexpr int32_t kFullRange = -2;
+    uint32_t low, span32;
+    int32_t p;
+    CG_HD void init() {
+        low = 0u;
+        span32 = 0u;
+        p = kFullRange;
+    }
+    // The bits' distance from low; the position of a full range put right.
+    CG_HD uint32_t exact_offset(const BitWindow &bw) {
+        if (span32 == 0u) p -= kFullRange;
+        return bw.bits(p) - low;
+    }
     // range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation
     // (dec_new.cu:277-301), both kinds of shift applied in one go.  On a table that is not increasing the
     // shift count is anything up to 31; every later read stays inside the table column and the stream.
-    CG_HD void update(uint32_t flo, uint32_t fhi, BitWindow &bw) {
-        offset -= flo;
+    CG_HD void exact_update(uint32_t flo, uint32_t fhi) {
+        const uint32_t d = fhi - flo - 1u;
         low += flo;
-        span32 = fhi - flo;
-        const uint32_t d = span32 - 1u;
-        const Renorm r = renorm_shift(low, low + d, d);
-        low = cg_fshl(0u, low, r.s);
-        span32 = cg_fshl(0u, span32, r.s);
-        offset = cg_fshl(bw.hi, offset, r.s);
-        bw.consume(r);
+        const uint32_t s = renorm_shift(low, low + d, d).s & 31u;
+        low = cg_fshl(0u, low, s);
+        span32 = cg_fshl(0u, fhi - flo, s);
+        p += static_cast<int32_t>(s);
+        if (span32 == 0u) p += kFullRange;
     }
 };
 
 // ---- decode loop: NS streams per lane, search depth chosen by the caller ---------------------------------
-// Table entries as the search takes them: 2^23 (1 + cdf / 2^16) as a float.  Its bits shifted by nine are cdf << 16, and
-// a comparison with an estimate of 2^23 (1 + offset / span) + 1, which is as whole a number, is the difference cut to
-// [0, 1], which is 0 or 1.  A search step is then a subtraction with saturation and a multiply-add on the entry's address
+// Table entries as the search takes them: 2^23 + cdf as a float.  Its bits shifted by sixteen are cdf << 16, and
+// a comparison with an estimate of floor(2^16 offset / span) + 1, which is as whole a number, is the difference cut to
+// [0, 1], which is 0 or 1.  A search step is then a multiply-add with saturation and one on the entry's address
 // (taken as a denormal float, which adds like an integer): both on the two floating-point pipes, where a compare and a
 // predicated add go to the integer pipes, which have half the rate and bind the loop.  8,192 Llama-7B tokens: 4.18 ms with
-// integer entries.
-CG_HD uint32_t search_entry(uint32_t cdf) { return 0x4B000000u | cdf << 7; }
+// integer entries, 4.00 with floats when that was measured.
+CG_HD uint32_t search_entry(uint32_t cdf) { return 0x4B000000u | cdf; }
 constexpr uint32_t kSearchPadding = 0x7F800000u;  // +inf: above every estimate
 CG_HD uint32_t ld_entry(Smem sm, uint32_t addr) {
 #if defined(__CUDA_ARCH__)
@@ -321,7 +347,7 @@ CG_HD uint32_t ld_entry(Smem sm, uint32_t addr) {
     return v == 0xFFFFFFFFu ? kSearchPadding : search_entry(v >> 16);
 #endif
 }
-CG_HD uint32_t entry_c16(uint32_t entry) { return cg_fshl(0u, entry, 9u); }  // cdf << 16
+CG_HD uint32_t entry_c16(uint32_t entry) { return cg_fshl(0u, entry, 16u); }  // cdf << 16
 
 // Exact search with a run-time depth (the rare path of decode_streams).
 CG_HD uint32_t exact_search(Smem sm, uint32_t col, uint32_t a_max, uint32_t span32, uint32_t target, int levels) {
@@ -343,14 +369,15 @@ CG_HD int fast_levels_for(int nsym, int full_levels) {
     return fl;
 }
 
-// 2^23 (1 + offset / span) + 1, to about 2 (see search_entry); anything when the span is the full 2^32 (span32 == 0).
+// 128 + (floor(2^16 offset / span) + 1) / 2^16, or one 2^16th off where the quotient is within 2^-6 or so of a whole number:
+// a float from 128 on has sixteen bits behind the point, so the rounding of the last addition is the floor (see search_entry).  Anything when the span is the full 2^32 (span32 == 0).
 CG_HD float ratio_estimate(uint32_t offset, uint32_t span32) {
 #if defined(__CUDA_ARCH__)
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_rn(span32)));
-    return __fmaf_rn(__uint2float_rn(offset), r * 8388608.0f, 8388609.0f);
+    return __fmaf_rz(__uint2float_rn(offset), r, 128.0f + 1.0f / 65536.0f);
 #else
-    return span32 ? static_cast<float>(offset) * (8388608.0f / static_cast<float>(span32)) + 8388609.0f : 8388609.0f;
+    return span32 ? 128.0f + static_cast<float>((static_cast<uint64_t>(offset) << 16) / span32 + 1u) * (1.0f / 65536.0f) : 128.0f;
 #endif
 }
 // address a, or a + STEP if the entry is not above the ratio
@@ -358,12 +385,12 @@ template <uint32_t STEP>
 CG_HD uint32_t search_step(uint32_t a, uint32_t entry, float ratio) {
 #if defined(__CUDA_ARCH__)
     float take;
-    asm("sub.rn.sat.f32 %0, %1, %2;" : "=f"(take) : "f"(ratio), "f"(__uint_as_float(entry)));
+    asm("{ .reg .f32 n; neg.f32 n, %2; fma.rn.sat.f32 %0, %1, 0f47800000, n; }" : "=f"(take) : "f"(ratio), "f"(__uint_as_float(entry)));
     return __float_as_uint(__fmaf_rn(take, __uint_as_float(STEP), __uint_as_float(a)));
 #else
     float e;
     __builtin_memcpy(&e, &entry, 4);
-    return ratio - e >= 1.0f ? a + STEP : a;
+    return ratio * 65536.0f - e >= 1.0f ? a + STEP : a;
 #endif
 }
 // Search steps: the candidate entry is kTableRowBytes << B bytes above `a`.
@@ -387,8 +414,8 @@ struct RatioSearch<-1> {
 // integer pipe a warp, measured).  The symbol is then checked exactly: the offset must lie inside its scaled
 // bounds, which the range update needs anyway.  The caller picks FL from what it knows about the symbols (a
 // row quantised to `bins` bins holds symbols 0 .. bins-2, so 2^FL >= bins is enough).  The result depends
-// on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol >= 2^FL - 1, a symbol that starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away
-// and the whole warp repeats that symbol with the exact, full-depth search.
+// on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol >= 2^FL - 1, a symbol that
+// starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away and the whole warp repeats that symbol with the exact, full-depth search.
 //
 // The table's last symbol has no upper entry.  With LAST_REPEATED the rows above its entry hold copies of it,
 // so that its bounds are equal and the check fails; otherwise they hold kSearchPadding and
@@ -397,46 +424,73 @@ struct RatioSearch<-1> {
 //   col[i]    table column of stream i (see decode_stream)
 //   det       address threshold of entry min(2^FL - 1, maxsym): column-independent because a column's offset
 //             inside a table row is below kTableRowBytes (det = table base + entry * kTableRowBytes)
-//   emit(a, t4)  receives the NS table-entry addresses of one token's symbols and four times the
-//             token's index (ntok >= 1)
+//   emit(a, t4)  receives the NS table-entry addresses of one token's symbols and the start value of t4
+//             plus four times the token's index (ntok >= 1)
 template <int FL, int NS, bool LAST_REPEATED = false, class Emit>
 CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int maxsym, int full_levels,
                           const uint8_t *const (&stream)[NS], const uint32_t (&len)[NS], int ntok, uint32_t lanes,
-                          Emit emit) {
+                          Emit emit, uint32_t t4 = 0u) {
     static_assert(FL >= 2, "the first level's entry is held in a register");
     BitWindow bw[NS];
     DecoderState st[NS];
-    uint32_t mid[NS], a_max[NS];
+    uint32_t mid[NS];
     constexpr uint32_t kTop = static_cast<uint32_t>(kTableRowBytes) << (FL - 1);
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
     for (int i = 0; i < NS; ++i) {
-        st[i].low = 0u;
-        st[i].span32 = 0u;
-        st[i].offset = bw[i].open(stream[i], len[i]);
-        a_max[i] = col[i] + static_cast<uint32_t>(maxsym) * kTableRowBytes;
+        st[i].init();
+        bw[i].open(stream[i], len[i]);
         mid[i] = ld_entry(sm, col[i] + kTop);
     }
     uint32_t a[NS], flo[NS], fhi[NS];
-    const uint32_t last4 = static_cast<uint32_t>(ntok - 1) * 4u;
-    uint32_t t4 = 0u;  // four times the token index: the caller's emit indexes 4-byte per-token data with it
-    // The inner loop is the common case and nothing else, left by one vote for a refill of the bit windows, for a
+    const uint32_t last4 = t4 + static_cast<uint32_t>(ntok - 1) * 4u;
+    bool odd = true;  // the first symbol starts from the full range
+    // The inner loop is the common case and nothing else, left by one vote for a window that has been read to its end, for a
     // symbol whose fast search failed and at the last token; with that code inside it, every pass executed more
     // instructions, whether it took that code or not.
     for (;;) {
+        if (odd) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) {
+                const uint32_t offset = st[i].exact_offset(bw[i]);
+                const uint32_t a_max = col[i] + static_cast<uint32_t>(maxsym) * kTableRowBytes;
+                a[i] = exact_search(sm, col[i], a_max, st[i].span32, offset, full_levels);
+                flo[i] = scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i])));
+                fhi[i] = (a[i] == a_max) ? st[i].span32
+                                            : scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i] + kTableRowBytes)));
+            }
+            emit(a, t4);
+            if (t4 == last4) break;  // no range update for the last symbol (dec_new.cu:273-275)
+            t4 += 4u;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int i = 0; i < NS; ++i) st[i].exact_update(flo[i], fhi[i]);
+        }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int i = 0; i < NS; ++i) bw[i].advance(st[i].p);
+        uint32_t low[NS], u[NS], s[NS];
+        int32_t p[NS];
+        bool rare;  // a symbol that fails the check
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
         for (;;) {
             float ratio[NS];
-            bool rare = false;  // a symbol that fails the check
-            int fewest = bw[0].nbits;
+            uint32_t bits[NS];
+            int32_t beyond = 0;
+            rare = false;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
             for (int i = 0; i < NS; ++i) {
-                ratio[i] = ratio_estimate(st[i].offset, st[i].span32);
+                bits[i] = bw[i].bits(st[i].p);
+                ratio[i] = ratio_estimate(bits[i] - st[i].low, st[i].span32);
                 a[i] = search_step<kTop>(col[i], mid[i], ratio[i]);
             }
 #if defined(__CUDA_ARCH__)
@@ -455,60 +509,42 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
 #pragma unroll
 #endif
             for (int i = 0; i < NS; ++i) {
-                flo[i] = cg_umulhi(st[i].span32, e0[i]);
-                fhi[i] = cg_umulhi(st[i].span32, e1[i]);
-                rare = rare | (st[i].offset - flo[i] >= fhi[i] - flo[i]);
-                fewest = fewest < bw[i].nbits ? fewest : bw[i].nbits;
+                const uint32_t f0 = cg_umulhi_wide(st[i].span32, e0[i]), f1 = cg_umulhi_wide(st[i].span32, e1[i]);
+                low[i] = st[i].low + f0;
+                u[i] = f1 - f0;
+                rare = rare | (bits[i] - low[i] >= u[i]);
                 if (!LAST_REPEATED) rare = rare | (a[i] >= det);
+                s[i] = renorm_shift_by_size(low[i], u[i]);
+                p[i] = st[i].p + static_cast<int32_t>(s[i]);
+                beyond |= p[i];
             }
-            if (cg_any_lane(lanes, rare | (fewest < BitWindow::kShort) | (t4 == last4))) break;
+            if (cg_any_lane(lanes, rare | ((beyond & ~31) != 0) | (t4 == last4))) break;
             emit(a, t4);
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-            for (int i = 0; i < NS; ++i) st[i].update(flo[i], fhi[i], bw[i]);
             t4 += 4u;
-        }
-        if (t4 == last4) break;
-        bool low = false, odd = false;
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-        for (int i = 0; i < NS; ++i) {
-            low = low || bw[i].short_of_bits();
-            odd = odd || st[i].offset - flo[i] >= fhi[i] - flo[i];
-            if (!LAST_REPEATED) odd = odd || a[i] >= det;
-        }
-        if (cg_any_lane(lanes, low)) {
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-            for (int i = 0; i < NS; ++i) bw[i].refill();
-        }
-        if (cg_any_lane(lanes, odd)) {
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
             for (int i = 0; i < NS; ++i) {
-                a[i] = exact_search(sm, col[i], a_max[i], st[i].span32, st[i].offset, full_levels);
-                flo[i] = scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i])));
-                fhi[i] = (a[i] == a_max[i]) ? st[i].span32
-                                            : scale_exact(st[i].span32, entry_c16(ld_entry(sm, a[i] + kTableRowBytes)));
+                st[i].low = cg_fshl(0u, low[i], s[i]);
+                st[i].span32 = cg_fshl(0u, u[i], s[i]);
+                st[i].p = p[i];
             }
         }
-        emit(a, t4);
+        odd = cg_any_lane(lanes, rare);
+        if (!odd) {
+            emit(a, t4);
+            if (t4 == last4) break;
+            t4 += 4u;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-        for (int i = 0; i < NS; ++i) st[i].update(flo[i], fhi[i], bw[i]);
-        t4 += 4u;
+            for (int i = 0; i < NS; ++i) {
+                st[i].low = cg_fshl(0u, low[i], s[i]);
+                st[i].span32 = cg_fshl(0u, u[i], s[i]);
+                st[i].p = p[i];
+            }
+        }
     }
-    // last symbol: no range update (dec_new.cu:273-275), so no new bits either
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-    for (int i = 0; i < NS; ++i) a[i] = exact_search(sm, col[i], a_max[i], st[i].span32, st[i].offset, full_levels);
-    emit(a, t4);
 }
 
 // One stream.  col: address of the stream's table column (see search_entry), rows kTableRowBytes apart,

@@ -2,6 +2,8 @@
 //
 // The per-stream loop lives in cg_coder.cuh; this file stages tables, offsets and scales around it
 // and writes either raw symbols (the torchac_cuda entry points) or dequantised 16-bit KV (fused path).
+#include <type_traits>
+
 #include "cg_common.cuh"
 
 namespace cg {
@@ -36,34 +38,60 @@ __device__ __forceinline__ void copy_run_async(void *smem, const void *global, i
 __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 constexpr int kMaxStagedLp = 33;  // longer tables would need more registers than the decode loop has
 __device__ __forceinline__ int staged_run_offset(int lp, int rows) { return rows * kRowBytes - lp * kGroup * 2; }
-// Thread t's channels are 2t and 2t + 1, in columns t and t + 64.  rows: the columns' rows, filled up with the last
-// entry.  Called by all threads.
-__device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int tid) {
-    constexpr int kHold = (kMaxStagedLp + 1) / 2;
-    const int off = staged_run_offset(lp, rows), below = off / kRowBytes, n = lp - 1;
-    const uint16_t *run = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(tab) + off) + 2 * tid * lp;
-    uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
-    const int direct = min(n, below);
-    for (int m = 0; m < direct; ++m) {
-        c0[m * kGroup] = search_entry(run[m]);
-        c1[m * kGroup] = search_entry(run[lp + m]);
-    }
-    uint32_t hold[kHold];
+// Thread t's channels are 2t and 2t + 1, in columns t and t + 64: their 2 lp entries are lp whole words of the run, which no
+// two lanes of a warp read from one bank when lp is odd.  Every thread holds its words before any of them spreads its own.
+// rows: the columns' rows, filled up with the last entry.  Called by all threads.
+template <int LP>
+__device__ __forceinline__ void spread_words(uint32_t *tab, int rows, int tid) {
+    const uint32_t *run = tab + (staged_run_offset(LP, rows) >> 2) + tid * LP;
+    uint32_t w[LP];
 #pragma unroll
-    for (int k = 0; k < kHold; ++k)
-        hold[k] = direct + k < n ? static_cast<uint32_t>(run[direct + k]) | static_cast<uint32_t>(run[lp + direct + k]) << 16 : 0u;
+    for (int k = 0; k < LP; ++k) w[k] = run[k];
+    __syncthreads();
+    uint32_t *c0 = tab + tid, *c1 = c0 + kGroup / 2, e = 0u;
+#pragma unroll
+    for (int h = 0; h < 2 * LP; ++h) {
+        const int m = h < LP ? h : h - LP;
+        if (m == LP - 1) continue;
+        e = __byte_perm(w[h >> 1], 0x4B000000u, h & 1 ? 0x7632 : 0x7610);  // search_entry of one half
+        (h < LP ? c0 : c1)[m * kGroup] = e;
+    }
+    const uint32_t last0 = c0[(LP - 2) * kGroup];
+    for (int m = LP - 1; m < rows; ++m) {
+        c0[m * kGroup] = last0;
+        c1[m * kGroup] = e;
+    }
+}
+__device__ __forceinline__ void spread_run(uint32_t *tab, int lp, int rows, int tid) {
+    if (lp == 33) return spread_words<33>(tab, rows, tid);
+    if (lp == 17) return spread_words<17>(tab, rows, tid);
+    const uint16_t *run = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(tab) + staged_run_offset(lp, rows)) + 2 * tid * lp;
+    uint32_t *c0 = tab + tid, *c1 = tab + tid + kGroup / 2;
+    const int n = lp - 1;
+    uint32_t hold[kMaxStagedLp - 1];
+#pragma unroll
+    for (int k = 0; k < kMaxStagedLp - 1; ++k)
+        hold[k] = k < n ? static_cast<uint32_t>(run[k]) | static_cast<uint32_t>(run[lp + k]) << 16 : 0u;
     const uint32_t last0 = search_entry(run[n - 1]), last1 = search_entry(run[lp + n - 1]);
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kHold; ++k)
-        if (direct + k < n) {
-            c0[(direct + k) * kGroup] = search_entry(hold[k] & 0xFFFFu);
-            c1[(direct + k) * kGroup] = search_entry(hold[k] >> 16);
+    for (int k = 0; k < kMaxStagedLp - 1; ++k)
+        if (k < n) {
+            c0[k * kGroup] = search_entry(hold[k] & 0xFFFFu);
+            c1[k * kGroup] = search_entry(hold[k] >> 16);
         }
     for (int m = n; m < rows; ++m) {
         c0[m * kGroup] = last0;
         c1[m * kGroup] = last1;
     }
+}
+
+// A lane behind the last channels decodes what the last lane before it does, from that one's columns, and stores the same to the
+// same place: whole warps run the loop, so that neither their votes nor their stores need a mask.
+__device__ __forceinline__ void borrow_stream(int64_t &start, int &len, uint32_t lanes) {
+    const int from = min(static_cast<int>(threadIdx.x & 31), 31 - __clz(static_cast<int>(lanes)));
+    start = __shfl_sync(0xFFFFFFFFu, start, from);
+    len = __shfl_sync(0xFFFFFFFFu, len, from);
 }
 
 // ---- symbol-output kernels (decode_fast_prefsum / decode_fast_new) -----------------------------------
@@ -131,8 +159,8 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
 }
 
 // The same with two adjacent channels per thread, whose symbols are adjacent bytes (see decode_dequant_multi_kernel):
-// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk: 168 us under counters, of which the last 272 of
-// 2,048 blocks, which find no room beside the first, take a third.
+// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk: 158 us under counters (168 with the window shifted at
+// every symbol), of which the last 272 of 2,048 blocks, which find no room beside the first, take a third.
 // Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
 // more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
 constexpr int kMultiBlocksPerSM = 12;
@@ -195,10 +223,11 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         for (int i = 0; i < 2; ++i) upper |= entry_c16(tab[kHalf * kGroup + tid + i * kThreads]) < (0x10000u - 2u * kHalf) << 16;
     }
     const bool shallow = LEVELS > 3 && !__syncthreads_or(upper);
-    if (!active) return;  // a thread reads its own columns only
+    if (lanes == 0u) return;  // no block barrier from here on
     bool bad = false;
     const uint8_t *streams[2];
-    uint32_t lens[2];
+    uint32_t lens[2], col[2];
+    const int c = min(c0, p.nchannels - 2);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         if (len[i] < 0) { len[i] = 0; bad = true; }
@@ -206,20 +235,27 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         if (start[i] > p.nbytes) { start[i] = p.nbytes; bad = true; }
         if (start[i] + len[i] > p.nbytes) { len[i] = p.nbytes - start[i]; bad = true; }
         if (len[i] > (1 << 20)) len[i] = 1 << 20;
+        int n = static_cast<int>(len[i]);
+        if (lanes != 0xFFFFFFFFu) borrow_stream(start[i], n, lanes);
+        col[i] = smem_addr(tab + min(tid, static_cast<int>(p.nchannels - blockIdx.x * kGroup) / 2 - 1) + i * kThreads);
         streams[i] = p.bytes + start[i];
-        lens[i] = static_cast<uint32_t>(len[i]);
+        lens[i] = static_cast<uint32_t>(n);
     }
-    if (bad && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
-    uint8_t *o = p.out + row * p.o0 + c0;
+    if (bad && active && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
+    uint8_t *o = p.out + row * p.o0 + c;
+    // the two symbols as bytes of one word: two multiply-adds on the entries' addresses as denormal floats (see search_entry),
+    // the first rounded down, the second exact
+    uint32_t less = 0x80000000u | ((col[0] >> 9) + (col[1] >> 1));
     int64_t o1 = p.o1;
-    asm volatile("" : "+l"(o1));
-    const uint32_t col[2] = {smem_addr(tab + tid), smem_addr(tab + tid + kThreads)};
+    asm volatile("" : "+l"(o1), "+r"(less));
     auto emit = [&](const uint32_t (&a)[2], uint32_t) {
-        *reinterpret_cast<uint16_t *>(o) = static_cast<uint16_t>((a[0] - col[0]) / kRowBytes | (a[1] - col[1]) / kRowBytes << 8);
+        const float m0 = __fmaf_rd(__uint_as_float(a[0]), 1.0f / kRowBytes, __uint_as_float(less));
+        const uint32_t both = __float_as_uint(__fmaf_rn(__uint_as_float(a[1]), 256.0f / kRowBytes, m0));
+        *reinterpret_cast<uint16_t *>(o) = static_cast<uint16_t>(both);
         o += o1;
     };
-    if (shallow) decode_streams<(LEVELS > 3 ? LEVELS - 1 : LEVELS), 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
-    else decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, lanes, emit);
+    if (shallow) decode_streams<(LEVELS > 3 ? LEVELS - 1 : LEVELS), 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, 0xFFFFFFFFu, emit);
+    else decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, 0xFFFFFFFFu, emit);
 }
 
 // ---- one warp per stream (kept for comparison) -------------------------------------------------------------
@@ -250,20 +286,20 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_warp_kernel(const SymDe
                              : 0u;
     BitWindow bw;
     DecoderState st;
-    st.low = 0u;
-    st.span32 = 0u;
-    st.offset = bw.open(p.bytes + start, static_cast<uint32_t>(len));
+    st.init();
+    bw.open(p.bytes + start, static_cast<uint32_t>(len));
     uint8_t *o = p.out + row * p.o0 + c * p.o2;
     for (int i = 0; i < p.ntokens; ++i) {
+        const uint32_t offset = st.exact_offset(bw);
         const uint32_t f = scale_exact(st.span32, c16);
-        const uint32_t votes = __ballot_sync(0xFFFFFFFFu, lane <= maxsym && f <= st.offset);
+        const uint32_t votes = __ballot_sync(0xFFFFFFFFu, lane <= maxsym && f <= offset);
         const int sym = 31 - __clz(static_cast<int>(votes | 1u));  // entry 0 is always taken
         if (lane == 0) o[i * p.o1] = static_cast<uint8_t>(sym);
         if (i == p.ntokens - 1) break;
         const uint32_t flo = __shfl_sync(0xFFFFFFFFu, f, sym);
         const uint32_t fnext = __shfl_sync(0xFFFFFFFFu, f, (sym + 1) & 31);
-        st.update(flo, sym == maxsym ? st.span32 : fnext, bw);
-        if (bw.low_water()) bw.refill();
+        st.exact_update(flo, sym == maxsym ? st.span32 : fnext);
+        if (st.p >= 32) bw.advance(st.p);
     }
 }
 
@@ -391,10 +427,11 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
 // values with one 2*NS-byte store.  Channel NS*t + i keeps its table in column t + i * (128 / NS), so a
 // warp still reads 32 different banks whatever entries its lanes are at.  The search depth is chosen
 // per block from the row's bin count (see decode_streams); the result does not depend on it.
-// Bound by instruction issue and by the two half-rate integer pipes (58.9 instructions for 32 symbols, four issue slots of
-// five): 8,192 Llama-7B tokens in 4.00 ms, 1,317 GB/s of algorithmic bytes; 4.18 ms with the search and the renormalisation on
-// the integer pipes and the rare cases inside the loop, 4.50 before the search on an estimate.
-// Needs a head size and output strides that are multiples of NS and output pointers aligned to 2*NS bytes.
+// Bound by instruction issue and by the two half-rate integer pipes (52.4 instructions for 32 symbols, four issue slots of
+// five).  8,192 Llama-7B tokens: 3.68 ms; 4.02 and 58.9 instructions with the window shifted at every symbol, the shift by
+// the interval's size less one, votes for the active lanes only, 64-bit steps and the tables staged by halves of words.
+// Needs a head size and output strides that are multiples of NS, output pointers aligned to 2*NS bytes and a block's output
+// within 32-bit offsets.
 template <int OUT_DT>
 __device__ __forceinline__ uint32_t pack_pair(float v0, float v1);
 template <>
@@ -482,7 +519,7 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     const int cq = cqf >= 0.0f && cqf < 64.0f ? static_cast<int>(cqf) : 64;
     uint32_t *tabs[NS];
 #pragma unroll
-    for (int i = 0; i < NS; ++i) tabs[i] = smem + tid + i * kThreads;
+    for (int i = 0; i < NS; ++i) tabs[i] = smem + min(tid, static_cast<int>(p.nchannels - blockIdx.x * kGroup) / NS - 1) + i * kThreads;
     if (run_staged) {
         wait_copies();
         __syncthreads();
@@ -553,36 +590,58 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     }
     if (bad && active && p.status) atomicOr(p.status, CG_S_BAD_LENGTHS);
     __syncthreads();
-    if (!active) {
+    if (lanes == 0u) {
         if (p.after == kAfterBatch) wait_for_launch_before();
         return;
     }
 
-    const int h = c0 / p.head_size, d = c0 - h * p.head_size;
-    uint16_t *o = static_cast<uint16_t *>(job.out) + layer * p.o_layer + kv * p.o_kv + h * p.o_head + d;
+    const int c = min(c0, p.nchannels - NS);
     uint32_t col[NS];
+    const uint8_t *streams[NS];
+    uint32_t lens[NS];
 #pragma unroll
-    for (int i = 0; i < NS; ++i) col[i] = smem_addr(tabs[i]);
-    // entry m of the row's (s - Cq)/Cq table is at lut + 4m = (a >> 7) + lut_k for an entry address a
-    // of column 0, because a - col is a multiple of 512; column i starts 4 * kThreads bytes further,
-    // which adds kThreads / 32 to (a >> 7)
-    uint32_t lut_k = smem_addr(lut) - (col[0] >> 7);
-    int64_t o_token = p.o_token;
-    uint32_t sc_a = smem_addr(scale_f);
+    for (int i = 0; i < NS; ++i) {
+        if (lanes != 0xFFFFFFFFu) borrow_stream(start[i], len[i], lanes);
+        col[i] = smem_addr(tabs[i]);
+        streams[i] = job.bytes + start[i];
+        lens[i] = static_cast<uint32_t>(len[i]);
+    }
+    // Byte offsets from the block's first head, which is the same for all threads, fit 32 bits (offsets_fit; DELTA takes any).
+    using Offset = std::conditional_t<DELTA, int64_t, uint32_t>;
+    const int h0 = blockIdx.x * kGroup / p.head_size, h = c / p.head_size, d = c - h * p.head_size;
+    char *out = reinterpret_cast<char *>(static_cast<uint16_t *>(job.out) + layer * p.o_layer + kv * p.o_kv + h0 * p.o_head);
+    Offset o = (static_cast<Offset>(h - h0) * static_cast<Offset>(p.o_head) + static_cast<Offset>(d)) * 2;
+    Offset o_token = static_cast<Offset>(p.o_token) * 2;
+    // entry m of the row's (s - Cq)/Cq table is at lut + 4m: a 128th of an entry's address, rounded down, plus a constant, taken
+    // as denormal floats (see search_entry), because a - col is a multiple of 512
+    uint32_t lut_k[NS];
+    const uint32_t sc_a = smem_addr(scale_f);
     int ntok_r = ntok;
     // keep the loop's invariants in registers instead of re-deriving them from kernel parameters
-    asm volatile("" : "+l"(o_token), "+r"(lut_k), "+r"(sc_a), "+r"(ntok_r));
+    if constexpr (DELTA) asm volatile("" : "+l"(o_token), "+r"(ntok_r));
+    else asm volatile("" : "+r"(o_token), "+r"(ntok_r));
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        lut_k[i] = smem_addr(lut) - (col[i] >> 7);
+        asm volatile("" : "+r"(lut_k[i]));
+    }
     float anchor[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i) anchor[i] = 0.0f;
-    auto emit = [&](const uint32_t (&a)[NS], uint32_t t4) {
+    // at: the address of the token's scale
+    auto emit = [&](const uint32_t (&a)[NS], uint32_t at) {
         // ((sym - Cq) / Cq) * max in fp32, then one round-to-nearest cast (cachegen_decoder.py:30-33,171-173)
-        const float s = ldsf32(sc_a);
+        const float s = ldsf32(at);
+
         float v[NS];
-        if (!DELTA || (t4 & group_mask) == 0u) {
+        uint32_t entry[NS];
+#pragma unroll
+        for (int i = 0; i < NS; ++i)
+            entry[i] = __float_as_uint(__fmaf_rd(__uint_as_float(a[i]), 4.0f / kRowBytes, __uint_as_float(lut_k[i])));
+        if (!DELTA || ((at - sc_a) & group_mask) == 0u) {
 #pragma unroll
             for (int i = 0; i < NS; ++i) {
-                v[i] = __fmul_rn(ldsf32((a[i] >> 7) + lut_k - i * (kThreads / 32)), s);
+                v[i] = __fmul_rn(ldsf32(entry[i]), s);
                 if (DELTA)  // what the encoder subtracted from the group's other tokens: the value in the KV dtype
                     anchor[i] = scale_dt == CG_BF16 ? Half16<CG_BF16>::to_float(Half16<CG_BF16>::from_float(v[i]))
                                                     : Half16<CG_F16>::to_float(Half16<CG_F16>::from_float(v[i]));
@@ -590,33 +649,25 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
         } else {
 #pragma unroll
             for (int i = 0; i < NS; ++i)
-                v[i] = __fadd_rn(anchor[i], __fmul_rn(ldsf32((a[i] >> 7) + lut_k - i * (kThreads / 32) + 4u * CG_MAX_LP), s));
+                v[i] = __fadd_rn(anchor[i], __fmul_rn(ldsf32(entry[i] + 4u * CG_MAX_LP), s));
         }
         if (NS == 2) {
-            *reinterpret_cast<uint32_t *>(o) = pack_pair<OUT_DT>(v[0], v[1]);
+            *reinterpret_cast<uint32_t *>(out + o) = pack_pair<OUT_DT>(v[0], v[1]);
         } else {
-            *reinterpret_cast<uint2 *>(o) = make_uint2(pack_pair<OUT_DT>(v[0], v[1]), pack_pair<OUT_DT>(v[2 % NS], v[3 % NS]));
+            *reinterpret_cast<uint2 *>(out + o) = make_uint2(pack_pair<OUT_DT>(v[0], v[1]), pack_pair<OUT_DT>(v[2 % NS], v[3 % NS]));
         }
         o += o_token;
-        sc_a += 4u;
     };
     const int maxsym = p.lp - 2;
     const int fl = fast_levels_for(2 * cq + 1, full_levels);
     const int top = (1 << fl) - 1;
     const uint32_t det = smem_addr(smem) + static_cast<uint32_t>(top < maxsym ? top : maxsym) * kRowBytes;
-    const uint8_t *streams[NS];
-    uint32_t lens[NS];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {
-        streams[i] = job.bytes + start[i];
-        lens[i] = static_cast<uint32_t>(len[i]);
-    }
     switch (fl) {
-    case 2: decode_streams<2, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 3: decode_streams<3, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 4: decode_streams<4, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    case 5: decode_streams<5, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
-    default: decode_streams<6, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, lanes, emit); break;
+    case 2: decode_streams<2, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 3: decode_streams<3, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 4: decode_streams<4, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 5: decode_streams<5, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    default: decode_streams<6, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
     }
     if (p.after == kAfterBatch) wait_for_launch_before();
 }
@@ -663,6 +714,13 @@ static bool multi_layout_ok(const FusedDecodeParams &p, int ns) {
     for (int j = 0; j < p.njobs; ++j)
         if (reinterpret_cast<uintptr_t>(p.jobs[j].out) & (2 * ns - 1)) return false;
     return true;
+}
+
+// A block's output within 32-bit byte offsets of its first head: 256 tokens of the heads that 128 channels touch.  A head's
+// tokens 2 GB apart in all go to the general kernel, which takes 64-bit steps.
+static bool offsets_fit(const FusedDecodeParams &p) {
+    const int64_t most = (int64_t{1} << 31) - p.head_size, heads = kGroup / p.head_size + 1;
+    return p.o_token >= 0 && p.o_head >= 0 && p.o_head <= most / heads && p.o_token <= (most - heads * p.o_head) / kSubTokens;
 }
 
 template <int NS, int OUT_DT, bool DELTA>
@@ -934,7 +992,7 @@ static int launch_fused_any(const FusedDecodeParams &p, int scale_dtype, int out
         return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, true>(p, scale_dtype, early, st)
                                    : launch_fused_multi<2, CG_BF16, true>(p, scale_dtype, early, st);
     }
-    if (multi_layout_ok(p, 2))
+    if (multi_layout_ok(p, 2) && offsets_fit(p))
         return out_dtype == CG_F16 ? launch_fused_multi<2, CG_F16, false>(p, scale_dtype, early, st)
                                    : launch_fused_multi<2, CG_BF16, false>(p, scale_dtype, early, st);
     if (scale_dtype == CG_F16 && out_dtype == CG_F16) return launch_fused<CG_F16, CG_F16>(p, early, st);
