@@ -122,52 +122,25 @@ struct Smem {
 // no word holds, does not come about.  (Only u = 2^31 at a multiple of 2^31 gives -1: see EncoderState::steps_at and
 // DecoderState.)
 //
-// Returns s and 2^s: for the words that are only shifted left a multiply does it off the integer pipe (a
-// shift, a compare or a select takes that pipe for two cycles a warp, and a multiply-high the multiply pipe for four).
-//
 // The conditional decrement is written as a predicated add: with `if (...) --s` the counters show two executed
 // instructions a symbol more.
-struct Renorm {
-    uint32_t s, p2;
-};
 // low, high = low + d, d (or u)
-CG_HD Renorm renorm_shift(uint32_t low, uint32_t high, uint32_t d) {
-    Renorm r;
-#if defined(__CUDA_ARCH__)
-    asm("{ .reg .u32 t, b; .reg .pred p;\n"
-        "bfind.shiftamt.u32 %0, %4;\n"
-        "shf.r.wrap.b32 b, 0x80000000, 0, %0;\n"
-        "lop3.b32 t, %2, %3, b, 0x28;\n"  // (low ^ high) & b
-        "setp.eq.u32 p, t, 0;\n"
-        "@p add.u32 %0, %0, -1;\n"
-        "shf.l.wrap.b32 %1, 0, 1, %0; }"
-        : "=&r"(r.s), "=r"(r.p2) : "r"(low), "r"(high), "r"(d));
-#else
-    r.s = d ? static_cast<uint32_t>(cg_clz(d)) : 0xFFFFFFFFu;
-    if (((low ^ high) & (0x80000000u >> (r.s & 31u))) == 0u) --r.s;
-    r.p2 = 1u << (r.s & 31u);
-#endif
-    return r;
-}
-// By the size u alone: two adds fewer where only the shift is wanted.
-CG_HD uint32_t renorm_shift_by_size(uint32_t low, uint32_t u) {
+CG_HD uint32_t renorm_shift(uint32_t low, uint32_t high, uint32_t d) {
 #if defined(__CUDA_ARCH__)
     uint32_t s;
-    asm("{ .reg .u32 t, b, h; .reg .pred p;\n"
-        "add.u32 h, %1, %2;\n"
-        "add.u32 h, h, -1;\n"
-        "bfind.shiftamt.u32 %0, %2;\n"
+    asm("{ .reg .u32 t, b; .reg .pred p;\n"
+        "bfind.shiftamt.u32 %0, %3;\n"
         "shf.r.wrap.b32 b, 0x80000000, 0, %0;\n"
-        "lop3.b32 t, %1, h, b, 0x28;\n"  // (low ^ high) & b
+        "lop3.b32 t, %1, %2, b, 0x28;\n"  // (low ^ high) & b
         "setp.eq.u32 p, t, 0;\n"
         "@p add.u32 %0, %0, -1; }"
-        : "=&r"(s) : "r"(low), "r"(u));
+        : "=&r"(s) : "r"(low), "r"(high), "r"(d));
     return s;
 #else
-    return renorm_shift(low, low + u - 1u, u).s;
+    const uint32_t s = d ? static_cast<uint32_t>(cg_clz(d)) : 0xFFFFFFFFu;
+    return ((low ^ high) & (0x80000000u >> (s & 31u))) == 0u ? s - 1u : s;
 #endif
 }
-
 // ---- warp votes and products -------------------------------------------------------------------------------------
 CG_HD bool cg_any_lane(uint32_t lanes, bool pred) {
 #if defined(__CUDA_ARCH__)
@@ -322,7 +295,7 @@ struct DecoderState {
     CG_HD void exact_update(uint32_t flo, uint32_t fhi) {
         const uint32_t d = fhi - flo - 1u;
         low += flo;
-        const uint32_t s = renorm_shift(low, low + d, d).s & 31u;
+        const uint32_t s = renorm_shift(low, low + d, d) & 31u;
         low = cg_fshl(0u, low, s);
         span32 = cg_fshl(0u, fhi - flo, s);
         p += static_cast<int32_t>(s);
@@ -514,7 +487,7 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
                 u[i] = f1 - f0;
                 rare = rare | (bits[i] - low[i] >= u[i]);
                 if (!LAST_REPEATED) rare = rare | (a[i] >= det);
-                s[i] = renorm_shift_by_size(low[i], u[i]);
+                s[i] = renorm_shift(low[i], cg_add_less_one(low[i], u[i]), u[i]);
                 p[i] = st[i].p + static_cast<int32_t>(s[i]);
                 beyond |= p[i];
             }
@@ -609,9 +582,27 @@ struct BitSinkT {
     // Moves the oldest 32 pending bits out where there are 32; needs nacc < 64.  Straight-line code: every lane of the
     // warp runs it whatever it needs.  Returns whether the held word, which went to the row (as number nwords - 2 now), has
     // carried into those in front of it, which is left to the caller.
-    CG_HD bool store_word_if_full() {
+    // DEEP: up to 63 bits were pending before the last shift, by s <= 31, which moved bits out of the accumulator: `above` is
+    // its upper word before that shift.
+    template <bool DEEP = false>
+    CG_HD bool store_word_if_full(uint32_t above = 0u, uint32_t s = 0u) {
 #if defined(__CUDA_ARCH__)
         uint32_t w, held, carry, left;
+        if (DEEP)
+        asm("{ .reg .pred p, q; .reg .u32 lo, hi, x;\n"
+            "add.u32 %3, %6, -32;\n"
+            "setp.ge.s32 p, %6, 32;\n"
+            "setp.ge.s32 q, %6, 64;\n"
+            "shf.l.wrap.b32 x, %8, 0, %9;\n"    // the bits above the accumulator
+            "selp.b32 lo, %5, %4, q;\n"
+            "selp.b32 hi, x, %5, q;\n"
+            "shf.r.wrap.b32 %0, lo, hi, %3;\n"
+            "shf.r.wrap.b32 %2, hi, 0, %3;\n"
+            "lop3.b32 %2, %2, %7, 1, 0x28;\n"
+            "@!p mov.u32 %2, 0;\n"
+            "add.u32 %1, %7, %2; }"
+            : "=&r"(w), "=&r"(held), "=&r"(carry), "=&r"(left) : "r"(acc_lo), "r"(acc_hi), "r"(nacc), "r"(hold), "r"(above), "r"(s));
+        else
         asm("{ .reg .pred p;\n"
             "add.u32 %3, %6, -32;\n"
             "setp.ge.s32 p, %6, 32;\n"
@@ -635,12 +626,14 @@ struct BitSinkT {
 #else
         if (nacc < 32) return false;
         nacc -= 32;
-        const uint32_t carry = ((acc_hi >> nacc) ^ hold) & 1u;
+        const uint32_t left = static_cast<uint32_t>(nacc) & 31u, x = s & 31u ? above >> (32u - (s & 31u)) : 0u;
+        const bool q = DEEP && nacc >= 32;
+        const uint32_t carry = (((q ? x : acc_hi) >> left) ^ hold) & 1u;
         hold += carry;
         const bool over = hold < carry;
         if (nwords && (!BOUNDED || nwords - 1u < cap_w)) row[(nwords - 1u) * STEP] = cg_bswap32(hold);
         ++nwords;
-        hold = cg_fshr_clamp(acc_lo, acc_hi, static_cast<uint32_t>(nacc));
+        hold = q ? cg_fshr_clamp(acc_hi, x, left) : cg_fshr_clamp(acc_lo, acc_hi, left);
         return over;
 #endif
     }
@@ -677,12 +670,22 @@ constexpr int kSinkHighWater = 44;
 // The same where the table was counted from the `ntokens` symbols that are coded with it: a symbol that occurs has at
 // least w = floor((0xFFFF - 63) / ntokens) + 1 of the 2^16 shares (normalize_cdf_value), hence an interval of
 // w * 2^14 - 1 values or more, and adds at most 18 - floor(log2 w) bits.  0: two symbols may not fit.
-CG_HD int pair_high_water(int ntokens) {
+CG_HD int counted_symbol_bits(int ntokens) {
     const uint32_t w = (0xFFFFu - 63u) / static_cast<uint32_t>(ntokens) + 1u;
-    const int most = 18 - (31 - cg_clz(w));
+    return 18 - (31 - cg_clz(w));
+}
+CG_HD int pair_high_water(int ntokens) {
+    const int most = counted_symbol_bits(ntokens);
     if (31 + 2 * most > 63) return 0;
     return 64 - 2 * most < kSinkHighWater ? 64 - 2 * most : kSinkHighWater;
 }
+// Marks where the last symbol in front of a vote may shift pending bits out of the accumulator, because its upper word from
+// before that shift is kept (store_word_if_full<true>): only what the symbols before it add has to stay below bit 64.  For two
+// symbols of 256 counted tokens 54 instead of 44, for one of any table 64: a stream that has not got a whole word when another is at
+// the mark is soon the next one there, so a word's store every 13 bits of the fastest of a warp's streams becomes one every 22.
+// The first only where pair_high_water is not 0: what a store leaves is below it then, too.
+CG_HD int deep_pair_high_water(int ntokens) { return 64 - counted_symbol_bits(ntokens); }
+constexpr int kDeepHighWater = 64;
 
 // The coder without the reference's count of pending bits.  low is the current 32-bit window of the
 // interval's lower end L, and all bits of L above the window are in the sink: a range update adds to
@@ -723,19 +726,23 @@ struct EncoderState {
     }
     // Range update for the symbol whose scaled bounds are [flo, fhi), then renormalisation, by the interval's size (see
     // renorm_shift) or, EXACT, by its size less one.
+    // Returns the shift; above: the accumulator's upper word before it.
     template <bool EXACT, class Sink>
-    CG_HD void take(uint32_t flo, uint32_t fhi, Sink &out) {
+    CG_HD uint32_t take(uint32_t flo, uint32_t fhi, Sink &out, uint32_t &above) {
         const uint32_t u = fhi - flo;
         add_to_low(flo, out);
-        shift(renorm_shift(low, cg_add_less_one(low, u), EXACT ? u - 1u : u), u, out);
+        const uint32_t s = renorm_shift(low, cg_add_less_one(low, u), EXACT ? u - 1u : u);
+        above = out.acc_hi;
+        shift(s, u, out);
+        return s;
     }
     template <class Sink>
-    CG_HD void shift(Renorm r, uint32_t u, Sink &out) {
-        out.acc_hi = cg_fshl(out.acc_lo, out.acc_hi, r.s);
-        out.acc_lo = cg_fshl(low, out.acc_lo, r.s);
-        low *= r.p2;
-        span32 = u * r.p2;
-        out.nacc += static_cast<int>(r.s);
+    CG_HD void shift(uint32_t s, uint32_t u, Sink &out) {
+        out.acc_hi = cg_fshl(out.acc_lo, out.acc_hi, s);
+        out.acc_lo = cg_fshl(low, out.acc_lo, s);
+        low = cg_fshl(0u, low, s);
+        span32 = cg_fshl(0u, u, s);
+        out.nacc += static_cast<int>(s);
     }
     // One symbol by the address a of its table entry, the next one ROW bytes further (enc_new.cu:257-295): whatever the
     // state, by one lane alone.
@@ -744,20 +751,21 @@ struct EncoderState {
         out.store_and_carry();
         if (span32 == 0u) half_scale(out);
         const uint32_t flo = cg_umulhi_wide(span32, sm.ld(a));
-        take<true>(flo, last ? span32 : cg_umulhi_wide(span32, sm.ld(a + ROW)), out);
+        uint32_t above;
+        take<true>(flo, last ? span32 : cg_umulhi_wide(span32, sm.ld(a + ROW)), out, above);
     }
     // G symbols (1 or 2) of NS streams a lane, by the addresses of their table entries.  The streams' chains are independent,
     // and ONE warp vote after them covers a full word in an accumulator: every lane that has one stores it as soon as one
-    // lane is at the high-water mark (kSinkHighWater for one symbol, pair_high_water for two).
+    // lane is at the high-water mark (kSinkHighWater for one symbol, pair_high_water for two; with DEEP kDeepHighWater and deep_pair_high_water).
     // LAST: a symbol may be its table's last, whose upper bound is the range's end (told by `last`; G is 1 then).
     // What hardly ever happens is not mended here but left to encode_again: a carry through a whole word of ones
     // (`carried`), and a range of 2^31 at a multiple of it, which leaves a span of 0, from where on no symbol has a size, so
     // that the span is still 0 at the stream's end.  Code for the like inside the loop cost five executed instructions a
     // symbol without ever being run.
-    template <int ROW, int G, int NS, bool LAST = false, class Sink>
+    template <int ROW, int G, int NS, bool LAST = false, bool DEEP = false, class Sink>
     static CG_HD void steps_at(Smem sm, const uint32_t (&a)[G][NS], EncoderState (&enc)[NS], Sink (&out)[NS], int high_water,
                                uint32_t lanes, bool (&carried)[NS], bool last = false) {
-        uint32_t e0[G][NS], e1[G][NS];
+        uint32_t e0[G][NS], e1[G][NS], s[NS], above[NS];
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -770,14 +778,14 @@ struct EncoderState {
 #pragma unroll
             for (int i = 0; i < NS; ++i) {
                 const uint32_t fhi = cg_umulhi_wide(enc[i].span32, e1[g][i]);
-                enc[i].template take<false>(cg_umulhi_wide(enc[i].span32, e0[g][i]), LAST && last ? enc[i].span32 : fhi, out[i]);
+                s[i] = enc[i].template take<false>(cg_umulhi_wide(enc[i].span32, e0[g][i]), LAST && last ? enc[i].span32 : fhi, out[i], above[i]);
             }
         bool full = false;
 #pragma unroll
         for (int i = 0; i < NS; ++i) full |= out[i].nacc >= high_water;
         if (cg_any_lane(lanes, full)) {
 #pragma unroll
-            for (int i = 0; i < NS; ++i) carried[i] |= out[i].store_word_if_full();
+            for (int i = 0; i < NS; ++i) carried[i] |= out[i].template store_word_if_full<DEEP>(above[i], s[i]);
         }
     }
     // whether a stream has met what steps_at leaves
@@ -787,8 +795,8 @@ struct EncoderState {
     // to two bits; returns the stream length in bytes
     template <class Sink>
     CG_HD uint32_t flush(Sink &out) {
-        if (span32) shift(renorm_shift(low, cg_add_less_one(low, span32), span32 - 1u), span32, out);  // see take
-        if (out.nacc < 64) out.store_and_carry();
+        out.store_and_carry();
+        if (span32) shift(renorm_shift(low, cg_add_less_one(low, span32), span32 - 1u), span32, out);  // see take: two bits at most
         add_to_low(0x40000000u, out);
         out.acc_hi = cg_fshl(out.acc_lo, out.acc_hi, 2u);
         out.acc_lo = cg_fshl(low, out.acc_lo, 2u);

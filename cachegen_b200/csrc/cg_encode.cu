@@ -36,8 +36,9 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint8_t
     return enc.flush(out);
 }
 
-// Bound by instruction issue, most of all on the integer pipe: one 256-token Llama-7B chunk in 99 us under counters (34.7
-// instructions for 32 symbols, 14.1 of them there); 108 (38.0, 17.5) with every symbol compared with the table's last one, 125
+// Bound by instruction issue, most of all on the integer pipe: one 256-token Llama-7B chunk in 95 us under counters (32.8
+// instructions for 32 symbols, 14.5 of them there); 99.5 (34.7) with words stored at 44 pending bits, shifts as multiplies and votes
+// of the active lanes, 108 (38.0, 17.5) with every symbol compared with the table's last one, 125
 // before the loop without rare cases and with symbols fetched a group ahead of the coder (three of eight stall cycles were loads).
 // NARROW: the symbols of a row lie within 4 GB of its first, so that a symbol's address is a 32-bit offset
 template <bool NARROW>
@@ -45,10 +46,10 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     extern __shared__ uint32_t tab[];
     const int tid = threadIdx.x;
     const int row = blockIdx.y, sub = blockIdx.z;
-    const int c = blockIdx.x * kGroup + tid;
-    // the lanes that encode together, taken while the warp is still converged
-    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, c < p.nchannels);
-    if (c >= p.nchannels) return;  // no block barrier in this kernel
+    if (blockIdx.x * kGroup + (tid & ~31) >= p.nchannels) return;  // no block barrier in this kernel
+    // a lane past the last channel repeats the last, with no room to write to, so that the votes need no mask
+    const int c = min(blockIdx.x * kGroup + tid, p.nchannels - 1);
+    const bool active = blockIdx.x * kGroup + tid < p.nchannels;
     const int nrows = gridDim.y;
     const int64_t g = static_cast<int64_t>(row) * p.nchannels + c;
     const int t0 = sub * kSubTokens;
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     const uint32_t col = smem_addr(tab + tid);
     const int64_t slot = static_cast<int64_t>(sub) * nrows * p.nchannels + g;
     BitSink out[1];
-    out[0].init(p.scratch + slot * p.stride, p.stride);
+    out[0].init(p.scratch + slot * p.stride, active ? p.stride : 0);
 
     using Offset = typename std::conditional<NARROW, uint32_t, int64_t>::type;
     const uint8_t *base = reinterpret_cast<const uint8_t *>(p.sym) + row * p.s0 + static_cast<int64_t>(t0) * p.s1;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     const auto code = [&](uint32_t sym) {
         largest = max(largest, sym);
         const uint32_t s = min(sym, top), a[1][1] = {{col + s * kRowBytes}};
-        EncoderState::steps_at<kRowBytes, 1, 1, true>(Smem{}, a, enc, out, kSinkHighWater, lanes, carried, s == top);
+        EncoderState::steps_at<kRowBytes, 1, 1, true, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried, s == top);
     };
     const Offset first = at;
     uint32_t buf[kPrefetch], next[kPrefetch];
@@ -97,14 +98,14 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
         uint32_t most = buf[0];
 #pragma unroll
         for (int j = 1; j < kPrefetch; ++j) most = max(most, buf[j]);
-        if (cg_any_lane(lanes, most >= top)) {
+        if (cg_any_lane(0xFFFFFFFFu, most >= top)) {
 #pragma unroll
             for (int j = 0; j < kPrefetch; ++j) code(buf[j]);
         } else {
 #pragma unroll
             for (int j = 0; j < kPrefetch; ++j) {
                 const uint32_t a[1][1] = {{col + buf[j] * kRowBytes}};
-                EncoderState::steps_at<kRowBytes, 1, 1>(Smem{}, a, enc, out, kSinkHighWater, lanes, carried);
+                EncoderState::steps_at<kRowBytes, 1, 1, false, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried);
             }
         }
 #pragma unroll
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
         code(__ldg(base + at));
         at += s1;
     }
+    if (!active) return;
     const uint32_t nbytes = enc[0].unsettled(carried[0]) ? encode_again<Offset>(col, base, first, s1, n, top, p.scratch + slot * p.stride, p.stride)
                                                          : enc[0].flush(out[0]);
     p.lengths[slot] = static_cast<int32_t>(nbytes);

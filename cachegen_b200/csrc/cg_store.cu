@@ -348,7 +348,7 @@ struct StoreParams {
     const uint32_t *sym4;
     TableOut out;
     int ntokens, nchannels, lp, nrows, nsub;
-    int high_water;       // see pair_high_water
+    int high_water;       // of two symbols a vote, see deep_pair_high_water; 0: one
     uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4 + 1, 32 lanes] words
     int64_t stride;
     int32_t *lengths;     // [nsub, nrows * C]
@@ -448,11 +448,14 @@ static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint32_
 // second read comes from the L2.  Otherwise the tables come from packed_tables_kernel.
 // The last block of a sub-chunk turns the group sizes into offsets, the last of all writes the tail.
 // Bound by instruction issue (the coder's serial step, half of it on the integer pipe): a 256-token Llama-7B
-// chunk takes 107 us with its tables under counters, 0.63 T symbols/s, 34.6 instructions for 32 symbols; 122 us and 40.4 with
-// the code for rare cases inside the loop, a mask kept as the interval's size and a vote a symbol.  Eight blocks an SM leave the compiler 64
+// chunk takes 104 us with its tables under counters, 0.64 T symbols/s, 32.9 instructions for 32 symbols; 107 us and 34.5 with the
+// shifts as multiplies by a power of two made for them and words stored at 44 pending bits, 122 us and 40.4 with
+// the code for rare cases inside the loop besides, and a vote a symbol.  33 us of it are there without the coder's loop (the counts,
+// the tables and two waves' latencies), 12 are the votes and stores.  Eight blocks an SM leave the compiler 64
 // registers.  (Seven, for two even waves of a chunk's 2,048 blocks, take the same.)
 // Two streams a thread share the step's vote and hide each other's latencies: 1,999 tokens of 32 layers x 1,024
-// channels in 164 us under counters (28.5 instructions for 32 symbols), 172 before the same change; 180 with one stream.
+// channels in 152 us under counters (26.4 instructions for 32 symbols), 164 (28.5) and 172 before the same changes; 180 with one
+// stream.  (One stream and 32, 40 and 48 warps an SM in place of 24: 168, 171 and 171 us at the time of the 164.)
 // G symbols a vote: two, unless the table may give a symbol more bits than the accumulator has room for twice (pair_high_water:
 // more than 21,824 tokens in one call).  The tables' part wants the warps more than the chains (a 256-token chunk
 // 129 us with two), so it keeps one; and so does a last group of channels that would leave the second without work.
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) w[s][k] = 4 * k < n ? written_symbols(sp[s] + k * C) : 0u;
         }
-        const int high_water = G == 1 ? kSinkHighWater : p.high_water;
+        const int high_water = G == 1 ? kDeepHighWater : p.high_water;
         constexpr int kAhead = 4 * kWordsAhead;
         int i = 0;
         for (;; i += kAhead) {
@@ -592,7 +595,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
                     for (int g = 0; g < G; ++g)
 #pragma unroll
                         for (int s = 0; s < NS; ++s) a[g][s] = entry_of(col[s], w[s][k], j + g);
-                    EncoderState::steps_at<kWarpRow, G>(Smem{}, a, enc, out, high_water, 0xFFFFFFFFu, carried);
+                    EncoderState::steps_at<kWarpRow, G, NS, false, true>(Smem{}, a, enc, out, high_water, 0xFFFFFFFFu, carried);
                 }
             }
 #pragma unroll
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
                     for (int k = 0; k + 1 < kWordsAhead; ++k) w[s][k] = w[s][k + 1];
                 }
             }
-            EncoderState::steps_at<kWarpRow, 1>(Smem{}, a, enc, out, kSinkHighWater, 0xFFFFFFFFu, carried);
+            EncoderState::steps_at<kWarpRow, 1, NS, false, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried);
         }
         int bits = bad ? CG_S_BAD_SYMBOL : 0;
 #pragma unroll
@@ -941,7 +944,7 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
         p.lp = k.max_bins + 1;
         p.nrows = z.nrows;
         p.nsub = z.nsub;
-        p.high_water = pair_high_water(k.ntokens);
+        p.high_water = pair_high_water(k.ntokens) ? deep_pair_high_water(k.ntokens) : 0;
         p.scratch = ws + z.scratch;
         p.stride = z.stride;
         p.lengths = reinterpret_cast<int32_t *>(ws + z.lengths);
