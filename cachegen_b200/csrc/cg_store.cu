@@ -231,14 +231,14 @@ __device__ __forceinline__ int store_counts(const uint32_t *hist, int lp, int cq
     return nz;
 }
 
-// One warp's tables, staged as 16-bit entries channel after channel, to their place: one contiguous run.
-__device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst, int n, int lane) {
+// Tables staged as 16-bit entries channel after channel to their place, one contiguous run, by `threads` threads.
+__device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst, int n, int thread, int threads) {
     if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (n & 7) == 0) {
         const uint4 *s = reinterpret_cast<const uint4 *>(stage);
         uint4 *d = reinterpret_cast<uint4 *>(dst);
-        for (int i = lane; i < n / 8; i += 32) d[i] = s[i];
+        for (int i = thread; i < n / 8; i += threads) d[i] = s[i];
     } else {
-        for (int i = lane; i < n; i += 32) dst[i] = stage[i];
+        for (int i = thread; i < n; i += threads) dst[i] = stage[i];
     }
 }
 
@@ -254,12 +254,13 @@ __device__ __forceinline__ void count_symbol(uint32_t addr) {
 }
 
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
-// block (slab, row), thread (channel, part) counts every kParts-th word of its channel, eight words a batch without a
-// condition inside.  1,999 tokens of 32 layers x 1,024 channels take 38 us under counters (3.9 instructions for 32 symbols); 57
-// and 9.4 with a test for the last word at each, and 512 threads a block, of which 384 wait while the 128 columns become
-// tables.  128, 512 and 1,024 threads: 56, 44 and 63 us; 12 and 16 words in flight: 40 and 39.  The updates alone, one a
+// block (slab, row); a lane counts four adjacent channels, a warp every kTableWarps-th word of them, four words a batch without a
+// condition inside.  Channel 4 l + j of the slab has column 32 j + l, so that the lanes of a warp are in 32 banks whichever of
+// their channels they count.  Bound by the latency of its loads: 1,999 tokens of 32 layers x 1,024 channels take 32 us under
+// counters (3.0 instructions for 32 symbols), 38 and 3.8 with a channel a lane and eight 4-byte loads in flight; 700 tokens of 80
+// layers x 1,024 channels 30 and 39.  Two and eight loads in flight: 32 and 33 us; 128 and 512 threads: 35 and 33.  The updates alone, one a
 // symbol at 1.1 cycles a warp and SM, would take 16.
-constexpr int kTableThreads = 256, kParts = kTableThreads / kGroup;
+constexpr int kTableThreads = 256, kTableWarps = kTableThreads / 32;
 struct TableJobs {
     TableOut out[CG_MAX_ENCODE_LEVELS];
     const uint32_t *sym4[CG_MAX_ENCODE_LEVELS];
@@ -268,78 +269,88 @@ struct TableJobs {
 };
 __global__ void __launch_bounds__(kTableThreads) packed_tables_kernel(const __grid_constant__ TableJobs jobs, int ntokens, int nchannels) {
     const TableOut &out = jobs.out[blockIdx.z];
-    const uint32_t *const sym4 = jobs.sym4[blockIdx.z];
     int32_t *const status = jobs.status[blockIdx.z];
     const int lp = jobs.lp[blockIdx.z];
     extern __shared__ uint4 smem4[];
     uint32_t *hist = reinterpret_cast<uint32_t *>(smem4);
     uint16_t *stage = reinterpret_cast<uint16_t *>(hist + lp * kGroup);
     __shared__ uint32_t nz_total;
-    const int tid = threadIdx.x, cl = tid % kGroup, part = tid / kGroup;
-    const int row = blockIdx.y, c = blockIdx.x * kGroup + cl;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = blockIdx.y, slab = blockIdx.x * kGroup, nch = min(kGroup, nchannels - slab);  // a multiple of 8
     for (int i = tid; i < lp * kGroup; i += kTableThreads) hist[i] = 0u;
     if (tid == 0) nz_total = 0u;
     __syncthreads();
     const int words = (ntokens + 3) / 4, whole = ntokens / 4;
-    if (c < nchannels) {
-        const uint32_t col = smem_addr(hist + (cl >> 5) * 32 * lp + (cl & 31));
-        const uint32_t *p = sym4 + static_cast<int64_t>(row) * words * nchannels + c;
-        constexpr int kAhead = 8;  // loads in flight
-        const int64_t step = static_cast<int64_t>(kParts) * nchannels;
-        int i = part;
-        p += static_cast<int64_t>(part) * nchannels;
-        for (; i + kParts * (kAhead - 1) < whole; i += kParts * kAhead) {
-            uint32_t w[kAhead], any = 0u;
+    if (4 * lane < nch) {
+        uint32_t col[4];
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) {
-                w[j] = __ldg(p);
+        for (int j = 0; j < 4; ++j) col[j] = smem_addr(hist + j * 32 * lp + lane);
+        const int64_t step = static_cast<int64_t>(kTableWarps) * nchannels;
+        const uint32_t *p = jobs.sym4[blockIdx.z] + (static_cast<int64_t>(row) * words + warp) * nchannels + slab + 4 * lane;
+        const auto count = [&](uint4 w) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                count_symbol(entry_of(col[0], w.x, k));
+                count_symbol(entry_of(col[1], w.y, k));
+                count_symbol(entry_of(col[2], w.z, k));
+                count_symbol(entry_of(col[3], w.w, k));
+            }
+        };
+        const auto cleaned = [](uint32_t w) { return w & 0x80808080u ? 0u : w; };  // reported by the coder
+        constexpr int kAhead = 4;  // loads in flight
+        int i = warp;
+        for (; i + kTableWarps * (kAhead - 1) < whole; i += kTableWarps * kAhead) {
+            uint4 w[kAhead];
+            uint32_t any = 0u;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                w[k] = __ldg(reinterpret_cast<const uint4 *>(p));
                 p += step;
             }
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) any |= w[j];
-            if (any & 0x80808080u) {  // reported by the coder
+            for (int k = 0; k < kAhead; ++k) any |= w[k].x | w[k].y | w[k].z | w[k].w;
+            if (any & 0x80808080u) {
 #pragma unroll
-                for (int j = 0; j < kAhead; ++j)
-                    if (w[j] & 0x80808080u) w[j] = 0u;
+                for (int k = 0; k < kAhead; ++k) w[k] = make_uint4(cleaned(w[k].x), cleaned(w[k].y), cleaned(w[k].z), cleaned(w[k].w));
             }
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) count_symbol(entry_of(col, w[j], k));
-            }
+            for (int k = 0; k < kAhead; ++k) count(w[k]);
         }
-        for (; i < words; i += kParts) {
-            uint32_t w = __ldg(p);
+        for (; i < words; i += kTableWarps) {
+            uint4 w = __ldg(reinterpret_cast<const uint4 *>(p));
             p += step;
-            if (w & 0x80808080u) w = 0u;
-            const int n = i < whole ? 4 : ntokens & 3;
-            for (int k = 0; k < n; ++k) count_symbol(col + ((w >> (8 * k)) & 0xFFu) * kWarpRow);
+            w = make_uint4(cleaned(w.x), cleaned(w.y), cleaned(w.z), cleaned(w.w));
+            if (i < whole) {
+                count(w);
+                continue;
+            }
+            for (int k = 0; k < (ntokens & 3); ++k) {
+                count_symbol(col[0] + ((w.x >> (8 * k)) & 0xFFu) * kWarpRow);
+                count_symbol(col[1] + ((w.y >> (8 * k)) & 0xFFu) * kWarpRow);
+                count_symbol(col[2] + ((w.z >> (8 * k)) & 0xFFu) * kWarpRow);
+                count_symbol(col[3] + ((w.w >> (8 * k)) & 0xFFu) * kWarpRow);
+            }
         }
     }
     __syncthreads();
     bool overflow = false;
     if (tid < kGroup) {
+        const int cl = 4 * lane + warp;  // the channel of column tid
         int nz = 0;
-        if (c < nchannels) {
+        if (cl < nch) {
             const int cq = static_cast<int>(half_range(__ldg(out.bins + row)));
-            uint32_t *column = hist + (cl >> 5) * 32 * lp + (cl & 31);
-            if (out.counts) nz = store_counts<32>(column, lp, cq, out.counts + __ldg(out.table_row_off + row) + c, nchannels, &overflow);
+            uint32_t *column = hist + warp * 32 * lp + lane;
+            if (out.counts) nz = store_counts<32>(column, lp, cq, out.counts + __ldg(out.table_row_off + row) + slab + cl, nchannels, &overflow);
             counts_to_column<32>(column, stage + cl * lp, lp, ntokens, cq);
         }
         if (out.group_nz) {
             nz = __reduce_add_sync(0xFFFFFFFFu, nz);
-            if ((tid & 31) == 0 && nz) atomicAdd(&nz_total, static_cast<uint32_t>(nz));
+            if (lane == 0 && nz) atomicAdd(&nz_total, static_cast<uint32_t>(nz));
         }
-        __syncwarp();
-        const int first = blockIdx.x * kGroup + (tid & ~31);
-        const int nch = min(32, nchannels - first);
-        if (nch > 0)
-            copy_tables(stage + (tid & ~31) * lp,
-                        reinterpret_cast<uint16_t *>(out.cdf) + (static_cast<int64_t>(row) * nchannels + first) * lp,
-                        nch * lp, tid & 31);
     }
     if (overflow && status) atomicOr(status, CG_S_COUNT_OVERFLOW);
     __syncthreads();
+    copy_tables(stage, reinterpret_cast<uint16_t *>(out.cdf) + (static_cast<int64_t>(row) * nchannels + slab) * lp, nch * lp, tid, kTableThreads);
     if (tid == 0 && out.group_nz) out.group_nz[row * gridDim.x + blockIdx.x] = nz_total;
 }
 
@@ -541,7 +552,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
         if (overflow) atomicOr(p.status, CG_S_COUNT_OVERFLOW);
         __syncwarp();
         const int first = blockIdx.x * kGroup + warp * 32, nch = min(32, p.nchannels - first);
-        copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp, nch * p.lp, lane);
+        copy_tables(stage + warp * 32 * p.lp, reinterpret_cast<uint16_t *>(p.out.cdf) + (row * C + first) * p.lp, nch * p.lp, lane, 32);
     } else if (any_active) {
         wait_for_launch_before();
 #pragma unroll
