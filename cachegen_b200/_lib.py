@@ -149,6 +149,26 @@ def lib():
     return L
 
 
+_calls = None
+
+
+def calls():
+    """The calls' host side in native code (csrc/cg_calls.cpp), which works through the library that lib() has loaded."""
+    global _calls
+    if _calls is None:
+        L = lib()
+        import torch  # noqa: F401  (its libraries have to be there first)
+        try:
+            from . import _calls as module
+        except ImportError as e:
+            raise CacheGenLibraryMissing(f"{os.path.join(_HERE, '_calls.so')} is missing or was built for another torch: build it with "
+                                         f"`python -m cachegen_b200.build --force` ({e})") from e
+        module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value
+                     for n in ("cg_decode_kv", "cg_encode_kv", "cg_encode_kv_workspace", "cg_encode_kv_wait", "cg_encode_kv_gather")})
+        _calls = module
+    return _calls
+
+
 def workspace_sizes(nrows, ntokens, nchannels) -> WorkspaceSizes:
     """cg_workspace_bytes: sizes of the caller-allocated buffers of the fused calls for one chunk."""
     out = WorkspaceSizes()

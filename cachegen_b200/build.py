@@ -1,4 +1,5 @@
-"""Builds libcachegen_b200.so in-tree with nvcc for sm_100a (no torch headers: a few seconds per file).
+"""Builds libcachegen_b200.so in-tree with nvcc for sm_100a (no torch headers: a few seconds per file), and _calls.so, the
+host side of the calls on torch's tensors, with the host compiler.
 
     python -m cachegen_b200.build [--force] [--verbose]
 """
@@ -12,6 +13,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libcachegen_b200.so")
 SOURCES = ["cg_api.cu", "cg_quant.cu", "cg_tables.cu", "cg_encode.cu", "cg_store.cu", "cg_decode.cu", "cg_host.cu"]
 HEADERS = [os.path.join(CSRC, "cg_common.cuh"), os.path.join(CSRC, "cg_coder.cuh"), os.path.join(CSRC, "cg_hostcopy.h"), os.path.join(PKG, "..", "include", "cachegen_b200.h")]
+CALLS = os.path.join(PKG, "_calls.so")
+CALLS_SOURCE = os.path.join(CSRC, "cg_calls.cpp")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC,-pthread"]
 
@@ -29,10 +32,31 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def calls_need_build():
+    return not os.path.exists(CALLS) or any(os.path.getmtime(d) > os.path.getmtime(CALLS) for d in (CALLS_SOURCE, HEADERS[-1]))
+
+
+def build_calls():
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    include = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+               os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-o", CALLS, CALLS_SOURCE,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f"-I{d}" for d in include] + [
+           "-L" + os.path.join(base, "lib")] + ["-l" + n for n in ("torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda")]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on cg_calls.cpp:\n{r.stdout}\n{r.stderr}")
+
+
 def build(force=False, verbose=False, extra_flags=(), out=None):
     """Compiles the library and returns its path.  `out` builds a second copy elsewhere (with
     `extra_flags`, e.g. -D switches) without touching the in-tree one; CACHEGEN_B200_LIB selects it."""
     target = out or LIB
+    if not out and (force or calls_need_build()):
+        build_calls()
     if not out and not force and not needs_build():
         return target
     flags = NVCC_FLAGS + list(extra_flags)

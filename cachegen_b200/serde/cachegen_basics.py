@@ -363,6 +363,22 @@ _bytes_at = ctypes.pythonapi.PyBytes_AsString
 _bytes_at.restype, _bytes_at.argtypes = ctypes.c_void_p, [ctypes.py_object]
 
 
+class BytesView:
+    """A byte string where a uint8 tensor over its bytes is expected for its address and size."""
+
+    def __init__(self, bs: bytes):
+        self.bs = bs
+
+    def data_ptr(self) -> int:
+        return _bytes_at(self.bs)
+
+    def numel(self) -> int:
+        return len(self.bs)
+
+    def to(self, device) -> torch.Tensor:
+        return torch.frombuffer(bytearray(self.bs), dtype=torch.uint8).to(device)
+
+
 def dump_blob(eo: "CacheGenGPUEncoderOutput") -> bytes:
     """The pickle of an encoded chunk, byte for byte what pickle.dump writes (cachegen_basics.py:146-151).
     Tensors that own their storage have their legacy streams built here; the others are left to torch."""
@@ -681,9 +697,16 @@ class _Staging:
 
     def whole_to_device(self, view_cpu: torch.Tensor, device) -> torch.Tensor:
         """One host buffer (any memory) to the GPU through the staging memory."""
-        self.open()
-        out = self.to_device(view_cpu, device)
-        self.send()
+        n = view_cpu.numel()
+        out = torch.empty(n, dtype=torch.uint8, device=device)
+        if n:
+            seg = _lib.HostSegment(view_cpu.data_ptr(), out.data_ptr(), n)
+            self.begin((n + 255) // 256 * 256)
+            try:
+                self._send(lambda on: _lib.lib().cg_host_upload(ctypes.byref(seg), 1, self.buf.data_ptr(), self.buf.numel(), on),
+                           out.device, None)
+            finally:
+                self.end()
         return out
 
     # -- from the GPU
@@ -728,8 +751,19 @@ class _Staging:
         """The bytes of a contiguous GPU tensor."""
         n = t.numel() * t.element_size()
         out = _bytes_new(None, n)
-        self.fetch([t])
-        self.collect([_bytes_at(out)])
+        seg = _lib.HostSegment(_bytes_at(out), t.data_ptr(), n)
+        self.begin((n + 255) // 256 * 256)
+        try:
+            with on_device(t.device):
+                on = torch.cuda.current_stream(t.device)
+                try:
+                    rc = _lib.lib().cg_host_download(ctypes.byref(seg), 1, self.buf.data_ptr(), self.buf.numel(), 0, on.cuda_stream)
+                    _lib.check(rc, "cg_host_download")
+                except BaseException:
+                    on.synchronize()  # transfers may still write to the buffer
+                    raise
+        finally:
+            self.end()
         return out
 
 

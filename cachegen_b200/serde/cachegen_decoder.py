@@ -236,6 +236,29 @@ def _device_of(eo):
     return eo.blob.device if isinstance(eo, flat_format.FlatChunk) else eo.cdf.device
 
 
+def _status_word(ws: dict, dev) -> torch.Tensor:
+    status = ws.get("status")
+    if status is None or status.device != dev:
+        with torch.inference_mode(False):  # kept, and written to by later calls in whatever mode those run
+            status = torch.zeros(1, dtype=torch.int32, device=dev)
+        ws["status"] = status
+    return status
+
+
+_ROW_OFFSETS = {_lib.CG_TABLES_COUNTS: ("table_row_off", flat_format.table_row_offsets),
+                _lib.CG_TABLES_SPARSE: ("mask_row_off", flat_format.mask_row_offsets)}
+
+
+def _row_offsets(ws: dict, kind: int, host_bins: _HostBins, nchannels: int, dev) -> torch.Tensor:
+    """Where the rows' byte counts, or masks, start in tables of this kind: a tensor that the workspace keeps."""
+    name, fn = _ROW_OFFSETS[kind]
+    t, key = ws.get(name), (nchannels, host_bins.values)
+    if t is None or t.device != dev or ws.get(name + "_of") != key:
+        t = torch.tensor(fn(host_bins.cpu, nchannels), dtype=torch.int64, device=dev)
+        ws[name], ws[name + "_of"] = t, key
+    return t
+
+
 class DecodePlan:
     """Everything cg_decode_kv needs for a list of encoded chunks, built once:
     device-resident inputs, the job descriptors, the output blob and the launch arguments.  Chunks are
@@ -287,20 +310,8 @@ class DecodePlan:
         if goff is None or goff.numel() < njobs_total * ngroups or goff.device != dev:
             goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)
             ws["group_off"] = goff
-        status = ws.get("status")
-        if status is None or status.device != dev:
-            with torch.inference_mode(False):  # kept, and written to by later calls in whatever mode those run
-                status = torch.zeros(1, dtype=torch.int32, device=dev)
-            ws["status"] = status
-        row_offs = {}
-        for kind, name, fn in ((_lib.CG_TABLES_COUNTS, "table_row_off", flat_format.table_row_offsets),
-                               (_lib.CG_TABLES_SPARSE, "mask_row_off", flat_format.mask_row_offsets)):
-            if any(v.table_kind == kind for v in views):
-                t, key = ws.get(name), (C, host_bins.values)
-                if t is None or t.device != dev or ws.get(name + "_of") != key:
-                    t = torch.tensor(fn(host_bins.cpu, C), dtype=torch.int64, device=dev)
-                    ws[name], ws[name + "_of"] = t, key
-                row_offs[kind] = t
+        status = _status_word(ws, dev)
+        row_offs = {kind: _row_offsets(ws, kind, host_bins, C, dev) for kind in _ROW_OFFSETS if any(v.table_kind == kind for v in views)}
 
         esz = out.element_size()
         self.keep = list(row_offs.values())  # tensors that must outlive the launches
@@ -409,8 +420,32 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
     strides).  `workspace` caches the small offset / status buffers between calls.  `host_bins`: the values of `bins`,
     when the caller knows them; read from the tensor otherwise, if the chunks ask for them.
     """
+    if delta is None and workspace is not None:
+        decoded = _decode_usual(encoder_outputs, bins, fmt, out_dtype, out, workspace, host_bins)
+        if decoded is not None:
+            return decoded
     return DecodePlan(encoder_outputs, bins, fmt, out_dtype, out=out, workspace=workspace, delta=delta,
                       host_bins=host_bins).run()
+
+
+def _decode_usual(encoder_outputs, bins, fmt, out_dtype, out, workspace, host_bins):
+    """What DecodePlan(...).run() does for chunks, all of one kind, of plain contiguous tensors on the current GPU, in native code.
+    None, and nothing has been done but for buffers that the workspace keeps, for any other chunks."""
+    if not encoder_outputs or type(encoder_outputs) is not list or fmt not in ("vllm", "huggingface") or out_dtype not in _DTYPES or not bins.is_cuda:
+        return None
+    kind, piece, flat = CacheGenGPUEncoderOutput, CacheGenGPUBytestream, None
+    if type(encoder_outputs[0]) is flat_format.FlatChunk:
+        header = encoder_outputs[0].header
+        if host_bins is None or header.table_kind == _lib.CG_TABLES_SPARSE and not host_bins.sparse:
+            return None
+        kind, piece, C = flat_format.FlatChunk, None, header.H * header.D
+        flat = (header.table_kind, host_bins.checksum(None), host_bins.counts_bytes(C), host_bins.sparse_bytes(C),
+                _row_offsets(workspace, header.table_kind, host_bins, C, bins.device) if header.table_kind in _ROW_OFFSETS else None)
+    decoded = _lib.calls().decode(encoder_outputs, kind, piece, bins, fmt == "vllm", out_dtype == torch.bfloat16, out, workspace,
+                                  _status_word(workspace, bins.device), flat)
+    if type(decoded) is int:
+        _lib.check(decoded, "cg_decode_kv")
+    return decoded
 
 
 _copy_streams = {}

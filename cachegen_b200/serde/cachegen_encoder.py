@@ -17,6 +17,7 @@ cg_encode_kv_flat).  quantize_and_tables and encode_streams are the same steps o
 import collections
 import ctypes
 import dataclasses
+import operator
 import threading
 from typing import Tuple
 
@@ -331,47 +332,48 @@ class _PendingChunk:
         step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
         self.nsub = (T + step - 1) // step
         self.lib = _lib.lib()
-        self.stream = torch.cuda.current_stream(dev) if stream is None else stream
-        self.stream_ptr = ctypes.c_void_p(self.stream.cuda_stream)
+        self.on = None if stream is None else stream.cuda_stream  # the stream's address; None: the current one
         self.bins = info.on(dev)
-        self.scales = torch.empty((2, L, T, 1), dtype=kv.dtype, device=dev) if with_counts else None
-        self.scales_k = self.scales[0] if with_counts else torch.empty((L, T, 1), dtype=kv.dtype, device=dev)
-        self.scales_v = self.scales[1] if with_counts else torch.empty((L, T, 1), dtype=kv.dtype, device=dev)
-        self.cdf = torch.empty((2 * L, H * D, max_bins + 1), dtype=torch.int16, device=dev)
-        need = self.lib.cg_encode_kv_workspace(L, T, H, D)
-        if need < 0:
-            _lib.check(need, "cg_encode_kv_workspace")
-        if workspace is None or workspace.numel() < need:
-            workspace = torch.empty(need, dtype=torch.uint8, device=dev)
-        self.workspace = workspace
         self.tail = _take_tail(self.nsub + 4)
         job = self.job = _lib.EncodeKvJob()
-        job.kv, job.bins, job.cdf = kv.data_ptr(), self.bins.data_ptr(), self.cdf.data_ptr()
-        job.scales_k, job.scales_v = self.scales_k.data_ptr(), self.scales_v.data_ptr()
-        job.workspace, job.workspace_bytes, job.tail = workspace.data_ptr(), workspace.numel(), self.tail.data_ptr()
-        job.s_layer, job.s_kv, job.s_token, job.s_head, _ = kv.stride()
-        job.dtype, job.nlayers, job.ntokens, job.nheads, job.head_size = _DTYPES[kv.dtype], L, T, H, D
-        job.max_bins = max_bins
-        self.counts = self.res_bins = None
-        if with_counts:
-            row_off, size, self.mask_off, self.mask_bytes = info.offsets(dev, H * D)
-            self.counts = torch.empty(size, dtype=torch.uint8, device=dev)
-            job.counts, job.table_row_off = self.counts.data_ptr(), row_off.data_ptr()
-        if delta is not None:
-            self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
-            job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
+        self.res_bins = None
         try:
-            if enqueue:
-                with on_device(dev):
-                    _lib.check(self.lib.cg_encode_kv(ctypes.byref(job), self.stream_ptr), "cg_encode_kv")
-            # made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do
-            self.lengths = [] if with_counts else [torch.empty((2 * L, H * D), dtype=torch.int32, device=dev)
-                                                   for _ in range(self.nsub)]
-            self.pointers = ctypes.c_void_p * self.nsub
-            self.length_pointers = self.pointers(*[t.data_ptr() for t in self.lengths])
+            if delta is not None:
+                self.res_bins = delta.residual_bins(info.cpu[:L], info.cpu[L:], dev)
+                job.delta_group, job.res_bins = delta.group, self.res_bins.data_ptr()
+            row_off = size = None
+            if with_counts:
+                row_off, size, self.mask_off, self.mask_bytes = info.offsets(dev, H * D)
+            self.start(workspace, row_off, size, enqueue)
+            self.lengths = []
+            if enqueue and not with_counts:
+                self.make_lengths()
         except BaseException:
             self.abandon()
             raise
+
+    def start(self, workspace, row_off, counts_bytes, enqueue):
+        """Makes the buffers (`workspace`, if it is large enough, is taken), fills the job in and launches its kernels."""
+        rc, self.on, self.scales, self.scales_k, self.scales_v, self.cdf, self.workspace, self.counts = _lib.calls().encode_start(
+            ctypes.addressof(self.job), self.kv, self.bins, self.max_bins, self.tail.data_ptr(), workspace, row_off, counts_bytes,
+            self.on, enqueue)
+        _lib.check(rc, "cg_encode_kv_workspace" if self.cdf is None else "cg_encode_kv")
+
+    def make_lengths(self):
+        """Made while the GPU works: what is done after its sizes have arrived is time in which it has nothing to do."""
+        self.lengths = [torch.empty((2 * self.L, self.H * self.D), dtype=torch.int32, device=self.dev) for _ in range(self.nsub)]
+
+    @property
+    def stream_ptr(self):
+        return ctypes.c_void_p(self.on)
+
+    @property
+    def pointers(self):
+        return ctypes.c_void_p * self.nsub
+
+    @property
+    def length_pointers(self):
+        return self.pointers(*[t.data_ptr() for t in self.lengths])
 
     def another(self, info, max_bins):
         """The same KV at other bins, prepared like this chunk (one without delta coding or counts) and not enqueued."""
@@ -379,43 +381,32 @@ class _PendingChunk:
             raise RuntimeError(f"bins describe {info.cpu.numel() // 2} layers, the KV blob has {self.L}")
         p = object.__new__(_PendingChunk)
         p.__dict__.update(self.__dict__)
-        p.tail, dev, dtype, shape = None, self.dev, self.kv.dtype, (self.L, self.T, 1)
-        p.info, p.max_bins, p.bins = info, max_bins, info.on(dev)
-        p.scales_k, p.scales_v = torch.empty(shape, dtype=dtype, device=dev), torch.empty(shape, dtype=dtype, device=dev)
-        p.cdf = torch.empty((2 * self.L, self.H * self.D, max_bins + 1), dtype=torch.int16, device=dev)
-        p.workspace = torch.empty(self.workspace.numel(), dtype=torch.uint8, device=dev)
-        p.lengths = [torch.empty((2 * self.L, self.H * self.D), dtype=torch.int32, device=dev) for _ in range(self.nsub)]
+        p.info, p.max_bins, p.bins = info, max_bins, info.on(self.dev)
         p.tail = _take_tail(self.nsub + 4)
-        job = p.job = _lib.EncodeKvJob.from_buffer_copy(self.job)
-        job.bins, job.cdf, job.max_bins = p.bins.data_ptr(), p.cdf.data_ptr(), max_bins
-        job.scales_k, job.scales_v = p.scales_k.data_ptr(), p.scales_v.data_ptr()
-        job.workspace, job.tail = p.workspace.data_ptr(), p.tail.data_ptr()
+        p.job = _lib.EncodeKvJob()
+        p.start(None, None, None, False)
         return p
 
-    def sizes(self):
-        """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts)."""
-        with on_device(self.dev):
-            _lib.check(self.lib.cg_encode_kv_wait(ctypes.byref(self.job), self.stream_ptr), "cg_encode_kv_wait")
-        host = self.tail[:self.nsub + 3].tolist()
-        _give_tail(self.tail)
-        self.tail = None
+    def sizes(self, lengths=None):
+        """Waits for (payload offsets [nsub + 1], status bits, number of non-zero byte counts, pieces): with `lengths`, the tensors
+        for them, the streams are gathered into pieces of their own as soon as their sizes are known."""
+        rc, host, pieces = _lib.calls().encode_finish(ctypes.addressof(self.job), self.dev.index, self.on, lengths)
+        if host is not None:
+            _give_tail(self.tail)
+            self.tail = None
+        _lib.check(rc, "cg_encode_kv_wait" if host is None else "cg_encode_kv_gather")
         bits = host[self.nsub + 1]
         if bits & ~_lib.CG_S_COUNT_OVERFLOW:
             raise RuntimeError("cachegen encode: " + _lib.status_text(bits & ~_lib.CG_S_COUNT_OVERFLOW))
-        return host[:self.nsub + 1], bits, host[self.nsub + 2]
+        return host[:self.nsub + 1], bits, host[self.nsub + 2], pieces
 
     def pieces(self):
         """Waits for the sizes; a tensor for every sub-chunk's streams (a view would pickle the whole buffer)."""
-        offs, _, _ = self.sizes()
+        offs = self.sizes()[0]
         return [torch.empty(offs[j + 1] - offs[j], dtype=torch.uint8, device=self.dev) for j in range(self.nsub)]
 
     def finish(self) -> CacheGenGPUEncoderOutput:
-        pieces = self.pieces()
-        with on_device(self.dev):
-            rc = self.lib.cg_encode_kv_gather(ctypes.byref(self.job), self.pointers(*[t.data_ptr() for t in pieces]),
-                                              self.length_pointers, self.stream_ptr)
-        _lib.check(rc, "cg_encode_kv_gather")
-        return self.output(pieces)
+        return self.output(self.sizes(self.lengths)[3])
 
     def output(self, pieces) -> CacheGenGPUEncoderOutput:
         step = CGBasics.CACHEGEN_GPU_MAX_TOKENS_PER_CHUNK
@@ -427,7 +418,8 @@ class _PendingChunk:
         """Gives the buffers up after an error: the GPU may still be writing to them, the pinned one among them, which
         would go to whoever asks torch for pinned memory next.  Nothing to do once the sizes have been read."""
         if self.tail is not None:
-            self.stream.synchronize()
+            (torch.cuda.current_stream(self.dev) if self.on is None else
+             torch.cuda.ExternalStream(self.on, device=self.dev)).synchronize()
             _give_tail(self.tail)
             self.tail = None
 
@@ -525,6 +517,8 @@ def _encode_infos(kv, infos) -> list:
             jobs = (_lib.EncodeKvJob * len(groups[-1]))(*[p.job for p in groups[-1]])
             with on_device(first.dev):
                 _lib.check(first.lib.cg_encode_kv_levels(jobs, len(jobs), first.stream_ptr), "cg_encode_kv_levels")
+            for p in groups[-1]:
+                p.make_lengths()
         result = []
         for group in groups:
             first = group[0]
@@ -569,11 +563,14 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     kmax = info.table_bins(max_bins)
     p = _PendingChunk(kv, info, kmax, delta=delta, with_counts=True)
     try:
-        offs, bits, nonzero = p.sizes()
+        # while the GPU works
+        f, checksum = _lib.FlatLayout(), info.checksum(delta)
+        off_masks, off_counts = flat_format.sparse_parts(2 * p.L, p.H * p.D, p.mask_bytes)
+        f.mask_row_off, f.off_masks, f.off_counts = p.mask_off.data_ptr(), off_masks, off_counts
+        offs, bits, nonzero, _ = p.sizes()
     finally:
         p.abandon()
     fits = bool(compact_tables) and not (bits & _lib.CG_S_COUNT_OVERFLOW)
-    off_masks, off_counts = flat_format.sparse_parts(2 * p.L, p.H * p.D, p.mask_bytes)
     if fits and compact_tables is True and info.sparse:
         kind, size = flat_format.TABLES_SPARSE, off_counts + nonzero
     elif fits:
@@ -581,20 +578,21 @@ def encode_flat(kv: torch.Tensor, key_bins: torch.Tensor, value_bins: torch.Tens
     else:
         kind, size = flat_format.TABLES_CDF, 2 * p.cdf.numel()
     header = flat_format.layout(p.L, p.H, p.D, p.T, kmax + 1, p.kv.dtype, kind, size, flat_format.LENGTHS_U16, offs,
-                                bins_checksum=info.checksum(delta))
+                                bins_checksum=checksum)
     head = header.pack()
     blob = torch.empty(header.total, dtype=torch.uint8, device=p.dev)
-    f = _lib.FlatLayout()
     sub_off = (ctypes.c_int64 * p.nsub)(*offs[:p.nsub])
-    f.blob, f.mask_row_off = blob.data_ptr(), p.mask_off.data_ptr()
-    f.header_host, f.header_bytes = ctypes.cast(ctypes.c_char_p(head), ctypes.c_void_p), len(head)
-    f.sub_off_host = ctypes.cast(sub_off, ctypes.c_void_p)
+    f.blob, f.table_kind = blob.data_ptr(), kind
+    f.header_host, f.header_bytes = ctypes.cast(head, ctypes.c_void_p), len(head)
+    f.sub_off_host = ctypes.addressof(sub_off)
     f.off_scales, f.off_tables, f.tables_bytes = header.off_scales, header.off_tables, size
     f.off_lengths, f.off_payload = header.off_lengths, header.off_payload
-    f.off_masks, f.off_counts, f.table_kind = off_masks, off_counts, kind
     with on_device(p.dev):
         _lib.check(p.lib.cg_encode_kv_flat(ctypes.byref(p.job), ctypes.byref(f), p.stream_ptr), "cg_encode_kv_flat")
     return flat_format.FlatChunk(blob, header)
+
+
+_settings_of = operator.attrgetter(*[f.name for f in dataclasses.fields(CacheGenConfig)])
 
 
 class CacheGenSerializer(Serializer):
@@ -692,7 +690,7 @@ class CacheGenSerializer(Serializer):
 
     def _level_info(self, config: CacheGenConfig) -> _BinsInfo:
         """The bins of a quality level, made once per setting."""
-        key = dataclasses.astuple(config)
+        key = _settings_of(config) if type(config) is CacheGenConfig else dataclasses.astuple(config)
         info = self._levels.get(key)
         if info is None:
             info = self._levels[key] = self._config_info(config)

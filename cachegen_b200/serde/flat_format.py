@@ -268,9 +268,13 @@ class FlatChunk:
 def wrap(buf, to_device) -> FlatChunk:
     """A bytes-like CGB2 container on a GPU: to_device makes the GPU tensor of a view of its bytes."""
     header = FlatHeader.parse(buf)
-    with warnings.catch_warnings():
-        warnings.simplefilter("ignore")  # a read-only buffer, and it is only read
-        view = torch.frombuffer(buf, dtype=torch.uint8)
+    if type(buf) is bytes:
+        from .cachegen_basics import BytesView
+        view = BytesView(buf)
+    else:
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")  # a read-only buffer, and it is only read
+            view = torch.frombuffer(buf, dtype=torch.uint8)
     return FlatChunk(to_device(view), header)
 
 
