@@ -57,10 +57,7 @@ int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool ea
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
 
-// cg_tables.cu: group offsets of sparse tables, and the tables in one pass once those are known
-int launch_sparse_write(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
-                        const uint32_t *group_off, void *masks, const int64_t *mask_row_off, uint8_t *out,
-                        cudaStream_t st);
+// cg_tables.cu: group offsets of sparse tables
 int launch_sparse_sizes(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
                         uint32_t *group_off, cudaStream_t st);
 
@@ -316,5 +313,11 @@ __device__ __forceinline__ float half_bits_to_float(uint16_t b, int dtype) {
 
 // Cq of do_dequantize / MAX of torch_quant_vectorized: bins // 2 - 1 on a float tensor.
 __device__ __forceinline__ float half_range(float bins) { return __fsub_rn(floorf(__fmul_rn(bins, 0.5f)), 1.0f); }
+
+// Symbols of a row that sparse tables store: all but the centre.
+__device__ __forceinline__ int stored_symbols(const float *bins, int row) {
+    const int n = 2 * static_cast<int>(half_range(__ldg(bins + row)));
+    return n < 32 ? n : 32;  // wider rows cannot be written in this form: the caller rules them out
+}
 
 }  // namespace cg

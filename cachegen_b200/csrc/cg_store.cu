@@ -720,7 +720,7 @@ __global__ void publish_tail_kernel(const int64_t *sub_off, const int32_t *statu
 constexpr int kGatherSubs = 64;
 struct GatherTargets {
     uint8_t *bytes[kGatherSubs];
-    void *lengths[kGatherSubs];  // int32 or uint16 [nrows, C]
+    int32_t *lengths[kGatherSubs];  // [nrows, C]
 };
 struct GatherJobs {
     const uint8_t *scratch[CG_MAX_ENCODE_LEVELS];
@@ -732,7 +732,7 @@ struct GatherJobs {
 // The gather of one sub-chunk's group (gather_run) into final buffers, its lengths beside it.  15 us under
 // counters a 256-token Llama-7B chunk (11.8 MB out of scratch that is read in full lines).  Ten blocks an SM are what the
 // shared memory allows (see gather_run).
-template <class Len, bool INTERLEAVED>
+template <bool INTERLEAVED>
 __global__ void __launch_bounds__(kGroup, 10) gather_kernel(const __grid_constant__ GatherJobs jobs, int64_t stride, int nchannels, int first,
                                                         const __grid_constant__ GatherTargets out) {
     const int job = (first + blockIdx.z) / jobs.nsub;  // sub-chunk after sub-chunk, job after job
@@ -745,32 +745,105 @@ __global__ void __launch_bounds__(kGroup, 10) gather_kernel(const __grid_constan
     const int64_t group = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
     const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * nchannels + c;
     const int len = c < nchannels ? __ldg(lengths + slot) : 0;
-    if (c < nchannels) static_cast<Len *>(out.lengths[blockIdx.z])[static_cast<int64_t>(row) * nchannels + c] = static_cast<Len>(len);
+    if (c < nchannels) out.lengths[blockIdx.z][static_cast<int64_t>(row) * nchannels + c] = len;
     const uint32_t *src = INTERLEAVED ? scratch_word(const_cast<uint8_t *>(scratch), stride, group, tid)
                                       : reinterpret_cast<const uint32_t *>(scratch + slot * stride);
     gather_run<INTERLEAVED ? 32 : 1>(src, min(len, static_cast<int>(stride)), out.bytes[blockIdx.z] + __ldg(group_off + group));
 }
 
-// Header, scales and the sparse tables' group offsets of a container (flat_format.py) to their places.
+// ---- a container (flat_format.py) in one launch ---------------------------------------------------------------
 constexpr int kMaxHeader = 128 + 8 * (65536 / kSubTokens + 1);
-struct FlatHeader {
-    uint8_t bytes[kMaxHeader];
+struct ContainerParams {
+    uint8_t header[kMaxHeader];
+    int64_t sub_off[kMaxHeader / 8];  // of the sub-chunks' streams in the payload
+    int header_bytes, nsub, nchannels, kind;
+    uint8_t *blob;
+    int64_t off_scales, off_tables, tables_bytes, off_lengths, off_payload, off_masks, off_counts;
+    const uint16_t *scales_k, *scales_v;
+    int64_t nscales;               // of each
+    const uint8_t *tables;         // byte counts, or int16 tables as they are (CG_TABLES_CDF)
+    const int64_t *count_row_off, *mask_row_off;
+    const float *bins;
+    const uint32_t *group_nz;
+    const uint8_t *scratch;
+    const int32_t *lengths;
+    const int64_t *group_off;
+    int64_t stride;
 };
-__global__ void __launch_bounds__(256) flat_front_kernel(const __grid_constant__ FlatHeader h, int header_bytes,
-                                                         uint8_t *blob, const uint16_t *scales_k,
-                                                         const uint16_t *scales_v, int64_t n, int64_t off_scales,
-                                                         const uint32_t *group_off, int ngroups, int64_t off_tables) {
-    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = i0; i < header_bytes; i += step) blob[i] = h.bytes[i];
-    uint16_t *s = reinterpret_cast<uint16_t *>(blob + off_scales);
-    for (int64_t i = i0; i < n; i += step) {
-        s[i] = scales_k[i];
-        s[n + i] = scales_v[i];
+
+// 16-bit stream lengths and streams of one sub-chunk's group, as gather_kernel; and in the blocks behind the sub-chunks' the rest:
+// masks and non-zero counts of the group in one pass over its byte counts, or a share of dense tables, a share of the scales and
+// group offsets, and in the first block the header and the zero bytes between the sections (the same KV gives the same bytes).
+// Bound by latency and, where the call is short, by its one launch: 61 tokens of 10 layers x 1,024 channels to a container and back as bytes
+// take 203 us, 218 with a clearing, two kernels and a gather, 15 us of launches, in its place.
+template <bool INTERLEAVED>
+__global__ void __launch_bounds__(kGroup, 10) container_kernel(const __grid_constant__ ContainerParams p) {
+    const int tid = threadIdx.x, row = blockIdx.y, nrows = gridDim.y, nslab = gridDim.x;
+    const int c = blockIdx.x * kGroup + tid, sub = blockIdx.z;
+    if (sub < p.nsub) {
+        const int64_t group = (static_cast<int64_t>(sub) * nrows + row) * nslab + blockIdx.x;
+        const int64_t slot = (static_cast<int64_t>(sub) * nrows + row) * p.nchannels + c;
+        const int len = c < p.nchannels ? __ldg(p.lengths + slot) : 0;
+        if (c < p.nchannels) reinterpret_cast<uint16_t *>(p.blob + p.off_lengths)[slot] = static_cast<uint16_t>(len);
+        const uint32_t *src = INTERLEAVED ? scratch_word(const_cast<uint8_t *>(p.scratch), p.stride, group, tid)
+                                          : reinterpret_cast<const uint32_t *>(p.scratch + slot * p.stride);
+        gather_run<INTERLEAVED ? 32 : 1>(src, min(len, static_cast<int>(p.stride)), p.blob + p.off_payload + p.sub_off[sub] + __ldg(p.group_off + group));
+        return;
     }
-    if (group_off) {
-        uint32_t *t = reinterpret_cast<uint32_t *>(blob + off_tables);
-        for (int64_t i = i0; i <= ngroups; i += step) t[i] = group_off[i];
+    const int block = row * nslab + blockIdx.x, blocks = nrows * nslab;
+    const int64_t i0 = static_cast<int64_t>(block) * kGroup + tid, step = static_cast<int64_t>(blocks) * kGroup;
+    uint8_t *const tables = p.blob + p.off_tables;
+    if (p.kind == CG_TABLES_SPARSE) {
+        __shared__ int warp_sums[kGroup / 32];
+        const int nstored = stored_symbols(p.bins, row);
+        const uint8_t *cnt = p.tables + __ldg(p.count_row_off + row) + c;
+        const int64_t at_mask = __ldg(p.mask_row_off + row);
+        uint32_t m = 0u, n[8] = {};
+        if (c < p.nchannels) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                if (j >= nstored) continue;
+                const uint32_t v = __ldg(cnt + static_cast<int64_t>(j) * p.nchannels);
+                n[j >> 2] |= v << (8 * (j & 3));
+                m |= (v ? 1u : 0u) << j;
+            }
+            uint8_t *mrow = tables + p.off_masks + at_mask;
+            if (nstored <= 16) reinterpret_cast<uint16_t *>(mrow)[c] = static_cast<uint16_t>(m);
+            else reinterpret_cast<uint32_t *>(mrow)[c] = m;
+            if (c == p.nchannels - 1)  // rows of masks start at multiples of four
+                for (int64_t k = at_mask + static_cast<int64_t>(p.nchannels) * (nstored <= 16 ? 2 : 4); k < __ldg(p.mask_row_off + row + 1); ++k)
+                    tables[p.off_masks + k] = 0;
+        }
+        const int excl = block_exclusive_scan_128(__popc(m), warp_sums, tid, nullptr);
+        uint8_t *o = tables + p.off_counts + __ldg(p.group_nz + block) + excl;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if ((m >> j) & 1u) *o++ = static_cast<uint8_t>(n[j >> 2] >> (8 * (j & 3)));
+        uint32_t *offsets = reinterpret_cast<uint32_t *>(tables);
+        for (int64_t i = i0; i <= blocks; i += step) offsets[i] = __ldg(p.group_nz + i);
+    } else {  // off_tables is a multiple of 16
+        const int64_t whole = (reinterpret_cast<uintptr_t>(p.tables) & 15) ? 0 : p.tables_bytes / 16;
+        for (int64_t i = i0; i < whole; i += step) reinterpret_cast<uint4 *>(tables)[i] = __ldg(reinterpret_cast<const uint4 *>(p.tables) + i);
+        for (int64_t i = whole * 16 + i0; i < p.tables_bytes; i += step) tables[i] = __ldg(p.tables + i);
     }
+    uint16_t *scales = reinterpret_cast<uint16_t *>(p.blob + p.off_scales);
+    for (int64_t i = i0; i < p.nscales; i += step) {
+        scales[i] = __ldg(p.scales_k + i);
+        scales[p.nscales + i] = __ldg(p.scales_v + i);
+    }
+    if (block) return;
+    for (int i = tid; i < p.header_bytes; i += kGroup) p.blob[i] = p.header[i];
+    const auto zero = [&](int64_t from, int64_t to) {
+        for (int64_t i = from + tid; i < to; i += kGroup) p.blob[i] = 0;
+    };
+    zero(p.header_bytes, p.off_scales);
+    zero(p.off_scales + 4 * p.nscales, p.off_tables);
+    if (p.kind == CG_TABLES_SPARSE) {
+        zero(p.off_tables + 4 * (static_cast<int64_t>(blocks) + 1), p.off_tables + p.off_masks);
+        zero(p.off_tables + p.off_masks + __ldg(p.mask_row_off + nrows), p.off_tables + p.off_counts);
+    }
+    zero(p.off_tables + p.tables_bytes, p.off_lengths);
+    zero(p.off_lengths + static_cast<int64_t>(p.nsub) * nrows * p.nchannels * 2, p.off_payload);
 }
 
 }  // namespace cg
@@ -1029,8 +1102,7 @@ extern "C" int cg_wait_word(const int64_t *word, void *stream) {
 }
 
 namespace {
-template <class Len>
-int launch_gather(const cg_encode_kv_job *jobs, int njobs, const Sizes &z, uint8_t *const *bytes, void *const *lengths, cudaStream_t st) {
+int launch_gather(const cg_encode_kv_job *jobs, int njobs, const Sizes &z, uint8_t *const *bytes, int32_t *const *lengths, cudaStream_t st) {
     GatherJobs g;
     g.nsub = z.nsub;
     for (int j = 0; j < njobs; ++j) {
@@ -1048,9 +1120,9 @@ int launch_gather(const cg_encode_kv_job *jobs, int njobs, const Sizes &z, uint8
         }
         const dim3 grid(z.nslab, z.nrows, n);
         if (fused_ok(jobs[0]))  // which of the two encoders wrote the scratch
-            gather_kernel<Len, true><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
+            gather_kernel<true><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
         else
-            gather_kernel<Len, false><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
+            gather_kernel<false><<<grid, kGroup, 0, st>>>(g, z.stride, z.nchannels, s0, t);
         if (int rc = check_launch()) return rc;
     }
     return CG_OK;
@@ -1075,8 +1147,7 @@ extern "C" int cg_encode_kv_levels_gather(const cg_encode_kv_job *jobs, int njob
     const Sizes z = sizes_of(jobs->nlayers, jobs->ntokens, jobs->nheads, jobs->head_size);
     for (int k = 0; k < z.nsub * njobs; ++k)
         if (!bytes_host[k] || !lengths_host[k]) return CG_E_NULL;
-    return launch_gather<int32_t>(jobs, njobs, z, bytes_host, reinterpret_cast<void *const *>(lengths_host),
-                                  static_cast<cudaStream_t>(stream));
+    return launch_gather(jobs, njobs, z, bytes_host, lengths_host, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int cg_encode_kv_flat(const cg_encode_kv_job *job, const cg_flat_layout *layout, void *stream) {
@@ -1092,36 +1163,37 @@ extern "C" int cg_encode_kv_flat(const cg_encode_kv_job *job, const cg_flat_layo
     if ((reinterpret_cast<uintptr_t>(f.blob) | f.off_scales | f.off_tables | f.off_lengths) & 15) return CG_E_ALIGN;
     if ((f.table_kind != CG_TABLES_CDF && !b.counts) || f.table_kind < CG_TABLES_CDF || f.table_kind > CG_TABLES_SPARSE) return CG_E_SHAPE;
     if (z.nsub > kMaxHeader / 8) return CG_E_CAPACITY;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool sparse = f.table_kind == CG_TABLES_SPARSE;
-    // the gaps between sections (and inside sparse tables) are zero: the same KV gives the same bytes
-    cudaError_t e = cudaMemsetAsync(f.blob, 0, static_cast<size_t>(sparse ? f.off_payload : f.off_tables), st);
-    if (e == cudaSuccess && !sparse) e = cudaMemsetAsync(f.blob + f.off_tables + f.tables_bytes, 0,
-                                                        static_cast<size_t>(f.off_payload - f.off_tables - f.tables_bytes), st);
-    if (e == cudaSuccess && !sparse)
-        e = cudaMemcpyAsync(f.blob + f.off_tables, f.table_kind == CG_TABLES_CDF ? static_cast<const void *>(b.cdf) : b.counts,
-                            static_cast<size_t>(f.tables_bytes), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return set_cuda_error(e);
     const uint8_t *ws = static_cast<const uint8_t *>(b.workspace);
-    const uint32_t *group_nz = reinterpret_cast<const uint32_t *>(ws + z.group_nz);
-    FlatHeader h;
-    memcpy(h.bytes, f.header_host, static_cast<size_t>(f.header_bytes));
-    flat_front_kernel<<<32, 256, 0, st>>>(h, static_cast<int>(f.header_bytes), f.blob, static_cast<const uint16_t *>(b.scales_k),
-                                          static_cast<const uint16_t *>(b.scales_v),
-                                          static_cast<int64_t>(b.nlayers) * b.ntokens, f.off_scales,
-                                          sparse ? group_nz : nullptr, z.nrows * z.nslab, f.off_tables);
-    if (int rc = check_launch()) return rc;
-    if (sparse)
-        if (int rc = launch_sparse_write(b.counts, b.table_row_off, b.bins, z.nrows, z.nchannels, group_nz,
-                                         f.blob + f.off_tables + f.off_masks, f.mask_row_off,
-                                         f.blob + f.off_tables + f.off_counts, st))
-            return rc;
-    uint8_t *bytes[kMaxHeader / 8];
-    void *lengths[kMaxHeader / 8];
-    const int64_t streams = static_cast<int64_t>(z.nrows) * z.nchannels;
-    for (int k = 0; k < z.nsub; ++k) {
-        bytes[k] = f.blob + f.off_payload + f.sub_off_host[k];
-        lengths[k] = f.blob + f.off_lengths + k * streams * 2;
-    }
-    return launch_gather<uint16_t>(job, 1, z, bytes, lengths, st);
+    ContainerParams p;
+    memcpy(p.header, f.header_host, static_cast<size_t>(f.header_bytes));
+    memcpy(p.sub_off, f.sub_off_host, 8 * static_cast<size_t>(z.nsub));
+    p.header_bytes = static_cast<int>(f.header_bytes);
+    p.nsub = z.nsub;
+    p.nchannels = z.nchannels;
+    p.kind = f.table_kind;
+    p.blob = f.blob;
+    p.off_scales = f.off_scales;
+    p.off_tables = f.off_tables;
+    p.tables_bytes = f.tables_bytes;
+    p.off_lengths = f.off_lengths;
+    p.off_payload = f.off_payload;
+    p.off_masks = f.off_masks;
+    p.off_counts = f.off_counts;
+    p.scales_k = static_cast<const uint16_t *>(b.scales_k);
+    p.scales_v = static_cast<const uint16_t *>(b.scales_v);
+    p.nscales = static_cast<int64_t>(b.nlayers) * b.ntokens;
+    p.tables = f.table_kind == CG_TABLES_CDF ? reinterpret_cast<const uint8_t *>(b.cdf) : b.counts;
+    p.count_row_off = b.table_row_off;
+    p.mask_row_off = f.mask_row_off;
+    p.bins = b.bins;
+    p.group_nz = reinterpret_cast<const uint32_t *>(ws + z.group_nz);
+    p.scratch = ws + z.scratch;
+    p.lengths = reinterpret_cast<const int32_t *>(ws + z.lengths);
+    p.group_off = reinterpret_cast<const int64_t *>(ws + z.group_off);
+    p.stride = z.stride;
+    const dim3 grid(z.nslab, z.nrows, z.nsub + 1);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (fused_ok(b)) container_kernel<true><<<grid, kGroup, 0, st>>>(p);  // which of the two encoders wrote the scratch
+    else container_kernel<false><<<grid, kGroup, 0, st>>>(p);
+    return check_launch();
 }

@@ -14,11 +14,6 @@ __device__ __forceinline__ uint32_t count_mask(const uint8_t *cnt, int64_t strid
     return m;
 }
 
-__device__ __forceinline__ int stored_symbols(const float *bins, int row) {
-    const int n = 2 * static_cast<int>(half_range(__ldg(bins + row)));
-    return n < 32 ? n : 32;  // wider rows cannot be written in this form: the caller rules them out
-}
-
 // pass 1: masks out, and the number of non-zero counts of every (row, group)
 __global__ void __launch_bounds__(kGroup) sparse_masks_kernel(const uint8_t *counts, const int64_t *count_row_off,
                                                               const float *bins, int nchannels, uint8_t *masks,
@@ -78,27 +73,6 @@ __global__ void __launch_bounds__(kGroup) sparse_pack_kernel(const uint8_t *coun
         if ((m >> j) & 1u) *o++ = __ldg(cnt + static_cast<int64_t>(j) * nchannels);
 }
 
-// masks and counts to their places in one pass, the group offsets being known (they came with the chunk's sizes):
-// where three passes and a scan each read the counts, one read; 6 us for 20 rows of 1,024 channels, latency
-__global__ void __launch_bounds__(kGroup) sparse_write_kernel(const uint8_t *counts, const int64_t *count_row_off,
-                                                              const float *bins, int nchannels, const uint32_t *group_off,
-                                                              uint8_t *masks, const int64_t *mask_row_off, uint8_t *out) {
-    __shared__ int warp_sums[kGroup / 32];
-    const int tid = threadIdx.x, row = blockIdx.y, c = blockIdx.x * kGroup + tid;
-    const int nstored = stored_symbols(bins, row);
-    const uint8_t *cnt = counts + __ldg(count_row_off + row) + c;
-    uint32_t m = 0;
-    if (c < nchannels) {
-        m = count_mask(cnt, nchannels, nstored);
-        uint8_t *mrow = masks + __ldg(mask_row_off + row);
-        if (nstored <= 16) reinterpret_cast<uint16_t *>(mrow)[c] = static_cast<uint16_t>(m);
-        else reinterpret_cast<uint32_t *>(mrow)[c] = m;
-    }
-    const int excl = block_exclusive_scan_128(__popc(m), warp_sums, tid, nullptr);
-    uint8_t *o = out + group_off[static_cast<int64_t>(row) * gridDim.x + blockIdx.x] + excl;
-    for (; m; m &= m - 1u) *o++ = __ldg(cnt + static_cast<int64_t>(__ffs(m) - 1) * nchannels);
-}
-
 // group sizes alone (no masks kept), then their offsets
 __global__ void __launch_bounds__(kGroup) sparse_sizes_kernel(const uint8_t *counts, const int64_t *count_row_off,
                                                               const float *bins, int nchannels, uint32_t *group_bytes) {
@@ -117,15 +91,6 @@ int launch_sparse_sizes(const uint8_t *counts, const int64_t *count_row_off, con
     sparse_sizes_kernel<<<grid, kGroup, 0, st>>>(counts, count_row_off, bins, nchannels, group_off);
     if (int rc = check_launch()) return rc;
     sparse_scan_kernel<<<1, 1024, 0, st>>>(group_off, nrows * static_cast<int>(grid.x));
-    return check_launch();
-}
-
-int launch_sparse_write(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
-                        const uint32_t *group_off, void *masks, const int64_t *mask_row_off, uint8_t *out,
-                        cudaStream_t st) {
-    const dim3 grid((nchannels + kGroup - 1) / kGroup, nrows);
-    sparse_write_kernel<<<grid, kGroup, 0, st>>>(counts, count_row_off, bins, nchannels, group_off,
-                                                 static_cast<uint8_t *>(masks), mask_row_off, out);
     return check_launch();
 }
 
