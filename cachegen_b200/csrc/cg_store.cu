@@ -983,9 +983,10 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
 
 extern "C" int cg_encode_kv(const cg_encode_kv_job *job, void *stream) { return encode_jobs(job, 1, true, stream); }
 
-extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void *stream) { return encode_jobs(jobs, njobs, false, stream); }
+// A single setting is what is left over in front of groups of four (see _encode_infos in cachegen_encoder.py).
+extern "C" int cg_encode_kv_levels(const cg_encode_kv_job *jobs, int njobs, void *stream) { return encode_jobs(jobs, njobs, njobs > 1, stream); }
 
-// alone: no other encode follows at once on the stream
+// alone: no other encode follows at once on the stream, or only behind several settings' coder
 static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void *stream) {
     if (njobs < 1) return CG_E_SHAPE;
     if (njobs > CG_MAX_ENCODE_LEVELS) return CG_E_CAPACITY;
@@ -1060,8 +1061,8 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
     const dim3 grid(z.nslab, z.nrows, z.nsub * njobs);
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
     // The coder of one sub-chunk starts under the quantiser's last blocks: 206 -> 202 us for a 256-token Llama-7B chunk.  Not
-    // where another quantiser follows at once, which then starts late (three quality levels 262 -> 285 us), and not behind or in
-    // front of the tables' kernel (1,999 tokens in one call 415 -> 420).
+    // where another quantiser follows at once, which then starts late, and not behind or in front of the tables' kernel (1,999
+    // tokens in one call 415 -> 420).  Three quality levels in one call 197 -> 193.5 us, five in two 278 -> 272.
     const bool early = alone && z.nsub == 1;
     const auto store = [&](auto kernel, int threads, size_t smem) {
         if (early) smem = spread_smem(static_cast<int64_t>(grid.x) * grid.y * grid.z, smem);
