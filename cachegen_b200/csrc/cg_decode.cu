@@ -731,17 +731,20 @@ static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool ear
 }
 
 // ---- group offsets ------------------------------------------------------------------------------------------
-// One cluster of eight blocks per job: every block sums the lengths of an eighth of the 128-channel groups and
+// One cluster of BLOCKS blocks per job: every block sums the lengths of its share of the 128-channel groups and
 // scans its sums, then adds the totals of the blocks before it, which it reads in their shared memory.  One
 // launch where a sum kernel and a scan kernel were two (5 us of 23 for a 37-token chunk), and nothing to zero.  Bound
-// by latency: 4.3 us for 20,480 lengths, 11 for 262,144.
+// by latency: 4.2 us for 20,480 lengths in eight blocks with four groups in flight a warp, 13.9 for 262,144, which take 10 in
+// sixteen blocks with eight.  Its blocks are launched early and wait for the launch in front before they read anything, the decode's
+// start once all of them have waited: 1 to 4 us less a call.
 struct OffsetJobs {
     const void *lengths[CG_MAX_DECODE_JOBS];
     int64_t *group_off[CG_MAX_DECODE_JOBS];
     int64_t expect[CG_MAX_DECODE_JOBS];
     int32_t kind[CG_MAX_DECODE_JOBS];
 };
-constexpr int kOffsetBlocks = 8, kOffsetThreads = 512, kMaxOffsetGroups = CG_MAX_OFFSET_GROUPS;
+constexpr int64_t kWideOffsets = 1024;
+constexpr int kOffsetThreads = 512, kMaxOffsetGroups = CG_MAX_OFFSET_GROUPS;
 
 // For callers that wait for the sum of one job's lengths (tail: host memory that the GPU can write): [0] the sum,
 // [1] 1 if a length is negative or above `longest`, [2] the word at `extra`, then [3] becomes 1.
@@ -757,30 +760,32 @@ __device__ __forceinline__ int clamped_length(int v, int longest, bool *bad) {
     return v;
 }
 
-__global__ void __cluster_dims__(kOffsetBlocks, 1, 1) __launch_bounds__(kOffsetThreads)
+template <int BLOCKS, int AHEAD>  // AHEAD: groups a warp has in flight
+__global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(kOffsetThreads)
 group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nchannels, int nslab, int32_t *status,
                      const StreamSizes sizes) {
     extern __shared__ int sums[];  // the groups of this block
     __shared__ int64_t warp_sums[kOffsetThreads / 32];
     __shared__ int64_t block_total;
     __shared__ uint32_t block_bad;
+    wait_for_launch_before();
     let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) block_bad = 0u;
-    const int j = blockIdx.x / kOffsetBlocks, rank = blockIdx.x % kOffsetBlocks;
-    const int ngroups = nrows * nslab, per = (ngroups + kOffsetBlocks - 1) / kOffsetBlocks;
+    const int j = blockIdx.x / BLOCKS, rank = blockIdx.x % BLOCKS;
+    const int ngroups = nrows * nslab, per = (ngroups + BLOCKS - 1) / BLOCKS;
     const int first = min(ngroups, rank * per), count = min(ngroups, first + per) - first;
     const bool u16 = jobs.kind[j] == CG_LENGTHS_U16;
     const void *lengths = jobs.lengths[j];
     // four lengths a load where the rows allow it
     const bool vec = nchannels % kGroup == 0 && (reinterpret_cast<uintptr_t>(lengths) & (u16 ? 7 : 15)) == 0;
     bool bad = false;
-    constexpr int kWarps = kOffsetThreads / 32, kAhead = 4;  // groups a warp has in flight
+    constexpr int kWarps = kOffsetThreads / 32;
     if (vec) {
-        for (int k0 = warp; k0 < count; k0 += kWarps * kAhead) {
-            int s[kAhead];
+        for (int k0 = warp; k0 < count; k0 += kWarps * AHEAD) {
+            int s[AHEAD];
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) {
+            for (int i = 0; i < AHEAD; ++i) {
                 const int k = k0 + i * kWarps;
                 const int64_t at = static_cast<int64_t>(first + k) * 32 + lane;
                 int4 q = make_int4(0, 0, 0, 0);
@@ -796,7 +801,7 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
                        clamped_length(q.z, sizes.longest, &bad) + clamped_length(q.w, sizes.longest, &bad);
             }
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) {
+            for (int i = 0; i < AHEAD; ++i) {
                 s[i] = __reduce_add_sync(0xFFFFFFFFu, s[i]);
                 if (lane == 0 && k0 + i * kWarps < count) sums[k0 + i * kWarps] = s[i];
             }
@@ -838,7 +843,7 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
     int64_t all = 0;
 #pragma unroll
-    for (int r = 0; r < kOffsetBlocks; ++r) {
+    for (int r = 0; r < BLOCKS; ++r) {
         uint32_t remote;
         int64_t v;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&block_total)), "r"(r));
@@ -854,7 +859,7 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
     if (status && (bad || (rank == 0 && tid == 0 && all != jobs.expect[j]))) atomicOr(status, CG_S_BAD_LENGTHS);
     if (sizes.tail && rank == 0 && tid == 0) {
         uint32_t any = 0;
-        for (int r = 0; r < kOffsetBlocks; ++r) {
+        for (int r = 0; r < BLOCKS; ++r) {
             uint32_t remote, v;
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&block_bad)), "r"(r));
             asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote));
@@ -879,9 +884,22 @@ static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int n
         o.kind[j] = jobs[j].length_kind;
     }
     const int nslab = (nchannels + kGroup - 1) / kGroup;
-    const size_t smem = static_cast<size_t>((static_cast<int64_t>(nrows) * nslab + kOffsetBlocks - 1) / kOffsetBlocks) * sizeof(int);
-    group_offsets_kernel<<<njobs * kOffsetBlocks, kOffsetThreads, smem, st>>>(o, nrows, nchannels, nslab, status, sizes);
-    return check_launch();
+    const int64_t groups = static_cast<int64_t>(nrows) * nslab;
+    const auto run = [&](auto kernel, int blocks) {
+        return launch(kernel, dim3(static_cast<unsigned>(njobs * blocks)), kOffsetThreads, static_cast<size_t>((groups + blocks - 1) / blocks) * sizeof(int),
+                      true, st, o, nrows, nchannels, nslab, status, sizes);
+    };
+    // Sixteen blocks where a warp of eight would take more than eight groups, in more than two rounds of loads.  20 tokens, us a
+    // call with eight and with sixteen: 640 groups 12.8 and 13.1, 768 12.9 and 12.9, 1,280 16.9 and 15.8, 2,048 25.4 and 23.4.
+    // Such clusters have to be allowed, and where a GPU (a part of one, say) has no room for them eight blocks do as well.
+    if (groups > kWideOffsets) {
+        const auto wide = group_offsets_kernel<16, 8>;
+        if (cudaFuncSetAttribute(wide, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            if (run(wide, 16) == CG_OK) return CG_OK;
+        }
+        cudaGetLastError();
+    }
+    return run(group_offsets_kernel<8, 4>, 8);
 }
 
 }  // namespace cg
