@@ -57,6 +57,12 @@ int launch(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, bool ea
     return e == cudaSuccess ? CG_OK : set_cuda_error(e);
 }
 
+// multiprocessors of the current device; 1 if it does not say
+inline int sm_count() {
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 ? sms : 1;
+}
+
 // cg_tables.cu: group offsets of sparse tables
 int launch_sparse_sizes(const uint8_t *counts, const int64_t *count_row_off, const float *bins, int nrows, int nchannels,
                         uint32_t *group_off, cudaStream_t st);

@@ -448,8 +448,12 @@ __device__ __forceinline__ uint32_t pack_pair<CG_BF16>(float v0, float v1) {
 // DELTA (anchor-token delta, see cg_decode_dequant_delta): in rows with residual bins every token that is
 // not the first of its group of delta_group adds its value, ((sym - Cq_a) / Cq_r) * max, to its
 // anchor's value as the KV dtype holds it; the sum is cast to the output type.
-template <int NS, int OUT_DT, bool DELTA>
-__global__ void __launch_bounds__(kGroup / NS, kMultiBlocksPerSM)
+// QUICK: see decode_streams; for grids of at most kQuickBlocksPerSM blocks an SM, which leaves the compiler the registers for it.
+// 256 tokens, us a call without and with it: 160 blocks 60.7 and 54.5, 512 66.6 and 62.2, 640 73.9 and 73.1, 1,280 105 and 126;
+// 37 tokens of 512 blocks 14.9 and 14.4.
+constexpr int kQuickBlocksPerSM = 4;
+template <int NS, int OUT_DT, bool DELTA, bool QUICK>
+__global__ void __launch_bounds__(kGroup / NS, QUICK ? kQuickBlocksPerSM + 1 : kMultiBlocksPerSM)
 decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int scale_dt, int full_levels) {
     constexpr int kThreads = kGroup / NS;
     constexpr int kWarps = kThreads / 32;
@@ -663,11 +667,11 @@ decode_dequant_multi_kernel(const __grid_constant__ FusedDecodeParams p, int sca
     const int top = (1 << fl) - 1;
     const uint32_t det = smem_addr(smem) + static_cast<uint32_t>(top < maxsym ? top : maxsym) * kRowBytes;
     switch (fl) {
-    case 2: decode_streams<2, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
-    case 3: decode_streams<3, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
-    case 4: decode_streams<4, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
-    case 5: decode_streams<5, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
-    default: decode_streams<6, NS, true>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 2: decode_streams<2, NS, true, QUICK>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 3: decode_streams<3, NS, true, QUICK>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 4: decode_streams<4, NS, true, QUICK>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    case 5: decode_streams<5, NS, true, QUICK>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
+    default: decode_streams<6, NS, true, QUICK>(Smem{}, col, det, maxsym, full_levels, streams, lens, ntok_r, 0xFFFFFFFFu, emit, sc_a); break;
     }
     if (p.after == kAfterBatch) wait_for_launch_before();
 }
@@ -726,8 +730,13 @@ static bool offsets_fit(const FusedDecodeParams &p) {
 template <int NS, int OUT_DT, bool DELTA>
 static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool early, cudaStream_t st) {
     const int full = search_levels(p.lp);
-    return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA>, dim3(p.nslab, 2 * p.nlayers, p.njobs), kGroup / NS,
-                  table_bytes(p.lp, full < 2 ? 2 : full), early, st, p, scale_dt, full);
+    const dim3 grid(p.nslab, 2 * p.nlayers, p.njobs);
+    const int64_t blocks = static_cast<int64_t>(grid.x) * grid.y * grid.z;
+    const size_t smem = table_bytes(p.lp, full < 2 ? 2 : full);
+    if (!DELTA && blocks <= static_cast<int64_t>(kQuickBlocksPerSM) * sm_count())
+        return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA, !DELTA>, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
+    const auto kernel = decode_dequant_multi_kernel<NS, OUT_DT, DELTA, false>;
+    return launch(kernel, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
 }
 
 // ---- group offsets ------------------------------------------------------------------------------------------

@@ -969,10 +969,7 @@ static int encode_separately(const cg_encode_kv_job &b, cudaStream_t st) {
 static size_t spread_smem(int64_t blocks, size_t dynamic) {
     constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024, kMostResident = 8;  // bytes of an SM, of each block; launch bounds
     const int64_t fit = kSmemPerSM / (static_cast<int64_t>(dynamic) + kMostStaticSmem + kReserved);
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-        return dynamic;
-    const int64_t share = (blocks + sms - 1) / sms;
+    const int64_t sms = sm_count(), share = (blocks + sms - 1) / sms;
     if (share >= (fit < kMostResident ? fit : kMostResident)) return dynamic;
     // the least that keeps one more out, so that the first of them find room beside the launch in front
     const size_t least = static_cast<size_t>(kSmemPerSM / (share + 1) - kReserved + 256);

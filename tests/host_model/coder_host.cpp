@@ -2,6 +2,7 @@
 // test-suite only: lets the tests drive the exact decode/encode step code against the oracle without
 // a GPU.  Not part of the shipped library.
 #include <cstring>
+#include <string.h>
 #include <vector>
 
 #include "../../cachegen_b200/csrc/cg_coder.cuh"
@@ -63,7 +64,7 @@ extern "C" void hm_decode_stream(const uint16_t *cdf, int lp, const uint8_t *byt
 // Two streams side by side through decode_streams, as the two-channels-per-thread kernel runs them:
 // tables in columns tid and tid + 64, search depth fl forced by the caller (any depth must give the
 // same symbols).  out receives the symbols interleaved: out[2 * token + stream].
-template <int FL>
+template <int FL, bool QUICK>
 static void run_pair(const uint16_t *cdf0, const uint16_t *cdf1, int lp, const uint8_t *b0, int64_t l0,
                      const uint8_t *b1, int64_t l1, int n, uint8_t *out, int tid) {
     const int full = search_levels(lp);
@@ -78,10 +79,20 @@ static void run_pair(const uint16_t *cdf0, const uint16_t *cdf1, int lp, const u
     const uint32_t det = static_cast<uint32_t>(top < maxsym ? top : maxsym) * kTableRowBytes;
     const uint8_t *const streams[2] = {b0, b1};
     const uint32_t lens[2] = {static_cast<uint32_t>(l0), static_cast<uint32_t>(l1)};
-    decode_streams<FL, 2>(rd, col, det, maxsym, full, streams, lens, n, 0xFFFFFFFFu, [&](const uint32_t(&a)[2], uint32_t) {
+    decode_streams<FL, 2, false, QUICK>(rd, col, det, maxsym, full, streams, lens, n, 0xFFFFFFFFu, [&](const uint32_t(&a)[2], uint32_t) {
         *out++ = static_cast<uint8_t>((a[0] - col[0]) / kTableRowBytes);
         *out++ = static_cast<uint8_t>((a[1] - col[1]) / kTableRowBytes);
     });
+}
+
+// The form for many warps and the one for few, which have to agree.
+template <int FL>
+static int both_forms(const uint16_t *cdf0, const uint16_t *cdf1, int lp, const uint8_t *b0, int64_t l0, const uint8_t *b1, int64_t l1, int n,
+                      uint8_t *out, int tid) {
+    std::vector<uint8_t> quick(2 * static_cast<size_t>(n));
+    run_pair<FL, false>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
+    run_pair<FL, true>(cdf0, cdf1, lp, b0, l0, b1, l1, n, quick.data(), tid);
+    return memcmp(out, quick.data(), quick.size()) ? -2 : 0;
 }
 
 extern "C" int hm_decode_pair(const uint16_t *cdf0, const uint16_t *cdf1, int lp, const uint8_t *b0, int64_t l0,
@@ -89,13 +100,12 @@ extern "C" int hm_decode_pair(const uint16_t *cdf0, const uint16_t *cdf1, int lp
     const int full = search_levels(lp);
     if (fl < 2 || fl > 6 || (fl > full && fl > 2) || tid < 0 || tid >= 64) return -1;
     switch (fl) {
-    case 2: run_pair<2>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid); break;
-    case 3: run_pair<3>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid); break;
-    case 4: run_pair<4>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid); break;
-    case 5: run_pair<5>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid); break;
-    default: run_pair<6>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid); break;
+    case 2: return both_forms<2>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
+    case 3: return both_forms<3>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
+    case 4: return both_forms<4>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
+    case 5: return both_forms<5>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
+    default: return both_forms<6>(cdf0, cdf1, lp, b0, l0, b1, l1, n, out, tid);
     }
-    return 0;
 }
 
 extern "C" int hm_fast_levels_for(int nsym, int full_levels) { return fast_levels_for(nsym, full_levels); }
