@@ -683,14 +683,35 @@ static size_t table_bytes(int lp, int levels) {
 }
 static_assert((CG_MAX_LP + 1) * kRowBytes + 4 * (kSubTokens + 2 * CG_MAX_LP) + 64 <= kSmemByItself, "a decoder block's shared memory");
 
+// Shared memory to ask for so that a grid leaves no short second wave.  Twelve blocks an SM, and then one to four more on each, whose
+// serial chains take most of a wave's time with next to nothing beside them: fewer at first, so that the others get company.
+// us a call of 256 tokens of 32 layers with twelve and with so many (blocks a multiprocessor): 1,792 blocks (13) 145.4 and 146.9 (8),
+// 1,920 (13) 154.3 and 148.2, 2,048 (14) 166 and 152.7, 2,112 (15) 161.1 and 159.7 (10), 2,176 (15) 170.2 and 160.6,
+// 2,240 (16) 171.2 and 160.5, 2,368 (16) 173.8 and 172.7; 2,560 (18) 181 and 183.5 with ten.  The extension module's decode of 2,048
+// blocks, whose path takes 336 us, 8 us less.
+template <class Kernel>
+static size_t evened_smem(Kernel kernel, int64_t blocks, size_t dynamic) {
+    constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024;  // bytes of an SM, of each block
+    const int64_t share = (blocks + sm_count() - 1) / sm_count();
+    if (share <= kMultiBlocksPerSM || share > kMultiBlocksPerSM + 4) return dynamic;
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return dynamic;
+    const int64_t fixed = static_cast<int64_t>(at.sharedSizeBytes) + kReserved;
+    if ((static_cast<int64_t>(dynamic) + fixed) * kMultiBlocksPerSM > kSmemPerSM) return dynamic;  // long tables: fewer as it is
+    const int64_t resident = share <= kMultiBlocksPerSM + 2 ? 8 : 10;
+    return static_cast<size_t>(kSmemPerSM / (resident + 1) - fixed + 256);  // the least that keeps one more out
+}
+
 // Instantiated search depths: 3..6, whatever the table length.
 template <int MODE>
 static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) {
     const int need = search_levels(p.lp);
     const dim3 grid((p.nchannels + kGroup - 1) / kGroup, nrows);
+    const int64_t blocks = static_cast<int64_t>(grid.x) * grid.y;
     const bool pairs = p.o2 == 1 && ((p.o0 | p.o1 | p.nchannels) & 1) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 1) == 0;
 #define CG_LAUNCH_SYM(L)                                                                                      \
-    return pairs ? launch(decode_symbols_pair_kernel<L, MODE>, grid, kGroup / 2, table_bytes(p.lp, L), MODE == 2, st, p) \
+    return pairs ? launch(decode_symbols_pair_kernel<L, MODE>, grid, kGroup / 2,                               \
+                          evened_smem(decode_symbols_pair_kernel<L, MODE>, blocks, table_bytes(p.lp, L)), MODE == 2, st, p) \
                  : launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
     if (need <= 3) CG_LAUNCH_SYM(3);
     if (need == 4) CG_LAUNCH_SYM(4);
@@ -736,7 +757,7 @@ static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool ear
     if (!DELTA && blocks <= static_cast<int64_t>(kQuickBlocksPerSM) * sm_count())
         return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA, !DELTA>, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
     const auto kernel = decode_dequant_multi_kernel<NS, OUT_DT, DELTA, false>;
-    return launch(kernel, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
+    return launch(kernel, grid, kGroup / NS, evened_smem(kernel, blocks, smem), early, st, p, scale_dt, full);
 }
 
 // ---- group offsets ------------------------------------------------------------------------------------------

@@ -50,3 +50,18 @@ def test_the_quick_form_at_every_depth(bins):
     assert torch.equal(many.view(torch.int16), one.repeat(1, 1, 120, 1, 1).view(torch.int16))
     x = kv.float()
     assert ((one.float() - x).abs() <= x.abs().amax((3, 4), keepdim=True) * (0.51 / (bins // 2 - 1))).all()
+
+
+@pytest.mark.parametrize("rows, channels", [(20, 512), (60, 4096), (64, 4096)])
+def test_symbols_come_back_at_either_side_of_a_wave(rows, channels):
+    from cachegen_b200 import torchac_cuda
+    sym = torch.randint(0, 31, (rows, 70, channels), generator=torch.Generator().manual_seed(rows)).to(torch.int8).cuda()
+    sym[: rows // 2] %= 9
+    from cachegen_b200.serde import cachegen_encoder as E
+    cdf = torchac_cuda.calculate_cdf(sym, 32)
+    buf = torch.empty((rows, channels, 520), dtype=torch.uint8, device="cuda")
+    lengths = torch.empty((rows, channels), dtype=torch.int32, device="cuda")
+    streams = E.encode_ntokens(cdf, sym, buf, lengths)
+    out = torch.empty((rows, 70, channels), dtype=torch.uint8, device="cuda")
+    torchac_cuda.decode_by_lengths(cdf, streams, lengths, out)
+    assert torch.equal(out.view(torch.int8), sym)
