@@ -42,15 +42,15 @@ __device__ __forceinline__ void quantize2(float x0, float x1, float f, uint64_t 
     asm("mov.b64 {%0, %1}, %2;" : "=r"(*b0), "=r"(*b1) : "l"(v));
 }
 
-// Pass 1.  A block takes four tokens of one row, all channels, eight adjacent ones a thread: the 16-bit values stay in
-// registers between the scales (a reduction over the block) and the symbols, so the KV is read once where an
+// Pass 1.  A block takes four tokens of one row, all channels, eight adjacent ones a thread in one or two runs: the 16-bit values
+// stay in registers between the scales (a reduction over the block) and the symbols, so the KV is read once where an
 // absmax pass and a quantise pass read it twice, and four tokens' symbols of a channel leave as one word.  Bound
-// by memory and by about as much issue: a 256-token Llama-7B chunk (134 MB in, 67 MB of symbols out) takes 38 us,
-// 5.3 TB/s, where the two passes took 31 + 61 us (the second with the histogram, which the coder does now).  9.3 instructions
-// for 32 symbols; with the layer and the half of the pair divided out of one grid dimension, the bins halved by a division and
-// every word zeroed before it is loaded 11.6, 40 us, and 63 where 1,999 tokens of 32 layers x 1,024 channels take 58.
-// Three blocks of 512 threads an SM (42 registers a thread) keep enough loads in flight; more than 4,096
-// channels need one block of up to 1,024 threads.
+// by memory: a 256-token Llama-7B chunk (134 MB in, 67 MB of symbols out) takes 33 us, 6.1 TB/s, where the two passes took
+// 31 + 61 us (the second with the histogram, which the coder does now).  With one run a thread, three blocks of sixteen warps an SM
+// all waited for loads or all computed: 39.7 us, and 59.3 where 5,120 channels take 41.5, 41 where 10 layers of 8,192 take 26, 19.6 and 17.6
+// for 2,048, 60.5 and 58 for 1,999 tokens of 32 layers x 1,024.  9.3 instructions for 32 symbols; with the layer and the half of the
+// pair divided out of one grid dimension, the bins halved by a division and every word zeroed before it is loaded 11.6.
+// Sixty-four registers and four blocks of eight warps an SM; five blocks (48 registers) 33.9 us, three 36.2.
 // The same KV at several bin settings takes one read and one reduction: only the quantisation is done for each.
 struct QuantizeOut {
     const float *bins;
@@ -62,7 +62,7 @@ struct QuantizeLevels {
     QuantizeOut level[CG_MAX_ENCODE_LEVELS];
     int n, nzeroed;
 };
-template <int DT, int THREADS, int BLOCKS, bool ONE>
+template <int DT, int THREADS, int BLOCKS, bool ONE, int RUNS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const KvView v, const __grid_constant__ QuantizeLevels q) {
     __shared__ uint4 part[32];
     __shared__ float4 factor_s[ONE ? 1 : CG_MAX_ENCODE_LEVELS];
@@ -71,29 +71,38 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const 
     let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int layer = blockIdx.y, kv = blockIdx.z, row = kv * v.nlayers + layer, t0 = blockIdx.x * kTokensPerWord;
-    const int C = v.nheads * v.head_size, c = tid * 8;
+    const int C = v.nheads * v.head_size;
     if (row == 0 && blockIdx.x == 0)  // the counters of the launches after this one
         for (int l = 0; l < nlevels; ++l)
             for (int i = tid; i < q.nzeroed; i += blockDim.x) q.level[l].zeroed[i] = 0u;
-    uint4 x[kTokensPerWord];
-    const int h = static_cast<int>(__umulhi(static_cast<uint32_t>(c), v.head_inv));
-    const uint16_t *p = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token + h * v.s_head + (c - h * v.head_size);
-    if (c < C && t0 + kTokensPerWord <= v.ntokens) {
+    // run r of this thread's channels starts at 8 (tid + blockDim.x r)
+    uint4 x[RUNS][kTokensPerWord];
+    const uint16_t *tokens = v.kv + layer * v.s_layer + kv * v.s_kv + t0 * v.s_token;
 #pragma unroll
-        for (int j = 0; j < kTokensPerWord; ++j) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
-    } else {
+    for (int r = 0; r < RUNS; ++r) {
+        const int c = (tid + r * static_cast<int>(blockDim.x)) * 8;
+        const int h = static_cast<int>(__umulhi(static_cast<uint32_t>(c), v.head_inv));
+        const uint16_t *p = tokens + h * v.s_head + (c - h * v.head_size);
+        if (c < C && t0 + kTokensPerWord <= v.ntokens) {
 #pragma unroll
-        for (int j = 0; j < kTokensPerWord; ++j) {
-            x[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (c < C && t0 + j < v.ntokens) x[j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+            for (int j = 0; j < kTokensPerWord; ++j) x[r][j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+        } else {
+#pragma unroll
+            for (int j = 0; j < kTokensPerWord; ++j) {
+                x[r][j] = make_uint4(0u, 0u, 0u, 0u);
+                if (c < C && t0 + j < v.ntokens) x[r][j] = __ldg(reinterpret_cast<const uint4 *>(p + j * v.s_token));
+            }
         }
     }
     // |x| as an ordered integer: 16-bit float magnitudes compare like their bit patterns
     uint32_t m[kTokensPerWord];
 #pragma unroll
     for (int j = 0; j < kTokensPerWord; ++j) {
-        const uint32_t a = __vmaxu2(__vmaxu2(x[j].x & 0x7FFF7FFFu, x[j].y & 0x7FFF7FFFu),
-                                    __vmaxu2(x[j].z & 0x7FFF7FFFu, x[j].w & 0x7FFF7FFFu));
+        uint32_t a = 0u;
+#pragma unroll
+        for (int r = 0; r < RUNS; ++r)
+            a = __vmaxu2(a, __vmaxu2(__vmaxu2(x[r][j].x & 0x7FFF7FFFu, x[r][j].y & 0x7FFF7FFFu),
+                                     __vmaxu2(x[r][j].z & 0x7FFF7FFFu, x[r][j].w & 0x7FFF7FFFu)));
         m[j] = __reduce_max_sync(0xFFFFFFFFu, max(a & 0xFFFFu, a >> 16));
     }
     if (lane == 0) part[warp] = make_uint4(m[0], m[1], m[2], m[3]);
@@ -121,37 +130,41 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) quantize_tokens_kernel(const 
         }
     }
     __syncthreads();
-    if (c >= C) return;
     const uint32_t keep = keep_s;
 #pragma unroll 1
     for (int l = 0; l < nlevels; ++l) {
         const float f[kTokensPerWord] = {factor_s[l].x, factor_s[l].y, factor_s[l].z, factor_s[l].w};
         const float MAX = l ? half_range(__ldg(q.level[l].bins + row)) : max_of_first;
         const uint64_t m2 = pack2(MAX, MAX);
-        uint32_t w[8];
 #pragma unroll
-        for (int k = 0; k < 8; k += 2) {
-            uint32_t b0[kTokensPerWord], b1[kTokensPerWord];
+        for (int r = 0; r < RUNS; ++r) {
+            const int c = (tid + r * static_cast<int>(blockDim.x)) * 8;
+            if (c >= C) break;
+            uint32_t w[8];
 #pragma unroll
-            for (int j = 0; j < kTokensPerWord; ++j) {
-                const uint32_t pair = k == 0 ? x[j].x : k == 2 ? x[j].y : k == 4 ? x[j].z : x[j].w;
-                quantize2(Half16<DT>::to_float(static_cast<uint16_t>(pair)), Half16<DT>::to_float(static_cast<uint16_t>(pair >> 16)),
-                          f[j], m2, &b0[j], &b1[j]);
+            for (int k = 0; k < 8; k += 2) {
+                uint32_t b0[kTokensPerWord], b1[kTokensPerWord];
+#pragma unroll
+                for (int j = 0; j < kTokensPerWord; ++j) {
+                    const uint32_t pair = k == 0 ? x[r][j].x : k == 2 ? x[r][j].y : k == 4 ? x[r][j].z : x[r][j].w;
+                    quantize2(Half16<DT>::to_float(static_cast<uint16_t>(pair)), Half16<DT>::to_float(static_cast<uint16_t>(pair >> 16)),
+                              f[j], m2, &b0[j], &b1[j]);
+                }
+                w[k] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410) & keep;
+                w[k + 1] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410) & keep;
             }
-            w[k] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410) & keep;
-            w[k + 1] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410) & keep;
-        }
-        // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
-        // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
-        const int max_bins = q.level[l].max_bins;
-        if (2.0f * MAX >= static_cast<float>(max_bins - 1)) {
-            const uint32_t limit = static_cast<uint32_t>(max_bins - 1) * 0x01010101u;
+            // The coder takes any byte above 127 for a bad symbol.  Inputs that are not finite give 255 as they are;
+            // other symbols stay below 2*Cq + 1, which only bin counts above max_bins put outside the table.
+            const int max_bins = q.level[l].max_bins;
+            if (2.0f * MAX >= static_cast<float>(max_bins - 1)) {
+                const uint32_t limit = static_cast<uint32_t>(max_bins - 1) * 0x01010101u;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] |= __vcmpgeu4(w[k], limit);
+                for (int k = 0; k < 8; ++k) w[k] |= __vcmpgeu4(w[k], limit);
+            }
+            uint4 *o = reinterpret_cast<uint4 *>(q.level[l].sym4 + (static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * C + c);
+            o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            o[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
-        uint4 *o = reinterpret_cast<uint4 *>(q.level[l].sym4 + (static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * C + c);
-        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -1042,18 +1055,20 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
         lp = p.lp > lp ? p.lp : lp;
     }
     const dim3 qgrid(static_cast<unsigned>(z.words), static_cast<unsigned>(jobs->nlayers), 2);
-    const int qthreads = (z.nchannels / 8 + 31) / 32 * 32;
-#define CG_LAUNCH_QT(DT, THREADS, BLOCKS)                                                                    \
-    njobs == 1 ? quantize_tokens_kernel<DT, THREADS, BLOCKS, true><<<qgrid, qthreads, 0, st>>>(v, q)          \
-               : quantize_tokens_kernel<DT, THREADS, BLOCKS, false><<<qgrid, qthreads, 0, st>>>(v, q)
-    if (b.dtype == CG_F16) {
-        if (qthreads <= 512) CG_LAUNCH_QT(CG_F16, 512, 3);
-        else CG_LAUNCH_QT(CG_F16, 1024, 1);
-    } else {
-        if (qthreads <= 512) CG_LAUNCH_QT(CG_BF16, 512, 3);
-        else CG_LAUNCH_QT(CG_BF16, 1024, 1);
-    }
+    // Two runs of channels a thread from 1,024 channels on; below, what half as many warps have no channels for would cost more
+    // (768 channels 7.6 us, 6.8 with one run).  Several settings want more registers.
+    const int runs = z.nchannels >= 1024 ? 2 : 1, qthreads = (z.nchannels / 8 + 32 * runs - 1) / (32 * runs) * 32;
+#define CG_LAUNCH_QT(DT, THREADS, BLOCKS, BLOCKS_MORE, RUNS)                                                         \
+    njobs == 1 ? quantize_tokens_kernel<DT, THREADS, BLOCKS, true, RUNS><<<qgrid, qthreads, 0, st>>>(v, q)            \
+               : quantize_tokens_kernel<DT, THREADS, BLOCKS_MORE, false, RUNS><<<qgrid, qthreads, 0, st>>>(v, q)
+#define CG_LAUNCH_QD(DT)                                      \
+    if (runs == 1) CG_LAUNCH_QT(DT, 128, 12, 12, 1);          \
+    else if (qthreads <= 256) CG_LAUNCH_QT(DT, 256, 4, 3, 2); \
+    else CG_LAUNCH_QT(DT, 512, 2, 2, 2)
+    if (b.dtype == CG_F16) CG_LAUNCH_QD(CG_F16);
+    else CG_LAUNCH_QD(CG_BF16);
 #undef CG_LAUNCH_QT
+#undef CG_LAUNCH_QD
     if (int rc = check_launch()) return rc;
     const dim3 grid(z.nslab, z.nrows, z.nsub * njobs);
     const size_t columns = static_cast<size_t>(lp) * kRowBytes, staged = static_cast<size_t>(lp) * kGroup * 2;
