@@ -203,6 +203,17 @@ __device__ __forceinline__ int block_exclusive_scan_128(int v, int *warp_sums, i
     return block_exclusive_scan<kGroup / 32>(v, warp_sums, tid, total);
 }
 
+// Shared-memory columns of a warp's 32 channels: entry m of lane l at word 32 m + l.  With rows of 128 bytes the
+// address of the entry that byte k of a word of symbols names is one dot product: the byte times 128, plus
+// the column.
+constexpr int kWarpRow = 128;
+__device__ __forceinline__ uint32_t entry_of(uint32_t col, uint32_t w, int k) {
+    return __dp4a(w, static_cast<uint32_t>(kWarpRow) << (8 * k), col);
+}
+__device__ __forceinline__ void count_symbol(uint32_t addr) {
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+}
+
 // ---- gather of a group's streams (second half of collect_bytes, cachegen_encoder.py:210-222) -----------------
 // Called by a block of kGroup threads, one stream each.  A warp's streams are one run of the output: each
 // lane shifts its words to the byte they start at and puts them together in shared memory (a word that two

@@ -139,22 +139,33 @@ __global__ void __launch_bounds__(256) residual_absmax_kernel(const uint16_t *__
 }
 
 // Counts to table (normalize_cdf_value, cal_cdf.cu:11-15,40-49), one thread per channel.
-// hist: shared uint32 [max_bins+1][kGroup], hist[v][c] = #{sym == v} for v < max_bins; the last row collects
+// hist: the channel's counts of `ntokens` symbols, STRIDE words apart, hist[v] = #{sym == v} for v < max_bins; the last one is of
 // the symbols outside the table (counted with min(sym, max_bins): no branch), which no entry reads.  Writes the channel's
-// lp = max_bins+1 entries to out16 (shared uint16 [kGroup][lp]).
-__device__ __forceinline__ void counts_to_table(const uint32_t *hist, int max_bins, int cl, uint16_t *out16) {
-    const int lp = max_bins + 1;
-    uint32_t total = 0;
-    for (int i = 0; i < max_bins; ++i) total += hist[i * kGroup + cl];
-    total &= 0xFFFFu;  // the reference accumulates in uint16
+// lp = max_bins+1 entries to out.
+template <int STRIDE>
+__device__ __forceinline__ void counts_to_table(const uint32_t *hist, int max_bins, int ntokens, uint16_t *out) {
+    const uint32_t total = (static_cast<uint32_t>(ntokens) - hist[max_bins * STRIDE]) & 0xFFFFu;  // the reference accumulates in uint16
     const uint32_t scale = 0xFFFFu - static_cast<uint32_t>(max_bins);
-    const bool pow2 = (total & (total - 1u)) == 0u;
-    const int sh = 31 - __clz(static_cast<int>(total | 1u));
     uint32_t cum = 0;
-    for (int i = 0; i <= max_bins; ++i) {
-        if (i) cum = (cum + hist[(i - 1) * kGroup + cl]) & 0xFFFFu;
-        const uint32_t nv = total ? (pow2 ? scale * cum >> sh : scale * cum / total) : 0u;
-        out16[cl * lp + i] = static_cast<uint16_t>(nv + i);
+    if ((total & (total - 1u)) == 0u) {
+        const int sh = 31 - __clz(static_cast<int>(total | 1u));
+#pragma unroll 8
+        for (int i = 0; i <= max_bins; ++i) {
+            const uint32_t n = hist[i * STRIDE];
+            out[i] = static_cast<uint16_t>((scale * cum >> sh) + i);
+            cum = (cum + n) & 0xFFFFu;
+        }
+    } else {
+        // the rounded-down reciprocal, whose product is at most one below the quotient
+        const uint32_t inv = 0xFFFFFFFFu / total;
+#pragma unroll 8
+        for (int i = 0; i <= max_bins; ++i) {
+            const uint32_t n = hist[i * STRIDE], prod = scale * cum;
+            uint32_t q = __umulhi(prod, inv);
+            if (prod - q * total >= total) ++q;
+            out[i] = static_cast<uint16_t>(q + i);
+            cum = (cum + n) & 0xFFFFu;
+        }
     }
 }
 
@@ -302,7 +313,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_cdf_kernel(
         }
     }
     __syncthreads();
-    if (tid < kGroup && c0 + tid < C) counts_to_table(hist, max_bins, tid, out16);
+    if (tid < kGroup && c0 + tid < C) counts_to_table<kGroup>(hist + tid, max_bins, T, out16 + tid * lp);
     if (counts_out) {
         // byte counts of the non-centre symbols, [symbol][channel] so that a warp writes a run of bytes
         const int cq = static_cast<int>(MAX);
@@ -328,13 +339,12 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_cdf_kernel(
     store_tables(out16, cdf_out, row, c0, C, lp, tid, kQuantThreads);
 }
 
-// calculate_cdf on int8 symbols: grid (nslab, nrows).  VEC: adjacent channels are adjacent bytes at 4-byte
-// boundaries, and a thread counts four channels of every eighth token, with one load for four symbols and
-// eight tokens in flight; the lanes of a warp start their counts at different ones of their four channels so that they
-// hit 32 banks.  Bound by issue and the latencies of its loads and barriers (70 % of the issue slots, integer pipe 50 %;
-// the updates alone would take 12 us): one 256-token Llama-7B chunk in 28 us, 36 with a condition at every load, 62 with a load
-// per symbol.  Otherwise
-// (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
+// calculate_cdf on int8 symbols: grid (nslab, nrows).  VEC: adjacent channels are adjacent bytes at 4-byte boundaries, and a lane
+// counts four channels of every eighth token, with one load for four symbols and 32 tokens in flight.  Channel 4 l + j of the
+// slab has column 32 j + l then (see entry_of), so that a warp's lanes are in 32 banks whatever they count.  Bound by issue and the
+// latencies of its loads and barriers: one 256-token Llama-7B chunk in 23.5 us (26 with sixteen tokens in flight, 30 with batches of
+// eight behind those of 32); 29.9 with eight in flight, the channels side by side, bytes picked in another order by each group of
+// lanes, and the counts summed before they were scaled; 36 with a condition at every load, 62 with a load per symbol.  The updates alone would take 12 us.  Otherwise (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
 template <bool VEC>
 __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t *__restrict__ sym, int64_t s0,
                                                                    int64_t s1, int64_t s2, int ntokens,
@@ -349,18 +359,11 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
     __syncthreads();
     const uint32_t top = static_cast<uint32_t>(max_bins);
     if (VEC) {
-        constexpr int kStep = kQuantThreads / 32, kAhead = 8;
+        constexpr int kStep = kQuantThreads / 32, kAhead = 32;
         const int q = tid & 31, c = c0 + 4 * q;
-        uint32_t place[4], pick[4];
+        uint32_t col[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t e = static_cast<uint32_t>(k + (q >> 3)) & 3u;
-            place[k] = smem_addr(hist + 4 * q + e);
-            pick[k] = 0x4440u + e;
-        }
-        const auto count = [&](uint32_t w, int k) {
-            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(__byte_perm(w, 0u, pick[k]) * kRowBytes + place[k]) : "memory");
-        };
+        for (int k = 0; k < 4; ++k) col[k] = smem_addr(hist + k * 32 * lp + q);
         if (c < nchannels) {
             const int8_t *p = sym + row * s0 + c + (tid >> 5) * s1;
             const int64_t step = kStep * s1;
@@ -383,13 +386,13 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
 #pragma unroll
                 for (int j = 0; j < kAhead; ++j)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) count(w[j], k);
+                    for (int k = 0; k < 4; ++k) count_symbol(entry_of(col[k], w[j], k));
             }
             for (; t0 < ntokens; t0 += kStep) {
                 const uint32_t w = __vminu4(__ldg(reinterpret_cast<const uint32_t *>(p)), most);
                 p += step;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) count(w, k);
+                for (int k = 0; k < 4; ++k) count_symbol(entry_of(col[k], w, k));
             }
         }
     } else {
@@ -398,12 +401,14 @@ __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t 
             const int8_t *p = sym + row * s0 + c * s2;
             for (int t = tid / kGroup; t < ntokens; t += kQuantThreads / kGroup) {
                 const uint32_t s = static_cast<uint8_t>(__ldg(p + t * s1));
-                atomicAdd(&hist[min(s, top) * kGroup + cl], 1u);
+                atomicAdd(&hist[((cl >> 5) * lp + min(s, top)) * 32 + (cl & 31)], 1u);
             }
         }
     }
     __syncthreads();
-    if (tid < kGroup && c0 + tid < nchannels) counts_to_table(hist, max_bins, tid, out16);
+    const int cl = VEC ? 4 * (tid & 31) + (tid >> 5) : tid;  // the channel of column tid
+    if (tid < kGroup && c0 + cl < nchannels)
+        counts_to_table<32>(hist + (tid >> 5) * 32 * lp + (tid & 31), max_bins, ntokens, out16 + cl * lp);
     __syncthreads();
     store_tables(out16, cdf_out, row, c0, nchannels, lp, tid, kQuantThreads);
 }

@@ -255,17 +255,6 @@ __device__ __forceinline__ void copy_tables(const uint16_t *stage, uint16_t *dst
     }
 }
 
-// Shared-memory columns of a warp's 32 channels: entry m of lane l at word 32 m + l.  With rows of 128 bytes the
-// address of the entry that byte k of a word of symbols names is one dot product: the byte times 128, plus
-// the column.
-constexpr int kWarpRow = 128;
-__device__ __forceinline__ uint32_t entry_of(uint32_t col, uint32_t w, int k) {
-    return __dp4a(w, static_cast<uint32_t>(kWarpRow) << (8 * k), col);
-}
-__device__ __forceinline__ void count_symbol(uint32_t addr) {
-    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
-}
-
 // Tables of a chunk of more than one sub-chunk (the coder's blocks build those of a single one themselves):
 // block (slab, row); a lane counts four adjacent channels, a warp every kTableWarps-th word of them, four words a batch without a
 // condition inside.  Channel 4 l + j of the slab has column 32 j + l, so that the lanes of a warp are in 32 banks whichever of
