@@ -51,8 +51,8 @@ HBM_FALLBACK_GBS = 6650.0
 # file and have to be re-captured when the kernel changes.  They come from a 2,048-token launch; DRAM
 # bytes (read + write) grow in proportion to the tokens of a launch.
 NCU_CAPTURE = {
-    (32, 32, 128): {"traffic_bytes_per_token": 1258.0e6 / 2048, "issue_active_pct": 83.9, "alu_pipe_pct": 56.1,
-                    "warp_instr_per_32_symbols": 58.9,
+    (32, 32, 128): {"traffic_bytes_per_token": 1265.9e6 / 2048, "issue_active_pct": 82.1, "alu_pipe_pct": 54.5,
+                    "warp_instr_per_32_symbols": 52.4,
                     "source": "ncu on a 2,048-token decode (dram__bytes_read.sum + dram__bytes_write.sum, "
                               "smsp__inst_executed.sum, issue and pipe activity), B200, kernel "
                               "decode_dequant_multi_kernel<2,0>"},
