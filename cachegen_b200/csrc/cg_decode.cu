@@ -793,12 +793,14 @@ __device__ __forceinline__ int clamped_length(int v, int longest, bool *bad) {
 template <int BLOCKS, int AHEAD>  // AHEAD: groups a warp has in flight
 __global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(kOffsetThreads)
 group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nchannels, int nslab, int32_t *status,
-                     const StreamSizes sizes) {
+                     const StreamSizes sizes, bool behind_another) {
     extern __shared__ int sums[];  // the groups of this block
     __shared__ int64_t warp_sums[kOffsetThreads / 32];
     __shared__ int64_t block_total;
     __shared__ uint32_t block_bad;
-    wait_for_launch_before();
+    // Behind another batch of the same call, whose blocks have waited for what is in front of both by the time these start, they run
+    // beside those; they only must not end first.
+    if (!behind_another) wait_for_launch_before();
     let_next_launch_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) block_bad = 0u;
@@ -902,10 +904,11 @@ group_offsets_kernel(const __grid_constant__ OffsetJobs jobs, int nrows, int nch
         *reinterpret_cast<volatile int64_t *>(sizes.tail + 3) = 1;
     }
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");  // the totals have been read
+    if (behind_another) wait_for_launch_before();
 }
 
 static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int nchannels, int32_t *status, cudaStream_t st,
-                          const StreamSizes &sizes = StreamSizes{nullptr, nullptr, 1 << 20}) {
+                          const StreamSizes &sizes = StreamSizes{nullptr, nullptr, 1 << 20}, bool behind_another = false) {
     OffsetJobs o;
     for (int j = 0; j < njobs; ++j) {
         o.lengths[j] = jobs[j].lengths;
@@ -917,7 +920,7 @@ static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int n
     const int64_t groups = static_cast<int64_t>(nrows) * nslab;
     const auto run = [&](auto kernel, int blocks) {
         return launch(kernel, dim3(static_cast<unsigned>(njobs * blocks)), kOffsetThreads, static_cast<size_t>((groups + blocks - 1) / blocks) * sizeof(int),
-                      true, st, o, nrows, nchannels, nslab, status, sizes);
+                      true, st, o, nrows, nchannels, nslab, status, sizes, behind_another);
     };
     // Sixteen blocks where a warp of eight would take more than eight groups, in more than two rounds of loads.  20 tokens, us a
     // call with eight and with sixteen: 640 groups 12.8 and 13.1, 768 12.9 and 12.9, 1,280 16.9 and 15.8, 2,048 25.4 and 23.4.
@@ -1146,7 +1149,7 @@ extern "C" int cg_decode_kv(const cg_decode_job *jobs_host, int njobs, int nlaye
         const int n = njobs - b < CG_MAX_DECODE_JOBS ? njobs - b : CG_MAX_DECODE_JOBS;
         int rc;
         if (fused_offsets) {
-            rc = launch_offsets(jobs_host + b, n, nrows, nchannels, status, st);
+            rc = launch_offsets(jobs_host + b, n, nrows, nchannels, status, st, StreamSizes{nullptr, nullptr, 1 << 20}, b > 0);
         } else {
             rc = CG_OK;
             for (int j = b; j < b + n && rc == CG_OK; ++j)

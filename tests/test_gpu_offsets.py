@@ -44,3 +44,28 @@ def test_offsets_follow_what_wrote_the_lengths(heads, layers):
         got = de.decode(eo)
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     de.check_status()
+
+
+def test_offsets_of_several_batches_beside_each_other():
+    """130 jobs are four batches, whose offsets are made at the same time: right behind a kernel that still writes the lengths, and again
+    and again into the same buffer, which the decode in front may still read."""
+    from cachegen_b200.config import LMCacheEngineConfig, LMCacheEngineMetadata
+    from cachegen_b200.serde import CacheGenConfig, CacheGenDeserializer, CacheGenSerializer
+    from cachegen_b200.synth import generate_kv
+    config = CacheGenConfig.from_model_name("Yukang/LongAlpaca-70B-16k").layer_slice(0, 10)
+    engine, meta = LMCacheEngineConfig.from_defaults(chunk_size=256), LMCacheEngineMetadata("m", 1, 0, "vllm")
+    ser, de = (CacheGenSerializer(engine, meta, config, table_max_bins=32), CacheGenDeserializer(engine, meta, config, out_dtype=torch.float16))
+    chunks = [ser.encode(generate_kv(10, 4, 128, 20 + i, seed=i, device="cuda", dtype=torch.float16)) for i in range(3)]
+    want = [de.decode(c).clone() for c in chunks]
+    lengths = [c.data_chunks[0].bytestream_lengths.clone() for c in chunks]
+    order = [i % 3 for i in range(130)]
+    for turn in range(6):
+        torch.cuda._sleep(200_000)
+        for c, n in zip(chunks, lengths):
+            c.data_chunks[0].bytestream_lengths.zero_()
+        for c, n in zip(chunks, lengths):
+            torch.add(n, 0, out=c.data_chunks[0].bytestream_lengths)
+        order = order[turn:] + order[:turn]
+        got = de.decode_many([chunks[i] for i in order])
+        assert torch.equal(got.view(torch.int16), torch.cat([want[i] for i in order], 2).view(torch.int16)), turn
+    de.check_status()
