@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         stage_table_column<true>(tab, p.cdf + g * p.lp, p.lp, rows, tid);
         stage_table_column<true>(tab, p.cdf + (g + 1) * p.lp, p.lp, rows, tid + kThreads);
     }
+    __syncwarp();  // lanes behind the last channel read the last active lane's columns, and a small table meets no block barrier below
     // One search step less where the upper half of the table holds next to nothing, in every channel of the block: the rows of
     // half the bins in a table made for all rows (52 of 64 of a Llama-7B chunk), whose symbols there have one share of 2^16
     // each.  Such a symbol takes the exact search.  175 -> 168 us under counters.

@@ -34,3 +34,14 @@ def test_symbols_of_an_overlapped_launch_are_not_read_as_constant_data():
     # the columns of ready tables are read with __ldg: the kernel that writes them has to have ended
     assert re.search(r"early = alone && z\.nsub == 1;", text)
     assert re.search(r"launch\(packed_tables_kernel, [^;]*, false, st, table_jobs", text)
+
+
+def test_borrowed_columns_are_read_behind_a_barrier():
+    """Lanes behind the last channel decode from columns that the last active lane of their warp has staged.  A barrier that every
+    lane meets whatever the table's size stands between the two, in each kernel that lends columns."""
+    text = open(os.path.join(ROOT, "cachegen_b200", "csrc", "cg_decode.cu")).read()
+    kernels = [k for k in re.split(r"(?=__global__)", text[:text.index("// ---- launch helpers")]) if "borrow_stream(start[i]" in k]
+    assert len(kernels) == 2
+    for k in kernels:
+        between = k[k.rindex("stage_table_column"):k.index("borrow_stream(start[i]")]
+        assert re.search(r"^    __sync(warp|threads)\(\);", between, re.M)  # a statement of the kernel's body itself, in no branch
