@@ -37,6 +37,24 @@ namespace cg {
 constexpr int kGroupChannels = 128;            // streams (threads) per coder block
 constexpr int kTableRowBytes = kGroupChannels * 4;  // bytes between table entries m and m+1 of a stream
 
+// ---- grids of the decoders --------------------------------------------------------------------------------
+constexpr int kMultiBlocksPerSM = 12;  // of the kernels with two channels a thread, at 33-entry tables
+
+// Blocks to have on an SM at a time where a grid of `chunks` chunks, the first of `ntokens` tokens, would leave a short second wave;
+// 0: as many as fit.  Twelve blocks an SM, and then two to four more on each, whose serial chains take most of a wave's time
+// with next to nothing beside them: eight or ten at first, so that the others get company.  256 tokens with twelve and so, 7B
+// settings: 32 layers x 32 heads (14 blocks an SM) 159.5 and 152.3 us, x 35 (16) 170.4 and 159.7, nine chunks of 32 x 4 (16) 169.7 and
+// 163.5; 70B settings: 80 x 14 (16) 174.5 and 162.3, 40 x 28 (16) 164.6 and 165.2.
+// Not where it would hold blocks back for longer than it saves: thirteen an SM (40 x 24 151.6 and 153.0), fourteen of several
+// chunks, whose blocks come in no order of their work (4 of 32 x 8, the last of 5 tokens, 124.4 and 141.7), short tables (17
+// entries, 40 x 25 134.9 and 138.1, nine chunks of level 1 at 64 tokens 46.1 and 47.1), few tokens (16 of 32 x 32 at 32 bins 20.7 and
+// 21.4) and delta coding (9 of 32 x 4 192.8 and 200.9).
+CG_HD int evened_blocks(int64_t blocks, int64_t sms, int levels, int chunks, int ntokens) {
+    const int64_t more = (blocks + sms - 1) / sms - kMultiBlocksPerSM;
+    if (levels != 5 || ntokens < 64 || more > 4) return 0;
+    return more > 2 ? 10 : more == 2 && chunks == 1 ? 8 : 0;
+}
+
 // ---- intrinsics with host stand-ins -----------------------------------------------------------------
 CG_HD int cg_clz(uint32_t x) {
 #if defined(__CUDA_ARCH__)

@@ -163,7 +163,6 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
 // every symbol), of which the last 272 of 2,048 blocks, which find no room beside the first, take a third.
 // Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
 // more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
-constexpr int kMultiBlocksPerSM = 12;
 template <int LEVELS, int MODE>
 __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_pair_kernel(const SymDecodeParams p) {
     extern __shared__ uint32_t tab[];
@@ -684,23 +683,16 @@ static size_t table_bytes(int lp, int levels) {
 }
 static_assert((CG_MAX_LP + 1) * kRowBytes + 4 * (kSubTokens + 2 * CG_MAX_LP) + 64 <= kSmemByItself, "a decoder block's shared memory");
 
-// Shared memory to ask for so that a grid leaves no short second wave.  Twelve blocks an SM, and then one to four more on each, whose
-// serial chains take most of a wave's time with next to nothing beside them: fewer at first, so that the others get company.
-// us a call of 256 tokens of 32 layers with twelve and with so many (blocks a multiprocessor): 1,792 blocks (13) 145.4 and 146.9 (8),
-// 1,920 (13) 154.3 and 148.2, 2,048 (14) 166 and 152.7, 2,112 (15) 161.1 and 159.7 (10), 2,176 (15) 170.2 and 160.6,
-// 2,240 (16) 171.2 and 160.5, 2,368 (16) 173.8 and 172.7; 2,560 (18) 181 and 183.5 with ten.  The extension module's decode of 2,048
-// blocks, whose path takes 336 us, 8 us less.
+// Shared memory to ask for so that a grid has as many blocks an SM as evened_blocks says.
 template <class Kernel>
-static size_t evened_smem(Kernel kernel, int64_t blocks, size_t dynamic) {
+static size_t evened_smem(Kernel kernel, int64_t blocks, int levels, int chunks, int ntokens, size_t dynamic) {
     constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024;  // bytes of an SM, of each block
-    const int64_t share = (blocks + sm_count() - 1) / sm_count();
-    if (share <= kMultiBlocksPerSM || share > kMultiBlocksPerSM + 4) return dynamic;
+    const int resident = evened_blocks(blocks, sm_count(), levels, chunks, ntokens);
     cudaFuncAttributes at;
-    if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return dynamic;
+    if (!resident || cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return dynamic;
     const int64_t fixed = static_cast<int64_t>(at.sharedSizeBytes) + kReserved;
-    if ((static_cast<int64_t>(dynamic) + fixed) * kMultiBlocksPerSM > kSmemPerSM) return dynamic;  // long tables: fewer as it is
-    const int64_t resident = share <= kMultiBlocksPerSM + 2 ? 8 : 10;
-    return static_cast<size_t>(kSmemPerSM / (resident + 1) - fixed + 256);  // the least that keeps one more out
+    const size_t least = static_cast<size_t>(kSmemPerSM / (resident + 1) - fixed + 256);  // that keeps one more out
+    return least > dynamic ? least : dynamic;
 }
 
 // Instantiated search depths: 3..6, whatever the table length.
@@ -712,7 +704,7 @@ static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) 
     const bool pairs = p.o2 == 1 && ((p.o0 | p.o1 | p.nchannels) & 1) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 1) == 0;
 #define CG_LAUNCH_SYM(L)                                                                                      \
     return pairs ? launch(decode_symbols_pair_kernel<L, MODE>, grid, kGroup / 2,                               \
-                          evened_smem(decode_symbols_pair_kernel<L, MODE>, blocks, table_bytes(p.lp, L)), MODE == 2, st, p) \
+                          evened_smem(decode_symbols_pair_kernel<L, MODE>, blocks, L, 1, p.ntokens, table_bytes(p.lp, L)), MODE == 2, st, p) \
                  : launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
     if (need <= 3) CG_LAUNCH_SYM(3);
     if (need == 4) CG_LAUNCH_SYM(4);
@@ -758,7 +750,7 @@ static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool ear
     if (!DELTA && blocks <= static_cast<int64_t>(kQuickBlocksPerSM) * sm_count())
         return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA, !DELTA>, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
     const auto kernel = decode_dequant_multi_kernel<NS, OUT_DT, DELTA, false>;
-    return launch(kernel, grid, kGroup / NS, evened_smem(kernel, blocks, smem), early, st, p, scale_dt, full);
+    return launch(kernel, grid, kGroup / NS, DELTA ? smem : evened_smem(kernel, blocks, full, p.njobs, p.jobs[0].ntokens, smem), early, st, p, scale_dt, full);
 }
 
 // ---- group offsets ------------------------------------------------------------------------------------------

@@ -65,3 +65,22 @@ def test_symbols_come_back_at_either_side_of_a_wave(rows, channels):
     out = torch.empty((rows, 70, channels), dtype=torch.uint8, device="cuda")
     torchac_cuda.decode_by_lengths(cdf, streams, lengths, out)
     assert torch.equal(out.view(torch.int8), sym)
+
+
+@pytest.mark.parametrize("heads, bins, tokens, delta", [(31, 32, 64, None), (32, 32, 70, None), (34, 32, 64, None), (37, 32, 65, None),
+                                                        (32, 16, 64, None), (32, 8, 64, None), (32, 62, 64, None), (32, 32, 63, None), (34, 32, 64, 16)])
+def test_grids_with_blocks_held_back(heads, bins, tokens, delta):
+    """One chunk of 14 to 16 blocks an SM, some of them held back, and the same streams twice in a grid that holds none back; tables of
+    other lengths, fewer tokens and delta coding, where none are."""
+    from cachegen_b200.serde import cachegen_decoder as M
+    from cachegen_b200.serde import cachegen_encoder as E
+    from cachegen_b200.serde.cachegen_basics import DeltaCoding
+    kv = torch.randn((32, 2, tokens, heads, 128), generator=torch.Generator("cuda").manual_seed(bins), device="cuda").half()
+    b, delta = torch.full((32,), float(bins)).cuda(), delta and DeltaCoding(delta)
+    eo = E.encode_function(kv, None, b, b, tokens, delta=delta)
+    one = M.decode_many([eo], torch.cat((b, b)), "vllm", torch.float16, workspace={}, delta=delta)
+    two = M.decode_many([eo] * 2, torch.cat((b, b)), "vllm", torch.float16, workspace={}, delta=delta)
+    assert torch.equal(two.view(torch.int16), one.repeat(1, 1, 2, 1, 1).view(torch.int16))
+    if delta is None:
+        x = kv.float()
+        assert ((one.float() - x).abs() <= x.abs().amax((3, 4), keepdim=True) * (0.51 / (bins // 2 - 1))).all()
