@@ -1,5 +1,6 @@
 """Builds libcachegen_b200.so in-tree with nvcc for sm_100a (no torch headers: a few seconds per file), and _calls.so, the
-host side of the calls on torch's tensors, with the host compiler.
+host side of the calls on torch's tensors, with the host compiler.  The library needs neither torch nor Python's headers;
+where those are not there it is built without _calls.so.
 
     python -m cachegen_b200.build [--force] [--verbose]
 """
@@ -55,10 +56,17 @@ def build(force=False, verbose=False, extra_flags=(), out=None):
     """Compiles the library and returns its path.  `out` builds a second copy elsewhere (with
     `extra_flags`, e.g. -D switches) without touching the in-tree one; CACHEGEN_B200_LIB selects it."""
     target = out or LIB
+    if out or force or needs_build():
+        build_library(target, out, verbose, extra_flags)
     if not out and (force or calls_need_build()):
-        build_calls()
-    if not out and not force and not needs_build():
-        return target
+        try:
+            build_calls()
+        except (ImportError, OSError, RuntimeError) as e:
+            print(f"{CALLS} was not built; {LIB} does not need it, the Python classes do: {e}", file=sys.stderr)
+    return target
+
+
+def build_library(target, out, verbose, extra_flags):
     flags = NVCC_FLAGS + list(extra_flags)
     if verbose:
         flags = flags + ["-Xptxas", "-v"]
@@ -80,7 +88,6 @@ def build(force=False, verbose=False, extra_flags=(), out=None):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    return target
 
 
 if __name__ == "__main__":
