@@ -1,6 +1,7 @@
 """ctypes binding of libcachegen_b200.so (declarations follow include/cachegen_b200.h)."""
 import ctypes
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # CACHEGEN_B200_LIB selects another build of the library (same ABI), e.g. one kept outside the package
@@ -152,20 +153,31 @@ def lib():
 _calls = None
 
 
-def calls():
+def native_calls():
     """The calls' host side in native code (csrc/cg_calls.cpp), which works through the library that lib() has loaded."""
+    L = lib()
+    import torch  # noqa: F401  (its libraries have to be there first)
+    try:
+        from . import _calls as module
+    except ImportError as e:
+        raise CacheGenLibraryMissing(f"{os.path.join(_HERE, '_calls.so')} is missing or was built for another torch: build it with "
+                                     f"`python -m cachegen_b200.build --force` ({e})") from e
+    module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value
+                 for n in ("cg_decode_kv", "cg_encode_kv", "cg_encode_kv_workspace", "cg_encode_kv_wait", "cg_encode_kv_gather")})
+    return module
+
+
+def calls():
+    """native_calls(), or the same entries in Python (_plain_calls.py) where that module cannot be had."""
     global _calls
     if _calls is None:
-        L = lib()
-        import torch  # noqa: F401  (its libraries have to be there first)
+        lib()
         try:
-            from . import _calls as module
-        except ImportError as e:
-            raise CacheGenLibraryMissing(f"{os.path.join(_HERE, '_calls.so')} is missing or was built for another torch: build it with "
-                                         f"`python -m cachegen_b200.build --force` ({e})") from e
-        module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value
-                     for n in ("cg_decode_kv", "cg_encode_kv", "cg_encode_kv_workspace", "cg_encode_kv_wait", "cg_encode_kv_gather")})
-        _calls = module
+            _calls = native_calls()
+        except CacheGenLibraryMissing as e:
+            from . import _plain_calls
+            warnings.warn(f"calls spend more time on the host: {e}", RuntimeWarning, stacklevel=2)
+            _calls = _plain_calls
     return _calls
 
 

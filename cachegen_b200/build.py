@@ -62,7 +62,7 @@ def build(force=False, verbose=False, extra_flags=(), out=None):
         try:
             build_calls()
         except (ImportError, OSError, RuntimeError) as e:
-            print(f"{CALLS} was not built; {LIB} does not need it, the Python classes do: {e}", file=sys.stderr)
+            print(f"{CALLS} was not built; the library does not need it, calls of the Python classes take longer: {e}", file=sys.stderr)
     return target
 
 
