@@ -157,10 +157,13 @@ def native_calls():
     """The calls' host side in native code (csrc/cg_calls.cpp), which works through the library that lib() has loaded."""
     L = lib()
     import torch  # noqa: F401  (its libraries have to be there first)
+    from . import build
     try:
         from . import _calls as module
+        if getattr(module, "built_for", "") != build.calls_built_for():
+            raise ImportError(f"built for {getattr(module, 'built_for', 'an unknown torch')}, this is {build.calls_built_for()}")
     except ImportError as e:
-        raise CacheGenLibraryMissing(f"{os.path.join(_HERE, '_calls.so')} is missing or was built for another torch: build it with "
+        raise CacheGenLibraryMissing(f"{build.CALLS} is missing or was built for another torch: build it with "
                                      f"`python -m cachegen_b200.build --force` ({e})") from e
     module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value
                  for n in ("cg_decode_kv", "cg_encode_kv", "cg_encode_kv_workspace", "cg_encode_kv_wait", "cg_encode_kv_gather")})

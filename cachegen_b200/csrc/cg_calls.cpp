@@ -480,5 +480,10 @@ PyMODINIT_FUNC PyInit__calls() {
     s_header = PyUnicode_InternFromString("header");
     s_sub_off = PyUnicode_InternFromString("sub_off");
     for (int k = 0; k < kHeaderFields; ++k) s_header_fields[k] = PyUnicode_InternFromString(kHeaderNames[k]);
-    return PyModule_Create(&module);
+    PyObject *const m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", CG_BUILT_FOR)) {  // see build.py
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
 }

@@ -57,3 +57,32 @@ def test_a_library_that_does_not_compile_is_an_error(builder, monkeypatch):
     monkeypatch.setattr(builder.subprocess, "run", lambda cmd, **kw: types.SimpleNamespace(returncode=1, stdout="", stderr="no"))
     with pytest.raises(RuntimeError, match="nvcc failed"):
         builder.build(force=True)
+
+
+def test_the_host_module_is_built_again_for_another_torch_and_replaced_whole(builder, monkeypatch):
+    import torch
+    builder.build(force=True)
+    made = [cmd for cmd in builder.commands if builder.CALLS_SOURCE in cmd]
+    assert len(made) == 1 and made[0][made[0].index("-o") + 1] != builder.CALLS  # written beside it, then put in its place
+    assert os.listdir(os.path.dirname(builder.CALLS)).count(os.path.basename(builder.CALLS)) == 1
+    assert not [n for n in os.listdir(os.path.dirname(builder.CALLS)) if n.startswith("_calls.so.")]
+    with open(builder.CALLS, "ab") as f:
+        f.write(builder.calls_built_for().encode())
+    assert not builder.calls_need_build()
+    monkeypatch.setattr(torch, "__version__", "9.9")
+    assert builder.calls_need_build()
+
+
+def test_a_compile_that_fails_leaves_the_host_module_as_it_is(builder, monkeypatch):
+    builder.build_calls()
+
+    def fails(cmd, **kw):
+        with open(cmd[cmd.index("-o") + 1], "w") as f:
+            f.write("half")
+        return types.SimpleNamespace(returncode=1, stdout="", stderr="no")
+
+    monkeypatch.setattr(builder.subprocess, "run", fails)
+    with pytest.raises(RuntimeError, match="failed on cg_calls"):
+        builder.build_calls()
+    assert open(builder.CALLS).read() == "built" and os.listdir(os.path.dirname(builder.CALLS)).count("_calls.so") == 1
+    assert not [n for n in os.listdir(os.path.dirname(builder.CALLS)) if n.startswith("_calls.so.")]

@@ -25,6 +25,15 @@ def test_the_entries_are_there(unbuilt):
     assert unbuilt.calls() is plain
 
 
+def test_a_module_of_another_torch_is_not_used(monkeypatch):
+    from cachegen_b200 import _lib, build
+    build.build()
+    _lib.native_calls()
+    monkeypatch.setattr(torch, "__version__", "9.9")
+    with pytest.raises(_lib.CacheGenLibraryMissing, match="this is torch 9.9"):
+        _lib.native_calls()
+
+
 def test_a_missing_library_is_still_an_error(unbuilt, monkeypatch):
     monkeypatch.setattr(unbuilt, "_lib", None)
     monkeypatch.setattr(unbuilt, "LIB_PATH", "/nowhere/libcachegen_b200.so")
