@@ -13,6 +13,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -33,7 +34,7 @@ decltype(&cg_encode_kv_gather) encode_kv_gather;
 
 // attribute names
 PyObject *s_cdf, *s_max_tensors_key, *s_max_tensors_value, *s_data_chunks, *s_num_heads, *s_head_size, *s_bytestream,
-    *s_bytestream_lengths, *s_ntokens, *s_blob, *s_header, *s_sub_off, *s_group_off;
+    *s_bytestream_lengths, *s_ntokens, *s_blob, *s_header, *s_sub_off, *s_group_off, *s_captured;
 const char *const kHeaderNames[] = {"L", "H", "D", "T", "lp", "nsub", "scale_code", "table_kind", "length_kind", "bins_checksum",
                                     "off_scales", "off_tables", "off_lengths", "off_payload"};
 enum HeaderField { kL, kH, kD, kT, kLp, kNsub, kScaleCode, kTableKind, kLengthKind, kChecksum, kOffScales, kOffTables, kOffLengths, kOffPayload, kHeaderFields };
@@ -234,6 +235,18 @@ bool add_container(PyObject *chunk, at::Device dev, const FlatBins &bins, Shape 
     return true;
 }
 
+// Adds a tensor to the set that a workspace holds for graphs (see _keep_for_graph in cachegen_decoder.py).
+bool keep_for_graph(PyObject *workspace, PyObject *tensor) {
+    if (tensor == Py_None) return true;
+    PyObject *held = PyDict_GetItem(workspace, s_captured);
+    if (!held) {
+        const Ref made(PySet_New(nullptr));
+        if (!made.p || PyDict_SetItem(workspace, s_captured, made.p)) return false;
+        held = made.p;
+    }
+    return PySet_Add(held, tensor) == 0;
+}
+
 // decode(chunks, chunk type, piece type or None, bins, vllm, bf16 out, out or None, workspace, status word, of containers
 //        (kind of tables, checksum, counts_bytes, sparse_bytes, row offsets or None))
 // -> the KV blob, or the library's error code, or None: not the usual case, nothing has been done.
@@ -284,14 +297,20 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
             out.is_conj() || out.is_neg())
             Py_RETURN_NONE;
     }
-    // the group offsets' buffer is kept in the workspace between calls
-    PyObject *const kept = PyDict_GetItem(a[7], s_group_off);
+    // The group offsets' buffer is kept in the workspace between calls.  A graph writes to its buffer at every replay: it gets one of
+    // its own memory, and what else it uses of the workspace's stays there when other calls replace it.
     at::Tensor goff;
-    if (plain(kept)) goff = THPVariable_Unpack(kept);
-    if (!usable(goff, at::kLong, dev) || goff.numel() < njobs * groups) {
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
         goff = make({njobs * groups}, at::TensorOptions().dtype(at::kLong).device(dev));
-        const Ref made(THPVariable_Wrap(goff));
-        if (PyDict_SetItem(a[7], s_group_off, made.p)) throw python_error();
+        if (!keep_for_graph(a[7], a[3]) || !keep_for_graph(a[7], a[8]) || (containers && !keep_for_graph(a[7], PyTuple_GET_ITEM(a[9], 4)))) throw python_error();
+    } else {
+        PyObject *const kept = PyDict_GetItem(a[7], s_group_off);
+        if (plain(kept)) goff = THPVariable_Unpack(kept);
+        if (!usable(goff, at::kLong, dev) || goff.numel() < njobs * groups) {
+            goff = make({njobs * groups}, at::TensorOptions().dtype(at::kLong).device(dev));
+            const Ref made(THPVariable_Wrap(goff));
+            if (PyDict_SetItem(a[7], s_group_off, made.p)) throw python_error();
+        }
     }
     const int64_t o_token = out.stride(vllm ? 2 : 3), o_head = out.stride(vllm ? 3 : 2);
     uint8_t *at_out = static_cast<uint8_t *>(out.data_ptr());
@@ -476,6 +495,7 @@ PyMODINIT_FUNC PyInit__calls() {
     s_bytestream_lengths = PyUnicode_InternFromString("bytestream_lengths");
     s_ntokens = PyUnicode_InternFromString("ntokens");
     s_group_off = PyUnicode_InternFromString("group_off");
+    s_captured = PyUnicode_InternFromString("captured");
     s_blob = PyUnicode_InternFromString("blob");
     s_header = PyUnicode_InternFromString("header");
     s_sub_off = PyUnicode_InternFromString("sub_off");

@@ -236,12 +236,22 @@ def _device_of(eo):
     return eo.blob.device if isinstance(eo, flat_format.FlatChunk) else eo.cdf.device
 
 
+def _keep_for_graph(ws: dict, *tensors) -> bool:
+    """Whether the current stream is being captured.  If so the launches of this call run again at every replay, whatever other calls do
+    to the workspace: what they use of it is held there for good."""
+    if not torch.cuda.is_current_stream_capturing():
+        return False
+    ws.setdefault("captured", set()).update(tensors)
+    return True
+
+
 def _status_word(ws: dict, dev) -> torch.Tensor:
     status = ws.get("status")
     if status is None or status.device != dev:
         with torch.inference_mode(False):  # kept, and written to by later calls in whatever mode those run
             status = torch.zeros(1, dtype=torch.int32, device=dev)
-        ws["status"] = status
+        if not _keep_for_graph(ws, status):  # (one that a graph makes is zero only once that has run)
+            ws["status"] = status
     return status
 
 
@@ -306,12 +316,14 @@ class DecodePlan:
         nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
         ngroups = NL * nslab
         njobs_total = sum(len(v.subs) for v in views)
-        goff = ws.get("group_off")
-        if goff is None or goff.numel() < njobs_total * ngroups or goff.device != dev:
-            goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)
-            ws["group_off"] = goff
         status = _status_word(ws, dev)
         row_offs = {kind: _row_offsets(ws, kind, host_bins, C, dev) for kind in _ROW_OFFSETS if any(v.table_kind == kind for v in views)}
+        goff = ws.get("group_off")
+        if _keep_for_graph(ws, bins, status, *row_offs.values()):
+            goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)  # of the graph's own memory
+        elif goff is None or goff.numel() < njobs_total * ngroups or goff.device != dev:
+            goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)
+            ws["group_off"] = goff
 
         esz = out.element_size()
         self.keep = list(row_offs.values())  # tensors that must outlive the launches
@@ -417,7 +429,8 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
     The chunks' tensors may live on the GPU or in (pinned) host memory; host tensors are copied to the
     GPU on the current stream first.  bins: float32 [2L] on the GPU (key bins then value bins).
     `out`, when given, must have the result's shape and dtype with a unit innermost stride (any other
-    strides).  `workspace` caches the small offset / status buffers between calls.  `host_bins`: the values of `bins`,
+    strides).  `workspace` caches the small offset / status buffers between calls; a graph that captures a decode needs it, or
+    the deserializer that has it, for as long as it is replayed.  `host_bins`: the values of `bins`,
     when the caller knows them; read from the tensor otherwise, if the chunks ask for them.
     """
     if delta is None and workspace is not None:
@@ -527,6 +540,7 @@ def _stage_flat(part: list, ws: dict, dev) -> list:
         with torch.inference_mode(False):
             arena = torch.empty(need, dtype=torch.uint8, device=dev)
         ws["arena"] = arena
+    _keep_for_graph(ws, arena)
     staged = []
     for eo, a in zip(part, starts):
         dst = arena[a:a + eo.blob.numel()]
