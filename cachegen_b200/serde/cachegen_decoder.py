@@ -446,6 +446,8 @@ def _decode_usual(encoder_outputs, bins, fmt, out_dtype, out, workspace, host_bi
     None, and nothing has been done but for buffers that the workspace keeps, for any other chunks."""
     if not encoder_outputs or type(encoder_outputs) is not list or fmt not in ("vllm", "huggingface") or out_dtype not in _DTYPES or not bins.is_cuda:
         return None
+    if not _on_gpu(encoder_outputs[0]):  # asked first: the rest takes a tenth of a short chunk's call
+        return None
     kind, piece, flat = CacheGenGPUEncoderOutput, CacheGenGPUBytestream, None
     if type(encoder_outputs[0]) is flat_format.FlatChunk:
         header = encoder_outputs[0].header
