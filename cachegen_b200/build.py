@@ -14,7 +14,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libcachegen_b200.so")
 SOURCES = ["cg_api.cu", "cg_quant.cu", "cg_tables.cu", "cg_encode.cu", "cg_store.cu", "cg_decode.cu", "cg_host.cu"]
-HEADERS = [os.path.join(CSRC, "cg_common.cuh"), os.path.join(CSRC, "cg_coder.cuh"), os.path.join(CSRC, "cg_hostcopy.h"), os.path.join(PKG, "..", "include", "cachegen_b200.h")]
+HEADERS = [os.path.join(CSRC, "cg_common.cuh"), os.path.join(CSRC, "cg_coder.cuh"), os.path.join(CSRC, "cg_hostcopy.h"),
+           os.path.join(PKG, "..", "include", "cachegen_b200.h")]
 CALLS = os.path.join(PKG, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 CALLS_SOURCE = os.path.join(CSRC, "cg_calls.cpp")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -37,7 +37,9 @@ PyObject *s_cdf, *s_max_tensors_key, *s_max_tensors_value, *s_data_chunks, *s_nu
     *s_bytestream_lengths, *s_ntokens, *s_blob, *s_header, *s_sub_off, *s_group_off, *s_captured;
 const char *const kHeaderNames[] = {"L", "H", "D", "T", "lp", "nsub", "scale_code", "table_kind", "length_kind", "bins_checksum",
                                     "off_scales", "off_tables", "off_lengths", "off_payload"};
-enum HeaderField { kL, kH, kD, kT, kLp, kNsub, kScaleCode, kTableKind, kLengthKind, kChecksum, kOffScales, kOffTables, kOffLengths, kOffPayload, kHeaderFields };
+enum HeaderField {
+    kL, kH, kD, kT, kLp, kNsub, kScaleCode, kTableKind, kLengthKind, kChecksum, kOffScales, kOffTables, kOffLengths, kOffPayload, kHeaderFields
+};
 PyObject *s_header_fields[kHeaderFields];
 
 // A new reference that is given back.
@@ -64,8 +66,8 @@ bool plain(PyObject *o) { return o && THPVariable_CheckExact(o); }
 
 // A plain contiguous tensor of this type on this GPU: the only kind that is taken as it is.
 bool usable(const at::Tensor &t, at::ScalarType type, at::Device dev) {
-    return t.defined() && t.unsafeGetTensorImpl()->has_storage() && t.layout() == at::kStrided && t.scalar_type() == type && t.device() == dev && t.is_contiguous() &&
-           !t.is_conj() && !t.is_neg();
+    return t.defined() && t.unsafeGetTensorImpl()->has_storage() && t.layout() == at::kStrided && t.scalar_type() == type &&
+           t.device() == dev && t.is_contiguous() && !t.is_conj() && !t.is_neg();
 }
 
 bool small_int(PyObject *o, int64_t *v) {
@@ -115,7 +117,8 @@ bool merge(const Shape &s, Shape *all, bool first) {
 bool add_chunk(PyObject *eo, PyTypeObject *piece_type, at::Device dev, Shape *all, bool first, std::vector<cg_decode_job> *jobs,
                std::vector<at::Tensor> *held) {
     Shape s;
-    if (!attribute_int(eo, s_num_heads, &s.H) || !attribute_int(eo, s_head_size, &s.D) || s.H <= 0 || s.D <= 0 || s.H > 0xFFFFFF || s.D > 0xFFFFFF) return false;
+    if (!attribute_int(eo, s_num_heads, &s.H) || !attribute_int(eo, s_head_size, &s.D)) return false;
+    if (s.H <= 0 || s.D <= 0 || s.H > 0xFFFFFF || s.D > 0xFFFFFF) return false;
     const size_t at = held->size();
     if (!attribute_tensor(eo, s_cdf, held) || !attribute_tensor(eo, s_max_tensors_key, held) || !attribute_tensor(eo, s_max_tensors_value, held))
         return false;
@@ -194,7 +197,9 @@ bool add_container(PyObject *chunk, at::Device dev, const FlatBins &bins, Shape 
     if (f[kChecksum] && f[kChecksum] != bins.checksum) return false;
     const int64_t table_bytes = f[kOffLengths] - f[kOffTables];
     if (f[kTableKind] != bins.kind) return false;
-    const int64_t least = bins.kind == CG_TABLES_COUNTS ? bins.counts_bytes : bins.kind == CG_TABLES_SPARSE ? bins.sparse_bytes : 4 * s.L * s.H * s.D * s.lp;
+    const int64_t least = bins.kind == CG_TABLES_COUNTS   ? bins.counts_bytes
+                          : bins.kind == CG_TABLES_SPARSE ? bins.sparse_bytes
+                                                          : 4 * s.L * s.H * s.D * s.lp;
     if (bins.kind > CG_TABLES_SPARSE || table_bytes < least) return false;
     if (bins.kind != CG_TABLES_CDF) {
         if (!usable(bins.row_off, at::kLong, dev) || bins.row_off.numel() != 2 * s.L + 1) return false;
@@ -293,8 +298,8 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
         out = make(shape, at::TensorOptions().dtype(type).device(dev));
     } else {
         out = THPVariable_Unpack(a[6]);
-        if (!out.unsafeGetTensorImpl()->has_storage() || out.layout() != at::kStrided || out.scalar_type() != type || out.device() != dev || out.sizes() != at::IntArrayRef(shape) || out.stride(4) != 1 ||
-            out.is_conj() || out.is_neg())
+        if (!out.unsafeGetTensorImpl()->has_storage() || out.layout() != at::kStrided || out.scalar_type() != type || out.device() != dev ||
+            out.sizes() != at::IntArrayRef(shape) || out.stride(4) != 1 || out.is_conj() || out.is_neg())
             Py_RETURN_NONE;
     }
     // The group offsets' buffer is kept in the workspace between calls.  A graph writes to its buffer at every replay: it gets one of
@@ -302,7 +307,8 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     at::Tensor goff;
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
         goff = make({njobs * groups}, at::TensorOptions().dtype(at::kLong).device(dev));
-        if (!keep_for_graph(a[7], a[3]) || !keep_for_graph(a[7], a[8]) || (containers && !keep_for_graph(a[7], PyTuple_GET_ITEM(a[9], 4)))) throw python_error();
+        for (PyObject *used : {a[3], a[8], containers ? PyTuple_GET_ITEM(a[9], 4) : Py_None})
+            if (!keep_for_graph(a[7], used)) throw python_error();
     } else {
         PyObject *const kept = PyDict_GetItem(a[7], s_group_off);
         if (plain(kept)) goff = THPVariable_Unpack(kept);
@@ -325,8 +331,9 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     int rc;
     {
         const WithoutGil released;
-        rc = decode_kv(jobs.data(), static_cast<int>(njobs), static_cast<int>(s.L), static_cast<int>(s.H), static_cast<int>(s.D), static_cast<int>(s.lp),
-                       static_cast<const float *>(bins.data_ptr()), 0, nullptr, code(s.scale), code(type), out.stride(0), out.stride(1), o_token,
+        rc = decode_kv(jobs.data(), static_cast<int>(njobs), static_cast<int>(s.L), static_cast<int>(s.H), static_cast<int>(s.D),
+                       static_cast<int>(s.lp), static_cast<const float *>(bins.data_ptr()), 0,
+                       nullptr, code(s.scale), code(type), out.stride(0), out.stride(1), o_token,
                        o_head, static_cast<int32_t *>(status.data_ptr()), stream.stream());
     }
     if (rc) return PyLong_FromLong(rc);
@@ -404,7 +411,8 @@ PyObject *encode_start(PyObject *, PyObject *const *a, Py_ssize_t n) {
         rc = encode_kv(&job, stream);
     }
     const auto wrap = [](const at::Tensor &t) { return t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None); };
-    return Py_BuildValue("(iKNNNNNN)", rc, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)), wrap(scales), wrap(scales_k), wrap(scales_v), wrap(cdf), wrap(workspace), wrap(counts));
+    return Py_BuildValue("(iKNNNNNN)", rc, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)), wrap(scales),
+                         wrap(scales_k), wrap(scales_v), wrap(cdf), wrap(workspace), wrap(counts));
     END_HANDLE_TH_ERRORS
 }
 

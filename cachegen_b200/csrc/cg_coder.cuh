@@ -384,7 +384,8 @@ CG_HD int fast_levels_for(int nsym, int full_levels) {
 }
 
 // 128 + (floor(2^16 offset / span) + 1) / 2^16, or one 2^16th off where the quotient is within 2^-6 or so of a whole number:
-// a float from 128 on has sixteen bits behind the point, so the rounding of the last addition is the floor (see search_entry).  Anything when the span is the full 2^32 (span32 == 0).
+// a float from 128 on has sixteen bits behind the point, so the rounding of the last addition is the floor (see search_entry).
+// Anything when the span is the full 2^32 (span32 == 0).
 CG_HD float ratio_estimate(uint32_t offset, uint32_t span32) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -462,7 +463,8 @@ struct QuarterSearch {
     static CG_HD uint32_t run(Smem sm, uint32_t a, float ratio) {
         if (B == 0) return RatioSearch<0>::run(sm, a, ratio);
         constexpr uint32_t kStep = static_cast<uint32_t>(kTableRowBytes) << (B > 0 ? B - 1 : 0);
-        return QuarterSearch<B - 2>::run(sm, search_quarter<kStep>(a, ld_entry(sm, a + kStep), ld_entry(sm, a + 2 * kStep), ld_entry(sm, a + 3 * kStep), ratio), ratio);
+        const uint32_t e0 = ld_entry(sm, a + kStep), e1 = ld_entry(sm, a + 2 * kStep), e2 = ld_entry(sm, a + 3 * kStep);
+        return QuarterSearch<B - 2>::run(sm, search_quarter<kStep>(a, e0, e1, e2, ratio), ratio);
     }
 };
 template <>
@@ -483,7 +485,8 @@ struct QuarterSearch<-2> {
 // bounds, which the range update needs anyway.  The caller picks FL from what it knows about the symbols (a
 // row quantised to `bins` bins holds symbols 0 .. bins-2, so 2^FL >= bins is enough).  The result depends
 // on neither: a symbol that fails the check -- an estimate on the wrong side of an entry, a symbol >= 2^FL - 1, a symbol that
-// starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away and the whole warp repeats that symbol with the exact, full-depth search.
+// starts from the full 2^32 range (its scaled bounds are both 0) -- is thrown away and the whole warp repeats that symbol with
+// the exact, full-depth search.
 //
 // QUICK: for few warps, which wait for one another's results more than for issue slots: two levels of the search at once, the first two
 // from registers, and the reciprocal of a size taken beside its renormalisation shift and not behind it.  More instructions, and more
@@ -558,7 +561,8 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
             rare = false;
             CG_UNROLL
             for (int i = 0; i < NS; ++i)
-                a[i] = QUICK ? search_quarter<kTop / 2>(col[i], low_quarter[i], mid[i], high_quarter[i], ratio[i]) : search_step<kTop>(col[i], mid[i], ratio[i]);
+                a[i] = QUICK ? search_quarter<kTop / 2>(col[i], low_quarter[i], mid[i], high_quarter[i], ratio[i])
+                             : search_step<kTop>(col[i], mid[i], ratio[i]);
             CG_UNROLL
             for (int i = 0; i < NS; ++i) a[i] = QUICK ? QuarterSearch<FL - 3>::run(sm, a[i], ratio[i]) : RatioSearch<FL - 2>::run(sm, a[i], ratio[i]);
             uint32_t e0[NS], e1[NS];
@@ -595,7 +599,8 @@ CG_HD void decode_streams(Smem sm, const uint32_t (&col)[NS], uint32_t det, int 
                 st[i].span32 = cg_fshl(0u, u[i], s[i]);
                 st[i].p = p[i];
                 bits[i] = bw[i].bits(st[i].p);
-                ratio[i] = QUICK ? ratio_estimate(bits[i] - st[i].low, st[i].span32, reciprocal[i], s[i]) : ratio_estimate(bits[i] - st[i].low, st[i].span32);
+                const uint32_t offset = bits[i] - st[i].low;
+                ratio[i] = QUICK ? ratio_estimate(offset, st[i].span32, reciprocal[i], s[i]) : ratio_estimate(offset, st[i].span32);
             }
         }
         odd = cg_any_lane(lanes, rare);

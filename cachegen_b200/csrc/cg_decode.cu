@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(kGroup) decode_symbols_kernel(const SymDecodeP
 }
 
 // The same with two adjacent channels per thread, whose symbols are adjacent bytes (see decode_dequant_multi_kernel):
-// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk: 158 us under counters (168 with the window shifted at
-// every symbol), of which the last 272 of 2,048 blocks, which find no room beside the first, take a third.
+// 64 threads a block, one 16-bit store a token.  One 256-token Llama-7B chunk (2,048 blocks): 153 us under counters, eight blocks
+// an SM (see evened_blocks), 158 with twelve; 168 with the window shifted at every symbol.
 // Shared memory (the tables) allows 12 blocks per SM at the usual table length of 33; asking for no
 // more leaves the compiler 80 registers a thread, which it needs to interleave the NS chains.
 template <int LEVELS, int MODE>
@@ -254,7 +254,8 @@ __global__ void __launch_bounds__(kGroup / 2, kMultiBlocksPerSM) decode_symbols_
         *reinterpret_cast<uint16_t *>(o) = static_cast<uint16_t>(both);
         o += o1;
     };
-    if (shallow) decode_streams<(LEVELS > 3 ? LEVELS - 1 : LEVELS), 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, 0xFFFFFFFFu, emit);
+    constexpr int kShallow = LEVELS > 3 ? LEVELS - 1 : LEVELS;
+    if (shallow) decode_streams<kShallow, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, 0xFFFFFFFFu, emit);
     else decode_streams<LEVELS, 2, true>(Smem{}, col, 0u, p.lp - 2, LEVELS, streams, lens, p.ntokens, 0xFFFFFFFFu, emit);
 }
 
@@ -428,8 +429,9 @@ __global__ void __launch_bounds__(kGroup) decode_dequant_kernel(const __grid_con
 // warp still reads 32 different banks whatever entries its lanes are at.  The search depth is chosen
 // per block from the row's bin count (see decode_streams); the result does not depend on it.
 // Bound by instruction issue and by the two half-rate integer pipes (52.4 instructions for 32 symbols, four issue slots of
-// five).  8,192 Llama-7B tokens: 3.68 ms; 4.02 and 58.9 instructions with the window shifted at every symbol, the shift by
-// the interval's size less one, votes for the active lanes only, 64-bit steps and the tables staged by halves of words.
+// five).  8,192 Llama-7B tokens: 3.66 ms; 3.68 with the loop begun in front of its estimate; 4.02 and 58.9 instructions with the
+// window shifted at every symbol, the shift by the interval's size less one, votes for the active lanes only, 64-bit steps and the
+// tables staged by halves of words besides.
 // Needs a head size and output strides that are multiples of NS, output pointers aligned to 2*NS bytes and a block's output
 // within 32-bit offsets.
 template <int OUT_DT>
@@ -750,7 +752,8 @@ static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool ear
     if (!DELTA && blocks <= static_cast<int64_t>(kQuickBlocksPerSM) * sm_count())
         return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA, !DELTA>, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
     const auto kernel = decode_dequant_multi_kernel<NS, OUT_DT, DELTA, false>;
-    return launch(kernel, grid, kGroup / NS, DELTA ? smem : evened_smem(kernel, blocks, full, p.njobs, p.jobs[0].ntokens, smem), early, st, p, scale_dt, full);
+    const size_t asked = DELTA ? smem : evened_smem(kernel, blocks, full, p.njobs, p.jobs[0].ntokens, smem);
+    return launch(kernel, grid, kGroup / NS, asked, early, st, p, scale_dt, full);
 }
 
 // ---- group offsets ------------------------------------------------------------------------------------------
@@ -912,8 +915,9 @@ static int launch_offsets(const cg_decode_job *jobs, int njobs, int nrows, int n
     const int nslab = (nchannels + kGroup - 1) / kGroup;
     const int64_t groups = static_cast<int64_t>(nrows) * nslab;
     const auto run = [&](auto kernel, int blocks) {
-        return launch(kernel, dim3(static_cast<unsigned>(njobs * blocks)), kOffsetThreads, static_cast<size_t>((groups + blocks - 1) / blocks) * sizeof(int),
-                      true, st, o, nrows, nchannels, nslab, status, sizes, behind_another);
+        const size_t sums = static_cast<size_t>((groups + blocks - 1) / blocks) * sizeof(int);
+        return launch(kernel, dim3(static_cast<unsigned>(njobs * blocks)), kOffsetThreads, sums, true, st,
+                      o, nrows, nchannels, nslab, status, sizes, behind_another);
     };
     // Sixteen blocks where a warp of eight would take more than eight groups, in more than two rounds of loads.  20 tokens, us a
     // call with eight and with sixteen: 640 groups 12.8 and 13.1, 768 12.9 and 12.9, 1,280 16.9 and 15.8, 2,048 25.4 and 23.4.

@@ -23,7 +23,8 @@ constexpr int kPrefetch = 16;  // symbols fetched ahead of the coder
 
 // See store_encode_kernel's encode_again.
 template <class Offset>
-static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint8_t *base, Offset at, Offset s1, int n, uint32_t top, uint8_t *to, int64_t stride) {
+static __device__ __noinline__ uint32_t encode_again(uint32_t col, const uint8_t *base, Offset at, Offset s1, int n, uint32_t top,
+                                                     uint8_t *to, int64_t stride) {
     BitSink out;
     EncoderState enc;
     out.init(to, stride);

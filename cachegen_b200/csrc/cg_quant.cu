@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_cdf_kernel(
 // slab has column 32 j + l then (see entry_of), so that a warp's lanes are in 32 banks whatever they count.  Bound by issue and the
 // latencies of its loads and barriers: one 256-token Llama-7B chunk in 23.5 us (26 with sixteen tokens in flight, 30 with batches of
 // eight behind those of 32); 29.9 with eight in flight, the channels side by side, bytes picked in another order by each group of
-// lanes, and the counts summed before they were scaled; 36 with a condition at every load, 62 with a load per symbol.  The updates alone would take 12 us.  Otherwise (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
+// lanes, and the counts summed before they were scaled.  The updates alone would take 12 us.
+// Otherwise (arbitrary strides) thread (channel = tid % 128, token parity = tid / 128).
 template <bool VEC>
 __global__ void __launch_bounds__(kQuantThreads) symbol_cdf_kernel(const int8_t *__restrict__ sym, int64_t s0,
                                                                    int64_t s1, int64_t s2, int ntokens,
