@@ -677,13 +677,16 @@ struct BitSinkT {
             if (v) return;
         }
     }
-    // Moves the oldest 32 pending bits out where there are 32.  Up to 63 may have been pending before the last shift, by s <= 31, which
-    // moved bits out of the accumulator: `above` is its upper word before that shift (any where nacc < 64).  Straight-line
-    // code: every lane of the warp runs it whatever it needs.  Returns whether the held word, which went to the row (as number
-    // nwords - 2 now), has carried into those in front of it, which is left to the caller.
-    CG_HD bool store_word_if_full(uint32_t above, uint32_t s) {
+    // Moves the oldest 32 pending bits out where there are 32; needs nacc < 64.  Straight-line code: every lane of the
+    // warp runs it whatever it needs.  Returns whether the held word, which went to the row (as number nwords - 2 now), has
+    // carried into those in front of it, which is left to the caller.
+    // DEEP: up to 63 bits were pending before the last shift, by s <= 31, which moved bits out of the accumulator: `above` is
+    // its upper word before that shift.
+    template <bool DEEP = false>
+    CG_HD bool store_word_if_full(uint32_t above = 0u, uint32_t s = 0u) {
 #if defined(__CUDA_ARCH__)
         uint32_t w, held, carry, left;
+        if (DEEP)
         asm("{ .reg .pred p, q; .reg .u32 lo, hi, x;\n"
             "add.u32 %3, %6, -32;\n"
             "setp.ge.s32 p, %6, 32;\n"
@@ -693,10 +696,20 @@ struct BitSinkT {
             "selp.b32 hi, x, %5, q;\n"
             "shf.r.wrap.b32 %0, lo, hi, %3;\n"
             "shf.r.wrap.b32 %2, hi, 0, %3;\n"
-            "lop3.b32 %2, %2, %7, 1, 0x28;\n"    // (hi >> left ^ hold) & 1
+            "lop3.b32 %2, %2, %7, 1, 0x28;\n"
             "@!p mov.u32 %2, 0;\n"
             "add.u32 %1, %7, %2; }"
             : "=&r"(w), "=&r"(held), "=&r"(carry), "=&r"(left) : "r"(acc_lo), "r"(acc_hi), "r"(nacc), "r"(hold), "r"(above), "r"(s));
+        else
+        asm("{ .reg .pred p;\n"
+            "add.u32 %3, %6, -32;\n"
+            "setp.ge.s32 p, %6, 32;\n"
+            "shf.r.clamp.b32 %0, %4, %5, %3;\n"  // the low word of (hi:lo) >> left
+            "shf.r.clamp.b32 %2, %5, 0, %3;\n"
+            "lop3.b32 %2, %2, %7, 1, 0x28;\n"    // (acc_hi >> left ^ hold) & 1
+            "@!p mov.u32 %2, 0;\n"
+            "add.u32 %1, %7, %2; }"
+            : "=&r"(w), "=r"(held), "=&r"(carry), "=&r"(left) : "r"(acc_lo), "r"(acc_hi), "r"(nacc), "r"(hold));
         const bool room = !BOUNDED || nwords - 1u < cap_w;
         asm volatile("{ .reg .pred p, q;\n"
             "setp.ge.s32 p, %2, 32;\n"
@@ -712,7 +725,7 @@ struct BitSinkT {
         if (nacc < 32) return false;
         nacc -= 32;
         const uint32_t left = static_cast<uint32_t>(nacc) & 31u, x = s & 31u ? above >> (32u - (s & 31u)) : 0u;
-        const bool q = nacc >= 32;
+        const bool q = DEEP && nacc >= 32;
         const uint32_t carry = (((q ? x : acc_hi) >> left) ^ hold) & 1u;
         hold += carry;
         const bool over = hold < carry;
@@ -723,7 +736,7 @@ struct BitSinkT {
 #endif
     }
     CG_HD void store_and_carry() {
-        if (store_word_if_full(0u, 0u)) carry_into_row(nwords - 2u);
+        if (store_word_if_full()) carry_into_row(nwords - 2u);
     }
     // zero-fills to a byte boundary; returns the stream length in bytes
     CG_HD uint32_t finish() {
@@ -748,21 +761,30 @@ struct BitSinkT {
 using BitSink = BitSinkT<1>;
 
 // ---- encoder state and step -----------------------------------------------------------------------------
-// Pending bits from which on a lane makes its warp store a word.  The last symbol in front of a vote may shift pending bits out of
-// the accumulator, because its upper word from before that shift is kept (store_word_if_full): only what the symbols
-// before it add has to stay below bit 64, in a lane that is below the mark and in one that has just stored.  A symbol adds at
-// most 18 (the updated interval of a strictly increasing table spans at least 2^14 values).  A low mark costs: a stream that
-// has no whole word when another is at the mark is soon the next one there.  For two symbols of 256 counted tokens 54 where a
-// mark for what the accumulator holds is 44: a word's store every 22 bits of the fastest of a warp's streams, not every 13.
-constexpr int kHighWater = 64;  // one symbol a vote, of any table
-// Two symbols a vote, of tables counted from the `ntokens` symbols that are coded with them: a symbol that occurs has at
+// Pending bits from which on a lane makes its warp store a word.  Whatever stays below it, or below 32 after the store, has
+// to take `symbols` more symbols' bits below bit 63.  A symbol adds at most 18 (the updated interval of a
+// strictly increasing table spans at least 2^14 values).  These are the marks of a store without the upper word; the kernels
+// use those below, and of pair_high_water only whether it is 0.
+constexpr int kSinkHighWater = 44;
+// The same where the table was counted from the `ntokens` symbols that are coded with it: a symbol that occurs has at
 // least w = floor((0xFFFF - 63) / ntokens) + 1 of the 2^16 shares (normalize_cdf_value), hence an interval of
-// w * 2^14 - 1 values or more, and adds at most 18 - floor(log2 w) bits.  0: they may not fit.
-CG_HD int pair_high_water(int ntokens) {
+// w * 2^14 - 1 values or more, and adds at most 18 - floor(log2 w) bits.  0: two symbols may not fit.
+CG_HD int counted_symbol_bits(int ntokens) {
     const uint32_t w = (0xFFFFu - 63u) / static_cast<uint32_t>(ntokens) + 1u;
-    const int most = 18 - (31 - cg_clz(w));
-    return 31 + 2 * most > 63 ? 0 : 64 - most;
+    return 18 - (31 - cg_clz(w));
 }
+CG_HD int pair_high_water(int ntokens) {
+    const int most = counted_symbol_bits(ntokens);
+    if (31 + 2 * most > 63) return 0;
+    return 64 - 2 * most < kSinkHighWater ? 64 - 2 * most : kSinkHighWater;
+}
+// Marks where the last symbol in front of a vote may shift pending bits out of the accumulator, because its upper word from
+// before that shift is kept (store_word_if_full<true>): only what the symbols before it add has to stay below bit 64.  For two
+// symbols of 256 counted tokens 54 instead of 44, for one of any table 64: a stream that has not got a whole word when another is at
+// the mark is soon the next one there, so a word's store every 13 bits of the fastest of a warp's streams becomes one every 22.
+// The first only where pair_high_water is not 0: what a store leaves is below it then, too.
+CG_HD int deep_pair_high_water(int ntokens) { return 64 - counted_symbol_bits(ntokens); }
+constexpr int kDeepHighWater = 64;
 
 // The coder without the reference's count of pending bits.  low is the current 32-bit window of the
 // interval's lower end L, and all bits of L above the window are in the sink: a range update adds to
@@ -833,24 +855,17 @@ struct EncoderState {
     }
     // G symbols (1 or 2) of NS streams a lane, by the addresses of their table entries.  The streams' chains are independent,
     // and ONE warp vote after them covers a full word in an accumulator: every lane that has one stores it as soon as one
-    // lane is at the high-water mark (kHighWater for one symbol, pair_high_water for two).
+    // lane is at the high-water mark: with DEEP, as the kernels run it, kDeepHighWater for one symbol and deep_pair_high_water for
+    // two, without it kSinkHighWater and pair_high_water.
     // LAST: a symbol may be its table's last, whose upper bound is the range's end (told by `last`; G is 1 then).
     // What hardly ever happens is not mended here but left to encode_again: a carry through a whole word of ones
     // (`carried`), and a range of 2^31 at a multiple of it, which leaves a span of 0, from where on no symbol has a size, so
     // that the span is still 0 at the stream's end.  Code for the like inside the loop cost five executed instructions a
     // symbol without ever being run.
-    template <int ROW, int G, int NS, bool LAST = false, class Sink>
+    template <int ROW, int G, int NS, bool LAST = false, bool DEEP = false, class Sink>
     static CG_HD void steps_at(Smem sm, const uint32_t (&a)[G][NS], EncoderState (&enc)[NS], Sink (&out)[NS], int high_water,
                                uint32_t lanes, bool (&carried)[NS], bool last = false) {
-        uint32_t s[NS], above[NS];
-        const bool full = take_at<ROW, G, NS, LAST>(sm, a, enc, out, high_water, last, s, above);
-        if (cg_any_lane(lanes, full)) store_at(out, s, above, carried);
-    }
-    // Its two parts: the symbols, and whether a stream is at the mark; and the store.
-    template <int ROW, int G, int NS, bool LAST, class Sink>
-    static CG_HD bool take_at(Smem sm, const uint32_t (&a)[G][NS], EncoderState (&enc)[NS], Sink (&out)[NS], int high_water, bool last,
-                              uint32_t (&s)[NS], uint32_t (&above)[NS]) {
-        uint32_t e0[G][NS], e1[G][NS];
+        uint32_t e0[G][NS], e1[G][NS], s[NS], above[NS];
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -868,12 +883,10 @@ struct EncoderState {
         bool full = false;
 #pragma unroll
         for (int i = 0; i < NS; ++i) full |= out[i].nacc >= high_water;
-        return full;
-    }
-    template <int NS, class Sink>
-    static CG_HD void store_at(Sink (&out)[NS], const uint32_t (&s)[NS], const uint32_t (&above)[NS], bool (&carried)[NS]) {
+        if (cg_any_lane(lanes, full)) {
 #pragma unroll
-        for (int i = 0; i < NS; ++i) carried[i] |= out[i].store_word_if_full(above[i], s[i]);
+            for (int i = 0; i < NS; ++i) carried[i] |= out[i].template store_word_if_full<DEEP>(above[i], s[i]);
+        }
     }
     // whether a stream has met what steps_at leaves
     CG_HD bool unsettled(bool carried) const { return carried | (span32 == 0u); }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
     const auto code = [&](uint32_t sym) {
         largest = max(largest, sym);
         const uint32_t s = min(sym, top), a[1][1] = {{col + s * kRowBytes}};
-        EncoderState::steps_at<kRowBytes, 1, 1, true>(Smem{}, a, enc, out, kHighWater, 0xFFFFFFFFu, carried, s == top);
+        EncoderState::steps_at<kRowBytes, 1, 1, true, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried, s == top);
     };
     const Offset first = at;
     uint32_t buf[kPrefetch], next[kPrefetch];
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kGroup, 8) encode_kernel(const EncodeParams p)
 #pragma unroll
             for (int j = 0; j < kPrefetch; ++j) {
                 const uint32_t a[1][1] = {{col + buf[j] * kRowBytes}};
-                EncoderState::steps_at<kRowBytes, 1, 1>(Smem{}, a, enc, out, kHighWater, 0xFFFFFFFFu, carried);
+                EncoderState::steps_at<kRowBytes, 1, 1, false, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried);
             }
         }
 #pragma unroll

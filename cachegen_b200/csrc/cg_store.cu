@@ -361,7 +361,7 @@ struct StoreParams {
     const uint32_t *sym4;
     TableOut out;
     int ntokens, nchannels, lp, nrows, nsub;
-    int high_water;       // of two symbols a vote, see pair_high_water; 0: one
+    int high_water;       // of two symbols a vote, see deep_pair_high_water; 0: one
     uint8_t *scratch;     // [nsub, nrows, nslab, 4 warps, stride / 4 + 1, 32 lanes] words
     int64_t stride;
     int32_t *lengths;     // [nsub, nrows * C]
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
 #pragma unroll
             for (int k = 0; k < kWordsAhead; ++k) w[s][k] = 4 * k < n ? written_symbols(sp[s] + k * C) : 0u;
         }
-        const int high_water = G == 1 ? kHighWater : p.high_water;
+        const int high_water = G == 1 ? kDeepHighWater : p.high_water;
         constexpr int kAhead = 4 * kWordsAhead;
         int i = 0;
         for (;; i += kAhead) {
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
                     for (int g = 0; g < G; ++g)
 #pragma unroll
                         for (int s = 0; s < NS; ++s) a[g][s] = entry_of(col[s], w[s][k], j + g);
-                    EncoderState::steps_at<kWarpRow, G, NS>(Smem{}, a, enc, out, high_water, 0xFFFFFFFFu, carried);
+                    EncoderState::steps_at<kWarpRow, G, NS, false, true>(Smem{}, a, enc, out, high_water, 0xFFFFFFFFu, carried);
                 }
             }
 #pragma unroll
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(kGroup / NS, NS == 1 ? 8 : 12) store_encode_ke
                     for (int k = 0; k + 1 < kWordsAhead; ++k) w[s][k] = w[s][k + 1];
                 }
             }
-            EncoderState::steps_at<kWarpRow, 1, NS>(Smem{}, a, enc, out, kHighWater, 0xFFFFFFFFu, carried);
+            EncoderState::steps_at<kWarpRow, 1, NS, false, true>(Smem{}, a, enc, out, kDeepHighWater, 0xFFFFFFFFu, carried);
         }
         int bits = bad ? CG_S_BAD_SYMBOL : 0;
 #pragma unroll
@@ -1028,7 +1028,7 @@ static int encode_jobs(const cg_encode_kv_job *jobs, int njobs, bool alone, void
         p.lp = k.max_bins + 1;
         p.nrows = z.nrows;
         p.nsub = z.nsub;
-        p.high_water = pair_high_water(k.ntokens);
+        p.high_water = pair_high_water(k.ntokens) ? deep_pair_high_water(k.ntokens) : 0;
         p.scratch = ws + z.scratch;
         p.stride = z.stride;
         p.lengths = reinterpret_cast<int32_t *>(ws + z.lengths);

@@ -367,6 +367,14 @@ class _PendingChunk:
     def stream_ptr(self):
         return ctypes.c_void_p(self.on)
 
+    @property
+    def pointers(self):
+        return ctypes.c_void_p * self.nsub
+
+    @property
+    def length_pointers(self):
+        return self.pointers(*[t.data_ptr() for t in self.lengths])
+
     def another(self, info, max_bins):
         """The same KV at other bins, prepared like this chunk (one without delta coding or counts) and not enqueued."""
         if info.cpu.numel() != 2 * self.L:

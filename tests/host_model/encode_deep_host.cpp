@@ -1,5 +1,5 @@
-// Host build of the encoder's loop as a warp runs it (the two parts of EncoderState::steps_at in cachegen_b200/csrc/cg_coder.cuh, with a
-// vote over several streams between them), for the CPU tests.
+// Host build of the encoder's loop as the kernels run it (EncoderState and BitSinkT of cachegen_b200/csrc/cg_coder.cuh with the
+// accumulator's upper word kept), for the CPU tests.
 #include <cstring>
 #include <vector>
 
@@ -14,58 +14,60 @@ using namespace cg;
 extern "C" int ed_encode(const uint16_t *cdf, int lp, const uint8_t *sym, int n, int lanes, uint8_t *out, int64_t cap, int counted,
                          int32_t *len, uint8_t *again, int *most, int *deepest) {
     if (counted && !pair_high_water(counted)) return -2;
-    const int group = counted ? 2 : 1, mark = counted ? pair_high_water(counted) : kHighWater;
+    const int group = counted ? 2 : 1, mark = counted ? deep_pair_high_water(counted) : kDeepHighWater;
     const uint32_t top = static_cast<uint32_t>(lp - 2);
     std::vector<uint32_t> tab(static_cast<size_t>(lp) * kGroupChannels * lanes);
     std::vector<uint32_t> rows(static_cast<size_t>(lanes) * (cap / 4 + 2));
     using Sink = BitSinkT<1, false>;
-    struct Lane {  // as the parts of steps_at take them
-        EncoderState enc[1];
-        Sink sink[1];
-        uint32_t s[1], above[1];
-        bool carried[1] = {};
-    };
-    std::vector<Lane> lane(lanes);
+    std::vector<Sink> sink(lanes);
+    std::vector<EncoderState> enc(lanes);
+    std::vector<uint32_t> above(lanes), s(lanes);
     const auto column = [&](int i) { return Smem{reinterpret_cast<uint8_t *>(tab.data() + static_cast<size_t>(i) * lp * kGroupChannels)}; };
     const auto row = [&](int i) { return reinterpret_cast<uint8_t *>(rows.data() + static_cast<size_t>(i) * (cap / 4 + 2) + 1); };
     for (int i = 0; i < lanes; ++i) {
         for (int m = 0; m < lp - 1; ++m) column(i).st(m * kTableRowBytes, static_cast<uint32_t>(cdf[i * lp + m]) << 16);
-        lane[i].sink[0].init(row(i), cap);
-        lane[i].enc[0].init();
-        lane[i].enc[0].half_scale(lane[i].sink[0]);
+        sink[i].init(row(i), cap);
+        enc[i].init();
+        enc[i].half_scale(sink[i]);
+        again[i] = 0;
     }
     *most = *deepest = 0;
-    for (int t = 0; t < n; t += t + group <= n ? group : 1) {
+    int t = 0;
+    for (; t + group <= n; t += group) {
         bool full = false;
         for (int i = 0; i < lanes; ++i) {
-            Lane &l = lane[i];
-            const auto at = [&](int g) { return static_cast<uint32_t>(sym[(t + g) * lanes + i]) * kTableRowBytes; };
-            if (counted && t + group <= n) {
-                const uint32_t a[2][1] = {{at(0)}, {at(1)}};
-                full |= EncoderState::take_at<kTableRowBytes, 2, 1, false>(column(i), a, l.enc, l.sink, mark, false, l.s, l.above);
-            } else if (counted) {
-                const uint32_t a[1][1] = {{at(0)}};
-                full |= EncoderState::take_at<kTableRowBytes, 1, 1, false>(column(i), a, l.enc, l.sink, kHighWater, false, l.s, l.above);
-            } else {
-                const uint32_t a[1][1] = {{at(0)}};
-                full |= EncoderState::take_at<kTableRowBytes, 1, 1, true>(column(i), a, l.enc, l.sink, mark, sym[t * lanes + i] == top, l.s, l.above);
+            for (int g = 0; g < group; ++g) {
+                const uint32_t m = sym[(t + g) * lanes + i], a = m * kTableRowBytes;
+                const bool last = !counted && m == top;
+                s[i] = enc[i].take<false>(cg_umulhi(enc[i].span32, column(i).ld(a)),
+                                          last ? enc[i].span32 : cg_umulhi(enc[i].span32, column(i).ld(a + kTableRowBytes)), sink[i], above[i]);
             }
-            const int after = l.sink[0].nacc, before = after - static_cast<int>(l.s[0]);
+            const int before = sink[i].nacc - static_cast<int>(s[i]);
             *most = before > *most ? before : *most;
-            *deepest = after > *deepest ? after : *deepest;
+            *deepest = sink[i].nacc > *deepest ? sink[i].nacc : *deepest;
+            full |= sink[i].nacc >= mark;
         }
-        for (int i = 0; full && i < lanes; ++i) EncoderState::store_at(lane[i].sink, lane[i].s, lane[i].above, lane[i].carried);
+        for (int i = 0; full && i < lanes; ++i) again[i] |= sink[i].store_word_if_full<true>(above[i], s[i]);
     }
-    for (int i = 0; i < lanes; ++i) {
-        EncoderState &enc = lane[i].enc[0];
-        Sink &sink = lane[i].sink[0];
-        again[i] = enc.unsettled(lane[i].carried[0]);
-        if (again[i]) {
-            sink.init(row(i), cap);
-            enc.init();
-            for (int k = 0; k < n; ++k) enc.step_alone<kTableRowBytes>(column(i), sym[k * lanes + i] * kTableRowBytes, !counted && sym[k * lanes + i] == top, sink);
+    for (; t < n; ++t)
+        for (int i = 0; i < lanes; ++i) {
+            const uint32_t a[1][1] = {{static_cast<uint32_t>(sym[t * lanes + i]) * kTableRowBytes}};
+            EncoderState e[1] = {enc[i]};
+            Sink o[1] = {sink[i]};
+            bool carried[1] = {again[i] != 0};
+            EncoderState::steps_at<kTableRowBytes, 1, 1, false, true>(column(i), a, e, o, kDeepHighWater, 0u, carried);
+            enc[i] = e[0];
+            sink[i] = o[0];
+            again[i] = carried[0];
         }
-        len[i] = static_cast<int32_t>(enc.flush(sink));
+    for (int i = 0; i < lanes; ++i) {
+        if (enc[i].unsettled(again[i])) {
+            again[i] = 1;
+            sink[i].init(row(i), cap);
+            enc[i].init();
+            for (int k = 0; k < n; ++k) enc[i].step_alone<kTableRowBytes>(column(i), sym[k * lanes + i] * kTableRowBytes, !counted && sym[k * lanes + i] == top, sink[i]);
+        }
+        len[i] = static_cast<int32_t>(enc[i].flush(sink[i]));
         if (len[i] > cap) return -1;
         memcpy(out + static_cast<size_t>(i) * cap, row(i), len[i]);
     }

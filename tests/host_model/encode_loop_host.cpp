@@ -19,7 +19,7 @@ extern "C" int64_t el_encode(const uint16_t *cdf, int lp, const uint8_t *sym, in
         for (int t = 0; t < kGroupChannels; ++t) tab[m * kGroupChannels + t] = static_cast<uint32_t>(cdf[m]) << 16;
     Smem sm{reinterpret_cast<uint8_t *>(tab.data())};
     const uint32_t col[2] = {4u, 400u}, top = static_cast<uint32_t>(lp - 2);
-    const int high_water = counted ? pair_high_water(counted) : kHighWater;
+    const int high_water = counted ? pair_high_water(counted) : kSinkHighWater;
     if (!high_water) return -2;
     using Sink = BitSinkT<1>;
     std::vector<uint32_t> row[2];
@@ -43,8 +43,8 @@ extern "C" int64_t el_encode(const uint16_t *cdf, int lp, const uint8_t *sym, in
     }
     for (; t < n; ++t) {
         const uint32_t a[1][2] = {{col[0] + sym[t] * kTableRowBytes, col[1] + sym[t] * kTableRowBytes}};
-        if (counted) EncoderState::steps_at<kTableRowBytes, 1>(sm, a, enc, sink, kHighWater, 0u, carried);
-        else EncoderState::steps_at<kTableRowBytes, 1, 2, true>(sm, a, enc, sink, kHighWater, 0u, carried, sym[t] == top);
+        if (counted) EncoderState::steps_at<kTableRowBytes, 1>(sm, a, enc, sink, kSinkHighWater, 0u, carried);
+        else EncoderState::steps_at<kTableRowBytes, 1, 2, true>(sm, a, enc, sink, kSinkHighWater, 0u, carried, sym[t] == top);
         *most = sink[0].nacc > *most ? sink[0].nacc : *most;
     }
     int64_t len[2];

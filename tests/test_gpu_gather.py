@@ -139,13 +139,13 @@ def test_the_finest_bins_are_gathered_like_others():
         try:
             size = p.sizes()[0][1]
             out = torch.empty(size, dtype=torch.uint8, device="cuda")
-            pointer, lengths = ((ctypes.c_void_p * 1)(t.data_ptr()) for t in (out, p.lengths[0]))
+            pointer = p.pointers(out.data_ptr())
             best = float("inf")
             for _ in range(12):
                 a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 a.record()
                 for _ in range(20):
-                    _lib.check(p.lib.cg_encode_kv_gather(ctypes.byref(p.job), pointer, lengths, p.stream_ptr), "gather")
+                    _lib.check(p.lib.cg_encode_kv_gather(ctypes.byref(p.job), pointer, p.length_pointers, p.stream_ptr), "gather")
                 b.record()
                 b.synchronize()
                 best = min(best, a.elapsed_time(b))
