@@ -316,10 +316,13 @@ class DecodePlan:
         nslab = (C + _lib.CG_GROUP_CHANNELS - 1) // _lib.CG_GROUP_CHANNELS
         ngroups = NL * nslab
         njobs_total = sum(len(v.subs) for v in views)
-        status = _status_word(ws, dev)
-        row_offs = {kind: _row_offsets(ws, kind, host_bins, C, dev) for kind in _ROW_OFFSETS if any(v.table_kind == kind for v in views)}
+        status = ws.get("status")
+        if status is None or status.device != dev:
+            status = _status_word(ws, dev)
+        row_offs = {kind: _row_offsets(ws, kind, host_bins, C, dev) for kind in {v.table_kind for v in views} if kind in _ROW_OFFSETS}
         goff = ws.get("group_off")
-        if _keep_for_graph(ws, bins, status, *row_offs.values()):
+        if torch.cuda.is_current_stream_capturing():
+            _keep_for_graph(ws, bins, status, *row_offs.values())
             goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)  # of the graph's own memory
         elif goff is None or goff.numel() < njobs_total * ngroups or goff.device != dev:
             goff = torch.empty(njobs_total * ngroups, dtype=torch.int64, device=dev)
@@ -444,9 +447,9 @@ def decode_many(encoder_outputs: List[CacheGenGPUEncoderOutput], bins: torch.Ten
 def _decode_usual(encoder_outputs, bins, fmt, out_dtype, out, workspace, host_bins):
     """What DecodePlan(...).run() does for chunks, all of one kind, of plain contiguous tensors on the current GPU, in native code.
     None, and nothing has been done but for buffers that the workspace keeps, for any other chunks."""
-    if not encoder_outputs or type(encoder_outputs) is not list or fmt not in ("vllm", "huggingface") or out_dtype not in _DTYPES or not bins.is_cuda:
+    if not encoder_outputs or not _on_gpu(encoder_outputs[0]):  # asked first: the rest takes a tenth of a short chunk's call
         return None
-    if not _on_gpu(encoder_outputs[0]):  # asked first: the rest takes a tenth of a short chunk's call
+    if type(encoder_outputs) is not list or fmt not in ("vllm", "huggingface") or out_dtype not in _DTYPES or not bins.is_cuda:
         return None
     kind, piece, flat = CacheGenGPUEncoderOutput, CacheGenGPUBytestream, None
     if type(encoder_outputs[0]) is flat_format.FlatChunk:
@@ -488,10 +491,10 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
     n = len(encoder_outputs)
     groups = max(1, min(groups, n))
     first = encoder_outputs[0]
-    dev = _device_of(first) if _on_gpu(first) else torch.device("cuda", torch.cuda.current_device())
     if groups == 1 or _on_gpu(first):
         return decode_many(encoder_outputs, bins, fmt, out_dtype, out=out,
                            workspace=workspaces[0] if workspaces else None, delta=delta, host_bins=host_bins)
+    dev = torch.device("cuda", torch.cuda.current_device())
     L, H, D = bins.numel() // 2, first.num_heads, first.head_size
     total_T = sum(_chunk_tokens(eo) for eo in encoder_outputs)
     shape = (L, 2, total_T, H, D) if fmt == "vllm" else (L, 2, H, total_T, D)
