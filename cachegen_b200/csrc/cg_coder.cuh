@@ -46,12 +46,17 @@ constexpr int kMultiBlocksPerSM = 12;  // of the kernels with two channels a thr
 // settings: 32 layers x 32 heads (14 blocks an SM) 159.5 and 152.3 us, x 35 (16) 170.4 and 159.7, nine chunks of 32 x 4 (16) 169.7 and
 // 163.5; 70B settings: 80 x 14 (16) 174.5 and 162.3, 40 x 28 (16) 164.6 and 165.2.
 // Not where it would hold blocks back for longer than it saves: thirteen an SM (40 x 24 151.6 and 153.0), fourteen of several
-// chunks, whose blocks come in no order of their work (4 of 32 x 8, the last of 5 tokens, 124.4 and 141.7), short tables (17
-// entries, 40 x 25 134.9 and 138.1, nine chunks of level 1 at 64 tokens 46.1 and 47.1), few tokens (16 of 32 x 32 at 32 bins 20.7 and
-// 21.4) and delta coding (9 of 32 x 4 192.8 and 200.9).
-CG_HD int evened_blocks(int64_t blocks, int64_t sms, int levels, int chunks, int ntokens) {
+// chunks, whose blocks come in no order of their work (4 of 32 x 8, the last of 5 tokens, 124.4 and 141.7), few tokens (16 of
+// 32 x 32 at 32 bins 20.7 and 21.4) and delta coding (9 of 32 x 4 192.8 and 200.9).
+// Short tables (5 to 17 entries): one chunk's KV only, from thirteen and three quarters an SM on.  Half the 7B bins, 32 x 32 141.3 and
+// 136.2, x 34 152.8 and 143.7, x 36 155.7 and 144.4; a quarter of them 126.1 and 120.1, 136.2 and 128.9, 140.0 and 130.1; rows that
+// are all alike 150.3 and 143.4, 151.9 and 153.4, 153.5 and 155.0.  Below, a fourteenth block that most SMs have not got costs more
+// than it gives (40 x 25 135.1 and 138.2); so do several chunks (nine of level 1 at 64 tokens 46.1 and 47.1) and, with rows alike,
+// symbols (32 x 32 85.5 and 94.7 for 150 tokens, where half the bins take 86.7 and 82.0).
+CG_HD int evened_blocks(int64_t blocks, int64_t sms, int levels, bool symbols, int chunks, int ntokens) {
     const int64_t more = (blocks + sms - 1) / sms - kMultiBlocksPerSM;
-    if (levels != 5 || ntokens < 64 || more > 4) return 0;
+    if (levels < 3 || levels > 5 || ntokens < 64 || more > 4) return 0;
+    if (levels < 5 && (symbols || chunks > 1 || 4 * blocks < 55 * sms)) return 0;
     return more > 2 ? 10 : more == 2 && chunks == 1 ? 8 : 0;
 }
 

@@ -687,9 +687,9 @@ static_assert((CG_MAX_LP + 1) * kRowBytes + 4 * (kSubTokens + 2 * CG_MAX_LP) + 6
 
 // Shared memory to ask for so that a grid has as many blocks an SM as evened_blocks says.
 template <class Kernel>
-static size_t evened_smem(Kernel kernel, int64_t blocks, int levels, int chunks, int ntokens, size_t dynamic) {
+static size_t evened_smem(Kernel kernel, int64_t blocks, int levels, bool symbols, int chunks, int ntokens, size_t dynamic) {
     constexpr int64_t kSmemPerSM = 228 * 1024, kReserved = 1024;  // bytes of an SM, of each block
-    const int resident = evened_blocks(blocks, sm_count(), levels, chunks, ntokens);
+    const int resident = evened_blocks(blocks, sm_count(), levels, symbols, chunks, ntokens);
     cudaFuncAttributes at;
     if (!resident || cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return dynamic;
     const int64_t fixed = static_cast<int64_t>(at.sharedSizeBytes) + kReserved;
@@ -706,7 +706,7 @@ static int launch_symbols(const SymDecodeParams &p, int nrows, cudaStream_t st) 
     const bool pairs = p.o2 == 1 && ((p.o0 | p.o1 | p.nchannels) & 1) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 1) == 0;
 #define CG_LAUNCH_SYM(L)                                                                                      \
     return pairs ? launch(decode_symbols_pair_kernel<L, MODE>, grid, kGroup / 2,                               \
-                          evened_smem(decode_symbols_pair_kernel<L, MODE>, blocks, L, 1, p.ntokens, table_bytes(p.lp, L)), MODE == 2, st, p) \
+                          evened_smem(decode_symbols_pair_kernel<L, MODE>, blocks, L, true, 1, p.ntokens, table_bytes(p.lp, L)), MODE == 2, st, p) \
                  : launch(decode_symbols_kernel<L, MODE>, grid, kGroup, table_bytes(p.lp, L), MODE == 2, st, p)
     if (need <= 3) CG_LAUNCH_SYM(3);
     if (need == 4) CG_LAUNCH_SYM(4);
@@ -752,7 +752,7 @@ static int launch_fused_multi(const FusedDecodeParams &p, int scale_dt, bool ear
     if (!DELTA && blocks <= static_cast<int64_t>(kQuickBlocksPerSM) * sm_count())
         return launch(decode_dequant_multi_kernel<NS, OUT_DT, DELTA, !DELTA>, grid, kGroup / NS, smem, early, st, p, scale_dt, full);
     const auto kernel = decode_dequant_multi_kernel<NS, OUT_DT, DELTA, false>;
-    const size_t asked = DELTA ? smem : evened_smem(kernel, blocks, full, p.njobs, p.jobs[0].ntokens, smem);
+    const size_t asked = DELTA ? smem : evened_smem(kernel, blocks, full, false, p.njobs, p.jobs[0].ntokens, smem);
     return launch(kernel, grid, kGroup / NS, asked, early, st, p, scale_dt, full);
 }
 

@@ -109,6 +109,6 @@ extern "C" int hm_decode_pair(const uint16_t *cdf0, const uint16_t *cdf1, int lp
 }
 
 extern "C" int hm_fast_levels_for(int nsym, int full_levels) { return fast_levels_for(nsym, full_levels); }
-extern "C" int hm_evened_blocks(int64_t blocks, int64_t sms, int levels, int chunks, int ntokens) {
-    return evened_blocks(blocks, sms, levels, chunks, ntokens);
+extern "C" int hm_evened_blocks(int64_t blocks, int64_t sms, int levels, int symbols, int chunks, int ntokens) {
+    return evened_blocks(blocks, sms, levels, symbols != 0, chunks, ntokens);
 }

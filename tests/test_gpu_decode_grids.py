@@ -70,8 +70,8 @@ def test_symbols_come_back_at_either_side_of_a_wave(rows, channels):
 @pytest.mark.parametrize("heads, bins, tokens, delta", [(31, 32, 64, None), (32, 32, 70, None), (34, 32, 64, None), (37, 32, 65, None),
                                                         (32, 16, 64, None), (32, 8, 64, None), (32, 62, 64, None), (32, 32, 63, None), (34, 32, 64, 16)])
 def test_grids_with_blocks_held_back(heads, bins, tokens, delta):
-    """One chunk of 14 to 16 blocks an SM, some of them held back, and the same streams twice in a grid that holds none back; tables of
-    other lengths, fewer tokens and delta coding, where none are."""
+    """One chunk of 14 to 16 blocks an SM, some of them held back, and the same streams twice in a grid that holds none back; long
+    tables, fewer tokens and delta coding, where none are."""
     from cachegen_b200.serde import cachegen_decoder as M
     from cachegen_b200.serde import cachegen_encoder as E
     from cachegen_b200.serde.cachegen_basics import DeltaCoding

@@ -132,10 +132,15 @@ def test_search_depth_for_a_bin_count(host_model):
 
 
 def test_blocks_are_held_back_where_it_was_found_to_gain(host_model):
-    f = lambda blocks, levels=5, chunks=1, tokens=256: host_model.hm_evened_blocks(ctypes.c_int64(blocks), ctypes.c_int64(148), levels, chunks, tokens)
+    def f(blocks, levels=5, chunks=1, tokens=256, symbols=0):
+        return host_model.hm_evened_blocks(ctypes.c_int64(blocks), ctypes.c_int64(148), levels, symbols, chunks, tokens)
     assert [f(148 * n) for n in (1, 12, 13, 14, 15, 16, 17, 30)] == [0, 0, 0, 8, 10, 10, 0, 0]
     assert [f(148 * 13 + 1), f(148 * 16 + 1)] == [8, 0]
     assert [f(148 * n, chunks=4) for n in (12, 13, 14, 15, 16, 17)] == [0, 0, 0, 10, 10, 0]
-    for levels in (2, 3, 4, 6):
+    for levels in (2, 6):
         assert not f(2048, levels) and not f(2240, levels)
+    for levels in (3, 4):
+        assert [f(n, levels) for n in (148 * 13, 2034, 2035, 2072, 2073, 148 * 16, 148 * 16 + 1)] == [0, 0, 8, 8, 10, 10, 0]
+        assert not f(2048, levels, chunks=2) and not f(2048, levels, symbols=1) and not f(2048, levels, tokens=63)
+    assert f(2048, symbols=1) == 8
     assert [f(2048, tokens=t) for t in (1, 63, 64)] == [0, 0, 8]
