@@ -504,6 +504,7 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
         raise RuntimeError("output tensor has the wrong shape")
     copy_stream = _copy_stream(dev)
     cur = torch.cuda.current_stream(dev)
+    captured = torch.cuda.is_current_stream_capturing()  # and so is the copy stream, which waits for it
     copy_stream.wait_stream(cur)
     if workspaces is None:
         workspaces = [dict() for _ in range(groups)]
@@ -516,7 +517,7 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
         tg = sum(_chunk_tokens(eo) for eo in part)
         view = out[:, :, t0:t0 + tg] if fmt == "vllm" else out[:, :, :, t0:t0 + tg]
         with torch.cuda.stream(copy_stream):
-            part = _stage_flat(part, workspaces[g], dev)
+            part = _stage_flat(part, workspaces[g], dev, captured)
             plan = DecodePlan(part, bins, fmt, out_dtype, out=view, workspace=workspaces[g], device=dev, delta=delta,
                               host_bins=host_bins)
             ready = torch.cuda.Event()
@@ -530,7 +531,7 @@ def decode_many_pipelined(encoder_outputs: List[CacheGenGPUEncoderOutput], bins:
     return out
 
 
-def _stage_flat(part: list, ws: dict, dev) -> list:
+def _stage_flat(part: list, ws: dict, dev, captured: bool) -> list:
     """Copies a group's CGB2 containers from host memory into one device buffer that the workspace
     keeps between calls (no allocation per call, nothing for the caching allocator to hold back while
     the previous call's kernels still run).  Chunks of other kinds are returned as they are."""
@@ -545,7 +546,8 @@ def _stage_flat(part: list, ws: dict, dev) -> list:
         with torch.inference_mode(False):
             arena = torch.empty(need, dtype=torch.uint8, device=dev)
         ws["arena"] = arena
-    _keep_for_graph(ws, arena)
+    if captured:
+        _keep_for_graph(ws, arena)
     staged = []
     for eo, a in zip(part, starts):
         dst = arena[a:a + eo.blob.numel()]
